@@ -3,6 +3,7 @@
 // routes the shapes they cover to the tcgen05 kernels declared in tc_kernels.cuh.
 #include <cuda_fp16.h>
 
+#include <algorithm>
 #include <cmath>
 #include <cstring>
 #include <map>
@@ -30,6 +31,9 @@ static void profile_collect(lf_context* ctx) {
 }
 
 
+void lf_block_cache_context(int device, int change);
+void lf_block_cache_release(int device);
+
 lf_status lf_arena_ensure(lf_context* ctx, size_t bytes) {
   if (ctx->arena_limit && bytes > ctx->arena_limit)
     return lf_fail(ctx, LF_ERR_MEMORY, "scratch arena of %zu bytes exceeds the limit of %zu bytes set for this context", bytes, ctx->arena_limit);
@@ -41,6 +45,7 @@ lf_status lf_arena_ensure(lf_context* ctx, size_t bytes) {
   cudaError_t e = cudaMalloc(&ctx->arena, want);
   if (e != cudaSuccess) {
     cudaGetLastError();
+    lf_block_cache_release(ctx->device);
     want = lf_align_up(bytes, (size_t)1 << 21);
     e = cudaMalloc(&ctx->arena, want);
   }
@@ -98,6 +103,7 @@ static lf_status context_create(int device_ordinal, void* stream, bool make_stre
       });
   }
   if (cudaMalloc(&ctx->tc_status, 16) == cudaSuccess) cudaMemset(ctx->tc_status, 0, 16);
+  lf_block_cache_context(device_ordinal, 1);
   *out = ctx;
   return LF_OK;
 }
@@ -108,6 +114,8 @@ void lf_context_destroy(lf_context* ctx) {
   profile_collect(ctx);
   if (ctx->arena) cudaFree(ctx->arena);
   if (ctx->tc_status) cudaFree(ctx->tc_status);
+  if (ctx->pinned) cudaFreeHost(ctx->pinned);
+  lf_block_cache_context(ctx->device, -1);
   if (ctx->ev0) cudaEventDestroy(ctx->ev0);
   if (ctx->ev1) cudaEventDestroy(ctx->ev1);
   if (ctx->owns_stream) cudaStreamDestroy(ctx->stream);
@@ -162,6 +170,10 @@ void lf_context_release_scratch(lf_context* ctx) {
   if (ctx->arena) cudaFree(ctx->arena);
   ctx->arena = nullptr;
   ctx->arena_bytes = 0;
+  if (ctx->pinned) cudaFreeHost(ctx->pinned);
+  ctx->pinned = nullptr;
+  ctx->pinned_used = 0;
+  lf_block_cache_release(ctx->device);
 }
 
 }  // extern "C"
@@ -188,8 +200,7 @@ void put_columns(hvec& dst, int total, int col0, const float* src, int in, int n
     for (int j = 0; j < n; ++j) dst[(size_t)i * total + col0 + j] = src[(size_t)i * src_ld + src_col0 + (size_t)j * src_step];
 }
 
-// Tensors of one operator are staged here while it is being built, then go to the device in one
-// allocation with one synchronisation (finish_uploads).
+// The layout functions hand their arrays over here, one per slot.
 struct PendingUploads {
   struct Item { int slot; hvec data; };
   std::vector<Item> items;
@@ -200,36 +211,6 @@ lf_status upload(lf_context* ctx, lf_weights* w, int slot, hvec host) {
   (void)ctx; (void)w;
   g_pending.items.push_back({slot, std::move(host)});
   return LF_OK;
-}
-
-lf_status finish_uploads(lf_context* ctx, lf_weights* w) {
-  size_t total = 0;
-  std::vector<size_t> offset;
-  for (auto& it : g_pending.items) {
-    offset.push_back(total);
-    total += lf_align_up(it.data.size() * sizeof(float) + 4, 256);
-  }
-  char* base = nullptr;
-  cudaError_t e = cudaMalloc(&base, total ? total : 256);
-  if (e != cudaSuccess) {
-    g_pending.items.clear();
-    cudaGetLastError();
-    return lf_fail(ctx, LF_ERR_MEMORY, "weight allocation of %zu bytes refused: %s", total, cudaGetErrorString(e));
-  }
-  w->owned.push_back(base);
-  lf_status s = LF_OK;
-  for (size_t i = 0; i < g_pending.items.size() && s == LF_OK; ++i) {
-    auto& it = g_pending.items[i];
-    float* dev = reinterpret_cast<float*>(base + offset[i]);
-    if (!it.data.empty() &&
-        cudaMemcpyAsync(dev, it.data.data(), it.data.size() * sizeof(float), cudaMemcpyHostToDevice, ctx->stream) != cudaSuccess) {
-      cudaGetLastError();
-      s = lf_fail(ctx, LF_ERR_CUDA, "weight upload failed");
-    }
-    w->f[it.slot] = dev;
-  }
-  if (cudaStreamSynchronize(ctx->stream) != cudaSuccess && s == LF_OK) s = lf_fail(ctx, LF_ERR_CUDA, "weight upload failed");
-  return s;      // the staged host copies stay until the tensor-core repacks have read them (lf_weights_create)
 }
 
 struct Expect { const char* name; int64_t count; };
@@ -490,7 +471,7 @@ lf_status build_opm_af2(lf_context* ctx, lf_weights* w, const float* const* t, c
 
 }  // namespace
 
-// Lays the operator's tensors out in the canonical arrays (staged on the host in g_pending).
+// Lays the operator's tensors out in the canonical arrays (on the host, in g_pending).
 static lf_status build_weights(lf_context* ctx, lf_weights* w, const float* const* tensors, const int64_t* counts, int n_tensors) {
   switch (w->kind) {
     case LF_WEIGHTS_TRIANGLE_AF2: return build_triangle_af2(ctx, w, tensors, counts, n_tensors);
@@ -508,16 +489,93 @@ static lf_status build_weights(lf_context* ctx, lf_weights* w, const float* cons
 }
 
 // ---------------------------------------------------------------------------
-// Weights from encoded tensors (int5 payloads as they sit in a bundle): the codes go to the device as they
-// are and one gather kernel decodes them straight into the canonical arrays, through a layout map that says,
-// for every element of every canonical array, which input tensor and which of its elements it is (or that it
-// is a constant zero).  The map is derived from the very functions that lay out float32 inputs, by running
-// them on stand-in tensors that hold their own element numbers, so the two paths cannot disagree; it
-// depends only on the operator's kind and shape and is cached per device.
+// Device memory of weights.  One block per operator holds its canonical arrays and everything derived from them; blocks
+// of closed operators wait in a cache per GPU for the next ones (a stack runner given weight objects prepares and closes
+// seven operators a block and call: an allocation and a release each cost 0.1 to 0.3 ms and a device synchronisation).
+// The cache is bounded, serves every context and thread of the process, and is given back when the GPU's last context
+// goes or scratch is released.  A block enters it only after the device is idle, so whichever stream takes it next is safe.
+
+namespace {
+
+constexpr size_t kBlockCacheLimit = (size_t)256 << 20;
+struct BlockCache {
+  std::mutex mutex;
+  std::multimap<size_t, void*> free;
+  size_t bytes = 0;
+  int contexts = 0;
+};
+BlockCache g_blocks[64];
+
+void block_cache_trim(int device) {      // with the cache's lock held
+  BlockCache& c = g_blocks[device];
+  for (auto& b : c.free) cudaFree(b.second);
+  c.free.clear();
+  c.bytes = 0;
+}
+
+// Sizes are rounded up to 64 KiB and reused for requests of at least three quarters of them.
+cudaError_t weight_block_take(int device, size_t want, void** out, size_t* got) {
+  const size_t size = lf_align_up(want ? want : 1, (size_t)1 << 16);
+  if (device >= 64) { *got = size; return cudaMalloc(out, size); }
+  std::lock_guard<std::mutex> lock(g_blocks[device].mutex);
+  BlockCache& c = g_blocks[device];
+  auto fit = c.free.lower_bound(size);
+  if (fit != c.free.end() && fit->first / 4 * 3 <= size) {
+    *out = fit->second;
+    *got = fit->first;
+    c.bytes -= fit->first;
+    c.free.erase(fit);
+    return cudaSuccess;
+  }
+  cudaError_t e = cudaMalloc(out, size);
+  if (e != cudaSuccess) {
+    cudaGetLastError();
+    block_cache_trim(device);
+    e = cudaMalloc(out, size);
+    if (e != cudaSuccess) cudaGetLastError();
+  }
+  *got = size;
+  return e;
+}
+
+// The caller has waited for the device.
+void weight_block_give(int device, void* block, size_t size) {
+  if (device >= 64) { cudaFree(block); return; }
+  std::lock_guard<std::mutex> lock(g_blocks[device].mutex);
+  BlockCache& c = g_blocks[device];
+  if (c.contexts == 0 || c.bytes + size > kBlockCacheLimit) { cudaFree(block); return; }
+  c.free.emplace(size, block);
+  c.bytes += size;
+}
+
+}  // namespace
+
+void lf_block_cache_context(int device, int change) {
+  if (device < 0 || device >= 64) return;
+  std::lock_guard<std::mutex> lock(g_blocks[device].mutex);
+  g_blocks[device].contexts += change;
+  if (change <= 0 && g_blocks[device].contexts <= 0) block_cache_trim(device);
+}
+
+void lf_block_cache_release(int device) {
+  if (device < 0 || device >= 64) return;
+  std::lock_guard<std::mutex> lock(g_blocks[device].mutex);
+  block_cache_trim(device);
+}
+
+// ---------------------------------------------------------------------------
+// Weights from the caller's tensors, float32 or encoded (int5 payloads as they sit in a bundle): the bytes go to the
+// device as they are, in one copy, and one gather kernel decodes and lays them out in the canonical arrays, through a
+// layout map that says, for every element of every canonical array, which input tensor and which of its elements it is
+// (or that it is a constant zero).  The map is derived from the layout functions above, by running them once on stand-in
+// tensors that hold their own element numbers; it depends only on the operator's kind and shape and is cached per
+// device.  Nothing here waits for the device: a later operator's bytes are staged while an earlier one's are laid out.
 
 namespace {
 
 constexpr int kMaxSources = 16;
+constexpr int32_t kMapZero = -1;
+constexpr int kMapIndexBits = 26;         // map entry: source tensor << 26 | element (limits an encoded tensor to 2^24 elements anyway)
 struct SourceTable {
   const uint8_t* base[kMaxSources];
   const __half* scales[kMaxSources];
@@ -529,9 +587,10 @@ __global__ void gather_decode_kernel(const int32_t* __restrict__ map, int64_t co
                                      float* __restrict__ out) {
   const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= count) return;
-  const int32_t tensor = map[2 * i], index = map[2 * i + 1];
+  const int32_t entry = map[i];
   float v = 0.f;
-  if (tensor >= 0) {
+  if (entry != kMapZero) {
+    const int tensor = entry >> kMapIndexBits, index = entry & ((1 << kMapIndexBits) - 1);
     const int block = src.block[tensor];
     if (block == 0) {
       v = reinterpret_cast<const float*>(src.base[tensor])[index];
@@ -546,47 +605,203 @@ __global__ void gather_decode_kernel(const int32_t* __restrict__ map, int64_t co
 }
 
 struct LayoutMaps {
-  std::vector<std::vector<int32_t>> slot;      // per canonical array: (tensor, element) pairs; tensor -1 = zero
+  std::vector<int32_t> map;                    // all canonical arrays, one after the other on 256-byte boundaries (kMapZero between them)
+  std::vector<size_t> offset;                  // element offset of each slot's array
+  std::vector<bool> present;
   lf_weights flags;                            // what the layout functions set besides the arrays
-  int32_t* device[64] = {nullptr};             // per device ordinal: all slots' maps, one after the other
+  int32_t* device[64] = {nullptr};
 };
 std::mutex g_maps_mutex;
 std::map<std::vector<int64_t>, LayoutMaps> g_maps;
 
-// Runs the layout functions once per input tensor, that tensor holding 1, 2, 3, ... and the others zeros: a
-// canonical element that comes out as v > 0 is element v - 1 of that tensor.
+// Runs the layout functions once on tensors whose elements are numbered 1, 2, 3, ... through all of them: a canonical
+// element that comes out as v > 0 is element v - 1 of that numbering, 0 is a constant zero.
 lf_status derive_maps(lf_context* ctx, int kind, const lf_weight_dims& dims, const int64_t* counts, int n, LayoutMaps& maps) {
   std::vector<std::vector<float>> fake(n);
   std::vector<const float*> ptr(n);
+  std::vector<int64_t> first(n + 1, 0);
+  for (int i = 0; i < n; ++i) first[i + 1] = first[i] + counts[i];
+  if (first[n] >= (1 << 24))
+    return lf_fail(ctx, LF_ERR_UNSUPPORTED, "the operator's tensors have %lld elements; a layout map holds up to 16777215", (long long)first[n]);
+  if (first[n] == 0) return lf_fail(ctx, LF_ERR_ARGUMENT, "no tensor has any element");
   for (int i = 0; i < n; ++i) {
-    if (counts[i] >= (1 << 24)) return lf_fail(ctx, LF_ERR_UNSUPPORTED, "tensor %d has %lld elements; encoded tensors are limited to 16777215", i, (long long)counts[i]);
-    fake[i].assign((size_t)counts[i], 0.f);
+    fake[i].resize((size_t)counts[i]);
+    for (int64_t e = 0; e < counts[i]; ++e) fake[i][(size_t)e] = (float)(first[i] + e + 1);
     ptr[i] = counts[i] ? fake[i].data() : nullptr;
   }
-  for (int i = 0; i < n; ++i) {
-    if (!counts[i]) continue;
-    for (int64_t e = 0; e < counts[i]; ++e) fake[i][(size_t)e] = (float)(e + 1);
-    lf_weights tmp;
-    tmp.kind = kind;
-    tmp.dims = dims;
-    g_pending.items.clear();
-    lf_status s = build_weights(ctx, &tmp, ptr.data(), counts, n);
-    if (s != LF_OK) { g_pending.items.clear(); return s; }
-    if (maps.slot.empty()) {
-      maps.slot.resize(tmp.f.size());
-      for (auto& it : g_pending.items) maps.slot[it.slot].assign(it.data.size() * 2, -1);
-      maps.flags = tmp;
-      maps.flags.f.clear();
+  lf_weights tmp;
+  tmp.kind = kind;
+  tmp.dims = dims;
+  g_pending.items.clear();
+  lf_status s = build_weights(ctx, &tmp, ptr.data(), counts, n);
+  if (s != LF_OK) { g_pending.items.clear(); return s; }
+  maps.offset.assign(tmp.f.size(), 0);
+  maps.present.assign(tmp.f.size(), false);
+  for (auto& it : g_pending.items) {
+    maps.offset[it.slot] = maps.map.size();
+    maps.present[it.slot] = true;
+    for (float v : it.data) {
+      if (v <= 0.f) { maps.map.push_back(kMapZero); continue; }
+      const int64_t id = (int64_t)v - 1;
+      const int t = (int)(std::upper_bound(first.begin(), first.end(), id) - first.begin()) - 1;
+      maps.map.push_back((int32_t)((int64_t)t << kMapIndexBits | (id - first[t])));
     }
-    for (auto& it : g_pending.items) {
-      auto& m = maps.slot[it.slot];
-      for (size_t e = 0; e < it.data.size(); ++e)
-        if (it.data[e] > 0.f) { m[2 * e] = i; m[2 * e + 1] = (int32_t)it.data[e] - 1; }
-    }
-    g_pending.items.clear();
-    std::fill(fake[i].begin(), fake[i].end(), 0.f);
+    maps.map.resize(lf_align_up(maps.map.size() + 1, 64), kMapZero);
   }
-  if (maps.slot.empty()) return lf_fail(ctx, LF_ERR_ARGUMENT, "no tensor has any element");
+  g_pending.items.clear();
+  maps.flags = tmp;
+  maps.flags.f.clear();
+  return LF_OK;
+}
+
+// Host bytes -> device through the context's pinned staging buffer; the source may be freed on return.
+constexpr size_t kPinnedBytes = (size_t)16 << 20;
+lf_status staged_upload(lf_context* ctx, const lf_encoded_tensor* tensors, const size_t* sizes, const size_t* offsets, int n, uint8_t* dst) {
+  if (!ctx->pinned && cudaMallocHost(&ctx->pinned, kPinnedBytes) != cudaSuccess) {
+    cudaGetLastError();
+    ctx->pinned = nullptr;
+    return lf_fail(ctx, LF_ERR_MEMORY, "pinned staging of %zu bytes refused", kPinnedBytes);
+  }
+  // tensors follow each other on the device as they do in the staging buffer: one copy for as many as fit
+  size_t run_src = 0, run_dst = 0, run = 0;
+  auto send = [&]() -> lf_status {
+    if (run) LF_CUDA(ctx, cudaMemcpyAsync(dst + run_dst, ctx->pinned + run_src, run, cudaMemcpyHostToDevice, ctx->stream));
+    run = 0;
+    return LF_OK;
+  };
+  for (int i = 0; i < n; ++i) {
+    for (size_t done = 0; done < sizes[i];) {
+      const size_t at = offsets[i] + done;
+      // keep the distance between tensors inside a run
+      size_t pos = run ? run_src + (at - run_dst) : lf_align_up(ctx->pinned_used, 256) + (at & 255);
+      if (pos >= kPinnedBytes) {
+        LF_TRY(send());
+        LF_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
+        pos = at & 255;
+      }
+      if (!run) { run_src = pos; run_dst = at; }
+      const size_t part = std::min(sizes[i] - done, kPinnedBytes - pos);
+      memcpy(ctx->pinned + pos, static_cast<const uint8_t*>(tensors[i].data) + done, part);
+      done += part;
+      run = pos + part - run_src;
+      ctx->pinned_used = pos + part;
+    }
+  }
+  return send();
+}
+
+void fill_flags(lf_weights* w, const lf_weights& from) {
+  w->dims = from.dims;
+  w->has_gate_bias = from.has_gate_bias; w->has_out_bias = from.has_out_bias;
+  w->has_pair_norm = from.has_pair_norm; w->has_pair_proj = from.has_pair_proj;
+}
+
+// The block of w: `canonical` bytes of canonical arrays, then what prepare_weights derives from them.
+lf_status take_block(lf_context* ctx, lf_weights* w, size_t canonical) {
+  WeightCursor dry{nullptr, canonical, true};
+  LF_TRY(tc::prepare_weights(ctx, w, dry));
+  if (weight_block_take(ctx->device, dry.offset, &w->block, &w->block_bytes) != cudaSuccess) {
+    w->block = nullptr;
+    return lf_fail(ctx, LF_ERR_MEMORY, "weight allocation of %zu bytes refused", dry.offset);
+  }
+  return LF_OK;
+}
+
+// Tensors too large for a layout map: laid out on the host, copied array by array.
+lf_status create_on_host(lf_context* ctx, lf_weights* w, const float* const* tensors, const int64_t* counts, int n) {
+  LF_TRY(build_weights(ctx, w, tensors, counts, n));
+  size_t total = 0;
+  for (auto& it : g_pending.items) total += lf_align_up(it.data.size() * sizeof(float) + 4, 256);
+  LF_TRY(take_block(ctx, w, total));
+  char* base = static_cast<char*>(w->block);
+  size_t at = 0;
+  for (auto& it : g_pending.items) {
+    w->f[it.slot] = reinterpret_cast<float*>(base + at);
+    if (!it.data.empty())
+      LF_CUDA(ctx, cudaMemcpyAsync(base + at, it.data.data(), it.data.size() * sizeof(float), cudaMemcpyHostToDevice, ctx->stream));
+    at += lf_align_up(it.data.size() * sizeof(float) + 4, 256);
+  }
+  LF_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
+  WeightCursor cur{base, total, false};
+  return tc::prepare_weights(ctx, w, cur);
+}
+
+// The layout map of this operator, on this context's device.
+lf_status find_maps(lf_context* ctx, int kind, const lf_weight_dims& dims, const std::vector<int64_t>& counts, LayoutMaps** out) {
+  std::vector<int64_t> key = {(int64_t)kind, dims.channels, dims.hidden, dims.heads, dims.head_dim, dims.pair_channels, dims.out_channels};
+  key.insert(key.end(), counts.begin(), counts.end());
+  std::lock_guard<std::mutex> lock(g_maps_mutex);
+  auto found = g_maps.find(key);
+  if (found == g_maps.end()) {
+    LayoutMaps fresh;
+    LF_TRY(derive_maps(ctx, kind, dims, counts.data(), (int)counts.size(), fresh));
+    found = g_maps.emplace(key, std::move(fresh)).first;
+  }
+  LayoutMaps& maps = found->second;
+  if (!maps.device[ctx->device]) {
+    int32_t* dev = nullptr;
+    LF_CUDA(ctx, cudaMalloc(&dev, maps.map.size() * sizeof(int32_t)));
+    cudaError_t e = cudaMemcpyAsync(dev, maps.map.data(), maps.map.size() * sizeof(int32_t), cudaMemcpyHostToDevice, ctx->stream);
+    if (e == cudaSuccess) e = cudaStreamSynchronize(ctx->stream);
+    if (e != cudaSuccess) { cudaFree(dev); LF_CUDA(ctx, e); }
+    maps.device[ctx->device] = dev;      // kept for the life of the process: one per operator shape
+  }
+  *out = &maps;
+  return LF_OK;
+}
+
+lf_status create_from_maps(lf_context* ctx, lf_weights* w, const LayoutMaps& maps, const lf_encoded_tensor* tensors, int n) {
+  std::vector<size_t> sizes(n), offsets(n);
+  size_t raw_bytes = 0;
+  for (int i = 0; i < n; ++i) {
+    sizes[i] = !tensors[i].count ? 0 : tensors[i].dtype == LF_TENSOR_F32 ? (size_t)tensors[i].count * 4 : (size_t)tensors[i].payload_bytes;
+    offsets[i] = raw_bytes;
+    raw_bytes += lf_align_up(sizes[i] + 4, 16);
+  }
+  fill_flags(w, maps.flags);
+  w->f.assign(maps.offset.size(), nullptr);
+  const size_t canonical = maps.map.size() * sizeof(float);
+  LF_TRY(take_block(ctx, w, canonical));
+  char* base = static_cast<char*>(w->block);
+  for (size_t sl = 0; sl < maps.offset.size(); ++sl)
+    if (maps.present[sl]) w->f[sl] = reinterpret_cast<float*>(base) + maps.offset[sl];
+  // the tensors' bytes pass through the scratch arena, or through a block of their own where its limit has no room for them
+  uint8_t* raw = nullptr;
+  void* own = nullptr;
+  size_t own_bytes = 0;
+  if (lf_arena_ensure(ctx, raw_bytes) == LF_OK) raw = reinterpret_cast<uint8_t*>(ctx->arena);
+  else if (weight_block_take(ctx->device, raw_bytes, &own, &own_bytes) == cudaSuccess) raw = static_cast<uint8_t*>(own);
+  else return lf_fail(ctx, LF_ERR_MEMORY, "weight staging of %zu bytes refused", raw_bytes);
+  lf_status s = staged_upload(ctx, tensors, sizes.data(), offsets.data(), n, raw);
+  if (s == LF_OK) {
+    SourceTable table{};
+    for (int i = 0; i < n; ++i) {
+      table.base[i] = raw + offsets[i];
+      if (tensors[i].dtype != LF_TENSOR_INT5) continue;
+      table.block[i] = tensors[i].block;
+      table.scales[i] = reinterpret_cast<const __half*>(raw + offsets[i] + tensors[i].scale_offset);
+      table.zeros[i] = reinterpret_cast<const __half*>(raw + offsets[i] + tensors[i].zero_offset);
+    }
+    const int64_t count = (int64_t)maps.map.size();
+    gather_decode_kernel<<<lf_ceil_div(count, 256), 256, 0, ctx->stream>>>(maps.device[ctx->device], count, table, reinterpret_cast<float*>(base));
+    ctx->launches++;
+    WeightCursor cur{base, canonical, false};
+    s = cudaGetLastError() == cudaSuccess ? tc::prepare_weights(ctx, w, cur) : lf_fail(ctx, LF_ERR_CUDA, "weight layout launch failed");
+  }
+  if (own) {
+    cudaDeviceSynchronize();
+    weight_block_give(ctx->device, own, own_bytes);
+  }
+  return s;
+}
+
+// Finishes a new weights object or takes it back.
+lf_status publish(lf_context* ctx, lf_weights* w, lf_status s, lf_weights** out) {
+  g_pending.items.clear();
+  if (s == LF_OK && (cudaEventCreateWithFlags(&w->ready, cudaEventDisableTiming) != cudaSuccess || cudaEventRecord(w->ready, ctx->stream) != cudaSuccess))
+    s = lf_fail(ctx, LF_ERR_CUDA, "weight preparation failed: %s", cudaGetErrorString(cudaGetLastError()));
+  if (s != LF_OK) { lf_weights_destroy(w); return s; }
+  *out = w;
   return LF_OK;
 }
 
@@ -602,18 +817,35 @@ lf_status lf_weights_create(lf_context* ctx, lf_weight_kind kind, const lf_weigh
   *out = nullptr;
   if (dims->channels <= 0) return lf_fail(ctx, LF_ERR_SHAPE, "channels must be a positive integer; received %d", dims->channels);
   cudaSetDevice(ctx->device);
-  g_pending.items.clear();
   lf_weights* w = new lf_weights();
   w->ctx = ctx;
+  w->device = ctx->device;
   w->kind = (int)kind;
   w->dims = *dims;
-  lf_status s = build_weights(ctx, w, tensors, counts, n_tensors);
-  if (s == LF_OK) s = finish_uploads(ctx, w);
-  if (s == LF_OK) s = tc::prepare_weights(ctx, w);
-  g_pending.items.clear();
-  if (s != LF_OK) { lf_weights_destroy(w); return s; }
-  *out = w;
-  return LF_OK;
+  int64_t total = 0;
+  bool mapped = n_tensors > 0 && n_tensors <= kMaxSources && ctx->device < 64;
+  for (int i = 0; i < n_tensors; ++i) {
+    if (counts[i] < 0 || (counts[i] > 0 && !tensors[i])) mapped = false;      // (the layout functions say which)
+    else total += counts[i];
+  }
+  lf_status s;
+  if (mapped && total > 0 && total < (1 << 24)) {
+    LayoutMaps* maps = nullptr;
+    s = find_maps(ctx, (int)kind, *dims, std::vector<int64_t>(counts, counts + n_tensors), &maps);
+    if (s == LF_OK) {
+      lf_encoded_tensor in[kMaxSources]{};
+      for (int i = 0; i < n_tensors; ++i) {
+        in[i].dtype = LF_TENSOR_F32;
+        in[i].data = tensors[i];
+        in[i].count = counts[i];
+      }
+      s = create_from_maps(ctx, w, *maps, in, n_tensors);
+    }
+  } else {
+    g_pending.items.clear();
+    s = create_on_host(ctx, w, tensors, counts, n_tensors);
+  }
+  return publish(ctx, w, s, out);
 }
 
 lf_status lf_weights_create_encoded(lf_context* ctx, lf_weight_kind kind, const lf_weight_dims* dims,
@@ -625,107 +857,37 @@ lf_status lf_weights_create_encoded(lf_context* ctx, lf_weight_kind kind, const 
   if (n_tensors <= 0 || n_tensors > kMaxSources) return lf_fail(ctx, LF_ERR_ARGUMENT, "expected 1 to %d tensors; received %d", kMaxSources, n_tensors);
   if (ctx->device < 0 || ctx->device >= 64) return lf_fail(ctx, LF_ERR_ARGUMENT, "device ordinal %d is out of range", ctx->device);
   std::vector<int64_t> counts(n_tensors);
-  size_t input_bytes = 0;
   for (int i = 0; i < n_tensors; ++i) {
     const lf_encoded_tensor& t = tensors[i];
     counts[i] = t.count;
     if (t.count < 0 || (t.count > 0 && !t.data)) return lf_fail(ctx, LF_ERR_ARGUMENT, "tensor %d is null", i);
-    if (t.dtype == LF_TENSOR_F32) input_bytes += lf_align_up((size_t)t.count * 4 + 4, 256);
-    else if (t.dtype == LF_TENSOR_INT5) {
+    if (t.dtype == LF_TENSOR_INT5) {
       if (t.block <= 0 || (t.block * 5) % 8) return lf_fail(ctx, LF_ERR_ARGUMENT, "tensor %d: group %d of 5 bits does not pack into whole bytes", i, t.block);
       const uint64_t groups = ((uint64_t)t.count + t.block - 1) / t.block, code_bytes = groups * (t.block * 5 / 8) + 1;
       if (t.scale_offset < code_bytes || t.scale_offset % 2 || t.zero_offset % 2 || t.scale_offset + groups * 2 > t.payload_bytes ||
           t.zero_offset + groups * 2 > t.payload_bytes)
         return lf_fail(ctx, LF_ERR_SHAPE, "tensor %d: int5 payload of %llu bytes does not hold %lld codes, scales and zeros", i,
                        (unsigned long long)t.payload_bytes, (long long)t.count);
-      input_bytes += lf_align_up((size_t)t.payload_bytes + 4, 256);
-    } else return lf_fail(ctx, LF_ERR_ARGUMENT, "tensor %d has unknown encoding %d", i, t.dtype);
+    } else if (t.dtype != LF_TENSOR_F32) return lf_fail(ctx, LF_ERR_ARGUMENT, "tensor %d has unknown encoding %d", i, t.dtype);
   }
   cudaSetDevice(ctx->device);
-
-  // the layout map of this kind and shape
-  std::vector<int64_t> key = {(int64_t)kind, dims->channels, dims->hidden, dims->heads, dims->head_dim, dims->pair_channels, dims->out_channels};
-  key.insert(key.end(), counts.begin(), counts.end());
   LayoutMaps* maps = nullptr;
-  {
-    std::lock_guard<std::mutex> lock(g_maps_mutex);
-    auto found = g_maps.find(key);
-    if (found == g_maps.end()) {
-      LayoutMaps fresh;
-      LF_TRY(derive_maps(ctx, (int)kind, *dims, counts.data(), n_tensors, fresh));
-      found = g_maps.emplace(key, std::move(fresh)).first;
-    }
-    maps = &found->second;
-    if (!maps->device[ctx->device]) {
-      size_t total = 0;
-      for (auto& m : maps->slot) total += m.size();
-      int32_t* dev = nullptr;
-      LF_CUDA(ctx, cudaMalloc(&dev, (total ? total : 1) * sizeof(int32_t)));
-      size_t at = 0;
-      for (auto& m : maps->slot) {
-        if (!m.empty()) LF_CUDA(ctx, cudaMemcpyAsync(dev + at, m.data(), m.size() * sizeof(int32_t), cudaMemcpyHostToDevice, ctx->stream));
-        at += m.size();
-      }
-      LF_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
-      maps->device[ctx->device] = dev;      // kept for the life of the process: one per operator shape
-    }
-  }
-
-  // inputs to the device as they are (scratch arena), canonical arrays in one allocation
-  LF_TRY(lf_arena_ensure(ctx, input_bytes));
-  ArenaCursor cur{ctx, 0, false};
-  SourceTable table{};
-  for (int i = 0; i < n_tensors; ++i) {
-    const lf_encoded_tensor& t = tensors[i];
-    if (!t.count) continue;
-    const size_t bytes = t.dtype == LF_TENSOR_F32 ? (size_t)t.count * 4 : (size_t)t.payload_bytes;
-    uint8_t* dev = cur.take<uint8_t>(bytes + 4);
-    LF_CUDA(ctx, cudaMemcpyAsync(dev, t.data, bytes, cudaMemcpyHostToDevice, ctx->stream));
-    table.base[i] = dev;
-    if (t.dtype == LF_TENSOR_INT5) {
-      table.block[i] = t.block;
-      table.scales[i] = reinterpret_cast<const __half*>(dev + t.scale_offset);
-      table.zeros[i] = reinterpret_cast<const __half*>(dev + t.zero_offset);
-    }
-  }
+  LF_TRY(find_maps(ctx, (int)kind, *dims, counts, &maps));
   lf_weights* w = new lf_weights();
   w->ctx = ctx;
+  w->device = ctx->device;
   w->kind = (int)kind;
-  w->dims = maps->flags.dims;
-  w->has_gate_bias = maps->flags.has_gate_bias; w->has_out_bias = maps->flags.has_out_bias;
-  w->has_pair_norm = maps->flags.has_pair_norm; w->has_pair_proj = maps->flags.has_pair_proj;
-  w->f.assign(maps->slot.size(), nullptr);
-  size_t total = 0;
-  std::vector<size_t> offset;
-  for (auto& m : maps->slot) { offset.push_back(total); total += lf_align_up(m.size() / 2 * sizeof(float) + 4, 256); }
-  char* base = nullptr;
-  cudaError_t e = cudaMalloc(&base, total ? total : 256);
-  if (e != cudaSuccess) { cudaGetLastError(); delete w; return lf_fail(ctx, LF_ERR_MEMORY, "weight allocation of %zu bytes refused: %s", total, cudaGetErrorString(e)); }
-  w->owned.push_back(base);
-  size_t at = 0;
-  for (size_t sl = 0; sl < maps->slot.size(); ++sl) {
-    const int64_t count = (int64_t)maps->slot[sl].size() / 2;
-    float* dst = reinterpret_cast<float*>(base + offset[sl]);
-    if (count) {
-      gather_decode_kernel<<<lf_ceil_div(count, 256), 256, 0, ctx->stream>>>(maps->device[ctx->device] + at, count, table, dst);
-      ctx->launches++;
-    }
-    w->f[sl] = dst;
-    at += maps->slot[sl].size();
-  }
-  lf_status s = cudaGetLastError() == cudaSuccess ? LF_OK : lf_fail(ctx, LF_ERR_CUDA, "weight decode launch failed");
-  g_pending.items.clear();                 // nothing is staged on the host: the repacks read the device arrays
-  if (s == LF_OK) s = tc::prepare_weights(ctx, w);
-  if (s == LF_OK && cudaStreamSynchronize(ctx->stream) != cudaSuccess) s = lf_fail(ctx, LF_ERR_CUDA, "weight decode failed");   // the caller's payloads may go
-  if (s != LF_OK) { lf_weights_destroy(w); return s; }
-  *out = w;
-  return LF_OK;
+  return publish(ctx, w, create_from_maps(ctx, w, *maps, tensors, n_tensors), out);
 }
 
 void lf_weights_destroy(lf_weights* w) {
   if (!w) return;
-  if (w->ctx) { cudaSetDevice(w->ctx->device); cudaStreamSynchronize(w->ctx->stream); }
-  for (void* p : w->owned) cudaFree(p);
+  cudaSetDevice(w->device);
+  if (w->ready) cudaEventDestroy(w->ready);
+  if (w->block) {
+    cudaDeviceSynchronize();      // nothing reads the block any more, on any stream
+    weight_block_give(w->device, w->block, w->block_bytes);
+  }
   delete w;
 }
 
@@ -1160,6 +1322,7 @@ lf_status lf_triangle_multiplication_run(lf_context* ctx, const lf_triangle_desc
   if (d->c_hidden <= 0) return lf_fail(ctx, LF_ERR_SHAPE, "cHidden must be a positive safe integer; received %d", d->c_hidden);
   LF_TRY(check_common(ctx, d->variance, d->precision, d->space, d->act_dtype, d->epsilon));
   const lf_weights* w = d->weights;
+  lf_weights_await(ctx, w);
   if (w->kind != LF_WEIGHTS_TRIANGLE_AF2 && w->kind != LF_WEIGHTS_TRIANGLE_AF3) return lf_fail(ctx, LF_ERR_ARGUMENT, "weights are not triangle weights");
   if (w->dims.channels != d->c_z || w->dims.hidden != d->c_hidden)
     return lf_fail(ctx, LF_ERR_SHAPE, "weights were packed for cZ %d, cHidden %d; the call has %d, %d", w->dims.channels, w->dims.hidden, d->c_z, d->c_hidden);
@@ -1187,6 +1350,7 @@ lf_status lf_attention_run(lf_context* ctx, const lf_attention_desc* d, lf_resul
     return lf_fail(ctx, LF_ERR_SHAPE, "attention dimensions must be positive safe integers");
   LF_TRY(check_common(ctx, d->variance, d->precision, d->space, d->act_dtype, d->epsilon));
   const lf_weights* w = d->weights;
+  lf_weights_await(ctx, w);
   const bool af3 = w->kind == LF_WEIGHTS_GRID_ATTENTION_AF3;
   if (!af3 && w->kind != LF_WEIGHTS_ATTENTION_AF2) return lf_fail(ctx, LF_ERR_ARGUMENT, "weights are not attention weights");
   if (w->dims.channels != d->channels || w->dims.heads != d->heads)
@@ -1240,6 +1404,7 @@ lf_status lf_transition_run(lf_context* ctx, const lf_transition_desc* d, lf_res
   if (d->rows <= 0 || d->channels <= 0 || d->hidden <= 0) return lf_fail(ctx, LF_ERR_SHAPE, "transition dimensions must be positive safe integers");
   LF_TRY(check_common(ctx, d->variance, d->precision, d->space, d->act_dtype, d->epsilon));
   const lf_weights* w = d->weights;
+  lf_weights_await(ctx, w);
   const bool af3 = w->kind == LF_WEIGHTS_TRANSITION_AF3;
   if (!af3 && w->kind != LF_WEIGHTS_TRANSITION_AF2) return lf_fail(ctx, LF_ERR_ARGUMENT, "weights are not transition weights");
   if (w->dims.channels != d->channels || w->dims.hidden != d->hidden)
@@ -1266,6 +1431,7 @@ lf_status lf_outer_product_mean_run(lf_context* ctx, const lf_opm_desc* d, lf_re
   if (d->c_outer > 32) return lf_fail(ctx, LF_ERR_UNSUPPORTED, "cOuter %d exceeds 32", d->c_outer);
   LF_TRY(check_common(ctx, d->variance, d->precision, d->space, d->act_dtype, d->layer_norm_epsilon));
   const lf_weights* w = d->weights;
+  lf_weights_await(ctx, w);
   if (w->kind != LF_WEIGHTS_OPM_AF2) return lf_fail(ctx, LF_ERR_ARGUMENT, "weights are not outer-product-mean weights");
   if (w->dims.channels != d->c_m || w->dims.hidden != d->c_outer || w->dims.out_channels != d->c_z)
     return lf_fail(ctx, LF_ERR_SHAPE, "weights were packed for cM %d, cOuter %d, cZ %d", w->dims.channels, w->dims.hidden, w->dims.out_channels);
@@ -1378,6 +1544,7 @@ lf_status lf_single_attention_run(lf_context* ctx, const lf_single_attention_des
   if (!d || !d->single || !d->pair || !d->seq_mask || !d->out || !d->weights) return lf_fail(ctx, LF_ERR_ARGUMENT, "single attention: null argument");
   if (d->tokens <= 0 || d->channels <= 0) return lf_fail(ctx, LF_ERR_SHAPE, "single attention dimensions must be positive safe integers");
   const lf_weights* w = d->weights;
+  lf_weights_await(ctx, w);
   if (w->kind != LF_WEIGHTS_SINGLE_ATTENTION_AF3) return lf_fail(ctx, LF_ERR_ARGUMENT, "weights are not single-attention weights");
   if (w->dims.channels != d->channels || w->dims.heads != d->heads || w->dims.head_dim != d->head_dim || w->dims.pair_channels != d->pair_channels)
     return lf_fail(ctx, LF_ERR_SHAPE, "weights were packed for %d channels, %d heads x %d, %d pair channels", w->dims.channels, w->dims.heads, w->dims.head_dim, w->dims.pair_channels);
@@ -1408,6 +1575,7 @@ lf_status lf_msa_attention_run(lf_context* ctx, const lf_msa_attention_desc* d, 
   if (!d || !d->msa || !d->msa_mask || !d->pair || !d->out || !d->weights) return lf_fail(ctx, LF_ERR_ARGUMENT, "MSA attention: null argument");
   if (d->sequences <= 0 || d->tokens <= 0 || d->channels <= 0) return lf_fail(ctx, LF_ERR_SHAPE, "MSA attention dimensions must be positive safe integers");
   const lf_weights* w = d->weights;
+  lf_weights_await(ctx, w);
   if (w->kind != LF_WEIGHTS_MSA_ATTENTION_AF3) return lf_fail(ctx, LF_ERR_ARGUMENT, "weights are not MSA attention weights");
   if (w->dims.channels != d->channels || w->dims.heads != d->heads || w->dims.head_dim != d->head_dim || w->dims.pair_channels != d->pair_channels)
     return lf_fail(ctx, LF_ERR_SHAPE, "weights were packed for %d channels, %d heads x %d, %d pair channels", w->dims.channels, w->dims.heads, w->dims.head_dim, w->dims.pair_channels);
@@ -1444,6 +1612,7 @@ template <typename T>
 void global_attention(lf_context* ctx, ArenaCursor& cur, const lf_global_attention_desc* d, const void* act, const float* mask,
                       void* out) {
   const lf_weights* w = d->weights;
+  lf_weights_await(ctx, w);
   const auto& f = w->f;
   const int S = d->sequences, n = d->length, c = d->channels, H = d->heads, hd = w->dims.head_dim, HD = H * hd, wide = 2 * hd + HD;
   const int64_t R = (int64_t)S * n;
@@ -1476,6 +1645,7 @@ lf_status lf_global_column_attention_run(lf_context* ctx, const lf_global_attent
     return lf_fail(ctx, LF_ERR_SHAPE, "global attention dimensions must be positive safe integers");
   LF_TRY(check_common(ctx, d->variance, d->precision, d->space, d->act_dtype, d->epsilon));
   const lf_weights* w = d->weights;
+  lf_weights_await(ctx, w);
   if (w->kind != LF_WEIGHTS_GLOBAL_ATTENTION_AF2) return lf_fail(ctx, LF_ERR_ARGUMENT, "weights are not global attention weights");
   if (w->dims.channels != d->channels || w->dims.heads != d->heads)
     return lf_fail(ctx, LF_ERR_SHAPE, "weights were packed for %d channels, %d heads; the call has %d, %d", w->dims.channels, w->dims.heads, d->channels, d->heads);
@@ -1531,6 +1701,7 @@ lf_status lf_pair_stack_run(lf_context* ctx, const lf_pair_stack_desc* d, lf_res
   if (d->c_z % d->heads != 0) return lf_fail(ctx, LF_ERR_SHAPE, "cZ %d is not a multiple of heads %d", d->c_z, d->heads);
   for (int b = d->first_block; b < d->first_block + d->n_blocks; ++b) {
     const lf_pair_block_weights& bw = d->blocks[b];
+    for (const lf_weights* w : {bw.triangle_outgoing, bw.triangle_incoming, bw.attention_starting, bw.attention_ending, bw.transition}) lf_weights_await(ctx, w);
     if (!bw.triangle_outgoing || !bw.triangle_incoming || !bw.attention_starting || !bw.attention_ending || !bw.transition)
       return lf_fail(ctx, LF_ERR_ARGUMENT, "block %d has a null weight handle", b);
     const bool af3 = bw.attention_starting->kind == LF_WEIGHTS_GRID_ATTENTION_AF3;
@@ -1596,6 +1767,7 @@ lf_status lf_pair_shard_step(lf_context* ctx, const lf_shard_step_desc* d, lf_re
   if (d->rows <= 0 || d->length <= 0 || d->ranks <= 0) return lf_fail(ctx, LF_ERR_SHAPE, "shard dimensions must be positive safe integers");
   if (d->act_dtype != LF_DTYPE_F32 && d->act_dtype != LF_DTYPE_BF16) return lf_fail(ctx, LF_ERR_ARGUMENT, "unknown activation dtype %d", d->act_dtype);
   const lf_weights* w = d->weights;
+  lf_weights_await(ctx, w);
   const int R = d->rows, n = d->length, ld = (n + 15) / 16 * 16;
   const bool tri = d->op >= LF_SHARD_TRIANGLE_PROJECT && d->op <= LF_SHARD_TRIANGLE_OUTPUT;
   const bool att = d->op >= LF_SHARD_ATTENTION_PROJECT && d->op <= LF_SHARD_ATTENTION_OUTPUT;
@@ -1663,6 +1835,7 @@ lf_status lf_pair_shard_exchange_step(lf_context* ctx, const lf_shard_step_desc*
     return lf_fail(ctx, LF_ERR_UNSUPPORTED, "exchange step: length must be a multiple of 16 and rows a multiple of 128; received %d, %d", d->length, d->rows);
   if (d->act_dtype != LF_DTYPE_F32 && d->act_dtype != LF_DTYPE_BF16) return lf_fail(ctx, LF_ERR_ARGUMENT, "unknown activation dtype %d", d->act_dtype);
   const lf_weights* w = d->weights;
+  lf_weights_await(ctx, w);
   const int R = d->rows, n = d->length, ld = n, G = d->ranks, rank = peers->rank, cpr = 128 / G;
   auto table = [&](void* const* src, tc::PeerPtrs& out, const char* name) -> lf_status {
     for (int g = 0; g < G; ++g) {

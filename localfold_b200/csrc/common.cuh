@@ -22,6 +22,9 @@ typedef __half op16;
 
 struct lf_context {
   int device = 0;
+  // Pinned staging of weight uploads: filled from the front, the stream is waited for when it is full.
+  char* pinned = nullptr;
+  size_t pinned_used = 0;
   cudaStream_t stream = nullptr;
   bool owns_stream = false;
   std::string error;
@@ -70,11 +73,13 @@ struct lf_weights {
   lf_context* ctx = nullptr;
   int kind = 0;
   lf_weight_dims dims{};
-  std::vector<float*> f;     // named by the per-kind enums in weights.cuh
+  std::vector<float*> f;     // named by the per-kind enums above
   std::vector<void*> h;      // fp16 repacks (tensor-core path)
   std::vector<void*> g;      // fp16 [n_out][k] operands of the plain tensor-core GEMM (widths the fused kernels do not take)
-  std::vector<void*> owned;  // every device allocation, for destroy
-  int bias_flags = 0;        // per 128-column group of the fused projection: bias is non-zero
+  int device = 0;
+  void* block = nullptr;     // the one device allocation behind all of them (weight_block_take)
+  size_t block_bytes = 0;
+  cudaEvent_t ready = nullptr;   // recorded on the creating context's stream when they have been prepared
   bool has_gate_bias = false, has_out_bias = false, has_pair_norm = false, has_pair_proj = false;
 };
 
@@ -124,7 +129,24 @@ struct ArenaCursor {
   }
 };
 
+// The same over a weights object's own allocation.
+struct WeightCursor {
+  char* base;
+  size_t offset;
+  bool dry;
+  template <typename T>
+  T* take(size_t count) {
+    T* p = dry ? nullptr : reinterpret_cast<T*>(base + offset);
+    offset += lf_align_up(count * sizeof(T) + 4, 256);
+    return p;
+  }
+};
+
 lf_status lf_arena_ensure(lf_context* ctx, size_t bytes);
+// Work on `ctx`'s stream that reads `w` comes after the preparation of w on another context's stream.
+static inline void lf_weights_await(lf_context* ctx, const lf_weights* w) {
+  if (w && w->ctx != ctx && w->ready) cudaStreamWaitEvent(ctx->stream, w->ready, 0);
+}
 // The pair stack with the pair left in host memory (pair_spill.cu).
 lf_status lf_pair_stack_spilled(lf_context* ctx, const lf_pair_stack_desc* d, lf_result* r);
 

@@ -69,6 +69,7 @@ extern "C" lf_status lf_triangle_multiplication_run_static(lf_context* ctx, cons
     return lf_fail(ctx, LF_ERR_UNSUPPORTED, "length %d exceeds the static scratch, which covers lengths up to %d; use lf_triangle_multiplication_run",
                    d->length, LF_STATIC_MAX_LENGTH);
   const lf_weights* w = d->weights;
+  lf_weights_await(ctx, w);
   if (w->kind != LF_WEIGHTS_TRIANGLE_AF2 && w->kind != LF_WEIGHTS_TRIANGLE_AF3) return lf_fail(ctx, LF_ERR_ARGUMENT, "weights are not triangle weights");
   if (d->c_z != 128 || d->c_hidden != 128 || w->dims.channels != 128 || w->dims.hidden != 128 || !tc::ln_gemm_supported(w) ||
       !tc::contract_supported(d->length, 128))

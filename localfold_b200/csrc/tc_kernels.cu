@@ -144,210 +144,6 @@ lf_status check_status(lf_context* ctx) {
 bool ln_gemm_supported(const lf_weights* w) { return w && !w->h.empty() && w->h[0] != nullptr; }
 bool pair_bias_supported(const lf_weights* w) { return w && w->h.size() >= 6 && w->h[4] != nullptr; }
 
-// The centre LayerNorm folded into the output projection: W' = diag(gain) Wz, s1[c] = sum_h fp16(W'[h][c]) (what the
-// tensor core will multiply the mean by), t[c] = bz[c] + sum_h offset[h] Wz[h][c]; fold = (s1 | t | bg + input offset through Wg).
-__global__ void triangle_fold_kernel(const float* __restrict__ wz, const float* __restrict__ gain, const float* __restrict__ offset,
-                                     const float* __restrict__ bz, const float* __restrict__ bg, const float* __restrict__ wg,
-                                     const float* __restrict__ in_offset, float* __restrict__ wfold, float* __restrict__ fold) {
-  const int c = threadIdx.x;
-  double s1 = 0.0, t = bz[c], g = bg[c];
-  for (int h = 0; h < 128; ++h) {
-    const float wf = gain[h] * wz[h * 128 + c];
-    wfold[h * 128 + c] = wf;
-    s1 += (double)__half2float(__float2half_rn(wf));
-    t += (double)offset[h] * wz[h * 128 + c];
-    g += (double)in_offset[h] * wg[h * 128 + c];      // the input LayerNorm's offset through the output gate
-  }
-  fold[c] = (float)s1;
-  fold[128 + c] = (float)t;
-  fold[256 + c] = (float)g;
-}
-
-// bf16/fp16 repacks for the tensor-core kernels: h[0] = swizzled fp16 image of the fused
-// projection W^T (plus the pair-bias projection rows for attention), h[1] = its bias vector.
-// weights w [K][ldw] float32, columns col0 .. col0+N-1 -> fp16 [N][K] (the plain GEMM wants k contiguous in both operands)
-__global__ void gemm_operand_kernel(const float* __restrict__ w, int K, int ldw, int col0, int N, op16* __restrict__ out) {
-  int64_t idx = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (idx >= (int64_t)N * K) return;
-  int n = (int)(idx / K), k = (int)(idx % K);
-  out[idx] = __float2half_rn(w[(int64_t)k * ldw + col0 + n]);
-}
-
-// ... with 16 more k columns: the bias in the first, zeros after it (the activations carry a column of ones there, so the
-// GEMM adds the bias)
-__global__ void gemm_operand_bias_kernel(const float* __restrict__ w, int K, int ldw, int N, const float* __restrict__ bias,
-                                         op16* __restrict__ out) {
-  int64_t idx = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  const int K2 = K + 16;
-  if (idx >= (int64_t)N * K2) return;
-  int n = (int)(idx / K2), k = (int)(idx % K2);
-  out[idx] = __float2half_rn(k < K ? w[(int64_t)k * ldw + n] : k == K ? bias[n] : 0.f);
-}
-
-lf_status prepare_weights(lf_context* ctx, lf_weights* w) {
-  const bool tri = w->kind == LF_WEIGHTS_TRIANGLE_AF2 || w->kind == LF_WEIGHTS_TRIANGLE_AF3;
-  const bool att = w->kind == LF_WEIGHTS_ATTENTION_AF2 || w->kind == LF_WEIGHTS_GRID_ATTENTION_AF3;
-  if (tri && w->dims.channels == 128 && w->dims.hidden == 128) {
-    op16* img = nullptr;
-    LF_CUDA(ctx, cudaMalloc(&img, 512 * 256));
-    w->owned.push_back(img);
-    LF_CUDA(ctx, cudaMemsetAsync(img, 0, 512 * 256, ctx->stream));
-    // the input LayerNorm's gain goes into the rows of the images, its offset into the biases: the kernels' producers
-    // hand the tensor core (x - mean) / std
-    pack_weight_image(ctx, w->f[TRI_W4], 128, 512, 512, 0, 512, img, 0, 1.0f, w->f[TRI_LN_G]);
-    float* b4 = nullptr;
-    LF_CUDA(ctx, cudaMalloc(&b4, 512 * sizeof(float))); w->owned.push_back(b4);
-    fold_bias(ctx, w->f[TRI_W4], 128, 512, 0, 512, w->f[TRI_LN_B], w->f[TRI_B4], 1.0f, b4);
-    w->h.assign(4, nullptr);
-    w->h[0] = img;
-    w->h[1] = b4;
-    // output kernel: rows 0..127 = (diag(gain) Wz)^T, rows 128..255 = Wg^T, plus the folded vectors
-    float* dfold = nullptr; float* dw = nullptr; op16* img2 = nullptr;
-    LF_CUDA(ctx, cudaMalloc(&dfold, 384 * 4)); w->owned.push_back(dfold);
-    LF_CUDA(ctx, cudaMalloc(&dw, 128 * 128 * 4)); w->owned.push_back(dw);
-    LF_CUDA(ctx, cudaMalloc(&img2, 256 * 256)); w->owned.push_back(img2);
-    triangle_fold_kernel<<<1, 128, 0, ctx->stream>>>(w->f[TRI_WZ], w->f[TRI_LNO_G], w->f[TRI_LNO_B], w->f[TRI_BZ], w->f[TRI_BG], w->f[TRI_WG],
-                                                     w->f[TRI_LN_B], dw, dfold);
-    pack_weight_image(ctx, dw, 128, 128, 256, 0, 128, img2, 0, 1.0f);
-    pack_weight_image(ctx, w->f[TRI_WG], 128, 128, 256, 0, 128, img2, 128, 1.0f, w->f[TRI_LN_G]);
-    LF_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
-    w->h[2] = img2;
-    w->h[3] = dfold;
-  } else if (att && w->dims.channels == 128 && w->dims.heads * w->dims.head_dim == 128 && w->dims.heads <= 16 &&
-             !w->has_pair_norm) {
-    op16* img = nullptr;
-    float* bias = nullptr;
-    LF_CUDA(ctx, cudaMalloc(&img, 528 * 256));
-    w->owned.push_back(img);
-    LF_CUDA(ctx, cudaMalloc(&bias, 528 * sizeof(float)));
-    w->owned.push_back(bias);
-    LF_CUDA(ctx, cudaMemsetAsync(img, 0, 528 * 256, ctx->stream));
-    LF_CUDA(ctx, cudaMemsetAsync(bias, 0, 528 * sizeof(float), ctx->stream));
-    // the query columns carry the head_dim^-1/2 logit scale
-    const float qs = 1.0f / sqrtf((float)w->dims.head_dim);
-    // the LayerNorm's gain goes into the rows of the image, its offset into the bias vector
-    pack_weight_image(ctx, w->f[ATT_W4], 128, 128, 528, 0, 512, img, 0, qs, w->f[ATT_LN_G]);
-    pack_weight_image(ctx, w->f[ATT_W4], 128, 384, 528, 128, 512, img, 128, 1.0f, w->f[ATT_LN_G]);
-    fold_bias(ctx, w->f[ATT_W4], 128, 128, 0, 512, w->f[ATT_LN_B], w->f[ATT_B4], qs, bias);
-    fold_bias(ctx, w->f[ATT_W4], 128, 384, 128, 512, w->f[ATT_LN_B], w->f[ATT_B4] + 128, 1.0f, bias + 128);
-    if (w->has_pair_proj) {
-      pack_weight_image(ctx, w->f[ATT_WB], 128, w->dims.heads, 528, 0, w->dims.heads, img, 512, 1.0f, w->f[ATT_LN_G]);
-      fold_bias(ctx, w->f[ATT_WB], 128, w->dims.heads, 0, w->dims.heads, w->f[ATT_LN_B], nullptr, 1.0f, bias + 512);
-    }
-    {
-      // which 128-column groups have a bias at all (the epilogue skips the others): 2 KiB read back once
-      std::vector<float> hb(512);
-      LF_CUDA(ctx, cudaMemcpyAsync(hb.data(), bias, 512 * sizeof(float), cudaMemcpyDeviceToHost, ctx->stream));
-      LF_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
-      w->bias_flags = 0;
-      for (int grp = 0; grp < 4; ++grp)
-        for (int i = 0; i < 128; ++i)
-          if (hb[grp * 128 + i] != 0.f) { w->bias_flags |= 1 << grp; break; }
-    }
-    w->h.assign(4, nullptr);
-    w->h[0] = img;
-    w->h[1] = bias;
-    op16* img2 = nullptr;
-    LF_CUDA(ctx, cudaMalloc(&img2, 128 * 256)); w->owned.push_back(img2);
-    pack_weight_image(ctx, w->f[ATT_WO], 128, 128, 128, 0, 128, img2, 0, 1.0f);
-    w->h[2] = img2;
-  }
-  if (w->has_pair_norm && w->has_pair_proj && w->dims.pair_channels == 128 && w->dims.heads <= 16 &&
-      (w->kind == LF_WEIGHTS_ATTENTION_AF2 || w->kind == LF_WEIGHTS_SINGLE_ATTENTION_AF3 || w->kind == LF_WEIGHTS_MSA_ATTENTION_AF3)) {
-    // pair bias from a 128-channel pair with a LayerNorm of its own: a 16-row image of the projection (gain in its
-    // rows, the offset's share as a bias) for the tensor-core projection kernel run with the bias chunk alone
-    op16* img = nullptr;
-    float* pb = nullptr;
-    LF_CUDA(ctx, cudaMalloc(&img, 16 * 256)); w->owned.push_back(img);
-    LF_CUDA(ctx, cudaMalloc(&pb, 16 * sizeof(float))); w->owned.push_back(pb);
-    LF_CUDA(ctx, cudaMemsetAsync(img, 0, 16 * 256, ctx->stream));
-    LF_CUDA(ctx, cudaMemsetAsync(pb, 0, 16 * sizeof(float), ctx->stream));
-    pack_weight_image(ctx, w->f[ATT_WB], 128, w->dims.heads, 16, 0, w->dims.heads, img, 0, 1.0f, w->f[ATT_PLN_G]);
-    fold_bias(ctx, w->f[ATT_WB], 128, w->dims.heads, 0, w->dims.heads, w->f[ATT_PLN_B], nullptr, 1.0f, pb);
-    if (w->h.size() < 6) w->h.resize(6, nullptr);
-    w->h[4] = img;
-    w->h[5] = pb;
-  }
-  if (w->kind == LF_WEIGHTS_TRANSITION_AF2 && w->dims.channels == 128 && w->dims.hidden == 512) {
-    // per 128-wide hidden chunk: W1 slice image (rows = hidden columns, K = 128 inputs), then W2 slice
-    // image (rows = 128 outputs, K = the chunk's 128 hidden channels)
-    op16* img = nullptr;
-    LF_CUDA(ctx, cudaMalloc(&img, 4 * 65536));
-    w->owned.push_back(img);
-    for (int cidx = 0; cidx < 4; ++cidx) {
-      pack_weight_image(ctx, w->f[TRN_W1], 128, 128, 128, cidx * 128, 512, img + cidx * 32768, 0, 1.0f, w->f[TRN_LN_G]);
-      pack_weight_image(ctx, w->f[TRN_W2] + (size_t)cidx * 128 * 128, 128, 128, 128, 0, 128, img + cidx * 32768 + 16384, 0, 1.0f);
-    }
-    float* b1 = nullptr;
-    LF_CUDA(ctx, cudaMalloc(&b1, 512 * sizeof(float))); w->owned.push_back(b1);
-    fold_bias(ctx, w->f[TRN_W1], 128, 512, 0, 512, w->f[TRN_LN_B], w->f[TRN_B1], 1.0f, b1);
-    w->h.assign(2, nullptr);
-    w->h[0] = img;
-    w->h[1] = b1;
-  }
-  if (w->kind == LF_WEIGHTS_TRANSITION_AF3 && w->dims.channels == 128 && w->dims.hidden == 512) {
-    // per 64-wide hidden chunk: W1 slice image of 128 rows (64 gate columns, then the matching 64 value
-    // columns; K = 128 inputs: 32 KiB), then W2 slice image (rows = 128 outputs, K = 64 hidden: 16 KiB)
-    op16* img = nullptr;
-    LF_CUDA(ctx, cudaMalloc(&img, 8 * 49152));
-    w->owned.push_back(img);
-    for (int cidx = 0; cidx < 8; ++cidx) {
-      op16* base = img + (size_t)cidx * 24576;
-      pack_weight_image(ctx, w->f[TRN_W1], 128, 64, 128, cidx * 64, 1024, base, 0, 1.0f, w->f[TRN_LN_G]);
-      pack_weight_image(ctx, w->f[TRN_W1], 128, 64, 128, 512 + cidx * 64, 1024, base, 64, 1.0f, w->f[TRN_LN_G]);
-      pack_weight_image(ctx, w->f[TRN_W2] + (size_t)cidx * 64 * 128, 64, 128, 128, 0, 128, base + 16384, 0, 1.0f);
-    }
-    float* b1 = nullptr;
-    LF_CUDA(ctx, cudaMalloc(&b1, 1024 * sizeof(float))); w->owned.push_back(b1);
-    fold_bias(ctx, w->f[TRN_W1], 128, 1024, 0, 1024, w->f[TRN_LN_B], w->f[TRN_B1], 1.0f, b1);
-    w->h.assign(2, nullptr);
-    w->h[0] = img;
-    w->h[1] = b1;
-  }
-  // Operands of the plain fp16 GEMM for the widths the fused kernels do not take: weights [k][n] -> fp16 [n][k]
-  auto operand = [&](const float* src, int K, int ldw, int col0, int N, op16* dst) {
-    gemm_operand_kernel<<<(unsigned)(((int64_t)N * K + 255) / 256), 256, 0, ctx->stream>>>(src, K, ldw, col0, N, dst);
-  };
-  auto alloc16 = [&](int64_t count, op16** out) -> lf_status {
-    LF_CUDA(ctx, cudaMalloc(out, (size_t)count * sizeof(op16)));
-    w->owned.push_back(*out);
-    return LF_OK;
-  };
-  if (w->kind == LF_WEIGHTS_ATTENTION_AF2 && (w->h.empty() || !w->h[0]) && w->dims.heads > 0 && w->dims.channels % w->dims.heads == 0 &&
-      w->dims.channels % 8 == 0) {
-    const int c = w->dims.channels, HD = c;          // heads * (channels / heads)
-    op16 *w4 = nullptr, *wo = nullptr;
-    LF_TRY(alloc16((int64_t)4 * HD * c, &w4));
-    LF_TRY(alloc16((int64_t)c * HD, &wo));
-    operand(w->f[ATT_W4], c, 4 * HD, 0, 4 * HD, w4);
-    operand(w->f[ATT_WO], HD, c, 0, c, wo);
-    w->g = {w4, wo};
-  }
-  if ((w->kind == LF_WEIGHTS_TRANSITION_AF2 || w->kind == LF_WEIGHTS_TRANSITION_AF3) && w->h.empty() &&
-      w->dims.channels % 8 == 0 && w->dims.hidden % 8 == 0) {
-    const int c = w->dims.channels, hd = w->dims.hidden, wide = w->kind == LF_WEIGHTS_TRANSITION_AF3 ? 2 * hd : hd;
-    op16 *w1 = nullptr, *w2 = nullptr;
-    LF_TRY(alloc16((int64_t)wide * (c + 16), &w1));      // first projection: [wide][c + 16], its bias in column c
-    LF_TRY(alloc16((int64_t)c * hd, &w2));
-    gemm_operand_bias_kernel<<<(unsigned)(((int64_t)wide * (c + 16) + 255) / 256), 256, 0, ctx->stream>>>(w->f[TRN_W1], c, wide, wide,
-                                                                                                       w->f[TRN_B1], w1);
-    operand(w->f[TRN_W2], hd, c, 0, c, w2);
-    w->g = {w1, w2};
-  }
-  if (w->kind == LF_WEIGHTS_OPM_AF2 && w->dims.channels % 8 == 0 && w->dims.hidden % 8 == 0 && w->dims.out_channels % 8 == 0) {
-    const int cm = w->dims.channels, c = w->dims.hidden, cz = w->dims.out_channels;
-    op16 *wlr = nullptr, *wout = nullptr;
-    LF_TRY(alloc16((int64_t)2 * c * cm, &wlr));
-    LF_TRY(alloc16((int64_t)cz * c * c, &wout));
-    operand(w->f[OPM_WL], cm, c, 0, c, wlr);
-    operand(w->f[OPM_WR], cm, c, 0, c, wlr + (int64_t)c * cm);
-    operand(w->f[OPM_WOUT], c * c, cz, 0, cz, wout);
-    w->g = {wlr, wout};
-  }
-  LF_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
-  return LF_OK;
-}
-
 // ---------------------------------------------------------------------------
 // Triangle contraction.
 //

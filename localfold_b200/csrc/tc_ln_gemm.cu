@@ -67,7 +67,6 @@ struct LnGemmParams {
   int ldq;                  // attention activations (q, k, v, gate, o) are stored in 8-row x 8-channel pieces: element (b, q, c)
                             // of a [batch][Q][128] tensor sits at b*ldq*128 + (q/8)*1024 + (c/8)*64 + (q%8)*8 + c%8, ldq = Q rounded up to 16
   int heads, bias_swap;
-  int bias_flags;           // bit (2*chunk + half): that 128-column group has a non-zero bias
   // output epilogues (attention output projection, triangle output): out = resid + f(acc)
   int a_is_op16;            // the A operand is an fp16 tensor of logical rows in 8 x 8 pieces (see ldq), copied as is (no LayerNorm)
   const void* resid;        // pair rows (memory order) to add, or null
@@ -146,6 +145,10 @@ ln_gemm_kernel(const __grid_constant__ CUtensorMap mapX, const __grid_constant__
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int64_t tiles = p.tile_per_row ? (int64_t)p.plane_rows * p.tile_per_row : (p.rows + LG_ROWS - 1) / LG_ROWS;
 
+  // attention projection: bit (2 * chunk + half) = that 128-column group has a non-zero bias (the epilogue skips the others)
+  __shared__ unsigned int bias_flags[1];
+  if (threadIdx.x == 0) bias_flags[0] = 0u;
+  if (EPI == LG_EPI_ATTENTION) __syncthreads();
   if (threadIdx.x == 0) {
     for (int s = 0; s < 2; ++s) {
       mbar_init(&x_full[s], 1);
@@ -165,7 +168,11 @@ ln_gemm_kernel(const __grid_constant__ CUtensorMap mapX, const __grid_constant__
     const uint4* src = reinterpret_cast<const uint4*>(p.wimg);
     uint4* dst = reinterpret_cast<uint4*>(sW);
     for (int i = threadIdx.x; i < w_bytes / 16; i += LG_THREADS) dst[i] = src[i];
-    for (int i = threadIdx.x; i < p.n_bias; i += LG_THREADS) sBias[i] = p.bias[i];
+    for (int i = threadIdx.x; i < p.n_bias; i += LG_THREADS) {
+      const float v = p.bias[i];
+      sBias[i] = v;
+      if (EPI == LG_EPI_ATTENTION && v != 0.f) atomicOr(bias_flags, 1u << (i >> 7));
+    }
     fence_async_smem();
   }
   if (warp == LG_MMA_WARP) { tmem_alloc(tmem_slot, 512); tmem_relinquish(); }
@@ -840,7 +847,7 @@ ln_gemm_kernel(const __grid_constant__ CUtensorMap mapX, const __grid_constant__
             op16* out = jr == 0 ? (second ? p.out_k : p.out_q) : (second ? p.out_g : p.out_v);
             const float4* bias4 = reinterpret_cast<const float4*>(sBias + jr * 256 + second * 128 + col0);
             const bool gate = (jr == 1 && second == 1);
-            const bool has_bias = (p.bias_flags >> (jr * 2 + second)) & 1;
+            const bool has_bias = (bias_flags[0] >> (jr * 2 + second)) & 1u;
             // destination of this row in the 8 x 8-piece layout: pieces along channels are 64 elements apart
             const uint32_t ur = (uint32_t)(valid ? r : 0), uq = (uint32_t)p.Q, rb = ur / uq, rq = ur % uq;
             op16* out_row = out + (int64_t)rb * p.ldq * 128 + (int64_t)(rq >> 3) * 1024 + (rq & 7) * 8;
@@ -921,40 +928,6 @@ ln_gemm_kernel(const __grid_constant__ CUtensorMap mapX, const __grid_constant__
   __syncthreads();
   if (*abort_flag) drain_after_abort();
   if (warp == LG_MMA_WARP) { tc_fence_after(); tmem_dealloc(tmem_base, 512); }
-}
-
-// W (in,out) float32 [K][n_out] -> fp16 image of W^T in the swizzled K-major layout
-// ([K/64 atoms][n_pad rows][128 B]); rows >= n_out are zero.
-__global__ void pack_weight_image_kernel(const float* __restrict__ w, int K, int n_out, int n_pad, int col0, int ld,
-                                         op16* __restrict__ img, int row0, float scale, const float* __restrict__ kscale) {
-  int idx = blockIdx.x * blockDim.x + threadIdx.x;
-  if (idx >= n_out * K) return;
-  int n = idx / K, k = idx % K;
-  int row = row0 + n;
-  size_t off = (size_t)(k >> 6) * ((size_t)n_pad * 128) + (size_t)row * 128 + ((((k & 63) >> 3) ^ (row & 7)) << 4) + (k & 7) * 2;
-  img[off / 2] = __float2half_rn(w[(size_t)k * ld + col0 + n] * scale * (kscale ? kscale[k] : 1.0f));
-}
-
-// kscale (optional, [K]): a LayerNorm gain folded into the rows of W, so that the kernel's producers only standardise
-void pack_weight_image(lf_context* ctx, const float* w, int K, int n_out, int n_pad, int col0, int ld, op16* img, int row0,
-                       float scale, const float* kscale) {
-  int total = n_out * K;
-  pack_weight_image_kernel<<<(total + 255) / 256, 256, 0, ctx->stream>>>(w, K, n_out, n_pad, col0, ld, img, row0, scale, kscale);
-}
-
-// The LayerNorm offset folded into a bias: b_out[c] = scale * (b_in[c] + sum_k offset[k] W[k][col0 + c]) (b_in optional)
-__global__ void fold_bias_kernel(const float* __restrict__ w, int K, int n_out, int col0, int ld, const float* __restrict__ offset,
-                                 const float* __restrict__ b_in, float scale, float* __restrict__ b_out) {
-  int c = blockIdx.x * blockDim.x + threadIdx.x;
-  if (c >= n_out) return;
-  double acc = b_in ? (double)b_in[c] : 0.0;
-  for (int k = 0; k < K; ++k) acc += (double)offset[k] * (double)w[(size_t)k * ld + col0 + c];
-  b_out[c] = (float)(acc * scale);
-}
-
-void fold_bias(lf_context* ctx, const float* w, int K, int n_out, int col0, int ld, const float* offset, const float* b_in, float scale,
-               float* b_out) {
-  fold_bias_kernel<<<(n_out + 127) / 128, 128, 0, ctx->stream>>>(w, K, n_out, col0, ld, offset, b_in, scale, b_out);
 }
 
 lf_status make_map_f32_rows(lf_context* ctx, CUtensorMap* map, const void* base, uint64_t d1, uint64_t d2, uint64_t stride1_bytes,
@@ -1112,7 +1085,6 @@ static lf_status attention_project_impl(lf_context* ctx, ArenaCursor& cur, const
   p.chunk_row0[0] = 0; p.chunk_row0[1] = 256; p.chunk_row0[2] = 512;
   p.out_q = q; p.out_k = k; p.out_v = v; p.out_g = g; p.out_bias = bias; p.ldb = ldb; p.heads = heads; p.bias_swap = bias_swap;
   p.ldq = (Q + 15) / 16 * 16;
-  p.bias_flags = w->bias_flags;
   p.status = (Status*)ctx->tc_status;
   const int64_t tiles = (p.rows + LG_ROWS - 1) / LG_ROWS;
   const int grid = (int)(tiles < ctx->sm_count ? tiles : ctx->sm_count);
