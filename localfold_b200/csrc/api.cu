@@ -9,8 +9,13 @@
 #include <map>
 #include <mutex>
 
+#include "f32_attention.cuh"
 #include "simt_kernels.cuh"
 #include "tc_kernels.cuh"
+
+namespace {
+void configure_attention_f32();
+}
 
 // ---------------------------------------------------------------------------
 // context
@@ -99,6 +104,7 @@ static lf_status context_create(int device_ordinal, void* stream, bool make_stre
       std::call_once(per_device[device_ordinal], [] {
         cudaFuncSetAttribute(simt::center_norm_kernel<float>, cudaFuncAttributeMaxDynamicSharedMemorySize, 512 * 33 * 4);
         cudaFuncSetAttribute(simt::center_norm_kernel<op16>, cudaFuncAttributeMaxDynamicSharedMemorySize, 512 * 33 * 4);
+        configure_attention_f32();
         cudaGetLastError();
       });
   }
@@ -923,6 +929,37 @@ void sgemm(lf_context* ctx, ArenaCursor& cur, bool ta, bool tb, int epi, int M, 
 #undef SG
 }
 
+// The float32 attention core: q | k | v | gate rows -> gated output rows.  Head widths are rounded up to the next instance.
+#define ATTENTION_WIDTHS(X) X(8) X(16) X(24) X(32) X(48) X(64)
+void attention_f32(lf_context* ctx, ArenaCursor& cur, const float* qkvg, const float* bias, const float* mask, f32mma::AttentionShape s, float* out) {
+  const int D = s.d <= 32 ? (s.d + 7) / 8 * 8 : s.d <= 48 ? 48 : 64;
+  // eight warps, or as many as the queries have groups of 16: the groups are spread evenly over the blocks; small query
+  // counts put several batch rows into a block.  A thread stages at most four groups of four channels: wq >= D / 8.
+  const int groups = lf_ceil_div(s.Q, 16), tiles = lf_ceil_div(groups, 8), least = D / 8;
+  s.wq = lf_ceil_div(groups, tiles);
+  if (s.wq < least) s.wq = least;
+  s.wb = 8 / s.wq < s.batch ? 8 / s.wq : s.batch;
+  while (s.wb > 1 && (int64_t)tiles * s.heads * lf_ceil_div(s.batch, s.wb) < ctx->sm_count) s.wb /= 2;
+  const dim3 grid(lf_ceil_div(groups, s.wq), lf_ceil_div(s.batch, s.wb), s.heads);
+  const size_t smem = f32mma::attention_smem(D, s.wb);
+#define ATTENTION_CASE(D_)                                                                                                                          \
+  case D_:                                                                                                                                          \
+    if (bias) LAUNCH(ctx, cur, (f32mma::attention_kernel<D_, true>), grid, 32 * s.wb * s.wq, smem, qkvg, bias, mask, s, out);                        \
+    else LAUNCH(ctx, cur, (f32mma::attention_kernel<D_, false>), grid, 32 * s.wb * s.wq, smem, qkvg, bias, mask, s, out);                            \
+    break;
+  switch (D) { ATTENTION_WIDTHS(ATTENTION_CASE) }
+#undef ATTENTION_CASE
+}
+
+void configure_attention_f32() {
+#define ATTENTION_CASE(D_)                                                                                                                               \
+  cudaFuncSetAttribute(f32mma::attention_kernel<D_, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)f32mma::attention_smem(D_, 64 / D_));   \
+  cudaFuncSetAttribute(f32mma::attention_kernel<D_, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)f32mma::attention_smem(D_, 64 / D_));
+  ATTENTION_WIDTHS(ATTENTION_CASE)
+#undef ATTENTION_CASE
+}
+#undef ATTENTION_WIDTHS
+
 // Device views of a call's activation buffers: staged through the arena for
 // host-space calls, used in place for device-space calls.
 struct Staging {
@@ -1090,9 +1127,8 @@ void att_f32(lf_context* ctx, ArenaCursor& cur, const AttArgs& a) {
     LAUNCH(ctx, cur, (simt::pair_bias_kernel<float>), lf_ceil_div(QQ, 8), 256, 0, nrm, a.Q, c, a.heads, nullptr, nullptr,
            f[ATT_WB], a.eps, a.variance, 1, a.bias_swap, bias);
   }
-  size_t smem = (size_t)(2 * 32 * (a.d + 1) + 8 * a.d) * sizeof(float);
-  LAUNCH(ctx, cur, simt::attention_kernel, dim3(lf_ceil_div(a.Q, 8), a.batch, a.heads), 256, smem, qkvg, bias, a.mask,
-         a.batch, a.Q, a.heads, a.d, a.transpose, a.mask_mode, a.clamp, 1.0f / sqrtf((float)a.d), o);
+  attention_f32(ctx, cur, qkvg, bias, a.mask,
+                f32mma::AttentionShape{a.batch, a.Q, a.heads, a.d, a.transpose, a.mask_mode, a.clamp, 1.0f / sqrtf((float)a.d), 1, 1}, o);
   float* proj = nrm;   // the normalised input is dead
   sgemm(ctx, cur, false, false, 0, (int)R, c, HD, o, HD, 0, f[ATT_WO], c, 0, proj, c, 0, f[ATT_BO], 0, 1);
   LAUNCH(ctx, cur, (simt::finish_kernel<T>), lf_ceil_div(R * c, 256), 256, 0, proj, (const float*)nullptr,

@@ -1,0 +1,398 @@
+// Gated attention core in float32, its products on the tensor cores: every float32 operand is taken apart into three
+// bf16 terms (8 + 8 + 8 significand bits, so nothing of it is lost) and a product into the six term products above
+// 2^-24, accumulated in float32.
+#pragma once
+
+#include "common.cuh"
+
+namespace f32mma {
+
+constexpr float kLog2E = 1.4426950408889634f;
+// 2^x (relative error 2^-22).  exp(l - m) is taken as 2^(l log2(e) - m log2(e)) with one rounding of the exponent, as
+// l - m would have; the factor that the rounding of m log2(e) makes is common to a row and divides out.
+__device__ __forceinline__ float exp2_(float x) {
+  float r;
+  asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
+  return r;
+}
+
+__device__ __forceinline__ uint32_t pack_bf16(float lo, float hi) {      // round to nearest
+  uint32_t r;
+  asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(r) : "f"(hi), "f"(lo));
+  return r;
+}
+// (x, y) = sum over the three terms; the remainders are exact
+__device__ __forceinline__ void split3(float x, float y, uint32_t (&t)[3]) {
+#pragma unroll
+  for (int i = 0; i < 3; ++i) {
+    t[i] = pack_bf16(x, y);
+    x -= __uint_as_float(t[i] << 16);
+    y -= __uint_as_float(t[i] & 0xffff0000u);
+  }
+}
+// The same by truncation, for probabilities (no conversion instruction).
+__device__ __forceinline__ void split3_cut(float x, float y, uint32_t (&t)[3]) {
+#pragma unroll
+  for (int i = 0; i < 3; ++i) {
+    t[i] = __byte_perm(__float_as_uint(x), __float_as_uint(y), 0x7632);
+    if (i < 2) {
+      x -= __uint_as_float(__float_as_uint(x) & 0xffff0000u);
+      y -= __uint_as_float(__float_as_uint(y) & 0xffff0000u);
+    }
+  }
+}
+
+__device__ __forceinline__ void mma16(float (&c)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
+  asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%0, %1, %2, %3};"
+               : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3]) : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
+}
+__device__ __forceinline__ void mma8(float (&c)[4], uint32_t a0, uint32_t a1, uint32_t b0) {
+  asm volatile("mma.sync.aligned.m16n8k8.row.col.f32.bf16.bf16.f32 {%0, %1, %2, %3}, {%4, %5}, {%6}, {%0, %1, %2, %3};"
+               : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3]) : "r"(a0), "r"(a1), "r"(b0));
+}
+template <bool TRANS>
+__device__ __forceinline__ void ldmatrix4(uint32_t (&r)[4], const void* row) {
+  const uint32_t a = (uint32_t)__cvta_generic_to_shared(row);
+  if (TRANS)
+    asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0, %1, %2, %3}, [%4];" : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(a) : "memory");
+  else
+    asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0, %1, %2, %3}, [%4];" : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(a) : "memory");
+}
+template <bool TRANS>
+__device__ __forceinline__ void ldmatrix2(uint32_t& r0, uint32_t& r1, const void* row) {
+  const uint32_t a = (uint32_t)__cvta_generic_to_shared(row);
+  if (TRANS) asm volatile("ldmatrix.sync.aligned.m8n8.x2.trans.shared.b16 {%0, %1}, [%2];" : "=r"(r0), "=r"(r1) : "r"(a) : "memory");
+  else asm volatile("ldmatrix.sync.aligned.m8n8.x2.shared.b16 {%0, %1}, [%2];" : "=r"(r0), "=r"(r1) : "r"(a) : "memory");
+}
+
+struct AttentionShape {
+  int batch, Q, heads, d;
+  int transpose, mask_mode, clamp;      // mask_mode 0: logit += 1e9 (m - 1); 1: logit += m > 0 ? 0 : -1e9
+  float scale;
+  int wb, wq;                           // warps of a block: wb batch rows x wq groups of 16 queries, wq >= D / 8
+};
+
+constexpr int AT_KT = 32;                                                     // keys per staged tile
+__host__ __device__ constexpr int at_pitch(int D) { return 8 * ((D / 8) | 1); }      // odd in 16-byte units: ldmatrix rows spread over the banks
+__host__ __device__ constexpr size_t attention_smem(int D, int wb) {
+  return (size_t)2 * wb * (2 * 3 * AT_KT * at_pitch(D) * 2 + AT_KT * 4);
+}
+
+//   qkvg: [rows][4 * HD] = (q | k | v | sigmoid(gate)) in logical row order
+//   bias: [H][Q][Q] or null; mask: indexed b * Q + j, or j * batch + b when transpose
+//   out:  [rows][HD] = softmax(.) v * gate
+// A warp owns 16 queries of one (batch row, head); Q and the running output stay in registers in the tensor core's
+// fragment layout, and probabilities become the A operand of P V without leaving them.  The warps of a block share K and
+// V tiles of 32 keys, which a thread fetches a tile ahead and splits once.  A row's reference is the maximum of its first
+// 32 logits, raised only when exponentials overflow 2^60: no maximum is searched otherwise.  P V of a tile goes into
+// fresh accumulators (the leading term product apart from the others) that are added to the output outside the tensor
+// core, so that whatever the tensor core's own additions lose is of a tile's share, not of the running sum: 2e-7
+// relative against float64, as the float32 form on the FMA pipe.
+// Bound by the latency of a warp's chain (a third of the tensor pipe, half of the issue slots, 16 warps an SM).  Measured,
+// 384 x 384 with 4 heads of 16: 0.51 ms, against 5.06 ms with a warp per query and a shuffle per key and 0.68 ms with
+// four queries a thread on packed FMAs; 203 x 203, 4 x 32: 0.19 ms against 0.98 and 0.24.
+template <int D, bool BIAS>
+__global__ void __launch_bounds__(256, D <= 16 || D == 32 ? 2 : 1)
+attention_kernel(const float* __restrict__ qkvg, const float* __restrict__ bias, const float* __restrict__ mask,
+                 const AttentionShape s, float* __restrict__ out) {
+  constexpr int KT = AT_KT, PITCH = at_pitch(D), NK = D / 16, TAIL = (D / 8) & 1, ND = D / 8;
+  constexpr int PLANE = KT * PITCH;                 // bf16 elements of one term of one tile
+  extern __shared__ uint4 at_sm[];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, g = lane >> 2, t = lane & 3;
+  const int wb = warp / s.wq, wq = warp % s.wq;
+  const int d = s.d, Q = s.Q, HD = s.heads * d, ld = 4 * HD;
+  const int h = blockIdx.z, b0 = blockIdx.y * s.wb, b = b0 + wb;
+  const int q0 = (blockIdx.x * s.wq + wq) * 16;
+  // [2 buffers][wb][K: 3 terms | V: 3 terms][KT][PITCH], then [2][wb][KT] mask terms
+  __nv_bfloat16* kv_s = reinterpret_cast<__nv_bfloat16*>(at_sm);
+  float* mask_s = reinterpret_cast<float*>(kv_s + 2 * s.wb * 6 * PLANE);
+  const int tiles = (Q + KT - 1) / KT;
+  const bool active = b < s.batch && q0 < Q;        // of the warp as a whole
+
+  // ---- staging: a thread carries up to four groups of four channels a tile (K, then V), at the same places of every
+  // tile; they are fetched a tile ahead and split when their buffer is free ----
+  constexpr int NU = 4, GROUPS = D / 4;
+  const bool vec = (d & 3) == 0;
+  const float* unit_src[NU];
+  int unit_dst[NU];                                  // element offset in the buffer; -1 = no such unit
+  int unit_j[NU];
+  float4 next[NU];
+  float next_mask = 0.f;
+#pragma unroll
+  for (int i = 0; i < NU; ++i) {
+    const int u = threadIdx.x + i * blockDim.x;
+    const int e = (u % GROUPS) * 4, which = (u / GROUPS) & 1, j = (u / (2 * GROUPS)) % KT, bb = u / (2 * GROUPS * KT);
+    unit_dst[i] = bb < s.wb ? (bb * 2 + which) * 3 * PLANE + j * PITCH + e : -1;
+    unit_j[i] = bb < s.wb && b0 + bb < s.batch && e < d ? j : Q;      // Q: nothing to fetch, zeros
+    unit_src[i] = qkvg + ((int64_t)(b0 + bb) * Q + j) * ld + (1 + which) * HD + h * d + e;
+  }
+  const int mask_bb = b0 + threadIdx.x / KT, mask_j = threadIdx.x % KT;
+  const bool mask_mine = threadIdx.x < s.wb * KT;
+  auto fetch = [&](int tile) {
+    const int j0 = tile * KT;
+#pragma unroll
+    for (int i = 0; i < NU; ++i) {
+      next[i] = make_float4(0.f, 0.f, 0.f, 0.f);
+      if (unit_j[i] < Q - j0) {
+        if (vec) next[i] = __ldg(reinterpret_cast<const float4*>(unit_src[i]));
+        else {
+          const int e = (threadIdx.x + i * blockDim.x) % GROUPS * 4;
+          next[i].x = __ldg(unit_src[i]);
+          if (e + 1 < d) next[i].y = __ldg(unit_src[i] + 1);
+          if (e + 2 < d) next[i].z = __ldg(unit_src[i] + 2);
+          if (e + 3 < d) next[i].w = __ldg(unit_src[i] + 3);
+        }
+      }
+      unit_src[i] += (int64_t)KT * ld;
+    }
+    if (mask_mine) {
+      const int j = j0 + mask_j;
+      next_mask = 0.f;
+      if (j < Q) {
+        const float m = mask_bb < s.batch ? __ldg(mask + (s.transpose ? (int64_t)j * s.batch + mask_bb : (int64_t)mask_bb * Q + j)) : 1.f;
+        next_mask = s.mask_mode == 0 ? 1e9f * (m - 1.0f) : (m > 0.f ? 0.f : -1e9f);
+      }
+    }
+  };
+  auto stage = [&](int tile) {
+    const int buf = tile & 1;
+    __nv_bfloat16* base = kv_s + buf * s.wb * 6 * PLANE;
+#pragma unroll
+    for (int i = 0; i < NU; ++i) {
+      if (unit_dst[i] < 0) continue;
+      uint32_t lo[3], hi[3];
+      split3(next[i].x, next[i].y, lo);
+      split3(next[i].z, next[i].w, hi);
+#pragma unroll
+      for (int k = 0; k < 3; ++k) *reinterpret_cast<uint2*>(base + unit_dst[i] + k * PLANE) = make_uint2(lo[k], hi[k]);
+    }
+    if (mask_mine) mask_s[buf * s.wb * KT + threadIdx.x] = next_mask;
+  };
+
+  fetch(0);
+
+  // ---- Q as A fragments of its three terms ----
+  uint32_t qa[3][NK > 0 ? NK : 1][4], qt[3][2];      // qt: the last 8 channels of an odd count of groups
+  const int row0 = q0 + g, row1 = q0 + g + 8;
+  auto q_pair = [&](int row, int e, uint32_t (&term)[3]) {
+    float x = 0.f, y = 0.f;
+    if (active && row < Q) {
+      const float* src = qkvg + ((int64_t)b * Q + row) * ld + h * d + e;
+      if (e < d) x = src[0];
+      if (e + 1 < d) y = src[1];
+    }
+    split3(x, y, term);
+  };
+#pragma unroll
+  for (int kk = 0; kk < NK; ++kk)
+#pragma unroll
+    for (int r = 0; r < 4; ++r) {
+      uint32_t term[3];
+      q_pair((r & 1) ? row1 : row0, kk * 16 + 2 * t + (r >> 1) * 8, term);
+#pragma unroll
+      for (int i = 0; i < 3; ++i) qa[i][kk][r] = term[i];
+    }
+  if (TAIL) {
+#pragma unroll
+    for (int r = 0; r < 2; ++r) {
+      uint32_t term[3];
+      q_pair(r ? row1 : row0, NK * 16 + 2 * t, term);
+#pragma unroll
+      for (int i = 0; i < 3; ++i) qt[i][r] = term[i];
+    }
+  }
+
+  // the bias of a tile's keys: this thread's two rows, eight columns each
+  const bool pairs = (Q & 1) == 0;
+  const float* bias0 = BIAS ? bias + ((int64_t)h * Q + (row0 < Q ? row0 : 0)) * Q + 2 * t : nullptr;
+  const float* bias1 = BIAS ? bias + ((int64_t)h * Q + (row1 < Q ? row1 : 0)) * Q + 2 * t : nullptr;
+  float bv[4][4];
+  auto load_bias = [&](int j0) {
+    if (!BIAS) return;
+#pragma unroll
+    for (int n = 0; n < 4; ++n) {
+      const int j = j0 + n * 8;
+      if (pairs && j + 2 * t < Q) {
+        const float2 x = __ldg(reinterpret_cast<const float2*>(bias0 + j)), y = __ldg(reinterpret_cast<const float2*>(bias1 + j));
+        bv[n][0] = x.x; bv[n][1] = x.y; bv[n][2] = y.x; bv[n][3] = y.y;
+      } else {
+        bv[n][0] = j + 2 * t < Q ? __ldg(bias0 + j) : 0.f;
+        bv[n][1] = j + 2 * t + 1 < Q ? __ldg(bias0 + j + 1) : 0.f;
+        bv[n][2] = j + 2 * t < Q ? __ldg(bias1 + j) : 0.f;
+        bv[n][3] = j + 2 * t + 1 < Q ? __ldg(bias1 + j + 1) : 0.f;
+      }
+    }
+  };
+
+  float o[ND][4];
+#pragma unroll
+  for (int n = 0; n < ND; ++n)
+#pragma unroll
+    for (int e = 0; e < 4; ++e) o[n][e] = 0.f;
+  float ref[2] = {0.f, 0.f}, ref2[2] = {0.f, 0.f}, sum[2] = {0.f, 0.f};      // of rows row0, row1; ref2 = ref log2(e)
+  if (active) load_bias(0);
+  stage(0);
+  if (tiles > 1) fetch(1);
+  for (int tile = 0; tile < tiles; ++tile) {
+    __syncthreads();                                  // the tile is staged, and nobody reads the other buffer any more
+    if (tile + 1 < tiles) stage(tile + 1);
+    if (tile + 2 < tiles) fetch(tile + 2);
+    if (!active) continue;
+    const int buf = tile & 1;
+    const __nv_bfloat16* k_s = kv_s + (buf * s.wb + wb) * 6 * PLANE;
+    const __nv_bfloat16* v_s = k_s + 3 * PLANE;
+    const float* ms = mask_s + (buf * s.wb + wb) * KT;
+    // ---- S = Q K^T for 32 keys (four accumulators in flight): small term products first, the leading one last ----
+    float l[4][4];
+#pragma unroll
+    for (int n = 0; n < 4; ++n)
+#pragma unroll
+      for (int e = 0; e < 4; ++e) l[n][e] = 0.f;
+    {
+      uint32_t kb[3][2][4];
+      // matrices (keys 0-7, k 0-7), (keys 0-7, k 8-15), (keys 8-15, k 0-7), (keys 8-15, k 8-15) of each 16 keys
+      const __nv_bfloat16* base = k_s + ((lane & 7) + (lane >> 4) * 8) * PITCH + ((lane >> 3) & 1) * 8;
+#pragma unroll
+      for (int kk = 0; kk < NK; ++kk) {
+#pragma unroll
+        for (int i = 0; i < 3; ++i)
+#pragma unroll
+          for (int grp = 0; grp < 2; ++grp) ldmatrix4<false>(kb[i][grp], base + i * PLANE + grp * 16 * PITCH + kk * 16);
+#pragma unroll
+        for (int order = 2; order >= 0; --order)        // terms i and order - i
+#pragma unroll
+          for (int i = 0; i <= order; ++i)
+#pragma unroll
+            for (int n = 0; n < 4; ++n) mma16(l[n], qa[i][kk], kb[order - i][n >> 1][(n & 1) * 2], kb[order - i][n >> 1][(n & 1) * 2 + 1]);
+      }
+      if (TAIL) {
+        // matrices: keys 0-7, 8-15, 16-23, 24-31 of the last eight channels
+#pragma unroll
+        for (int i = 0; i < 3; ++i) ldmatrix4<false>(kb[i][0], k_s + i * PLANE + lane * PITCH + NK * 16);
+#pragma unroll
+        for (int order = 2; order >= 0; --order)
+#pragma unroll
+          for (int i = 0; i <= order; ++i)
+#pragma unroll
+            for (int n = 0; n < 4; ++n) mma8(l[n], qt[i][0], qt[i][1], kb[order - i][0][n]);
+      }
+    }
+    // ---- logits ----
+#pragma unroll
+    for (int n = 0; n < 4; ++n) {
+      const float2 m2 = *reinterpret_cast<const float2*>(ms + n * 8 + 2 * t);
+#pragma unroll
+      for (int e = 0; e < 4; ++e) {
+        l[n][e] = fmaf(l[n][e], s.scale, (e & 1) ? m2.y : m2.x);
+        if (BIAS) l[n][e] += bv[n][e];
+        if (s.clamp) l[n][e] = fminf(fmaxf(l[n][e], -1e8f), 1e8f);
+      }
+    }
+    if (tile * KT + KT > Q) {                           // past the end: not keys at all
+#pragma unroll
+      for (int n = 0; n < 4; ++n)
+#pragma unroll
+        for (int e = 0; e < 4; ++e)
+          if (tile * KT + n * 8 + 2 * t + (e & 1) >= Q) l[n][e] = -INFINITY;
+    }
+    if (BIAS && tile + 1 < tiles) load_bias(tile * KT + KT);      // for the next tile
+    auto row_max = [&](int r) {
+      float m = fmaxf(l[0][2 * r], l[0][2 * r + 1]);
+#pragma unroll
+      for (int n = 1; n < 4; ++n) m = fmaxf(m, fmaxf(l[n][2 * r], l[n][2 * r + 1]));
+      m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, 1));
+      return fmaxf(m, __shfl_xor_sync(0xffffffffu, m, 2));
+    };
+    if (tile == 0) {
+#pragma unroll
+      for (int r = 0; r < 2; ++r) { ref[r] = row_max(r); ref2[r] = ref[r] * kLog2E; }      // key 0 exists: finite
+    }
+    float p[4][4], ps[2];
+    auto exponentials = [&]() {
+      float a[4], c[4];
+#pragma unroll
+      for (int n = 0; n < 4; ++n) {
+#pragma unroll
+        for (int e = 0; e < 4; ++e) p[n][e] = exp2_(fmaf(l[n][e], kLog2E, -ref2[e >> 1]));
+        a[n] = p[n][0] + p[n][1];
+        c[n] = p[n][2] + p[n][3];
+      }
+      ps[0] = (a[0] + a[1]) + (a[2] + a[3]);
+      ps[1] = (c[0] + c[1]) + (c[2] + c[3]);
+    };
+    exponentials();
+    constexpr float kBig = 1.1529215e18f;      // 2^60
+    if (__any_sync(0xffffffffu, !(ps[0] <= kBig) || !(ps[1] <= kBig))) {
+#pragma unroll
+      for (int r = 0; r < 2; ++r) {
+        const float next = fmaxf(ref[r], row_max(r)), next2 = next * kLog2E, c = exp2_(ref2[r] - next2);
+        ref[r] = next;
+        ref2[r] = next2;
+        sum[r] *= c;
+#pragma unroll
+        for (int n = 0; n < ND; ++n) { o[n][2 * r] *= c; o[n][2 * r + 1] *= c; }
+      }
+      exponentials();
+    }
+    sum[0] += ps[0];
+    sum[1] += ps[1];
+    // ---- P V: the leading product and the others in accumulators of their own ----
+    float f[ND][4], fc[ND][4];
+#pragma unroll
+    for (int n = 0; n < ND; ++n)
+#pragma unroll
+      for (int e = 0; e < 4; ++e) f[n][e] = fc[n][e] = 0.f;
+#pragma unroll
+    for (int grp = 0; grp < 2; ++grp) {
+      uint32_t pa[3][4];
+#pragma unroll
+      for (int r = 0; r < 4; ++r) {
+        uint32_t term[3];
+        split3_cut(p[grp * 2 + (r >> 1)][(r & 1) * 2], p[grp * 2 + (r >> 1)][(r & 1) * 2 + 1], term);      // (row0, keys 2t), (row1, same), then keys + 8
+#pragma unroll
+        for (int i = 0; i < 3; ++i) pa[i][r] = term[i];
+      }
+#pragma unroll
+      for (int np = 0; np < ND; np += 2) {
+        uint32_t vb[3][4];
+#pragma unroll
+        for (int i = 0; i < 3; ++i) {
+          const __nv_bfloat16* base = v_s + i * PLANE + (grp * 16 + (lane & 15)) * PITCH + np * 8;
+          if (np + 1 < ND) ldmatrix4<true>(vb[i], base + (lane >> 4) * 8);
+          else ldmatrix2<true>(vb[i][0], vb[i][1], base);
+        }
+#pragma unroll
+        for (int order = 2; order >= 0; --order)
+#pragma unroll
+          for (int i = 0; i <= order; ++i) {
+            mma16(order ? fc[np] : f[np], pa[i], vb[order - i][0], vb[order - i][1]);
+            if (np + 1 < ND) mma16(order ? fc[np + 1] : f[np + 1], pa[i], vb[order - i][2], vb[order - i][3]);
+          }
+      }
+    }
+#pragma unroll
+    for (int n = 0; n < ND; ++n)
+#pragma unroll
+      for (int e = 0; e < 4; ++e) o[n][e] += f[n][e] + fc[n][e];
+  }
+  if (!active) return;
+#pragma unroll
+  for (int r = 0; r < 2; ++r) {
+    sum[r] += __shfl_xor_sync(0xffffffffu, sum[r], 1);
+    sum[r] += __shfl_xor_sync(0xffffffffu, sum[r], 2);
+    const int row = r ? row1 : row0;
+    if (row >= Q) continue;
+    const float inv = 1.0f / sum[r];
+    const float* gate = qkvg + ((int64_t)b * Q + row) * ld + 3 * HD + h * d;
+    float* dst = out + ((int64_t)b * Q + row) * HD + h * d;
+#pragma unroll
+    for (int n = 0; n < ND; ++n)
+#pragma unroll
+      for (int e = 0; e < 2; ++e) {
+        const int c = n * 8 + 2 * t + e;
+        if (c < d) dst[c] = o[n][2 * r + e] * inv * gate[c];
+      }
+  }
+}
+
+}  // namespace f32mma

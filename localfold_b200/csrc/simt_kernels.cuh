@@ -540,78 +540,6 @@ __global__ void symmetrise_sum_kernel(const float* __restrict__ half, int tokens
 }
 
 // ---------------------------------------------------------------------------
-// Gated attention core, float32, online softmax.  One warp per query, 8 queries
-// per block, key/value tiles of 32 rows staged in shared memory.
-//   qkvg: [rows][4*HD] = (q | k | v | sigmoid(gate)) in logical row order
-//   bias: [H][Q][Q] or null; mask: indexed b*Q+j, or j*batch+b when transpose
-//   mask_mode 0: logit += 1e9*(m-1); 1: logit += (m > 0 ? 0 : -1e9)
-//   clamp: limit the logit to +-1e8 after all terms are added
-//   out: [rows][HD] = softmax(.) v * gate
-__global__ void __launch_bounds__(256)
-attention_kernel(const float* __restrict__ qkvg, const float* __restrict__ bias,
-                 const float* __restrict__ mask, int batch, int Q, int heads, int d,
-                 int transpose, int mask_mode, int clamp, float scale, float* __restrict__ out) {
-  extern __shared__ float sm[];
-  const int HD = heads * d;
-  const int ld = 4 * HD;
-  float* Ks = sm;                    // [32][d+1]
-  float* Vs = Ks + 32 * (d + 1);     // [32][d+1]
-  float* Qs = Vs + 32 * (d + 1);     // [8][d]
-  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-  const int b = blockIdx.y, h = blockIdx.z;
-  const int qi = blockIdx.x * 8 + w;
-  const bool active = qi < Q;
-  const int64_t rowbase = (int64_t)b * Q;
-  if (active) for (int e = lane; e < d; e += 32) Qs[w * d + e] = qkvg[(rowbase + qi) * ld + h * d + e];
-  float run_max = -INFINITY, run_sum = 0.f, o0 = 0.f, o1 = 0.f;
-  for (int j0 = 0; j0 < Q; j0 += 32) {
-    __syncthreads();
-    for (int idx = threadIdx.x; idx < 32 * d; idx += 256) {
-      int j = idx / d, e = idx % d;
-      float kv = 0.f, vv = 0.f;
-      if (j0 + j < Q) {
-        const float* row = qkvg + (rowbase + j0 + j) * ld + h * d + e;
-        kv = row[HD];
-        vv = row[2 * HD];
-      }
-      Ks[j * (d + 1) + e] = kv;
-      Vs[j * (d + 1) + e] = vv;
-    }
-    __syncthreads();
-    if (!active) continue;
-    int j = j0 + lane;
-    float logit = -INFINITY;
-    if (j < Q) {
-      float dot = 0.f;
-      for (int e = 0; e < d; ++e) dot = fmaf(Qs[w * d + e], Ks[lane * (d + 1) + e], dot);
-      float m = mask[transpose ? (int64_t)j * batch + b : rowbase + j];
-      logit = dot * scale;
-      logit += mask_mode == 0 ? 1e9f * (m - 1.0f) : (m > 0.f ? 0.f : -1e9f);
-      if (bias) logit += bias[((int64_t)h * Q + qi) * Q + j];
-      if (clamp) logit = fminf(fmaxf(logit, -1e8f), 1e8f);
-    }
-    float tile_max = warp_max(logit);
-    float new_max = fmaxf(run_max, tile_max);
-    float corr = __expf(run_max - new_max);   // exp(-inf) = 0 on the first tile
-    float p = j < Q ? expf(logit - new_max) : 0.f;
-    run_sum = run_sum * corr + warp_sum(p);
-    run_max = new_max;
-    o0 *= corr; o1 *= corr;
-    int lim = min(32, Q - j0);
-    for (int jj = 0; jj < lim; ++jj) {
-      float pj = __shfl_sync(0xffffffffu, p, jj);
-      if (lane < d) o0 = fmaf(pj, Vs[jj * (d + 1) + lane], o0);
-      if (lane + 32 < d) o1 = fmaf(pj, Vs[jj * (d + 1) + lane + 32], o1);
-    }
-  }
-  if (!active) return;
-  const float* grow = qkvg + (rowbase + qi) * ld + 3 * HD + h * d;
-  float* orow = out + (rowbase + qi) * HD + h * d;
-  if (lane < d) orow[lane] = o0 / run_sum * grow[lane];
-  if (lane + 32 < d) orow[lane + 32] = o1 / run_sum * grow[lane + 32];
-}
-
-// ---------------------------------------------------------------------------
 // Transition glue: SwiGLU over a [rows][2*inter] tensor, gate half first.
 __global__ void swiglu_kernel(const float* __restrict__ wide, int64_t rows, int inter, float* __restrict__ out) {
   int64_t idx = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
