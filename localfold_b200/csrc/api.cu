@@ -10,6 +10,7 @@
 #include <mutex>
 
 #include "f32_attention.cuh"
+#include "row_kernels.cuh"
 #include "simt_kernels.cuh"
 #include "tc_kernels.cuh"
 
@@ -102,8 +103,10 @@ static lf_status context_create(int device_ordinal, void* stream, bool make_stre
     static std::once_flag per_device[64];
     if (device_ordinal < 64)
       std::call_once(per_device[device_ordinal], [] {
-        cudaFuncSetAttribute(simt::center_norm_kernel<float>, cudaFuncAttributeMaxDynamicSharedMemorySize, 512 * 33 * 4);
-        cudaFuncSetAttribute(simt::center_norm_kernel<op16>, cudaFuncAttributeMaxDynamicSharedMemorySize, 512 * 33 * 4);
+        cudaFuncSetAttribute(rows::center_norm_terms_kernel<float>, cudaFuncAttributeMaxDynamicSharedMemorySize, 512 * 33 * 4);
+        cudaFuncSetAttribute(rows::center_norm_terms_kernel<op16>, cudaFuncAttributeMaxDynamicSharedMemorySize, 512 * 33 * 4);
+        cudaFuncSetAttribute(rows::global_mean_kernel<float>, cudaFuncAttributeMaxDynamicSharedMemorySize, 16 * 513 * 4);
+        cudaFuncSetAttribute(rows::global_mean_kernel<bf16>, cudaFuncAttributeMaxDynamicSharedMemorySize, 16 * 513 * 4);
         configure_attention_f32();
         cudaGetLastError();
       });
@@ -807,7 +810,32 @@ lf_status publish(lf_context* ctx, lf_weights* w, lf_status s, lf_weights** out)
   if (s == LF_OK && (cudaEventCreateWithFlags(&w->ready, cudaEventDisableTiming) != cudaSuccess || cudaEventRecord(w->ready, ctx->stream) != cudaSuccess))
     s = lf_fail(ctx, LF_ERR_CUDA, "weight preparation failed: %s", cudaGetErrorString(cudaGetLastError()));
   if (s != LF_OK) { lf_weights_destroy(w); return s; }
+  w->f32 = new lf_f32_operands();
   *out = w;
+  return LF_OK;
+}
+
+// The operands of the float32 GEMM, made at the first call that needs them.
+lf_status f32_operands(lf_context* ctx, const lf_weights* w, const SplitMatrix** g) {
+  lf_f32_operands& o = *w->f32;
+  std::lock_guard<std::mutex> lock(o.mutex);
+  if (!o.made) {
+    WeightCursor dry{nullptr, 0, true};
+    LF_TRY(tc::prepare_f32_operands(ctx, w, dry, o.g));
+    if (!o.block && weight_block_take(w->device, dry.offset, &o.block, &o.block_bytes) != cudaSuccess) {
+      o.block = nullptr;
+      return lf_fail(ctx, LF_ERR_MEMORY, "float32 operands of %zu bytes refused", dry.offset);
+    }
+    WeightCursor cur{static_cast<char*>(o.block), 0, false};
+    LF_TRY(tc::prepare_f32_operands(ctx, w, cur, o.g));
+    if (!o.ready) LF_CUDA(ctx, cudaEventCreateWithFlags(&o.ready, cudaEventDisableTiming));
+    LF_CUDA(ctx, cudaEventRecord(o.ready, ctx->stream));
+    o.ctx = ctx;
+    o.made = true;
+  } else if (o.ctx != ctx) {
+    LF_CUDA(ctx, cudaStreamWaitEvent(ctx->stream, o.ready, 0));
+  }
+  *g = o.g;
   return LF_OK;
 }
 
@@ -891,8 +919,13 @@ void lf_weights_destroy(lf_weights* w) {
   cudaSetDevice(w->device);
   if (w->ready) cudaEventDestroy(w->ready);
   if (w->block) {
-    cudaDeviceSynchronize();      // nothing reads the block any more, on any stream
+    cudaDeviceSynchronize();      // nothing reads the blocks any more, on any stream
     weight_block_give(w->device, w->block, w->block_bytes);
+  }
+  if (w->f32) {
+    if (w->f32->ready) cudaEventDestroy(w->f32->ready);
+    if (w->f32->block) weight_block_give(w->device, w->f32->block, w->f32->block_bytes);
+    delete w->f32;
   }
   delete w;
 }
@@ -931,7 +964,7 @@ void sgemm(lf_context* ctx, ArenaCursor& cur, bool ta, bool tb, int epi, int M, 
 
 // The float32 attention core: q | k | v | gate rows -> gated output rows.  Head widths are rounded up to the next instance.
 #define ATTENTION_WIDTHS(X) X(8) X(16) X(24) X(32) X(48) X(64)
-void attention_f32(lf_context* ctx, ArenaCursor& cur, const float* qkvg, const float* bias, const float* mask, f32mma::AttentionShape s, float* out) {
+void attention_f32(lf_context* ctx, ArenaCursor& cur, const float* qkvg, const float* bias, const float* mask, f32mma::AttentionShape s, bf16* out) {
   const int D = s.d <= 32 ? (s.d + 7) / 8 * 8 : s.d <= 48 ? 48 : 64;
   // eight warps, or as many as the queries have groups of 16: the groups are spread evenly over the blocks; small query
   // counts put several batch rows into a block.  A thread stages at most four groups of four channels: wq >= D / 8.
@@ -959,6 +992,55 @@ void configure_attention_f32() {
 #undef ATTENTION_CASE
 }
 #undef ATTENTION_WIDTHS
+
+bool aligned16(const void* p) { return ((uintptr_t)p & 15) == 0; }
+
+// LayerNorm of `count` rows of c channels in one of its output forms; widths with a register form take it, others a warp a row.
+template <typename T, int OUT>
+void layer_norm(lf_context* ctx, ArenaCursor& cur, const void* act, int64_t count, int c, const float* gamma, const float* beta, float eps,
+                int variance, int transpose, int batch, int Q, void* out, int64_t term_stride = 0) {
+  const T* in = (const T*)act;
+#define LN_CASE(NV_, L_, R_)                                                                                                                    \
+  LAUNCH(ctx, cur, (rows::layer_norm_rows_kernel<T, NV_, L_, OUT, R_>), lf_ceil_div(count, 256 / L_ * R_), 256, 0, in, count, gamma, beta, eps, \
+         variance, transpose, batch, Q, out, term_stride)
+  const bool wide = aligned16(act) && count < ((int64_t)1 << 32);
+  if (wide && c == 64) LN_CASE(1, 16, 4);
+  else if (wide && c == 128) LN_CASE(1, 32, 4);
+  else if (wide && c == 256) LN_CASE(2, 32, 2);
+  else if (wide && c == 384) LN_CASE(3, 32, 1);
+  else if (wide && c == 512) LN_CASE(4, 32, 1);
+  else if (OUT == rows::LN_TERMS)
+    LAUNCH(ctx, cur, (rows::layer_norm_terms_kernel<T>), lf_ceil_div(count, 8), 256, 0, in, count, c, (c + 7) / 8 * 8, gamma, beta, eps, variance,
+           transpose, batch, Q, (bf16*)out, term_stride);
+  else if (OUT == rows::LN_HALF_ONE)
+    LAUNCH(ctx, cur, (simt::layer_norm_kernel<T, op16, true>), lf_ceil_div(count, 8), 256, 0, in, count, c, gamma, beta, eps, variance, transpose,
+           batch, Q, (op16*)out);
+  else if (OUT == rows::LN_HALF)
+    LAUNCH(ctx, cur, (simt::layer_norm_kernel<T, op16>), lf_ceil_div(count, 8), 256, 0, in, count, c, gamma, beta, eps, variance, transpose, batch, Q,
+           (op16*)out);
+  else
+    LAUNCH(ctx, cur, (simt::layer_norm_kernel<T>), lf_ceil_div(count, 8), 256, 0, in, count, c, gamma, beta, eps, variance, transpose, batch, Q,
+           (float*)out);
+#undef LN_CASE
+}
+
+template <typename T>
+void finish(lf_context* ctx, ArenaCursor& cur, const float* proj, const float* gate, const void* resid, int64_t count, int c, int transpose, int batch,
+            int Q, void* out) {
+  if ((c & 3) == 0 && aligned16(resid) && aligned16(out) && count < ((int64_t)1 << 32))
+    LAUNCH(ctx, cur, (rows::finish4_kernel<T>), lf_ceil_div(count * (c / 4), 256), 256, 0, proj, gate, (const T*)resid, count, c, transpose, batch, Q, (T*)out);
+  else
+    LAUNCH(ctx, cur, (simt::finish_kernel<T>), lf_ceil_div(count * c, 256), 256, 0, proj, gate, (const T*)resid, count, c, transpose, batch, Q, (T*)out);
+}
+
+// A terms matrix of `count` rows of c (rows of whole groups of eight) out of the arena.
+SplitMatrix take_terms(ArenaCursor& cur, int64_t count, int c) {
+  SplitMatrix m;
+  m.ld = (c + 7) / 8 * 8;
+  m.term_stride = count * m.ld;
+  m.p = cur.take<bf16>(3 * m.term_stride);
+  return m;
+}
 
 // Device views of a call's activation buffers: staged through the arena for
 // host-space calls, used in place for device-space calls.
@@ -988,7 +1070,7 @@ struct Staging {
 
 size_t dtype_size(int dt) { return dt == LF_DTYPE_BF16 ? 2 : 4; }
 
-// ---- triangle multiplication, float32 SIMT path ----
+// ---- triangle multiplication ----
 struct TriArgs {
   int n, cz, c, incoming, variance, residual, divide;
   float eps;
@@ -997,92 +1079,104 @@ struct TriArgs {
   const lf_weights* w;
 };
 
+// The widths the fused 16-bit kernels do not take, and float32 mode: every projection as a float32 GEMM on split operands.  The contraction
+// too, or - in 16-bit mode - on fp16 operands a, b, x with float32 accumulation.
 template <typename T>
-void tri_f32(lf_context* ctx, ArenaCursor& cur, const TriArgs& a) {
+lf_status tri_generic(lf_context* ctx, ArenaCursor& cur, const TriArgs& a, bool half) {
   const int64_t P = (int64_t)a.n * a.n;
   const int cz = a.cz, c = a.c, n = a.n;
   const auto& f = a.w->f;
-  float* zn = cur.take<float>(P * cz);
+  const SplitMatrix* g = nullptr;
+  SplitMatrix none[3];
+  if (cur.dry) g = none; else LF_TRY(f32_operands(ctx, a.w, &g));
+  const SplitMatrix zn = take_terms(cur, P, cz);
+  const int ld = half ? (n + 15) / 16 * 16 : (n + 7) / 8 * 8;      // (fp16: rows start on 32-byte boundaries)
+  const int64_t plane = (int64_t)n * ld;
+  const size_t base = cur.offset;
   float* p4 = cur.take<float>(P * 4 * c);
-  float* ga = cur.take<float>(P * c);
-  float* gb = cur.take<float>(P * c);
-  float* x = cur.take<float>(P * c);
-  LAUNCH(ctx, cur, (simt::layer_norm_kernel<T>), lf_ceil_div(P, 8), 256, 0, (const T*)a.z, P, cz, f[TRI_LN_G],
-         f[TRI_LN_B], a.eps, a.variance, 0, 1, 1, zn);
-  sgemm(ctx, cur, false, false, simt::EPI_NONE, (int)P, 4 * c, cz, zn, cz, 0, f[TRI_W4], 4 * c, 0, p4, 4 * c, 0, f[TRI_B4], 0, 1);
-  LAUNCH(ctx, cur, (simt::trimul_gate_kernel<float>), dim3(lf_ceil_div(P, 32), lf_ceil_div(c, 32)), dim3(32, 8), 0, p4,
-         a.mask, P, c, n, n, ga, gb);
-  if (!a.incoming)   // x[i][j] = sum_k a[i][k] b[j][k]
-    sgemm(ctx, cur, false, true, 0, n, n, n, ga, n, P, gb, n, P, x, n, P, nullptr, 0, c);
-  else               // x[i][j] = sum_k b[k][i] a[k][j]
-    sgemm(ctx, cur, true, false, 0, n, n, n, gb, n, P, ga, n, P, x, n, P, nullptr, 0, c);
-  // xn reuses p4's storage (p4 is dead), then the two output GEMMs
-  float* xn = p4;
-  float* proj = p4 + P * c;
-  float* gate = p4 + P * c + P * cz;   // needs 4c >= c + 2cz: checked by the caller
-  LAUNCH(ctx, cur, (simt::center_norm_kernel<float>), lf_ceil_div(P, 32), 256, (size_t)c * 33 * sizeof(float), x, P, c, n, n,
-         f[TRI_LNO_G], f[TRI_LNO_B], a.eps, a.variance, a.divide ? 1.0f / n : 1.0f, xn);
-  sgemm(ctx, cur, false, false, 0, (int)P, cz, c, xn, c, 0, f[TRI_WZ], cz, 0, proj, cz, 0, f[TRI_BZ], 0, 1);
-  sgemm(ctx, cur, false, false, 0, (int)P, cz, cz, zn, cz, 0, f[TRI_WG], cz, 0, gate, cz, 0, f[TRI_BG], 0, 1);
-  LAUNCH(ctx, cur, (simt::finish_kernel<T>), lf_ceil_div(P * cz, 256), 256, 0, proj, gate,
-         a.residual ? (const T*)a.z : (const T*)nullptr, P, cz, 0, 1, 1, (T*)a.out);
+  const size_t p4_end = cur.offset;
+  layer_norm<T, rows::LN_TERMS>(ctx, cur, a.z, P, cz, f[TRI_LN_G], f[TRI_LN_B], a.eps, a.variance, 0, 1, 1, (void*)zn.p, zn.term_stride);
+  LF_TRY(tc::gemm_f32(ctx, cur, 0, zn, g[0], (int)P, 4 * c, cz, 1, {p4, nullptr, 4 * c, 0, 0, f[TRI_B4], 4 * c, 0, 0, 0}));
+  float x_scale = 1.0f;
+  const void* x = nullptr;
+  int ldx = ld;
+  if (half) {
+    op16* ga = cur.take<op16>(plane * c);
+    op16* gb = cur.take<op16>(plane * c);
+    op16* xh = cur.take<op16>(plane * c);
+    LAUNCH(ctx, cur, (simt::trimul_gate_kernel<op16>), dim3(lf_ceil_div(P, 32), lf_ceil_div(c, 32)), dim3(32, 8), 0, p4, a.mask, P, c, n, ld, ga, gb);
+    // x is stored as fp16 scaled by a power of two near 1/sqrt(n) so that sums over n terms stay far from the fp16
+    // limits; the centre LayerNorm undoes the scale exactly.
+    x_scale = ldexpf(1.0f, -(int)(0.5f * log2f((float)n)));
+    LF_TRY(tc::contract(ctx, cur, ga, gb, xh, n, ld, c, a.incoming, x_scale));
+    x = xh;
+  } else {
+    SplitMatrix ga, gb;
+    ga.ld = gb.ld = ld;
+    ga.batch_stride = gb.batch_stride = plane;
+    ga.term_stride = gb.term_stride = plane * c;
+    ga.p = cur.take<bf16>(3 * plane * c);
+    gb.p = cur.take<bf16>(3 * plane * c);
+    ldx = (n + 3) / 4 * 4;
+    float* xf = cur.take<float>((int64_t)n * ldx * c);
+    LAUNCH(ctx, cur, rows::trimul_gate_terms_kernel, dim3((unsigned)(n * lf_ceil_div(n, 32)), lf_ceil_div(c, 32)), 256, 0, p4, a.mask, c, n, ld, (bf16*)ga.p,
+           (bf16*)gb.p, ga.term_stride);
+    // outgoing x[i][j] = sum_k a[i][k] b[j][k]; incoming x[i][j] = sum_k b[k][i] a[k][j]
+    const tc::Gemm3Out to{xf, nullptr, ldx, (int64_t)n * ldx, 0, nullptr, 0, 0, 0, 0};
+    if (!a.incoming) LF_TRY(tc::gemm_f32(ctx, cur, 0, ga, gb, n, n, n, c, to));
+    else LF_TRY(tc::gemm_f32(ctx, cur, 1, gb, ga, n, n, n, c, to));
+    x = xf;
+  }
+  // p4 is dead: the normalised x and the two outputs take its place where they fit
+  const size_t end = cur.offset;
+  cur.offset = base;
+  SplitMatrix xn = take_terms(cur, P, c);
+  float* proj = cur.take<float>(P * cz);
+  float* gate = cur.take<float>(P * cz);
+  if (cur.offset > p4_end) {
+    cur.offset = end;
+    xn = take_terms(cur, P, c);
+    proj = cur.take<float>(P * cz);
+    gate = cur.take<float>(P * cz);
+  } else cur.offset = end;
+  const dim3 tiles((unsigned)(n * lf_ceil_div(n, 32)));
+  const size_t smem = (size_t)c * 33 * sizeof(float);
+  const float prescale = (a.divide ? 1.0f / n : 1.0f) / x_scale;
+  if (half)
+    LAUNCH(ctx, cur, (rows::center_norm_terms_kernel<op16>), tiles, 256, smem, (const op16*)x, c, n, ldx, f[TRI_LNO_G], f[TRI_LNO_B], a.eps, a.variance, prescale,
+           (int)xn.ld, (bf16*)xn.p, xn.term_stride);
+  else
+    LAUNCH(ctx, cur, (rows::center_norm_terms_kernel<float>), tiles, 256, smem, (const float*)x, c, n, ldx, f[TRI_LNO_G], f[TRI_LNO_B], a.eps, a.variance, prescale,
+           (int)xn.ld, (bf16*)xn.p, xn.term_stride);
+  LF_TRY(tc::gemm_f32(ctx, cur, 0, xn, g[1], (int)P, cz, c, 1, {proj, nullptr, cz, 0, 0, f[TRI_BZ], cz, 0, 0, 0}));
+  LF_TRY(tc::gemm_f32(ctx, cur, 0, zn, g[2], (int)P, cz, cz, 1, {gate, nullptr, cz, 0, 0, f[TRI_BG], cz, 0, 0, 0}));
+  finish<T>(ctx, cur, proj, gate, a.residual ? a.z : nullptr, P, cz, 0, 1, 1, a.out);
+  return LF_OK;
 }
 
-// 16-bit path: float32 LayerNorm statistics and gates, fp16 operands a, b, x with
-// float32 accumulation on the tensor cores for the contraction.
-template <typename T>
+// 16-bit path at 128 channels: fp16 operands a, b, x, float32 LayerNorm statistics and gates, everything on the fused kernels.
 lf_status tri_bf16(lf_context* ctx, ArenaCursor& cur, const TriArgs& a) {
-  const int64_t P = (int64_t)a.n * a.n;
-  const int cz = a.cz, c = a.c, n = a.n;
+  const int c = a.c, n = a.n;
   const int ld = (n + 15) / 16 * 16;        // rows start on 32-byte boundaries (TMA needs 16, the 256-bit stores 32)
   const int64_t plane = (int64_t)n * ld;
-  const auto& f = a.w->f;
-  float* zn = cur.take<float>(P * cz);
-  float* p4 = cur.take<float>(P * 4 * c);
   op16* ga = cur.take<op16>(plane * c);
   op16* gb = cur.take<op16>(plane * c);
   op16* x = cur.take<op16>(plane * c);
-  if (!tc::ln_gemm_supported(a.w))
-    LAUNCH(ctx, cur, (simt::layer_norm_kernel<T>), lf_ceil_div(P, 8), 256, 0, (const T*)a.z, P, cz, f[TRI_LN_G],
-           f[TRI_LN_B], a.eps, a.variance, 0, 1, 1, zn);
-  if (tc::ln_gemm_supported(a.w)) {
-    LF_TRY(tc::triangle_project(ctx, cur, a.z, a.act_dtype, a.mask, n, n, ld, a.variance, a.eps, a.w, ga, gb));
-  } else {
-    sgemm(ctx, cur, false, false, simt::EPI_NONE, (int)P, 4 * c, cz, zn, cz, 0, f[TRI_W4], 4 * c, 0, p4, 4 * c, 0, f[TRI_B4], 0, 1);
-    LAUNCH(ctx, cur, (simt::trimul_gate_kernel<op16>), dim3(lf_ceil_div(P, 32), lf_ceil_div(c, 32)), dim3(32, 8), 0, p4,
-           a.mask, P, c, n, ld, ga, gb);
-  }
-  // x is stored as fp16 scaled by a power of two near 1/sqrt(n) so that sums over n terms
-  // stay far from the fp16 limits; the centre LayerNorm undoes the scale exactly.
+  LF_TRY(tc::triangle_project(ctx, cur, a.z, a.act_dtype, a.mask, n, n, ld, a.variance, a.eps, a.w, ga, gb));
+  // (x is scaled as in tri_generic)
   const float xscale = ldexpf(1.0f, -(int)(0.5f * log2f((float)n)));
   LF_TRY(tc::contract(ctx, cur, ga, gb, x, n, ld, c, a.incoming, xscale));
-  if (tc::ln_gemm_supported(a.w)) {
-    const float xs = xscale * (a.divide ? (float)n : 1.0f);
-    LF_TRY(tc::triangle_output(ctx, cur, x, n, n, ld, a.eps * xs * xs, a.z, a.act_dtype, a.variance, a.eps, a.w,
-                               a.residual ? a.z : nullptr, a.out));
-    return LF_OK;
-  }
-  float* xn = p4;
-  float* proj = p4 + P * c;
-  float* gate = p4 + P * c + P * cz;
-  LAUNCH(ctx, cur, (simt::center_norm_kernel<op16>), lf_ceil_div(P, 32), 256, (size_t)c * 33 * sizeof(float), x, P, c, n, ld,
-         f[TRI_LNO_G], f[TRI_LNO_B], a.eps, a.variance, (a.divide ? 1.0f / n : 1.0f) / xscale, xn);
-  sgemm(ctx, cur, false, false, 0, (int)P, cz, c, xn, c, 0, f[TRI_WZ], cz, 0, proj, cz, 0, f[TRI_BZ], 0, 1);
-  sgemm(ctx, cur, false, false, 0, (int)P, cz, cz, zn, cz, 0, f[TRI_WG], cz, 0, gate, cz, 0, f[TRI_BG], 0, 1);
-  LAUNCH(ctx, cur, (simt::finish_kernel<T>), lf_ceil_div(P * cz, 256), 256, 0, proj, gate,
-         a.residual ? (const T*)a.z : (const T*)nullptr, P, cz, 0, 1, 1, (T*)a.out);
-  return LF_OK;
+  const float xs = xscale * (a.divide ? (float)n : 1.0f);
+  return tc::triangle_output(ctx, cur, x, n, n, ld, a.eps * xs * xs, a.z, a.act_dtype, a.variance, a.eps, a.w, a.residual ? a.z : nullptr, a.out);
 }
 
 lf_status tri_dispatch(lf_context* ctx, ArenaCursor& cur, const TriArgs& a, int precision) {
-  if (precision == LF_PRECISION_BF16 && tc::contract_supported(a.n, a.c)) {
-    return a.act_dtype == LF_DTYPE_BF16 ? tri_bf16<bf16>(ctx, cur, a) : tri_bf16<float>(ctx, cur, a);
-  }
-  if (a.act_dtype == LF_DTYPE_BF16) tri_f32<bf16>(ctx, cur, a); else tri_f32<float>(ctx, cur, a);
-  return LF_OK;
+  const bool half = precision == LF_PRECISION_BF16 && tc::contract_supported(a.n, a.c);
+  if (half && tc::ln_gemm_supported(a.w)) return tri_bf16(ctx, cur, a);
+  return a.act_dtype == LF_DTYPE_BF16 ? tri_generic<bf16>(ctx, cur, a, half) : tri_generic<float>(ctx, cur, a, half);
 }
 
-// ---- attention engine, float32 SIMT path ----
+// ---- attention engine, float32 path ----
 struct AttArgs {
   int batch, Q, ch, heads, d, transpose, variance, residual;
   int bias_mode;       // 0 none, 1 from a separate pair tensor, 2 from the normalised input
@@ -1096,43 +1190,94 @@ struct AttArgs {
   const lf_weights* w;
 };
 
-template <typename T>
-void att_f32(lf_context* ctx, ArenaCursor& cur, const AttArgs& a) {
-  const int64_t R = (int64_t)a.batch * a.Q;
-  const int HD = a.heads * a.d, c = a.ch;
+// The pair bias of a.bias_mode 1 (a pair tensor with a LayerNorm of its own) as float32 [heads][Q][Q].
+lf_status separate_bias(lf_context* ctx, ArenaCursor& cur, const AttArgs& a, float* bias) {
   const auto& f = a.w->f;
-  float* nrm = cur.take<float>(R * c);
-  float* qkvg = cur.take<float>(R * 4 * HD);
-  float* bias = a.bias_mode ? cur.take<float>((int64_t)a.heads * a.Q * a.Q) : nullptr;
-  float* o = cur.take<float>(R * HD);
-  LAUNCH(ctx, cur, (simt::layer_norm_kernel<T>), lf_ceil_div(R, 8), 256, 0, (const T*)a.act, R, c, f[ATT_LN_G],
-         f[ATT_LN_B], a.eps, a.variance, a.transpose, a.batch, a.Q, nrm);
-  sgemm(ctx, cur, false, false, simt::EPI_SIGMOID_FROM_COL, (int)R, 4 * HD, c, nrm, c, 0, f[ATT_W4], 4 * HD, 0, qkvg,
-        4 * HD, 0, f[ATT_B4], 3 * HD, 1);
   const int64_t QQ = (int64_t)a.Q * a.Q;
-  if (a.bias_mode == 1 && a.tc_pair_bias && tc::pair_bias_supported(a.w) && !a.bias_swap) {
+  if (a.tc_pair_bias && tc::pair_bias_supported(a.w) && !a.bias_swap) {
     // the pair-sized pass of this operator: LayerNorm of the pair and its projection onto the heads, fp16 out
     const int ldb = (a.Q + 15) / 16 * 16;
     op16* b16 = cur.take<op16>((int64_t)a.heads * a.Q * ldb);
-    (void)tc::pair_bias_project(ctx, cur, a.pair, a.pair_dtype, a.Q, a.pair_variance, a.pair_eps, a.heads, a.w, b16, ldb);
+    LF_TRY(tc::pair_bias_project(ctx, cur, a.pair, a.pair_dtype, a.Q, a.pair_variance, a.pair_eps, a.heads, a.w, b16, ldb));
     LAUNCH(ctx, cur, simt::widen_bias_kernel, lf_ceil_div(QQ * a.heads, 256), 256, 0, b16, a.heads, a.Q, ldb, bias);
-  } else if (a.bias_mode == 1) {
-    if (a.pair_dtype == LF_DTYPE_BF16)
-      LAUNCH(ctx, cur, (simt::pair_bias_kernel<bf16>), lf_ceil_div(QQ, 8), 256, 0, (const bf16*)a.pair, a.Q, a.pair_ch,
-             a.heads, f[ATT_PLN_G], f[ATT_PLN_B], f[ATT_WB], a.pair_eps, a.pair_variance, 0, a.bias_swap, bias);
-    else
-      LAUNCH(ctx, cur, (simt::pair_bias_kernel<float>), lf_ceil_div(QQ, 8), 256, 0, (const float*)a.pair, a.Q, a.pair_ch,
-             a.heads, f[ATT_PLN_G], f[ATT_PLN_B], f[ATT_WB], a.pair_eps, a.pair_variance, 0, a.bias_swap, bias);
-  } else if (a.bias_mode == 2) {
-    LAUNCH(ctx, cur, (simt::pair_bias_kernel<float>), lf_ceil_div(QQ, 8), 256, 0, nrm, a.Q, c, a.heads, nullptr, nullptr,
-           f[ATT_WB], a.eps, a.variance, 1, a.bias_swap, bias);
-  }
+  } else if (a.pair_dtype == LF_DTYPE_BF16)
+    LAUNCH(ctx, cur, (simt::pair_bias_kernel<bf16>), lf_ceil_div(QQ, 8), 256, 0, (const bf16*)a.pair, a.Q, a.pair_ch, a.heads, f[ATT_PLN_G], f[ATT_PLN_B],
+           f[ATT_WB], a.pair_eps, a.pair_variance, 0, a.bias_swap, bias);
+  else
+    LAUNCH(ctx, cur, (simt::pair_bias_kernel<float>), lf_ceil_div(QQ, 8), 256, 0, (const float*)a.pair, a.Q, a.pair_ch, a.heads, f[ATT_PLN_G], f[ATT_PLN_B],
+           f[ATT_WB], a.pair_eps, a.pair_variance, 0, a.bias_swap, bias);
+  return LF_OK;
+}
+
+template <typename T>
+lf_status att_f32(lf_context* ctx, ArenaCursor& cur, const AttArgs& a) {
+  const int64_t R = (int64_t)a.batch * a.Q;
+  const int HD = a.heads * a.d, c = a.ch;
+  const auto& f = a.w->f;
+  const SplitMatrix* g = nullptr;
+  SplitMatrix none[3];
+  if (cur.dry) g = none; else LF_TRY(f32_operands(ctx, a.w, &g));
+  const SplitMatrix nrm = take_terms(cur, R, c);
+  // q | k | v | sigmoid(gate), and the pair bias columns when the bias comes from the normalised input
+  const int wide = 4 * HD + (a.bias_mode == 2 ? a.heads : 0), ldq = (wide + 3) / 4 * 4;
+  float* qkvg = cur.take<float>(R * ldq);
+  float* bias = a.bias_mode ? cur.take<float>((int64_t)a.heads * a.Q * a.Q) : nullptr;
+  const SplitMatrix o = take_terms(cur, R, HD);
+  float* proj = cur.take<float>(R * c);
+  layer_norm<T, rows::LN_TERMS>(ctx, cur, a.act, R, c, f[ATT_LN_G], f[ATT_LN_B], a.eps, a.variance, a.transpose, a.batch, a.Q, (void*)nrm.p, nrm.term_stride);
+  LF_TRY(tc::gemm_f32(ctx, cur, 0, nrm, g[0], (int)R, wide, c, 1, {qkvg, nullptr, ldq, 0, 0, f[ATT_B4], 4 * HD, 0, 3 * HD, 4 * HD}));
+  if (a.bias_mode == 1) LF_TRY(separate_bias(ctx, cur, a, bias));
+  else if (a.bias_mode == 2)
+    LAUNCH(ctx, cur, rows::bias_columns_kernel, lf_ceil_div((int64_t)a.Q * a.Q, 256), 256, 0, qkvg, (int64_t)ldq, 4 * HD, a.Q, a.heads, a.bias_swap, bias);
   attention_f32(ctx, cur, qkvg, bias, a.mask,
-                f32mma::AttentionShape{a.batch, a.Q, a.heads, a.d, a.transpose, a.mask_mode, a.clamp, 1.0f / sqrtf((float)a.d), 1, 1}, o);
-  float* proj = nrm;   // the normalised input is dead
-  sgemm(ctx, cur, false, false, 0, (int)R, c, HD, o, HD, 0, f[ATT_WO], c, 0, proj, c, 0, f[ATT_BO], 0, 1);
-  LAUNCH(ctx, cur, (simt::finish_kernel<T>), lf_ceil_div(R * c, 256), 256, 0, proj, (const float*)nullptr,
-         a.residual ? (const T*)a.act : (const T*)nullptr, R, c, a.transpose, a.batch, a.Q, (T*)a.out);
+                f32mma::AttentionShape{a.batch, a.Q, a.heads, a.d, a.transpose, a.mask_mode, a.clamp, 1.0f / sqrtf((float)a.d), ldq, o.ld, o.term_stride, 1, 1},
+                (bf16*)o.p);
+  LF_TRY(tc::gemm_f32(ctx, cur, 0, o, g[1], (int)R, c, HD, 1, {proj, nullptr, c, 0, 0, f[ATT_BO], c, 0, 0, 0}));
+  finish<T>(ctx, cur, proj, nullptr, a.residual ? a.act : nullptr, R, c, a.transpose, a.batch, a.Q, a.out);
+  return LF_OK;
+}
+
+// AF3 MSA pair-weighted averaging (no query, no key): the weights are the softmax of the pair bias under one key mask - a token
+// that any sequence covers is a key for all of them - so they are the same for every sequence and are made once; the
+// averages over the tokens are then one GEMM per head, [i][j] x [j][(sequence, channel)].  As the attention of every
+// sequence by itself this took 11.2 ms (1.4 ms on the tensor cores) for 512 sequences of 384 tokens, 8 heads of 8.
+lf_status msa_average(lf_context* ctx, ArenaCursor& cur, const AttArgs& a) {
+  const int S = a.batch, n = a.Q, H = a.heads, d = a.d, HD = H * d, c = a.ch;
+  const int64_t R = (int64_t)S * n;
+  const auto& f = a.w->f;
+  const SplitMatrix* g = nullptr;
+  SplitMatrix none[3];
+  if (cur.dry) g = none; else LF_TRY(f32_operands(ctx, a.w, &g));
+  float* bias = cur.take<float>((int64_t)H * n * n);
+  float* key = cur.take<float>(n);
+  SplitMatrix w, v;
+  w.ld = (n + 7) / 8 * 8;
+  w.batch_stride = (int64_t)n * w.ld;
+  w.term_stride = H * w.batch_stride;
+  w.p = cur.take<bf16>(3 * w.term_stride);
+  const SplitMatrix nrm = take_terms(cur, R, c);
+  float* vg = cur.take<float>(R * 2 * HD);
+  v.ld = ((int64_t)S * d + 7) / 8 * 8;
+  v.batch_stride = (int64_t)n * v.ld;
+  v.term_stride = H * v.batch_stride;
+  v.p = cur.take<bf16>(3 * v.term_stride);
+  const int64_t ldx = ((int64_t)S * d + 3) / 4 * 4;
+  float* x = cur.take<float>((int64_t)H * n * ldx);
+  const SplitMatrix o = take_terms(cur, R, HD);
+  float* proj = cur.take<float>(R * c);
+  if ((int64_t)S * d > 0x7fffffff) return lf_fail(ctx, LF_ERR_SHAPE, "too many sequences for one average");
+  LF_TRY(separate_bias(ctx, cur, a, bias));
+  LAUNCH(ctx, cur, rows::key_mask_kernel, lf_ceil_div(n, 32), dim3(32, 32), 0, a.mask, S, n, key);
+  LAUNCH(ctx, cur, rows::average_weights_kernel, dim3(lf_ceil_div(n, 32), H), 256, 0, bias, key, n, (int)w.ld, (bf16*)w.p, w.term_stride);
+  layer_norm<float, rows::LN_TERMS>(ctx, cur, a.act, R, c, f[ATT_LN_G], f[ATT_LN_B], a.eps, a.variance, 0, 1, 1, (void*)nrm.p, nrm.term_stride);
+  LF_TRY(tc::gemm_f32(ctx, cur, 0, nrm, g[0], (int)R, 2 * HD, c, 1, {vg, nullptr, 2 * HD, 0, 0, f[ATT_B4] ? f[ATT_B4] + 2 * HD : nullptr, 2 * HD, 0, HD, 2 * HD}));
+  LAUNCH(ctx, cur, rows::average_values_kernel, dim3(lf_ceil_div(S, 128), n, H), 128, 0, vg, (int64_t)2 * HD, S, n, H, d, (int)v.ld, (bf16*)v.p, v.term_stride);
+  LF_TRY(tc::gemm_f32(ctx, cur, 1, w, v, n, S * d, n, H, {x, nullptr, ldx, (int64_t)n * ldx, 0, nullptr, 0, 0, 0, 0}));
+  LAUNCH(ctx, cur, rows::average_gate_kernel, lf_ceil_div(R * (o.ld / 2), 256), 256, 0, x, ldx, vg + HD, (int64_t)2 * HD, S, n, H, d, (int)o.ld, (bf16*)o.p,
+         o.term_stride);
+  LF_TRY(tc::gemm_f32(ctx, cur, 0, o, g[1], (int)R, c, HD, 1, {proj, nullptr, c, 0, 0, f[ATT_BO], c, 0, 0, 0}));
+  finish<float>(ctx, cur, proj, nullptr, a.residual ? a.act : nullptr, R, c, 0, 1, 1, a.out);
+  return LF_OK;
 }
 
 // 16-bit path: tensor-core LayerNorm + q/k/v/gate/bias projection, then the attention core.
@@ -1197,8 +1342,7 @@ lf_status att_mixed(lf_context* ctx, ArenaCursor& cur, const AttArgs& a) {
   op16* v16 = k16 + RP * 128;
   op16* g16 = v16 + RP * 128;
   op16* o16 = cur.take<op16>(RP * 128);
-  LAUNCH(ctx, cur, (simt::layer_norm_kernel<T, op16>), lf_ceil_div(R, 8), 256, 0, (const T*)a.act, R, c, f[ATT_LN_G],
-         f[ATT_LN_B], a.eps, a.variance, a.transpose, a.batch, a.Q, nrm);
+  layer_norm<T, rows::LN_HALF>(ctx, cur, a.act, R, c, f[ATT_LN_G], f[ATT_LN_B], a.eps, a.variance, a.transpose, a.batch, a.Q, nrm);
   LF_TRY(hgemm(ctx, cur, nrm, gemm_operand(a.w, 0), qkvg, R, 4 * HD, c));
   if (ldb != a.Q && !cur.dry) {
     // padding rows and columns are read as keys past the end (masked out): they must hold finite values
@@ -1234,38 +1378,41 @@ lf_status att_dispatch(lf_context* ctx, ArenaCursor& cur, const AttArgs& a, int 
   }
   AttArgs b = a;
   b.tc_pair_bias = precision == LF_PRECISION_BF16 ? 1 : 0;
-  if (b.act_dtype == LF_DTYPE_BF16) att_f32<bf16>(ctx, cur, b); else att_f32<float>(ctx, cur, b);
-  return LF_OK;
+  return b.act_dtype == LF_DTYPE_BF16 ? att_f32<bf16>(ctx, cur, b) : att_f32<float>(ctx, cur, b);
 }
 
-// ---- transition, float32 SIMT path (row-chunked so the wide hidden stays bounded) ----
+// ---- transition, float32 path (row-chunked so the wide hidden stays bounded) ----
 struct TrnArgs {
   int64_t rows; int ch, hidden, swiglu, variance, residual; float eps; int act_dtype;
   const void* act; void* out; const lf_weights* w;
 };
 
 template <typename T>
-void trn_f32(lf_context* ctx, ArenaCursor& cur, const TrnArgs& a) {
+lf_status trn_f32(lf_context* ctx, ArenaCursor& cur, const TrnArgs& a) {
   const auto& f = a.w->f;
   const int c = a.ch, hd = a.hidden, wide = a.swiglu ? 2 * hd : hd;
   const int64_t chunk = a.rows < (1 << 18) ? a.rows : (1 << 18);
-  float* nrm = cur.take<float>(chunk * c);
-  float* h1 = cur.take<float>(chunk * wide);
-  float* h2 = a.swiglu ? cur.take<float>(chunk * hd) : h1;
+  const SplitMatrix* g = nullptr;
+  SplitMatrix none[3];
+  if (cur.dry) g = none; else LF_TRY(f32_operands(ctx, a.w, &g));
+  const SplitMatrix nrm = take_terms(cur, chunk, c), hid = take_terms(cur, chunk, hd);
+  float* h1 = a.swiglu ? cur.take<float>(chunk * wide) : nullptr;
   float* proj = cur.take<float>(chunk * c);
   for (int64_t r0 = 0; r0 < a.rows; r0 += chunk) {
-    int64_t rows = a.rows - r0 < chunk ? a.rows - r0 : chunk;
+    const int64_t count = a.rows - r0 < chunk ? a.rows - r0 : chunk;
     const T* in = (const T*)a.act + r0 * c;
     T* out = (T*)a.out + r0 * c;
-    LAUNCH(ctx, cur, (simt::layer_norm_kernel<T>), lf_ceil_div(rows, 8), 256, 0, in, rows, c, f[TRN_LN_G], f[TRN_LN_B],
-           a.eps, a.variance, 0, 1, 1, nrm);
-    sgemm(ctx, cur, false, false, a.swiglu ? simt::EPI_NONE : simt::EPI_RELU, (int)rows, wide, c, nrm, c, 0, f[TRN_W1],
-          wide, 0, h1, wide, 0, f[TRN_B1], 0, 1);
-    if (a.swiglu) LAUNCH(ctx, cur, simt::swiglu_kernel, lf_ceil_div(rows * hd, 256), 256, 0, h1, rows, hd, h2);
-    sgemm(ctx, cur, false, false, 0, (int)rows, c, hd, h2, hd, 0, f[TRN_W2], c, 0, proj, c, 0, f[TRN_B2], 0, 1);
-    LAUNCH(ctx, cur, (simt::finish_kernel<T>), lf_ceil_div(rows * c, 256), 256, 0, proj, (const float*)nullptr,
-           a.residual ? in : (const T*)nullptr, rows, c, 0, 1, 1, out);
+    layer_norm<T, rows::LN_TERMS>(ctx, cur, in, count, c, f[TRN_LN_G], f[TRN_LN_B], a.eps, a.variance, 0, 1, 1, (void*)nrm.p, nrm.term_stride);
+    if (a.swiglu) {
+      LF_TRY(tc::gemm_f32(ctx, cur, 0, nrm, g[0], (int)count, wide, c, 1, {h1, nullptr, wide, 0, 0, f[TRN_B1], wide, 0, 0, 0}));
+      LAUNCH(ctx, cur, rows::swiglu_terms_kernel, lf_ceil_div(count * (hid.ld / 2), 256), 256, 0, h1, count, hd, (int)hid.ld, (bf16*)hid.p, hid.term_stride);
+    } else {
+      LF_TRY(tc::gemm_f32(ctx, cur, 0, nrm, g[0], (int)count, wide, c, 1, {nullptr, (bf16*)hid.p, hid.ld, 0, hid.term_stride, f[TRN_B1], wide, 1, 0, 0}));
+    }
+    LF_TRY(tc::gemm_f32(ctx, cur, 0, hid, g[1], (int)count, c, hd, 1, {proj, nullptr, c, 0, 0, f[TRN_B2], c, 0, 0, 0}));
+    finish<T>(ctx, cur, proj, nullptr, a.residual ? in : (const T*)nullptr, count, c, 0, 1, 1, out);
   }
+  return LF_OK;
 }
 
 // 16-bit path for the widths the fused transition kernel does not take (the MSA transitions, other pair widths):
@@ -1282,20 +1429,19 @@ lf_status trn_half(lf_context* ctx, ArenaCursor& cur, const TrnArgs& a) {
   const op16* w1 = gemm_operand(a.w, 0);
   const op16* w2 = gemm_operand(a.w, 1);
   for (int64_t r0 = 0; r0 < a.rows; r0 += chunk) {
-    int64_t rows = a.rows - r0 < chunk ? a.rows - r0 : chunk;
+    const int64_t count = a.rows - r0 < chunk ? a.rows - r0 : chunk;
     const T* in = (const T*)a.act + r0 * c;
     T* out = (T*)a.out + r0 * c;
-    LAUNCH(ctx, cur, (simt::layer_norm_kernel<T, op16, true>), lf_ceil_div(rows, 8), 256, 0, in, rows, c, f[TRN_LN_G], f[TRN_LN_B],
-           a.eps, a.variance, 0, 1, 1, nrm);
+    layer_norm<T, rows::LN_HALF_ONE>(ctx, cur, in, count, c, f[TRN_LN_G], f[TRN_LN_B], a.eps, a.variance, 0, 1, 1, nrm);
     if (a.swiglu) {
-      LF_TRY(hgemm(ctx, cur, nrm, w1, h1, rows, wide, c16));
-      LAUNCH(ctx, cur, simt::hidden_act_half_kernel, lf_ceil_div(rows * hd, 256), 256, 0, h1, (const float*)nullptr, rows, hd, wide, 1, h2);
+      LF_TRY(hgemm(ctx, cur, nrm, w1, h1, count, wide, c16));
+      LAUNCH(ctx, cur, simt::hidden_act_half_kernel, lf_ceil_div(count * hd, 256), 256, 0, h1, (const float*)nullptr, count, hd, wide, 1, h2);
     } else {
-      LF_TRY(hgemm(ctx, cur, nrm, w1, h1, rows, wide, c16, nullptr, 1));     // ReLU in the GEMM's epilogue
+      LF_TRY(hgemm(ctx, cur, nrm, w1, h1, count, wide, c16, nullptr, 1));     // ReLU in the GEMM's epilogue
     }
-    LF_TRY(hgemm(ctx, cur, h2, w2, nrm, rows, c, hd));
-    LAUNCH(ctx, cur, (simt::finish_half_kernel<T>), lf_ceil_div(rows * c / 8, 256), 256, 0, nrm, 1.0f, f[TRN_B2],
-           a.residual ? in : (const T*)nullptr, rows, c, 0, 1, 1, out);
+    LF_TRY(hgemm(ctx, cur, h2, w2, nrm, count, c, hd));
+    LAUNCH(ctx, cur, (simt::finish_half_kernel<T>), lf_ceil_div(count * c / 8, 256), 256, 0, nrm, 1.0f, f[TRN_B2],
+           a.residual ? in : (const T*)nullptr, count, c, 0, 1, 1, out);
   }
   return LF_OK;
 }
@@ -1305,8 +1451,7 @@ lf_status trn_dispatch(lf_context* ctx, ArenaCursor& cur, const TrnArgs& a, int 
     return tc::transition_run(ctx, cur, a.act, a.act_dtype, a.rows, a.variance, a.eps, a.w, a.residual ? a.act : nullptr, a.out);
   if (precision == LF_PRECISION_BF16 && hgemm_supported(a.w))
     return a.act_dtype == LF_DTYPE_BF16 ? trn_half<bf16>(ctx, cur, a) : trn_half<float>(ctx, cur, a);
-  if (a.act_dtype == LF_DTYPE_BF16) trn_f32<bf16>(ctx, cur, a); else trn_f32<float>(ctx, cur, a);
-  return LF_OK;
+  return a.act_dtype == LF_DTYPE_BF16 ? trn_f32<bf16>(ctx, cur, a) : trn_f32<float>(ctx, cur, a);
 }
 
 // Runs `body` twice: a dry pass that sizes the arena, then the real pass.
@@ -1517,8 +1662,7 @@ lf_status lf_outer_product_mean_run(lf_context* ctx, const lf_opm_desc* d, lf_re
       const op16* wout = gemm_operand(w, 1);
       op16* proj16 = cur.take<op16>((int64_t)ni * N * cz);
       float* counts = cur.take<float>((int64_t)N * N);
-      LAUNCH(ctx, cur, (simt::layer_norm_kernel<float, op16>), lf_ceil_div(rows, 8), 256, 0, msa, rows, cm, f[OPM_LN_G], f[OPM_LN_B],
-             d->layer_norm_epsilon, d->variance, 0, 1, 1, nrm16);
+      layer_norm<float, rows::LN_HALF>(ctx, cur, msa, rows, cm, f[OPM_LN_G], f[OPM_LN_B], d->layer_norm_epsilon, d->variance, 0, 1, 1, nrm16);
       LF_TRY(hgemm(ctx, cur, nrm16, wlr, lr16, rows, 2 * c, cm));
       LAUNCH(ctx, cur, simt::opm_split_half_kernel, lf_ceil_div(rows * c, 256), 256, 0, lr16, f[OPM_BL], f[OPM_BR], mask, rows, c, left16, right16);
       LAUNCH(ctx, cur, simt::opm_counts_kernel, lf_ceil_div((int64_t)((N + 3) / 4) * N, 256), 256, 0, mask, S, N, counts);
@@ -1536,8 +1680,7 @@ lf_status lf_outer_product_mean_run(lf_context* ctx, const lf_opm_desc* d, lf_re
       st.flush();
       return LF_OK;
     }
-    LAUNCH(ctx, cur, (simt::layer_norm_kernel<float>), lf_ceil_div(rows, 8), 256, 0, msa, rows, cm, f[OPM_LN_G], f[OPM_LN_B],
-           d->layer_norm_epsilon, d->variance, 0, 1, 1, nrm);
+    layer_norm<float, rows::LN_F32>(ctx, cur, msa, rows, cm, f[OPM_LN_G], f[OPM_LN_B], d->layer_norm_epsilon, d->variance, 0, 1, 1, nrm);
     sgemm(ctx, cur, false, false, 0, (int)rows, c, cm, nrm, cm, 0, f[OPM_WL], c, 0, left, c, 0, f[OPM_BL], 0, 1);
     sgemm(ctx, cur, false, false, 0, (int)rows, c, cm, nrm, cm, 0, f[OPM_WR], c, 0, right, c, 0, f[OPM_BR], 0, 1);
     if (tc_outer) LAUNCH(ctx, cur, simt::mask_rows_half_kernel, lf_ceil_div(rows * c, 256), 256, 0, left, right, mask, rows, c, left16, right16);
@@ -1600,7 +1743,7 @@ lf_status lf_single_attention_run(lf_context* ctx, const lf_single_attention_des
     a.mask = (const float*)st.in(d->seq_mask, (size_t)n * 4);
     a.pair = st.in(d->pair, (size_t)n * n * d->pair_channels * dtype_size(a.pair_dtype));
     a.out = st.out(d->out, (size_t)n * d->channels * 4);
-    att_f32<float>(ctx, cur, a);
+    LF_TRY(att_f32<float>(ctx, cur, a));
     st.flush();
     return LF_OK;
   });
@@ -1629,13 +1772,10 @@ lf_status lf_msa_attention_run(lf_context* ctx, const lf_msa_attention_desc* d, 
     a.mask_mode = 0; a.clamp = 0; a.eps = 1e-5f; a.pair_eps = 1e-5f; a.act_dtype = LF_DTYPE_F32; a.w = w;
     a.tc_pair_bias = d->precision == LF_PRECISION_BF16 ? 1 : 0;
     a.act = st.in(d->msa, R * d->channels * 4);
-    const float* msa_mask = (const float*)st.in(d->msa_mask, R * 4);
-    float* key_mask = cur.take<float>(R);
-    LAUNCH(ctx, cur, simt::msa_key_mask_kernel, lf_ceil_div(n, 128), 128, 0, msa_mask, S, n, key_mask);
-    a.mask = key_mask;
+    a.mask = (const float*)st.in(d->msa_mask, R * 4);
     a.pair = st.in(d->pair, (size_t)n * n * d->pair_channels * dtype_size(a.pair_dtype));
     a.out = st.out(d->out, R * d->channels * 4);
-    att_f32<float>(ctx, cur, a);
+    LF_TRY(msa_average(ctx, cur, a));
     st.flush();
     return LF_OK;
   });
@@ -1645,30 +1785,34 @@ lf_status lf_msa_attention_run(lf_context* ctx, const lf_msa_attention_desc* d, 
 
 namespace {
 template <typename T>
-void global_attention(lf_context* ctx, ArenaCursor& cur, const lf_global_attention_desc* d, const void* act, const float* mask,
-                      void* out) {
+lf_status global_attention(lf_context* ctx, ArenaCursor& cur, const lf_global_attention_desc* d, const void* act, const float* mask, void* out) {
   const lf_weights* w = d->weights;
-  lf_weights_await(ctx, w);
   const auto& f = w->f;
-  const int S = d->sequences, n = d->length, c = d->channels, H = d->heads, hd = w->dims.head_dim, HD = H * hd, wide = 2 * hd + HD;
+  const int S = d->sequences, n = d->length, c = d->channels, H = d->heads, hd = w->dims.head_dim, HD = H * hd, wide = 2 * hd + HD, ld = (wide + 3) / 4 * 4;
   const int64_t R = (int64_t)S * n;
-  float* nrm = cur.take<float>(R * c);
-  float* kvg = cur.take<float>(R * wide);
+  const SplitMatrix* g = nullptr;
+  SplitMatrix none[3];
+  if (cur.dry) g = none; else LF_TRY(f32_operands(ctx, w, &g));
+  const SplitMatrix nrm = take_terms(cur, R, c), gated = take_terms(cur, R, HD);
+  float* kvg = cur.take<float>(R * ld);
+  float* sums = cur.take<float>((int64_t)n * (c + 1));
   float* q = cur.take<float>((int64_t)n * HD);
   float* attended = cur.take<float>((int64_t)n * HD);
-  float* gated = cur.take<float>(R * HD);
-  LAUNCH(ctx, cur, (simt::layer_norm_kernel<T>), lf_ceil_div(R, 8), 256, 0, (const T*)act, R, c, f[GLB_LN_G], f[GLB_LN_B],
-         d->epsilon, d->variance, 0, 1, 1, nrm);
-  sgemm(ctx, cur, false, false, simt::EPI_SIGMOID_FROM_COL, (int)R, wide, c, nrm, c, 0, f[GLB_W3], wide, 0, kvg, wide, 0, f[GLB_B3],
-        2 * hd, 1);
-  LAUNCH(ctx, cur, simt::global_query_kernel, n, 128, (size_t)c * sizeof(float), nrm, mask, S, n, c, HD, 1.0f / sqrtf((float)hd),
-         f[GLB_WQ], q);
-  LAUNCH(ctx, cur, simt::global_attend_kernel, dim3(n, H), 64, 0, q, kvg, wide, mask, S, n, H, hd, attended);
-  LAUNCH(ctx, cur, simt::global_gate_kernel, lf_ceil_div(R * HD, 256), 256, 0, kvg, wide, 2 * hd, attended, R, n, HD, gated);
-  float* proj = nrm;   // the normalised input is dead
-  sgemm(ctx, cur, false, false, 0, (int)R, c, HD, gated, HD, 0, f[GLB_WO], c, 0, proj, c, 0, f[GLB_BO], 0, 1);
-  LAUNCH(ctx, cur, (simt::finish_kernel<T>), lf_ceil_div(R * c, 256), 256, 0, proj, (const float*)nullptr,
-         d->residual ? (const T*)act : (const T*)nullptr, R, c, 0, 1, 1, (T*)out);
+  float* proj = cur.take<float>(R * c);
+  layer_norm<T, rows::LN_TERMS>(ctx, cur, act, R, c, f[GLB_LN_G], f[GLB_LN_B], d->epsilon, d->variance, 0, 1, 1, (void*)nrm.p, nrm.term_stride);
+  LF_TRY(tc::gemm_f32(ctx, cur, 0, nrm, g[0], (int)R, wide, c, 1, {kvg, nullptr, ld, 0, 0, f[GLB_B3], wide, 0, 2 * hd, wide}));
+  const bool wide_rows = c > 512;      // more channels than a lane keeps: the sums of the normalised rows, from their terms
+  if (wide_rows) LAUNCH(ctx, cur, rows::global_mean_terms_kernel, n, 512, 0, nrm.p, nrm.ld, nrm.term_stride, mask, S, n, c, sums);
+  else
+    LAUNCH(ctx, cur, (rows::global_mean_kernel<T>), n, 512, (size_t)16 * (c + 1) * sizeof(float), (const T*)act, mask, S, n, c, d->epsilon, d->variance, sums);
+  LAUNCH(ctx, cur, rows::global_query_kernel, n, 128, (size_t)c * sizeof(float), sums, wide_rows ? nullptr : f[GLB_LN_G], f[GLB_LN_B], c, HD, 1.0f / sqrtf((float)hd), f[GLB_WQ], q);
+  if (hd <= 8) LAUNCH(ctx, cur, rows::global_attend_kernel<8>, dim3(n, lf_ceil_div(H, 2)), 256, 0, q, kvg, (int64_t)ld, mask, S, n, H, hd, attended);
+  else LAUNCH(ctx, cur, rows::global_attend_kernel<32>, dim3(n, lf_ceil_div(H, 2)), 256, 0, q, kvg, (int64_t)ld, mask, S, n, H, hd, attended);
+  LAUNCH(ctx, cur, rows::global_gate_kernel, lf_ceil_div(R * (gated.ld / 2), 256), 256, 0, kvg, (int64_t)ld, 2 * hd, attended, R, n, HD, (int)gated.ld,
+         (bf16*)gated.p, gated.term_stride);
+  LF_TRY(tc::gemm_f32(ctx, cur, 0, gated, g[1], (int)R, c, HD, 1, {proj, nullptr, c, 0, 0, f[GLB_BO], c, 0, 0, 0}));
+  finish<T>(ctx, cur, proj, nullptr, d->residual ? act : nullptr, R, c, 0, 1, 1, out);
+  return LF_OK;
 }
 }  // namespace
 
@@ -1693,8 +1837,8 @@ lf_status lf_global_column_attention_run(lf_context* ctx, const lf_global_attent
     const void* act = st.in(d->activations, R * d->channels * es);
     const float* mask = (const float*)st.in(d->mask, R * sizeof(float));
     void* out = st.out(d->out, R * d->channels * es);
-    if (d->act_dtype == LF_DTYPE_BF16) global_attention<bf16>(ctx, cur, d, act, mask, out);
-    else global_attention<float>(ctx, cur, d, act, mask, out);
+    if (d->act_dtype == LF_DTYPE_BF16) LF_TRY(global_attention<bf16>(ctx, cur, d, act, mask, out));
+    else LF_TRY(global_attention<float>(ctx, cur, d, act, mask, out));
     st.flush();
     return LF_OK;
   });

@@ -9,6 +9,7 @@
 #include <cstdarg>
 #include <cstdint>
 #include <cstdio>
+#include <mutex>
 #include <string>
 #include <vector>
 
@@ -67,6 +68,27 @@ enum { OPM_LN_G, OPM_LN_B, OPM_WL, OPM_BL, OPM_WR, OPM_BR, OPM_WOUT, OPM_BOUT, O
 // global column attention: W3 = (key | value | gate) columns, B3 their biases (zero but for the gate)
 enum { GLB_LN_G, GLB_LN_B, GLB_WQ, GLB_W3, GLB_B3, GLB_WO, GLB_BO, GLB_COUNT };
 
+// A float32 matrix as three bf16 terms that add up to it: term t at p + t * term_stride, rows of ld, batch entries batch_stride
+// apart (strides in elements, multiples of 8).
+struct SplitMatrix {
+  const bf16* p = nullptr;
+  int64_t ld = 0, batch_stride = 0, term_stride = 0;
+};
+
+// Operands of the float32 GEMM, [n_out][k] terms: made at the first float32 call that uses the weights, kept with them.
+//   triangle: fused projection, output projection, output gate; attention: fused projection (with the pair bias columns when
+//   the bias comes from the normalised input; values and gate alone for the MSA averaging), output projection;
+//   transition: both projections; global attention: key | value | gate, output projection
+struct lf_f32_operands {
+  std::mutex mutex;
+  bool made = false;
+  lf_context* ctx = nullptr;
+  void* block = nullptr;
+  size_t block_bytes = 0;
+  cudaEvent_t ready = nullptr;
+  SplitMatrix g[3];
+};
+
 // Canonical device-resident weights.  Every linear is stored (in,out) row-major
 // float32 in `f[...]`; tensor-core kernels keep extra fp16 repacks (swizzled operand images) in `h[...]`.
 struct lf_weights {
@@ -79,6 +101,7 @@ struct lf_weights {
   int device = 0;
   void* block = nullptr;     // the one device allocation behind all of them (weight_block_take)
   size_t block_bytes = 0;
+  lf_f32_operands* f32 = nullptr;
   cudaEvent_t ready = nullptr;   // recorded on the creating context's stream when they have been prepared
   bool has_gate_bias = false, has_out_bias = false, has_pair_norm = false, has_pair_proj = false;
 };

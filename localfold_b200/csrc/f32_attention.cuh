@@ -69,6 +69,8 @@ struct AttentionShape {
   int batch, Q, heads, d;
   int transpose, mask_mode, clamp;      // mask_mode 0: logit += 1e9 (m - 1); 1: logit += m > 0 ? 0 : -1e9
   float scale;
+  int64_t ld;                           // floats from one row of q | k | v | gate to the next (a multiple of 4)
+  int64_t ldo, term_stride;             // output rows and terms, in bf16 elements
   int wb, wq;                           // warps of a block: wb batch rows x wq groups of 16 queries, wq >= D / 8
 };
 
@@ -78,9 +80,9 @@ __host__ __device__ constexpr size_t attention_smem(int D, int wb) {
   return (size_t)2 * wb * (2 * 3 * AT_KT * at_pitch(D) * 2 + AT_KT * 4);
 }
 
-//   qkvg: [rows][4 * HD] = (q | k | v | sigmoid(gate)) in logical row order
+//   qkvg: [rows][ld] = (q | k | v | sigmoid(gate) | ...) in logical row order
 //   bias: [H][Q][Q] or null; mask: indexed b * Q + j, or j * batch + b when transpose
-//   out:  [rows][HD] = softmax(.) v * gate
+//   out:  [3][rows][ldo] = softmax(.) v * gate as terms, the operand of the output projection
 // A warp owns 16 queries of one (batch row, head); Q and the running output stay in registers in the tensor core's
 // fragment layout, and probabilities become the A operand of P V without leaving them.  The warps of a block share K and
 // V tiles of 32 keys, which a thread fetches a tile ahead and splits once.  A row's reference is the maximum of its first
@@ -94,13 +96,14 @@ __host__ __device__ constexpr size_t attention_smem(int D, int wb) {
 template <int D, bool BIAS>
 __global__ void __launch_bounds__(256, D <= 16 || D == 32 ? 2 : 1)
 attention_kernel(const float* __restrict__ qkvg, const float* __restrict__ bias, const float* __restrict__ mask,
-                 const AttentionShape s, float* __restrict__ out) {
+                 const AttentionShape s, __nv_bfloat16* __restrict__ out) {
   constexpr int KT = AT_KT, PITCH = at_pitch(D), NK = D / 16, TAIL = (D / 8) & 1, ND = D / 8;
   constexpr int PLANE = KT * PITCH;                 // bf16 elements of one term of one tile
   extern __shared__ uint4 at_sm[];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, g = lane >> 2, t = lane & 3;
   const int wb = warp / s.wq, wq = warp % s.wq;
-  const int d = s.d, Q = s.Q, HD = s.heads * d, ld = 4 * HD;
+  const int d = s.d, Q = s.Q, HD = s.heads * d;
+  const int64_t ld = s.ld;
   const int h = blockIdx.z, b0 = blockIdx.y * s.wb, b = b0 + wb;
   const int q0 = (blockIdx.x * s.wq + wq) * 16;
   // [2 buffers][wb][K: 3 terms | V: 3 terms][KT][PITCH], then [2][wb][KT] mask terms
@@ -172,7 +175,7 @@ attention_kernel(const float* __restrict__ qkvg, const float* __restrict__ bias,
   fetch(0);
 
   // ---- Q as A fragments of its three terms ----
-  uint32_t qa[3][NK > 0 ? NK : 1][4], qt[3][2];      // qt: the last 8 channels of an odd count of groups
+  uint32_t qa[3][NK > 0 ? NK : 1][4], qt[3][2];      // qt: the last 8 channels of an odd number of them
   const int row0 = q0 + g, row1 = q0 + g + 8;
   auto q_pair = [&](int row, int e, uint32_t (&term)[3]) {
     float x = 0.f, y = 0.f;
@@ -252,29 +255,33 @@ attention_kernel(const float* __restrict__ qkvg, const float* __restrict__ bias,
       uint32_t kb[3][2][4];
       // matrices (keys 0-7, k 0-7), (keys 0-7, k 8-15), (keys 8-15, k 0-7), (keys 8-15, k 8-15) of each 16 keys
       const __nv_bfloat16* base = k_s + ((lane & 7) + (lane >> 4) * 8) * PITCH + ((lane >> 3) & 1) * 8;
+      // the term products below the leading one first, over all channels; the leading ones last
 #pragma unroll
-      for (int kk = 0; kk < NK; ++kk) {
+      for (int pass = 2; pass >= 0; pass -= 2) {
 #pragma unroll
-        for (int i = 0; i < 3; ++i)
+        for (int kk = 0; kk < NK; ++kk) {
 #pragma unroll
-          for (int grp = 0; grp < 2; ++grp) ldmatrix4<false>(kb[i][grp], base + i * PLANE + grp * 16 * PITCH + kk * 16);
+          for (int i = 0; i <= pass; ++i)
 #pragma unroll
-        for (int order = 2; order >= 0; --order)        // terms i and order - i
+            for (int grp = 0; grp < 2; ++grp) ldmatrix4<false>(kb[i][grp], base + i * PLANE + grp * 16 * PITCH + kk * 16);
 #pragma unroll
-          for (int i = 0; i <= order; ++i)
+          for (int order = pass; order >= (pass ? 1 : 0); --order)        // terms i and order - i
 #pragma unroll
-            for (int n = 0; n < 4; ++n) mma16(l[n], qa[i][kk], kb[order - i][n >> 1][(n & 1) * 2], kb[order - i][n >> 1][(n & 1) * 2 + 1]);
-      }
-      if (TAIL) {
-        // matrices: keys 0-7, 8-15, 16-23, 24-31 of the last eight channels
+            for (int i = 0; i <= order; ++i)
 #pragma unroll
-        for (int i = 0; i < 3; ++i) ldmatrix4<false>(kb[i][0], k_s + i * PLANE + lane * PITCH + NK * 16);
+              for (int n = 0; n < 4; ++n) mma16(l[n], qa[i][kk], kb[order - i][n >> 1][(n & 1) * 2], kb[order - i][n >> 1][(n & 1) * 2 + 1]);
+        }
+        if (TAIL) {
+          // matrices: keys 0-7, 8-15, 16-23, 24-31 of the last eight channels
 #pragma unroll
-        for (int order = 2; order >= 0; --order)
+          for (int i = 0; i <= pass; ++i) ldmatrix4<false>(kb[i][0], k_s + i * PLANE + lane * PITCH + NK * 16);
 #pragma unroll
-          for (int i = 0; i <= order; ++i)
+          for (int order = pass; order >= (pass ? 1 : 0); --order)
 #pragma unroll
-            for (int n = 0; n < 4; ++n) mma8(l[n], qt[i][0], qt[i][1], kb[order - i][0][n]);
+            for (int i = 0; i <= order; ++i)
+#pragma unroll
+              for (int n = 0; n < 4; ++n) mma8(l[n], qt[i][0], qt[i][1], kb[order - i][0][n]);
+        }
       }
     }
     // ---- logits ----
@@ -384,14 +391,23 @@ attention_kernel(const float* __restrict__ qkvg, const float* __restrict__ bias,
     if (row >= Q) continue;
     const float inv = 1.0f / sum[r];
     const float* gate = qkvg + ((int64_t)b * Q + row) * ld + 3 * HD + h * d;
-    float* dst = out + ((int64_t)b * Q + row) * HD + h * d;
+    __nv_bfloat16* dst = out + ((int64_t)b * Q + row) * s.ldo + h * d;
 #pragma unroll
-    for (int n = 0; n < ND; ++n)
+    for (int n = 0; n < ND; ++n) {
+      const int c = n * 8 + 2 * t;
+      if (c >= d) continue;
+      uint32_t term[3];
+      split3(o[n][2 * r] * inv * gate[c], c + 1 < d ? o[n][2 * r + 1] * inv * gate[c + 1] : 0.f, term);
 #pragma unroll
-      for (int e = 0; e < 2; ++e) {
-        const int c = n * 8 + 2 * t + e;
-        if (c < d) dst[c] = o[n][2 * r + e] * inv * gate[c];
+      for (int i = 0; i < 3; ++i) {
+        __nv_bfloat16* cell = dst + i * s.term_stride + c;
+        if (!(d & 1)) *reinterpret_cast<uint32_t*>(cell) = term[i];
+        else {
+          *cell = __ushort_as_bfloat16((unsigned short)(term[i] & 0xffffu));
+          if (c + 1 < d) cell[1] = __ushort_as_bfloat16((unsigned short)(term[i] >> 16));
+        }
       }
+    }
   }
 }
 

@@ -1,0 +1,282 @@
+// Float32 GEMM on tcgen05: operands taken apart into three bf16 terms (8 + 8 + 8 significand bits, nothing is lost), a
+// product of two values into the six term products above 2^-24, float32 accumulation.
+#include <cuda.h>
+
+#include "tc05.cuh"
+#include "tc_kernels.cuh"
+
+namespace tc {
+
+using namespace tc05;
+
+// One 128 x 128 output tile of one batch entry per work item.  A k block of 64 holds the three terms of both operands
+// (96 KiB a stage, two stages); the leading product goes into one TMEM accumulator and the five others into a second
+// one (2 x 128 columns, double-buffered), so the tensor core's own additions, which truncate, act on the correction apart
+// from the sum.  The epilogue adds the two and keeps the sum of the k blocks in its registers, in round-to-nearest, while the
+// accumulators start afresh: errors against float64 are at or below those of a float32 FMA chain (1.9e-7 against
+// 3.1e-7 to 4.8e-7 for the triangle update at 203 to 700; with all of k in TMEM 1.3e-6 for a transition of 384 channels).
+// Warp roles: 0 = TMA producer, 1 = MMA issuer (owns TMEM), 2..9 = epilogue (lane quadrant = warp % 4, half of the columns).
+// Bound by the operands' way from L2 into shared memory (96 KiB per 768 cycles of tensor work).  41 209 x 512 x 128: 28
+// TFLOP/s with 4 x 4 results a thread on the FMA pipe.
+constexpr int G3_BM = 128, G3_BN = 128, G3_BK = 64, G3_STAGES = 2, G3_EPI = 8;
+constexpr int G3_PLANE = G3_BM * G3_BK * 2;            // 16 KiB: one term of one operand
+constexpr int G3_STAGE = 6 * G3_PLANE;
+constexpr int G3_OUT = 4096;                           // per epilogue warp: 32 rows x 32 columns of float32
+constexpr int G3_SMEM = G3_STAGES * G3_STAGE + G3_EPI * G3_OUT + 256 + 1024;
+constexpr int G3_THREADS = 64 + 32 * G3_EPI;
+constexpr int G3_CHUNK = 1;                            // k blocks per accumulation in TMEM
+
+struct Gemm3Params {
+  int m, n, k, batch;
+  float* out;                  // [batch][m][ldo] float32, or null
+  bf16* terms;                 // ... or its three terms, [3][batch][m][ldo]
+  int64_t ldo, batch_stride, term_stride;
+  const float* bias;           // or null
+  int bias_n, relu, sigmoid_col0, sigmoid_col1;
+  Status* status;
+};
+
+// kind::f16 with bf16 operands
+__host__ __device__ constexpr uint32_t make_idesc_bf16(int M, int N, int major) {
+  return make_idesc_f16(M, N, major, major) | (1u << 7) | (1u << 10);
+}
+
+template <int MAJOR>      // 0: k contiguous in both operands; 1: the row index contiguous in both
+__global__ void __launch_bounds__(G3_THREADS, 1)
+gemm3_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant__ CUtensorMap mapB, const Gemm3Params p) {
+  extern __shared__ uint8_t smem_raw[];
+  uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
+  uint8_t* out_stage = smem + G3_STAGES * G3_STAGE;
+  uint64_t* bars = reinterpret_cast<uint64_t*>(out_stage + G3_EPI * G3_OUT);
+  uint64_t* full = bars;                       // [STAGES]
+  uint64_t* empty = bars + G3_STAGES;          // [STAGES]
+  uint64_t* tmem_full = empty + G3_STAGES;     // [2]
+  uint64_t* tmem_empty = tmem_full + 2;        // [2]
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(tmem_empty + 2);
+  volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
+
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int tiles_m = (p.m + G3_BM - 1) / G3_BM, tiles_n = (p.n + G3_BN - 1) / G3_BN, per = tiles_m * tiles_n;
+  const int64_t total = (int64_t)p.batch * per;
+  const int kblocks = (p.k + G3_BK - 1) / G3_BK;
+
+  if (threadIdx.x == 0) {
+    for (int s = 0; s < G3_STAGES; ++s) { mbar_init(&full[s], 1); mbar_init(&empty[s], 1); }
+    for (int b = 0; b < 2; ++b) { mbar_init(&tmem_full[b], 1); mbar_init(&tmem_empty[b], G3_EPI); }
+    *abort_flag = 0;
+    fence_barrier_init();
+  }
+  if (warp == 1) { tmem_alloc(tmem_slot, 512); tmem_relinquish(); }
+  tc_fence_before();
+  __syncthreads();
+  tc_fence_after();
+  const uint32_t tmem_base = *tmem_slot;
+
+  if (warp == 0) {
+    if (lane == 0) {
+      prefetch_tensormap(&mapA);
+      prefetch_tensormap(&mapB);
+      int stage = 0; uint32_t phase = 0;
+      bool ok = true;
+      for (int64_t t = blockIdx.x; t < total && ok; t += gridDim.x) {
+        const int h = (int)(t / per), rem = (int)(t % per), mi = rem / tiles_n, nj = rem % tiles_n;
+        for (int kb = 0; kb < kblocks; ++kb) {
+          if (!mbar_wait(&empty[stage], phase ^ 1, abort_flag, p.status, 101)) { ok = false; break; }
+          uint8_t* sA = smem + stage * G3_STAGE;
+          uint8_t* sB = sA + 3 * G3_PLANE;
+          mbar_expect_tx(&full[stage], G3_STAGE);
+          if (MAJOR == 0) {      // [term][128 rows][64 k]
+            tma_load_4d(sA, &mapA, &full[stage], kb * G3_BK, mi * G3_BM, h, 0);
+            tma_load_4d(sB, &mapB, &full[stage], kb * G3_BK, nj * G3_BN, h, 0);
+          } else {               // per 64 rows: [term][64 k][64 rows]
+#pragma unroll
+            for (int q = 0; q < 2; ++q) {
+              tma_load_4d(sA + q * 3 * (G3_PLANE / 2), &mapA, &full[stage], mi * G3_BM + q * 64, kb * G3_BK, h, 0);
+              tma_load_4d(sB + q * 3 * (G3_PLANE / 2), &mapB, &full[stage], nj * G3_BN + q * 64, kb * G3_BK, h, 0);
+            }
+          }
+          if (++stage == G3_STAGES) { stage = 0; phase ^= 1; }
+        }
+      }
+    }
+  } else if (warp == 1) {
+    if (lane == 0) {
+      constexpr uint32_t idesc = make_idesc_bf16(G3_BM, G3_BN, MAJOR);
+      int stage = 0; uint32_t phase = 0;
+      uint32_t it = 0;
+      bool ok = true;
+      for (int64_t t = blockIdx.x; t < total && ok; t += gridDim.x) {
+        for (int kb = 0; kb < kblocks; ++kb) {
+          const uint32_t d = tmem_base + (it & 1) * 256;
+          const int kc = kb % G3_CHUNK;
+          if (kc == 0) {
+            if (!mbar_wait(&tmem_empty[it & 1], ((it >> 1) & 1) ^ 1, abort_flag, p.status, 102)) { ok = false; break; }
+            tc_fence_after();
+          }
+          if (!mbar_wait(&full[stage], phase, abort_flag, p.status, 103)) { ok = false; break; }
+          tc_fence_after();
+          const uint32_t a0 = smem_u32(smem + stage * G3_STAGE), b0 = a0 + 3 * G3_PLANE;
+#pragma unroll
+          for (int kk = 0; kk < G3_BK / 16; ++kk) {
+            // operand descriptor of one term
+            auto desc = [&](uint32_t base, int term) {
+              return MAJOR == 0 ? make_smem_desc(base + term * G3_PLANE + kk * 32, 16, 1024)
+                                : make_smem_desc(base + term * (G3_PLANE / 2) + kk * 2048, 3 * (G3_PLANE / 2), 1024);
+            };
+            const uint32_t more = (kc | kk) != 0 ? 1u : 0u;
+            umma_f16(d + 128, desc(a0, 2), desc(b0, 0), idesc, more);
+            umma_f16(d + 128, desc(a0, 1), desc(b0, 1), idesc, 1u);
+            umma_f16(d + 128, desc(a0, 0), desc(b0, 2), idesc, 1u);
+            umma_f16(d + 128, desc(a0, 1), desc(b0, 0), idesc, 1u);
+            umma_f16(d + 128, desc(a0, 0), desc(b0, 1), idesc, 1u);
+            umma_f16(d, desc(a0, 0), desc(b0, 0), idesc, more);
+          }
+          umma_commit(&empty[stage]);
+          if (++stage == G3_STAGES) { stage = 0; phase ^= 1; }
+          if (kc == G3_CHUNK - 1 || kb == kblocks - 1) { umma_commit(&tmem_full[it & 1]); ++it; }
+        }
+      }
+    }
+  } else {
+    const int q = warp & 3, half = (warp - 2) >> 2;      // TMEM lane quadrant, half of the tile's columns
+    uint8_t* stage = out_stage + (warp - 2) * G3_OUT;
+    const int chunks = (kblocks + G3_CHUNK - 1) / G3_CHUNK;
+    uint32_t it = 0;
+    bool ok = true;
+    for (int64_t t = blockIdx.x; t < total && ok; t += gridDim.x) {
+      const int h = (int)(t / per), rem = (int)(t % per), mi = rem / tiles_n, nj = rem % tiles_n;
+      float acc[64];
+#pragma unroll 1
+      for (int c = 0; c < chunks; ++c, ++it) {
+        if (!mbar_wait(&tmem_full[it & 1], (it >> 1) & 1, abort_flag, p.status, 104)) { ok = false; break; }
+        tc_fence_after();
+        const uint32_t d = tmem_base + ((uint32_t)(q * 32) << 16) + (it & 1) * 256 + half * 64;
+#pragma unroll
+        for (int c16 = 0; c16 < 4; ++c16) {
+          uint32_t lead[16], rest[16];
+          tmem_ld16(d + c16 * 16, lead);
+          tmem_ld16(d + 128 + c16 * 16, rest);
+          tmem_ld_wait();
+#pragma unroll
+          for (int e = 0; e < 16; ++e) {
+            const float v = __uint_as_float(lead[e]) + __uint_as_float(rest[e]);
+            acc[c16 * 16 + e] = c ? acc[c16 * 16 + e] + v : v;
+          }
+        }
+        tc_fence_before();
+        __syncwarp();
+        if (lane == 0) mbar_arrive(&tmem_empty[it & 1]);
+      }
+      if (!ok) break;
+      const int row0 = mi * G3_BM + q * 32;
+#pragma unroll
+      for (int ch = 0; ch < 2; ++ch) {                   // 32 columns at a time
+        const int col0 = nj * G3_BN + half * 64 + ch * 32;
+        float* v = acc + ch * 32;
+        if (p.bias) {
+#pragma unroll
+          for (int e = 0; e < 32; ++e) v[e] += col0 + e < p.bias_n ? __ldg(p.bias + col0 + e) : 0.f;
+        }
+        if (p.relu) {
+#pragma unroll
+          for (int e = 0; e < 32; ++e) v[e] = fmaxf(v[e], 0.f);
+        }
+        if (col0 + 32 > p.sigmoid_col0 && col0 < p.sigmoid_col1) {
+#pragma unroll
+          for (int e = 0; e < 32; ++e)
+            if (col0 + e >= p.sigmoid_col0 && col0 + e < p.sigmoid_col1) v[e] = 1.0f / (1.0f + expf(-v[e]));
+        }
+        if (p.out) {
+          // the warp's 32 x 32 values turned round in shared memory (16-byte pieces swizzled by row): whole 128-byte runs leave
+#pragma unroll
+          for (int k4 = 0; k4 < 8; ++k4)
+            *reinterpret_cast<float4*>(stage + lane * 128 + ((k4 ^ (lane & 7)) << 4)) = make_float4(v[k4 * 4], v[k4 * 4 + 1], v[k4 * 4 + 2], v[k4 * 4 + 3]);
+          __syncwarp();
+#pragma unroll
+          for (int i = 0; i < 8; ++i) {
+            const int r = i * 4 + (lane >> 3), piece = lane & 7, col = col0 + piece * 4;
+            const float4 x = *reinterpret_cast<const float4*>(stage + r * 128 + ((piece ^ (r & 7)) << 4));
+            if (row0 + r < p.m) {
+              float* dst = p.out + (int64_t)h * p.batch_stride + (int64_t)(row0 + r) * p.ldo + col;
+              if (col + 4 <= p.n && (p.ldo & 3) == 0) *reinterpret_cast<float4*>(dst) = x;
+              else {
+                if (col < p.n) dst[0] = x.x;
+                if (col + 1 < p.n) dst[1] = x.y;
+                if (col + 2 < p.n) dst[2] = x.z;
+                if (col + 3 < p.n) dst[3] = x.w;
+              }
+            }
+          }
+          __syncwarp();
+        } else {
+          // ... or their terms, 64-byte runs a row and term (ldo a multiple of 8)
+#pragma unroll 1
+          for (int term = 0; term < 3; ++term) {
+            uint32_t w[16];
+#pragma unroll
+            for (int e = 0; e < 16; ++e) {
+              const __nv_bfloat162 b2 = __floats2bfloat162_rn(v[2 * e], v[2 * e + 1]);
+              w[e] = *reinterpret_cast<const uint32_t*>(&b2);
+              v[2 * e] -= __low2float(b2);
+              v[2 * e + 1] -= __high2float(b2);
+            }
+#pragma unroll
+            for (int k4 = 0; k4 < 4; ++k4)
+              *reinterpret_cast<uint4*>(stage + lane * 64 + ((k4 ^ ((lane >> 1) & 3)) << 4)) = make_uint4(w[k4 * 4], w[k4 * 4 + 1], w[k4 * 4 + 2], w[k4 * 4 + 3]);
+            __syncwarp();
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+              const int r = i * 8 + (lane >> 2), piece = lane & 3, col = col0 + piece * 8;
+              const uint4 x = *reinterpret_cast<const uint4*>(stage + r * 64 + ((piece ^ ((r >> 1) & 3)) << 4));
+              if (row0 + r < p.m && col < p.ldo)
+                *reinterpret_cast<uint4*>(p.terms + term * p.term_stride + (int64_t)h * p.batch_stride + (int64_t)(row0 + r) * p.ldo + col) = x;
+            }
+            __syncwarp();
+          }
+        }
+      }
+    }
+  }
+
+  tc_fence_before();
+  __syncthreads();
+  if (*abort_flag) drain_after_abort();
+  if (warp == 1) { tc_fence_after(); tmem_dealloc(tmem_base, 512); }
+}
+
+void configure_gemm3() {
+  cudaFuncSetAttribute(gemm3_kernel<0>, cudaFuncAttributeMaxDynamicSharedMemorySize, G3_SMEM);
+  cudaFuncSetAttribute(gemm3_kernel<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, G3_SMEM);
+}
+
+lf_status make_map_terms(lf_context* ctx, CUtensorMap* map, const SplitMatrix& a, uint64_t d0, uint64_t d1, uint64_t batch, uint32_t b1);
+
+lf_status gemm_f32(lf_context* ctx, ArenaCursor& cur, int major, const SplitMatrix& a, const SplitMatrix& b, int m, int n, int k, int batch,
+                   const Gemm3Out& o) {
+  if (cur.dry) return LF_OK;
+  if (a.ld % 8 || b.ld % 8 || a.batch_stride % 8 || b.batch_stride % 8 || a.term_stride % 8 || b.term_stride % 8 || (o.terms && o.ld % 8))
+    return lf_fail(ctx, LF_ERR_ARGUMENT, "split operands need strides of whole groups of eight");
+  CUtensorMap ma, mb;
+  if (major == 0) {
+    LF_TRY(make_map_terms(ctx, &ma, a, k, m, batch, G3_BM));
+    LF_TRY(make_map_terms(ctx, &mb, b, k, n, batch, G3_BN));
+  } else {
+    LF_TRY(make_map_terms(ctx, &ma, a, m, k, batch, G3_BK));
+    LF_TRY(make_map_terms(ctx, &mb, b, n, k, batch, G3_BK));
+  }
+  Gemm3Params p{};
+  p.m = m; p.n = n; p.k = k; p.batch = batch;
+  p.out = o.out; p.terms = o.terms; p.ldo = o.ld; p.batch_stride = o.batch_stride; p.term_stride = o.term_stride;
+  p.bias = o.bias; p.bias_n = o.bias_n; p.relu = o.relu; p.sigmoid_col0 = o.sigmoid_col0; p.sigmoid_col1 = o.sigmoid_col1;
+  p.status = (Status*)ctx->tc_status;
+  const int64_t tiles = (int64_t)batch * ((m + G3_BM - 1) / G3_BM) * ((n + G3_BN - 1) / G3_BN);
+  const int grid = (int)(tiles < ctx->sm_count ? tiles : ctx->sm_count);
+  lf_prof_begin(ctx, LF_KERNEL_SIMT);
+  if (major == 0) gemm3_kernel<0><<<grid, G3_THREADS, G3_SMEM, ctx->stream>>>(ma, mb, p);
+  else gemm3_kernel<1><<<grid, G3_THREADS, G3_SMEM, ctx->stream>>>(ma, mb, p);
+  lf_prof_end(ctx);
+  ctx->launches++;
+  return LF_OK;
+}
+
+}  // namespace tc

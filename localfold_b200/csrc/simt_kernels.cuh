@@ -202,40 +202,6 @@ __global__ void trimul_gate_kernel(const float* __restrict__ p4, const float* __
   }
 }
 
-// LayerNorm over the hidden channel of a channel-major tensor x[h][i][ld] -> xn[p][h].
-// One block handles 32 pairs; the tile [c][32] sits in shared memory (c <= 512).
-template <typename TIn>
-__global__ void center_norm_kernel(const TIn* __restrict__ x, int64_t pairs, int c, int n, int ld,
-                                   const float* __restrict__ gamma, const float* __restrict__ beta,
-                                   float eps, int variance, float prescale, float* __restrict__ xn) {
-  extern __shared__ float tile[];   // [c][33]
-  int64_t p0 = (int64_t)blockIdx.x * 32;
-  int tx = threadIdx.x & 31, w = threadIdx.x >> 5, nw = blockDim.x >> 5;
-  for (int h = w; h < c; h += nw) {
-    int64_t p = p0 + tx;
-    tile[h * 33 + tx] = p < pairs ? to_f(x[((int64_t)h * n + p / n) * ld + p % n]) * prescale : 0.f;
-  }
-  __syncthreads();
-  // warp w normalises pairs w, w+nw, ...
-  for (int r = w; r < 32; r += nw) {
-    int64_t p = p0 + r;
-    if (p >= pairs) continue;
-    float s = 0.f, ss = 0.f;
-    for (int h = tx; h < c; h += 32) { float v = tile[h * 33 + r]; s += v; ss += v * v; }
-    s = warp_sum(s);
-    float mean = s / c, var;
-    if (variance == 2) { ss = warp_sum(ss); var = ss / c - mean * mean; }
-    else {
-      float acc = 0.f;
-      for (int h = tx; h < c; h += 32) { float d = tile[h * 33 + r] - mean; acc += d * d; }
-      var = warp_sum(acc) / c;
-    }
-    float inv = rsqrtf(var + eps);
-    inv = inv * (1.5f - 0.5f * (var + eps) * inv * inv);
-    for (int h = tx; h < c; h += 32) xn[p * c + h] = (tile[h * 33 + r] - mean) * inv * gamma[h] + beta[h];
-  }
-}
-
 // out[dst(r)][c] = (resid ? resid[dst(r)][c] : 0) + proj[r][c] * (gate ? sigmoid(gate[r][c]) : 1)
 // dst(r) follows the transposed-orientation rule of the attention operator.
 template <typename TAct>
@@ -253,26 +219,6 @@ __global__ void finish_kernel(const float* __restrict__ proj, const float* __res
   if (gate) v *= sigmoidf_(gate[idx]);
   if (resid) v += to_f(resid[dst * ch + c]);
   out[dst * ch + c] = from_f<TAct>(v);
-}
-
-// q, k, v, gate as four fp16 [rows][HD] tensors -> one float32 [rows][4*HD] tensor
-__global__ void unpack_qkvg_kernel(const __half* __restrict__ q, const __half* __restrict__ k, const __half* __restrict__ v,
-                                   const __half* __restrict__ g, int64_t rows, int HD, float* __restrict__ out) {
-  int64_t idx = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (idx >= rows * HD) return;
-  int64_t r = idx / HD;
-  int c = (int)(idx % HD);
-  float* o = out + r * 4 * HD + c;
-  o[0] = __half2float(q[idx]);
-  o[HD] = __half2float(k[idx]);
-  o[2 * HD] = __half2float(v[idx]);
-  o[3 * HD] = __half2float(g[idx]);
-}
-
-template <typename TIn>
-__global__ void to_float_kernel(const TIn* __restrict__ in, int64_t n, float* __restrict__ out) {
-  int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i < n) out[i] = to_f(in[i]);
 }
 
 // ---------------------------------------------------------------------------
@@ -316,83 +262,6 @@ __global__ void pair_bias_kernel(const TIn* __restrict__ pair, int Q, int ch, in
     acc = warp_sum(acc);
     if (lane == 0) out[(int64_t)h * pairs + dst] = acc;
   }
-}
-
-// Global column attention (extra-MSA stack).  Query of a column: the masked mean over the sequences of the
-// normalised rows, projected onto heads x d and scaled.  One block per column; shared memory: c floats.
-__global__ void global_query_kernel(const float* __restrict__ nrm, const float* __restrict__ mask, int S, int n, int c,
-                                    int HD, float scale, const float* __restrict__ wq, float* __restrict__ q) {
-  extern __shared__ float means[];
-  __shared__ float red[32];
-  const int col = blockIdx.x, tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
-  float count = 0.f;
-  for (int s = tid; s < S; s += blockDim.x) count += mask[(int64_t)s * n + col];
-  count = warp_sum(count);
-  if (lane == 0) red[wid] = count;
-  __syncthreads();
-  float total_count = 0.f;
-  for (int w = 0; w < (int)(blockDim.x >> 5); ++w) total_count += red[w];
-  const float denominator = 1e-10f + total_count;
-  for (int ch = tid; ch < c; ch += blockDim.x) {
-    float total = 0.f;
-    for (int s = 0; s < S; ++s) total = fmaf(nrm[((int64_t)s * n + col) * c + ch], mask[(int64_t)s * n + col], total);
-    means[ch] = total / denominator;
-  }
-  __syncthreads();
-  for (int slot = tid; slot < HD; slot += blockDim.x) {
-    float r = 0.f;
-    for (int ch = 0; ch < c; ++ch) r = fmaf(means[ch], wq[(int64_t)ch * HD + slot], r);
-    q[(int64_t)col * HD + slot] = r * scale;
-  }
-}
-
-// Softmax over the sequences of q(column, head) . k(sequence, column) with masked sequences at -1e9, applied to
-// the values: one block of 64 threads per (column, head), each thread an online softmax over its sequences,
-// combined through shared memory.  k at columns 0..d-1 and v at d..2d-1 of rows of `ld` floats; d <= 32.
-__global__ void global_attend_kernel(const float* __restrict__ q, const float* __restrict__ kv, int ld,
-                                     const float* __restrict__ mask, int S, int n, int heads, int d,
-                                     float* __restrict__ attended) {
-  __shared__ float part_max[64], part_den[64], part_acc[64 * 32];
-  const int col = blockIdx.x, h = blockIdx.y, tid = threadIdx.x;
-  float qv[32], acc[32];
-  for (int e = 0; e < d; ++e) { qv[e] = q[((int64_t)col * heads + h) * d + e]; acc[e] = 0.f; }
-  float maximum = -1e30f, den = 0.f;
-  for (int s = tid; s < S; s += 64) {
-    const float* row = kv + ((int64_t)s * n + col) * ld;
-    float logit = 0.f;
-    for (int e = 0; e < d; ++e) logit = fmaf(qv[e], row[e], logit);
-    if (mask[(int64_t)s * n + col] == 0.f) logit = -1e9f;
-    const float next = fmaxf(maximum, logit);
-    const float prev_scale = __expf(maximum - next), weight = __expf(logit - next);
-    den = den * prev_scale + weight;
-    for (int e = 0; e < d; ++e) acc[e] = acc[e] * prev_scale + weight * row[d + e];
-    maximum = next;
-  }
-  part_max[tid] = maximum;
-  part_den[tid] = den;
-  for (int e = 0; e < d; ++e) part_acc[tid * 32 + e] = acc[e];
-  __syncthreads();
-  if (tid < d) {
-    float top = -1e30f;
-    for (int t = 0; t < 64; ++t) top = fmaxf(top, part_max[t]);
-    float dsum = 0.f, num = 0.f;
-    for (int t = 0; t < 64; ++t) {
-      const float w = __expf(part_max[t] - top);
-      dsum += part_den[t] * w;
-      num += part_acc[t * 32 + tid] * w;
-    }
-    attended[((int64_t)col * heads + h) * d + tid] = num / dsum;
-  }
-}
-
-// gated[r][slot] = sigmoid-gate[r][slot] (columns gate0.. of rows of `ld`) * attended[column of r][slot]
-__global__ void global_gate_kernel(const float* __restrict__ kvg, int ld, int gate0, const float* __restrict__ attended,
-                                   int64_t rows, int n, int HD, float* __restrict__ gated) {
-  int64_t idx = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (idx >= rows * HD) return;
-  const int64_t r = idx / HD;
-  const int slot = (int)(idx % HD);
-  gated[idx] = kvg[r * ld + gate0 + slot] * attended[(r % n) * HD + slot];
 }
 
 // Attention activations between the projections and the tensor-core attention core: 128 channels (four
@@ -518,16 +387,6 @@ __global__ void widen_bias_kernel(const __half* __restrict__ in, int heads, int 
   out[idx] = __half2float(in[hq * ld + k]);
 }
 
-// One key mask for every sequence of an MSA: out[s][t] = max over s' of mask[s'][t] (AF3 pair-weighted
-// averaging: a token any sequence covers is a key for all of them).
-__global__ void msa_key_mask_kernel(const float* __restrict__ mask, int sequences, int tokens, float* __restrict__ out) {
-  int t = blockIdx.x * blockDim.x + threadIdx.x;
-  if (t >= tokens) return;
-  float largest = 0.f;
-  for (int s = 0; s < sequences; ++s) largest = fmaxf(largest, mask[(int64_t)s * tokens + t]);
-  for (int s = 0; s < sequences; ++s) out[(int64_t)s * tokens + t] = largest;
-}
-
 // out[i][j][b] = half[i][j][b] + half[j][i][b]: a sum over the two token orders, not a mean.
 __global__ void symmetrise_sum_kernel(const float* __restrict__ half, int tokens, int bins, float* __restrict__ out) {
   int64_t idx = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
@@ -537,18 +396,6 @@ __global__ void symmetrise_sum_kernel(const float* __restrict__ half, int tokens
   int64_t p = idx / bins;
   int i = (int)(p / tokens), j = (int)(p % tokens);
   out[idx] = half[idx] + half[((int64_t)j * tokens + i) * bins + b];
-}
-
-// ---------------------------------------------------------------------------
-// Transition glue: SwiGLU over a [rows][2*inter] tensor, gate half first.
-__global__ void swiglu_kernel(const float* __restrict__ wide, int64_t rows, int inter, float* __restrict__ out) {
-  int64_t idx = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (idx >= rows * inter) return;
-  int64_t r = idx / inter;
-  int i = (int)(idx % inter);
-  float g = wide[r * 2 * inter + i];
-  float v = wide[r * 2 * inter + inter + i];
-  out[idx] = g * sigmoidf_(g) * v;
 }
 
 // ---------------------------------------------------------------------------

@@ -68,6 +68,20 @@ lf_status make_map_tiled_act(lf_context* ctx, CUtensorMap* map, const void* base
   return LF_OK;
 }
 
+// The three bf16 terms of a float32 matrix, seen as (d0 contiguous, d1 rows, batch, term); boxes of 64 x b1 x 1 x all three terms
+lf_status make_map_terms(lf_context* ctx, CUtensorMap* map, const SplitMatrix& a, uint64_t d0, uint64_t d1, uint64_t batch, uint32_t b1) {
+  if (!g_encode) return lf_fail(ctx, LF_ERR_CUDA, "cuTensorMapEncodeTiled is not available from this driver");
+  cuuint64_t dims[4] = {d0, d1, batch, 3};
+  cuuint64_t strides[3] = {(cuuint64_t)a.ld * 2, (cuuint64_t)(a.batch_stride ? a.batch_stride : a.ld * (int64_t)d1) * 2, (cuuint64_t)a.term_stride * 2};
+  cuuint32_t box[4] = {64, b1, 1, 3};
+  cuuint32_t estr[4] = {1, 1, 1, 1};
+  CUresult r = g_encode(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 4, const_cast<bf16*>(a.p), dims, strides, box, estr,
+                        CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+                        CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+  if (r != CUDA_SUCCESS) return lf_fail(ctx, LF_ERR_CUDA, "cuTensorMapEncodeTiled (terms) failed with code %d", (int)r);
+  return LF_OK;
+}
+
 // float32 rows of 128 channels seen as (channel, d1, d2); boxes of 32 channels (one 128-byte swizzled row) x b1 x b2
 lf_status make_map_f32_rows(lf_context* ctx, CUtensorMap* map, const void* base, uint64_t d1, uint64_t d2, uint64_t stride1_bytes,
                             uint64_t stride2_bytes, uint32_t b1, uint32_t b2) {
@@ -429,6 +443,7 @@ void configure_once() {
     configure_ln_gemm();
     configure_attention();
     configure_transition();
+    configure_gemm3();
     cudaGetLastError();
   });
 }

@@ -18,6 +18,22 @@ lf_status prepare_weights(lf_context* ctx, lf_weights* w, WeightCursor& cur);
 // Reads the device status word; LF_ERR_TIMEOUT if a bounded wait expired in a kernel.
 lf_status check_status(lf_context* ctx);
 
+// Float32 GEMM on the tensor cores (f32_gemm.cu), batched: out[b][i][j] = act(sum_k A(b, i, k) B(b, j, k) + bias[j]), both operands
+// as bf16 terms; major 0: k contiguous (A [m][ld], B [n][ld]); major 1: the row index contiguous (A [k][ld], B [k][ld]).
+struct Gemm3Out {
+  float* out;                  // float32 result, or null:
+  bf16* terms;                 // its terms (ld a multiple of 8)
+  int64_t ld, batch_stride, term_stride;
+  const float* bias;           // or null; columns from bias_n on have none
+  int bias_n, relu;
+  int sigmoid_col0, sigmoid_col1;      // columns through a sigmoid (empty range: none)
+};
+void configure_gemm3();
+lf_status gemm_f32(lf_context* ctx, ArenaCursor& cur, int major, const SplitMatrix& a, const SplitMatrix& b, int m, int n, int k, int batch,
+                   const Gemm3Out& o);
+// The weights' operands of it (lf_f32_operands), out of `cur`.
+lf_status prepare_f32_operands(lf_context* ctx, const lf_weights* w, WeightCursor& cur, SplitMatrix* g);
+
 // Triangle contraction, batched over the c channels of channel-major fp16
 // operands a, b [c][n][ld] (ld a multiple of 8, elements past n never read):
 //   outgoing: x[h][i][j] = scale * sum_k a[h][i][k] * b[h][j][k]

@@ -14,6 +14,7 @@ enum JobKind {
   JOB_OPERAND,    // ... -> fp16 [n_out][K] (the plain GEMM wants k contiguous in both operands)
   JOB_BIASED,     // ... -> fp16 [n_out][K + 16], bias in k column K and zeros after it (the activations carry a column of ones there)
   JOB_FOLD,       // float [n_out]: scale * (bias[c] + sum_k vec[k] W[k][col0 + c]): a LayerNorm offset folded into a bias
+  JOB_TERMS,      // ... -> three bf16 terms [3][rows][n_pad] at row0, zeros past K (n_pad = K rounded up to 8)
   JOB_COLSUM      // float [n_out]: sum_k fp16(vec[k] W[k][col0 + c]): what the tensor core multiplies the mean by
 };
 struct Job {
@@ -23,8 +24,9 @@ struct Job {
   void* out;
   float scale;
   int kind, K, ld, col0, n_out, n_fill, n_pad, row0;      // columns n_out .. n_fill - 1 are written as zeros
+  int64_t term_stride;
 };
-constexpr int kMaxJobs = 26;
+constexpr int kMaxJobs = 26;      // 2.1 KiB of kernel parameters
 struct JobList { Job j[kMaxJobs]; int count; };
 
 __global__ void __launch_bounds__(256) weight_jobs_kernel(const __grid_constant__ JobList list) {
@@ -50,12 +52,22 @@ __global__ void __launch_bounds__(256) weight_jobs_kernel(const __grid_constant_
     return;
   }
   // consecutive threads take consecutive columns of a row of W, so that the reads coalesce
-  const int K2 = j.kind == JOB_BIASED ? j.K + 16 : j.K;
+  const int K2 = j.kind == JOB_BIASED ? j.K + 16 : j.kind == JOB_TERMS ? j.n_pad : j.K;
   op16* out = reinterpret_cast<op16*>(j.out);
   for (int64_t i = first; i < (int64_t)K2 * j.n_fill; i += stride) {
     const int k = (int)(i / j.n_fill), n = (int)(i % j.n_fill);
     float v = 0.f;
-    if (n < j.n_out) v = k < j.K ? j.w[(int64_t)k * j.ld + j.col0 + n] : k == j.K ? j.bias[n] : 0.f;
+    if (n < j.n_out) v = k < j.K ? j.w[(int64_t)k * j.ld + j.col0 + n] : k == j.K && j.kind == JOB_BIASED ? j.bias[n] : 0.f;
+    if (j.kind == JOB_TERMS) {
+      bf16* t = reinterpret_cast<bf16*>(j.out) + (int64_t)(j.row0 + n) * K2 + k;
+#pragma unroll
+      for (int e = 0; e < 3; ++e) {
+        const bf16 b = __float2bfloat16_rn(v);
+        t[e * j.term_stride] = b;
+        v -= __bfloat162float(b);
+      }
+      continue;
+    }
     if (j.kind == JOB_IMAGE) {
       v = v * j.scale * (j.vec ? j.vec[k] : 1.0f);
       const int row = j.row0 + n;
@@ -199,6 +211,63 @@ lf_status prepare_weights(lf_context* ctx, lf_weights* w, WeightCursor& cur) {
     prep.operand(f[OPM_WR], cm, c, c, wlr + (int64_t)c * cm);
     prep.operand(f[OPM_WOUT], c * c, cz, cz, wout);
     w->g = {wlr, wout};
+  }
+  prep.flush();
+  if (!cur.dry && cudaGetLastError() != cudaSuccess) return lf_fail(ctx, LF_ERR_CUDA, "weight preparation launch failed");
+  return LF_OK;
+}
+
+lf_status prepare_f32_operands(lf_context* ctx, const lf_weights* w, WeightCursor& cur, SplitMatrix* g) {
+  const auto& f = w->f;
+  const auto& dims = w->dims;
+  Preparer prep{ctx, cur};
+  struct Part { const float* w; int ld, col0, n; };
+  auto operand = [&](SplitMatrix& out, int K, std::initializer_list<Part> parts) {
+    const int ld = (K + 7) / 8 * 8;
+    int n = 0, row = 0;
+    for (const Part& q : parts) n += q.n;
+    bf16* p = cur.take<bf16>((size_t)3 * n * ld);
+    out.p = p;
+    out.ld = ld;
+    out.batch_stride = 0;
+    out.term_stride = (int64_t)n * ld;
+    for (const Part& q : parts) {
+      if (q.n) prep.push(Job{q.w, nullptr, nullptr, p, 1.0f, JOB_TERMS, K, q.ld, q.col0, q.n, q.n, ld, row, out.term_stride});
+      row += q.n;
+    }
+  };
+  const int c = dims.channels, HD = dims.heads * dims.head_dim;
+  switch (w->kind) {
+    case LF_WEIGHTS_TRIANGLE_AF2:
+    case LF_WEIGHTS_TRIANGLE_AF3:
+      operand(g[0], c, {{f[TRI_W4], 4 * dims.hidden, 0, 4 * dims.hidden}});
+      operand(g[1], dims.hidden, {{f[TRI_WZ], c, 0, c}});
+      operand(g[2], c, {{f[TRI_WG], c, 0, c}});
+      break;
+    case LF_WEIGHTS_TRANSITION_AF2:
+    case LF_WEIGHTS_TRANSITION_AF3: {
+      const int wide = w->kind == LF_WEIGHTS_TRANSITION_AF3 ? 2 * dims.hidden : dims.hidden;
+      operand(g[0], c, {{f[TRN_W1], wide, 0, wide}});
+      operand(g[1], dims.hidden, {{f[TRN_W2], c, 0, c}});
+      break;
+    }
+    case LF_WEIGHTS_GLOBAL_ATTENTION_AF2: {
+      const int wide = 2 * dims.head_dim + HD;
+      operand(g[0], c, {{f[GLB_W3], wide, 0, wide}});
+      operand(g[1], HD, {{f[GLB_WO], c, 0, c}});
+      break;
+    }
+    case LF_WEIGHTS_MSA_ATTENTION_AF3:
+      operand(g[0], c, {{f[ATT_W4], 4 * HD, 2 * HD, 2 * HD}});
+      operand(g[1], HD, {{f[ATT_WO], c, 0, c}});
+      break;
+    case LF_WEIGHTS_ATTENTION_AF2:
+    case LF_WEIGHTS_GRID_ATTENTION_AF3:
+    case LF_WEIGHTS_SINGLE_ATTENTION_AF3:
+      operand(g[0], c, {{f[ATT_W4], 4 * HD, 0, 4 * HD}, {f[ATT_WB], dims.heads, 0, w->has_pair_proj && !w->has_pair_norm ? dims.heads : 0}});
+      operand(g[1], HD, {{f[ATT_WO], c, 0, c}});
+      break;
+    default: return lf_fail(ctx, LF_ERR_UNSUPPORTED, "weights of kind %d have no float32 GEMM operands", w->kind);
   }
   prep.flush();
   if (!cur.dry && cudaGetLastError() != cudaSuccess) return lf_fail(ctx, LF_ERR_CUDA, "weight preparation launch failed");
