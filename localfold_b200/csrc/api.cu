@@ -962,17 +962,16 @@ void sgemm(lf_context* ctx, ArenaCursor& cur, bool ta, bool tb, int epi, int M, 
 #undef SG
 }
 
-// The float32 attention core: q | k | v | gate rows -> gated output rows.  Head widths are rounded up to the next instance.
+// The float32 attention core: terms of q | k | v | gate -> terms of the gated output.
+constexpr int kAttentionSmem = 96 * 1024;      // two blocks an SM
 #define ATTENTION_WIDTHS(X) X(8) X(16) X(24) X(32) X(48) X(64)
-void attention_f32(lf_context* ctx, ArenaCursor& cur, const float* qkvg, const float* bias, const float* mask, f32mma::AttentionShape s, bf16* out) {
-  const int D = s.d <= 32 ? (s.d + 7) / 8 * 8 : s.d <= 48 ? 48 : 64;
+void attention_f32(lf_context* ctx, ArenaCursor& cur, int D, const bf16* qkvg, const float* bias, const float* mask, f32mma::AttentionShape s, bf16* out) {
   // eight warps, or as many as the queries have groups of 16: the groups are spread evenly over the blocks; small query
-  // counts put several batch rows into a block.  A thread stages at most four groups of four channels: wq >= D / 8.
-  const int groups = lf_ceil_div(s.Q, 16), tiles = lf_ceil_div(groups, 8), least = D / 8;
+  // counts put several batch rows into a block
+  const int groups = lf_ceil_div(s.Q, 16), tiles = lf_ceil_div(groups, 8);
   s.wq = lf_ceil_div(groups, tiles);
-  if (s.wq < least) s.wq = least;
   s.wb = 8 / s.wq < s.batch ? 8 / s.wq : s.batch;
-  while (s.wb > 1 && (int64_t)tiles * s.heads * lf_ceil_div(s.batch, s.wb) < ctx->sm_count) s.wb /= 2;
+  while (s.wb > 1 && ((int64_t)tiles * s.heads * lf_ceil_div(s.batch, s.wb) < ctx->sm_count || f32mma::attention_smem(D, s.wb) > kAttentionSmem)) s.wb /= 2;
   const dim3 grid(lf_ceil_div(groups, s.wq), lf_ceil_div(s.batch, s.wb), s.heads);
   const size_t smem = f32mma::attention_smem(D, s.wb);
 #define ATTENTION_CASE(D_)                                                                                                                          \
@@ -986,8 +985,8 @@ void attention_f32(lf_context* ctx, ArenaCursor& cur, const float* qkvg, const f
 
 void configure_attention_f32() {
 #define ATTENTION_CASE(D_)                                                                                                                               \
-  cudaFuncSetAttribute(f32mma::attention_kernel<D_, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)f32mma::attention_smem(D_, 64 / D_));   \
-  cudaFuncSetAttribute(f32mma::attention_kernel<D_, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)f32mma::attention_smem(D_, 64 / D_));
+  cudaFuncSetAttribute(f32mma::attention_kernel<D_, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, kAttentionSmem);   \
+  cudaFuncSetAttribute(f32mma::attention_kernel<D_, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, kAttentionSmem);
   ATTENTION_WIDTHS(ATTENTION_CASE)
 #undef ATTENTION_CASE
 }
@@ -1212,27 +1211,30 @@ lf_status separate_bias(lf_context* ctx, ArenaCursor& cur, const AttArgs& a, flo
 template <typename T>
 lf_status att_f32(lf_context* ctx, ArenaCursor& cur, const AttArgs& a) {
   const int64_t R = (int64_t)a.batch * a.Q;
-  const int HD = a.heads * a.d, c = a.ch;
+  const int c = a.ch;
   const auto& f = a.w->f;
   const SplitMatrix* g = nullptr;
   SplitMatrix none[3];
   if (cur.dry) g = none; else LF_TRY(f32_operands(ctx, a.w, &g));
   const SplitMatrix nrm = take_terms(cur, R, c);
-  // q | k | v | sigmoid(gate), and the pair bias columns when the bias comes from the normalised input
-  const int wide = 4 * HD + (a.bias_mode == 2 ? a.heads : 0), ldq = (wide + 3) / 4 * 4;
-  float* qkvg = cur.take<float>(R * ldq);
+  // q | k | v | sigmoid(gate) with heads of D channels, and the pair bias columns when the bias comes from the normalised input
+  const int D = f32_head_width(a.d), HDp = a.heads * D, wide = 4 * HDp + (a.bias_mode == 2 ? a.heads : 0);
+  const SplitMatrix qkvg = take_terms(cur, R, wide);
   float* bias = a.bias_mode ? cur.take<float>((int64_t)a.heads * a.Q * a.Q) : nullptr;
-  const SplitMatrix o = take_terms(cur, R, HD);
+  const SplitMatrix o = take_terms(cur, R, HDp);
   float* proj = cur.take<float>(R * c);
   layer_norm<T, rows::LN_TERMS>(ctx, cur, a.act, R, c, f[ATT_LN_G], f[ATT_LN_B], a.eps, a.variance, a.transpose, a.batch, a.Q, (void*)nrm.p, nrm.term_stride);
-  LF_TRY(tc::gemm_f32(ctx, cur, 0, nrm, g[0], (int)R, wide, c, 1, {qkvg, nullptr, ldq, 0, 0, f[ATT_B4], 4 * HD, 0, 3 * HD, 4 * HD}));
+  LF_TRY(tc::gemm_f32(ctx, cur, 0, nrm, g[0], (int)R, wide, c, 1,
+                      {nullptr, (bf16*)qkvg.p, qkvg.ld, 0, qkvg.term_stride, reinterpret_cast<const float*>(g[2].p), 4 * HDp, 0, 3 * HDp, 4 * HDp}));
   if (a.bias_mode == 1) LF_TRY(separate_bias(ctx, cur, a, bias));
   else if (a.bias_mode == 2)
-    LAUNCH(ctx, cur, rows::bias_columns_kernel, lf_ceil_div((int64_t)a.Q * a.Q, 256), 256, 0, qkvg, (int64_t)ldq, 4 * HD, a.Q, a.heads, a.bias_swap, bias);
-  attention_f32(ctx, cur, qkvg, bias, a.mask,
-                f32mma::AttentionShape{a.batch, a.Q, a.heads, a.d, a.transpose, a.mask_mode, a.clamp, 1.0f / sqrtf((float)a.d), ldq, o.ld, o.term_stride, 1, 1},
+    LAUNCH(ctx, cur, rows::bias_columns_kernel, lf_ceil_div((int64_t)a.Q * a.Q, 256), 256, 0, qkvg.p, qkvg.ld, qkvg.term_stride, 4 * HDp, a.Q, a.heads,
+           a.bias_swap, bias);
+  attention_f32(ctx, cur, D, qkvg.p, bias, a.mask,
+                f32mma::AttentionShape{a.batch, a.Q, a.heads, a.transpose, a.mask_mode, a.clamp, 1.0f / sqrtf((float)a.d), qkvg.ld, qkvg.term_stride, o.ld,
+                                       o.term_stride, 1, 1},
                 (bf16*)o.p);
-  LF_TRY(tc::gemm_f32(ctx, cur, 0, o, g[1], (int)R, c, HD, 1, {proj, nullptr, c, 0, 0, f[ATT_BO], c, 0, 0, 0}));
+  LF_TRY(tc::gemm_f32(ctx, cur, 0, o, g[1], (int)R, c, HDp, 1, {proj, nullptr, c, 0, 0, f[ATT_BO], c, 0, 0, 0}));
   finish<T>(ctx, cur, proj, nullptr, a.residual ? a.act : nullptr, R, c, a.transpose, a.batch, a.Q, a.out);
   return LF_OK;
 }

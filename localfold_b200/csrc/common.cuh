@@ -76,9 +76,11 @@ struct SplitMatrix {
 };
 
 // Operands of the float32 GEMM, [n_out][k] terms: made at the first float32 call that uses the weights, kept with them.
-//   triangle: fused projection, output projection, output gate; attention: fused projection (with the pair bias columns when
-//   the bias comes from the normalised input; values and gate alone for the MSA averaging), output projection;
+//   triangle: fused projection, output projection, output gate; attention: fused projection with heads padded to
+//   f32_head_width (and the pair bias columns when the bias comes from the normalised input), output projection, and at
+//   g[2].p the projection's bias (float32); MSA averaging: values | gate, output projection;
 //   transition: both projections; global attention: key | value | gate, output projection
+constexpr int f32_head_width(int d) { return d <= 32 ? (d + 7) / 8 * 8 : d <= 48 ? 48 : 64; }      // the attention core's instances
 struct lf_f32_operands {
   std::mutex mutex;
   bool made = false;

@@ -65,13 +65,20 @@ __device__ __forceinline__ void ldmatrix2(uint32_t& r0, uint32_t& r1, const void
   else asm volatile("ldmatrix.sync.aligned.m8n8.x2.shared.b16 {%0, %1}, [%2];" : "=r"(r0), "=r"(r1) : "r"(a) : "memory");
 }
 
+// global -> shared without passing through registers; bytes 0 writes zeros
+__device__ __forceinline__ void copy_async16(void* dst, const void* src, int bytes) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"((uint32_t)__cvta_generic_to_shared(dst)), "l"(src), "r"(bytes) : "memory");
+}
+__device__ __forceinline__ void copy_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+__device__ __forceinline__ void copy_async_wait() { asm volatile("cp.async.wait_group 0;" ::: "memory"); }
+
 struct AttentionShape {
-  int batch, Q, heads, d;
+  int batch, Q, heads;
   int transpose, mask_mode, clamp;      // mask_mode 0: logit += 1e9 (m - 1); 1: logit += m > 0 ? 0 : -1e9
   float scale;
-  int64_t ld;                           // floats from one row of q | k | v | gate to the next (a multiple of 4)
-  int64_t ldo, term_stride;             // output rows and terms, in bf16 elements
-  int wb, wq;                           // warps of a block: wb batch rows x wq groups of 16 queries, wq >= D / 8
+  int64_t ld, term_stride;              // rows and terms of q | k | v | gate, in bf16 elements (multiples of 8)
+  int64_t ldo, out_stride;              // ... and of the output
+  int wb, wq;                           // warps of a block: wb batch rows x wq groups of 16 queries
 };
 
 constexpr int AT_KT = 32;                                                     // keys per staged tile
@@ -80,12 +87,13 @@ __host__ __device__ constexpr size_t attention_smem(int D, int wb) {
   return (size_t)2 * wb * (2 * 3 * AT_KT * at_pitch(D) * 2 + AT_KT * 4);
 }
 
-//   qkvg: [rows][ld] = (q | k | v | sigmoid(gate) | ...) in logical row order
+//   qkvg: [3][rows][ld] = terms of (q | k | v | sigmoid(gate) | ...) in logical row order, a head of each D channels wide
+//         (the projection's weights are padded to the instance's width, so nothing here is conditional on the true one)
 //   bias: [H][Q][Q] or null; mask: indexed b * Q + j, or j * batch + b when transpose
 //   out:  [3][rows][ldo] = softmax(.) v * gate as terms, the operand of the output projection
 // A warp owns 16 queries of one (batch row, head); Q and the running output stay in registers in the tensor core's
 // fragment layout, and probabilities become the A operand of P V without leaving them.  The warps of a block share K and
-// V tiles of 32 keys, which a thread fetches a tile ahead and splits once.  A row's reference is the maximum of its first
+// V tiles of 32 keys, copied a tile ahead as the projection wrote them.  A row's reference is the maximum of its first
 // 32 logits, raised only when exponentials overflow 2^60: no maximum is searched otherwise.  P V of a tile goes into
 // fresh accumulators (the leading term product apart from the others) that are added to the output outside the tensor
 // core, so that whatever the tensor core's own additions lose is of a tile's share, not of the running sum: 2e-7
@@ -94,15 +102,15 @@ __host__ __device__ constexpr size_t attention_smem(int D, int wb) {
 // 384 x 384 with 4 heads of 16: 0.51 ms, against 5.06 ms with a warp per query and a shuffle per key and 0.68 ms with
 // four queries a thread on packed FMAs; 203 x 203, 4 x 32: 0.19 ms against 0.98 and 0.24.
 template <int D, bool BIAS>
-__global__ void __launch_bounds__(256, D <= 16 || D == 32 ? 2 : 1)
-attention_kernel(const float* __restrict__ qkvg, const float* __restrict__ bias, const float* __restrict__ mask,
+__global__ void __launch_bounds__(256, D <= 32 ? 2 : 1)
+attention_kernel(const __nv_bfloat16* __restrict__ qkvg, const float* __restrict__ bias, const float* __restrict__ mask,
                  const AttentionShape s, __nv_bfloat16* __restrict__ out) {
   constexpr int KT = AT_KT, PITCH = at_pitch(D), NK = D / 16, TAIL = (D / 8) & 1, ND = D / 8;
   constexpr int PLANE = KT * PITCH;                 // bf16 elements of one term of one tile
   extern __shared__ uint4 at_sm[];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, g = lane >> 2, t = lane & 3;
   const int wb = warp / s.wq, wq = warp % s.wq;
-  const int d = s.d, Q = s.Q, HD = s.heads * d;
+  const int Q = s.Q, HD = s.heads * D;
   const int64_t ld = s.ld;
   const int h = blockIdx.z, b0 = blockIdx.y * s.wb, b = b0 + wb;
   const int q0 = (blockIdx.x * s.wq + wq) * 16;
@@ -112,96 +120,44 @@ attention_kernel(const float* __restrict__ qkvg, const float* __restrict__ bias,
   const int tiles = (Q + KT - 1) / KT;
   const bool active = b < s.batch && q0 < Q;        // of the warp as a whole
 
-  // ---- staging: a thread carries up to four groups of four channels a tile (K, then V), at the same places of every
-  // tile; they are fetched a tile ahead and split when their buffer is free ----
-  constexpr int NU = 4, GROUPS = D / 4;
-  const bool vec = (d & 3) == 0;
-  const float* unit_src[NU];
-  int unit_dst[NU];                                  // element offset in the buffer; -1 = no such unit
-  int unit_j[NU];
-  float4 next[NU];
-  float next_mask = 0.f;
-#pragma unroll
-  for (int i = 0; i < NU; ++i) {
-    const int u = threadIdx.x + i * blockDim.x;
-    const int e = (u % GROUPS) * 4, which = (u / GROUPS) & 1, j = (u / (2 * GROUPS)) % KT, bb = u / (2 * GROUPS * KT);
-    unit_dst[i] = bb < s.wb ? (bb * 2 + which) * 3 * PLANE + j * PITCH + e : -1;
-    unit_j[i] = bb < s.wb && b0 + bb < s.batch && e < d ? j : Q;      // Q: nothing to fetch, zeros
-    unit_src[i] = qkvg + ((int64_t)(b0 + bb) * Q + j) * ld + (1 + which) * HD + h * d + e;
-  }
-  const int mask_bb = b0 + threadIdx.x / KT, mask_j = threadIdx.x % KT;
-  const bool mask_mine = threadIdx.x < s.wb * KT;
-  auto fetch = [&](int tile) {
-    const int j0 = tile * KT;
-#pragma unroll
-    for (int i = 0; i < NU; ++i) {
-      next[i] = make_float4(0.f, 0.f, 0.f, 0.f);
-      if (unit_j[i] < Q - j0) {
-        if (vec) next[i] = __ldg(reinterpret_cast<const float4*>(unit_src[i]));
-        else {
-          const int e = (threadIdx.x + i * blockDim.x) % GROUPS * 4;
-          next[i].x = __ldg(unit_src[i]);
-          if (e + 1 < d) next[i].y = __ldg(unit_src[i] + 1);
-          if (e + 2 < d) next[i].z = __ldg(unit_src[i] + 2);
-          if (e + 3 < d) next[i].w = __ldg(unit_src[i] + 3);
-        }
-      }
-      unit_src[i] += (int64_t)KT * ld;
-    }
-    if (mask_mine) {
-      const int j = j0 + mask_j;
-      next_mask = 0.f;
-      if (j < Q) {
-        const float m = mask_bb < s.batch ? __ldg(mask + (s.transpose ? (int64_t)j * s.batch + mask_bb : (int64_t)mask_bb * Q + j)) : 1.f;
-        next_mask = s.mask_mode == 0 ? 1e9f * (m - 1.0f) : (m > 0.f ? 0.f : -1e9f);
-      }
-    }
-  };
+  // ---- staging: 16-byte copies of eight channels of one term ----
   auto stage = [&](int tile) {
-    const int buf = tile & 1;
-    __nv_bfloat16* base = kv_s + buf * s.wb * 6 * PLANE;
-#pragma unroll
-    for (int i = 0; i < NU; ++i) {
-      if (unit_dst[i] < 0) continue;
-      uint32_t lo[3], hi[3];
-      split3(next[i].x, next[i].y, lo);
-      split3(next[i].z, next[i].w, hi);
-#pragma unroll
-      for (int k = 0; k < 3; ++k) *reinterpret_cast<uint2*>(base + unit_dst[i] + k * PLANE) = make_uint2(lo[k], hi[k]);
+    const int j0 = tile * KT, buf = tile & 1;
+    for (int u = threadIdx.x; u < s.wb * 6 * KT * ND; u += blockDim.x) {
+      const int e = (u % ND) * 8, j = (u / ND) % KT, part = (u / (ND * KT)) % 6, bb = u / (ND * KT * 6);      // part: K terms, V terms
+      const int which = part / 3, term = part % 3;
+      const bool ok = j0 + j < Q && b0 + bb < s.batch;
+      const __nv_bfloat16* src = ok ? qkvg + term * s.term_stride + ((int64_t)(b0 + bb) * Q + j0 + j) * ld + (1 + which) * HD + h * D + e : qkvg;
+      copy_async16(kv_s + ((buf * s.wb + bb) * 6 + part) * PLANE + j * PITCH + e, src, ok ? 16 : 0);
     }
-    if (mask_mine) mask_s[buf * s.wb * KT + threadIdx.x] = next_mask;
+    copy_async_commit();
+    for (int u = threadIdx.x; u < s.wb * KT; u += blockDim.x) {
+      const int j = j0 + u % KT, bb = b0 + u / KT;
+      float term = 0.f;
+      if (j < Q && bb < s.batch) {
+        const float m = __ldg(mask + (s.transpose ? (int64_t)j * s.batch + bb : (int64_t)bb * Q + j));
+        term = s.mask_mode == 0 ? 1e9f * (m - 1.0f) : (m > 0.f ? 0.f : -1e9f);
+      }
+      mask_s[buf * s.wb * KT + u] = term;
+    }
   };
-
-  fetch(0);
+  stage(0);
 
   // ---- Q as A fragments of its three terms ----
   uint32_t qa[3][NK > 0 ? NK : 1][4], qt[3][2];      // qt: the last 8 channels of an odd number of them
   const int row0 = q0 + g, row1 = q0 + g + 8;
-  auto q_pair = [&](int row, int e, uint32_t (&term)[3]) {
-    float x = 0.f, y = 0.f;
-    if (active && row < Q) {
-      const float* src = qkvg + ((int64_t)b * Q + row) * ld + h * d + e;
-      if (e < d) x = src[0];
-      if (e + 1 < d) y = src[1];
-    }
-    split3(x, y, term);
+  auto q_pair = [&](int row, int term, int e) {
+    return active && row < Q ? *reinterpret_cast<const uint32_t*>(qkvg + term * s.term_stride + ((int64_t)b * Q + row) * ld + h * D + e) : 0u;
   };
 #pragma unroll
-  for (int kk = 0; kk < NK; ++kk)
+  for (int i = 0; i < 3; ++i) {
 #pragma unroll
-    for (int r = 0; r < 4; ++r) {
-      uint32_t term[3];
-      q_pair((r & 1) ? row1 : row0, kk * 16 + 2 * t + (r >> 1) * 8, term);
+    for (int kk = 0; kk < NK; ++kk)
 #pragma unroll
-      for (int i = 0; i < 3; ++i) qa[i][kk][r] = term[i];
-    }
-  if (TAIL) {
+      for (int r = 0; r < 4; ++r) qa[i][kk][r] = q_pair((r & 1) ? row1 : row0, i, kk * 16 + 2 * t + (r >> 1) * 8);
+    if (TAIL) {
 #pragma unroll
-    for (int r = 0; r < 2; ++r) {
-      uint32_t term[3];
-      q_pair(r ? row1 : row0, NK * 16 + 2 * t, term);
-#pragma unroll
-      for (int i = 0; i < 3; ++i) qt[i][r] = term[i];
+      for (int r = 0; r < 2; ++r) qt[i][r] = q_pair(r ? row1 : row0, i, NK * 16 + 2 * t);
     }
   }
 
@@ -234,12 +190,10 @@ attention_kernel(const float* __restrict__ qkvg, const float* __restrict__ bias,
     for (int e = 0; e < 4; ++e) o[n][e] = 0.f;
   float ref[2] = {0.f, 0.f}, ref2[2] = {0.f, 0.f}, sum[2] = {0.f, 0.f};      // of rows row0, row1; ref2 = ref log2(e)
   if (active) load_bias(0);
-  stage(0);
-  if (tiles > 1) fetch(1);
   for (int tile = 0; tile < tiles; ++tile) {
+    copy_async_wait();
     __syncthreads();                                  // the tile is staged, and nobody reads the other buffer any more
     if (tile + 1 < tiles) stage(tile + 1);
-    if (tile + 2 < tiles) fetch(tile + 2);
     if (!active) continue;
     const int buf = tile & 1;
     const __nv_bfloat16* k_s = kv_s + (buf * s.wb + wb) * 6 * PLANE;
@@ -390,23 +344,21 @@ attention_kernel(const float* __restrict__ qkvg, const float* __restrict__ bias,
     const int row = r ? row1 : row0;
     if (row >= Q) continue;
     const float inv = 1.0f / sum[r];
-    const float* gate = qkvg + ((int64_t)b * Q + row) * ld + 3 * HD + h * d;
-    __nv_bfloat16* dst = out + ((int64_t)b * Q + row) * s.ldo + h * d;
+    const __nv_bfloat16* gate = qkvg + ((int64_t)b * Q + row) * ld + 3 * HD + h * D + 2 * t;
+    __nv_bfloat16* dst = out + ((int64_t)b * Q + row) * s.ldo + h * D + 2 * t;
 #pragma unroll
     for (int n = 0; n < ND; ++n) {
-      const int c = n * 8 + 2 * t;
-      if (c >= d) continue;
-      uint32_t term[3];
-      split3(o[n][2 * r] * inv * gate[c], c + 1 < d ? o[n][2 * r + 1] * inv * gate[c + 1] : 0.f, term);
+      float gx = 0.f, gy = 0.f;
 #pragma unroll
-      for (int i = 0; i < 3; ++i) {
-        __nv_bfloat16* cell = dst + i * s.term_stride + c;
-        if (!(d & 1)) *reinterpret_cast<uint32_t*>(cell) = term[i];
-        else {
-          *cell = __ushort_as_bfloat16((unsigned short)(term[i] & 0xffffu));
-          if (c + 1 < d) cell[1] = __ushort_as_bfloat16((unsigned short)(term[i] >> 16));
-        }
+      for (int i = 2; i >= 0; --i) {
+        const uint32_t w = *reinterpret_cast<const uint32_t*>(gate + i * s.term_stride + n * 8);
+        gx += __uint_as_float(w << 16);
+        gy += __uint_as_float(w & 0xffff0000u);
       }
+      uint32_t term[3];
+      split3(o[n][2 * r] * inv * gx, o[n][2 * r + 1] * inv * gy, term);
+#pragma unroll
+      for (int i = 0; i < 3; ++i) *reinterpret_cast<uint32_t*>(dst + i * s.out_stride + n * 8) = term[i];
     }
   }
 }

@@ -15,6 +15,9 @@ enum JobKind {
   JOB_BIASED,     // ... -> fp16 [n_out][K + 16], bias in k column K and zeros after it (the activations carry a column of ones there)
   JOB_FOLD,       // float [n_out]: scale * (bias[c] + sum_k vec[k] W[k][col0 + c]): a LayerNorm offset folded into a bias
   JOB_TERMS,      // ... -> three bf16 terms [3][rows][n_pad] at row0, zeros past K (n_pad = K rounded up to 8)
+  JOB_HEADS,      // the fused attention projection as terms, every head of d channels (row0) padded with zero rows to D (n_pad)
+  JOB_HEADS_BIAS, // ... its bias vector, as float32
+  JOB_HEADS_OUT,  // the output projection as terms, the k of every head padded likewise
   JOB_COLSUM      // float [n_out]: sum_k fp16(vec[k] W[k][col0 + c]): what the tensor core multiplies the mean by
 };
 struct Job {
@@ -47,6 +50,30 @@ __global__ void __launch_bounds__(256) weight_jobs_kernel(const __grid_constant_
       if (lane == 0) {
         if (j.bias && c < j.n_out) acc += (double)j.bias[c];
         reinterpret_cast<float*>(j.out)[c] = (float)(acc * j.scale);
+      }
+    }
+    return;
+  }
+  const int d = j.row0, D = j.n_pad;      // of the head forms
+  if (j.kind == JOB_HEADS_BIAS) {
+    for (int64_t n = first; n < j.n_fill; n += stride) reinterpret_cast<float*>(j.out)[n] = n % D < d ? j.w[n / D * d + n % D] : 0.f;
+    return;
+  }
+  if (j.kind == JOB_HEADS || j.kind == JOB_HEADS_OUT) {
+    // [n_fill][ld8(K)] (heads along n) or [n_out][n_fill] (heads along k)
+    const bool out_proj = j.kind == JOB_HEADS_OUT;
+    const int kk = out_proj ? j.n_fill : (j.K + 7) / 8 * 8, nn = out_proj ? j.n_out : j.n_fill;
+    for (int64_t i = first; i < (int64_t)kk * nn; i += stride) {
+      const int k = (int)(i / nn), n = (int)(i % nn);
+      float v = 0.f;
+      if (out_proj) { if (k % D < d) v = j.w[(int64_t)(k / D * d + k % D) * j.ld + n]; }
+      else if (k < j.K && n % D < d) v = j.w[(int64_t)k * j.ld + n / D * d + n % D];
+      bf16* t = reinterpret_cast<bf16*>(j.out) + (int64_t)n * kk + k;
+#pragma unroll
+      for (int e = 0; e < 3; ++e) {
+        const bf16 b = __float2bfloat16_rn(v);
+        t[e * j.term_stride] = b;
+        v -= __bfloat162float(b);
       }
     }
     return;
@@ -264,8 +291,20 @@ lf_status prepare_f32_operands(lf_context* ctx, const lf_weights* w, WeightCurso
     case LF_WEIGHTS_ATTENTION_AF2:
     case LF_WEIGHTS_GRID_ATTENTION_AF3:
     case LF_WEIGHTS_SINGLE_ATTENTION_AF3:
-      operand(g[0], c, {{f[ATT_W4], 4 * HD, 0, 4 * HD}, {f[ATT_WB], dims.heads, 0, w->has_pair_proj && !w->has_pair_norm ? dims.heads : 0}});
-      operand(g[1], HD, {{f[ATT_WO], c, 0, c}});
+      {
+        const int d = dims.head_dim, D = f32_head_width(d), wide = 4 * dims.heads * D, own_bias = w->has_pair_proj && !w->has_pair_norm ? dims.heads : 0;
+        const int ld = (c + 7) / 8 * 8;
+        bf16* p = cur.take<bf16>((size_t)3 * (wide + own_bias) * ld);
+        g[0] = SplitMatrix{p, ld, 0, (int64_t)(wide + own_bias) * ld};
+        prep.push(Job{f[ATT_W4], nullptr, nullptr, p, 1.0f, JOB_HEADS, c, 4 * HD, 0, 4 * HD, wide, D, d, g[0].term_stride});
+        if (own_bias) prep.push(Job{f[ATT_WB], nullptr, nullptr, p, 1.0f, JOB_TERMS, c, own_bias, 0, own_bias, own_bias, ld, wide, g[0].term_stride});
+        bf16* po = cur.take<bf16>((size_t)3 * c * dims.heads * D);
+        g[1] = SplitMatrix{po, (int64_t)dims.heads * D, 0, (int64_t)c * dims.heads * D};
+        prep.push(Job{f[ATT_WO], nullptr, nullptr, po, 1.0f, JOB_HEADS_OUT, HD, c, 0, c, dims.heads * D, D, d, g[1].term_stride});
+        float* bias = cur.take<float>(wide);
+        g[2].p = reinterpret_cast<const bf16*>(bias);
+        prep.push(Job{f[ATT_B4], nullptr, nullptr, bias, 1.0f, JOB_HEADS_BIAS, 0, 0, 0, 4 * HD, wide, D, d, 0});
+      }
       break;
     default: return lf_fail(ctx, LF_ERR_UNSUPPORTED, "weights of kind %d have no float32 GEMM operands", w->kind);
   }
