@@ -90,6 +90,9 @@ LF_API lf_status lf_context_create_on_stream(int device_ordinal, void* stream, l
 /* The cudaStream_t every call of this context enqueues on.  Work the caller enqueues elsewhere is
  * not ordered with the library's: use this stream, or events, or lf_context_synchronize. */
 LF_API void* lf_context_stream(const lf_context* ctx);
+/* Work enqueued on the context's stream from here on comes after what `stream` holds now (no host wait).  For inputs
+ * that other code produces on a stream of its own. */
+LF_API lf_status lf_context_await(lf_context* ctx, void* stream);
 LF_API void lf_context_destroy(lf_context* ctx);
 LF_API const char* lf_last_error(const lf_context* ctx);
 LF_API lf_status lf_context_synchronize(lf_context* ctx);
@@ -438,6 +441,9 @@ typedef struct lf_pair_stack_desc {
   int32_t order;               /* lf_pair_block_order */
 } lf_pair_stack_desc;
 LF_API lf_status lf_pair_stack_run(lf_context* ctx, const lf_pair_stack_desc* d, lf_result* r);
+/* The same with a host-space pair read from `pair_in` and the result written to desc->pair (which need not hold the
+ * input); NULL reads desc->pair.  Device-space calls update desc->pair in place and take NULL. */
+LF_API lf_status lf_pair_stack_run_from(lf_context* ctx, const lf_pair_stack_desc* desc, const void* pair_in, lf_result* result);
 
 /* ---- row-sharded pair stack (several GPUs) ------------------------------- */
 

@@ -140,12 +140,12 @@ class ShardPeers(ctypes.Structure):
 
 
 EXPORTS = (
-    "lf_version", "lf_context_create", "lf_context_create_on_stream", "lf_context_stream", "lf_context_destroy", "lf_last_error", "lf_context_synchronize",
+    "lf_version", "lf_context_create", "lf_context_create_on_stream", "lf_context_stream", "lf_context_await", "lf_context_destroy", "lf_last_error", "lf_context_synchronize",
     "lf_context_launch_count", "lf_context_profile", "lf_context_profile_read", "lf_context_reserve", "lf_context_release_scratch", "lf_context_limit_scratch", "lf_weights_create", "lf_weights_create_encoded",
     "lf_weights_destroy", "lf_int5_decode", "lf_triangle_multiplication_run",
     "lf_triangle_multiplication_run_static", "lf_attention_run",
     "lf_transition_run", "lf_outer_product_mean_run", "lf_single_attention_run", "lf_msa_attention_run",
-    "lf_global_column_attention_run", "lf_distogram_logits_run", "lf_pair_stack_run",
+    "lf_global_column_attention_run", "lf_distogram_logits_run", "lf_pair_stack_run", "lf_pair_stack_run_from",
     "lf_pair_shard_step", "lf_pair_shard_exchange_step", "lf_pair_planes_scatter", "lf_peer_buffer_create", "lf_peer_buffer_open", "lf_peer_buffer_close",
     "lf_peer_buffer_destroy", "lf_pair_transpose_scatter",
 )
@@ -168,6 +168,7 @@ def load():
     lib.lf_context_create_on_stream.argtypes = [ctypes.c_int, c_void_p, ctypes.POINTER(c_void_p)]
     lib.lf_context_stream.argtypes = [c_void_p]
     lib.lf_context_stream.restype = c_void_p
+    lib.lf_context_await.argtypes = [c_void_p, c_void_p]
     lib.lf_context_destroy.argtypes = [c_void_p]
     lib.lf_context_destroy.restype = None
     lib.lf_context_synchronize.argtypes = [c_void_p]
@@ -197,6 +198,7 @@ def load():
                        ("lf_distogram_logits_run", DistogramDesc), ("lf_pair_stack_run", PairStackDesc),
                        ("lf_pair_shard_step", ShardStepDesc)):
         getattr(lib, name).argtypes = [c_void_p, ctypes.POINTER(desc), ctypes.POINTER(Result)]
+    lib.lf_pair_stack_run_from.argtypes = [c_void_p, ctypes.POINTER(PairStackDesc), c_void_p, ctypes.POINTER(Result)]
     lib.lf_pair_shard_exchange_step.argtypes = [c_void_p, ctypes.POINTER(ShardStepDesc), ctypes.POINTER(ShardPeers),
                                                 ctypes.POINTER(Result)]
     lib.lf_pair_planes_scatter.argtypes = [c_void_p, c_void_p, c_int32, c_int32, c_int32, c_int32, c_int32, ctypes.POINTER(c_void_p)]

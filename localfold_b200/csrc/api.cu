@@ -79,6 +79,15 @@ lf_status lf_context_create_on_stream(int device_ordinal, void* stream, lf_conte
 
 void* lf_context_stream(const lf_context* ctx) { return ctx ? (void*)ctx->stream : nullptr; }
 
+lf_status lf_context_await(lf_context* ctx, void* stream) {
+  if (!ctx) return LF_ERR_ARGUMENT;
+  if ((cudaStream_t)stream == ctx->stream) return LF_OK;
+  cudaSetDevice(ctx->device);
+  LF_CUDA(ctx, cudaEventRecord(ctx->inputs, (cudaStream_t)stream));
+  LF_CUDA(ctx, cudaStreamWaitEvent(ctx->stream, ctx->inputs, 0));
+  return LF_OK;
+}
+
 static lf_status context_create(int device_ordinal, void* stream, bool make_stream, lf_context** out) {
   if (!out) return LF_ERR_ARGUMENT;
   *out = nullptr;
@@ -96,6 +105,7 @@ static lf_status context_create(int device_ordinal, void* stream, bool make_stre
   }
   cudaEventCreate(&ctx->ev0);
   cudaEventCreate(&ctx->ev1);
+  cudaEventCreateWithFlags(&ctx->inputs, cudaEventDisableTiming);
   cudaDeviceProp prop;
   if (cudaGetDeviceProperties(&prop, device_ordinal) == cudaSuccess) ctx->sm_count = prop.multiProcessorCount;
   tc::configure_once();
@@ -112,6 +122,7 @@ static lf_status context_create(int device_ordinal, void* stream, bool make_stre
       });
   }
   if (cudaMalloc(&ctx->tc_status, 16) == cudaSuccess) cudaMemset(ctx->tc_status, 0, 16);
+  if (cudaMallocHost(&ctx->status_host, 16) != cudaSuccess) { cudaGetLastError(); ctx->status_host = nullptr; }
   lf_block_cache_context(device_ordinal, 1);
   *out = ctx;
   return LF_OK;
@@ -127,6 +138,8 @@ void lf_context_destroy(lf_context* ctx) {
   lf_block_cache_context(ctx->device, -1);
   if (ctx->ev0) cudaEventDestroy(ctx->ev0);
   if (ctx->ev1) cudaEventDestroy(ctx->ev1);
+  if (ctx->inputs) cudaEventDestroy(ctx->inputs);
+  if (ctx->status_host) cudaFreeHost(ctx->status_host);
   if (ctx->owns_stream) cudaStreamDestroy(ctx->stream);
   delete ctx;
 }
@@ -135,8 +148,7 @@ const char* lf_last_error(const lf_context* ctx) { return ctx ? ctx->error.c_str
 
 lf_status lf_context_synchronize(lf_context* ctx) {
   if (!ctx) return LF_ERR_ARGUMENT;
-  LF_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
-  return tc::check_status(ctx);
+  return tc::check_status(ctx);      // (waits for the stream)
 }
 
 uint64_t lf_context_launch_count(const lf_context* ctx) { return ctx ? ctx->launches : 0; }
@@ -1473,9 +1485,8 @@ lf_status run_with_arena(lf_context* ctx, lf_result* r, bool timed, F body) {
   float ms = 0.f;
   if (timed) {
     cudaEventRecord(ctx->ev1, ctx->stream);
-    LF_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
+    LF_TRY(tc::check_status(ctx));      // (waits for the stream)
     cudaEventElapsedTime(&ms, ctx->ev0, ctx->ev1);
-    LF_TRY(tc::check_status(ctx));
   }
   LF_CUDA(ctx, cudaGetLastError());
   if (r) { r->elapsed_ms = ms; r->peak_bytes = ctx->arena_peak; r->launches = (uint32_t)(ctx->launches - before); }
@@ -1871,7 +1882,9 @@ lf_status lf_distogram_logits_run(lf_context* ctx, const lf_distogram_desc* d, l
   });
 }
 
-lf_status lf_pair_stack_run(lf_context* ctx, const lf_pair_stack_desc* d, lf_result* r) {
+lf_status lf_pair_stack_run(lf_context* ctx, const lf_pair_stack_desc* d, lf_result* r) { return lf_pair_stack_run_from(ctx, d, nullptr, r); }
+
+lf_status lf_pair_stack_run_from(lf_context* ctx, const lf_pair_stack_desc* d, const void* pair_in, lf_result* r) {
   if (!ctx) return LF_ERR_ARGUMENT;
   if (!d || !d->pair || !d->mask || !d->blocks) return lf_fail(ctx, LF_ERR_ARGUMENT, "pair stack: null argument");
   if (d->length <= 0 || d->c_z <= 0 || d->c_hidden <= 0 || d->heads <= 0 || d->transition_hidden <= 0)
@@ -1893,12 +1906,13 @@ lf_status lf_pair_stack_run(lf_context* ctx, const lf_pair_stack_desc* d, lf_res
       return lf_fail(ctx, LF_ERR_ARGUMENT, "block %d: triangle attention needs a normalized-input pair projection", b);
   }
   const bool host = d->space == LF_SPACE_HOST;
+  if (pair_in && !host) return lf_fail(ctx, LF_ERR_ARGUMENT, "pair stack: a device-space pair is updated in place");
   const int n = d->length, cz = d->c_z;
   const size_t P = (size_t)n * n, es = dtype_size(d->act_dtype);
   const lf_status status = run_with_arena(ctx, r, host, [&](ArenaCursor& cur) -> lf_status {
     Staging st{ctx, &cur, host};
     void* pair = host ? st.out(d->pair, P * cz * es) : d->pair;
-    if (host && !cur.dry) cudaMemcpyAsync(pair, d->pair, P * cz * es, cudaMemcpyHostToDevice, ctx->stream);
+    if (host && !cur.dry) cudaMemcpyAsync(pair, pair_in ? pair_in : d->pair, P * cz * es, cudaMemcpyHostToDevice, ctx->stream);
     const float* mask = (const float*)st.in(d->mask, P * 4);
     const size_t scratch_base = cur.offset;
     for (int b = d->first_block; b < d->first_block + d->n_blocks; ++b) {
@@ -1939,7 +1953,10 @@ lf_status lf_pair_stack_run(lf_context* ctx, const lf_pair_stack_desc* d, lf_res
     return LF_OK;
   });
   // The device cannot hold the pair beside the operators' scratch: leave the pair in the caller's buffer and stream it through in chunks.
-  if (status == LF_ERR_MEMORY && host) return lf_pair_stack_spilled(ctx, d, r);
+  if (status == LF_ERR_MEMORY && host) {
+    if (pair_in && pair_in != d->pair) memcpy(d->pair, pair_in, P * cz * es);
+    return lf_pair_stack_spilled(ctx, d, r);
+  }
   return status;
 }
 

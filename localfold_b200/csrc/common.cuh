@@ -37,6 +37,8 @@ struct lf_context {
   size_t arena_limit = 0;      // 0 = none; otherwise requests above it are refused without asking the driver (lf_context_limit_scratch)
   uint64_t launches = 0;
   cudaEvent_t ev0 = nullptr, ev1 = nullptr;
+  cudaEvent_t inputs = nullptr;      // lf_context_await
+  void* status_host = nullptr;       // pinned copy of *tc_status
   int sm_count = 148;
   void* tc_status = nullptr;   // device word the tensor-core kernels set when a bounded wait expires
   // Optional per-kernel-family timing (CUDA events on the context's stream).

@@ -143,11 +143,15 @@ lf_status make_map_plane_runs(lf_context* ctx, CUtensorMap* map, const void* bas
   return LF_OK;
 }
 
+// Waits for the context's stream; the status word comes back behind its work, in the same wait.
 lf_status check_status(lf_context* ctx) {
-  if (!ctx->tc_status) return LF_OK;
-  Status st;
-  if (cudaMemcpy(&st, ctx->tc_status, sizeof st, cudaMemcpyDeviceToHost) != cudaSuccess)
-    return lf_fail(ctx, LF_ERR_CUDA, "reading the kernel status word failed: %s", cudaGetErrorString(cudaGetLastError()));
+  Status st{};
+  if (ctx->tc_status) {
+    Status* to = ctx->status_host ? static_cast<Status*>(ctx->status_host) : &st;
+    LF_CUDA(ctx, cudaMemcpyAsync(to, ctx->tc_status, sizeof st, cudaMemcpyDeviceToHost, ctx->stream));
+    LF_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
+    st = *to;
+  } else LF_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
   if (st.code != 0) {
     cudaMemset(ctx->tc_status, 0, sizeof st);
     return lf_fail(ctx, LF_ERR_TIMEOUT, "a bounded wait expired in a tensor-core kernel (wait %u, block %u)", st.where, st.block);

@@ -15,7 +15,7 @@ struct PeerPtrs { void* p[kMaxPeers]; };
 void configure_once();
 // Tensor-core operands of the weights, out of the weights' own allocation (tc_weights.cu); a dry cursor only adds sizes up.
 lf_status prepare_weights(lf_context* ctx, lf_weights* w, WeightCursor& cur);
-// Reads the device status word; LF_ERR_TIMEOUT if a bounded wait expired in a kernel.
+// Waits for the stream and reads the device status word; LF_ERR_TIMEOUT if a bounded wait expired in a kernel.
 lf_status check_status(lf_context* ctx);
 
 // Float32 GEMM on the tensor cores (f32_gemm.cu), batched: out[b][i][j] = act(sum_k A(b, i, k) B(b, j, k) + bias[j]), both operands

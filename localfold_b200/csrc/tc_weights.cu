@@ -110,9 +110,12 @@ struct Preparer {
   lf_context* ctx;
   WeightCursor& cur;
   JobList list{};
+  int64_t most = 0;      // elements of the largest job
   void push(const Job& j) {
     if (cur.dry) return;
     list.j[list.count++] = j;
+    const int64_t elements = (int64_t)j.K * j.n_fill;
+    if (elements > most) most = elements;
     if (list.count == kMaxJobs) flush();
   }
   void image(const float* w, int K, int n_out, int n_pad, int col0, int ld, op16* img, int row0, float scale, const float* gain = nullptr, int n_fill = 0) {
@@ -126,9 +129,12 @@ struct Preparer {
   }
   void flush() {
     if (cur.dry || list.count == 0) return;
-    weight_jobs_kernel<<<dim3(32, list.count), 256, 0, ctx->stream>>>(list);
+    // eight elements a thread of the largest job
+    const int blocks = most / 2048 < 16 ? 16 : most / 2048 > 592 ? 592 : (int)(most / 2048);
+    weight_jobs_kernel<<<dim3(blocks, list.count), 256, 0, ctx->stream>>>(list);
     ctx->launches++;
     list.count = 0;
+    most = 0;
   }
 };
 

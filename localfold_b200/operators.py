@@ -81,20 +81,20 @@ class Device:
         self.ordinal = ordinal
         self.stream = int(self.lib.lf_context_stream(handle) or 0)
         self._finalizer = weakref.finalize(self, self.lib.lf_context_destroy, handle)
-        self._torch_stream = None
-        if stream is None:
-            _own_stream_devices.setdefault(int(ordinal), weakref.WeakSet()).add(self)
+        self._own_stream = stream is None
 
     def wait_for_torch(self):
         """Makes the context's own stream wait (on the device, no host wait) for the work torch has enqueued so
         far on its current stream of this GPU: device tensors handed to a call are usually produced there."""
-        import torch
-        current = torch.cuda.current_stream(self.ordinal)
-        if int(current.cuda_stream) == self.stream:
-            return
-        if self._torch_stream is None:
-            self._torch_stream = torch.cuda.ExternalStream(self.stream, device=self.ordinal)
-        self._torch_stream.wait_event(current.record_event())
+        self.check(self.lib.lf_context_await(self.handle, ctypes.c_void_p(_torch_stream(self.ordinal))))
+
+    def call(self, function, desc, device_space, *extra):
+        """One library call on a descriptor; its device tensors may still be being written by torch."""
+        if device_space and self._own_stream:
+            self.wait_for_torch()
+        res = nat.Result()
+        self.check(function(self.handle, ctypes.byref(desc), *extra, ctypes.byref(res)))
+        return res
 
     def require_current_stream(self, what):
         """Raises unless torch's current stream on this device is the context's stream: collectives and
@@ -144,7 +144,13 @@ class Device:
 
 
 _default_device = None
-_own_stream_devices = {}      # GPU ordinal -> contexts that run on a stream of their own
+
+
+def _torch_stream(ordinal):
+    """torch's current stream on a GPU as a ``cudaStream_t``."""
+    import torch
+    raw = getattr(torch._C, "_cuda_getCurrentRawStream", None)
+    return int(raw(ordinal)) if raw is not None else int(torch.cuda.current_stream(ordinal).cuda_stream)
 
 
 def create_device(ordinal: int = 0) -> Device:
@@ -237,9 +243,6 @@ class _Buffer:
         if self.is_device:
             if not value.is_contiguous():
                 raise ValueError("device tensors must be contiguous")
-            # a context with a stream of its own reads this tensor after torch's pending work on it
-            for ctx in tuple(_own_stream_devices.get(value.device.index, ())):
-                ctx.wait_for_torch()
             self.keep = value
             self.ptr = value.data_ptr()
             self.count = value.numel()
@@ -365,8 +368,7 @@ class _TriangleMultiplicationGpu:
                                     float(input.get("epsilon") or 1e-5),
                                     nat.SPACE_DEVICE if z.is_device else nat.SPACE_HOST, z.dtype,
                                     z.ptr, mask.ptr, obuf.ptr, w.handle)
-            res = nat.Result()
-            dev.check(dev.lib.lf_triangle_multiplication_run(dev.handle, ctypes.byref(desc), ctypes.byref(res)))
+            res = dev.call(dev.lib.lf_triangle_multiplication_run, desc, desc.space == nat.SPACE_DEVICE)
             return _result(dev, res, output)
         finally:
             if owned is not None:
@@ -476,8 +478,7 @@ class AttentionGpu:
                                      float(input.get("epsilon") or 1e-5),
                                      nat.SPACE_DEVICE if act.is_device else nat.SPACE_HOST, act.dtype,
                                      act.ptr, mask.ptr, pair_ptr, obuf.ptr, w.handle)
-            res = nat.Result()
-            dev.check(dev.lib.lf_attention_run(dev.handle, ctypes.byref(desc), ctypes.byref(res)))
+            res = dev.call(dev.lib.lf_attention_run, desc, desc.space == nat.SPACE_DEVICE)
             return _result(dev, res, output)
         finally:
             if owned is not None:
@@ -514,8 +515,7 @@ class Af3GridSelfAttentionGpu:
                                      float(opts.get("epsilon") or 1e-5),
                                      nat.SPACE_DEVICE if p.is_device else nat.SPACE_HOST, p.dtype,
                                      p.ptr, m.ptr, None, obuf.ptr, weights.handle)
-            res = nat.Result()
-            dev.check(dev.lib.lf_attention_run(dev.handle, ctypes.byref(desc), ctypes.byref(res)))
+            res = dev.call(dev.lib.lf_attention_run, desc, desc.space == nat.SPACE_DEVICE)
             return _result(dev, res, output)
         finally:
             if owned is not None:
@@ -554,8 +554,7 @@ class TransitionGpu:
                                       1 if opts.get("residual") else 0, float(input.get("epsilon") or 1e-5),
                                       nat.SPACE_DEVICE if act.is_device else nat.SPACE_HOST, act.dtype,
                                       act.ptr, obuf.ptr, w.handle)
-            res = nat.Result()
-            dev.check(dev.lib.lf_transition_run(dev.handle, ctypes.byref(desc), ctypes.byref(res)))
+            res = dev.call(dev.lib.lf_transition_run, desc, desc.space == nat.SPACE_DEVICE)
             return _result(dev, res, output)
         finally:
             if owned is not None:
@@ -586,8 +585,7 @@ class Af3TransitionGpu:
                                       1 if opts.get("residual") else 0, float(opts.get("epsilon") or 1e-5),
                                       nat.SPACE_DEVICE if act.is_device else nat.SPACE_HOST, act.dtype,
                                       act.ptr, obuf.ptr, weights.handle)
-            res = nat.Result()
-            dev.check(dev.lib.lf_transition_run(dev.handle, ctypes.byref(desc), ctypes.byref(res)))
+            res = dev.call(dev.lib.lf_transition_run, desc, desc.space == nat.SPACE_DEVICE)
             return _result(dev, res, output)
         finally:
             if owned is not None:
@@ -637,8 +635,7 @@ class OuterProductMeanGpu:
                                float(input.get("normalizationEpsilon") or 1e-3),
                                nat.SPACE_DEVICE if act.is_device else nat.SPACE_HOST, obuf.dtype,
                                act.ptr, mask.ptr, obuf.ptr, w.handle, 1 if input.get("biasAfterNorm") else 0)
-            res = nat.Result()
-            dev.check(dev.lib.lf_outer_product_mean_run(dev.handle, ctypes.byref(desc), ctypes.byref(res)))
+            res = dev.call(dev.lib.lf_outer_product_mean_run, desc, desc.space == nat.SPACE_DEVICE)
             return _result(dev, res, output)
         finally:
             if owned is not None:
@@ -691,8 +688,7 @@ class Af3SingleAttentionGpu:
                                            1 if opts.get("residual") else 0,
                                            nat.SPACE_DEVICE if s.is_device else nat.SPACE_HOST, p.dtype,
                                            s.ptr, p.ptr, m.ptr, obuf.ptr, weights.handle)
-            res = nat.Result()
-            dev.check(dev.lib.lf_single_attention_run(dev.handle, ctypes.byref(desc), ctypes.byref(res)))
+            res = dev.call(dev.lib.lf_single_attention_run, desc, desc.space == nat.SPACE_DEVICE)
             return _result(dev, res, output)
         finally:
             if owned is not None:
@@ -736,8 +732,7 @@ class GlobalColumnAttentionGpu:
                                            1 if opts.get("residual") else 0, float(input.get("epsilon") or 1e-5),
                                            nat.SPACE_DEVICE if act.is_device else nat.SPACE_HOST, act.dtype,
                                            act.ptr, mask.ptr, obuf.ptr, w.handle)
-            res = nat.Result()
-            dev.check(dev.lib.lf_global_column_attention_run(dev.handle, ctypes.byref(desc), ctypes.byref(res)))
+            res = dev.call(dev.lib.lf_global_column_attention_run, desc, desc.space == nat.SPACE_DEVICE)
             return _result(dev, res, output)
         finally:
             if owned is not None:
@@ -787,8 +782,7 @@ class Af3MsaAttentionGpu:
                                         1 if opts.get("residual") else 0,
                                         nat.SPACE_DEVICE if a.is_device else nat.SPACE_HOST, p.dtype,
                                         a.ptr, m.ptr, p.ptr, obuf.ptr, weights.handle)
-            res = nat.Result()
-            dev.check(dev.lib.lf_msa_attention_run(dev.handle, ctypes.byref(desc), ctypes.byref(res)))
+            res = dev.call(dev.lib.lf_msa_attention_run, desc, desc.space == nat.SPACE_DEVICE)
             return _result(dev, res, output)
         finally:
             if owned is not None:
@@ -820,8 +814,7 @@ def distogram_logits(device, pair, tokens, channels, half_logits, bias=None):
         obuf = _Buffer(output)
     desc = nat.DistogramDesc(tokens, channels, bins, nat.SPACE_DEVICE if p.is_device else nat.SPACE_HOST, p.dtype,
                              p.ptr, wb.ptr, None if bb is None else bb.ptr, obuf.ptr)
-    res = nat.Result()
-    dev.check(dev.lib.lf_distogram_logits_run(dev.handle, ctypes.byref(desc), ctypes.byref(res)))
+    res = dev.call(dev.lib.lf_distogram_logits_run, desc, desc.space == nat.SPACE_DEVICE)
     return _result(dev, res, output)
 
 

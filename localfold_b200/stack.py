@@ -61,6 +61,16 @@ class PreparedPairBlock:
             w.close()
 
 
+def _same_shapes(blocks):
+    """Whether the weight objects of a stack all have the first one's tensors: then the others are as valid as it is."""
+    def shapes(value):
+        if isinstance(value, dict):
+            return {k: shapes(v) for k, v in value.items()}
+        return getattr(value, "shape", value if isinstance(value, (int, bool, type(None))) else type(value))
+    first = shapes(blocks[0])
+    return all(shapes(b) == first for b in blocks[1:])
+
+
 class PairStackGpu:
     """The five pair updates of ``n_blocks`` blocks on a resident pair
     (``ExtraMsaPairStackGpu`` without its OuterProductMean:
@@ -108,7 +118,7 @@ class PairStackGpu:
                 raise ValueError("inplace needs a contiguous float32 array")
             target, output = p, pair
         else:
-            output = np.array(pair, np.float32, copy=True).reshape(n, n, c_z)
+            output = np.empty((n, n, c_z), np.float32)
             target = _Buffer(output)
         count = len(self.blocks) - first_block if n_blocks is None else n_blocks
         desc = nat.PairStackDesc(n, c_z, c_hidden, self.blocks[0].heads, self.blocks[0].transition_hidden,
@@ -117,8 +127,8 @@ class PairStackGpu:
                                  nat.SPACE_DEVICE if p.is_device else nat.SPACE_HOST, target.dtype,
                                  target.ptr, m.ptr, self._table, len(self.blocks), first_block, count,
                                  nat.ORDER_TEMPLATE if opts.get("order") == "template" else nat.ORDER_EVOFORMER)
-        res = nat.Result()
-        dev.check(dev.lib.lf_pair_stack_run(dev.handle, ctypes.byref(desc), ctypes.byref(res)))
+        source = ctypes.c_void_p(p.ptr) if target is not p else None      # host arrays: read from the input, written to the output
+        res = dev.call(dev.lib.lf_pair_stack_run_from, desc, p.is_device, source)
         return {"pair": output, "elapsedMilliseconds": float(res.elapsed_ms),
                 "memory": {"peakBytes": int(res.peak_bytes)}, "launches": int(res.launches), "blocks": count}
 
@@ -248,7 +258,6 @@ class EvoformerStackGpu:
                     if input.get("onBlockDone"):
                         input["onBlockDone"](index)
                 stop.record(stream)
-                dev.synchronize()
             finally:
                 dev.synchronize()
                 for block in owned:
@@ -323,25 +332,33 @@ class Af3PairformerStackGpu:
             seq_mask = None
             if single is not None:
                 seq_mask, _ = resident(state["seqMask"], (n,))
-            stack = PairStackGpu(dev).prepare(blocks, cz, cz)
-            single_w = []
-            if single is not None:       # resident weights of the single track, prepared before the first block runs
-                for b in range(first, len(blocks)):
+            def prepare(b):
+                stacks[b] = PairStackGpu(dev).prepare([blocks[b]], cz, cz)
+                if single is not None:
                     t = blocks[b]["singleTransition"]
-                    single_w.append((prepare_single_attention_weights(dev, blocks[b], cs, cz),
-                                     PreparedWeights(dev, nat.WEIGHTS_TRANSITION_AF3,
-                                                     {"channels": cs, "hidden": int(t["transition2"].shape[0])},
-                                                     [t[k] for k in TRANSITION_AF3_ORDER])))
+                    single_w[b] = (prepare_single_attention_weights(dev, blocks[b], cs, cz),
+                                   PreparedWeights(dev, nat.WEIGHTS_TRANSITION_AF3,
+                                                   {"channels": cs, "hidden": int(t["transition2"].shape[0])},
+                                                   [t[k] for k in TRANSITION_AF3_ORDER]))
+
+            stacks, single_w = {}, {}
             launches = 0
             sub = {"precision": opts.get("precision", "f32"), "residual": True}
             start, stop = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
             start.record(stream)
             try:
+                # A block's resident weights are prepared while the GPU works on the block before; when the blocks are not
+                # all of one shape, all of them before the first block runs, so that a wrong tensor is found before any update.
+                if not _same_shapes(blocks):
+                    for b in range(len(blocks)):
+                        prepare(b)
                 for b in range(first, len(blocks)):
-                    r = stack.run(pair, pair_mask, opts, first_block=b, n_blocks=1, dialect=dialect)
+                    if b not in stacks:
+                        prepare(b)
+                    r = stacks[b].run(pair, pair_mask, opts, n_blocks=1, dialect=dialect)
                     launches += r["launches"]
                     if single is not None:
-                        att_w, trn_w = single_w[b - first]
+                        att_w, trn_w = single_w[b]
                         r = Af3SingleAttentionGpu(dev).run(single, pair, seq_mask, {"n": n, "channels": cs, "pairChannels": cz},
                                                            att_w, sub)
                         single.copy_(r["output"])
@@ -351,11 +368,11 @@ class Af3PairformerStackGpu:
                     if opts.get("onBlockDone"):
                         opts["onBlockDone"](b)
                 stop.record(stream)
-                dev.synchronize()
             finally:
                 dev.synchronize()
-                stack.close()
-                for pair_of in single_w:
+                for stack in stacks.values():
+                    stack.close()
+                for pair_of in single_w.values():
                     for w in pair_of:
                         w.close()
             elapsed = start.elapsed_time(stop)
@@ -414,8 +431,8 @@ class Af3MsaStackGpu:
             pair, pair_given = resident(state["pair"], (n, n, cz))
             msa_mask, _ = resident(state["msaMask"], (S, n))
             pair_mask, _ = resident(state["pairMask"], (n, n))
-            prepared = []
-            for w in blocks:      # resident weights of the MSA track, prepared before the first block runs
+            def prepare(b):
+                w = blocks[b]
                 opm = w["outerProductMean"]
                 co = int(opm["outerChannels"])
                 zero = np.zeros(co, np.float32)
@@ -424,20 +441,34 @@ class Af3MsaStackGpu:
                            "rightWeight": opm["rightProjection"], "rightBias": opm.get("rightProjectionBias", zero),
                            "outputWeight": opm["outputW"], "outputBias": opm["outputB"]}
                 t = w["msaTransition"]
-                prepared.append((co,
-                                 PreparedWeights(dev, nat.WEIGHTS_OPM_AF2, {"channels": cm, "hidden": co, "out_channels": cz},
-                                                 [opm_af2[k] for k in OPM_WEIGHT_ORDER]),
-                                 prepare_msa_attention_weights(dev, w["msaAttention1"], cm, cz),
-                                 PreparedWeights(dev, nat.WEIGHTS_TRANSITION_AF3,
-                                                 {"channels": cm, "hidden": int(np.asarray(t["transition2"]).shape[0])},
-                                                 [t[k] for k in TRANSITION_AF3_ORDER])))
-            stack = PairStackGpu(dev).prepare(blocks, cz, cz)
+                prepared[b] = (co,
+                               PreparedWeights(dev, nat.WEIGHTS_OPM_AF2, {"channels": cm, "hidden": co, "out_channels": cz},
+                                               [opm_af2[k] for k in OPM_WEIGHT_ORDER]),
+                               prepare_msa_attention_weights(dev, w["msaAttention1"], cm, cz),
+                               PreparedWeights(dev, nat.WEIGHTS_TRANSITION_AF3,
+                                               {"channels": cm, "hidden": int(np.asarray(t["transition2"]).shape[0])},
+                                               [t[k] for k in TRANSITION_AF3_ORDER]))
+
+            def prepare_pair(b):
+                stacks[b] = PairStackGpu(dev).prepare([blocks[b]], cz, cz)
+
+            prepared, stacks = {}, {}
             sub = {"precision": opts.get("precision", "f32"), "residual": True}
             launches = 0
             start, stop = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
             start.record(stream)
             try:
-                for b, (co, opm_w, att_w, trn_w) in enumerate(prepared):
+                # (resident weights are prepared as in the pairformer stack; a single block's all before it runs)
+                if len(blocks) == 1 or not _same_shapes(blocks):
+                    for b in range(len(blocks)):
+                        prepare(b)
+                        prepare_pair(b)
+                for b in range(len(blocks)):
+                    if b not in prepared:
+                        prepare(b)
+                        prepare_pair(b)
+                    co, opm_w, att_w, trn_w = prepared[b]
+
                     def outer_product():
                         return OuterProductMeanGpu(dev).run({"sequences": S, "length": n, "cM": cm, "cOuter": co, "cZ": cz,
                                                              "activations": msa, "mask": msa_mask, "weights": opm_w,
@@ -457,15 +488,15 @@ class Af3MsaStackGpu:
                     else:
                         launches += outer_product()
                         launches += update_msa()
-                    launches += stack.run(pair, pair_mask, opts, first_block=b, n_blocks=1, dialect=dialect)["launches"]
+                    launches += stacks[b].run(pair, pair_mask, opts, n_blocks=1, dialect=dialect)["launches"]
                     if opts.get("onBlock"):
                         opts["onBlock"](b)
                 stop.record(stream)
-                dev.synchronize()
             finally:
                 dev.synchronize()
-                stack.close()
-                for _, opm_w, att_w, trn_w in prepared:
+                for stack in stacks.values():
+                    stack.close()
+                for _, opm_w, att_w, trn_w in prepared.values():
                     for w in (opm_w, att_w, trn_w):
                         w.close()
             out = {"elapsedMilliseconds": float(start.elapsed_time(stop)), "memory": {"peakBytes": 0}, "launches": launches}
