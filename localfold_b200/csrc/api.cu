@@ -9,13 +9,13 @@
 #include <map>
 #include <mutex>
 
-#include "f32_attention.cuh"
+#include "mma_attention.cuh"
 #include "row_kernels.cuh"
 #include "simt_kernels.cuh"
 #include "tc_kernels.cuh"
 
 namespace {
-void configure_attention_f32();
+void configure_mma_attention();
 }
 
 // ---------------------------------------------------------------------------
@@ -113,11 +113,11 @@ static lf_status context_create(int device_ordinal, void* stream, bool make_stre
     static std::once_flag per_device[64];
     if (device_ordinal < 64)
       std::call_once(per_device[device_ordinal], [] {
-        cudaFuncSetAttribute(rows::center_norm_terms_kernel<float>, cudaFuncAttributeMaxDynamicSharedMemorySize, 512 * 33 * 4);
-        cudaFuncSetAttribute(rows::center_norm_terms_kernel<op16>, cudaFuncAttributeMaxDynamicSharedMemorySize, 512 * 33 * 4);
+        cudaFuncSetAttribute(rows::center_norm_kernel<float, rows::LN_TERMS>, cudaFuncAttributeMaxDynamicSharedMemorySize, 512 * 33 * 4);
+        cudaFuncSetAttribute(rows::center_norm_kernel<op16, rows::LN_HALF>, cudaFuncAttributeMaxDynamicSharedMemorySize, 512 * 33 * 4);
         cudaFuncSetAttribute(rows::global_mean_kernel<float>, cudaFuncAttributeMaxDynamicSharedMemorySize, 16 * 513 * 4);
         cudaFuncSetAttribute(rows::global_mean_kernel<bf16>, cudaFuncAttributeMaxDynamicSharedMemorySize, 16 * 513 * 4);
-        configure_attention_f32();
+        configure_mma_attention();
         cudaGetLastError();
       });
   }
@@ -974,31 +974,37 @@ void sgemm(lf_context* ctx, ArenaCursor& cur, bool ta, bool tb, int epi, int M, 
 #undef SG
 }
 
-// The float32 attention core: terms of q | k | v | gate -> terms of the gated output.
+// The attention core for any head width: terms of q | k | v | gate, or fp16, -> the gated output likewise.
 constexpr int kAttentionSmem = 96 * 1024;      // two blocks an SM
 #define ATTENTION_WIDTHS(X) X(8) X(16) X(24) X(32) X(48) X(64)
-void attention_f32(lf_context* ctx, ArenaCursor& cur, int D, const bf16* qkvg, const float* bias, const float* mask, f32mma::AttentionShape s, bf16* out) {
+template <int TERMS>
+void mma_attention_core(lf_context* ctx, ArenaCursor& cur, int D, const void* qkvg, const void* bias, const float* mask, mma_attention::AttentionShape s,
+                        void* out) {
   // eight warps, or as many as the queries have groups of 16: the groups are spread evenly over the blocks; small query
   // counts put several batch rows into a block
   const int groups = lf_ceil_div(s.Q, 16), tiles = lf_ceil_div(groups, 8);
   s.wq = lf_ceil_div(groups, tiles);
   s.wb = 8 / s.wq < s.batch ? 8 / s.wq : s.batch;
-  while (s.wb > 1 && ((int64_t)tiles * s.heads * lf_ceil_div(s.batch, s.wb) < ctx->sm_count || f32mma::attention_smem(D, s.wb) > kAttentionSmem)) s.wb /= 2;
+  while (s.wb > 1 && ((int64_t)tiles * s.heads * lf_ceil_div(s.batch, s.wb) < ctx->sm_count || mma_attention::attention_smem(D, TERMS, s.wb) > kAttentionSmem))
+    s.wb /= 2;
   const dim3 grid(lf_ceil_div(groups, s.wq), lf_ceil_div(s.batch, s.wb), s.heads);
-  const size_t smem = f32mma::attention_smem(D, s.wb);
-#define ATTENTION_CASE(D_)                                                                                                                          \
-  case D_:                                                                                                                                          \
-    if (bias) LAUNCH(ctx, cur, (f32mma::attention_kernel<D_, true>), grid, 32 * s.wb * s.wq, smem, qkvg, bias, mask, s, out);                        \
-    else LAUNCH(ctx, cur, (f32mma::attention_kernel<D_, false>), grid, 32 * s.wb * s.wq, smem, qkvg, bias, mask, s, out);                            \
+  const size_t smem = mma_attention::attention_smem(D, TERMS, s.wb);
+  const uint16_t* in = (const uint16_t*)qkvg;
+#define ATTENTION_CASE(D_)                                                                                                                             \
+  case D_:                                                                                                                                             \
+    if (bias) LAUNCH(ctx, cur, (mma_attention::attention_kernel<D_, TERMS, true>), grid, 32 * s.wb * s.wq, smem, in, bias, mask, s, (uint16_t*)out);    \
+    else LAUNCH(ctx, cur, (mma_attention::attention_kernel<D_, TERMS, false>), grid, 32 * s.wb * s.wq, smem, in, bias, mask, s, (uint16_t*)out);        \
     break;
   switch (D) { ATTENTION_WIDTHS(ATTENTION_CASE) }
 #undef ATTENTION_CASE
 }
 
-void configure_attention_f32() {
-#define ATTENTION_CASE(D_)                                                                                                                               \
-  cudaFuncSetAttribute(f32mma::attention_kernel<D_, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, kAttentionSmem);   \
-  cudaFuncSetAttribute(f32mma::attention_kernel<D_, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, kAttentionSmem);
+void configure_mma_attention() {
+#define ATTENTION_CASE(D_)                                                                                                              \
+  cudaFuncSetAttribute(mma_attention::attention_kernel<D_, 3, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, kAttentionSmem);   \
+  cudaFuncSetAttribute(mma_attention::attention_kernel<D_, 3, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, kAttentionSmem);  \
+  cudaFuncSetAttribute(mma_attention::attention_kernel<D_, 1, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, kAttentionSmem);   \
+  cudaFuncSetAttribute(mma_attention::attention_kernel<D_, 1, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, kAttentionSmem);
   ATTENTION_WIDTHS(ATTENTION_CASE)
 #undef ATTENTION_CASE
 }
@@ -1081,6 +1087,19 @@ struct Staging {
 
 size_t dtype_size(int dt) { return dt == LF_DTYPE_BF16 ? 2 : 4; }
 
+// 16-bit GEMM on the tensor cores for activations of any width: out[m][n] = sum_k a[m][k] w[n][k], fp16 operands
+// with k contiguous, float32 accumulation, fp16 result (the triangle contraction's kernel on one plane).
+lf_status hgemm(lf_context* ctx, ArenaCursor& cur, const op16* a, const op16* w, op16* out, int64_t M, int N, int K,
+                const float* bias = nullptr, int relu = 0) {
+  if (M > 0x7fffffff) return lf_fail(ctx, LF_ERR_SHAPE, "too many rows for one projection");
+  return tc::contract_gemm(ctx, cur, a, w, out, (int)M, N, K, bias, relu);
+}
+
+// the weights' fp16 [n_out][k] GEMM operands, made when the weights were prepared (null: none for this width)
+const op16* gemm_operand(const lf_weights* w, int slot) {
+  return slot < (int)w->g.size() ? (const op16*)w->g[slot] : nullptr;
+}
+
 // ---- triangle multiplication ----
 struct TriArgs {
   int n, cz, c, incoming, variance, residual, divide;
@@ -1090,10 +1109,9 @@ struct TriArgs {
   const lf_weights* w;
 };
 
-// The widths the fused 16-bit kernels do not take, and float32 mode: every projection as a float32 GEMM on split operands.  The contraction
-// too, or - in 16-bit mode - on fp16 operands a, b, x with float32 accumulation.
+// Float32 mode: every projection and the contraction as a float32 GEMM on split operands.
 template <typename T>
-lf_status tri_generic(lf_context* ctx, ArenaCursor& cur, const TriArgs& a, bool half) {
+lf_status tri_f32(lf_context* ctx, ArenaCursor& cur, const TriArgs& a) {
   const int64_t P = (int64_t)a.n * a.n;
   const int cz = a.cz, c = a.c, n = a.n;
   const auto& f = a.w->f;
@@ -1101,43 +1119,26 @@ lf_status tri_generic(lf_context* ctx, ArenaCursor& cur, const TriArgs& a, bool 
   SplitMatrix none[3];
   if (cur.dry) g = none; else LF_TRY(f32_operands(ctx, a.w, &g));
   const SplitMatrix zn = take_terms(cur, P, cz);
-  const int ld = half ? (n + 15) / 16 * 16 : (n + 7) / 8 * 8;      // (fp16: rows start on 32-byte boundaries)
+  const int ld = (n + 7) / 8 * 8, ldx = (n + 3) / 4 * 4;
   const int64_t plane = (int64_t)n * ld;
   const size_t base = cur.offset;
   float* p4 = cur.take<float>(P * 4 * c);
   const size_t p4_end = cur.offset;
   layer_norm<T, rows::LN_TERMS>(ctx, cur, a.z, P, cz, f[TRI_LN_G], f[TRI_LN_B], a.eps, a.variance, 0, 1, 1, (void*)zn.p, zn.term_stride);
   LF_TRY(tc::gemm_f32(ctx, cur, 0, zn, g[0], (int)P, 4 * c, cz, 1, {p4, nullptr, 4 * c, 0, 0, f[TRI_B4], 4 * c, 0, 0, 0}));
-  float x_scale = 1.0f;
-  const void* x = nullptr;
-  int ldx = ld;
-  if (half) {
-    op16* ga = cur.take<op16>(plane * c);
-    op16* gb = cur.take<op16>(plane * c);
-    op16* xh = cur.take<op16>(plane * c);
-    LAUNCH(ctx, cur, (simt::trimul_gate_kernel<op16>), dim3(lf_ceil_div(P, 32), lf_ceil_div(c, 32)), dim3(32, 8), 0, p4, a.mask, P, c, n, ld, ga, gb);
-    // x is stored as fp16 scaled by a power of two near 1/sqrt(n) so that sums over n terms stay far from the fp16
-    // limits; the centre LayerNorm undoes the scale exactly.
-    x_scale = ldexpf(1.0f, -(int)(0.5f * log2f((float)n)));
-    LF_TRY(tc::contract(ctx, cur, ga, gb, xh, n, ld, c, a.incoming, x_scale));
-    x = xh;
-  } else {
-    SplitMatrix ga, gb;
-    ga.ld = gb.ld = ld;
-    ga.batch_stride = gb.batch_stride = plane;
-    ga.term_stride = gb.term_stride = plane * c;
-    ga.p = cur.take<bf16>(3 * plane * c);
-    gb.p = cur.take<bf16>(3 * plane * c);
-    ldx = (n + 3) / 4 * 4;
-    float* xf = cur.take<float>((int64_t)n * ldx * c);
-    LAUNCH(ctx, cur, rows::trimul_gate_terms_kernel, dim3((unsigned)(n * lf_ceil_div(n, 32)), lf_ceil_div(c, 32)), 256, 0, p4, a.mask, c, n, ld, (bf16*)ga.p,
-           (bf16*)gb.p, ga.term_stride);
-    // outgoing x[i][j] = sum_k a[i][k] b[j][k]; incoming x[i][j] = sum_k b[k][i] a[k][j]
-    const tc::Gemm3Out to{xf, nullptr, ldx, (int64_t)n * ldx, 0, nullptr, 0, 0, 0, 0};
-    if (!a.incoming) LF_TRY(tc::gemm_f32(ctx, cur, 0, ga, gb, n, n, n, c, to));
-    else LF_TRY(tc::gemm_f32(ctx, cur, 1, gb, ga, n, n, n, c, to));
-    x = xf;
-  }
+  SplitMatrix ga, gb;
+  ga.ld = gb.ld = ld;
+  ga.batch_stride = gb.batch_stride = plane;
+  ga.term_stride = gb.term_stride = plane * c;
+  ga.p = cur.take<bf16>(3 * plane * c);
+  gb.p = cur.take<bf16>(3 * plane * c);
+  float* xf = cur.take<float>((int64_t)n * ldx * c);
+  LAUNCH(ctx, cur, rows::trimul_gate_terms_kernel, dim3((unsigned)(n * lf_ceil_div(n, 32)), lf_ceil_div(c, 32)), 256, 0, p4, a.mask, c, n, ld, (bf16*)ga.p,
+         (bf16*)gb.p, ga.term_stride);
+  // outgoing x[i][j] = sum_k a[i][k] b[j][k]; incoming x[i][j] = sum_k b[k][i] a[k][j]
+  const tc::Gemm3Out to{xf, nullptr, ldx, (int64_t)n * ldx, 0, nullptr, 0, 0, 0, 0};
+  if (!a.incoming) LF_TRY(tc::gemm_f32(ctx, cur, 0, ga, gb, n, n, n, c, to));
+  else LF_TRY(tc::gemm_f32(ctx, cur, 1, gb, ga, n, n, n, c, to));
   // p4 is dead: the normalised x and the two outputs take its place where they fit
   const size_t end = cur.offset;
   cur.offset = base;
@@ -1152,13 +1153,8 @@ lf_status tri_generic(lf_context* ctx, ArenaCursor& cur, const TriArgs& a, bool 
   } else cur.offset = end;
   const dim3 tiles((unsigned)(n * lf_ceil_div(n, 32)));
   const size_t smem = (size_t)c * 33 * sizeof(float);
-  const float prescale = (a.divide ? 1.0f / n : 1.0f) / x_scale;
-  if (half)
-    LAUNCH(ctx, cur, (rows::center_norm_terms_kernel<op16>), tiles, 256, smem, (const op16*)x, c, n, ldx, f[TRI_LNO_G], f[TRI_LNO_B], a.eps, a.variance, prescale,
-           (int)xn.ld, (bf16*)xn.p, xn.term_stride);
-  else
-    LAUNCH(ctx, cur, (rows::center_norm_terms_kernel<float>), tiles, 256, smem, (const float*)x, c, n, ldx, f[TRI_LNO_G], f[TRI_LNO_B], a.eps, a.variance, prescale,
-           (int)xn.ld, (bf16*)xn.p, xn.term_stride);
+  LAUNCH(ctx, cur, (rows::center_norm_kernel<float, rows::LN_TERMS>), tiles, 256, smem, xf, c, n, ldx, f[TRI_LNO_G], f[TRI_LNO_B], a.eps, a.variance,
+         a.divide ? 1.0f / n : 1.0f, (int)xn.ld, (void*)xn.p, xn.term_stride);
   LF_TRY(tc::gemm_f32(ctx, cur, 0, xn, g[1], (int)P, cz, c, 1, {proj, nullptr, cz, 0, 0, f[TRI_BZ], cz, 0, 0, 0}));
   LF_TRY(tc::gemm_f32(ctx, cur, 0, zn, g[2], (int)P, cz, cz, 1, {gate, nullptr, cz, 0, 0, f[TRI_BG], cz, 0, 0, 0}));
   finish<T>(ctx, cur, proj, gate, a.residual ? a.z : nullptr, P, cz, 0, 1, 1, a.out);
@@ -1174,17 +1170,49 @@ lf_status tri_bf16(lf_context* ctx, ArenaCursor& cur, const TriArgs& a) {
   op16* gb = cur.take<op16>(plane * c);
   op16* x = cur.take<op16>(plane * c);
   LF_TRY(tc::triangle_project(ctx, cur, a.z, a.act_dtype, a.mask, n, n, ld, a.variance, a.eps, a.w, ga, gb));
-  // (x is scaled as in tri_generic)
+  // x is stored as fp16 scaled by a power of two near 1/sqrt(n) so that sums over n terms stay far from the fp16 limits;
+  // the centre LayerNorm undoes the scale exactly.
   const float xscale = ldexpf(1.0f, -(int)(0.5f * log2f((float)n)));
   LF_TRY(tc::contract(ctx, cur, ga, gb, x, n, ld, c, a.incoming, xscale));
   const float xs = xscale * (a.divide ? (float)n : 1.0f);
   return tc::triangle_output(ctx, cur, x, n, n, ld, a.eps * xs * xs, a.z, a.act_dtype, a.variance, a.eps, a.w, a.residual ? a.z : nullptr, a.out);
 }
 
+// 16-bit path at other widths (whole groups of eight): the projections as fp16 GEMMs, the contraction as above.  64 channels,
+// N = 384: 0.20 ms an update, 0.57 ms with the projections as float32 GEMMs.
+template <typename T>
+lf_status tri_half(lf_context* ctx, ArenaCursor& cur, const TriArgs& a) {
+  const int64_t P = (int64_t)a.n * a.n;
+  const int cz = a.cz, c = a.c, n = a.n, ld = (n + 15) / 16 * 16;
+  const int64_t plane = (int64_t)n * ld;
+  const auto& f = a.w->f;
+  op16* zn = cur.take<op16>(P * cz);
+  op16* p4 = cur.take<op16>(P * 4 * c);
+  op16* ga = cur.take<op16>(plane * c);
+  op16* gb = cur.take<op16>(plane * c);
+  op16* x = cur.take<op16>(plane * c);
+  op16* xn = cur.take<op16>(P * c);
+  op16* proj = cur.take<op16>(P * cz);
+  op16* gate = cur.take<op16>(P * cz);
+  layer_norm<T, rows::LN_HALF>(ctx, cur, a.z, P, cz, f[TRI_LN_G], f[TRI_LN_B], a.eps, a.variance, 0, 1, 1, zn);
+  LF_TRY(hgemm(ctx, cur, zn, gemm_operand(a.w, 0), p4, P, 4 * c, cz, f[TRI_B4]));
+  LAUNCH(ctx, cur, rows::trimul_gate_half_kernel, dim3((unsigned)(n * lf_ceil_div(n, 64)), lf_ceil_div(c, 32)), 256, 0, p4, a.mask, c, n, ld, ga, gb);
+  const float xscale = ldexpf(1.0f, -(int)(0.5f * log2f((float)n)));
+  LF_TRY(tc::contract(ctx, cur, ga, gb, x, n, ld, c, a.incoming, xscale));
+  LAUNCH(ctx, cur, (rows::center_norm_kernel<op16, rows::LN_HALF>), dim3((unsigned)(n * lf_ceil_div(n, 32))), 256, (size_t)c * 33 * sizeof(float), x, c, n, ld,
+         f[TRI_LNO_G], f[TRI_LNO_B], a.eps, a.variance, (a.divide ? 1.0f / n : 1.0f) / xscale, c, (void*)xn, (int64_t)0);
+  LF_TRY(hgemm(ctx, cur, xn, gemm_operand(a.w, 1), proj, P, cz, c, f[TRI_BZ]));
+  LF_TRY(hgemm(ctx, cur, zn, gemm_operand(a.w, 2), gate, P, cz, cz, f[TRI_BG]));
+  LAUNCH(ctx, cur, (rows::finish_gate_half_kernel<T>), lf_ceil_div(P * (cz / 8), 256), 256, 0, proj, gate, a.residual ? (const T*)a.z : (const T*)nullptr,
+         P * (cz / 8), (T*)a.out);
+  return LF_OK;
+}
+
 lf_status tri_dispatch(lf_context* ctx, ArenaCursor& cur, const TriArgs& a, int precision) {
   const bool half = precision == LF_PRECISION_BF16 && tc::contract_supported(a.n, a.c);
   if (half && tc::ln_gemm_supported(a.w)) return tri_bf16(ctx, cur, a);
-  return a.act_dtype == LF_DTYPE_BF16 ? tri_generic<bf16>(ctx, cur, a, half) : tri_generic<float>(ctx, cur, a, half);
+  if (half && a.w->g.size() == 3) return a.act_dtype == LF_DTYPE_BF16 ? tri_half<bf16>(ctx, cur, a) : tri_half<float>(ctx, cur, a);
+  return a.act_dtype == LF_DTYPE_BF16 ? tri_f32<bf16>(ctx, cur, a) : tri_f32<float>(ctx, cur, a);
 }
 
 // ---- attention engine, float32 path ----
@@ -1230,7 +1258,7 @@ lf_status att_f32(lf_context* ctx, ArenaCursor& cur, const AttArgs& a) {
   if (cur.dry) g = none; else LF_TRY(f32_operands(ctx, a.w, &g));
   const SplitMatrix nrm = take_terms(cur, R, c);
   // q | k | v | sigmoid(gate) with heads of D channels, and the pair bias columns when the bias comes from the normalised input
-  const int D = f32_head_width(a.d), HDp = a.heads * D, wide = 4 * HDp + (a.bias_mode == 2 ? a.heads : 0);
+  const int D = head_width(a.d), HDp = a.heads * D, wide = 4 * HDp + (a.bias_mode == 2 ? a.heads : 0);
   const SplitMatrix qkvg = take_terms(cur, R, wide);
   float* bias = a.bias_mode ? cur.take<float>((int64_t)a.heads * a.Q * a.Q) : nullptr;
   const SplitMatrix o = take_terms(cur, R, HDp);
@@ -1242,10 +1270,9 @@ lf_status att_f32(lf_context* ctx, ArenaCursor& cur, const AttArgs& a) {
   else if (a.bias_mode == 2)
     LAUNCH(ctx, cur, rows::bias_columns_kernel, lf_ceil_div((int64_t)a.Q * a.Q, 256), 256, 0, qkvg.p, qkvg.ld, qkvg.term_stride, 4 * HDp, a.Q, a.heads,
            a.bias_swap, bias);
-  attention_f32(ctx, cur, D, qkvg.p, bias, a.mask,
-                f32mma::AttentionShape{a.batch, a.Q, a.heads, a.transpose, a.mask_mode, a.clamp, 1.0f / sqrtf((float)a.d), qkvg.ld, qkvg.term_stride, o.ld,
-                                       o.term_stride, 1, 1},
-                (bf16*)o.p);
+  mma_attention_core<3>(ctx, cur, D, qkvg.p, bias, a.mask,
+                        {a.batch, a.Q, a.heads, a.transpose, a.mask_mode, a.clamp, 1.0f / sqrtf((float)a.d), qkvg.ld, qkvg.term_stride, o.ld, o.term_stride, 0, 0, 1, 1},
+                        (void*)o.p);
   LF_TRY(tc::gemm_f32(ctx, cur, 0, o, g[1], (int)R, c, HDp, 1, {proj, nullptr, c, 0, 0, f[ATT_BO], c, 0, 0, 0}));
   finish<T>(ctx, cur, proj, nullptr, a.residual ? a.act : nullptr, R, c, a.transpose, a.batch, a.Q, a.out);
   return LF_OK;
@@ -1321,19 +1348,6 @@ lf_status att_bf16(lf_context* ctx, ArenaCursor& cur, const AttArgs& a) {
   return LF_OK;
 }
 
-// 16-bit GEMM on the tensor cores for activations of any width: out[m][n] = sum_k a[m][k] w[n][k], fp16 operands
-// with k contiguous, float32 accumulation, fp16 result (the triangle contraction's kernel on one plane).
-lf_status hgemm(lf_context* ctx, ArenaCursor& cur, const op16* a, const op16* w, op16* out, int64_t M, int N, int K,
-                const float* bias = nullptr, int relu = 0) {
-  if (M > 0x7fffffff) return lf_fail(ctx, LF_ERR_SHAPE, "too many rows for one projection");
-  return tc::contract_gemm(ctx, cur, a, w, out, (int)M, N, K, bias, relu);
-}
-
-// the weights' fp16 [n_out][k] GEMM operands, made when the weights were prepared (null: none for this width)
-const op16* gemm_operand(const lf_weights* w, int slot) {
-  return slot < (int)w->g.size() ? (const op16*)w->g[slot] : nullptr;
-}
-
 bool hgemm_supported(const lf_weights* w) { return gemm_operand(w, 0) && gemm_operand(w, 1) && tc::contract_supported(1, 1); }
 
 // 16-bit path for the shapes the fused projection kernel does not take (MSA row attention with pair bias: c_m = 256,
@@ -1382,11 +1396,40 @@ lf_status att_mixed(lf_context* ctx, ArenaCursor& cur, const AttArgs& a) {
   return LF_OK;
 }
 
+// 16-bit path for the head widths (or head counts, or the own pair bias at other widths) that the tcgen05 core does not take: LayerNorm to
+// fp16, q / k / v / gate (and the own pair bias) as one fp16 GEMM, the mma.sync core on fp16 rows, the output projection as a second GEMM.
+template <typename T>
+lf_status att_half(lf_context* ctx, ArenaCursor& cur, const AttArgs& a) {
+  const int64_t R = (int64_t)a.batch * a.Q;
+  const int D = head_width(a.d), HDp = a.heads * D, c = a.ch, ldb = (a.Q + 15) / 16 * 16;
+  const bool own_bias = a.w->has_pair_proj && !a.w->has_pair_norm;
+  const int wide = (4 * HDp + (own_bias ? a.heads : 0) + 7) / 8 * 8;
+  const auto& f = a.w->f;
+  op16* nrm = cur.take<op16>(R * c);
+  op16* qkvg = cur.take<op16>(R * wide);
+  op16* bias = a.bias_mode ? cur.take<op16>((int64_t)a.heads * a.Q * ldb) : nullptr;
+  op16* o = cur.take<op16>(R * HDp);
+  layer_norm<T, rows::LN_HALF>(ctx, cur, a.act, R, c, f[ATT_LN_G], f[ATT_LN_B], a.eps, a.variance, a.transpose, a.batch, a.Q, nrm);
+  LF_TRY(hgemm(ctx, cur, nrm, gemm_operand(a.w, 0), qkvg, R, wide, c, (const float*)a.w->g[2]));
+  if (a.bias_mode == 1) LF_TRY(tc::pair_bias_project(ctx, cur, a.pair, a.pair_dtype, a.Q, a.pair_variance, a.pair_eps, a.heads, a.w, bias, ldb));
+  else if (a.bias_mode == 2)
+    LAUNCH(ctx, cur, rows::bias_columns_half_kernel, lf_ceil_div((int64_t)a.Q * ldb, 256), 256, 0, qkvg, (int64_t)wide, 4 * HDp, a.Q, ldb, a.heads, a.bias_swap, bias);
+  mma_attention_core<1>(ctx, cur, D, qkvg, bias, a.mask,
+                        {a.batch, a.Q, a.heads, a.transpose, a.mask_mode, a.clamp, 1.0f / sqrtf((float)a.d), wide, 0, HDp, 0, 1, ldb, 1, 1}, o);
+  LF_TRY(hgemm(ctx, cur, o, gemm_operand(a.w, 1), nrm, R, c, HDp));      // (the normalised input is dead)
+  LAUNCH(ctx, cur, (simt::finish_half_kernel<T>), lf_ceil_div(R * c / 8, 256), 256, 0, nrm, 1.0f, f[ATT_BO],
+         a.residual ? (const T*)a.act : (const T*)nullptr, R, c, a.transpose, a.batch, a.Q, (T*)a.out);
+  return LF_OK;
+}
+
 lf_status att_dispatch(lf_context* ctx, ArenaCursor& cur, const AttArgs& a, int precision) {
   if (precision == LF_PRECISION_BF16 && a.bias_mode != 1 && a.heads == 4 && a.d == 32 && tc::ln_gemm_supported(a.w)) {
     return a.act_dtype == LF_DTYPE_BF16 ? att_bf16<bf16>(ctx, cur, a) : att_bf16<float>(ctx, cur, a);
   }
-  if (precision == LF_PRECISION_BF16 && a.d == 32 && a.heads % 4 == 0 && hgemm_supported(a.w) &&
+  if (precision == LF_PRECISION_BF16 && a.w->head_form && tc::contract_supported(1, 1) &&
+      (a.bias_mode != 1 || (tc::pair_bias_supported(a.w) && !a.bias_swap)))
+    return a.act_dtype == LF_DTYPE_BF16 ? att_half<bf16>(ctx, cur, a) : att_half<float>(ctx, cur, a);
+  if (precision == LF_PRECISION_BF16 && a.d == 32 && a.heads % 4 == 0 && !a.w->head_form && hgemm_supported(a.w) &&
       (a.bias_mode == 0 || (a.bias_mode == 1 && tc::pair_bias_supported(a.w) && !a.bias_swap))) {
     return a.act_dtype == LF_DTYPE_BF16 ? att_mixed<bf16>(ctx, cur, a) : att_mixed<float>(ctx, cur, a);
   }

@@ -79,10 +79,10 @@ struct SplitMatrix {
 
 // Operands of the float32 GEMM, [n_out][k] terms: made at the first float32 call that uses the weights, kept with them.
 //   triangle: fused projection, output projection, output gate; attention: fused projection with heads padded to
-//   f32_head_width (and the pair bias columns when the bias comes from the normalised input), output projection, and at
+//   head_width (and the pair bias columns when the bias comes from the normalised input), output projection, and at
 //   g[2].p the projection's bias (float32); MSA averaging: values | gate, output projection;
 //   transition: both projections; global attention: key | value | gate, output projection
-constexpr int f32_head_width(int d) { return d <= 32 ? (d + 7) / 8 * 8 : d <= 48 ? 48 : 64; }      // the attention core's instances
+constexpr int head_width(int d) { return d <= 32 ? (d + 7) / 8 * 8 : d <= 48 ? 48 : 64; }      // the attention core's instances
 struct lf_f32_operands {
   std::mutex mutex;
   bool made = false;
@@ -102,6 +102,7 @@ struct lf_weights {
   std::vector<float*> f;     // named by the per-kind enums above
   std::vector<void*> h;      // fp16 repacks (tensor-core path)
   std::vector<void*> g;      // fp16 [n_out][k] operands of the plain tensor-core GEMM (widths the fused kernels do not take)
+  bool head_form = false;    // g is (fused projection with heads padded to head_width and the own pair bias rows, output projection, float32 bias)
   int device = 0;
   void* block = nullptr;     // the one device allocation behind all of them (weight_block_take)
   size_t block_bytes = 0;

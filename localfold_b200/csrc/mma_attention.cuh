@@ -1,11 +1,13 @@
-// Gated attention core in float32, its products on the tensor cores: every float32 operand is taken apart into three
-// bf16 terms (8 + 8 + 8 significand bits, so nothing of it is lost) and a product into the six term products above
-// 2^-24, accumulated in float32.
+// Gated attention core for any head width, its products on the tensor cores.  TERMS = 3, float32: every operand is taken apart into
+// three bf16 terms (8 + 8 + 8 significand bits, so nothing of it is lost) and a product into the six term products above
+// 2^-24, accumulated in float32.  TERMS = 1, 16-bit mode (head widths the tcgen05 core does not take): fp16 operands.
 #pragma once
+
+#include <type_traits>
 
 #include "common.cuh"
 
-namespace f32mma {
+namespace mma_attention {
 
 constexpr float kLog2E = 1.4426950408889634f;
 // 2^x (relative error 2^-22).  exp(l - m) is taken as 2^(l log2(e) - m log2(e)) with one rounding of the exponent, as
@@ -46,6 +48,18 @@ __device__ __forceinline__ void mma16(float (&c)[4], const uint32_t (&a)[4], uin
   asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%0, %1, %2, %3};"
                : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3]) : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
 }
+__device__ __forceinline__ void mma16h(float (&c)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
+  asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%0, %1, %2, %3};"
+               : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3]) : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
+}
+__device__ __forceinline__ void mma8h(float (&c)[4], uint32_t a0, uint32_t a1, uint32_t b0) {
+  asm volatile("mma.sync.aligned.m16n8k8.row.col.f32.f16.f16.f32 {%0, %1, %2, %3}, {%4, %5}, {%6}, {%0, %1, %2, %3};"
+               : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3]) : "r"(a0), "r"(a1), "r"(b0));
+}
+__device__ __forceinline__ uint32_t pack_half(float lo, float hi) {
+  const __half2 h = __floats2half2_rn(lo, hi);
+  return *reinterpret_cast<const uint32_t*>(&h);
+}
 __device__ __forceinline__ void mma8(float (&c)[4], uint32_t a0, uint32_t a1, uint32_t b0) {
   asm volatile("mma.sync.aligned.m16n8k8.row.col.f32.bf16.bf16.f32 {%0, %1, %2, %3}, {%4, %5}, {%6}, {%0, %1, %2, %3};"
                : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3]) : "r"(a0), "r"(a1), "r"(b0));
@@ -76,21 +90,23 @@ struct AttentionShape {
   int batch, Q, heads;
   int transpose, mask_mode, clamp;      // mask_mode 0: logit += 1e9 (m - 1); 1: logit += m > 0 ? 0 : -1e9
   float scale;
-  int64_t ld, term_stride;              // rows and terms of q | k | v | gate, in bf16 elements (multiples of 8)
+  int64_t ld, term_stride;              // rows and terms of q | k | v | gate, in 16-bit elements (multiples of 8)
   int64_t ldo, out_stride;              // ... and of the output
+  int gate_logits;                      // fp16: the gate columns hold logits (the projection applies no sigmoid)
+  int ldb;                              // fp16 bias: elements from one query's keys to the next (even)
   int wb, wq;                           // warps of a block: wb batch rows x wq groups of 16 queries
 };
 
 constexpr int AT_KT = 32;                                                     // keys per staged tile
 __host__ __device__ constexpr int at_pitch(int D) { return 8 * ((D / 8) | 1); }      // odd in 16-byte units: ldmatrix rows spread over the banks
-__host__ __device__ constexpr size_t attention_smem(int D, int wb) {
-  return (size_t)2 * wb * (2 * 3 * AT_KT * at_pitch(D) * 2 + AT_KT * 4);
+__host__ __device__ constexpr size_t attention_smem(int D, int terms, int wb) {
+  return (size_t)2 * wb * (2 * terms * AT_KT * at_pitch(D) * 2 + AT_KT * 4);
 }
 
-//   qkvg: [3][rows][ld] = terms of (q | k | v | sigmoid(gate) | ...) in logical row order, a head of each D channels wide
+//   qkvg: [TERMS][rows][ld] = terms of (q | k | v | sigmoid(gate) | ...) in logical row order, a head of each D channels wide
 //         (the projection's weights are padded to the instance's width, so nothing here is conditional on the true one)
-//   bias: [H][Q][Q] or null; mask: indexed b * Q + j, or j * batch + b when transpose
-//   out:  [3][rows][ldo] = softmax(.) v * gate as terms, the operand of the output projection
+//   bias: float32 [H][Q][Q], or fp16 [H][Q][ldb], or null; mask: indexed b * Q + j, or j * batch + b when transpose
+//   out:  [TERMS][rows][ldo] = softmax(.) v * gate as terms, the operand of the output projection
 // A warp owns 16 queries of one (batch row, head); Q and the running output stay in registers in the tensor core's
 // fragment layout, and probabilities become the A operand of P V without leaving them.  The warps of a block share K and
 // V tiles of 32 keys, copied a tile ahead as the projection wrote them.  A row's reference is the maximum of its first
@@ -101,10 +117,13 @@ __host__ __device__ constexpr size_t attention_smem(int D, int wb) {
 // Bound by the latency of a warp's chain (a third of the tensor pipe, half of the issue slots, 16 warps an SM).  Measured,
 // 384 x 384 with 4 heads of 16: 0.51 ms, against 5.06 ms with a warp per query and a shuffle per key and 0.68 ms with
 // four queries a thread on packed FMAs; 203 x 203, 4 x 32: 0.19 ms against 0.98 and 0.24.
-template <int D, bool BIAS>
-__global__ void __launch_bounds__(256, D <= 32 ? 2 : 1)
-attention_kernel(const __nv_bfloat16* __restrict__ qkvg, const float* __restrict__ bias, const float* __restrict__ mask,
-                 const AttentionShape s, __nv_bfloat16* __restrict__ out) {
+template <int D, int TERMS, bool BIAS>
+__global__ void __launch_bounds__(256, TERMS == 3 && D > 32 ? 1 : TERMS == 1 && D <= 16 ? 3 : 2)
+attention_kernel(const uint16_t* __restrict__ qkvg, const void* __restrict__ bias_any, const float* __restrict__ mask,
+                 const AttentionShape s, uint16_t* __restrict__ out) {
+  typedef typename std::conditional<TERMS == 1, __half, float>::type TBias;
+  const TBias* bias = static_cast<const TBias*>(bias_any);
+  constexpr int TOP = TERMS - 1;                    // highest order of a term product that is kept: i + j <= TOP
   constexpr int KT = AT_KT, PITCH = at_pitch(D), NK = D / 16, TAIL = (D / 8) & 1, ND = D / 8;
   constexpr int PLANE = KT * PITCH;                 // bf16 elements of one term of one tile
   extern __shared__ uint4 at_sm[];
@@ -114,21 +133,21 @@ attention_kernel(const __nv_bfloat16* __restrict__ qkvg, const float* __restrict
   const int64_t ld = s.ld;
   const int h = blockIdx.z, b0 = blockIdx.y * s.wb, b = b0 + wb;
   const int q0 = (blockIdx.x * s.wq + wq) * 16;
-  // [2 buffers][wb][K: 3 terms | V: 3 terms][KT][PITCH], then [2][wb][KT] mask terms
-  __nv_bfloat16* kv_s = reinterpret_cast<__nv_bfloat16*>(at_sm);
-  float* mask_s = reinterpret_cast<float*>(kv_s + 2 * s.wb * 6 * PLANE);
+  // [2 buffers][wb][K: TERMS | V: TERMS][KT][PITCH], then [2][wb][KT] mask terms
+  uint16_t* kv_s = reinterpret_cast<uint16_t*>(at_sm);
+  float* mask_s = reinterpret_cast<float*>(kv_s + 2 * s.wb * 2 * TERMS * PLANE);
   const int tiles = (Q + KT - 1) / KT;
   const bool active = b < s.batch && q0 < Q;        // of the warp as a whole
 
   // ---- staging: 16-byte copies of eight channels of one term ----
   auto stage = [&](int tile) {
     const int j0 = tile * KT, buf = tile & 1;
-    for (int u = threadIdx.x; u < s.wb * 6 * KT * ND; u += blockDim.x) {
-      const int e = (u % ND) * 8, j = (u / ND) % KT, part = (u / (ND * KT)) % 6, bb = u / (ND * KT * 6);      // part: K terms, V terms
-      const int which = part / 3, term = part % 3;
+    for (int u = threadIdx.x; u < s.wb * 2 * TERMS * KT * ND; u += blockDim.x) {
+      const int e = (u % ND) * 8, j = (u / ND) % KT, part = (u / (ND * KT)) % (2 * TERMS), bb = u / (ND * KT * 2 * TERMS);      // part: K terms, V terms
+      const int which = part / TERMS, term = part % TERMS;
       const bool ok = j0 + j < Q && b0 + bb < s.batch;
-      const __nv_bfloat16* src = ok ? qkvg + term * s.term_stride + ((int64_t)(b0 + bb) * Q + j0 + j) * ld + (1 + which) * HD + h * D + e : qkvg;
-      copy_async16(kv_s + ((buf * s.wb + bb) * 6 + part) * PLANE + j * PITCH + e, src, ok ? 16 : 0);
+      const uint16_t* src = ok ? qkvg + term * s.term_stride + ((int64_t)(b0 + bb) * Q + j0 + j) * ld + (1 + which) * HD + h * D + e : qkvg;
+      copy_async16(kv_s + ((buf * s.wb + bb) * 2 * TERMS + part) * PLANE + j * PITCH + e, src, ok ? 16 : 0);
     }
     copy_async_commit();
     for (int u = threadIdx.x; u < s.wb * KT; u += blockDim.x) {
@@ -143,14 +162,14 @@ attention_kernel(const __nv_bfloat16* __restrict__ qkvg, const float* __restrict
   };
   stage(0);
 
-  // ---- Q as A fragments of its three terms ----
-  uint32_t qa[3][NK > 0 ? NK : 1][4], qt[3][2];      // qt: the last 8 channels of an odd number of them
+  // ---- Q as A fragments of its terms ----
+  uint32_t qa[TERMS][NK > 0 ? NK : 1][4], qt[TERMS][2];      // qt: the last 8 channels of an odd number of them
   const int row0 = q0 + g, row1 = q0 + g + 8;
   auto q_pair = [&](int row, int term, int e) {
     return active && row < Q ? *reinterpret_cast<const uint32_t*>(qkvg + term * s.term_stride + ((int64_t)b * Q + row) * ld + h * D + e) : 0u;
   };
 #pragma unroll
-  for (int i = 0; i < 3; ++i) {
+  for (int i = 0; i < TERMS; ++i) {
 #pragma unroll
     for (int kk = 0; kk < NK; ++kk)
 #pragma unroll
@@ -162,9 +181,10 @@ attention_kernel(const __nv_bfloat16* __restrict__ qkvg, const float* __restrict
   }
 
   // the bias of a tile's keys: this thread's two rows, eight columns each
-  const bool pairs = (Q & 1) == 0;
-  const float* bias0 = BIAS ? bias + ((int64_t)h * Q + (row0 < Q ? row0 : 0)) * Q + 2 * t : nullptr;
-  const float* bias1 = BIAS ? bias + ((int64_t)h * Q + (row1 < Q ? row1 : 0)) * Q + 2 * t : nullptr;
+  const int64_t bias_ld = TERMS == 1 ? s.ldb : Q;
+  const bool pairs = TERMS == 1 || (Q & 1) == 0;
+  const TBias* bias0 = BIAS ? bias + ((int64_t)h * Q + (row0 < Q ? row0 : 0)) * bias_ld + 2 * t : nullptr;
+  const TBias* bias1 = BIAS ? bias + ((int64_t)h * Q + (row1 < Q ? row1 : 0)) * bias_ld + 2 * t : nullptr;
   float bv[4][4];
   auto load_bias = [&](int j0) {
     if (!BIAS) return;
@@ -172,8 +192,17 @@ attention_kernel(const __nv_bfloat16* __restrict__ qkvg, const float* __restrict
     for (int n = 0; n < 4; ++n) {
       const int j = j0 + n * 8;
       if (pairs && j + 2 * t < Q) {
-        const float2 x = __ldg(reinterpret_cast<const float2*>(bias0 + j)), y = __ldg(reinterpret_cast<const float2*>(bias1 + j));
+        float2 x, y;
+        if constexpr (TERMS == 1) {
+          x = __half22float2(__ldg(reinterpret_cast<const __half2*>(bias0 + j)));
+          y = __half22float2(__ldg(reinterpret_cast<const __half2*>(bias1 + j)));
+        } else {
+          x = __ldg(reinterpret_cast<const float2*>(bias0 + j));
+          y = __ldg(reinterpret_cast<const float2*>(bias1 + j));
+        }
         bv[n][0] = x.x; bv[n][1] = x.y; bv[n][2] = y.x; bv[n][3] = y.y;
+      } else if constexpr (TERMS == 1) {
+        bv[n][0] = bv[n][1] = bv[n][2] = bv[n][3] = 0.f;
       } else {
         bv[n][0] = j + 2 * t < Q ? __ldg(bias0 + j) : 0.f;
         bv[n][1] = j + 2 * t + 1 < Q ? __ldg(bias0 + j + 1) : 0.f;
@@ -188,6 +217,7 @@ attention_kernel(const __nv_bfloat16* __restrict__ qkvg, const float* __restrict
   for (int n = 0; n < ND; ++n)
 #pragma unroll
     for (int e = 0; e < 4; ++e) o[n][e] = 0.f;
+  bool far = false;
   float ref[2] = {0.f, 0.f}, ref2[2] = {0.f, 0.f}, sum[2] = {0.f, 0.f};      // of rows row0, row1; ref2 = ref log2(e)
   if (active) load_bias(0);
   for (int tile = 0; tile < tiles; ++tile) {
@@ -196,8 +226,8 @@ attention_kernel(const __nv_bfloat16* __restrict__ qkvg, const float* __restrict
     if (tile + 1 < tiles) stage(tile + 1);
     if (!active) continue;
     const int buf = tile & 1;
-    const __nv_bfloat16* k_s = kv_s + (buf * s.wb + wb) * 6 * PLANE;
-    const __nv_bfloat16* v_s = k_s + 3 * PLANE;
+    const uint16_t* k_s = kv_s + (buf * s.wb + wb) * 2 * TERMS * PLANE;
+    const uint16_t* v_s = k_s + TERMS * PLANE;
     const float* ms = mask_s + (buf * s.wb + wb) * KT;
     // ---- S = Q K^T for 32 keys (four accumulators in flight): small term products first, the leading one last ----
     float l[4][4];
@@ -206,12 +236,12 @@ attention_kernel(const __nv_bfloat16* __restrict__ qkvg, const float* __restrict
 #pragma unroll
       for (int e = 0; e < 4; ++e) l[n][e] = 0.f;
     {
-      uint32_t kb[3][2][4];
+      uint32_t kb[TERMS][2][4];
       // matrices (keys 0-7, k 0-7), (keys 0-7, k 8-15), (keys 8-15, k 0-7), (keys 8-15, k 8-15) of each 16 keys
-      const __nv_bfloat16* base = k_s + ((lane & 7) + (lane >> 4) * 8) * PITCH + ((lane >> 3) & 1) * 8;
+      const uint16_t* base = k_s + ((lane & 7) + (lane >> 4) * 8) * PITCH + ((lane >> 3) & 1) * 8;
       // the term products below the leading one first, over all channels; the leading ones last
 #pragma unroll
-      for (int pass = 2; pass >= 0; pass -= 2) {
+      for (int pass = TOP; pass >= 0; pass -= 2) {
 #pragma unroll
         for (int kk = 0; kk < NK; ++kk) {
 #pragma unroll
@@ -223,7 +253,10 @@ attention_kernel(const __nv_bfloat16* __restrict__ qkvg, const float* __restrict
 #pragma unroll
             for (int i = 0; i <= order; ++i)
 #pragma unroll
-              for (int n = 0; n < 4; ++n) mma16(l[n], qa[i][kk], kb[order - i][n >> 1][(n & 1) * 2], kb[order - i][n >> 1][(n & 1) * 2 + 1]);
+              for (int n = 0; n < 4; ++n) {
+                const uint32_t b0 = kb[order - i][n >> 1][(n & 1) * 2], b1 = kb[order - i][n >> 1][(n & 1) * 2 + 1];
+                if (TERMS == 1) mma16h(l[n], qa[i][kk], b0, b1); else mma16(l[n], qa[i][kk], b0, b1);
+              }
         }
         if (TAIL) {
           // matrices: keys 0-7, 8-15, 16-23, 24-31 of the last eight channels
@@ -234,7 +267,9 @@ attention_kernel(const __nv_bfloat16* __restrict__ qkvg, const float* __restrict
 #pragma unroll
             for (int i = 0; i <= order; ++i)
 #pragma unroll
-              for (int n = 0; n < 4; ++n) mma8(l[n], qt[i][0], qt[i][1], kb[order - i][0][n]);
+              for (int n = 0; n < 4; ++n) {
+                if (TERMS == 1) mma8h(l[n], qt[i][0], qt[i][1], kb[order - i][0][n]); else mma8(l[n], qt[i][0], qt[i][1], kb[order - i][0][n]);
+              }
         }
       }
     }
@@ -264,9 +299,13 @@ attention_kernel(const __nv_bfloat16* __restrict__ qkvg, const float* __restrict
       m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, 1));
       return fmaxf(m, __shfl_xor_sync(0xffffffffu, m, 2));
     };
+    // a reference of a masked row is near -1e9, where its product with log2(e) is rounded to whole powers of two: such
+    // rows subtract first
+    auto update_far = [&]() { far = __any_sync(0xffffffffu, fabsf(ref[0]) > 65536.f || fabsf(ref[1]) > 65536.f); };
     if (tile == 0) {
 #pragma unroll
       for (int r = 0; r < 2; ++r) { ref[r] = row_max(r); ref2[r] = ref[r] * kLog2E; }      // key 0 exists: finite
+      update_far();
     }
     float p[4][4], ps[2];
     auto exponentials = [&]() {
@@ -274,7 +313,8 @@ attention_kernel(const __nv_bfloat16* __restrict__ qkvg, const float* __restrict
 #pragma unroll
       for (int n = 0; n < 4; ++n) {
 #pragma unroll
-        for (int e = 0; e < 4; ++e) p[n][e] = exp2_(fmaf(l[n][e], kLog2E, -ref2[e >> 1]));
+        for (int e = 0; e < 4; ++e)
+          p[n][e] = exp2_(far ? (l[n][e] - ref[e >> 1]) * kLog2E : fmaf(l[n][e], kLog2E, -ref2[e >> 1]));
         a[n] = p[n][0] + p[n][1];
         c[n] = p[n][2] + p[n][3];
       }
@@ -282,17 +322,19 @@ attention_kernel(const __nv_bfloat16* __restrict__ qkvg, const float* __restrict
       ps[1] = (c[0] + c[1]) + (c[2] + c[3]);
     };
     exponentials();
-    constexpr float kBig = 1.1529215e18f;      // 2^60
+    constexpr float kBig = TERMS == 1 ? 32768.0f : 1.1529215e18f;      // fp16 probabilities stay in range; 2^60
     if (__any_sync(0xffffffffu, !(ps[0] <= kBig) || !(ps[1] <= kBig))) {
 #pragma unroll
       for (int r = 0; r < 2; ++r) {
-        const float next = fmaxf(ref[r], row_max(r)), next2 = next * kLog2E, c = exp2_(ref2[r] - next2);
+        const float next = fmaxf(ref[r], row_max(r)), next2 = next * kLog2E;
+        const float c = exp2_(far ? (ref[r] - next) * kLog2E : ref2[r] - next2);
         ref[r] = next;
         ref2[r] = next2;
         sum[r] *= c;
 #pragma unroll
         for (int n = 0; n < ND; ++n) { o[n][2 * r] *= c; o[n][2 * r + 1] *= c; }
       }
+      update_far();
       exponentials();
     }
     sum[0] += ps[0];
@@ -305,36 +347,47 @@ attention_kernel(const __nv_bfloat16* __restrict__ qkvg, const float* __restrict
       for (int e = 0; e < 4; ++e) f[n][e] = fc[n][e] = 0.f;
 #pragma unroll
     for (int grp = 0; grp < 2; ++grp) {
-      uint32_t pa[3][4];
+      uint32_t pa[TERMS][4];
 #pragma unroll
-      for (int r = 0; r < 4; ++r) {
-        uint32_t term[3];
-        split3_cut(p[grp * 2 + (r >> 1)][(r & 1) * 2], p[grp * 2 + (r >> 1)][(r & 1) * 2 + 1], term);      // (row0, keys 2t), (row1, same), then keys + 8
+      for (int r = 0; r < 4; ++r) {      // (row0, keys 2t), (row1, same), then keys + 8
+        const float x = p[grp * 2 + (r >> 1)][(r & 1) * 2], y = p[grp * 2 + (r >> 1)][(r & 1) * 2 + 1];
+        if constexpr (TERMS == 1) pa[0][r] = pack_half(x, y);
+        else {
+          uint32_t term[3];
+          split3_cut(x, y, term);
 #pragma unroll
-        for (int i = 0; i < 3; ++i) pa[i][r] = term[i];
+          for (int i = 0; i < 3; ++i) pa[i][r] = term[i];
+        }
       }
 #pragma unroll
       for (int np = 0; np < ND; np += 2) {
-        uint32_t vb[3][4];
+        uint32_t vb[TERMS][4];
 #pragma unroll
-        for (int i = 0; i < 3; ++i) {
-          const __nv_bfloat16* base = v_s + i * PLANE + (grp * 16 + (lane & 15)) * PITCH + np * 8;
+        for (int i = 0; i < TERMS; ++i) {
+          const uint16_t* base = v_s + i * PLANE + (grp * 16 + (lane & 15)) * PITCH + np * 8;
           if (np + 1 < ND) ldmatrix4<true>(vb[i], base + (lane >> 4) * 8);
           else ldmatrix2<true>(vb[i][0], vb[i][1], base);
         }
+        if constexpr (TERMS == 1) {
+          mma16h(o[np], pa[0], vb[0][0], vb[0][1]);
+          if (np + 1 < ND) mma16h(o[np + 1], pa[0], vb[0][2], vb[0][3]);
+        } else {
 #pragma unroll
-        for (int order = 2; order >= 0; --order)
+          for (int order = TOP; order >= 0; --order)
 #pragma unroll
-          for (int i = 0; i <= order; ++i) {
-            mma16(order ? fc[np] : f[np], pa[i], vb[order - i][0], vb[order - i][1]);
-            if (np + 1 < ND) mma16(order ? fc[np + 1] : f[np + 1], pa[i], vb[order - i][2], vb[order - i][3]);
-          }
+            for (int i = 0; i <= order; ++i) {
+              mma16(order ? fc[np] : f[np], pa[i], vb[order - i][0], vb[order - i][1]);
+              if (np + 1 < ND) mma16(order ? fc[np + 1] : f[np + 1], pa[i], vb[order - i][2], vb[order - i][3]);
+            }
+        }
       }
     }
+    if (TERMS > 1) {
 #pragma unroll
     for (int n = 0; n < ND; ++n)
 #pragma unroll
       for (int e = 0; e < 4; ++e) o[n][e] += f[n][e] + fc[n][e];
+    }
   }
   if (!active) return;
 #pragma unroll
@@ -344,23 +397,29 @@ attention_kernel(const __nv_bfloat16* __restrict__ qkvg, const float* __restrict
     const int row = r ? row1 : row0;
     if (row >= Q) continue;
     const float inv = 1.0f / sum[r];
-    const __nv_bfloat16* gate = qkvg + ((int64_t)b * Q + row) * ld + 3 * HD + h * D + 2 * t;
-    __nv_bfloat16* dst = out + ((int64_t)b * Q + row) * s.ldo + h * D + 2 * t;
+    const uint16_t* gate = qkvg + ((int64_t)b * Q + row) * ld + 3 * HD + h * D + 2 * t;
+    uint16_t* dst = out + ((int64_t)b * Q + row) * s.ldo + h * D + 2 * t;
 #pragma unroll
     for (int n = 0; n < ND; ++n) {
-      float gx = 0.f, gy = 0.f;
+      if constexpr (TERMS == 1) {
+        float2 g2 = __half22float2(*reinterpret_cast<const __half2*>(gate + n * 8));
+        if (s.gate_logits) { g2.x = 1.0f / (1.0f + __expf(-g2.x)); g2.y = 1.0f / (1.0f + __expf(-g2.y)); }
+        *reinterpret_cast<uint32_t*>(dst + n * 8) = pack_half(o[n][2 * r] * inv * g2.x, o[n][2 * r + 1] * inv * g2.y);
+      } else {
+        float gx = 0.f, gy = 0.f;
 #pragma unroll
-      for (int i = 2; i >= 0; --i) {
-        const uint32_t w = *reinterpret_cast<const uint32_t*>(gate + i * s.term_stride + n * 8);
-        gx += __uint_as_float(w << 16);
-        gy += __uint_as_float(w & 0xffff0000u);
+        for (int i = 2; i >= 0; --i) {
+          const uint32_t w = *reinterpret_cast<const uint32_t*>(gate + i * s.term_stride + n * 8);
+          gx += __uint_as_float(w << 16);
+          gy += __uint_as_float(w & 0xffff0000u);
+        }
+        uint32_t term[3];
+        split3(o[n][2 * r] * inv * gx, o[n][2 * r + 1] * inv * gy, term);
+#pragma unroll
+        for (int i = 0; i < 3; ++i) *reinterpret_cast<uint32_t*>(dst + i * s.out_stride + n * 8) = term[i];
       }
-      uint32_t term[3];
-      split3(o[n][2 * r] * inv * gx, o[n][2 * r + 1] * inv * gy, term);
-#pragma unroll
-      for (int i = 0; i < 3; ++i) *reinterpret_cast<uint32_t*>(dst + i * s.out_stride + n * 8) = term[i];
     }
   }
 }
 
-}  // namespace f32mma
+}  // namespace mma_attention

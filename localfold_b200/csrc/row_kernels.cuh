@@ -217,12 +217,12 @@ trimul_gate_terms_kernel(const float* __restrict__ p4, const float* __restrict__
   }
 }
 
-// LayerNorm over the channels of a channel-major x[h][i][ld] -> terms [3][pairs][ldc].  A block takes 32 pairs of one pair
-// row; the tile [c][32] sits in shared memory.
-template <typename TIn>
+// LayerNorm over the channels of a channel-major x[h][i][ld] -> [pairs][ldc] as terms or as fp16.  A block takes 32 pairs of one
+// pair row; the tile [c][32] sits in shared memory.
+template <typename TIn, int OUT>
 __global__ void __launch_bounds__(256)
-center_norm_terms_kernel(const TIn* __restrict__ x, int c, int n, int ld, const float* __restrict__ gamma, const float* __restrict__ beta,
-                         float eps, int variance, float prescale, int ldc, bf16* __restrict__ xn, int64_t term_stride) {
+center_norm_kernel(const TIn* __restrict__ x, int c, int n, int ld, const float* __restrict__ gamma, const float* __restrict__ beta,
+                   float eps, int variance, float prescale, int ldc, void* __restrict__ xn, int64_t term_stride) {
   extern __shared__ float tile[];   // [c][33]
   const int tiles = (n + 31) / 32, i = blockIdx.x / tiles, k0 = (blockIdx.x % tiles) * 32;
   const int tx = threadIdx.x & 31, w = threadIdx.x >> 5;
@@ -244,11 +244,15 @@ center_norm_terms_kernel(const TIn* __restrict__ x, int c, int n, int ld, const 
     inv = inv * (1.5f - 0.5f * (var + eps) * inv * inv);
     const int64_t row = ((int64_t)i * n + k0 + r) * ldc;
     for (int h = tx * 2; h < ldc; h += 64) {
-      uint32_t t[3];
-      split_pair(h < c ? (tile[h * 33 + r] - mean) * inv * gamma[h] + beta[h] : 0.f,
-                 h + 1 < c ? (tile[(h + 1) * 33 + r] - mean) * inv * gamma[h + 1] + beta[h + 1] : 0.f, t);
+      const float v0 = h < c ? (tile[h * 33 + r] - mean) * inv * gamma[h] + beta[h] : 0.f;
+      const float v1 = h + 1 < c ? (tile[(h + 1) * 33 + r] - mean) * inv * gamma[h + 1] + beta[h + 1] : 0.f;
+      if (OUT == LN_HALF) *reinterpret_cast<__half2*>(reinterpret_cast<__half*>(xn) + row + h) = __floats2half2_rn(v0, v1);
+      else {
+        uint32_t t[3];
+        split_pair(v0, v1, t);
 #pragma unroll
-      for (int e = 0; e < 3; ++e) *reinterpret_cast<uint32_t*>(xn + e * term_stride + row + h) = t[e];
+        for (int e = 0; e < 3; ++e) *reinterpret_cast<uint32_t*>(reinterpret_cast<bf16*>(xn) + e * term_stride + row + h) = t[e];
+      }
     }
   }
 }
@@ -280,6 +284,63 @@ __global__ void finish4_kernel(const float* __restrict__ proj, const float* __re
     for (int e = 0; e < 4; ++e) v[e] += x[e];
   }
   store4(out + dst * ch + c, v);
+}
+
+// 16-bit form: fp16 rows (ap | ag | bp | bg), eight channels a load -> fp16 planes [c][n][ld] (c a multiple of 8, ld of 16; zeros
+// past n).  A block turns 64 pairs x 32 channels of one pair row round in shared memory.
+__global__ void __launch_bounds__(256)
+trimul_gate_half_kernel(const __half* __restrict__ p4, const float* __restrict__ mask, int c, int n, int ld, __half* __restrict__ a, __half* __restrict__ b) {
+  __shared__ __half ta[32][72], tb[32][72];
+  const int tiles = (n + 63) / 64, i = blockIdx.x / tiles, k0 = (blockIdx.x % tiles) * 64, h0 = blockIdx.y * 32;
+  {
+    const int r = threadIdx.x >> 2, hg = (threadIdx.x & 3) * 8, k = k0 + r, h = h0 + hg;
+    if (k < n && h < c) {
+      const int64_t p = (int64_t)i * n + k;
+      const __half* row = p4 + p * 4 * c + h;
+      const float m = mask[p];
+      uint4 raw[4];
+#pragma unroll
+      for (int q = 0; q < 4; ++q) raw[q] = *reinterpret_cast<const uint4*>(row + (int64_t)q * c);
+#pragma unroll
+      for (int e = 0; e < 8; ++e) {
+        auto at = [&](int q) { return __half2float(reinterpret_cast<const __half*>(&raw[q])[e]); };
+        ta[hg + e][r] = __float2half_rn(at(0) * sigmoidf_(at(1)) * m);
+        tb[hg + e][r] = __float2half_rn(at(2) * sigmoidf_(at(3)) * m);
+      }
+    } else {
+#pragma unroll
+      for (int e = 0; e < 8; ++e) ta[hg + e][r] = tb[hg + e][r] = __float2half_rn(0.f);
+    }
+  }
+  __syncthreads();
+  const int hh = threadIdx.x >> 3, k8 = (threadIdx.x & 7) * 8, h = h0 + hh;
+  if (h < c && k0 + k8 < ld) {
+    const int64_t o = ((int64_t)h * n + i) * ld + k0 + k8;
+    *reinterpret_cast<uint4*>(a + o) = *reinterpret_cast<const uint4*>(&ta[hh][k8]);
+    *reinterpret_cast<uint4*>(b + o) = *reinterpret_cast<const uint4*>(&tb[hh][k8]);
+  }
+}
+
+// out[r][c] = (resid ? resid[r][c] : 0) + proj[r][c] * sigmoid(gate[r][c]), fp16 projections, eight channels a thread (ch a multiple of 8)
+template <typename TAct>
+__global__ void finish_gate_half_kernel(const __half* __restrict__ proj, const __half* __restrict__ gate, const TAct* __restrict__ resid, int64_t count,
+                                        TAct* __restrict__ out) {
+  const int64_t idx = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (idx >= count) return;
+  const uint4 p = *reinterpret_cast<const uint4*>(proj + idx * 8), g = *reinterpret_cast<const uint4*>(gate + idx * 8);
+  float v[8];
+#pragma unroll
+  for (int e = 0; e < 8; ++e) v[e] = __half2float(reinterpret_cast<const __half*>(&p)[e]) * sigmoidf_(__half2float(reinterpret_cast<const __half*>(&g)[e]));
+  simt::add_store8<TAct>(v, resid ? resid + idx * 8 : nullptr, out + idx * 8);
+}
+
+// fp16 columns col0 .. col0 + heads of rows (i * Q + j) -> bias[h][i][ldb] (zeros past Q), or its transpose when `swap`
+__global__ void bias_columns_half_kernel(const __half* __restrict__ in, int64_t ld, int col0, int Q, int ldb, int heads, int swap, __half* __restrict__ out) {
+  const int64_t idx = (int64_t)blockIdx.x * blockDim.x + threadIdx.x, plane = (int64_t)Q * ldb;
+  if (idx >= plane) return;
+  const uint32_t i = (uint32_t)(idx / ldb), j = (uint32_t)(idx % ldb);
+  const __half* row = in + (swap ? (int64_t)j * Q + i : (int64_t)i * Q + j) * ld + col0;
+  for (int h = 0; h < heads; ++h) out[h * plane + idx] = j < (uint32_t)Q ? row[h] : __float2half_rn(0.f);
 }
 
 // columns col0 .. col0 + heads of rows (i * Q + j) of a terms matrix -> bias[h][i][j], or [h][j][i] when `swap`

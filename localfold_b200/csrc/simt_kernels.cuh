@@ -165,43 +165,6 @@ sgemm_kernel(int M, int N, int K, const float* __restrict__ A, int64_t lda, int6
 }
 
 // ---------------------------------------------------------------------------
-// Triangle multiplication glue.
-// p4: [pairs][4c] = (ap | ag | bp | bg).  a[h][p] = mask[p] * ap * sigmoid(ag), b likewise,
-// channel-major with row stride ld >= n (plane = n*ld elements).  32x32 tile transpose
-// through shared memory so both sides coalesce.
-template <typename TOut>
-__global__ void trimul_gate_kernel(const float* __restrict__ p4, const float* __restrict__ mask,
-                                   int64_t pairs, int c, int n, int ld, TOut* __restrict__ a, TOut* __restrict__ b) {
-  __shared__ float ta[32][33];
-  __shared__ float tb[32][33];
-  int64_t p0 = (int64_t)blockIdx.x * 32;
-  int h0 = blockIdx.y * 32;
-  int tx = threadIdx.x, ty = threadIdx.y;   // 32 x 8
-  for (int r = ty; r < 32; r += 8) {
-    int64_t p = p0 + r;
-    int h = h0 + tx;
-    float va = 0.f, vb = 0.f;
-    if (p < pairs && h < c) {
-      const float* row = p4 + p * 4 * c;
-      float m = mask[p];
-      va = row[h] * sigmoidf_(row[c + h]) * m;
-      vb = row[2 * c + h] * sigmoidf_(row[3 * c + h]) * m;
-    }
-    ta[r][tx] = va;
-    tb[r][tx] = vb;
-  }
-  __syncthreads();
-  for (int r = ty; r < 32; r += 8) {
-    int h = h0 + r;
-    int64_t p = p0 + tx;
-    if (h < c && p < pairs) {
-      int64_t o = ((int64_t)h * n + p / n) * ld + p % n;
-      a[o] = from_f<TOut>(ta[tx][r]);
-      b[o] = from_f<TOut>(tb[tx][r]);
-    }
-  }
-}
-
 // out[dst(r)][c] = (resid ? resid[dst(r)][c] : 0) + proj[r][c] * (gate ? sigmoid(gate[r][c]) : 1)
 // dst(r) follows the transposed-orientation rule of the attention operator.
 template <typename TAct>

@@ -42,14 +42,15 @@ def test_transition_edges(dev, rows, c, hidden, af3):
 
 
 @pytest.mark.parametrize("n,c,incoming", [(1, 8, False), (63, 16, True), (64, 32, False), (65, 24, True), (127, 8, False), (129, 16, True), (200, 12, False), (530, 8, False), (530, 8, True)])
-def test_triangle_edges(dev, n, c, incoming):
+@pytest.mark.parametrize("precision,tol", [("f32", 2e-6), ("bf16", 8e-3)])
+def test_triangle_edges(dev, n, c, incoming, precision, tol):
     import localfold_b200 as lf
     d = syn.draw(3100 + n)
     z, mask, w = d.normal(n, n, c), syn.residue_pair_mask(n, 0.1 if n > 1 else 0.0), syn.af2_triangle_weights(d, c, c)
     op = (lf.TriangleMultiplicationIncomingGpu if incoming else lf.TriangleMultiplicationOutgoingGpu)(dev)
-    got = op.run({"shape": {"length": n, "cZ": c, "cHidden": c}, "z": z, "mask": mask, "weights": w}, {"precision": "f32"})["output"]
+    got = op.run({"shape": {"length": n, "cZ": c, "cHidden": c}, "z": z, "mask": mask, "weights": w}, {"precision": precision})["output"]
     want = oracle.trimul_af2(z, mask, w, c, incoming=incoming)
-    assert oracle.relative_l2(got, want) <= 2e-6
+    assert oracle.relative_l2(got, want) <= tol
 
 
 @pytest.mark.parametrize("S,n,cm,heads,dim", [(1, 1, 16, 2, 8), (3, 31, 64, 8, 8), (130, 33, 64, 8, 8), (17, 129, 40, 3, 12), (9, 65, 24, 2, 5)])
