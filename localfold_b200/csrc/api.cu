@@ -985,10 +985,15 @@ void mma_attention_core(lf_context* ctx, ArenaCursor& cur, int D, const void* qk
   const int groups = lf_ceil_div(s.Q, 16), tiles = lf_ceil_div(groups, 8);
   s.wq = lf_ceil_div(groups, tiles);
   s.wb = 8 / s.wq < s.batch ? 8 / s.wq : s.batch;
-  while (s.wb > 1 && ((int64_t)tiles * s.heads * lf_ceil_div(s.batch, s.wb) < ctx->sm_count || mma_attention::attention_smem(D, TERMS, s.wb) > kAttentionSmem))
-    s.wb /= 2;
+  while (s.wb > 1 && (int64_t)tiles * s.heads * lf_ceil_div(s.batch, s.wb) < ctx->sm_count) s.wb /= 2;
+  // key tiles as long as two blocks' (three in the fp16 form) shared memory allows, up to 128 keys: a barrier a tile
+  auto bytes = [&](int kt) { return mma_attention::attention_smem(D, TERMS, s.wb, kt, (s.Q < 1024 ? lf_ceil_div(s.Q, kt) : lf_ceil_div(1024, kt)) * kt); };
+  s.kt = 128;
+  while (s.kt > 32 && (s.kt >= 2 * s.Q || bytes(s.kt) > (TERMS == 1 ? kAttentionSmem * 2 / 3 : kAttentionSmem))) s.kt /= 2;
+  while (s.wb > 1 && bytes(s.kt) > kAttentionSmem) s.wb /= 2;
+  s.mk = (s.Q < 1024 ? lf_ceil_div(s.Q, s.kt) : lf_ceil_div(1024, s.kt)) * s.kt;
   const dim3 grid(lf_ceil_div(groups, s.wq), lf_ceil_div(s.batch, s.wb), s.heads);
-  const size_t smem = mma_attention::attention_smem(D, TERMS, s.wb);
+  const size_t smem = bytes(s.kt);
   const uint16_t* in = (const uint16_t*)qkvg;
 #define ATTENTION_CASE(D_)                                                                                                                             \
   case D_:                                                                                                                                             \
@@ -1271,7 +1276,7 @@ lf_status att_f32(lf_context* ctx, ArenaCursor& cur, const AttArgs& a) {
     LAUNCH(ctx, cur, rows::bias_columns_kernel, lf_ceil_div((int64_t)a.Q * a.Q, 256), 256, 0, qkvg.p, qkvg.ld, qkvg.term_stride, 4 * HDp, a.Q, a.heads,
            a.bias_swap, bias);
   mma_attention_core<3>(ctx, cur, D, qkvg.p, bias, a.mask,
-                        {a.batch, a.Q, a.heads, a.transpose, a.mask_mode, a.clamp, 1.0f / sqrtf((float)a.d), qkvg.ld, qkvg.term_stride, o.ld, o.term_stride, 0, 0, 1, 1},
+                        {a.batch, a.Q, a.heads, a.transpose, a.mask_mode, a.clamp, 1.0f / sqrtf((float)a.d), qkvg.ld, qkvg.term_stride, o.ld, o.term_stride, 0, 0, 1, 1, 0, 0},
                         (void*)o.p);
   LF_TRY(tc::gemm_f32(ctx, cur, 0, o, g[1], (int)R, c, HDp, 1, {proj, nullptr, c, 0, 0, f[ATT_BO], c, 0, 0, 0}));
   finish<T>(ctx, cur, proj, nullptr, a.residual ? a.act : nullptr, R, c, a.transpose, a.batch, a.Q, a.out);
@@ -1415,7 +1420,7 @@ lf_status att_half(lf_context* ctx, ArenaCursor& cur, const AttArgs& a) {
   else if (a.bias_mode == 2)
     LAUNCH(ctx, cur, rows::bias_columns_half_kernel, lf_ceil_div((int64_t)a.Q * ldb, 256), 256, 0, qkvg, (int64_t)wide, 4 * HDp, a.Q, ldb, a.heads, a.bias_swap, bias);
   mma_attention_core<1>(ctx, cur, D, qkvg, bias, a.mask,
-                        {a.batch, a.Q, a.heads, a.transpose, a.mask_mode, a.clamp, 1.0f / sqrtf((float)a.d), wide, 0, HDp, 0, 1, ldb, 1, 1}, o);
+                        {a.batch, a.Q, a.heads, a.transpose, a.mask_mode, a.clamp, 1.0f / sqrtf((float)a.d), wide, 0, HDp, 0, 1, ldb, 1, 1, 0, 0}, o);
   LF_TRY(hgemm(ctx, cur, o, gemm_operand(a.w, 1), nrm, R, c, HDp));      // (the normalised input is dead)
   LAUNCH(ctx, cur, (simt::finish_half_kernel<T>), lf_ceil_div(R * c / 8, 256), 256, 0, nrm, 1.0f, f[ATT_BO],
          a.residual ? (const T*)a.act : (const T*)nullptr, R, c, a.transpose, a.batch, a.Q, (T*)a.out);
@@ -1492,7 +1497,7 @@ lf_status trn_half(lf_context* ctx, ArenaCursor& cur, const TrnArgs& a) {
     layer_norm<T, rows::LN_HALF_ONE>(ctx, cur, in, count, c, f[TRN_LN_G], f[TRN_LN_B], a.eps, a.variance, 0, 1, 1, nrm);
     if (a.swiglu) {
       LF_TRY(hgemm(ctx, cur, nrm, w1, h1, count, wide, c16));
-      LAUNCH(ctx, cur, simt::hidden_act_half_kernel, lf_ceil_div(count * hd, 256), 256, 0, h1, (const float*)nullptr, count, hd, wide, 1, h2);
+      LAUNCH(ctx, cur, rows::swiglu_half_kernel, dim3(lf_ceil_div(hd / 8, 32), (unsigned)lf_ceil_div(count, 8)), dim3(32, 8), 0, h1, count, hd, h2);
     } else {
       LF_TRY(hgemm(ctx, cur, nrm, w1, h1, count, wide, c16, nullptr, 1));     // ReLU in the GEMM's epilogue
     }
@@ -1721,7 +1726,10 @@ lf_status lf_outer_product_mean_run(lf_context* ctx, const lf_opm_desc* d, lf_re
       layer_norm<float, rows::LN_HALF>(ctx, cur, msa, rows, cm, f[OPM_LN_G], f[OPM_LN_B], d->layer_norm_epsilon, d->variance, 0, 1, 1, nrm16);
       LF_TRY(hgemm(ctx, cur, nrm16, wlr, lr16, rows, 2 * c, cm));
       LAUNCH(ctx, cur, simt::opm_split_half_kernel, lf_ceil_div(rows * c, 256), 256, 0, lr16, f[OPM_BL], f[OPM_BR], mask, rows, c, left16, right16);
-      LAUNCH(ctx, cur, simt::opm_counts_kernel, lf_ceil_div((int64_t)((N + 3) / 4) * N, 256), 256, 0, mask, S, N, counts);
+      // coverage counts[i][j] = sum_s mask[s][i] mask[s][j]: a GEMM on the mask's terms (exact for masks of zeros and ones)
+      const SplitMatrix mt = take_terms(cur, S, N);
+      LAUNCH(ctx, cur, rows::to_terms_kernel, lf_ceil_div((int64_t)S * (mt.ld / 2), 256), 256, 0, mask, (int64_t)S, N, (int)mt.ld, (bf16*)mt.p, mt.term_stride);
+      LF_TRY(tc::gemm_f32(ctx, cur, 1, mt, mt, N, N, S, 1, {counts, nullptr, N, 0, 0, nullptr, 0, 0, 0, 0}));
       for (int i0 = 0; i0 < N; i0 += ni) {
         int cnt = N - i0 < ni ? N - i0 : ni;
         LF_TRY(tc::contract_outer(ctx, cur, left16 + (int64_t)i0 * c, right16, outer16, cnt, N, c, S, outer_scale));
@@ -1859,12 +1867,15 @@ lf_status global_attention(lf_context* ctx, ArenaCursor& cur, const lf_global_at
   LF_TRY(tc::gemm_f32(ctx, cur, 0, nrm, g[0], (int)R, wide, c, 1, {kvg, nullptr, ld, 0, 0, f[GLB_B3], wide, 0, 2 * hd, wide}));
   const bool wide_rows = c > 512;      // more channels than a lane keeps: the sums of the normalised rows, from their terms
   if (wide_rows) LAUNCH(ctx, cur, rows::global_mean_terms_kernel, n, 512, 0, nrm.p, nrm.ld, nrm.term_stride, mask, S, n, c, sums);
+  else if (c == 64 && aligned16(act)) LAUNCH(ctx, cur, (rows::global_mean_rows_kernel<T, 1, 16>), n, 512, 0, (const T*)act, mask, S, n, d->epsilon, d->variance, sums);
+  else if (c == 128 && aligned16(act)) LAUNCH(ctx, cur, (rows::global_mean_rows_kernel<T, 1, 32>), n, 512, 0, (const T*)act, mask, S, n, d->epsilon, d->variance, sums);
   else
     LAUNCH(ctx, cur, (rows::global_mean_kernel<T>), n, 512, (size_t)16 * (c + 1) * sizeof(float), (const T*)act, mask, S, n, c, d->epsilon, d->variance, sums);
   LAUNCH(ctx, cur, rows::global_query_kernel, n, 128, (size_t)c * sizeof(float), sums, wide_rows ? nullptr : f[GLB_LN_G], f[GLB_LN_B], c, HD, 1.0f / sqrtf((float)hd), f[GLB_WQ], q);
-  if (hd <= 8) LAUNCH(ctx, cur, rows::global_attend_kernel<8>, dim3(n, lf_ceil_div(H, 2)), 256, 0, q, kvg, (int64_t)ld, mask, S, n, H, hd, attended);
-  else LAUNCH(ctx, cur, rows::global_attend_kernel<32>, dim3(n, lf_ceil_div(H, 2)), 256, 0, q, kvg, (int64_t)ld, mask, S, n, H, hd, attended);
-  LAUNCH(ctx, cur, rows::global_gate_kernel, lf_ceil_div(R * (gated.ld / 2), 256), 256, 0, kvg, (int64_t)ld, 2 * hd, attended, R, n, HD, (int)gated.ld,
+  if (hd <= 8) LAUNCH(ctx, cur, (rows::global_attend_kernel<8, 4>), dim3(n, lf_ceil_div(H, 4)), 256, 0, q, kvg, (int64_t)ld, mask, S, n, H, hd, attended);
+  else LAUNCH(ctx, cur, (rows::global_attend_kernel<32, 1>), dim3(n, H), 256, 0, q, kvg, (int64_t)ld, mask, S, n, H, hd, attended);
+  const int per = lf_ceil_div((int64_t)n * (gated.ld / 4), 256);
+  LAUNCH(ctx, cur, rows::global_gate_kernel, (unsigned)((int64_t)per * S), 256, 0, kvg, (int64_t)ld, 2 * hd, attended, per, n, HD, (int)gated.ld,
          (bf16*)gated.p, gated.term_stride);
   LF_TRY(tc::gemm_f32(ctx, cur, 0, gated, g[1], (int)R, c, HD, 1, {proj, nullptr, c, 0, 0, f[GLB_BO], c, 0, 0, 0}));
   finish<T>(ctx, cur, proj, nullptr, d->residual ? act : nullptr, R, c, 0, 1, 1, out);

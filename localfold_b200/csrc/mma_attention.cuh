@@ -95,12 +95,14 @@ struct AttentionShape {
   int gate_logits;                      // fp16: the gate columns hold logits (the projection applies no sigmoid)
   int ldb;                              // fp16 bias: elements from one query's keys to the next (even)
   int wb, wq;                           // warps of a block: wb batch rows x wq groups of 16 queries
+  int kt;                               // keys of a staged tile, a multiple of 32
+  int mk;                               // keys whose mask terms are held at a time, a multiple of kt
 };
 
-constexpr int AT_KT = 32;                                                     // keys per staged tile
+constexpr int AT_STEP = 32;                                                   // keys of one step of a warp
 __host__ __device__ constexpr int at_pitch(int D) { return 8 * ((D / 8) | 1); }      // odd in 16-byte units: ldmatrix rows spread over the banks
-__host__ __device__ constexpr size_t attention_smem(int D, int terms, int wb) {
-  return (size_t)2 * wb * (2 * terms * AT_KT * at_pitch(D) * 2 + AT_KT * 4);
+__host__ __device__ constexpr size_t attention_smem(int D, int terms, int wb, int kt, int mk) {
+  return (size_t)wb * (2 * 2 * terms * kt * at_pitch(D) * 2 + mk * 4);
 }
 
 //   qkvg: [TERMS][rows][ld] = terms of (q | k | v | sigmoid(gate) | ...) in logical row order, a head of each D channels wide
@@ -109,7 +111,8 @@ __host__ __device__ constexpr size_t attention_smem(int D, int terms, int wb) {
 //   out:  [TERMS][rows][ldo] = softmax(.) v * gate as terms, the operand of the output projection
 // A warp owns 16 queries of one (batch row, head); Q and the running output stay in registers in the tensor core's
 // fragment layout, and probabilities become the A operand of P V without leaving them.  The warps of a block share K and
-// V tiles of 32 keys, copied a tile ahead as the projection wrote them.  A row's reference is the maximum of its first
+// V tiles of kt keys, copied a tile ahead as the projection wrote them, and step through them 32 keys at a time; mask terms
+// are fetched mk keys at a time (a fetch per tile had the block wait for it at every barrier).  A row's reference is the maximum of its first
 // 32 logits, raised only when exponentials overflow 2^60: no maximum is searched otherwise.  P V of a tile goes into
 // fresh accumulators (the leading term product apart from the others) that are added to the output outside the tensor
 // core, so that whatever the tensor core's own additions lose is of a tile's share, not of the running sum: 2e-7
@@ -124,8 +127,8 @@ attention_kernel(const uint16_t* __restrict__ qkvg, const void* __restrict__ bia
   typedef typename std::conditional<TERMS == 1, __half, float>::type TBias;
   const TBias* bias = static_cast<const TBias*>(bias_any);
   constexpr int TOP = TERMS - 1;                    // highest order of a term product that is kept: i + j <= TOP
-  constexpr int KT = AT_KT, PITCH = at_pitch(D), NK = D / 16, TAIL = (D / 8) & 1, ND = D / 8;
-  constexpr int PLANE = KT * PITCH;                 // bf16 elements of one term of one tile
+  constexpr int KT = AT_STEP, PITCH = at_pitch(D), NK = D / 16, TAIL = (D / 8) & 1, ND = D / 8;
+  const int plane = s.kt * PITCH;                   // elements of one term of one staged tile
   extern __shared__ uint4 at_sm[];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, g = lane >> 2, t = lane & 3;
   const int wb = warp / s.wq, wq = warp % s.wq;
@@ -133,31 +136,39 @@ attention_kernel(const uint16_t* __restrict__ qkvg, const void* __restrict__ bia
   const int64_t ld = s.ld;
   const int h = blockIdx.z, b0 = blockIdx.y * s.wb, b = b0 + wb;
   const int q0 = (blockIdx.x * s.wq + wq) * 16;
-  // [2 buffers][wb][K: TERMS | V: TERMS][KT][PITCH], then [2][wb][KT] mask terms
+  // [2 buffers][wb][K: TERMS | V: TERMS][kt][PITCH], then [wb][mk] mask terms
   uint16_t* kv_s = reinterpret_cast<uint16_t*>(at_sm);
-  float* mask_s = reinterpret_cast<float*>(kv_s + 2 * s.wb * 2 * TERMS * PLANE);
-  const int tiles = (Q + KT - 1) / KT;
+  float* mask_s = reinterpret_cast<float*>(kv_s + 2 * s.wb * 2 * TERMS * plane);
+  const int tiles = (Q + s.kt - 1) / s.kt;
   const bool active = b < s.batch && q0 < Q;        // of the warp as a whole
 
   // ---- staging: 16-byte copies of eight channels of one term ----
   auto stage = [&](int tile) {
-    const int j0 = tile * KT, buf = tile & 1;
-    for (int u = threadIdx.x; u < s.wb * 2 * TERMS * KT * ND; u += blockDim.x) {
-      const int e = (u % ND) * 8, j = (u / ND) % KT, part = (u / (ND * KT)) % (2 * TERMS), bb = u / (ND * KT * 2 * TERMS);      // part: K terms, V terms
-      const int which = part / TERMS, term = part % TERMS;
-      const bool ok = j0 + j < Q && b0 + bb < s.batch;
-      const uint16_t* src = ok ? qkvg + term * s.term_stride + ((int64_t)(b0 + bb) * Q + j0 + j) * ld + (1 + which) * HD + h * D + e : qkvg;
-      copy_async16(kv_s + ((buf * s.wb + bb) * 2 * TERMS + part) * PLANE + j * PITCH + e, src, ok ? 16 : 0);
+    const int j0 = tile * s.kt, buf = tile & 1;
+    for (int u = threadIdx.x; u < s.kt * ND; u += blockDim.x) {      // (key, eight channels), then every batch row, K or V and term
+      const int e = (u % ND) * 8, j = u / ND;
+      for (int bb = 0; bb < s.wb; ++bb) {
+        const bool ok = j0 + j < Q && b0 + bb < s.batch;
+        const uint16_t* src = ok ? qkvg + ((int64_t)(b0 + bb) * Q + j0 + j) * ld + HD + h * D + e : qkvg;
+        uint16_t* dst = kv_s + (buf * s.wb + bb) * 2 * TERMS * plane + j * PITCH + e;
+#pragma unroll
+        for (int which = 0; which < 2; ++which)
+#pragma unroll
+          for (int i = 0; i < TERMS; ++i)
+            copy_async16(dst + (which * TERMS + i) * plane, ok ? src + which * HD + i * s.term_stride : src, ok ? 16 : 0);
+      }
     }
     copy_async_commit();
-    for (int u = threadIdx.x; u < s.wb * KT; u += blockDim.x) {
-      const int j = j0 + u % KT, bb = b0 + u / KT;
+  };
+  auto fetch_mask = [&](int j0) {
+    for (int u = threadIdx.x; u < s.wb * s.mk; u += blockDim.x) {
+      const int j = j0 + u % s.mk, bb = b0 + u / s.mk;
       float term = 0.f;
       if (j < Q && bb < s.batch) {
         const float m = __ldg(mask + (s.transpose ? (int64_t)j * s.batch + bb : (int64_t)bb * Q + j));
         term = s.mask_mode == 0 ? 1e9f * (m - 1.0f) : (m > 0.f ? 0.f : -1e9f);
       }
-      mask_s[buf * s.wb * KT + u] = term;
+      mask_s[u] = term;
     }
   };
   stage(0);
@@ -218,17 +229,26 @@ attention_kernel(const uint16_t* __restrict__ qkvg, const void* __restrict__ bia
 #pragma unroll
     for (int e = 0; e < 4; ++e) o[n][e] = 0.f;
   bool far = false;
+  int mask0 = 0;                                      // first key of the mask terms at hand
   float ref[2] = {0.f, 0.f}, ref2[2] = {0.f, 0.f}, sum[2] = {0.f, 0.f};      // of rows row0, row1; ref2 = ref log2(e)
   if (active) load_bias(0);
   for (int tile = 0; tile < tiles; ++tile) {
     copy_async_wait();
     __syncthreads();                                  // the tile is staged, and nobody reads the other buffer any more
     if (tile + 1 < tiles) stage(tile + 1);
+    if (tile * s.kt % s.mk == 0) {
+      mask0 = tile * s.kt;
+      fetch_mask(mask0);
+      __syncthreads();
+    }
     if (!active) continue;
     const int buf = tile & 1;
-    const uint16_t* k_s = kv_s + (buf * s.wb + wb) * 2 * TERMS * PLANE;
-    const uint16_t* v_s = k_s + TERMS * PLANE;
-    const float* ms = mask_s + (buf * s.wb + wb) * KT;
+#pragma unroll 1
+    for (int step = 0; step < s.kt && tile * s.kt + step < Q; step += KT) {
+    const int key0 = tile * s.kt + step;
+    const uint16_t* k_s = kv_s + (buf * s.wb + wb) * 2 * TERMS * plane + step * PITCH;
+    const uint16_t* v_s = k_s + TERMS * plane;
+    const float* ms = mask_s + wb * s.mk + key0 - mask0;
     // ---- S = Q K^T for 32 keys (four accumulators in flight): small term products first, the leading one last ----
     float l[4][4];
 #pragma unroll
@@ -247,7 +267,7 @@ attention_kernel(const uint16_t* __restrict__ qkvg, const void* __restrict__ bia
 #pragma unroll
           for (int i = 0; i <= pass; ++i)
 #pragma unroll
-            for (int grp = 0; grp < 2; ++grp) ldmatrix4<false>(kb[i][grp], base + i * PLANE + grp * 16 * PITCH + kk * 16);
+            for (int grp = 0; grp < 2; ++grp) ldmatrix4<false>(kb[i][grp], base + i * plane + grp * 16 * PITCH + kk * 16);
 #pragma unroll
           for (int order = pass; order >= (pass ? 1 : 0); --order)        // terms i and order - i
 #pragma unroll
@@ -261,7 +281,7 @@ attention_kernel(const uint16_t* __restrict__ qkvg, const void* __restrict__ bia
         if (TAIL) {
           // matrices: keys 0-7, 8-15, 16-23, 24-31 of the last eight channels
 #pragma unroll
-          for (int i = 0; i <= pass; ++i) ldmatrix4<false>(kb[i][0], k_s + i * PLANE + lane * PITCH + NK * 16);
+          for (int i = 0; i <= pass; ++i) ldmatrix4<false>(kb[i][0], k_s + i * plane + lane * PITCH + NK * 16);
 #pragma unroll
           for (int order = pass; order >= (pass ? 1 : 0); --order)
 #pragma unroll
@@ -284,14 +304,14 @@ attention_kernel(const uint16_t* __restrict__ qkvg, const void* __restrict__ bia
         if (s.clamp) l[n][e] = fminf(fmaxf(l[n][e], -1e8f), 1e8f);
       }
     }
-    if (tile * KT + KT > Q) {                           // past the end: not keys at all
+    if (key0 + KT > Q) {                           // past the end: not keys at all
 #pragma unroll
       for (int n = 0; n < 4; ++n)
 #pragma unroll
         for (int e = 0; e < 4; ++e)
-          if (tile * KT + n * 8 + 2 * t + (e & 1) >= Q) l[n][e] = -INFINITY;
+          if (key0 + n * 8 + 2 * t + (e & 1) >= Q) l[n][e] = -INFINITY;
     }
-    if (BIAS && tile + 1 < tiles) load_bias(tile * KT + KT);      // for the next tile
+    if (BIAS && key0 + KT < Q) load_bias(key0 + KT);      // for the next step
     auto row_max = [&](int r) {
       float m = fmaxf(l[0][2 * r], l[0][2 * r + 1]);
 #pragma unroll
@@ -302,7 +322,7 @@ attention_kernel(const uint16_t* __restrict__ qkvg, const void* __restrict__ bia
     // a reference of a masked row is near -1e9, where its product with log2(e) is rounded to whole powers of two: such
     // rows subtract first
     auto update_far = [&]() { far = __any_sync(0xffffffffu, fabsf(ref[0]) > 65536.f || fabsf(ref[1]) > 65536.f); };
-    if (tile == 0) {
+    if (key0 == 0) {
 #pragma unroll
       for (int r = 0; r < 2; ++r) { ref[r] = row_max(r); ref2[r] = ref[r] * kLog2E; }      // key 0 exists: finite
       update_far();
@@ -310,11 +330,23 @@ attention_kernel(const uint16_t* __restrict__ qkvg, const void* __restrict__ bia
     float p[4][4], ps[2];
     auto exponentials = [&]() {
       float a[4], c[4];
+      // exponents: l log2(e) - ref2, or of rows near -1e9 (l - ref) log2(e) - a pass of its own in front
+      float x[4][4], shift[2] = {-ref2[0], -ref2[1]};
+#pragma unroll
+      for (int n = 0; n < 4; ++n)
+#pragma unroll
+        for (int e = 0; e < 4; ++e) x[n][e] = l[n][e];
+      if (far) {
+        shift[0] = shift[1] = 0.f;
+#pragma unroll
+        for (int n = 0; n < 4; ++n)
+#pragma unroll
+          for (int e = 0; e < 4; ++e) x[n][e] -= ref[e >> 1];
+      }
 #pragma unroll
       for (int n = 0; n < 4; ++n) {
 #pragma unroll
-        for (int e = 0; e < 4; ++e)
-          p[n][e] = exp2_(far ? (l[n][e] - ref[e >> 1]) * kLog2E : fmaf(l[n][e], kLog2E, -ref2[e >> 1]));
+        for (int e = 0; e < 4; ++e) p[n][e] = exp2_(fmaf(x[n][e], kLog2E, shift[e >> 1]));
         a[n] = p[n][0] + p[n][1];
         c[n] = p[n][2] + p[n][3];
       }
@@ -364,7 +396,7 @@ attention_kernel(const uint16_t* __restrict__ qkvg, const void* __restrict__ bia
         uint32_t vb[TERMS][4];
 #pragma unroll
         for (int i = 0; i < TERMS; ++i) {
-          const uint16_t* base = v_s + i * PLANE + (grp * 16 + (lane & 15)) * PITCH + np * 8;
+          const uint16_t* base = v_s + i * plane + (grp * 16 + (lane & 15)) * PITCH + np * 8;
           if (np + 1 < ND) ldmatrix4<true>(vb[i], base + (lane >> 4) * 8);
           else ldmatrix2<true>(vb[i][0], vb[i][1], base);
         }
@@ -387,6 +419,7 @@ attention_kernel(const uint16_t* __restrict__ qkvg, const void* __restrict__ bia
     for (int n = 0; n < ND; ++n)
 #pragma unroll
       for (int e = 0; e < 4; ++e) o[n][e] += f[n][e] + fc[n][e];
+    }
     }
   }
   if (!active) return;

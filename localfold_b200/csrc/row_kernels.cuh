@@ -95,9 +95,10 @@ layer_norm_rows_kernel(const TIn* __restrict__ in, int64_t count, const float* _
     float inv = rsqrtf(var + eps);
     inv = inv * (1.5f - 0.5f * (var + eps) * inv * inv);      // one Newton step: rsqrtf is 2 ulp
     const int64_t row = first + r * GROUPS;
-    if (row >= count) continue;
+    const bool ok = row < count;      // (no lane leaves the loop: the row groups of a warp share its shuffles)
 #pragma unroll
     for (int k = 0; k < NV; ++k) {
+      if (!ok) break;
       const int c = (k * L + l) * 4;
       const float4 g = __ldg(reinterpret_cast<const float4*>(gamma + c)), b = __ldg(reinterpret_cast<const float4*>(beta + c));
       float y[4] = {(v[r][k][0] - mean) * inv * g.x + b.x, (v[r][k][1] - mean) * inv * g.y + b.y, (v[r][k][2] - mean) * inv * g.z + b.z,
@@ -106,7 +107,7 @@ layer_norm_rows_kernel(const TIn* __restrict__ in, int64_t count, const float* _
       else if (OUT == LN_TERMS) store_terms4(reinterpret_cast<bf16*>(out) + row * CH + c, term_stride, y);
       else store4(reinterpret_cast<__half*>(out) + row * (OUT == LN_HALF_ONE ? CH + 16 : CH) + c, y);
     }
-    if (OUT == LN_HALF_ONE && l < 2)
+    if (OUT == LN_HALF_ONE && ok && l < 2)
       *reinterpret_cast<uint4*>(reinterpret_cast<__half*>(out) + row * (CH + 16) + CH + l * 8) = make_uint4(l == 0 ? 0x3c00u : 0u, 0u, 0u, 0u);
   }
 }
@@ -174,6 +175,22 @@ __global__ void swiglu_terms_kernel(const float* __restrict__ wide, int64_t coun
   split_pair(v[0], v[1], t);
 #pragma unroll
   for (int i = 0; i < 3; ++i) *reinterpret_cast<uint32_t*>(out + i * term_stride + row * ld + c) = t[i];
+}
+
+// ... on fp16 (inter a multiple of 8): silu(gate half) * value half, eight channels a thread
+__global__ void swiglu_half_kernel(const __half* __restrict__ wide, int64_t count, int inter, __half* __restrict__ out) {
+  const int c = (blockIdx.x * 32 + threadIdx.x) * 8;
+  const int64_t row = (int64_t)blockIdx.y * 8 + threadIdx.y;
+  if (c >= inter || row >= count) return;
+  const uint4 g = *reinterpret_cast<const uint4*>(wide + row * 2 * inter + c), x = *reinterpret_cast<const uint4*>(wide + row * 2 * inter + inter + c);
+  uint4 o;
+  __half2* h = reinterpret_cast<__half2*>(&o);
+#pragma unroll
+  for (int e = 0; e < 4; ++e) {
+    const float2 a = __half22float2(reinterpret_cast<const __half2*>(&g)[e]), b = __half22float2(reinterpret_cast<const __half2*>(&x)[e]);
+    h[e] = __floats2half2_rn(a.x * sigmoidf_(a.x) * b.x, a.y * sigmoidf_(a.y) * b.y);
+  }
+  *reinterpret_cast<uint4*>(out + row * inter + c) = o;
 }
 
 // p4 rows (ap | ag | bp | bg) -> the contraction's operands a, b = mask * p * sigmoid(g) as terms, channel-major
@@ -512,6 +529,69 @@ global_mean_kernel(const T* __restrict__ act, const float* __restrict__ mask, in
   }
 }
 
+// ... of rows of 4 * NV * L channels: L lanes a row, four rows of each lane group in flight
+template <typename T, int NV, int L>
+__global__ void __launch_bounds__(512)
+global_mean_rows_kernel(const T* __restrict__ act, const float* __restrict__ mask, int S, int n, float eps, int variance, float* __restrict__ sums) {
+  constexpr int CH = 4 * NV * L, GROUPS = 512 / L;
+  __shared__ float part[GROUPS][CH + 1];
+  const int col = blockIdx.x, l = threadIdx.x % L, g = threadIdx.x / L;
+  float acc[NV][4], count = 0.f;
+#pragma unroll
+  for (int k = 0; k < NV; ++k)
+#pragma unroll
+    for (int e = 0; e < 4; ++e) acc[k][e] = 0.f;
+  for (int base = 0; base < S; base += 4 * GROUPS) {      // (the same trips for both row groups of a warp: they share its shuffles)
+    const int s0 = base + g;
+    float v[4][NV][4], m[4];
+#pragma unroll
+    for (int r = 0; r < 4; ++r) {
+      const int s = s0 + r * GROUPS;
+      m[r] = s < S ? __ldg(mask + (int64_t)s * n + col) : 0.f;
+#pragma unroll
+      for (int k = 0; k < NV; ++k) {
+        if (s < S) load4(act + ((int64_t)s * n + col) * CH + (k * L + l) * 4, v[r][k]);
+        else v[r][k][0] = v[r][k][1] = v[r][k][2] = v[r][k][3] = 0.f;
+      }
+    }
+#pragma unroll
+    for (int r = 0; r < 4; ++r) {
+      float sum = 0.f, sq = 0.f;
+#pragma unroll
+      for (int k = 0; k < NV; ++k) sum += (v[r][k][0] + v[r][k][1]) + (v[r][k][2] + v[r][k][3]);
+#pragma unroll
+      for (int o = L / 2; o > 0; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
+      const float mean = sum * (1.0f / CH);
+#pragma unroll
+      for (int k = 0; k < NV; ++k)
+#pragma unroll
+        for (int e = 0; e < 4; ++e) { const float d = variance == 2 ? v[r][k][e] : v[r][k][e] - mean; sq = fmaf(d, d, sq); }
+#pragma unroll
+      for (int o = L / 2; o > 0; o >>= 1) sq += __shfl_xor_sync(0xffffffffu, sq, o);
+      const float var = variance == 2 ? sq * (1.0f / CH) - mean * mean : sq * (1.0f / CH);
+      float inv = rsqrtf(var + eps);
+      inv = inv * (1.5f - 0.5f * (var + eps) * inv * inv) * m[r];
+      count += m[r];
+#pragma unroll
+      for (int k = 0; k < NV; ++k)
+#pragma unroll
+        for (int e = 0; e < 4; ++e) acc[k][e] = fmaf(v[r][k][e] - mean, inv, acc[k][e]);
+    }
+  }
+#pragma unroll
+  for (int k = 0; k < NV; ++k)
+#pragma unroll
+    for (int e = 0; e < 4; ++e) part[g][(k * L + l) * 4 + e] = acc[k][e];
+  if (l == 0) part[g][CH] = count;
+  __syncthreads();
+  for (int ch = threadIdx.x; ch <= CH; ch += 512) {
+    float total = 0.f;
+#pragma unroll
+    for (int k = 0; k < GROUPS; ++k) total += part[k][ch];
+    sums[(int64_t)col * (CH + 1) + ch] = total;
+  }
+}
+
 // ... of rows wider than that, from their normalised terms (gain and offset applied)
 __global__ void __launch_bounds__(512)
 global_mean_terms_kernel(const bf16* __restrict__ nrm, int64_t ld, int64_t term_stride, const float* __restrict__ mask, int S, int n, int c,
@@ -547,33 +627,50 @@ __global__ void global_query_kernel(const float* __restrict__ sums, const float*
 }
 
 // Softmax over the sequences of q(column, head) . k(sequence, column), masked sequences at -1e9, applied to the values; k at
-// columns 0 .. d - 1 and v at d .. 2d - 1 of rows of `ld` floats, d <= D.  One block per column and pair of heads: a key and value row is
-// read once for both; a thread keeps an online softmax of its sequences, the block combines them by shuffles.
-template <int D>
+// columns 0 .. d - 1 and v at d .. 2d - 1 of rows of `ld` floats (a multiple of 4), d <= D.  One block per column and HB heads: a key and
+// value row is read once for all of them, in 16-byte loads where d is whole groups of four; a thread keeps an online
+// softmax of its sequences, the block combines them by shuffles.
+template <int D, int HB>
 __global__ void __launch_bounds__(256)
 global_attend_kernel(const float* __restrict__ q, const float* __restrict__ kv, int64_t ld, const float* __restrict__ mask, int S, int n, int heads,
                      int d, float* __restrict__ attended) {
-  __shared__ float part[8][2][D + 2];
-  const int col = blockIdx.x, h0 = blockIdx.y * 2, lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-  float qv[2][D], acc[2][D], top[2] = {-1e30f, -1e30f}, den[2] = {0.f, 0.f};
+  __shared__ float part[8][HB][D + 2], q_s[HB][D];
+  const int col = blockIdx.x, h0 = blockIdx.y * HB, lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  for (int u = threadIdx.x; u < HB * D; u += 256) {
+    const int h = u / D, e = u % D;
+    q_s[h][e] = e < d && h0 + h < heads ? q[((int64_t)col * heads + h0 + h) * d + e] : 0.f;
+  }
+  __syncthreads();
+  float acc[HB][D], top[HB], den[HB];
 #pragma unroll
-  for (int h = 0; h < 2; ++h)
+  for (int h = 0; h < HB; ++h) {
+    top[h] = -1e30f;
+    den[h] = 0.f;
 #pragma unroll
-    for (int e = 0; e < D; ++e) {
-      qv[h][e] = e < d && h0 + h < heads ? q[((int64_t)col * heads + h0 + h) * d + e] : 0.f;
-      acc[h][e] = 0.f;
-    }
+    for (int e = 0; e < D; ++e) acc[h][e] = 0.f;
+  }
+  const bool vec = (d & 3) == 0;
   for (int s = threadIdx.x; s < S; s += 256) {
     const float* row = kv + ((int64_t)s * n + col) * ld;
     float k[D], v[D];
+    if (vec) {
 #pragma unroll
-    for (int e = 0; e < D; ++e) { k[e] = e < d ? row[e] : 0.f; v[e] = e < d ? row[d + e] : 0.f; }
+      for (int e = 0; e < D; e += 4) {
+        float4 a = make_float4(0.f, 0.f, 0.f, 0.f), b = a;
+        if (e < d) { a = *reinterpret_cast<const float4*>(row + e); b = *reinterpret_cast<const float4*>(row + d + e); }
+        k[e] = a.x; k[e + 1] = a.y; k[e + 2] = a.z; k[e + 3] = a.w;
+        v[e] = b.x; v[e + 1] = b.y; v[e + 2] = b.z; v[e + 3] = b.w;
+      }
+    } else {
+#pragma unroll
+      for (int e = 0; e < D; ++e) { k[e] = e < d ? row[e] : 0.f; v[e] = e < d ? row[d + e] : 0.f; }
+    }
     const bool masked = mask[(int64_t)s * n + col] == 0.f;
 #pragma unroll
-    for (int h = 0; h < 2; ++h) {
+    for (int h = 0; h < HB; ++h) {
       float logit = 0.f;
 #pragma unroll
-      for (int e = 0; e < D; ++e) logit = fmaf(qv[h][e], k[e], logit);
+      for (int e = 0; e < D; ++e) logit = fmaf(q_s[h][e], k[e], logit);
       if (masked) logit = -1e9f;
       const float next = fmaxf(top[h], logit), keep = __expf(top[h] - next), weight = __expf(logit - next);
       top[h] = next;
@@ -583,7 +680,7 @@ global_attend_kernel(const float* __restrict__ q, const float* __restrict__ kv, 
     }
   }
 #pragma unroll
-  for (int h = 0; h < 2; ++h) {
+  for (int h = 0; h < HB; ++h) {
     const float all = simt::warp_max(top[h]), keep = __expf(top[h] - all);
     const float total = warp_sum(den[h] * keep);
     if (lane == 0) { part[w][h][D] = all; part[w][h][D + 1] = total; }
@@ -594,7 +691,7 @@ global_attend_kernel(const float* __restrict__ q, const float* __restrict__ kv, 
     }
   }
   __syncthreads();
-  for (int u = threadIdx.x; u < 2 * d; u += 256) {
+  for (int u = threadIdx.x; u < HB * d; u += 256) {
     const int h = u / d, e = u % d;
     if (h0 + h >= heads) continue;
     float all = -1e30f, total = 0.f, num = 0.f;
@@ -608,20 +705,19 @@ global_attend_kernel(const float* __restrict__ q, const float* __restrict__ kv, 
   }
 }
 
-// gate[r][slot] (columns gate0.. of rows of `ld`) * attended[column of r][slot] -> terms with rows of ldo
-__global__ void global_gate_kernel(const float* __restrict__ kvg, int64_t ld, int gate0, const float* __restrict__ attended, int64_t count, int n, int HD,
-                                   int ldo, bf16* __restrict__ out, int64_t term_stride) {
-  const int64_t idx = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  const int l2 = ldo >> 1;
-  if (idx >= count * l2) return;
-  const int64_t r = idx / l2;
-  const int c = (int)(idx % l2) * 2;
-  const float* g = kvg + r * ld + gate0;
-  const float* x = attended + (r % n) * HD;
-  uint32_t t[3];
-  split_pair(c < HD ? g[c] * x[c] : 0.f, c + 1 < HD ? g[c + 1] * x[c + 1] : 0.f, t);
+// gate[(s, col)][slot] (columns gate0.. of rows of `ld`) * attended[col][slot] -> terms with rows of ldo (a multiple of 8); `per` blocks a sequence
+__global__ void global_gate_kernel(const float* __restrict__ kvg, int64_t ld, int gate0, const float* __restrict__ attended, int per, int n, int HD, int ldo,
+                                   bf16* __restrict__ out, int64_t term_stride) {
+  const uint32_t idx = blockIdx.x % per * blockDim.x + threadIdx.x, l4 = (uint32_t)ldo >> 2;
+  if (idx >= (uint32_t)n * l4) return;
+  const uint32_t col = idx / l4, c = idx % l4 * 4;
+  const int64_t r = (int64_t)(blockIdx.x / per) * n + col;
+  const float* g = kvg + r * ld + gate0 + c;
+  const float* x = attended + (int64_t)col * HD + c;
+  float v[4];
 #pragma unroll
-  for (int e = 0; e < 3; ++e) *reinterpret_cast<uint32_t*>(out + e * term_stride + r * ldo + c) = t[e];
+  for (int e = 0; e < 4; ++e) v[e] = (int)c + e < HD ? g[e] * x[e] : 0.f;
+  store_terms4(out + r * ldo + c, term_stride, v);
 }
 
 }  // namespace rows

@@ -321,25 +321,6 @@ __global__ void finish_half_kernel(const __half* __restrict__ proj, float scale,
   add_store8<TAct>(v, rs, o);
 }
 
-// Transition hidden layer on the fp16 projection h [rows][wide] into out [rows][hidden] (out may be h when wide == hidden):
-//   relu:   out[r][j] = relu(h[r][j] + b[j]), wide = hidden
-//   swiglu: out[r][j] = silu(h[r][j] + b[j]) * (h[r][hidden + j] + b[hidden + j]), wide = 2 hidden
-__global__ void hidden_act_half_kernel(const __half* h, const float* __restrict__ bias, int64_t rows, int hidden, int wide,
-                                       int swiglu, __half* out) {
-  int64_t idx = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (idx >= rows * hidden) return;
-  int64_t r = idx / hidden;
-  int j = (int)(idx % hidden);
-  const __half* row = h + r * wide;
-  float g = __half2float(row[j]) + (bias ? bias[j] : 0.f);
-  if (swiglu) {
-    float v = __half2float(row[hidden + j]) + (bias ? bias[hidden + j] : 0.f);
-    out[idx] = __float2half_rn(g * sigmoidf_(g) * v);
-  } else {
-    out[idx] = __float2half_rn(fmaxf(g, 0.f));
-  }
-}
-
 // fp16 pair bias [heads][Q][ld] (rows padded to ld) -> float32 [heads][Q][Q]
 __global__ void widen_bias_kernel(const __half* __restrict__ in, int heads, int Q, int ld, float* __restrict__ out) {
   int64_t idx = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
@@ -385,28 +366,6 @@ __global__ void opm_split_half_kernel(const __half* __restrict__ lr, const float
   float m = mask[r];
   a16[idx] = __float2half_rn((__half2float(lr[r * 2 * c + a]) + bl[a]) * m);
   b16[idx] = __float2half_rn((__half2float(lr[r * 2 * c + c + a]) + br[a]) * m);
-}
-
-// counts[i][j] = sum_s mask[s][i] mask[s][j]
-__global__ void opm_counts_kernel(const float* __restrict__ mask, int S, int N, float* __restrict__ counts) {
-  // four rows i per thread: a value of column j is loaded once for four products
-  int64_t idx = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  const int n4 = (N + 3) >> 2;
-  if (idx >= (int64_t)n4 * N) return;
-  const int i0 = (int)(idx / N) * 4, j = (int)(idx % N);
-  int ii[4];
-#pragma unroll
-  for (int e = 0; e < 4; ++e) ii[e] = i0 + e < N ? i0 + e : N - 1;
-  float cnt[4] = {0.f, 0.f, 0.f, 0.f};
-  for (int s = 0; s < S; ++s) {
-    const float* row = mask + (int64_t)s * N;
-    const float mj = row[j];
-#pragma unroll
-    for (int e = 0; e < 4; ++e) cnt[e] = fmaf(row[ii[e]], mj, cnt[e]);
-  }
-#pragma unroll
-  for (int e = 0; e < 4; ++e)
-    if (i0 + e < N) counts[(int64_t)(i0 + e) * N + j] = cnt[e];
 }
 
 // out[i][j][z] = (proj[(i - i0) N + j][z] * scale + bout[z]) / (eps + counts[i][j]) (+ resid), or with the bias after
