@@ -1355,47 +1355,44 @@ lf_status att_bf16(lf_context* ctx, ArenaCursor& cur, const AttArgs& a) {
 
 bool hgemm_supported(const lf_weights* w) { return gemm_operand(w, 0) && gemm_operand(w, 1) && tc::contract_supported(1, 1); }
 
+// Whether an output projection can leave as float32 rows straight from its GEMM: float32 activations, updated in place
+// (the rows are added to where they live) or written without a residual.
+template <typename T>
+bool rows_in_place(int residual, const void* act, const void* out, int c) {
+  return sizeof(T) == 4 && (!residual || act == out) && tc::gemm_rows_supported(out, c);
+}
+
 // 16-bit path for the shapes the fused projection kernel does not take (MSA row attention with pair bias: c_m = 256,
-// 8 heads of 32; MSA column attention): LayerNorm to fp16, the q/k/v/gate projection as one tensor-core GEMM, the
-// attention core on four heads at a time (logits, softmax and P V in tensor memory), the output projection as a
-// second GEMM, bias and residual in float32.
+// 8 heads of 32; MSA column attention): LayerNorm to fp16, the q/k/v/gate projection as one tensor-core GEMM that writes the
+// core's pieces, the attention core on four heads at a time (logits, softmax and P V in tensor memory), the output
+// projection as a second GEMM that reads pieces and adds its rows to the activations.
 template <typename T>
 lf_status att_mixed(lf_context* ctx, ArenaCursor& cur, const AttArgs& a) {
   const int64_t R = (int64_t)a.batch * a.Q;
   const int HD = a.heads * a.d, c = a.ch, groups = a.heads / 4;
   const auto& f = a.w->f;
   const int ldb = (a.Q + 15) / 16 * 16;
-  const int64_t RP = (int64_t)a.batch * ldb;
+  const int64_t RP = (int64_t)a.batch * ldb;      // rows padded per batch row
   op16* nrm = cur.take<op16>(R * c);
-  op16* qkvg = cur.take<op16>(R * 4 * HD);
-  op16* o = cur.take<op16>(R * HD);
+  op16* qkvg = cur.take<op16>(4 * groups * RP * 128);      // q | k | v | gate, groups of four heads each
+  op16* o = cur.take<op16>(groups * RP * 128);
   op16* bias16 = a.bias_mode ? cur.take<op16>((int64_t)a.heads * a.Q * ldb) : nullptr;
-  op16* q16 = cur.take<op16>(4 * RP * 128);      // q | k | v | gate of one group of four heads
-  op16* k16 = q16 + RP * 128;
-  op16* v16 = k16 + RP * 128;
-  op16* g16 = v16 + RP * 128;
-  op16* o16 = cur.take<op16>(RP * 128);
   layer_norm<T, rows::LN_HALF>(ctx, cur, a.act, R, c, f[ATT_LN_G], f[ATT_LN_B], a.eps, a.variance, a.transpose, a.batch, a.Q, nrm);
-  LF_TRY(hgemm(ctx, cur, nrm, gemm_operand(a.w, 0), qkvg, R, 4 * HD, c));
-  if (ldb != a.Q && !cur.dry) {
-    // padding rows and columns are read as keys past the end (masked out): they must hold finite values
-    if (bias16) cudaMemsetAsync(bias16, 0, (size_t)a.heads * a.Q * ldb * sizeof(op16), ctx->stream);
-    cudaMemsetAsync(k16, 0, (size_t)RP * 128 * sizeof(op16), ctx->stream);
-    cudaMemsetAsync(v16, 0, (size_t)RP * 128 * sizeof(op16), ctx->stream);
-  }
-  if (a.bias_mode == 1)
+  LF_TRY(tc::gemm_pieces(ctx, cur, nrm, gemm_operand(a.w, 0), qkvg, a.batch, a.Q, ldb, c, HD, f[ATT_B4], 1.0f / sqrtf((float)a.d)));
+  if (a.bias_mode == 1) {
+    // padding columns are read as keys past the end (masked out): they must hold finite values
+    if (ldb != a.Q && !cur.dry) cudaMemsetAsync(bias16, 0, (size_t)a.heads * a.Q * ldb * sizeof(op16), ctx->stream);
     LF_TRY(tc::pair_bias_project(ctx, cur, a.pair, a.pair_dtype, a.Q, a.pair_variance, a.pair_eps, a.heads, a.w, bias16, ldb));
-  const int64_t pieces = (int64_t)a.batch * ((a.Q + 7) / 8) * 128;      // threads of the repack kernels
-  const float qscale = 1.0f / sqrtf((float)a.d);
-  for (int gi = 0; gi < groups; ++gi) {
-    LAUNCH(ctx, cur, simt::rows_to_pieces_kernel<op16>, dim3((unsigned)lf_ceil_div(pieces, 256), 4), 256, 0, qkvg, HD, gi, f[ATT_B4], qscale,
-           a.batch, a.Q, ldb, q16, RP * 128);
-    LF_TRY(tc::attention_core(ctx, cur, q16, k16, v16, g16, bias16 ? bias16 + (int64_t)gi * 4 * a.Q * ldb : nullptr, ldb, a.mask, a.batch,
-                              a.Q, a.transpose, a.mask_mode, a.clamp, o16));
-    LAUNCH(ctx, cur, simt::pieces_to_rows_kernel<op16>, lf_ceil_div(pieces, 256), 256, 0, o16, a.batch, a.Q, ldb, (int64_t)HD, gi * 128, o);
   }
+  for (int gi = 0; gi < groups; ++gi) {
+    auto part = [&](int kind) { return qkvg + ((int64_t)kind * groups + gi) * RP * 128; };
+    LF_TRY(tc::attention_core(ctx, cur, part(0), part(1), part(2), part(3), bias16 ? bias16 + (int64_t)gi * 4 * a.Q * ldb : nullptr, ldb, a.mask, a.batch,
+                              a.Q, a.transpose, a.mask_mode, a.clamp, o + (int64_t)gi * RP * 128));
+  }
+  if (rows_in_place<T>(a.residual, a.act, a.out, c))
+    return tc::gemm_rows_f32(ctx, cur, o, 1, gemm_operand(a.w, 1), (float*)a.out, a.residual, a.batch, a.Q, ldb, a.transpose, c, HD, f[ATT_BO]);
   op16* proj = nrm;   // the normalised input is dead
-  LF_TRY(hgemm(ctx, cur, o, gemm_operand(a.w, 1), proj, R, c, HD));
+  LF_TRY(tc::gemm_rows_half(ctx, cur, o, gemm_operand(a.w, 1), proj, a.batch, a.Q, ldb, c, HD));
   LAUNCH(ctx, cur, (simt::finish_half_kernel<T>), lf_ceil_div(R * c / 8, 256), 256, 0, proj, 1.0f, f[ATT_BO],
          a.residual ? (const T*)a.act : (const T*)nullptr, R, c, a.transpose, a.batch, a.Q, (T*)a.out);
   return LF_OK;
@@ -1421,6 +1418,8 @@ lf_status att_half(lf_context* ctx, ArenaCursor& cur, const AttArgs& a) {
     LAUNCH(ctx, cur, rows::bias_columns_half_kernel, lf_ceil_div((int64_t)a.Q * ldb, 256), 256, 0, qkvg, (int64_t)wide, 4 * HDp, a.Q, ldb, a.heads, a.bias_swap, bias);
   mma_attention_core<1>(ctx, cur, D, qkvg, bias, a.mask,
                         {a.batch, a.Q, a.heads, a.transpose, a.mask_mode, a.clamp, 1.0f / sqrtf((float)a.d), wide, 0, HDp, 0, 1, ldb, 1, 1, 0, 0}, o);
+  if (rows_in_place<T>(a.residual, a.act, a.out, c))
+    return tc::gemm_rows_f32(ctx, cur, o, 0, gemm_operand(a.w, 1), (float*)a.out, a.residual, a.batch, a.Q, 0, a.transpose, c, HDp, f[ATT_BO]);
   LF_TRY(hgemm(ctx, cur, o, gemm_operand(a.w, 1), nrm, R, c, HDp));      // (the normalised input is dead)
   LAUNCH(ctx, cur, (simt::finish_half_kernel<T>), lf_ceil_div(R * c / 8, 256), 256, 0, nrm, 1.0f, f[ATT_BO],
          a.residual ? (const T*)a.act : (const T*)nullptr, R, c, a.transpose, a.batch, a.Q, (T*)a.out);
@@ -1500,6 +1499,10 @@ lf_status trn_half(lf_context* ctx, ArenaCursor& cur, const TrnArgs& a) {
       LAUNCH(ctx, cur, rows::swiglu_half_kernel, dim3(lf_ceil_div(hd / 8, 32), (unsigned)lf_ceil_div(count, 8)), dim3(32, 8), 0, h1, count, hd, h2);
     } else {
       LF_TRY(hgemm(ctx, cur, nrm, w1, h1, count, wide, c16, nullptr, 1));     // ReLU in the GEMM's epilogue
+    }
+    if (rows_in_place<T>(a.residual, a.act, a.out, c)) {
+      LF_TRY(tc::gemm_rows_f32(ctx, cur, h2, 0, w2, (float*)out, a.residual, 1, (int)count, 0, 0, c, hd, f[TRN_B2]));
+      continue;
     }
     LF_TRY(hgemm(ctx, cur, h2, w2, nrm, count, c, hd));
     LAUNCH(ctx, cur, (simt::finish_half_kernel<T>), lf_ceil_div(count * c / 8, 256), 256, 0, nrm, 1.0f, f[TRN_B2],

@@ -227,76 +227,6 @@ __global__ void pair_bias_kernel(const TIn* __restrict__ pair, int Q, int ch, in
   }
 }
 
-// Attention activations between the projections and the tensor-core attention core: 128 channels (four
-// heads of 32) of logical rows (b, q) as fp16 8-row x 8-channel pieces, element (b, q, c) at
-// b*ldq*128 + (q/8)*1024 + (c/8)*64 + (q%8)*8 + c%8.  `src` rows hold q | k | v | gate, HD columns each;
-// blockIdx.y = which of the four, written to dst + blockIdx.y * kind_stride from columns kind*HD + group*128 ..;
-// value = (src + bias[col]) (bias may be null), times qscale for the query, through a sigmoid for the gate.
-template <typename TSrc>
-__global__ void rows_to_pieces_kernel(const TSrc* __restrict__ src, int HD, int group, const float* __restrict__ bias,
-                                      float qscale, int batch, int Q, int ldq, __half* __restrict__ dst, int64_t kind_stride) {
-  // one thread per (row, 8-channel piece); a warp takes 8 rows x 4 pieces, which it writes as 512 contiguous bytes
-  int64_t idx = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  const int q8 = (Q + 7) >> 3;
-  if (idx >= (int64_t)batch * q8 * 128) return;
-  const int kind = blockIdx.y;
-  const int col0 = kind * HD + group * 128;
-  const float scale = kind == 0 ? qscale : 1.0f;
-  const int piece = (int)((idx >> 3) & 15);
-  const int64_t rg = idx >> 7;
-  const int b = (int)(rg / q8), q = (int)(rg % q8) * 8 + (int)(idx & 7);
-  if (q >= Q) return;
-  const int64_t r = (int64_t)b * Q + q;
-  const TSrc* x = src + r * 4 * HD + col0 + piece * 8;
-  float in[8];
-  if (sizeof(TSrc) == 2) {      // fp16 rows: one 16-byte load
-    const uint4 raw = *reinterpret_cast<const uint4*>(x);
-    const __half* hx = reinterpret_cast<const __half*>(&raw);
-#pragma unroll
-    for (int e = 0; e < 8; ++e) in[e] = __half2float(hx[e]);
-  } else {
-#pragma unroll
-    for (int e = 0; e < 8; ++e) in[e] = to_f(x[e]);
-  }
-  float v[8];
-#pragma unroll
-  for (int e = 0; e < 8; ++e) {
-    float t = in[e];
-    if (bias) t += bias[col0 + piece * 8 + e];
-    t *= scale;
-    v[e] = kind == 3 ? sigmoidf_(t) : t;
-  }
-  __half2 h[4];
-#pragma unroll
-  for (int e = 0; e < 4; ++e) h[e] = __floats2half2_rn(v[2 * e], v[2 * e + 1]);
-  __half* out = dst + kind * kind_stride + (int64_t)b * ldq * 128 + (int64_t)(q >> 3) * 1024 + piece * 64 + (q & 7) * 8;
-  *reinterpret_cast<uint4*>(out) = *reinterpret_cast<const uint4*>(h);
-}
-
-// ... and back: the core's output pieces into columns col0 .. col0+127 of rows of `ld` elements
-template <typename TDst>
-__global__ void pieces_to_rows_kernel(const __half* __restrict__ src, int batch, int Q, int ldq, int64_t ld, int col0,
-                                      TDst* __restrict__ dst) {
-  int64_t idx = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;      // the thread order of rows_to_pieces_kernel
-  const int q8 = (Q + 7) >> 3;
-  if (idx >= (int64_t)batch * q8 * 128) return;
-  const int piece = (int)((idx >> 3) & 15);
-  const int64_t rg = idx >> 7;
-  const int b = (int)(rg / q8), q = (int)(rg % q8) * 8 + (int)(idx & 7);
-  if (q >= Q) return;
-  const int64_t r = (int64_t)b * Q + q;
-  const __half* in = src + (int64_t)b * ldq * 128 + (int64_t)(q >> 3) * 1024 + piece * 64 + (q & 7) * 8;
-  uint4 raw = *reinterpret_cast<const uint4*>(in);
-  const __half* h = reinterpret_cast<const __half*>(&raw);
-  TDst* out = dst + r * ld + col0 + piece * 8;
-  if (sizeof(TDst) == 2) {      // fp16 rows: the piece's 16 bytes as they are
-    *reinterpret_cast<uint4*>(out) = raw;
-  } else {
-#pragma unroll
-    for (int e = 0; e < 8; ++e) out[e] = from_f<TDst>(__half2float(h[e]));
-  }
-}
-
 // Glue of the 16-bit GEMM path (activations x weights on the tensor cores through the contraction kernel).
 // out[dst(r)][c] = (resid ? resid[dst(r)][c] : 0) + (proj[r][c] * scale + bias[c]) for an fp16 projection;
 // eight channels per thread (ch a multiple of 8)

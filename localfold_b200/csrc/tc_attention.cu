@@ -150,8 +150,8 @@ flash_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_constant__ C
         else {
           mbar_expect_tx(q_full, 2 * FA_Q_BYTES);
           // coordinates: channel and row inside a piece, piece along channels (8 per head pair), piece along rows, batch row
-          tma_load_5d(sQ, &mapQ, q_full, 0, 0, hp * 8, (2 * qp) * (FA_TILE / 8), b);
-          tma_load_5d(sQ + FA_Q_BYTES, &mapQ, q_full, 0, 0, hp * 8, (2 * qp + 1) * (FA_TILE / 8), b);
+          tma_load_4d(sQ, &mapQ, q_full, 0, hp * 2, (2 * qp) * (FA_TILE / 8), b);
+          tma_load_4d(sQ + FA_Q_BYTES, &mapQ, q_full, 0, hp * 2, (2 * qp + 1) * (FA_TILE / 8), b);
         }
       }
       ok = __shfl_sync(0xffffffffu, ok ? 1 : 0, 0) != 0;
@@ -161,8 +161,8 @@ flash_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_constant__ C
           if (!mbar_wait(&kv_empty[st], ((n_kv / FA_STAGES) & 1) ^ 1, abort_flag, p.status, 21)) ok = false;   // not parked: the ring is only a few tiles deep
           else {
             mbar_expect_tx(&kv_full[st], 2 * FA_KV_BYTES);
-            tma_load_5d(sK + st * FA_KV_BYTES, &mapK, &kv_full[st], 0, 0, hp * 8, t * (FA_KT / 8), b);
-            tma_load_5d(sV + st * FA_KV_BYTES, &mapV, &kv_full[st], 0, 0, hp * 8, t * (FA_KT / 8), b);
+            tma_load_4d(sK + st * FA_KV_BYTES, &mapK, &kv_full[st], 0, hp * 2, t * (FA_KT / 8), b);
+            tma_load_4d(sV + st * FA_KV_BYTES, &mapV, &kv_full[st], 0, hp * 2, t * (FA_KT / 8), b);
           }
         }
         ok = __shfl_sync(0xffffffffu, ok ? 1 : 0, 0) != 0;

@@ -52,19 +52,20 @@ lf_status make_map_f16_3d_ext(lf_context* ctx, CUtensorMap* map, const void* bas
 // Attention activations q, k, v, gate, o: fp16 [batch][ldq][128] stored as 8-row x 8-channel pieces of 128
 // contiguous bytes (element (b, q, c) at b*ldq*128 + (q/8)*1024 + (c/8)*64 + (q%8)*8 + c%8).  A warp whose
 // threads own consecutive rows then writes whole 128-byte lines with 16-byte stores, and a piece is exactly
-// one core matrix of the tensor core's unswizzled operand format.  The map's dimensions are (channel in
-// piece, row in piece, piece along channels, piece along rows, batch row) - strides increasing - and a
-// box of `rows` rows x 64 channels lands in shared memory as [rows/8][8 pieces][8 rows][16 B].
+// one core matrix of the tensor core's unswizzled operand format.  The map's dimensions are (position in four
+// neighbouring pieces, group of four pieces, piece along rows, batch row), and a box of `rows` rows x 64 channels lands in
+// shared memory as [rows/8][8 pieces][8 rows][16 B].  (The innermost dimension is what a copy moves at a time: with the 16 bytes of
+// a piece's row there, a store of 128 x 256 took 9000 cycles.)
 lf_status make_map_tiled_act(lf_context* ctx, CUtensorMap* map, const void* base, int ldq, int batch, int rows) {
   if (!g_encode) return lf_fail(ctx, LF_ERR_CUDA, "cuTensorMapEncodeTiled is not available from this driver");
-  cuuint64_t dims[5] = {8, 8, 16, (cuuint64_t)(ldq / 8), (cuuint64_t)batch};
-  cuuint64_t strides[4] = {16, 128, 2048, (cuuint64_t)ldq * 256};
-  cuuint32_t box[5] = {8, 8, 8, (cuuint32_t)(rows / 8), 1};
-  cuuint32_t estr[5] = {1, 1, 1, 1, 1};
-  CUresult r = g_encode(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 5, const_cast<void*>(base), dims, strides, box, estr,
+  cuuint64_t dims[4] = {256, 4, (cuuint64_t)(ldq / 8), (cuuint64_t)batch};
+  cuuint64_t strides[3] = {512, 2048, (cuuint64_t)ldq * 256};
+  cuuint32_t box[4] = {256, 2, (cuuint32_t)(rows / 8), 1};
+  cuuint32_t estr[4] = {1, 1, 1, 1};
+  CUresult r = g_encode(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 4, const_cast<void*>(base), dims, strides, box, estr,
                         CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
                         CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-  if (r != CUDA_SUCCESS) return lf_fail(ctx, LF_ERR_CUDA, "cuTensorMapEncodeTiled (5-d) failed with code %d", (int)r);
+  if (r != CUDA_SUCCESS) return lf_fail(ctx, LF_ERR_CUDA, "cuTensorMapEncodeTiled (pieces) failed with code %d", (int)r);
   return LF_OK;
 }
 
@@ -124,6 +125,28 @@ lf_status make_map_f32_rows16(lf_context* ctx, CUtensorMap* map, const void* bas
                         CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_64B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
                         CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
   if (r != CUDA_SUCCESS) return lf_fail(ctx, LF_ERR_CUDA, "cuTensorMapEncodeTiled (float32 rows, 16 channels) failed with code %d", (int)r);
+  return LF_OK;
+}
+
+// float32 rows of any width, 128-byte swizzled boxes of 32 channels
+lf_status make_map_f32_any(lf_context* ctx, CUtensorMap* map, const void* base, const uint64_t (&dims)[3], const uint64_t (&strides)[2], const uint32_t (&box)[3]) {
+  if (!g_encode) return lf_fail(ctx, LF_ERR_CUDA, "cuTensorMapEncodeTiled is not available from this driver");
+  cuuint64_t d[3] = {dims[0], dims[1], dims[2]}, st[2] = {strides[0], strides[1]};
+  cuuint32_t b[3] = {box[0], box[1], box[2]}, estr[3] = {1, 1, 1};
+  CUresult r = g_encode(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 3, const_cast<void*>(base), d, st, b, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
+                        CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+  if (r != CUDA_SUCCESS) return lf_fail(ctx, LF_ERR_CUDA, "cuTensorMapEncodeTiled (float32, any width) failed with code %d", (int)r);
+  return LF_OK;
+}
+
+// the outer product mean's sums grouped per pair, fp16 [cnt i][n j][32 a][32 b] seen as (b, a, j, i): boxes of one i, two j (64-byte swizzle)
+lf_status make_map_grouped(lf_context* ctx, CUtensorMap* map, const void* base, uint64_t n, uint64_t cnt) {
+  if (!g_encode) return lf_fail(ctx, LF_ERR_CUDA, "cuTensorMapEncodeTiled is not available from this driver");
+  cuuint64_t dims[4] = {32, 32, n, cnt}, strides[3] = {64, 2048, n * 2048};
+  cuuint32_t box[4] = {32, 32, 2, 1}, estr[4] = {1, 1, 1, 1};
+  CUresult r = g_encode(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 4, const_cast<void*>(base), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
+                        CU_TENSOR_MAP_SWIZZLE_64B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+  if (r != CUDA_SUCCESS) return lf_fail(ctx, LF_ERR_CUDA, "cuTensorMapEncodeTiled (grouped sums) failed with code %d", (int)r);
   return LF_OK;
 }
 
@@ -448,6 +471,7 @@ void configure_once() {
     configure_attention();
     configure_transition();
     configure_gemm3();
+    configure_gemm();
     cudaGetLastError();
   });
 }
@@ -472,15 +496,10 @@ lf_status contract_scatter(lf_context* ctx, ArenaCursor& cur, const op16* a, con
                        rows_per_rank, ch0);
 }
 
-lf_status contract_gemm(lf_context* ctx, ArenaCursor& cur, const op16* a, const op16* w, op16* out, int m_rows, int n_out,
-                        int k_len, const float* bias, int relu) {
-  return contract_impl(ctx, cur, a, w, out, m_rows, n_out, k_len, k_len, n_out, 0, 0, 1, 0, 1.0f, nullptr, 0, 0,
-                       ContractExtra{bias, relu, 0, 0, 1});
-}
-
 lf_status contract_outer(lf_context* ctx, ArenaCursor& cur, const op16* left, const op16* right, op16* out, int cnt, int n, int c,
                          int k_len, float scale) {
   if (c % 8 != 0) return lf_fail(ctx, LF_ERR_UNSUPPORTED, "the grouped outer product needs c in whole groups of 8");
+  if (c == 32) return gemm_outer32(ctx, cur, left, right, out, cnt, n, k_len, scale);
   // x[(i, a)][(j, b)] = scale * sum_s left[s][(i, a)] right[s][(j, b)]: both operands MN-major, the kernel's "b" is its M operand
   return contract_impl(ctx, cur, right, left, out, cnt * c, n * c, k_len, n * c, n * c, 0, 0, 1, 1, scale, nullptr, 0, 0,
                        ContractExtra{nullptr, 0, c, n, 0});

@@ -46,7 +46,21 @@ lf_status contract(lf_context* ctx, ArenaCursor& cur, const op16* a, const op16*
 lf_status contract_rect(lf_context* ctx, ArenaCursor& cur, const op16* a, const op16* b, op16* x, int m_rows, int n_rows,
                         int k_len, int ld_ab, int ldx, int64_t x_plane, int col0, int c, int incoming, float scale);
 
-// The same kernel as a plain fp16 GEMM: out[m][n] = act(sum_k a[m][k] w[n][k] + bias[n]) (k contiguous in both
+// Plain fp16 GEMMs (tc_gemm.cu), weights [n_out][k]:
+void configure_gemm();
+// q | k | v | gate of rows (b, q) as the attention core reads them: [q, k, v, gate][width / 128][batch][ldq * 128] in 8 x 8 pieces (see
+// attention_project), value (acc + bias) * (qscale for q), gate through a sigmoid; rows Q .. ldq hold finite values
+lf_status gemm_pieces(lf_context* ctx, ArenaCursor& cur, const op16* a, const op16* w, op16* out, int batch, int Q, int ldq, int k_len, int width,
+                      const float* bias, float qscale);
+// out[dst(b, q)][n_out] (+)= a w^T + bias in float32; a = rows (b, q), or pieces [k / 128][batch][ldq * 128] when a_pieces; dst is row q * batch + b
+// when transposed
+bool gemm_rows_supported(const void* out, int n_out);
+lf_status gemm_rows_f32(lf_context* ctx, ArenaCursor& cur, const op16* a, int a_pieces, const op16* w, float* out, int add, int batch, int Q, int ldq,
+                        int transposed, int n_out, int k_len, const float* bias);
+lf_status gemm_rows_half(lf_context* ctx, ArenaCursor& cur, const op16* a_pieces, const op16* w, op16* out, int batch, int Q, int ldq, int n_out, int k_len);
+lf_status gemm_outer32(lf_context* ctx, ArenaCursor& cur, const op16* left, const op16* right, op16* out, int cnt, int n, int k_len, float scale);
+lf_status gemm_planes(lf_context* ctx, ArenaCursor& cur, const op16* a, const op16* b, op16* x, int n, int ld, int c, int incoming, float scale);
+// As rows: out[m][n] = act(sum_k a[m][k] w[n][k] + bias[n]) (k contiguous in both
 // operands, k_len and n_out multiples of 8; bias may be null; act = ReLU when `relu`), fp16 result.
 lf_status contract_gemm(lf_context* ctx, ArenaCursor& cur, const op16* a, const op16* w, op16* out, int m_rows, int n_out,
                         int k_len, const float* bias, int relu);
