@@ -19,8 +19,8 @@ using namespace tc05;
 constexpr int GM_BM = 128, GM_BN = 256, GM_BK = 64, GM_STAGES = 3, GM_EPI = 16;
 constexpr int GM_A_BYTES = GM_BM * GM_BK * 2, GM_B_BYTES = GM_BN * GM_BK * 2, GM_STAGE = GM_A_BYTES + GM_B_BYTES;
 constexpr int GM_OUT = 4096;                  // per epilogue warp: 32 rows x 128 bytes
-constexpr int GM_BIAS = 4096;                 // bias values kept in shared memory
-constexpr int GM_SMEM = GM_STAGES * GM_STAGE + GM_EPI * GM_OUT + GM_BIAS * 4 + 256 + 1024;
+constexpr int GM_SHARE = GM_BN / 4;           // columns of an epilogue warp
+constexpr int GM_SMEM = GM_STAGES * GM_STAGE + GM_EPI * (GM_OUT + GM_SHARE * 4) + 256 + 1024;
 constexpr int GM_THREADS = 64 + 32 * GM_EPI;
 
 enum { GM_HALF = 0, GM_PIECES = 1, GM_F32 = 2, GM_GROUPED = 3 };
@@ -38,6 +38,17 @@ struct GemmParams {
   Status* status;
 };
 
+__device__ __forceinline__ float ex2_approx(float x) {
+  float y;
+  asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+  return y;
+}
+__device__ __forceinline__ float rcp_approx(float x) {
+  float y;
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+  return y;
+}
+
 template <int MAJOR, int EPI>
 __global__ void __launch_bounds__(GM_THREADS, 1)
 gemm_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant__ CUtensorMap mapB, const __grid_constant__ CUtensorMap mapO,
@@ -45,8 +56,8 @@ gemm_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant__ CU
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
   uint8_t* out_stage = smem + GM_STAGES * GM_STAGE;
-  float* bias_s = reinterpret_cast<float*>(out_stage + GM_EPI * GM_OUT);
-  uint64_t* bars = reinterpret_cast<uint64_t*>(bias_s + GM_BIAS);
+  float* bias_s = reinterpret_cast<float*>(out_stage + GM_EPI * GM_OUT);      // [epilogue warp][its columns]
+  uint64_t* bars = reinterpret_cast<uint64_t*>(bias_s + GM_EPI * GM_SHARE);
   uint64_t* full = bars;                       // [STAGES]
   uint64_t* empty = bars + GM_STAGES;          // [STAGES]
   uint64_t* tmem_full = empty + GM_STAGES;     // [2]
@@ -56,9 +67,8 @@ gemm_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant__ CU
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int tiles_m = (p.m + GM_BM - 1) / GM_BM, tiles_n = (p.n + GM_BN - 1) / GM_BN, per = tiles_m * tiles_n;
-  const int64_t total = (int64_t)p.batch * per;
+  const int total = p.batch * per;
   const int kblocks = (p.k + GM_BK - 1) / GM_BK;
-  const bool bias_local = p.bias && p.n <= GM_BIAS;
 
   if (threadIdx.x == 0) {
     for (int s = 0; s < GM_STAGES; ++s) { mbar_init(&full[s], 1); mbar_init(&empty[s], 1); }
@@ -67,14 +77,18 @@ gemm_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant__ CU
     fence_barrier_init();
   }
   if (warp == 1) { tmem_alloc(tmem_slot, 512); tmem_relinquish(); }
-  if (bias_local) {      // (zeros up to the tile's end: the columns past n are clipped, but read)
-    const int padded = tiles_n * GM_BN < GM_BIAS ? tiles_n * GM_BN : GM_BIAS;
-    for (int i = threadIdx.x; i < padded; i += GM_THREADS) bias_s[i] = i < p.n ? __ldg(p.bias + i) : 0.f;
-  }
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
+  // Work item t: N tiles of one M tile are neighbours (their A tile is read once from memory), shifted from M tile to M tile so
+  // that no block keeps one N tile (the gate columns of the pieces cost more than the others).
+  auto locate = [&](int t, int& h, int& mi, int& nj) {
+    const int row = t / tiles_n;
+    h = row / tiles_m;
+    mi = row - h * tiles_m;
+    nj = (t - row * tiles_n + row) % tiles_n;
+  };
 
   if (warp == 0) {
     if (lane == 0) {
@@ -82,8 +96,9 @@ gemm_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant__ CU
       prefetch_tensormap(&mapB);
       int stage = 0; uint32_t phase = 0;
       bool ok = true;
-      for (int64_t t = blockIdx.x; t < total && ok; t += gridDim.x) {
-        const int h = (int)(t / per), rem = (int)(t % per), mi = rem / tiles_n, nj = rem % tiles_n;
+      for (int t = blockIdx.x; t < total && ok; t += gridDim.x) {
+        int h, mi, nj;
+        locate(t, h, mi, nj);
         const int hb = EPI == GM_HALF && MAJOR == 0 && p.batch > 1 && !p.a_pieces ? h : 0;      // B of the plane (weights have one)
         for (int kb = 0; kb < kblocks; ++kb) {
           if (!mbar_wait(&empty[stage], phase ^ 1, abort_flag, p.status, 111)) { ok = false; break; }
@@ -109,8 +124,9 @@ gemm_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant__ CU
       int stage = 0; uint32_t phase = 0;
       uint32_t it = 0;
       bool ok = true;
-      for (int64_t t = blockIdx.x; t < total && ok; t += gridDim.x, ++it) {
-        const int nj = (int)(t % per) % tiles_n;
+      for (int t = blockIdx.x; t < total && ok; t += gridDim.x, ++it) {
+        int h, mi, nj;
+        locate(t, h, mi, nj);
         const int left = p.n - nj * GM_BN;
         const uint32_t idesc = make_idesc_f16(GM_BM, left >= GM_BN ? GM_BN : (left + 15) / 16 * 16, MAJOR, MAJOR);
         if (!mbar_wait(&tmem_empty[it & 1], ((it >> 1) & 1) ^ 1, abort_flag, p.status, 112)) break;
@@ -136,17 +152,33 @@ gemm_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant__ CU
   } else {
     const int q = warp & 3, part = (warp - 2) >> 2;      // TMEM lane quadrant, 64 of the tile's 256 columns
     uint8_t* stage = out_stage + (warp - 2) * GM_OUT;
+    float* bias = bias_s + (warp - 2) * GM_SHARE;
     uint32_t it = 0;
+    int held = -1;      // first column of the bias share in shared memory
     if (lane == 0) prefetch_tensormap(&mapO);
-    for (int64_t t = blockIdx.x; t < total; t += gridDim.x, ++it) {
-      const int h = (int)(t / per), rem = (int)(t % per), mi = rem / tiles_n, nj = rem % tiles_n;
+    for (int t = blockIdx.x; t < total; t += gridDim.x, ++it) {
+      int h, mi, nj;
+      locate(t, h, mi, nj);
+      const int col0 = nj * GM_BN + part * GM_SHARE, row0 = mi * GM_BM + q * 32;
+      const bool mine = col0 < p.n && row0 < p.m;
+      // of the pieces: q is scaled, the gate's exponent is -log2(e) (acc + bias)
+      const int kind = EPI == GM_PIECES ? col0 / p.width : 0;
+      const float scale = EPI != GM_PIECES ? p.scale : kind == 0 ? p.qscale : kind == 3 ? -1.4426950408889634f : 1.0f;
+      if (mine && held != col0) {
+        held = col0;
+        __syncwarp();
+#pragma unroll
+        for (int e = 0; e < GM_SHARE; e += 32) {
+          const int c = col0 + e + lane;
+          bias[e + lane] = p.bias && c < p.n ? __ldg(p.bias + c) * (EPI == GM_PIECES ? scale : 1.0f) : 0.f;
+        }
+        __syncwarp();
+      }
       if (!mbar_wait(&tmem_full[it & 1], (it >> 1) & 1, abort_flag, p.status, 114)) break;
       tc_fence_after();
-      const int col0 = nj * GM_BN + part * 64, row0 = mi * GM_BM + q * 32;
-      const bool mine = col0 < p.n && row0 < p.m;
       uint32_t r[2][32];
       if (mine) {
-        const uint32_t d = tmem_base + ((uint32_t)(q * 32) << 16) + (it & 1) * GM_BN + part * 64;
+        const uint32_t d = tmem_base + ((uint32_t)(q * 32) << 16) + (it & 1) * GM_BN + part * GM_SHARE;
         tmem_ld32(d, r[0]);
         tmem_ld32(d + 32, r[1]);
         tmem_ld_wait();
@@ -157,16 +189,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant__ CU
       __syncwarp();
       if (lane == 0) mbar_arrive(&tmem_empty[it & 1]);      // the share is in registers: the accumulator may be overwritten
       if (!mine) continue;
-      float scale = p.scale;
-      const int kind = EPI == GM_PIECES ? col0 / p.width : 0;
-      if (EPI == GM_PIECES && kind == 0) scale = p.qscale;
       auto value = [&](int half, int e) { return __uint_as_float(r[half][e]); };
-      auto bias4 = [&](int c) {      // of columns c .. c + 3
-        if (!p.bias) return make_float4(0.f, 0.f, 0.f, 0.f);
-        if (bias_local) return *reinterpret_cast<const float4*>(bias_s + c);
-        return make_float4(c < p.n ? __ldg(p.bias + c) : 0.f, c + 1 < p.n ? __ldg(p.bias + c + 1) : 0.f, c + 2 < p.n ? __ldg(p.bias + c + 2) : 0.f,
-                           c + 3 < p.n ? __ldg(p.bias + c + 3) : 0.f);
-      };
       if (EPI == GM_F32) {
 #pragma unroll
         for (int half = 0; half < 2; ++half) {
@@ -175,7 +198,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant__ CU
           __syncwarp();
 #pragma unroll
           for (int k4 = 0; k4 < 8; ++k4) {
-            const float4 b = bias4(col0 + half * 32 + k4 * 4);
+            const float4 b = *reinterpret_cast<const float4*>(bias + half * 32 + k4 * 4);
             *reinterpret_cast<float4*>(stage + lane * 128 + ((k4 ^ (lane & 7)) << 4)) =
                 make_float4(fmaf(value(half, k4 * 4), scale, b.x), fmaf(value(half, k4 * 4 + 1), scale, b.y), fmaf(value(half, k4 * 4 + 2), scale, b.z),
                             fmaf(value(half, k4 * 4 + 3), scale, b.w));
@@ -199,20 +222,19 @@ gemm_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant__ CU
           float v[8];
 #pragma unroll
           for (int e = 0; e < 8; e += 4) {
-            float4 b = make_float4(0.f, 0.f, 0.f, 0.f);
-            if (p.bias) b = bias4(col0 + c8 * 8 + e);
-            v[e] = fmaf(value(half, e0 + e), scale, EPI == GM_PIECES ? b.x * scale : b.x);
-            v[e + 1] = fmaf(value(half, e0 + e + 1), scale, EPI == GM_PIECES ? b.y * scale : b.y);
-            v[e + 2] = fmaf(value(half, e0 + e + 2), scale, EPI == GM_PIECES ? b.z * scale : b.z);
-            v[e + 3] = fmaf(value(half, e0 + e + 3), scale, EPI == GM_PIECES ? b.w * scale : b.w);
+            const float4 b = *reinterpret_cast<const float4*>(bias + c8 * 8 + e);
+            v[e] = fmaf(value(half, e0 + e), scale, b.x);
+            v[e + 1] = fmaf(value(half, e0 + e + 1), scale, b.y);
+            v[e + 2] = fmaf(value(half, e0 + e + 2), scale, b.z);
+            v[e + 3] = fmaf(value(half, e0 + e + 3), scale, b.w);
           }
-          if (EPI == GM_PIECES && kind == 3) {      // the gate
+          if (EPI == GM_PIECES && kind == 3) {
 #pragma unroll
-            for (int e = 0; e < 8; ++e) v[e] = __fdividef(1.0f, 1.0f + __expf(-v[e]));
+            for (int e = 0; e < 8; ++e) v[e] = rcp_approx(1.0f + ex2_approx(v[e]));
           }
 #pragma unroll
           for (int e = 0; e < 4; ++e) w[e] = pack_half2(v[2 * e], v[2 * e + 1]);
-          if (p.relu) {
+          if (EPI == GM_HALF && p.relu) {
 #pragma unroll
             for (int e = 0; e < 4; ++e) {
               const __half2 m = __hmax2(*reinterpret_cast<const __half2*>(&w[e]), __float2half2_rn(0.f));
