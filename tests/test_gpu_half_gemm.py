@@ -31,7 +31,8 @@ def test_transition(dev, rows, c, hidden):
 
 
 @pytest.mark.parametrize("q,batch,heads,transpose,bias", [(1, 3, 8, False, False), (7, 5, 12, True, False), (31, 2, 8, False, True), (33, 130, 8, True, False),
-                                                          (127, 2, 8, False, True), (129, 3, 8, True, False), (257, 2, 12, False, True)])
+                                                          (127, 2, 8, False, True), (129, 3, 8, True, False), (257, 2, 12, False, True),
+                                                          (260, 1, 8, False, True), (300, 3, 8, False, True)])
 def test_attention_pieces(dev, q, batch, heads, transpose, bias):
     import localfold_b200 as lf
     d = syn.draw(4100 + q)
