@@ -27,6 +27,7 @@ constexpr int LG_ROWS = 128;
 constexpr int LG_K = 128;
 constexpr int LG_A_BYTES = LG_ROWS * LG_K * 2;          // 32 KiB per stage, two 16 KiB k-atoms
 constexpr int LG_MAX_CHUNKS = 3;
+constexpr int LG_MASKS = 3;                             // triangle projection: tiles whose masks are held
 
 struct LnGemmParams {
   const void* act;          // [rows][128] f32 or bf16, memory order
@@ -54,10 +55,7 @@ struct LnGemmParams {
   // its [ch_per_rank][peer_plane_rows][ld] buffer, at rows peer_row0 + local row; stores go to the peers' memory
   int peer_ranks, ch_per_rank, peer_plane_rows, peer_row0;
   PeerPtrs peer_a, peer_b;
-  const float* mask_pad;    // tiles along the pair rows (tile_per_row): the mask with rows zero-padded to mask_ld
-  int mask_ld;
-  int plane_tma;            // the planes are written by TMA from staging rows (maps in PlaneMaps), plane_box_h planes per copy
-  int plane_box_h;
+  int plane_box_h;          // planes per copy of a warp's 32 (maps in PlaneMaps)
   // attention projection epilogue
   op16* out_q; op16* out_k; op16* out_v; op16* out_g;   // logical rows, stored in 8 x 8 pieces (see ldq)
   op16* out_bias;           // fp16 [heads][batch rows][ldb] (head, query, key)
@@ -82,19 +80,21 @@ struct LnGemmParams {
 
 // Tensor maps of the triangle projection's destinations: entry 2 * owner + (0 for a, 1 for b) covers that rank's
 // [ch_per_rank][plane rows][ld] buffer (one owner = this device's whole planes).
-constexpr int LG_MAX_PLANE_OWNERS = 8;
-struct PlaneMaps { CUtensorMap m[2 * LG_MAX_PLANE_OWNERS]; };
+// (as many as the launch needs: a kernel's parameters are copied on every launch)
+template <int OWNERS>
+struct PlaneMaps { CUtensorMap m[OWNERS ? 2 * OWNERS : 1]; };
 
 enum { LG_EPI_TRIANGLE = 0, LG_EPI_ATTENTION = 1, LG_EPI_OUTPUT = 2, LG_EPI_TRI_OUT = 3 };
 
 // sigmoid(v) = 0.5 + 0.5 * tanh(v / 2): one MUFU operation.  tanh.approx.f32 has a relative
 // error of 2^-11, so the gate is good to about 2.4e-4 absolute - the precision of the fp16
 // operand it multiplies.
-__device__ __forceinline__ float sigmoid_fast(float v) {
+__device__ __forceinline__ float tanh_approx(float v) {
   float t;
-  asm("tanh.approx.f32 %0, %1;" : "=f"(t) : "f"(0.5f * v));
-  return fmaf(0.5f, t, 0.5f);
+  asm("tanh.approx.f32 %0, %1;" : "=f"(t) : "f"(v));
+  return t;
 }
+__device__ __forceinline__ float sigmoid_fast(float v) { return fmaf(0.5f, tanh_approx(0.5f * v), 0.5f); }
 
 // Rows of tile t: linear tiling, or (i, k-tile) tiles that never straddle a pair row.
 __device__ __forceinline__ void tile_rows(const LnGemmParams& p, int64_t t, int64_t& base, int& count) {
@@ -112,9 +112,9 @@ __device__ __forceinline__ void tile_rows(const LnGemmParams& p, int64_t t, int6
 }
 
 
-template <int EPI>
+template <int EPI, int OWNERS = 0>
 __global__ void __launch_bounds__(LG_THREADS, 1)
-ln_gemm_kernel(const __grid_constant__ CUtensorMap mapX, const __grid_constant__ CUtensorMap mapO, const __grid_constant__ PlaneMaps planes,
+ln_gemm_kernel(const __grid_constant__ CUtensorMap mapX, const __grid_constant__ CUtensorMap mapO, const __grid_constant__ PlaneMaps<OWNERS> planes,
                const __grid_constant__ LnGemmParams p) {
   // two operand stages everywhere; the triangle output also keeps two raw x tiles, and the epilogue of a tile stages its
   // output rows in that tile's x buffer, which its MMAs have finished with by then
@@ -126,27 +126,27 @@ ln_gemm_kernel(const __grid_constant__ CUtensorMap mapX, const __grid_constant__
   uint8_t* sA = smem + w_bytes;                       // 2 stages (w_bytes is a multiple of 1024: n_pad % 8 == 0... x256)
   uint8_t* sX = sA + NS * LG_A_BYTES;                 // triangle output only: the raw x tile
   uint8_t* sStage = sX + (EPI == LG_EPI_TRI_OUT ? NS * LG_A_BYTES : 0);   // attention output: per epilogue warp 32 rows x 128 B of the pair
-  // (triangle projection: per group of four epilogue warps 32 channels x 128 B of an operand plane)
+  // (triangle projection: per epilogue warp 32 channels x 64 B of an operand plane; sStat holds the masks of three tiles and the
+  // bias is kept in registers)
   float* sBias = reinterpret_cast<float*>(sStage + (EPI == LG_EPI_OUTPUT ? LG_EPI_WARPS * 4096
-                                                    : EPI == LG_EPI_TRIANGLE ? 4 * 4096 : 0));
-  float* sStat = sBias + 544 + 256;                   // [2 stages][2][128]: inverse std, inverse std * mean
-  uint64_t* bars = reinterpret_cast<uint64_t*>(sStat + 512);
+                                                    : EPI == LG_EPI_TRIANGLE ? LG_EPI_WARPS * 2048 : 0));
+  float* sStat = sBias + (EPI == LG_EPI_TRIANGLE ? 0 : 544 + 256);      // [2 stages][2][128]: inverse std, inverse std * mean
+  uint64_t* bars = reinterpret_cast<uint64_t*>(sStat + (EPI == LG_EPI_TRIANGLE ? LG_MASKS * LG_ROWS : 512));
   uint64_t* a_full = bars;          // [2]
   uint64_t* a_empty = bars + 2;     // [2]
   uint64_t* acc_full = bars + 4;    // [2]
   uint64_t* acc_empty = bars + 6;   // [2]
   uint64_t* x_full = bars + 8;      // [2] TMA bytes of the x tile
   uint64_t* stat_full = bars + 10;  // [2] row statistics of the x tile written
-  uint64_t* stage_bar = bars + 12;  // [16] hand-over of staging rows: triangle projection 0..3 slices written (count 4), 4..7 rows read;
-                                    // triangle output 8..9: the epilogue warps (count 16) are done with the x buffer of that stage
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 12 + LG_EPI_WARPS);
+  uint64_t* stage_bar = bars + 12;  // triangle output [2]: the epilogue warps are done with the x buffer of that stage; triangle projection [3]: with a tile's mask
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 16);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int64_t tiles = p.tile_per_row ? (int64_t)p.plane_rows * p.tile_per_row : (p.rows + LG_ROWS - 1) / LG_ROWS;
 
   // attention projection: bit (2 * chunk + half) = that 128-column group has a non-zero bias (the epilogue skips the others)
-  __shared__ unsigned int bias_flags[1];
+  unsigned int* bias_flags = reinterpret_cast<unsigned int*>(tmem_slot + 2);
   if (threadIdx.x == 0) bias_flags[0] = 0u;
   if (EPI == LG_EPI_ATTENTION) __syncthreads();
   if (threadIdx.x == 0) {
@@ -156,10 +156,9 @@ ln_gemm_kernel(const __grid_constant__ CUtensorMap mapX, const __grid_constant__
       mbar_init(&a_full[s], LG_PROD_WARPS);
       mbar_init(&a_empty[s], 1);
       mbar_init(&acc_full[s], 1);
-      mbar_init(&acc_empty[s], LG_EPI_WARPS);
+      mbar_init(&acc_empty[s], EPI == LG_EPI_TRIANGLE ? LG_EPI_WARPS / 2 : LG_EPI_WARPS);
     }
-    for (int i = 0; i < LG_EPI_WARPS; ++i)
-      mbar_init(&stage_bar[i], (EPI == LG_EPI_TRIANGLE && i < 4) ? 4 : (EPI == LG_EPI_TRI_OUT && (i == 8 || i == 9)) ? LG_EPI_WARPS : 1);
+    for (int i = 0; i < 4; ++i) mbar_init(&stage_bar[i], LG_EPI_WARPS);
     *abort_flag = 0;
     fence_barrier_init();
   }
@@ -168,7 +167,7 @@ ln_gemm_kernel(const __grid_constant__ CUtensorMap mapX, const __grid_constant__
     const uint4* src = reinterpret_cast<const uint4*>(p.wimg);
     uint4* dst = reinterpret_cast<uint4*>(sW);
     for (int i = threadIdx.x; i < w_bytes / 16; i += LG_THREADS) dst[i] = src[i];
-    for (int i = threadIdx.x; i < p.n_bias; i += LG_THREADS) {
+    for (int i = threadIdx.x; EPI != LG_EPI_TRIANGLE && i < p.n_bias; i += LG_THREADS) {
       const float v = p.bias[i];
       sBias[i] = v;
       if (EPI == LG_EPI_ATTENTION && v != 0.f) atomicOr(bias_flags, 1u << (i >> 7));
@@ -202,14 +201,21 @@ ln_gemm_kernel(const __grid_constant__ CUtensorMap mapX, const __grid_constant__
         const uint32_t row_bytes = p.act_bf16 ? LG_K * 2u : LG_K * 4u;
         bulk_prefetch_l2(reinterpret_cast<const uint8_t*>(p.act) + nb * row_bytes, (uint32_t)nc * row_bytes);
       }
-      if (!mbar_wait(&a_empty[s], ph ^ 1, abort_flag, p.status, 10)) break;
-      uint8_t* tile = sA + s * LG_A_BYTES;
       int64_t row_base;
       int row_count;
       tile_rows(p, t, row_base, row_count);
+      float mask = 0.f;
+      if (EPI == LG_EPI_TRIANGLE && lane < 16 && pw * 16 + lane < row_count) mask = __ldg(p.mask + row_base + pw * 16 + lane);
+      if (!mbar_wait(&a_empty[s], ph ^ 1, abort_flag, p.status, 10)) break;
+      uint8_t* tile = sA + s * LG_A_BYTES;
+      if (EPI == LG_EPI_TRIANGLE) {
+        // three tiles' masks: the epilogue of the tile three back has read its own
+        if (!mbar_wait(&stage_bar[it % LG_MASKS], ((uint32_t)(it / LG_MASKS) & 1u) ^ 1u, abort_flag, p.status, 20)) break;
+        if (lane < 16) sStat[(it % LG_MASKS) * LG_ROWS + pw * 16 + lane] = mask;
+      }
       if (EPI == LG_EPI_TRI_OUT && pw == 0) {
         // the x buffer of this stage doubled as the staging rows of the tile two back: its copies must have read them
-        if (!mbar_wait(&stage_bar[8 + s], ph ^ 1, abort_flag, p.status, 21)) break;
+        if (!mbar_wait(&stage_bar[s], ph ^ 1, abort_flag, p.status, 21)) break;
         if (lane == 0) {
           // x[h][i][k0 .. k0+127] for all 128 channels: two boxes of 64 pairs x 128 channels
           const int i = (int)(t / p.tile_per_row), k0 = (int)(t % p.tile_per_row) * LG_ROWS;
@@ -455,12 +461,84 @@ ln_gemm_kernel(const __grid_constant__ CUtensorMap mapX, const __grid_constant__
         if (!ok) break;
       }
     }
+  } else if (EPI == LG_EPI_TRIANGLE) {
+    // ---------------- epilogue of the triangle projection ----------------
+    // TMEM lane = hidden channel h, columns = the tile's pair rows (projection at 0..127, gate at 128..255).  A warp owns 32
+    // channels x 64 pair rows of one operand (parts 0, 1: a; 2, 3: b) and shares nothing with the others but the accumulator: two passes of
+    // 32 rows into its own staging rows (64 bytes, 64-byte swizzle), each sent off by its own copy.  (Groups of four warps that filled 128-byte
+    // rows together spent the tile on hand-overs: 62 -> 47 us at 384 x 384 pairs, 224 -> 142 us at 701 x 701, 1502 -> 1140 us at 2048 x 2048.)
+    const int q = warp & 3, j = warp >> 3, k0 = ((warp >> 2) & 1) * 64, h = q * 32 + lane;
+    const float bias_p = 0.5f * __ldg(p.bias + j * 256 + h), bias_g = 0.5f * __ldg(p.bias + j * 256 + 128 + h);
+    const uint32_t acc = tmem_base + ((uint32_t)(q * 32) << 16) + j * 256;
+    uint8_t* stage = sStage + warp * 2048;
+    const uint32_t un = (uint32_t)p.n;
+    int it = 0;
+    for (int64_t t = blockIdx.x; t < tiles; t += gridDim.x, ++it) {
+      int64_t row_base;
+      int row_count;
+      tile_rows(p, t, row_base, row_count);
+      const float* mask = sStat + (it % LG_MASKS) * LG_ROWS + k0;
+      if (!mbar_wait(&acc_full[j], it & 1, abort_flag, p.status, 13)) break;
+      tc_fence_after();
+#pragma unroll
+      for (int pass = 0; pass < 2; ++pass) {
+        const bool some = k0 + pass * 32 < row_count;      // (the whole warp alike)
+        uint32_t pk[16];
+        if (some) {
+#pragma unroll
+          for (int c = 0; c < 2; ++c) {
+            uint32_t pv[16], gv[16];
+            tmem_ld16(acc + k0 + pass * 32 + c * 16, pv);
+            tmem_ld16(acc + 128 + k0 + pass * 32 + c * 16, gv);
+            tmem_ld_wait();
+#pragma unroll
+            for (int g4 = 0; g4 < 4; ++g4) {
+              const float4 m = *reinterpret_cast<const float4*>(mask + pass * 32 + c * 16 + g4 * 4);
+              const float mm[4] = {m.x, m.y, m.z, m.w};
+              float val[4];
+#pragma unroll
+              for (int e = 0; e < 4; ++e) {
+                // mask (x + b) sigmoid(y) = (x / 2 + b / 2) (mask + mask tanh(y / 2))
+                const float u = fmaf(__uint_as_float(pv[g4 * 4 + e]), 0.5f, bias_p), y = fmaf(__uint_as_float(gv[g4 * 4 + e]), 0.5f, bias_g);
+                val[e] = u * fmaf(mm[e], tanh_approx(y), mm[e]);
+              }
+              pk[c * 8 + g4 * 2] = pack_half2(val[0], val[1]);
+              pk[c * 8 + g4 * 2 + 1] = pack_half2(val[2], val[3]);
+            }
+          }
+        }
+        if (pass == 1) {
+          tc_fence_before();
+          __syncwarp();
+          if (lane == 0) { mbar_arrive(&acc_empty[j]); mbar_arrive(&stage_bar[it % LG_MASKS]); }
+        }
+        if (!some) continue;
+        if (lane == 0) bulk_wait_read();      // the previous copy has read the staging rows
+        __syncwarp();
+#pragma unroll
+        for (int c = 0; c < 4; ++c)
+          *reinterpret_cast<uint4*>(stage + lane * 64 + (((uint32_t)c ^ (((uint32_t)lane >> 1) & 3u)) << 4)) =
+              make_uint4(pk[c * 4], pk[c * 4 + 1], pk[c * 4 + 2], pk[c * 4 + 3]);
+        fence_async_smem();
+        __syncwarp();
+        if (lane == 0) {
+          int ti, tk;      // n is a multiple of 64 or the tiles lie along the pair rows: a run never straddles two of them
+          if (p.tile_per_row) { ti = (int)(t / p.tile_per_row); tk = (int)(t % p.tile_per_row) * LG_ROWS + k0 + pass * 32; }
+          else { const uint32_t r = (uint32_t)row_base + k0 + pass * 32; ti = (int)(r / un); tk = (int)(r % un); }
+          for (int h0 = 0; h0 < 32; h0 += p.plane_box_h) {
+            const int hh = q * 32 + h0, owner = hh / p.ch_per_rank;
+            tma_store_3d(&planes.m[OWNERS > 1 ? 2 * owner + j : j], stage + h0 * 64, tk, p.peer_row0 + ti, hh - owner * p.ch_per_rank);
+          }
+          bulk_commit();
+        }
+      }
+    }
   } else {
     // ---------------- epilogue ----------------
     const int q = warp & 3, part = warp >> 2;   // part: which quarter of the chunk's columns
     const int row = q * 32 + lane;
     const uint32_t lane_addr = (uint32_t)(q * 32) << 16;
-    uint32_t g = 0, staged = 0;
+    uint32_t g = 0;
     bool ok = true;
     int it = 0;
     for (int64_t t = blockIdx.x; t < tiles && ok; t += gridDim.x, ++it) {
@@ -492,200 +570,7 @@ ln_gemm_kernel(const __grid_constant__ CUtensorMap mapX, const __grid_constant__
         if (!mbar_wait(&acc_full[b], (g >> 1) & 1, abort_flag, p.status, 13)) { ok = false; break; }
         tc_fence_after();
         const uint32_t acc = tmem_base + lane_addr + b * 256;
-        if (EPI == LG_EPI_TRIANGLE) {
-          // TMEM lane = hidden channel h, columns = the tile's pair rows (projection at 0..127,
-          // gate at 128..255).  Each thread owns one channel and writes runs of consecutive k.
-          const int h = row;
-          const float bias_p = sBias[j * 256 + h], bias_g = sBias[j * 256 + 128 + h];
-          op16* plane_base;
-          if (p.peer_ranks >= 1) {
-            const int owner = h / p.ch_per_rank;
-            plane_base = reinterpret_cast<op16*>(j == 0 ? p.peer_a.p[owner] : p.peer_b.p[owner]) +
-                         ((int64_t)(h - owner * p.ch_per_rank) * p.peer_plane_rows + p.peer_row0) * p.ld;
-          } else {
-            plane_base = (j == 0 ? p.out_a : p.out_b) + (int64_t)h * p.plane_rows * p.ld;
-          }
-          const bool vec = (p.n & 15) == 0;
-          const uint32_t un = (uint32_t)p.n;
-          // rows of this warp's quarter: r0 .. r0+31, as (i, k) with 32-bit arithmetic
-          const uint32_t r0 = (uint32_t)(t * LG_ROWS) + part * 32;
-          uint32_t ii = r0 / un, kk0 = r0 % un;
-          if (p.plane_tma && !p.tile_per_row) {
-            // The four warps that share this warp's 32 channels fill staging rows of 64 k (128 bytes, 128-byte swizzle),
-            // 16 k each, twice per chunk; one of them sends the rows off as one copy per owner.  A request to the L2
-            // then carries 128 bytes: with a thread's own 32-byte stores (one line in each of 32 planes per
-            // instruction) the request rate, not the bytes, bounded this kernel.
-            uint8_t* stage = sStage + q * 4096;
-            uint64_t* grp_full = &stage_bar[q];        // count 4: the warps' slices are written
-            uint64_t* grp_free = &stage_bar[4 + q];    // count 1: the copy has finished reading the rows
-#pragma unroll 1
-            for (int pass = 0; pass < 2; ++pass) {
-              const int c0 = pass * 64 + part * 16;
-              uint32_t pv[16], gv[16];
-              tmem_ld16(acc + c0, pv);
-              tmem_ld16(acc + 128 + c0, gv);
-              tmem_ld_wait();
-              const int64_t r64 = t * LG_ROWS + pass * 64;     // n is a multiple of 64: a run lies inside one pair row and
-              if (r64 >= p.rows) break;                        // is in range or out of it as a whole, for all four warps alike
-              const float4* m4 = reinterpret_cast<const float4*>(p.mask + r64 + part * 16);
-              uint32_t pk[8];
-#pragma unroll
-              for (int g4 = 0; g4 < 4; ++g4) {
-                const float4 m = __ldg(m4 + g4);
-                const float mm[4] = {m.x, m.y, m.z, m.w};
-                float val[4];
-#pragma unroll
-                for (int e = 0; e < 4; ++e)
-                  val[e] = mm[e] * (__uint_as_float(pv[g4 * 4 + e]) + bias_p) * sigmoid_fast(__uint_as_float(gv[g4 * 4 + e]) + bias_g);
-                pk[g4 * 2] = pack_half2(val[0], val[1]);
-                pk[g4 * 2 + 1] = pack_half2(val[2], val[3]);
-              }
-              if (part == 0 && staged > 0) {
-                if (lane == 0) { bulk_wait_read(); mbar_arrive(grp_free); }
-                __syncwarp();
-              }
-              if (!mbar_wait(grp_free, (staged & 1u) ^ 1u, abort_flag, p.status, 19)) { ok = false; break; }
-              const uint32_t sw = (uint32_t)lane & 7u;
-              *reinterpret_cast<uint4*>(stage + lane * 128 + (((uint32_t)(part * 2) ^ sw) << 4)) = make_uint4(pk[0], pk[1], pk[2], pk[3]);
-              *reinterpret_cast<uint4*>(stage + lane * 128 + (((uint32_t)(part * 2 + 1) ^ sw) << 4)) = make_uint4(pk[4], pk[5], pk[6], pk[7]);
-              fence_async_smem();
-              __syncwarp();
-              if (lane == 0) mbar_arrive(grp_full);
-              if (part == 0) {
-                if (!mbar_wait(grp_full, staged & 1u, abort_flag, p.status, 20)) { ok = false; break; }
-                if (lane == 0) {
-                  const uint32_t u64 = (uint32_t)r64;
-                  const int ti = (int)(u64 / un), tk = (int)(u64 % un);
-                  for (int h0 = 0; h0 < 32; h0 += p.plane_box_h) {
-                    const int hh = q * 32 + h0, owner = hh / p.ch_per_rank;
-                    tma_store_3d(&planes.m[2 * owner + j], stage + h0 * 128, tk, p.peer_row0 + ti, hh - owner * p.ch_per_rank);
-                  }
-                  bulk_commit();
-                }
-                __syncwarp();
-              }
-              ++staged;
-            }
-            if (!ok) break;
-          } else if (p.plane_tma) {
-            // The same for a length that is not a multiple of 64: the tiles lie along the pair rows, a row's last run is
-            // clipped by the copy, the mask comes from its padded copy (or element by element).  Kept apart from the
-            // aligned form above, which measured 18 % slower per launch with these cases folded into it.
-            uint8_t* stage = sStage + q * 4096;
-            uint64_t* grp_full = &stage_bar[q];        // count 4: the warps' slices are written
-            uint64_t* grp_free = &stage_bar[4 + q];    // count 1: the copy has finished reading the rows
-#pragma unroll 1
-            for (int pass = 0; pass < 2; ++pass) {
-              const int c0 = pass * 64 + part * 16;
-              // A run of 64 k lies inside one pair row: n is a multiple of 64, or the tiles are laid along the pair rows
-              // (tile_per_row) and the run past a row's end is clipped by the copy.  It is in range or out of it as a
-              // whole, for all four warps alike.
-              const int64_t r64 = row_base + pass * 64;
-              if (pass * 64 >= row_count) break;
-              // (tiles along the pair rows read a copy of the mask whose rows are padded with zeros to whole tiles)
-              const float4* m4 = reinterpret_cast<const float4*>(
-                  p.tile_per_row ? p.mask_pad + (t / p.tile_per_row) * p.mask_ld + (t % p.tile_per_row) * LG_ROWS + pass * 64 + part * 16
-                                 : p.mask + r64 + part * 16);
-              // the pass's 16 mask values first, all loads in flight together
-              float mv[16];
-              if (p.tile_per_row && !p.mask_pad) {   // ragged rows of the flat mask: no alignment, nothing read past the row's end
-#pragma unroll
-                for (int e = 0; e < 16; ++e) {
-                  const int in_tile = pass * 64 + part * 16 + e;
-                  mv[e] = in_tile < row_count ? __ldg(p.mask + row_base + in_tile) : 0.f;
-                }
-              } else {
-#pragma unroll
-                for (int g4 = 0; g4 < 4; ++g4) {
-                  const float4 m = __ldg(m4 + g4);
-                  mv[g4 * 4] = m.x; mv[g4 * 4 + 1] = m.y; mv[g4 * 4 + 2] = m.z; mv[g4 * 4 + 3] = m.w;
-                }
-              }
-              // (the mask loads above are in flight while the accumulator columns come out of tensor memory)
-              uint32_t pv[16], gv[16];
-              tmem_ld16(acc + c0, pv);
-              tmem_ld16(acc + 128 + c0, gv);
-              tmem_ld_wait();
-              uint32_t pk[8];
-#pragma unroll
-              for (int g4 = 0; g4 < 4; ++g4) {
-                const float mm[4] = {mv[g4 * 4], mv[g4 * 4 + 1], mv[g4 * 4 + 2], mv[g4 * 4 + 3]};
-                float val[4];
-#pragma unroll
-                for (int e = 0; e < 4; ++e)
-                  val[e] = mm[e] * (__uint_as_float(pv[g4 * 4 + e]) + bias_p) * sigmoid_fast(__uint_as_float(gv[g4 * 4 + e]) + bias_g);
-                pk[g4 * 2] = pack_half2(val[0], val[1]);
-                pk[g4 * 2 + 1] = pack_half2(val[2], val[3]);
-              }
-              if (part == 0 && staged > 0) {
-                if (lane == 0) { bulk_wait_read(); mbar_arrive(grp_free); }
-                __syncwarp();
-              }
-              if (!mbar_wait(grp_free, (staged & 1u) ^ 1u, abort_flag, p.status, 19)) { ok = false; break; }
-              const uint32_t sw = (uint32_t)lane & 7u;
-              *reinterpret_cast<uint4*>(stage + lane * 128 + (((uint32_t)(part * 2) ^ sw) << 4)) = make_uint4(pk[0], pk[1], pk[2], pk[3]);
-              *reinterpret_cast<uint4*>(stage + lane * 128 + (((uint32_t)(part * 2 + 1) ^ sw) << 4)) = make_uint4(pk[4], pk[5], pk[6], pk[7]);
-              fence_async_smem();
-              __syncwarp();
-              if (lane == 0) mbar_arrive(grp_full);
-              if (part == 0) {
-                if (!mbar_wait(grp_full, staged & 1u, abort_flag, p.status, 20)) { ok = false; break; }
-                if (lane == 0) {
-                  const uint32_t u64 = (uint32_t)r64;
-                  int ti, tk;
-                  if (p.tile_per_row) { ti = (int)(t / p.tile_per_row); tk = (int)(t % p.tile_per_row) * LG_ROWS + pass * 64; }
-                  else { ti = (int)(u64 / un); tk = (int)(u64 % un); }
-                  for (int h0 = 0; h0 < 32; h0 += p.plane_box_h) {
-                    const int hh = q * 32 + h0, owner = hh / p.ch_per_rank;
-                    tma_store_3d(&planes.m[2 * owner + j], stage + h0 * 128, tk, p.peer_row0 + ti, hh - owner * p.ch_per_rank);
-                  }
-                  bulk_commit();
-                }
-                __syncwarp();
-              }
-              ++staged;
-            }
-            if (!ok) break;
-          } else
-#pragma unroll 1
-          for (int c0 = part * 32; c0 < part * 32 + 32; c0 += 16) {
-            uint32_t pv[16], gv[16];
-            tmem_ld16(acc + c0, pv);
-            tmem_ld16(acc + 128 + c0, gv);
-            tmem_ld_wait();
-            const int64_t r16 = t * LG_ROWS + c0;
-            if (r16 < p.rows) {
-              if (vec) {
-                const float4* m4 = reinterpret_cast<const float4*>(p.mask + r16);
-                uint32_t pk[8];
-#pragma unroll
-                for (int g4 = 0; g4 < 4; ++g4) {
-                  const float4 m = __ldg(m4 + g4);
-                  const float mm[4] = {m.x, m.y, m.z, m.w};
-                  float val[4];
-#pragma unroll
-                  for (int e = 0; e < 4; ++e)
-                    val[e] = mm[e] * (__uint_as_float(pv[g4 * 4 + e]) + bias_p) * sigmoid_fast(__uint_as_float(gv[g4 * 4 + e]) + bias_g);
-                  pk[g4 * 2] = pack_half2(val[0], val[1]);
-                  pk[g4 * 2 + 1] = pack_half2(val[2], val[3]);
-                }
-                st_global_v8(plane_base + (int64_t)ii * p.ld + kk0, pk);
-              } else {
-#pragma unroll
-                for (int e = 0; e < 16; ++e) {
-                  const int64_t r = r16 + e;
-                  if (r < p.rows) {
-                    const uint32_t ur = (uint32_t)r;
-                    const float v1 = __ldg(p.mask + r) * (__uint_as_float(pv[e]) + bias_p) * sigmoid_fast(__uint_as_float(gv[e]) + bias_g);
-                    plane_base[(int64_t)(ur / un) * p.ld + ur % un] = __float2half_rn(v1);
-                  }
-                }
-              }
-            }
-            kk0 += 16;
-            if (kk0 >= un) { kk0 -= un; ++ii; }
-          }
-        } else if ((EPI == LG_EPI_OUTPUT || EPI == LG_EPI_TRI_OUT) && p.tma_out) {
+        if ((EPI == LG_EPI_OUTPUT || EPI == LG_EPI_TRI_OUT) && p.tma_out) {
           // thread = pair row; the warp's 32 rows x 32 channels are written to its staging rows (128 B each,
           // 16-byte pieces swizzled by row so that the row-per-thread accesses spread over the banks) and leave
           // as one TMA copy (a reduce-add when the pair is updated in place): no global load or store
@@ -915,13 +800,13 @@ ln_gemm_kernel(const __grid_constant__ CUtensorMap mapX, const __grid_constant__
       }
       if (EPI == LG_EPI_TRI_OUT && ok) {
         // this warp is done with the stage's x buffer once its copies have read their rows
-        if (lane == 0) { bulk_wait_read(); mbar_arrive(&stage_bar[8 + it % NS]); }
+        if (lane == 0) { bulk_wait_read(); mbar_arrive(&stage_bar[it % NS]); }
         __syncwarp();
       }
     }
   }
 
-  if ((((EPI == LG_EPI_OUTPUT || EPI == LG_EPI_TRI_OUT) && p.tma_out) || (EPI == LG_EPI_TRIANGLE && p.plane_tma)) && warp < LG_EPI_WARPS &&
+  if ((((EPI == LG_EPI_OUTPUT || EPI == LG_EPI_TRI_OUT) && p.tma_out) || EPI == LG_EPI_TRIANGLE) && warp < LG_EPI_WARPS &&
       lane == 0)
     bulk_wait_all();   // this thread's stores have landed
   tc_fence_before();
@@ -936,13 +821,15 @@ lf_status make_map_f32_rows(lf_context* ctx, CUtensorMap* map, const void* base,
 lf_status make_map_f32_rows_half(lf_context* ctx, CUtensorMap* map, const void* base, uint64_t d1, uint64_t d2, uint64_t stride1_bytes,
                                  uint64_t stride2_bytes, uint32_t b1, uint32_t b2);
 
-static int ln_gemm_smem(int n_pad, bool tri_out = false, bool staged_out = false, bool plane_stage = false) {
-  return n_pad * 256 + (tri_out ? 4 : 2) * LG_A_BYTES + (staged_out ? LG_EPI_WARPS * 4096 : 0) + (plane_stage ? 4 * 4096 : 0) +
-         (544 + 256 + 512) * 4 + 512 + 1024;
+static int ln_gemm_smem(int n_pad, bool tri_out = false, bool staged_out = false) {
+  return n_pad * 256 + (tri_out ? 4 : 2) * LG_A_BYTES + (staged_out ? LG_EPI_WARPS * 4096 : 0) + (544 + 256 + 512) * 4 + 256 + 1024;
 }
+constexpr int LG_TRIANGLE_SMEM = 512 * 256 + 2 * LG_A_BYTES + LG_EPI_WARPS * 2048 + LG_MASKS * LG_ROWS * 4 + 256 + 1024;
+static_assert(LG_TRIANGLE_SMEM <= 232448, "shared memory of the triangle projection");
 
 void configure_ln_gemm() {
-  cudaFuncSetAttribute(ln_gemm_kernel<LG_EPI_TRIANGLE>, cudaFuncAttributeMaxDynamicSharedMemorySize, ln_gemm_smem(512, false, false, true));
+  cudaFuncSetAttribute(ln_gemm_kernel<LG_EPI_TRIANGLE, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, LG_TRIANGLE_SMEM);
+  cudaFuncSetAttribute(ln_gemm_kernel<LG_EPI_TRIANGLE, kMaxPeers>, cudaFuncAttributeMaxDynamicSharedMemorySize, LG_TRIANGLE_SMEM);
   cudaFuncSetAttribute(ln_gemm_kernel<LG_EPI_ATTENTION>, cudaFuncAttributeMaxDynamicSharedMemorySize, ln_gemm_smem(528));
   cudaFuncSetAttribute(ln_gemm_kernel<LG_EPI_OUTPUT>, cudaFuncAttributeMaxDynamicSharedMemorySize, ln_gemm_smem(128, false, true));
   cudaFuncSetAttribute(ln_gemm_kernel<LG_EPI_TRI_OUT>, cudaFuncAttributeMaxDynamicSharedMemorySize, ln_gemm_smem(256, true, false));
@@ -952,12 +839,12 @@ void configure_ln_gemm() {
 lf_status make_map_plane_runs(lf_context* ctx, CUtensorMap* map, const void* base, uint64_t n, uint64_t plane_rows, uint64_t planes,
                               uint64_t ld, uint32_t box_h);
 
-// Destinations of the triangle projection as tensor maps, when the shape allows the staged copies (at most
-// LG_MAX_PLANE_OWNERS owners); otherwise the kernel stores with its own threads.
-static lf_status plane_maps(lf_context* ctx, LnGemmParams& p, PlaneMaps& pm, const PeerPtrs& a, const PeerPtrs& b, int owners,
-                            int plane_rows) {
-  p.plane_tma = 0;
-  if (owners > LG_MAX_PLANE_OWNERS || 128 % owners != 0 || p.ld % 8 != 0) return LF_OK;
+// The triangle projection into its owners' planes.
+template <int OWNERS>
+static lf_status launch_triangle(lf_context* ctx, LnGemmParams& p, const PeerPtrs& a, const PeerPtrs& b, int owners, int rows, int plane_rows) {
+  PlaneMaps<OWNERS> pm{};
+  if (owners > OWNERS || 128 % owners != 0 || p.ld % 8 != 0)
+    return lf_fail(ctx, LF_ERR_UNSUPPORTED, "triangle projection: %d owners of operand rows of %d values", owners, p.ld);
   // a length that is not a multiple of 64: tiles along the pair rows, so that a run never straddles two of them
   if ((p.n & 63) != 0) p.tile_per_row = (p.n + LG_ROWS - 1) / LG_ROWS;
   p.ch_per_rank = 128 / owners;
@@ -968,66 +855,35 @@ static lf_status plane_maps(lf_context* ctx, LnGemmParams& p, PlaneMaps& pm, con
     LF_TRY(make_map_plane_runs(ctx, &pm.m[2 * o + 1], b.p[o], (uint64_t)p.n, (uint64_t)plane_rows, (uint64_t)p.ch_per_rank, (uint64_t)p.ld,
                                (uint32_t)p.plane_box_h));
   }
-  p.plane_tma = 1;
+  const int64_t tiles = p.tile_per_row ? (int64_t)rows * p.tile_per_row : (p.rows + LG_ROWS - 1) / LG_ROWS;
+  const int grid = (int)(tiles < ctx->sm_count ? tiles : ctx->sm_count);
+  lf_prof_begin(ctx, LF_KERNEL_LN_GEMM);
+  ln_gemm_kernel<LG_EPI_TRIANGLE, OWNERS><<<grid, LG_THREADS, LG_TRIANGLE_SMEM, ctx->stream>>>(CUtensorMap{}, CUtensorMap{}, pm, p);
+  lf_prof_end(ctx);
+  ctx->launches++;
   return LF_OK;
-}
-
-// mask [rows][n] -> [rows][mld], zeros past n
-__global__ void pad_mask_kernel(const float* __restrict__ mask, int rows, int n, int mld, float* __restrict__ out) {
-  int64_t idx = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (idx >= (int64_t)rows * mld) return;
-  const int i = (int)(idx / mld), k = (int)(idx % mld);
-  out[idx] = k < n ? mask[(int64_t)i * n + k] : 0.f;
-}
-
-// A length that is not a multiple of 64 runs the projection with tiles along the pair rows; they read the mask from a
-// copy padded to whole tiles when the call's arena has room planned for one (taken in the sizing pass too), and
-// element by element otherwise.
-static const float* padded_mask(lf_context* ctx, ArenaCursor& cur, const float* mask, int rows, int n, int& mld) {
-  mld = (n & 63) && cur.sized_by_dry_pass ? (n + LG_ROWS - 1) / LG_ROWS * LG_ROWS : 0;
-  if (!mld) return nullptr;
-  float* out = cur.take<float>((int64_t)rows * mld);
-  if (!cur.dry) {
-    pad_mask_kernel<<<(unsigned)(((int64_t)rows * mld + 255) / 256), 256, 0, ctx->stream>>>(mask, rows, n, mld, out);
-    ctx->launches++;
-  }
-  return out;
 }
 
 lf_status triangle_project(lf_context* ctx, ArenaCursor& cur, const void* z, int act_dtype, const float* mask, int rows,
                            int n, int ld, int variance, float eps, const lf_weights* w, op16* a, op16* b) {
-  int mld = 0;
-  const float* mask_pad = padded_mask(ctx, cur, mask, rows, n, mld);
   if (cur.dry) return LF_OK;
   LnGemmParams p{};
-  p.mask_pad = mask_pad; p.mask_ld = mld;
   p.act = z; p.act_bf16 = act_dtype == LF_DTYPE_BF16; p.rows = (int64_t)rows * n; p.transpose = 0; p.batch = 1; p.Q = 1;
   p.plane_rows = rows;
   p.eps = eps; p.variance = variance;
   p.wimg = (const uint8_t*)w->h[0]; p.n_pad = 512; p.bias = (const float*)w->h[1]; p.n_bias = 512;
   p.n_chunks = 2; p.chunk_n[0] = 256; p.chunk_n[1] = 256; p.chunk_row0[0] = 0; p.chunk_row0[1] = 256;
   p.mask = mask; p.out_a = a; p.out_b = b; p.n = n; p.ld = ld; p.status = (Status*)ctx->tc_status;
-  PlaneMaps pm{};
   PeerPtrs pa{}, pb{};
   pa.p[0] = a; pb.p[0] = b;
-  LF_TRY(plane_maps(ctx, p, pm, pa, pb, 1, rows));
-  const int64_t tiles = (p.rows + LG_ROWS - 1) / LG_ROWS;
-  const int grid = (int)(tiles < ctx->sm_count ? tiles : ctx->sm_count);
-  lf_prof_begin(ctx, LF_KERNEL_LN_GEMM);
-  ln_gemm_kernel<LG_EPI_TRIANGLE><<<grid, LG_THREADS, ln_gemm_smem(512, false, false, true), ctx->stream>>>(CUtensorMap{}, CUtensorMap{}, pm, p);
-  lf_prof_end(ctx);
-  ctx->launches++;
-  return LF_OK;
+  return launch_triangle<1>(ctx, p, pa, pb, 1, rows, rows);
 }
 
 lf_status triangle_project_scatter(lf_context* ctx, ArenaCursor& cur, const void* z, int act_dtype, const float* mask, int rows,
                                    int n, int ld, int variance, float eps, const lf_weights* w, const PeerPtrs& a_peers,
                                    const PeerPtrs& b_peers, int ranks, int row0) {
-  int mld = 0;
-  const float* mask_pad = padded_mask(ctx, cur, mask, rows, n, mld);
   if (cur.dry) return LF_OK;
   LnGemmParams p{};
-  p.mask_pad = mask_pad; p.mask_ld = mld;
   p.act = z; p.act_bf16 = act_dtype == LF_DTYPE_BF16; p.rows = (int64_t)rows * n; p.transpose = 0; p.batch = 1; p.Q = 1;
   p.plane_rows = rows;
   p.eps = eps; p.variance = variance;
@@ -1037,15 +893,7 @@ lf_status triangle_project_scatter(lf_context* ctx, ArenaCursor& cur, const void
   p.peer_ranks = ranks; p.ch_per_rank = 128 / ranks; p.peer_plane_rows = n; p.peer_row0 = row0;
   p.peer_a = a_peers; p.peer_b = b_peers;
   p.out_a = (op16*)a_peers.p[0]; p.out_b = (op16*)b_peers.p[0];      // ranks == 1: plain form
-  PlaneMaps pm{};
-  LF_TRY(plane_maps(ctx, p, pm, a_peers, b_peers, ranks, n));
-  const int64_t tiles = (p.rows + LG_ROWS - 1) / LG_ROWS;
-  const int grid = (int)(tiles < ctx->sm_count ? tiles : ctx->sm_count);
-  lf_prof_begin(ctx, LF_KERNEL_LN_GEMM);
-  ln_gemm_kernel<LG_EPI_TRIANGLE><<<grid, LG_THREADS, ln_gemm_smem(512, false, false, true), ctx->stream>>>(CUtensorMap{}, CUtensorMap{}, pm, p);
-  lf_prof_end(ctx);
-  ctx->launches++;
-  return LF_OK;
+  return launch_triangle<kMaxPeers>(ctx, p, a_peers, b_peers, ranks, rows, n);
 }
 
 static lf_status attention_project_impl(lf_context* ctx, ArenaCursor& cur, const void* act, int act_dtype, int batch, int Q,
@@ -1089,7 +937,7 @@ static lf_status attention_project_impl(lf_context* ctx, ArenaCursor& cur, const
   const int64_t tiles = (p.rows + LG_ROWS - 1) / LG_ROWS;
   const int grid = (int)(tiles < ctx->sm_count ? tiles : ctx->sm_count);
   lf_prof_begin(ctx, LF_KERNEL_LN_GEMM);
-  ln_gemm_kernel<LG_EPI_ATTENTION><<<grid, LG_THREADS, ln_gemm_smem(528), ctx->stream>>>(CUtensorMap{}, CUtensorMap{}, PlaneMaps{}, p);
+  ln_gemm_kernel<LG_EPI_ATTENTION><<<grid, LG_THREADS, ln_gemm_smem(528), ctx->stream>>>(CUtensorMap{}, CUtensorMap{}, PlaneMaps<0>{}, p);
   lf_prof_end(ctx);
   ctx->launches++;
   return LF_OK;
@@ -1114,7 +962,7 @@ lf_status pair_bias_project(lf_context* ctx, ArenaCursor& cur, const void* pair,
   const int64_t tiles = (p.rows + LG_ROWS - 1) / LG_ROWS;
   const int grid = (int)(tiles < ctx->sm_count ? tiles : ctx->sm_count);
   lf_prof_begin(ctx, LF_KERNEL_LN_GEMM);
-  ln_gemm_kernel<LG_EPI_ATTENTION><<<grid, LG_THREADS, ln_gemm_smem(16), ctx->stream>>>(CUtensorMap{}, CUtensorMap{}, PlaneMaps{}, p);
+  ln_gemm_kernel<LG_EPI_ATTENTION><<<grid, LG_THREADS, ln_gemm_smem(16), ctx->stream>>>(CUtensorMap{}, CUtensorMap{}, PlaneMaps<0>{}, p);
   lf_prof_end(ctx);
   ctx->launches++;
   return LF_OK;
@@ -1151,7 +999,7 @@ lf_status attention_output(lf_context* ctx, ArenaCursor& cur, const op16* o, int
   const int grid = (int)(tiles < ctx->sm_count ? tiles : ctx->sm_count);
   lf_prof_begin(ctx, LF_KERNEL_LN_GEMM);
   // the fp16 rows are in logical order; the transposed scatter happens in the epilogue (or in the tensor map)
-  ln_gemm_kernel<LG_EPI_OUTPUT><<<grid, LG_THREADS, ln_gemm_smem(128, false, true), ctx->stream>>>(CUtensorMap{}, mo, PlaneMaps{}, p);
+  ln_gemm_kernel<LG_EPI_OUTPUT><<<grid, LG_THREADS, ln_gemm_smem(128, false, true), ctx->stream>>>(CUtensorMap{}, mo, PlaneMaps<0>{}, p);
   lf_prof_end(ctx);
   ctx->launches++;
   return LF_OK;
@@ -1182,7 +1030,7 @@ lf_status triangle_output(lf_context* ctx, ArenaCursor& cur, const op16* x, int 
   p.tma_out = (!p.out_bf16 && (resid == nullptr || resid == out)) ? 1 : 0;
   if (p.tma_out) LF_TRY(make_map_f32_rows_half(ctx, &mo, out, (uint64_t)n, (uint64_t)rows, 512, (uint64_t)n * 512, 32, 1));
   lf_prof_begin(ctx, LF_KERNEL_TRIANGLE_OUTPUT);
-  ln_gemm_kernel<LG_EPI_TRI_OUT><<<grid, LG_THREADS, ln_gemm_smem(256, true, false), ctx->stream>>>(mapX, mo, PlaneMaps{}, p);
+  ln_gemm_kernel<LG_EPI_TRI_OUT><<<grid, LG_THREADS, ln_gemm_smem(256, true, false), ctx->stream>>>(mapX, mo, PlaneMaps<0>{}, p);
   lf_prof_end(ctx);
   ctx->launches++;
   return LF_OK;
