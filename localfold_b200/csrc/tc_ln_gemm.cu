@@ -185,19 +185,143 @@ ln_gemm_kernel(const __grid_constant__ CUtensorMap mapX, const __grid_constant__
     // Eight lanes share a row, so one warp instruction covers four rows and a row statistic needs
     // three shuffle steps.  A lane's 16 channels are interleaved with its neighbours' so that every
     // load instruction reads 128 contiguous bytes per row: float input, element e is channel
-    // 32 (e / 4) + 4 j + e % 4; 16-bit input, channel 64 (e / 8) + 8 j + e % 8.  Each warp owns 16 rows of the tile, handled as two
-    // groups of two row-quads; the loads of a group are all issued before any is consumed.
+    // 32 (e / 4) + 4 j + e % 4; 16-bit input, channel 64 (e / 8) + 8 j + e % 8.  Each warp owns 16 rows of the tile, taken 8
+    // at a time.  These warps set the pace of a tile (the loads of 8 rows come back after ~1500 cycles, normalising them takes as long), so
+    // the attention projections load 16-bit rows one unit of 8 ahead (output 38 -> 33 us at 384 x 384 pairs, 125 -> 105 us at 701 x 701
+    // in bfloat16; in the triangle kernels the registers are short: 404 -> 454 us, output).  Floats would need units of 4 rows for that,
+    // whose single chain costs more than the overlap gains (triangle output 52 -> 65 us at 384 x 384).
     const int pw = warp - LG_EPI_WARPS;
     const int sub = lane >> 3, j = lane & 7;
+    const bool half_input = p.a_is_op16 || p.act_bf16;
+    constexpr bool AHEAD = EPI == LG_EPI_ATTENTION || EPI == LG_EPI_OUTPUT;
+    auto source_row = [&](int64_t r) {
+      if (!p.transpose || p.a_is_op16) return r;
+      const uint32_t ur = (uint32_t)r, uq = (uint32_t)p.Q;
+      return (int64_t)(ur % uq) * p.batch + ur / uq;
+    };
+    auto load_half = [&](int64_t t, int unit, uint4 (&raw)[4]) {
+      int64_t row_base;
+      int row_count;
+      tile_rows(p, t, row_base, row_count);
+#pragma unroll
+      for (int u = 0; u < 2; ++u) {
+        const int row = pw * 16 + unit * 8 + u * 4 + sub;
+        raw[u * 2] = raw[u * 2 + 1] = make_uint4(0u, 0u, 0u, 0u);
+        if (row < row_count) {
+          const int64_t r = source_row(row_base + row);
+          if (p.a_is_op16) {
+            // rows in 8 x 8 pieces: channels 8 j .. + 7 are piece j of the row, channels 64 + 8 j .. piece 8 + j
+            const uint32_t ur = (uint32_t)r, uq = (uint32_t)p.Q, rb = ur / uq, rq = ur % uq;
+            const uint4* g = reinterpret_cast<const uint4*>(reinterpret_cast<const op16*>(p.act) + (int64_t)rb * p.ldq * 128 +
+                                                            (int64_t)(rq >> 3) * 1024 + j * 64 + (rq & 7) * 8);
+            raw[u * 2] = g[0];
+            raw[u * 2 + 1] = g[64];
+          } else {
+            const uint4* g = reinterpret_cast<const uint4*>(reinterpret_cast<const bf16*>(p.act) + r * LG_K + 8 * j);
+            raw[u * 2] = g[0];
+            raw[u * 2 + 1] = g[8];
+          }
+        }
+      }
+    };
+    // (x - mean) / std of a lane's 16 values (the gain and offset of the LayerNorm live in the weight image and the bias)
+    auto normalise = [&](const float (&v)[16], bool valid, uint32_t (&packed)[8]) {
+      float s4[4] = {0.f, 0.f, 0.f, 0.f};      // four chains instead of one of 16 dependent additions
+#pragma unroll
+      for (int e = 0; e < 16; ++e) s4[e & 3] += v[e];
+      float sum = (s4[0] + s4[1]) + (s4[2] + s4[3]);
+      sum += __shfl_xor_sync(0xffffffffu, sum, 1);
+      sum += __shfl_xor_sync(0xffffffffu, sum, 2);
+      sum += __shfl_xor_sync(0xffffffffu, sum, 4);
+      const float mean = sum * (1.0f / LG_K);
+      float q4[4] = {0.f, 0.f, 0.f, 0.f};
+      if (p.variance == 2) {
+#pragma unroll
+        for (int e = 0; e < 16; ++e) q4[e & 3] = fmaf(v[e], v[e], q4[e & 3]);
+      } else {
+#pragma unroll
+        for (int e = 0; e < 16; ++e) { const float d = v[e] - mean; q4[e & 3] = fmaf(d, d, q4[e & 3]); }
+      }
+      float sq = (q4[0] + q4[1]) + (q4[2] + q4[3]);
+      sq += __shfl_xor_sync(0xffffffffu, sq, 1);
+      sq += __shfl_xor_sync(0xffffffffu, sq, 2);
+      sq += __shfl_xor_sync(0xffffffffu, sq, 4);
+      const float var = p.variance == 2 ? sq * (1.0f / LG_K) - mean * mean : sq * (1.0f / LG_K);
+      float inv = rsqrtf(var + p.eps);
+      inv = inv * (1.5f - 0.5f * (var + p.eps) * inv * inv);
+      const float shift = -mean * inv;
+#pragma unroll
+      for (int e = 0; e < 8; ++e) packed[e] = valid ? pack_half2(fmaf(v[2 * e], inv, shift), fmaf(v[2 * e + 1], inv, shift)) : 0u;
+    };
+    auto store_half = [&](uint8_t* tile, int row_count, int unit, const uint4 (&raw)[4]) {
+#pragma unroll
+      for (int u = 0; u < 2; ++u) {
+        const int row = pw * 16 + unit * 8 + u * 4 + sub;
+        uint32_t packed[8];
+#pragma unroll
+        for (int w = 0; w < 2; ++w) {
+          const uint4& r = raw[u * 2 + w];
+          packed[w * 4] = r.x; packed[w * 4 + 1] = r.y; packed[w * 4 + 2] = r.z; packed[w * 4 + 3] = r.w;
+        }
+        if (!p.a_is_op16) {
+          float v[16];
+#pragma unroll
+          for (int e = 0; e < 8; ++e) {
+            const __nv_bfloat162 h2 = *reinterpret_cast<const __nv_bfloat162*>(&packed[e]);
+            v[e * 2] = __low2float(h2);
+            v[e * 2 + 1] = __high2float(h2);
+          }
+          normalise(v, row < row_count, packed);
+        }
+        // channels 64 w + 8 j .. + 7: k-atom w, 16-byte chunk j of the row
+#pragma unroll
+        for (int w = 0; w < 2; ++w)
+          *reinterpret_cast<uint4*>(tile + (uint32_t)w * (LG_ROWS * 128) + swizzle128_offset((uint32_t)row, (uint32_t)j)) =
+              make_uint4(packed[w * 4], packed[w * 4 + 1], packed[w * 4 + 2], packed[w * 4 + 3]);
+      }
+    };
+    auto float_rows = [&](uint8_t* tile, int64_t row_base, int row_count, int unit) {
+      float v[2][16];
+#pragma unroll
+      for (int u = 0; u < 2; ++u) {
+        const int row = pw * 16 + unit * 8 + u * 4 + sub;
+        if (row < row_count) {
+          const float4* g = reinterpret_cast<const float4*>(reinterpret_cast<const float*>(p.act) + source_row(row_base + row) * LG_K + 4 * j);
+#pragma unroll
+          for (int w = 0; w < 4; ++w) {
+            const float4 f = g[w * 8];
+            v[u][w * 4] = f.x; v[u][w * 4 + 1] = f.y; v[u][w * 4 + 2] = f.z; v[u][w * 4 + 3] = f.w;
+          }
+        } else {
+#pragma unroll
+          for (int e = 0; e < 16; ++e) v[u][e] = 0.f;
+        }
+      }
+#pragma unroll
+      for (int u = 0; u < 2; ++u) {
+        const int row = pw * 16 + unit * 8 + u * 4 + sub;
+        uint32_t packed[8];
+        normalise(v[u], row < row_count, packed);
+        // channels 32 w + 4 j .. + 3: k-atom w / 2, 16-byte chunk 4 (w % 2) + j / 2, its half j % 2
+#pragma unroll
+        for (int w = 0; w < 4; ++w)
+          *reinterpret_cast<uint2*>(tile + (uint32_t)(w >> 1) * (LG_ROWS * 128) +
+                                    swizzle128_offset((uint32_t)row, (uint32_t)((w & 1) * 4 + (j >> 1))) + (j & 1) * 8) =
+              make_uint2(packed[w * 2], packed[w * 2 + 1]);
+      }
+    };
+    uint4 even[4], odd[4];
+    if (AHEAD && half_input && blockIdx.x < tiles) load_half(blockIdx.x, 0, even);
     int it = 0;
     for (int64_t t = blockIdx.x; t < tiles; t += gridDim.x, ++it) {
       const int s = it % NS;
       const uint32_t ph = (uint32_t)(it / NS) & 1u;
-      if (pw == 0 && lane == 0 && !p.a_is_op16 && !p.transpose && t + gridDim.x < tiles) {
+      const int64_t after = t + gridDim.x;
+      if (pw == 0 && lane == 0 && !p.a_is_op16 && !p.transpose && after < tiles) {
         // rows of a tile are contiguous: ask for this CTA's next tile now, so that its loads find the rows in L2
         int64_t nb;
         int nc;
-        tile_rows(p, t + gridDim.x, nb, nc);
+        tile_rows(p, after, nb, nc);
         const uint32_t row_bytes = p.act_bf16 ? LG_K * 2u : LG_K * 4u;
         bulk_prefetch_l2(reinterpret_cast<const uint8_t*>(p.act) + nb * row_bytes, (uint32_t)nc * row_bytes);
       }
@@ -224,109 +348,19 @@ ln_gemm_kernel(const __grid_constant__ CUtensorMap mapX, const __grid_constant__
           tma_load_3d(sX + s * LG_A_BYTES + LG_A_BYTES / 2, &mapX, &x_full[s], k0 + 64, i, 0);
         }
       }
+      if (AHEAD && half_input) {
+        load_half(t, 1, odd);
+        store_half(tile, row_count, 0, even);
+        if (after < tiles) load_half(after, 0, even);
+        store_half(tile, row_count, 1, odd);
+      } else {
 #pragma unroll 1
-      for (int grp = 0; grp < 2; ++grp) {
-        float v[2][16];
-#pragma unroll
-        for (int u = 0; u < 2; ++u) {
-          const int row = pw * 16 + (grp * 2 + u) * 4 + sub;
-          const int64_t r = row_base + row;
-          if (row < row_count) {
-            int64_t src = r;
-            if (p.transpose && !p.a_is_op16) { const uint32_t ur = (uint32_t)r, uq = (uint32_t)p.Q; src = (int64_t)(ur % uq) * p.batch + ur / uq; }
-            if (p.a_is_op16) {
-              // rows in 8 x 8 pieces: channels 8 j .. + 7 are piece j of the row, channels 64 + 8 j .. piece 8 + j
-              const uint32_t ur = (uint32_t)r, uq = (uint32_t)p.Q, rb = ur / uq, rq = ur % uq;
-              const uint4* g = reinterpret_cast<const uint4*>(reinterpret_cast<const op16*>(p.act) + (int64_t)rb * p.ldq * 128 +
-                                                              (int64_t)(rq >> 3) * 1024 + j * 64 + (rq & 7) * 8);
-#pragma unroll
-              for (int w4 = 0; w4 < 2; ++w4) {
-                const uint4 raw = g[w4 * 64];
-                const uint32_t words[4] = {raw.x, raw.y, raw.z, raw.w};
-#pragma unroll
-                for (int e = 0; e < 4; ++e) {
-                  const float2 f2 = __half22float2(*reinterpret_cast<const __half2*>(&words[e]));
-                  v[u][w4 * 8 + e * 2] = f2.x;
-                  v[u][w4 * 8 + e * 2 + 1] = f2.y;
-                }
-              }
-            } else if (p.act_bf16) {
-              const uint4* g = reinterpret_cast<const uint4*>(reinterpret_cast<const bf16*>(p.act) + src * LG_K + 8 * j);
-#pragma unroll
-              for (int w4 = 0; w4 < 2; ++w4) {
-                const uint4 raw = g[w4 * 8];
-                const uint32_t words[4] = {raw.x, raw.y, raw.z, raw.w};
-#pragma unroll
-                for (int e = 0; e < 4; ++e) {
-                  const __nv_bfloat162 h2 = *reinterpret_cast<const __nv_bfloat162*>(&words[e]);
-                  v[u][w4 * 8 + e * 2] = __low2float(h2);
-                  v[u][w4 * 8 + e * 2 + 1] = __high2float(h2);
-                }
-              }
-            } else {
-              const float4* g = reinterpret_cast<const float4*>(reinterpret_cast<const float*>(p.act) + src * LG_K + 4 * j);
-#pragma unroll
-              for (int w4 = 0; w4 < 4; ++w4) {
-                const float4 f = g[w4 * 8];
-                v[u][w4 * 4] = f.x; v[u][w4 * 4 + 1] = f.y; v[u][w4 * 4 + 2] = f.z; v[u][w4 * 4 + 3] = f.w;
-              }
-            }
+        for (int unit = 0; unit < 2; ++unit) {
+          if (half_input) {
+            load_half(t, unit, even);
+            store_half(tile, row_count, unit, even);
           } else {
-#pragma unroll
-            for (int e = 0; e < 16; ++e) v[u][e] = 0.f;
-          }
-        }
-#pragma unroll
-        for (int u = 0; u < 2; ++u) {
-          const int row = pw * 16 + (grp * 2 + u) * 4 + sub;
-          const bool valid = row < row_count;
-          uint32_t packed[8];
-          if (p.a_is_op16) {
-#pragma unroll
-            for (int e = 0; e < 8; ++e) packed[e] = pack_half2(v[u][2 * e], v[u][2 * e + 1]);
-          } else {
-          float s4[4] = {0.f, 0.f, 0.f, 0.f};      // four chains instead of one of 16 dependent additions
-#pragma unroll
-          for (int e = 0; e < 16; ++e) s4[e & 3] += v[u][e];
-          float sum = (s4[0] + s4[1]) + (s4[2] + s4[3]);
-          sum += __shfl_xor_sync(0xffffffffu, sum, 1);
-          sum += __shfl_xor_sync(0xffffffffu, sum, 2);
-          sum += __shfl_xor_sync(0xffffffffu, sum, 4);
-          const float mean = sum * (1.0f / LG_K);
-          float q4[4] = {0.f, 0.f, 0.f, 0.f};
-          if (p.variance == 2) {
-#pragma unroll
-            for (int e = 0; e < 16; ++e) q4[e & 3] = fmaf(v[u][e], v[u][e], q4[e & 3]);
-          } else {
-#pragma unroll
-            for (int e = 0; e < 16; ++e) { const float d = v[u][e] - mean; q4[e & 3] = fmaf(d, d, q4[e & 3]); }
-          }
-          float sq = (q4[0] + q4[1]) + (q4[2] + q4[3]);
-          sq += __shfl_xor_sync(0xffffffffu, sq, 1);
-          sq += __shfl_xor_sync(0xffffffffu, sq, 2);
-          sq += __shfl_xor_sync(0xffffffffu, sq, 4);
-          const float var = p.variance == 2 ? sq * (1.0f / LG_K) - mean * mean : sq * (1.0f / LG_K);
-          float inv = rsqrtf(var + p.eps);
-          inv = inv * (1.5f - 0.5f * (var + p.eps) * inv * inv);
-          // the gain and offset of the LayerNorm live in the weight image and the bias: the operand is (x - mean) / std
-          const float shift = -mean * inv;
-#pragma unroll
-          for (int e = 0; e < 8; ++e)
-            packed[e] = valid ? pack_half2(fmaf(v[u][2 * e], inv, shift), fmaf(v[u][2 * e + 1], inv, shift)) : 0u;
-          }
-          if (p.a_is_op16 || p.act_bf16) {
-            // channels 64 w + 8 j .. + 7: k-atom w, 16-byte chunk j of the row
-#pragma unroll
-            for (int w2 = 0; w2 < 2; ++w2)
-              *reinterpret_cast<uint4*>(tile + (uint32_t)w2 * (LG_ROWS * 128) + swizzle128_offset((uint32_t)row, (uint32_t)j)) =
-                  make_uint4(packed[w2 * 4], packed[w2 * 4 + 1], packed[w2 * 4 + 2], packed[w2 * 4 + 3]);
-          } else {
-            // channels 32 w + 4 j .. + 3: k-atom w / 2, 16-byte chunk 4 (w % 2) + j / 2, its half j % 2
-#pragma unroll
-            for (int w4 = 0; w4 < 4; ++w4)
-              *reinterpret_cast<uint2*>(tile + (uint32_t)(w4 >> 1) * (LG_ROWS * 128) +
-                                        swizzle128_offset((uint32_t)row, (uint32_t)((w4 & 1) * 4 + (j >> 1))) + (j & 1) * 8) =
-                  make_uint2(packed[w4 * 2], packed[w4 * 2 + 1]);
+            float_rows(tile, row_base, row_count, unit);
           }
         }
       }
