@@ -1326,6 +1326,13 @@ lf_status msa_average(lf_context* ctx, ArenaCursor& cur, const AttArgs& a) {
   return LF_OK;
 }
 
+// The padding the attention core reads (as keys past the end, masked out) must hold finite values.
+void pad_attention(lf_context* ctx, ArenaCursor& cur, op16* k, op16* v, op16* bias, int batch, int heads, int Q, int ldq) {
+  if (ldq == Q || (!k && !bias)) return;
+  const int64_t rows = (k ? (int64_t)batch * 16 : 0) > (bias ? (int64_t)heads * Q : 0) ? (int64_t)batch * 16 : (int64_t)heads * Q;
+  LAUNCH(ctx, cur, rows::attention_padding_kernel, lf_ceil_div(rows * (ldq - Q), 256), 256, 0, (uint16_t*)k, (uint16_t*)v, (uint16_t*)bias, batch, heads, Q, ldq);
+}
+
 // 16-bit path: tensor-core LayerNorm + q/k/v/gate/bias projection, then the attention core.
 template <typename T>
 lf_status att_bf16(lf_context* ctx, ArenaCursor& cur, const AttArgs& a) {
@@ -1339,12 +1346,7 @@ lf_status att_bf16(lf_context* ctx, ArenaCursor& cur, const AttArgs& a) {
   op16* g = cur.take<op16>(RP * HD);
   op16* bias = a.bias_mode ? cur.take<op16>((int64_t)a.heads * a.Q * ldb) : nullptr;
   op16* o16 = cur.take<op16>(RP * HD);
-  if (ldb != a.Q && !cur.dry) {
-    // the padding rows and columns are read (as keys past the end, masked out): they must hold finite values
-    if (bias) cudaMemsetAsync(bias, 0, (size_t)a.heads * a.Q * ldb * sizeof(op16), ctx->stream);
-    cudaMemsetAsync(k, 0, (size_t)RP * HD * sizeof(op16), ctx->stream);
-    cudaMemsetAsync(v, 0, (size_t)RP * HD * sizeof(op16), ctx->stream);
-  }
+  pad_attention(ctx, cur, k, v, bias, a.batch, a.heads, a.Q, ldb);
   LF_TRY(tc::attention_project(ctx, cur, a.act, a.act_dtype, a.batch, a.Q, a.transpose, a.variance, a.eps, a.heads, a.d,
                                a.bias_swap, a.w, q, k, v, g, bias, ldb));
   LF_TRY(tc::attention_core(ctx, cur, q, k, v, g, bias, ldb, a.mask, a.batch, a.Q, a.transpose, a.mask_mode, a.clamp, o16));
@@ -1380,8 +1382,7 @@ lf_status att_mixed(lf_context* ctx, ArenaCursor& cur, const AttArgs& a) {
   layer_norm<T, rows::LN_HALF>(ctx, cur, a.act, R, c, f[ATT_LN_G], f[ATT_LN_B], a.eps, a.variance, a.transpose, a.batch, a.Q, nrm);
   LF_TRY(tc::gemm_pieces(ctx, cur, nrm, gemm_operand(a.w, 0), qkvg, a.batch, a.Q, ldb, c, HD, f[ATT_B4], 1.0f / sqrtf((float)a.d)));
   if (a.bias_mode == 1) {
-    // padding columns are read as keys past the end (masked out): they must hold finite values
-    if (ldb != a.Q && !cur.dry) cudaMemsetAsync(bias16, 0, (size_t)a.heads * a.Q * ldb * sizeof(op16), ctx->stream);
+    pad_attention(ctx, cur, nullptr, nullptr, bias16, a.batch, a.heads, a.Q, ldb);
     LF_TRY(tc::pair_bias_project(ctx, cur, a.pair, a.pair_dtype, a.Q, a.pair_variance, a.pair_eps, a.heads, a.w, bias16, ldb));
   }
   for (int gi = 0; gi < groups; ++gi) {

@@ -720,4 +720,19 @@ __global__ void global_gate_kernel(const float* __restrict__ kvg, int64_t ld, in
   store_terms4(out + r * ldo + c, term_stride, v);
 }
 
+// The attention core reads keys and bias columns up to a whole group of 16 and masks what is past Q: it only has to be finite.  Zeros in
+// rows Q .. ldq - 1 of k and v (8 x 8 pieces, [batch][ldq][128] each; or null) and columns Q .. ldq - 1 of the bias [heads * Q][ldq] (or null).
+// Only the padding is written: clearing the whole tensors took 90 us at 701 x 701 pairs.
+__global__ void attention_padding_kernel(uint16_t* __restrict__ k, uint16_t* __restrict__ v, uint16_t* __restrict__ bias, int batch, int heads, int Q, int ldq) {
+  const int pad = ldq - Q;
+  const int64_t idx = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (k && idx < (int64_t)batch * pad * 16) {
+    const int piece = (int)(idx & 15), row = Q + (int)((idx >> 4) % pad);
+    const int64_t at = (idx >> 4) / pad * ldq * 128 + (int64_t)(row >> 3) * 1024 + piece * 64 + (row & 7) * 8;
+    *reinterpret_cast<uint4*>(k + at) = make_uint4(0u, 0u, 0u, 0u);
+    *reinterpret_cast<uint4*>(v + at) = make_uint4(0u, 0u, 0u, 0u);
+  }
+  if (bias && idx < (int64_t)heads * Q * pad) bias[idx / pad * ldq + Q + idx % pad] = 0;
+}
+
 }  // namespace rows
