@@ -953,7 +953,7 @@ namespace {
   do {                                                                       \
     if (!(cur).dry) {                                                        \
       lf_prof_begin((ctx), LF_KERNEL_SIMT);                                  \
-      kernel<<<(grid), (block), (smem), (ctx)->stream>>>(__VA_ARGS__);       \
+      lf_launch((ctx), kernel, (grid), (block), (smem), __VA_ARGS__);        \
       lf_prof_end((ctx));                                                    \
       (ctx)->launches++;                                                     \
     }                                                                        \

@@ -71,6 +71,7 @@ gemm3_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant__ C
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
+  lf_chain();
 
   if (warp == 0) {
     if (lane == 0) {
@@ -272,8 +273,8 @@ lf_status gemm_f32(lf_context* ctx, ArenaCursor& cur, int major, const SplitMatr
   const int64_t tiles = (int64_t)batch * ((m + G3_BM - 1) / G3_BM) * ((n + G3_BN - 1) / G3_BN);
   const int grid = (int)(tiles < ctx->sm_count ? tiles : ctx->sm_count);
   lf_prof_begin(ctx, LF_KERNEL_SIMT);
-  if (major == 0) gemm3_kernel<0><<<grid, G3_THREADS, G3_SMEM, ctx->stream>>>(ma, mb, p);
-  else gemm3_kernel<1><<<grid, G3_THREADS, G3_SMEM, ctx->stream>>>(ma, mb, p);
+  if (major == 0) lf_launch(ctx, gemm3_kernel<0>, grid, G3_THREADS, G3_SMEM, ma, mb, p);
+  else lf_launch(ctx, gemm3_kernel<1>, grid, G3_THREADS, G3_SMEM, ma, mb, p);
   lf_prof_end(ctx);
   ctx->launches++;
   return LF_OK;

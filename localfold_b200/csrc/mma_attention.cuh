@@ -124,6 +124,7 @@ template <int D, int TERMS, bool BIAS>
 __global__ void __launch_bounds__(256, TERMS == 3 && D > 32 ? 1 : TERMS == 1 && D <= 16 ? 3 : 2)
 attention_kernel(const uint16_t* __restrict__ qkvg, const void* __restrict__ bias_any, const float* __restrict__ mask,
                  const AttentionShape s, uint16_t* __restrict__ out) {
+  lf_chain();
   typedef typename std::conditional<TERMS == 1, __half, float>::type TBias;
   const TBias* bias = static_cast<const TBias*>(bias_any);
   constexpr int TOP = TERMS - 1;                    // highest order of a term product that is kept: i + j <= TOP

@@ -61,6 +61,7 @@ template <typename TIn, int NV, int L, int OUT, int R>
 __global__ void __launch_bounds__(256)
 layer_norm_rows_kernel(const TIn* __restrict__ in, int64_t count, const float* __restrict__ gamma, const float* __restrict__ beta, float eps,
                        int variance, int transpose, int batch, int Q, void* __restrict__ out, int64_t term_stride) {
+  lf_chain();
   constexpr int CH = 4 * NV * L, GROUPS = 256 / L;
   const int l = threadIdx.x % L;
   const int64_t first = (int64_t)blockIdx.x * (GROUPS * R) + threadIdx.x / L;
@@ -117,6 +118,7 @@ template <typename TIn>
 __global__ void layer_norm_terms_kernel(const TIn* __restrict__ in, int64_t count, int ch, int ld, const float* __restrict__ gamma,
                                         const float* __restrict__ beta, float eps, int variance, int transpose, int batch, int Q,
                                         bf16* __restrict__ out, int64_t term_stride) {
+  lf_chain();
   const int lane = threadIdx.x & 31;
   const int64_t row = (int64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
   if (row >= count) return;
@@ -147,6 +149,7 @@ __global__ void layer_norm_terms_kernel(const TIn* __restrict__ in, int64_t coun
 
 // float32 rows of `ch` -> terms with rows of ld
 __global__ void to_terms_kernel(const float* __restrict__ in, int64_t count, int ch, int ld, bf16* __restrict__ out, int64_t term_stride) {
+  lf_chain();
   const int64_t idx = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   const int l2 = ld >> 1;
   if (idx >= count * l2) return;
@@ -160,6 +163,7 @@ __global__ void to_terms_kernel(const float* __restrict__ in, int64_t count, int
 
 // SwiGLU over [rows][2 inter] (gate half first) -> terms with rows of ld
 __global__ void swiglu_terms_kernel(const float* __restrict__ wide, int64_t count, int inter, int ld, bf16* __restrict__ out, int64_t term_stride) {
+  lf_chain();
   const int64_t idx = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   const int l2 = ld >> 1;
   if (idx >= count * l2) return;
@@ -179,6 +183,7 @@ __global__ void swiglu_terms_kernel(const float* __restrict__ wide, int64_t coun
 
 // ... on fp16 (inter a multiple of 8): silu(gate half) * value half, eight channels a thread
 __global__ void swiglu_half_kernel(const __half* __restrict__ wide, int64_t count, int inter, __half* __restrict__ out) {
+  lf_chain();
   const int c = (blockIdx.x * 32 + threadIdx.x) * 8;
   const int64_t row = (int64_t)blockIdx.y * 8 + threadIdx.y;
   if (c >= inter || row >= count) return;
@@ -199,6 +204,7 @@ __global__ void swiglu_half_kernel(const __half* __restrict__ wide, int64_t coun
 __global__ void __launch_bounds__(256)
 trimul_gate_terms_kernel(const float* __restrict__ p4, const float* __restrict__ mask, int c, int n, int ld, bf16* __restrict__ a,
                          bf16* __restrict__ b, int64_t term_stride) {
+  lf_chain();
   __shared__ float ta[32][33], tb[32][33];
   const int tiles = (n + 31) / 32, i = blockIdx.x / tiles, k0 = (blockIdx.x % tiles) * 32, h0 = blockIdx.y * 32;
   const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
@@ -240,6 +246,7 @@ template <typename TIn, int OUT>
 __global__ void __launch_bounds__(256)
 center_norm_kernel(const TIn* __restrict__ x, int c, int n, int ld, const float* __restrict__ gamma, const float* __restrict__ beta,
                    float eps, int variance, float prescale, int ldc, void* __restrict__ xn, int64_t term_stride) {
+  lf_chain();
   extern __shared__ float tile[];   // [c][33]
   const int tiles = (n + 31) / 32, i = blockIdx.x / tiles, k0 = (blockIdx.x % tiles) * 32;
   const int tx = threadIdx.x & 31, w = threadIdx.x >> 5;
@@ -279,6 +286,7 @@ center_norm_kernel(const TIn* __restrict__ x, int c, int n, int ld, const float*
 template <typename TAct>
 __global__ void finish4_kernel(const float* __restrict__ proj, const float* __restrict__ gate, const TAct* __restrict__ resid, int64_t count,
                                int ch, int transpose, int batch, int Q, TAct* __restrict__ out) {
+  lf_chain();
   const int64_t idx = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   const int c4 = ch >> 2;
   if (idx >= count * c4) return;
@@ -307,6 +315,7 @@ __global__ void finish4_kernel(const float* __restrict__ proj, const float* __re
 // past n).  A block turns 64 pairs x 32 channels of one pair row round in shared memory.
 __global__ void __launch_bounds__(256)
 trimul_gate_half_kernel(const __half* __restrict__ p4, const float* __restrict__ mask, int c, int n, int ld, __half* __restrict__ a, __half* __restrict__ b) {
+  lf_chain();
   __shared__ __half ta[32][72], tb[32][72];
   const int tiles = (n + 63) / 64, i = blockIdx.x / tiles, k0 = (blockIdx.x % tiles) * 64, h0 = blockIdx.y * 32;
   {
@@ -342,6 +351,7 @@ trimul_gate_half_kernel(const __half* __restrict__ p4, const float* __restrict__
 template <typename TAct>
 __global__ void finish_gate_half_kernel(const __half* __restrict__ proj, const __half* __restrict__ gate, const TAct* __restrict__ resid, int64_t count,
                                         TAct* __restrict__ out) {
+  lf_chain();
   const int64_t idx = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (idx >= count) return;
   const uint4 p = *reinterpret_cast<const uint4*>(proj + idx * 8), g = *reinterpret_cast<const uint4*>(gate + idx * 8);
@@ -353,6 +363,7 @@ __global__ void finish_gate_half_kernel(const __half* __restrict__ proj, const _
 
 // fp16 columns col0 .. col0 + heads of rows (i * Q + j) -> bias[h][i][ldb] (zeros past Q), or its transpose when `swap`
 __global__ void bias_columns_half_kernel(const __half* __restrict__ in, int64_t ld, int col0, int Q, int ldb, int heads, int swap, __half* __restrict__ out) {
+  lf_chain();
   const int64_t idx = (int64_t)blockIdx.x * blockDim.x + threadIdx.x, plane = (int64_t)Q * ldb;
   if (idx >= plane) return;
   const uint32_t i = (uint32_t)(idx / ldb), j = (uint32_t)(idx % ldb);
@@ -362,6 +373,7 @@ __global__ void bias_columns_half_kernel(const __half* __restrict__ in, int64_t 
 
 // columns col0 .. col0 + heads of rows (i * Q + j) of a terms matrix -> bias[h][i][j], or [h][j][i] when `swap`
 __global__ void bias_columns_kernel(const bf16* __restrict__ in, int64_t ld, int64_t term_stride, int col0, int Q, int heads, int swap, float* __restrict__ out) {
+  lf_chain();
   const int64_t idx = (int64_t)blockIdx.x * blockDim.x + threadIdx.x, pairs = (int64_t)Q * Q;
   if (idx >= pairs) return;
   const uint32_t i = (uint32_t)idx / (uint32_t)Q, j = (uint32_t)idx % (uint32_t)Q;
@@ -374,6 +386,7 @@ __global__ void bias_columns_kernel(const bf16* __restrict__ in, int64_t ld, int
 
 // key[t] = max over the sequences of mask[s][t]; one warp per 32 tokens and slice of the sequences, combined in shared memory
 __global__ void __launch_bounds__(1024) key_mask_kernel(const float* __restrict__ mask, int sequences, int tokens, float* __restrict__ key) {
+  lf_chain();
   __shared__ float part[32][33];
   const int t = blockIdx.x * 32 + threadIdx.x;
   float largest = 0.f;
@@ -390,6 +403,7 @@ __global__ void __launch_bounds__(1024) key_mask_kernel(const float* __restrict_
 // softmax over j of bias[h][i][j] + 1e9 (key[j] - 1) -> terms of its transpose, [3][h][j][ld] with i contiguous
 __global__ void __launch_bounds__(256)
 average_weights_kernel(const float* __restrict__ bias, const float* __restrict__ key, int n, int ld, bf16* __restrict__ out, int64_t term_stride) {
+  lf_chain();
   __shared__ float tile[32][33], top[32], inv[32];
   const int h = blockIdx.y, i0 = blockIdx.x * 32, tx = threadIdx.x & 31, w = threadIdx.x >> 5;
   const float* b = bias + ((int64_t)h * n + i0) * n;
@@ -427,6 +441,7 @@ average_weights_kernel(const float* __restrict__ bias, const float* __restrict__
 // threads take consecutive sequences of one (head, j)
 __global__ void average_values_kernel(const float* __restrict__ v, int64_t ld, int S, int n, int heads, int d, int lds, bf16* __restrict__ out,
                                       int64_t term_stride) {
+  lf_chain();
   const int s = blockIdx.x * blockDim.x + threadIdx.x, j = blockIdx.y, h = blockIdx.z;
   if (s >= S) return;
   const float* src = v + ((int64_t)s * n + j) * ld + h * d;
@@ -458,6 +473,7 @@ __global__ void average_values_kernel(const float* __restrict__ v, int64_t ld, i
 // o[(s, i)][h * d + e] = x[h][i][s * d + e] * gate[(s, i)][h * d + e] -> terms with rows of ldo
 __global__ void average_gate_kernel(const float* __restrict__ x, int64_t ldx, const float* __restrict__ gate, int64_t ldg, int S, int n, int heads,
                                     int d, int ldo, bf16* __restrict__ out, int64_t term_stride) {
+  lf_chain();
   const int64_t idx = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   const int l2 = ldo >> 1;
   if (idx >= (int64_t)S * n * l2) return;
@@ -483,6 +499,7 @@ __global__ void average_gate_kernel(const float* __restrict__ x, int64_t ldx, co
 template <typename T>
 __global__ void __launch_bounds__(512)
 global_mean_kernel(const T* __restrict__ act, const float* __restrict__ mask, int S, int n, int c, float eps, int variance, float* __restrict__ sums) {
+  lf_chain();
   extern __shared__ float part[];      // [16 warps][c + 1]
   const int col = blockIdx.x, lane = threadIdx.x & 31, w = threadIdx.x >> 5;
   float acc[16], count = 0.f;          // channels lane, lane + 32, ... (c <= 512)
@@ -533,6 +550,7 @@ global_mean_kernel(const T* __restrict__ act, const float* __restrict__ mask, in
 template <typename T, int NV, int L>
 __global__ void __launch_bounds__(512)
 global_mean_rows_kernel(const T* __restrict__ act, const float* __restrict__ mask, int S, int n, float eps, int variance, float* __restrict__ sums) {
+  lf_chain();
   constexpr int CH = 4 * NV * L, GROUPS = 512 / L;
   __shared__ float part[GROUPS][CH + 1];
   const int col = blockIdx.x, l = threadIdx.x % L, g = threadIdx.x / L;
@@ -596,6 +614,7 @@ global_mean_rows_kernel(const T* __restrict__ act, const float* __restrict__ mas
 __global__ void __launch_bounds__(512)
 global_mean_terms_kernel(const bf16* __restrict__ nrm, int64_t ld, int64_t term_stride, const float* __restrict__ mask, int S, int n, int c,
                          float* __restrict__ sums) {
+  lf_chain();
   const int col = blockIdx.x;
   for (int ch = threadIdx.x; ch <= c; ch += 512) {
     float total = 0.f;
@@ -611,6 +630,7 @@ global_mean_terms_kernel(const bf16* __restrict__ nrm, int64_t ld, int64_t term_
 // q[col][slot] = scale * sum_ch mean[ch] wq[ch][slot], mean = (gamma sum + beta count) / (1e-10 + count), or sum / (1e-10 + count) without gamma
 __global__ void global_query_kernel(const float* __restrict__ sums, const float* __restrict__ gamma, const float* __restrict__ beta, int c, int HD,
                                     float scale, const float* __restrict__ wq, float* __restrict__ q) {
+  lf_chain();
   extern __shared__ float means[];
   const int col = blockIdx.x;
   const float count = sums[(int64_t)col * (c + 1) + c], denominator = 1e-10f + count;
@@ -634,6 +654,7 @@ template <int D, int HB>
 __global__ void __launch_bounds__(256)
 global_attend_kernel(const float* __restrict__ q, const float* __restrict__ kv, int64_t ld, const float* __restrict__ mask, int S, int n, int heads,
                      int d, float* __restrict__ attended) {
+  lf_chain();
   __shared__ float part[8][HB][D + 2], q_s[HB][D];
   const int col = blockIdx.x, h0 = blockIdx.y * HB, lane = threadIdx.x & 31, w = threadIdx.x >> 5;
   for (int u = threadIdx.x; u < HB * D; u += 256) {
@@ -708,6 +729,7 @@ global_attend_kernel(const float* __restrict__ q, const float* __restrict__ kv, 
 // gate[(s, col)][slot] (columns gate0.. of rows of `ld`) * attended[col][slot] -> terms with rows of ldo (a multiple of 8); `per` blocks a sequence
 __global__ void global_gate_kernel(const float* __restrict__ kvg, int64_t ld, int gate0, const float* __restrict__ attended, int per, int n, int HD, int ldo,
                                    bf16* __restrict__ out, int64_t term_stride) {
+  lf_chain();
   const uint32_t idx = blockIdx.x % per * blockDim.x + threadIdx.x, l4 = (uint32_t)ldo >> 2;
   if (idx >= (uint32_t)n * l4) return;
   const uint32_t col = idx / l4, c = idx % l4 * 4;
@@ -724,6 +746,7 @@ __global__ void global_gate_kernel(const float* __restrict__ kvg, int64_t ld, in
 // rows Q .. ldq - 1 of k and v (8 x 8 pieces, [batch][ldq][128] each; or null) and columns Q .. ldq - 1 of the bias [heads * Q][ldq] (or null).
 // Only the padding is written: clearing the whole tensors took 90 us at 701 x 701 pairs.
 __global__ void attention_padding_kernel(uint16_t* __restrict__ k, uint16_t* __restrict__ v, uint16_t* __restrict__ bias, int batch, int heads, int Q, int ldq) {
+  lf_chain();
   const int pad = ldq - Q;
   const int64_t idx = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (k && idx < (int64_t)batch * pad * 16) {

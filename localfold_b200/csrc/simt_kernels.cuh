@@ -59,6 +59,7 @@ __global__ void layer_norm_kernel(const TIn* __restrict__ in, int64_t rows, int 
                                   const float* __restrict__ gamma, const float* __restrict__ beta,
                                   float eps, int variance, int transpose, int batch, int Q,
                                   TOut* __restrict__ out) {
+  lf_chain();
   int lane = threadIdx.x & 31;
   int64_t row = (int64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
   if (row >= rows) return;
@@ -97,6 +98,7 @@ __global__ void __launch_bounds__(256)
 sgemm_kernel(int M, int N, int K, const float* __restrict__ A, int64_t lda, int64_t strideA,
              const float* __restrict__ B, int64_t ldb, int64_t strideB, float* __restrict__ C,
              int64_t ldc, int64_t strideC, const float* __restrict__ bias, int epi_col0) {
+  lf_chain();
   constexpr int BM = 64, BN = 64, BK = 16;
   __shared__ float As[BK][BM + 4];
   __shared__ float Bs[BK][BN + 4];
@@ -171,6 +173,7 @@ template <typename TAct>
 __global__ void finish_kernel(const float* __restrict__ proj, const float* __restrict__ gate,
                               const TAct* __restrict__ resid, int64_t rows, int ch, int transpose,
                               int batch, int Q, TAct* __restrict__ out) {
+  lf_chain();
   int64_t idx = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   int64_t total = rows * ch;
   if (idx >= total) return;
@@ -192,6 +195,7 @@ __global__ void pair_bias_kernel(const TIn* __restrict__ pair, int Q, int ch, in
                                  const float* __restrict__ gamma, const float* __restrict__ beta,
                                  const float* __restrict__ w, float eps, int variance, int normalized,
                                  int swap, float* __restrict__ out) {
+  lf_chain();
   int lane = threadIdx.x & 31;
   int64_t pairs = (int64_t)Q * Q;
   int64_t p = (int64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
@@ -234,6 +238,7 @@ template <typename TAct>
 __global__ void finish_half_kernel(const __half* __restrict__ proj, float scale, const float* __restrict__ bias,
                                    const TAct* __restrict__ resid, int64_t rows, int ch, int transpose,
                                    int batch, int Q, TAct* __restrict__ out) {
+  lf_chain();
   int64_t idx = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   const int c8 = ch >> 3;
   if (idx >= rows * c8) return;
@@ -253,6 +258,7 @@ __global__ void finish_half_kernel(const __half* __restrict__ proj, float scale,
 
 // fp16 pair bias [heads][Q][ld] (rows padded to ld) -> float32 [heads][Q][Q]
 __global__ void widen_bias_kernel(const __half* __restrict__ in, int heads, int Q, int ld, float* __restrict__ out) {
+  lf_chain();
   int64_t idx = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   int64_t total = (int64_t)heads * Q * Q;
   if (idx >= total) return;
@@ -263,6 +269,7 @@ __global__ void widen_bias_kernel(const __half* __restrict__ in, int heads, int 
 
 // out[i][j][b] = half[i][j][b] + half[j][i][b]: a sum over the two token orders, not a mean.
 __global__ void symmetrise_sum_kernel(const float* __restrict__ half, int tokens, int bins, float* __restrict__ out) {
+  lf_chain();
   int64_t idx = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   int64_t total = (int64_t)tokens * tokens * bins;
   if (idx >= total) return;
@@ -278,6 +285,7 @@ __global__ void symmetrise_sum_kernel(const float* __restrict__ half, int tokens
 // the same into fp16 copies (operands of the tensor-core outer product)
 __global__ void mask_rows_half_kernel(const float* __restrict__ a, const float* __restrict__ b, const float* __restrict__ mask,
                                       int64_t rows, int c, __half* __restrict__ a16, __half* __restrict__ b16) {
+  lf_chain();
   int64_t idx = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (idx >= rows * c) return;
   float m = mask[idx / c];
@@ -289,6 +297,7 @@ __global__ void mask_rows_half_kernel(const float* __restrict__ a, const float* 
 __global__ void opm_split_half_kernel(const __half* __restrict__ lr, const float* __restrict__ bl, const float* __restrict__ br,
                                       const float* __restrict__ mask, int64_t rows, int c, __half* __restrict__ a16,
                                       __half* __restrict__ b16) {
+  lf_chain();
   int64_t idx = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (idx >= rows * c) return;
   int64_t r = idx / c;
@@ -304,6 +313,7 @@ template <typename TAct>
 __global__ void opm_finish_half_kernel(const __half* __restrict__ proj, float scale, const float* __restrict__ bout,
                                        const float* __restrict__ counts, int N, int cz, int i0, int cnt, float norm_eps,
                                        int bias_after_norm, const TAct* __restrict__ resid, TAct* __restrict__ out) {
+  lf_chain();
   int64_t idx = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;      // eight channels per thread (cz a multiple of 8)
   const int z8 = cz >> 3;
   if (idx >= (int64_t)cnt * N * z8) return;
@@ -326,6 +336,7 @@ __global__ void opm_finish_half_kernel(const __half* __restrict__ proj, float sc
 
 __global__ void mask_rows_kernel(float* __restrict__ a, float* __restrict__ b, const float* __restrict__ mask,
                                  int64_t rows, int c) {
+  lf_chain();
   int64_t idx = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (idx >= rows * c) return;
   float m = mask[idx / c];
@@ -343,6 +354,7 @@ __global__ void opm_output_kernel(const TOuter* __restrict__ outer, float outer_
                                   int S, int N, int c, int cz, int i0, float norm_eps,
                                   int bias_after_norm, const TAct* __restrict__ resid,
                                   TAct* __restrict__ out) {
+  lf_chain();
   extern __shared__ float sm[];     // [JT][c*c] + counts[JT]
   const int cc = c * c;
   float* tile = sm;
@@ -389,6 +401,7 @@ __global__ void opm_output_kernel(const TOuter* __restrict__ outer, float outer_
 __global__ void int5_decode_kernel(const uint8_t* __restrict__ codes, const __half* __restrict__ scales,
                                    const __half* __restrict__ zeros, int64_t elements, int block,
                                    float* __restrict__ out) {
+  lf_chain();
   int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= elements) return;
   int64_t g = i / block;

@@ -151,6 +151,7 @@ flash_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_constant__ C
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
+  lf_chain();
 
   // The 16 softmax warps (warpgroups 0-3) hold a tile's logits and probabilities in registers; the
   // producer and issuer warps (warpgroup 4) need few and hand theirs over.  Each role's code follows
@@ -567,8 +568,8 @@ lf_status attention_core(lf_context* ctx, ArenaCursor& cur, const op16* q, const
   if (items > INT32_MAX) return lf_fail(ctx, LF_ERR_UNSUPPORTED, "attention over %d rows of %d queries exceeds the work index", batch, Q);
   const int grid = (int)(items < ctx->sm_count ? items : ctx->sm_count);
   lf_prof_begin(ctx, LF_KERNEL_ATTENTION);
-  if (rows) flash_kernel<true><<<grid, FA_THREADS, FlashForm<true>::SMEM, ctx->stream>>>(mq, mk, mv, mb, p);
-  else flash_kernel<false><<<grid, FA_THREADS, FlashForm<false>::SMEM, ctx->stream>>>(mq, mk, mv, mb, p);
+  if (rows) lf_launch(ctx, flash_kernel<true>, grid, FA_THREADS, FlashForm<true>::SMEM, mq, mk, mv, mb, p);
+  else lf_launch(ctx, flash_kernel<false>, grid, FA_THREADS, FlashForm<false>::SMEM, mq, mk, mv, mb, p);
   lf_prof_end(ctx);
   ctx->launches++;
   return LF_OK;

@@ -81,6 +81,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant__ CU
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
+  lf_chain();
   // Work item t: N tiles of one M tile are neighbours (their A tile is read once from memory), shifted from M tile to M tile so
   // that no block keeps one N tile (the gate columns of the pieces cost more than the others).
   auto locate = [&](int t, int& h, int& mi, int& nj) {
@@ -291,7 +292,7 @@ static lf_status launch(lf_context* ctx, int family, const CUtensorMap& ma, cons
   const int64_t tiles = (int64_t)p.batch * ((p.m + GM_BM - 1) / GM_BM) * ((p.n + GM_BN - 1) / GM_BN);
   const int grid = (int)(tiles < ctx->sm_count ? tiles : ctx->sm_count);
   lf_prof_begin(ctx, family);
-  gemm_kernel<MAJOR, EPI><<<grid, GM_THREADS, GM_SMEM, ctx->stream>>>(ma, mb, mo, p);
+  lf_launch(ctx, gemm_kernel<MAJOR, EPI>, grid, GM_THREADS, GM_SMEM, ma, mb, mo, p);
   lf_prof_end(ctx);
   ctx->launches++;
   return LF_OK;

@@ -255,6 +255,7 @@ contract_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant_
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
+  lf_chain();
 
   if (warp == 0) {
     if (lane == 0) {
@@ -527,7 +528,7 @@ static lf_status contract_impl(lf_context* ctx, ArenaCursor& cur, const op16* a,
   const int grid = tiles < ctx->sm_count ? tiles : ctx->sm_count;
   lf_prof_begin(ctx, LF_KERNEL_TRIANGLE_CONTRACT);
 #define CT_LAUNCH(MAJ, EWN) \
-  contract_kernel<MAJ, EWN><<<grid, ct_threads(EWN), ct_smem(EWN), ctx->stream>>>(mapA, mapB, x, m_rows, n_rows, k_len, ldx, x_plane, col0, c, \
+  lf_launch(ctx, contract_kernel<MAJ, EWN>, grid, ct_threads(EWN), ct_smem(EWN), mapA, mapB, x, m_rows, n_rows, k_len, ldx, x_plane, col0, c, \
       scale, (Status*)ctx->tc_status, peers ? *peers : PeerPtrs{}, rows_per_rank, ch0, ex)
   const bool wide_epilogue = (ex.staged || ex.group_c) && !peers;      // the plain-GEMM uses
   if (!incoming) { if (wide_epilogue) CT_LAUNCH(0, 8); else CT_LAUNCH(0, 4); }

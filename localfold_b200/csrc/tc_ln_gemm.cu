@@ -148,7 +148,6 @@ ln_gemm_kernel(const __grid_constant__ CUtensorMap mapX, const __grid_constant__
   // attention projection: bit (2 * chunk + half) = that 128-column group has a non-zero bias (the epilogue skips the others)
   unsigned int* bias_flags = reinterpret_cast<unsigned int*>(tmem_slot + 2);
   if (threadIdx.x == 0) bias_flags[0] = 0u;
-  if (EPI == LG_EPI_ATTENTION) __syncthreads();
   if (threadIdx.x == 0) {
     for (int s = 0; s < 2; ++s) {
       mbar_init(&x_full[s], 1);
@@ -162,6 +161,9 @@ ln_gemm_kernel(const __grid_constant__ CUtensorMap mapX, const __grid_constant__
     *abort_flag = 0;
     fence_barrier_init();
   }
+  if (warp == LG_MMA_WARP) { tmem_alloc(tmem_slot, 512); tmem_relinquish(); }
+  __syncthreads();
+  lf_chain();
   // resident weights: straight copy of the pre-swizzled image
   {
     const uint4* src = reinterpret_cast<const uint4*>(p.wimg);
@@ -174,7 +176,6 @@ ln_gemm_kernel(const __grid_constant__ CUtensorMap mapX, const __grid_constant__
     }
     fence_async_smem();
   }
-  if (warp == LG_MMA_WARP) { tmem_alloc(tmem_slot, 512); tmem_relinquish(); }
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
@@ -892,7 +893,7 @@ static lf_status launch_triangle(lf_context* ctx, LnGemmParams& p, const PeerPtr
   const int64_t tiles = p.tile_per_row ? (int64_t)rows * p.tile_per_row : (p.rows + LG_ROWS - 1) / LG_ROWS;
   const int grid = (int)(tiles < ctx->sm_count ? tiles : ctx->sm_count);
   lf_prof_begin(ctx, LF_KERNEL_LN_GEMM);
-  ln_gemm_kernel<LG_EPI_TRIANGLE, OWNERS><<<grid, LG_THREADS, LG_TRIANGLE_SMEM, ctx->stream>>>(CUtensorMap{}, CUtensorMap{}, pm, p);
+  lf_launch(ctx, ln_gemm_kernel<LG_EPI_TRIANGLE, OWNERS>, grid, LG_THREADS, LG_TRIANGLE_SMEM, CUtensorMap{}, CUtensorMap{}, pm, p);
   lf_prof_end(ctx);
   ctx->launches++;
   return LF_OK;
@@ -971,7 +972,7 @@ static lf_status attention_project_impl(lf_context* ctx, ArenaCursor& cur, const
   const int64_t tiles = (p.rows + LG_ROWS - 1) / LG_ROWS;
   const int grid = (int)(tiles < ctx->sm_count ? tiles : ctx->sm_count);
   lf_prof_begin(ctx, LF_KERNEL_LN_GEMM);
-  ln_gemm_kernel<LG_EPI_ATTENTION><<<grid, LG_THREADS, ln_gemm_smem(528), ctx->stream>>>(CUtensorMap{}, CUtensorMap{}, PlaneMaps<0>{}, p);
+  lf_launch(ctx, ln_gemm_kernel<LG_EPI_ATTENTION, 0>, grid, LG_THREADS, ln_gemm_smem(528), CUtensorMap{}, CUtensorMap{}, PlaneMaps<0>{}, p);
   lf_prof_end(ctx);
   ctx->launches++;
   return LF_OK;
@@ -996,7 +997,7 @@ lf_status pair_bias_project(lf_context* ctx, ArenaCursor& cur, const void* pair,
   const int64_t tiles = (p.rows + LG_ROWS - 1) / LG_ROWS;
   const int grid = (int)(tiles < ctx->sm_count ? tiles : ctx->sm_count);
   lf_prof_begin(ctx, LF_KERNEL_LN_GEMM);
-  ln_gemm_kernel<LG_EPI_ATTENTION><<<grid, LG_THREADS, ln_gemm_smem(16), ctx->stream>>>(CUtensorMap{}, CUtensorMap{}, PlaneMaps<0>{}, p);
+  lf_launch(ctx, ln_gemm_kernel<LG_EPI_ATTENTION, 0>, grid, LG_THREADS, ln_gemm_smem(16), CUtensorMap{}, CUtensorMap{}, PlaneMaps<0>{}, p);
   lf_prof_end(ctx);
   ctx->launches++;
   return LF_OK;
@@ -1033,7 +1034,7 @@ lf_status attention_output(lf_context* ctx, ArenaCursor& cur, const op16* o, int
   const int grid = (int)(tiles < ctx->sm_count ? tiles : ctx->sm_count);
   lf_prof_begin(ctx, LF_KERNEL_LN_GEMM);
   // the fp16 rows are in logical order; the transposed scatter happens in the epilogue (or in the tensor map)
-  ln_gemm_kernel<LG_EPI_OUTPUT><<<grid, LG_THREADS, ln_gemm_smem(128, false, true), ctx->stream>>>(CUtensorMap{}, mo, PlaneMaps<0>{}, p);
+  lf_launch(ctx, ln_gemm_kernel<LG_EPI_OUTPUT, 0>, grid, LG_THREADS, ln_gemm_smem(128, false, true), CUtensorMap{}, mo, PlaneMaps<0>{}, p);
   lf_prof_end(ctx);
   ctx->launches++;
   return LF_OK;
@@ -1064,7 +1065,7 @@ lf_status triangle_output(lf_context* ctx, ArenaCursor& cur, const op16* x, int 
   p.tma_out = (!p.out_bf16 && (resid == nullptr || resid == out)) ? 1 : 0;
   if (p.tma_out) LF_TRY(make_map_f32_rows_half(ctx, &mo, out, (uint64_t)n, (uint64_t)rows, 512, (uint64_t)n * 512, 32, 1));
   lf_prof_begin(ctx, LF_KERNEL_TRIANGLE_OUTPUT);
-  ln_gemm_kernel<LG_EPI_TRI_OUT><<<grid, LG_THREADS, ln_gemm_smem(256, true, false), ctx->stream>>>(mapX, mo, PlaneMaps<0>{}, p);
+  lf_launch(ctx, ln_gemm_kernel<LG_EPI_TRI_OUT, 0>, grid, LG_THREADS, ln_gemm_smem(256, true, false), mapX, mo, PlaneMaps<0>{}, p);
   lf_prof_end(ctx);
   ctx->launches++;
   return LF_OK;

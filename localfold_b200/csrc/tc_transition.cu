@@ -97,9 +97,11 @@ __global__ void __launch_bounds__(TR_THREADS, 1) transition_kernel(const __grid_
     *abort_flag = 0;
     fence_barrier_init();
   }
+  if (warp == 24) { tmem_alloc(tmem_slot, 512); tmem_relinquish(); }
+  __syncthreads();
+  lf_chain();
   for (int i = threadIdx.x; i < (SWIGLU ? 1024 : 512); i += TR_THREADS) sB1[i] = p.b1[i];
   if (threadIdx.x < 128) sB2[threadIdx.x] = p.b2[threadIdx.x];
-  if (warp == 24) { tmem_alloc(tmem_slot, 512); tmem_relinquish(); }
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
@@ -522,9 +524,9 @@ lf_status transition_run(lf_context* ctx, ArenaCursor& cur, const void* act, int
   const int grid = (int)(tiles < ctx->sm_count ? tiles : ctx->sm_count);
   lf_prof_begin(ctx, LF_KERNEL_TRANSITION);
   if (w->kind == LF_WEIGHTS_TRANSITION_AF3)
-    transition_kernel<true><<<grid, TR_THREADS, TR_SMEM, ctx->stream>>>(mo, p);
+    lf_launch(ctx, transition_kernel<true>, grid, TR_THREADS, TR_SMEM, mo, p);
   else
-    transition_kernel<false><<<grid, TR_THREADS, TR_SMEM, ctx->stream>>>(mo, p);
+    lf_launch(ctx, transition_kernel<false>, grid, TR_THREADS, TR_SMEM, mo, p);
   lf_prof_end(ctx);
   ctx->launches++;
   return LF_OK;
