@@ -230,24 +230,21 @@ ln_gemm_kernel(const __grid_constant__ CUtensorMap mapX, const __grid_constant__
       float s4[4] = {0.f, 0.f, 0.f, 0.f};      // four chains instead of one of 16 dependent additions
 #pragma unroll
       for (int e = 0; e < 16; ++e) s4[e & 3] += v[e];
-      float sum = (s4[0] + s4[1]) + (s4[2] + s4[3]);
-      sum += __shfl_xor_sync(0xffffffffu, sum, 1);
-      sum += __shfl_xor_sync(0xffffffffu, sum, 2);
-      sum += __shfl_xor_sync(0xffffffffu, sum, 4);
-      const float mean = sum * (1.0f / LG_K);
+      // mean and sum of squared differences of the lane's 16 values, then of 32, 64 and 128 by pairwise merging (Chan, Golub and
+      // LeVeque): as accurate as two passes, and the two reductions across lanes are one chain of three exchanges
+      float mean = ((s4[0] + s4[1]) + (s4[2] + s4[3])) * (1.0f / 16.0f);
       float q4[4] = {0.f, 0.f, 0.f, 0.f};
-      if (p.variance == 2) {
 #pragma unroll
-        for (int e = 0; e < 16; ++e) q4[e & 3] = fmaf(v[e], v[e], q4[e & 3]);
-      } else {
-#pragma unroll
-        for (int e = 0; e < 16; ++e) { const float d = v[e] - mean; q4[e & 3] = fmaf(d, d, q4[e & 3]); }
-      }
+      for (int e = 0; e < 16; ++e) { const float d = v[e] - mean; q4[e & 3] = fmaf(d, d, q4[e & 3]); }
       float sq = (q4[0] + q4[1]) + (q4[2] + q4[3]);
-      sq += __shfl_xor_sync(0xffffffffu, sq, 1);
-      sq += __shfl_xor_sync(0xffffffffu, sq, 2);
-      sq += __shfl_xor_sync(0xffffffffu, sq, 4);
-      const float var = p.variance == 2 ? sq * (1.0f / LG_K) - mean * mean : sq * (1.0f / LG_K);
+#pragma unroll
+      for (int step = 1; step < 8; step *= 2) {
+        const float other = __shfl_xor_sync(0xffffffffu, mean, step), more = __shfl_xor_sync(0xffffffffu, sq, step);
+        const float d = other - mean;
+        sq = fmaf(d * d, 8.0f * step, sq + more);
+        mean = 0.5f * (mean + other);
+      }
+      const float var = sq * (1.0f / LG_K);
       float inv = rsqrtf(var + p.eps);
       inv = inv * (1.5f - 0.5f * (var + p.eps) * inv * inv);
       const float shift = -mean * inv;
