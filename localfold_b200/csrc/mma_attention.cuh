@@ -93,7 +93,7 @@ struct AttentionShape {
   int64_t ld, term_stride;              // rows and terms of q | k | v | gate, in 16-bit elements (multiples of 8)
   int64_t ldo, out_stride;              // ... and of the output
   int gate_logits;                      // fp16: the gate columns hold logits (the projection applies no sigmoid)
-  int ldb;                              // fp16 bias: elements from one query's keys to the next (even)
+  int ldb;                              // fp16 bias: elements from one query's keys to the next (a multiple of 8, as the bias's address)
   int wb, wq;                           // warps of a block: wb batch rows x wq groups of 16 queries
   int kt;                               // keys of a staged tile, a multiple of 32
   int mk;                               // keys whose mask terms are held at a time, a multiple of kt
@@ -101,8 +101,13 @@ struct AttentionShape {
 
 constexpr int AT_STEP = 32;                                                   // keys of one step of a warp
 __host__ __device__ constexpr int at_pitch(int D) { return 8 * ((D / 8) | 1); }      // odd in 16-byte units: ldmatrix rows spread over the banks
+// fp16: a step's 32 keys are dealt to the tensor core's columns so that a thread holds eight neighbouring ones (column 8 n + 2 t + e is key
+// 8 t + 2 n + e): its bias and mask terms are then whole 16-byte pieces, two loads a row and step instead of eight (291 -> 227 us, 384 x
+// 384 with 4 heads of 16).  Rows of every eight keys are shifted by 32 bytes, so that the rows of a matrix still spread over the banks.  A
+// float32 bias has no such pieces where the length is odd, and keeps the plain order.
+__host__ __device__ constexpr int at_rows(int D, int terms, int keys) { return keys * (at_pitch(D) + (terms == 1 ? 2 : 0)); }
 __host__ __device__ constexpr size_t attention_smem(int D, int terms, int wb, int kt, int mk) {
-  return (size_t)wb * (2 * 2 * terms * kt * at_pitch(D) * 2 + mk * 4);
+  return (size_t)wb * (2 * 2 * terms * at_rows(D, terms, kt) * 2 + mk * 4);
 }
 
 //   qkvg: [TERMS][rows][ld] = terms of (q | k | v | sigmoid(gate) | ...) in logical row order, a head of each D channels wide
@@ -129,7 +134,7 @@ attention_kernel(const uint16_t* __restrict__ qkvg, const void* __restrict__ bia
   const TBias* bias = static_cast<const TBias*>(bias_any);
   constexpr int TOP = TERMS - 1;                    // highest order of a term product that is kept: i + j <= TOP
   constexpr int KT = AT_STEP, PITCH = at_pitch(D), NK = D / 16, TAIL = (D / 8) & 1, ND = D / 8;
-  const int plane = s.kt * PITCH;                   // elements of one term of one staged tile
+  const int plane = at_rows(D, TERMS, s.kt);        // elements of one term of one staged tile
   extern __shared__ uint4 at_sm[];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, g = lane >> 2, t = lane & 3;
   const int wb = warp / s.wq, wq = warp % s.wq;
@@ -151,7 +156,7 @@ attention_kernel(const uint16_t* __restrict__ qkvg, const void* __restrict__ bia
       for (int bb = 0; bb < s.wb; ++bb) {
         const bool ok = j0 + j < Q && b0 + bb < s.batch;
         const uint16_t* src = ok ? qkvg + ((int64_t)(b0 + bb) * Q + j0 + j) * ld + HD + h * D + e : qkvg;
-        uint16_t* dst = kv_s + (buf * s.wb + bb) * 2 * TERMS * plane + j * PITCH + e;
+        uint16_t* dst = kv_s + (buf * s.wb + bb) * 2 * TERMS * plane + j * PITCH + (TERMS == 1 ? (j >> 3) * 16 : 0) + e;
 #pragma unroll
         for (int which = 0; which < 2; ++which)
 #pragma unroll
@@ -194,35 +199,39 @@ attention_kernel(const uint16_t* __restrict__ qkvg, const void* __restrict__ bia
 
   // the bias of a tile's keys: this thread's two rows, eight columns each
   const int64_t bias_ld = TERMS == 1 ? s.ldb : Q;
-  const bool pairs = TERMS == 1 || (Q & 1) == 0;
-  const TBias* bias0 = BIAS ? bias + ((int64_t)h * Q + (row0 < Q ? row0 : 0)) * bias_ld + 2 * t : nullptr;
-  const TBias* bias1 = BIAS ? bias + ((int64_t)h * Q + (row1 < Q ? row1 : 0)) * bias_ld + 2 * t : nullptr;
-  float bv[4][4];
+  const bool pairs = (Q & 1) == 0;
+  constexpr int KEY_T = TERMS == 1 ? 8 : 2, KEY_N = TERMS == 1 ? 2 : 8;      // keys from a thread to the next and from a group of eight columns to the next
+  const TBias* bias0 = BIAS ? bias + ((int64_t)h * Q + (row0 < Q ? row0 : 0)) * bias_ld + KEY_T * t : nullptr;
+  const TBias* bias1 = BIAS ? bias + ((int64_t)h * Q + (row1 < Q ? row1 : 0)) * bias_ld + KEY_T * t : nullptr;
+  float bv[TERMS == 1 ? 1 : 4][4];
+  uint4 bh[2];                                      // fp16: the eight values of each row as they come
   auto load_bias = [&](int j0) {
     if (!BIAS) return;
+    if constexpr (TERMS == 1) {
+      bh[0] = bh[1] = make_uint4(0u, 0u, 0u, 0u);
+      if (j0 + 8 * t + 8 <= s.ldb) {
+        bh[0] = __ldg(reinterpret_cast<const uint4*>(bias0 + j0));
+        bh[1] = __ldg(reinterpret_cast<const uint4*>(bias1 + j0));
+      }
+    } else {
 #pragma unroll
-    for (int n = 0; n < 4; ++n) {
-      const int j = j0 + n * 8;
-      if (pairs && j + 2 * t < Q) {
-        float2 x, y;
-        if constexpr (TERMS == 1) {
-          x = __half22float2(__ldg(reinterpret_cast<const __half2*>(bias0 + j)));
-          y = __half22float2(__ldg(reinterpret_cast<const __half2*>(bias1 + j)));
+      for (int n = 0; n < 4; ++n) {
+        const int j = j0 + n * 8;
+        if (pairs && j + 2 * t < Q) {
+          const float2 x = __ldg(reinterpret_cast<const float2*>(bias0 + j)), y = __ldg(reinterpret_cast<const float2*>(bias1 + j));
+          bv[n][0] = x.x; bv[n][1] = x.y; bv[n][2] = y.x; bv[n][3] = y.y;
         } else {
-          x = __ldg(reinterpret_cast<const float2*>(bias0 + j));
-          y = __ldg(reinterpret_cast<const float2*>(bias1 + j));
+          bv[n][0] = j + 2 * t < Q ? __ldg(bias0 + j) : 0.f;
+          bv[n][1] = j + 2 * t + 1 < Q ? __ldg(bias0 + j + 1) : 0.f;
+          bv[n][2] = j + 2 * t < Q ? __ldg(bias1 + j) : 0.f;
+          bv[n][3] = j + 2 * t + 1 < Q ? __ldg(bias1 + j + 1) : 0.f;
         }
-        bv[n][0] = x.x; bv[n][1] = x.y; bv[n][2] = y.x; bv[n][3] = y.y;
-      } else if constexpr (TERMS == 1) {
-        bv[n][0] = bv[n][1] = bv[n][2] = bv[n][3] = 0.f;
-      } else {
-        bv[n][0] = j + 2 * t < Q ? __ldg(bias0 + j) : 0.f;
-        bv[n][1] = j + 2 * t + 1 < Q ? __ldg(bias0 + j + 1) : 0.f;
-        bv[n][2] = j + 2 * t < Q ? __ldg(bias1 + j) : 0.f;
-        bv[n][3] = j + 2 * t + 1 < Q ? __ldg(bias1 + j + 1) : 0.f;
       }
     }
   };
+
+  // fp16: where the row of column lane % 8 of column group n lies (group n + 2 is four keys further on)
+  auto row_of = [&](int n) { return (((lane & 7) >> 1) * 8 + n * 2 + (lane & 1)) * PITCH + ((lane & 7) >> 1) * 16; };
 
   float o[ND][4];
 #pragma unroll
@@ -247,7 +256,7 @@ attention_kernel(const uint16_t* __restrict__ qkvg, const void* __restrict__ bia
 #pragma unroll 1
     for (int step = 0; step < s.kt && tile * s.kt + step < Q; step += KT) {
     const int key0 = tile * s.kt + step;
-    const uint16_t* k_s = kv_s + (buf * s.wb + wb) * 2 * TERMS * plane + step * PITCH;
+    const uint16_t* k_s = kv_s + (buf * s.wb + wb) * 2 * TERMS * plane + at_rows(D, TERMS, step);
     const uint16_t* v_s = k_s + TERMS * plane;
     const float* ms = mask_s + wb * s.mk + key0 - mask0;
     // ---- S = Q K^T for 32 keys (four accumulators in flight): small term products first, the leading one last ----
@@ -259,7 +268,7 @@ attention_kernel(const uint16_t* __restrict__ qkvg, const void* __restrict__ bia
     {
       uint32_t kb[TERMS][2][4];
       // matrices (keys 0-7, k 0-7), (keys 0-7, k 8-15), (keys 8-15, k 0-7), (keys 8-15, k 8-15) of each 16 keys
-      const uint16_t* base = k_s + ((lane & 7) + (lane >> 4) * 8) * PITCH + ((lane >> 3) & 1) * 8;
+      const uint16_t* base = k_s + (TERMS == 1 ? row_of(lane >> 4) : ((lane & 7) + (lane >> 4) * 8) * PITCH) + ((lane >> 3) & 1) * 8;
       // the term products below the leading one first, over all channels; the leading ones last
 #pragma unroll
       for (int pass = TOP; pass >= 0; pass -= 2) {
@@ -268,7 +277,7 @@ attention_kernel(const uint16_t* __restrict__ qkvg, const void* __restrict__ bia
 #pragma unroll
           for (int i = 0; i <= pass; ++i)
 #pragma unroll
-            for (int grp = 0; grp < 2; ++grp) ldmatrix4<false>(kb[i][grp], base + i * plane + grp * 16 * PITCH + kk * 16);
+            for (int grp = 0; grp < 2; ++grp) ldmatrix4<false>(kb[i][grp], base + i * plane + grp * (TERMS == 1 ? 4 : 16) * PITCH + kk * 16);
 #pragma unroll
           for (int order = pass; order >= (pass ? 1 : 0); --order)        // terms i and order - i
 #pragma unroll
@@ -282,7 +291,7 @@ attention_kernel(const uint16_t* __restrict__ qkvg, const void* __restrict__ bia
         if (TAIL) {
           // matrices: keys 0-7, 8-15, 16-23, 24-31 of the last eight channels
 #pragma unroll
-          for (int i = 0; i <= pass; ++i) ldmatrix4<false>(kb[i][0], k_s + i * plane + lane * PITCH + NK * 16);
+          for (int i = 0; i <= pass; ++i) ldmatrix4<false>(kb[i][0], k_s + i * plane + (TERMS == 1 ? row_of(lane >> 3) : lane * PITCH) + NK * 16);
 #pragma unroll
           for (int order = pass; order >= (pass ? 1 : 0); --order)
 #pragma unroll
@@ -297,11 +306,24 @@ attention_kernel(const uint16_t* __restrict__ qkvg, const void* __restrict__ bia
     // ---- logits ----
 #pragma unroll
     for (int n = 0; n < 4; ++n) {
-      const float2 m2 = *reinterpret_cast<const float2*>(ms + n * 8 + 2 * t);
+      const float2 m2 = *reinterpret_cast<const float2*>(ms + KEY_T * t + KEY_N * n);
+      float add[4] = {0.f, 0.f, 0.f, 0.f};
+      if constexpr (BIAS && TERMS == 1) {
+#pragma unroll
+        for (int r = 0; r < 2; ++r) {
+          const uint32_t w = n == 0 ? bh[r].x : n == 1 ? bh[r].y : n == 2 ? bh[r].z : bh[r].w;
+          const float2 v = __half22float2(*reinterpret_cast<const __half2*>(&w));
+          add[2 * r] = v.x;
+          add[2 * r + 1] = v.y;
+        }
+      } else if constexpr (BIAS) {
+#pragma unroll
+        for (int e = 0; e < 4; ++e) add[e] = bv[n][e];
+      }
 #pragma unroll
       for (int e = 0; e < 4; ++e) {
         l[n][e] = fmaf(l[n][e], s.scale, (e & 1) ? m2.y : m2.x);
-        if (BIAS) l[n][e] += bv[n][e];
+        if (BIAS) l[n][e] += add[e];
         if (s.clamp) l[n][e] = fminf(fmaxf(l[n][e], -1e8f), 1e8f);
       }
     }
@@ -310,7 +332,7 @@ attention_kernel(const uint16_t* __restrict__ qkvg, const void* __restrict__ bia
       for (int n = 0; n < 4; ++n)
 #pragma unroll
         for (int e = 0; e < 4; ++e)
-          if (key0 + n * 8 + 2 * t + (e & 1) >= Q) l[n][e] = -INFINITY;
+          if (key0 + KEY_T * t + KEY_N * n + (e & 1) >= Q) l[n][e] = -INFINITY;
     }
     if (BIAS && key0 + KT < Q) load_bias(key0 + KT);      // for the next step
     auto row_max = [&](int r) {
@@ -397,7 +419,7 @@ attention_kernel(const uint16_t* __restrict__ qkvg, const void* __restrict__ bia
         uint32_t vb[TERMS][4];
 #pragma unroll
         for (int i = 0; i < TERMS; ++i) {
-          const uint16_t* base = v_s + i * plane + (grp * 16 + (lane & 15)) * PITCH + np * 8;
+          const uint16_t* base = v_s + i * plane + (TERMS == 1 ? row_of((lane >> 3) & 1) + grp * 4 * PITCH : (grp * 16 + (lane & 15)) * PITCH) + np * 8;
           if (np + 1 < ND) ldmatrix4<true>(vb[i], base + (lane >> 4) * 8);
           else ldmatrix2<true>(vb[i][0], vb[i][1], base);
         }
