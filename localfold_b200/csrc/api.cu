@@ -1204,8 +1204,17 @@ lf_status tri_half(lf_context* ctx, ArenaCursor& cur, const TriArgs& a) {
   LAUNCH(ctx, cur, rows::trimul_gate_half_kernel, dim3((unsigned)(n * lf_ceil_div(n, 64)), lf_ceil_div(c, 32)), 256, 0, p4, a.mask, c, n, ld, ga, gb);
   const float xscale = ldexpf(1.0f, -(int)(0.5f * log2f((float)n)));
   LF_TRY(tc::contract(ctx, cur, ga, gb, x, n, ld, c, a.incoming, xscale));
-  LAUNCH(ctx, cur, (rows::center_norm_kernel<op16, rows::LN_HALF>), dim3((unsigned)(n * lf_ceil_div(n, 32))), 256, (size_t)c * 33 * sizeof(float), x, c, n, ld,
-         f[TRI_LNO_G], f[TRI_LNO_B], a.eps, a.variance, (a.divide ? 1.0f / n : 1.0f) / xscale, c, (void*)xn, (int64_t)0);
+  const float center_scale = (a.divide ? 1.0f / n : 1.0f) / xscale;
+  const unsigned center_tiles = (unsigned)(n * lf_ceil_div(n, 64));
+  const size_t center_smem = ((size_t)c * 72 + (size_t)64 * (c + 8)) * sizeof(op16);
+#define CENTER_HALF(G_) LAUNCH(ctx, cur, (rows::center_norm_half_kernel<G_>), center_tiles, 256, center_smem, x, c, n, ld, f[TRI_LNO_G], f[TRI_LNO_B], a.eps, a.variance, center_scale, xn)
+  if (c <= 32) CENTER_HALF(4);
+  else if (c <= 64) CENTER_HALF(8);
+  else if (c <= 128) CENTER_HALF(16);
+  else
+    LAUNCH(ctx, cur, (rows::center_norm_kernel<op16, rows::LN_HALF>), dim3((unsigned)(n * lf_ceil_div(n, 32))), 256, (size_t)c * 33 * sizeof(float), x, c, n, ld,
+           f[TRI_LNO_G], f[TRI_LNO_B], a.eps, a.variance, center_scale, c, (void*)xn, (int64_t)0);
+#undef CENTER_HALF
   LF_TRY(hgemm(ctx, cur, xn, gemm_operand(a.w, 1), proj, P, cz, c, f[TRI_BZ]));
   LF_TRY(hgemm(ctx, cur, zn, gemm_operand(a.w, 2), gate, P, cz, cz, f[TRI_BG]));
   LAUNCH(ctx, cur, (rows::finish_gate_half_kernel<T>), lf_ceil_div(P * (cz / 8), 256), 256, 0, proj, gate, a.residual ? (const T*)a.z : (const T*)nullptr,

@@ -41,7 +41,7 @@ def test_transition_edges(dev, rows, c, hidden, af3):
     assert oracle.relative_l2(got, want) <= 1e-6
 
 
-@pytest.mark.parametrize("n,c,incoming", [(1, 8, False), (63, 16, True), (64, 32, False), (65, 24, True), (127, 8, False), (129, 16, True), (200, 12, False), (530, 8, False), (530, 8, True)])
+@pytest.mark.parametrize("n,c,incoming", [(1, 8, False), (63, 16, True), (64, 32, False), (65, 24, True), (127, 8, False), (129, 16, True), (200, 12, False), (530, 8, False), (530, 8, True), (70, 72, False), (33, 136, True)])
 @pytest.mark.parametrize("precision,tol", [("f32", 2e-6), ("bf16", 8e-3)])
 def test_triangle_edges(dev, n, c, incoming, precision, tol):
     import localfold_b200 as lf
