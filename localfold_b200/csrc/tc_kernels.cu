@@ -200,24 +200,17 @@ constexpr int CT_A_BYTES = CT_BM * CT_BK * 2;   // 16 KiB
 constexpr int CT_B_BYTES = CT_BN * CT_BK * 2;   // 32 KiB
 constexpr int CT_STAGE_BYTES = CT_A_BYTES + CT_B_BYTES;
 constexpr int CT_OUT_STAGE = 32 * 256;          // per epilogue warp: 32 rows x 128 fp16 columns, for stores into a peer's memory
-// EW epilogue warps: 4 for the triangle contraction (long k loops hide the epilogue), 8 for the plain GEMMs, whose k
+// EW epilogue warps: 4 for the triangle contraction (long k loops hide the epilogue), 8 for the grouped outer product, whose k
 // loop of 4 to 16 blocks is shorter than a 4-warp epilogue of the 128 x 256 tile; the 8-warp form gives a stage
 // of the operand ring to the four extra staging areas.
 constexpr int ct_stages(int ew) { return ew == 8 ? 3 : CT_STAGES; }
 constexpr int ct_smem(int ew) { return ct_stages(ew) * CT_STAGE_BYTES + 1024 /*alignment slack*/ + 256 /*barriers*/ + ew * CT_OUT_STAGE; }
 constexpr int ct_threads(int ew) { return 64 + 32 * ew; }
 
-// Extras of the plain-GEMM uses of the kernel (local stores): a bias per output column and a ReLU in the epilogue;
-// `group_c` > 0: rows are (i, a) and columns (j, b) with a, b < group_c, and element (i, a, j, b) is stored at
-// ((i * group_n + j) * group_c + a) * group_c + b - the outer product mean's sums grouped per pair (i, j), which a
-// warp writes as whole 2 * group_c^2-byte runs.  `staged`: local rows leave in 256-byte runs through the staging
-// rows, as rows bound for a peer do (a GEMM with a short k loop is bound by its stores otherwise).
-struct ContractExtra { const float* bias; int relu; int group_c; int group_n; int staged; };
-
-__device__ __forceinline__ uint32_t relu_half2(uint32_t v) {      // max(v, 0) on two packed fp16 values
-  const __half2 r = __hmax2(*reinterpret_cast<const __half2*>(&v), __float2half2_rn(0.f));
-  return *reinterpret_cast<const uint32_t*>(&r);
-}
+// The outer product mean's use: with `group_c` > 0 rows are (i, a) and columns (j, b) with a, b < group_c, and element (i, a, j, b) is stored at
+// ((i * group_n + j) * group_c + a) * group_c + b - the sums grouped per pair (i, j), which a warp writes as whole
+// 2 * group_c^2-byte runs.
+struct ContractExtra { int group_c; int group_n; };
 
 template <int MAJOR, int EW = 4>
 __global__ void __launch_bounds__(ct_threads(EW), 1)
@@ -341,16 +334,15 @@ contract_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant_
         dst_row = x + (int64_t)h * x_plane + (int64_t)gi * ldx + col0;
       }
       const int col_limit = (n_rows + 15) / 16 * 16 < ldx - col0 ? (n_rows + 15) / 16 * 16 : ldx - col0;
-      if (rows_per_rank > 0 || ex.staged) {
+      if (rows_per_rank > 0) {
         // Rows bound for another GPU leave in 256-byte runs: a thread holds a row of the accumulator, so its
         // own stores would be 16-byte pieces 32 rows apart, which NVLink carries as 32 small packets.  The
         // warp's 32 rows x 128 columns are turned round in shared memory (16-byte pieces swizzled by row)
         // and written two rows per instruction, 16 lanes x 16 bytes each.
         uint8_t* stage = out_stage + (warp - 2) * CT_OUT_STAGE;
         const int g_row0 = mi * CT_BM + q * 32;            // the warp's rows share an owner: rows_per_rank % 128 == 0
-        const int owner = rows_per_rank > 0 && g_row0 < m_rows ? g_row0 / rows_per_rank : 0;
-        op16* owner_base = rows_per_rank > 0 ? reinterpret_cast<op16*>(xpeer.p[owner]) + (int64_t)(ch0 + h) * x_plane + col0
-                                             : x + (int64_t)h * x_plane + col0;
+        const int owner = g_row0 < m_rows ? g_row0 / rows_per_rank : 0;
+        op16* owner_base = reinterpret_cast<op16*>(xpeer.p[owner]) + (int64_t)(ch0 + h) * x_plane + col0;
 #pragma unroll 1
         for (int half = (EW == 8 ? chalf : 0); half < (EW == 8 ? chalf + 1 : 2); ++half) {
 #pragma unroll 1
@@ -363,24 +355,11 @@ contract_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant_
               float o[8];
 #pragma unroll
               for (int e = 0; e < 8; ++e) o[e] = __uint_as_float(r[v * 8 + e]) * scale;
-              if (ex.bias) {
-                const int gj = nj * CT_BN + half * 128 + (cc * 4 + v) * 8;
-                if (gj + 8 <= n_rows) {      // bias is 16-byte aligned and gj a multiple of 8
-                  const float4 b0 = __ldg(reinterpret_cast<const float4*>(ex.bias + gj));
-                  const float4 b1 = __ldg(reinterpret_cast<const float4*>(ex.bias + gj + 4));
-                  o[0] += b0.x; o[1] += b0.y; o[2] += b0.z; o[3] += b0.w;
-                  o[4] += b1.x; o[5] += b1.y; o[6] += b1.z; o[7] += b1.w;
-                } else {
-#pragma unroll
-                  for (int e = 0; e < 8; ++e) o[e] += gj + e < n_rows ? __ldg(ex.bias + gj + e) : 0.f;
-                }
-              }
               uint4 pk;
               pk.x = pack_half2(o[0], o[1]);
               pk.y = pack_half2(o[2], o[3]);
               pk.z = pack_half2(o[4], o[5]);
               pk.w = pack_half2(o[6], o[7]);
-              if (ex.relu) { pk.x = relu_half2(pk.x); pk.y = relu_half2(pk.y); pk.z = relu_half2(pk.z); pk.w = relu_half2(pk.w); }
               *reinterpret_cast<uint4*>(stage + lane * 256 + (((cc * 4 + v) ^ (lane & 15)) << 4)) = pk;
             }
           }
@@ -410,23 +389,11 @@ contract_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant_
               float o[8];
 #pragma unroll
               for (int e = 0; e < 8; ++e) o[e] = __uint_as_float(r[v * 8 + e]) * scale;
-              if (ex.bias) {
-                if (gj + 8 <= n_rows) {      // bias is 16-byte aligned and gj a multiple of 8
-                  const float4 b0 = __ldg(reinterpret_cast<const float4*>(ex.bias + gj));
-                  const float4 b1 = __ldg(reinterpret_cast<const float4*>(ex.bias + gj + 4));
-                  o[0] += b0.x; o[1] += b0.y; o[2] += b0.z; o[3] += b0.w;
-                  o[4] += b1.x; o[5] += b1.y; o[6] += b1.z; o[7] += b1.w;
-                } else {
-#pragma unroll
-                  for (int e = 0; e < 8; ++e) o[e] += gj + e < n_rows ? __ldg(ex.bias + gj + e) : 0.f;
-                }
-              }
               uint4 pk;
               pk.x = pack_half2(o[0], o[1]);
               pk.y = pack_half2(o[2], o[3]);
               pk.z = pack_half2(o[4], o[5]);
               pk.w = pack_half2(o[6], o[7]);
-              if (ex.relu) { pk.x = relu_half2(pk.x); pk.y = relu_half2(pk.y); pk.z = relu_half2(pk.z); pk.w = relu_half2(pk.w); }
               if (ex.group_c) {
                 const int gc = ex.group_c;
                 *reinterpret_cast<uint4*>(x + ((((int64_t)(gi / gc) * ex.group_n + gj / gc) * gc + gi % gc) * gc + gj % gc)) = pk;
@@ -466,7 +433,6 @@ void configure_once() {
   std::call_once(per_device[dev], [] {
     cudaFuncSetAttribute(contract_kernel<0, 4>, cudaFuncAttributeMaxDynamicSharedMemorySize, ct_smem(4));
     cudaFuncSetAttribute(contract_kernel<1, 4>, cudaFuncAttributeMaxDynamicSharedMemorySize, ct_smem(4));
-    cudaFuncSetAttribute(contract_kernel<0, 8>, cudaFuncAttributeMaxDynamicSharedMemorySize, ct_smem(8));
     cudaFuncSetAttribute(contract_kernel<1, 8>, cudaFuncAttributeMaxDynamicSharedMemorySize, ct_smem(8));
     configure_ln_gemm();
     configure_attention();
@@ -482,7 +448,7 @@ bool contract_supported(int n, int c) { return n >= 1 && c >= 1 && g_encode != n
 static lf_status contract_impl(lf_context* ctx, ArenaCursor& cur, const op16* a, const op16* b, op16* x, int m_rows, int n_rows,
                                int k_len, int ld_ab, int ldx, int64_t x_plane, int col0, int c, int incoming, float scale,
                                const PeerPtrs* peers, int rows_per_rank, int ch0,
-                               ContractExtra ex = ContractExtra{nullptr, 0, 0, 0, 0});
+                               ContractExtra ex = ContractExtra{0, 0});
 
 lf_status contract_rect(lf_context* ctx, ArenaCursor& cur, const op16* a, const op16* b, op16* x, int m_rows, int n_rows,
                         int k_len, int ld_ab, int ldx, int64_t x_plane, int col0, int c, int incoming, float scale) {
@@ -503,7 +469,7 @@ lf_status contract_outer(lf_context* ctx, ArenaCursor& cur, const op16* left, co
   if (c == 32) return gemm_outer32(ctx, cur, left, right, out, cnt, n, k_len, scale);
   // x[(i, a)][(j, b)] = scale * sum_s left[s][(i, a)] right[s][(j, b)]: both operands MN-major, the kernel's "b" is its M operand
   return contract_impl(ctx, cur, right, left, out, cnt * c, n * c, k_len, n * c, n * c, 0, 0, 1, 1, scale, nullptr, 0, 0,
-                       ContractExtra{nullptr, 0, c, n, 0});
+                       ContractExtra{c, n});
 }
 
 static lf_status contract_impl(lf_context* ctx, ArenaCursor& cur, const op16* a, const op16* b, op16* x, int m_rows, int n_rows,
@@ -530,9 +496,9 @@ static lf_status contract_impl(lf_context* ctx, ArenaCursor& cur, const op16* a,
 #define CT_LAUNCH(MAJ, EWN) \
   lf_launch(ctx, contract_kernel<MAJ, EWN>, grid, ct_threads(EWN), ct_smem(EWN), mapA, mapB, x, m_rows, n_rows, k_len, ldx, x_plane, col0, c, \
       scale, (Status*)ctx->tc_status, peers ? *peers : PeerPtrs{}, rows_per_rank, ch0, ex)
-  const bool wide_epilogue = (ex.staged || ex.group_c) && !peers;      // the plain-GEMM uses
-  if (!incoming) { if (wide_epilogue) CT_LAUNCH(0, 8); else CT_LAUNCH(0, 4); }
-  else { if (wide_epilogue) CT_LAUNCH(1, 8); else CT_LAUNCH(1, 4); }
+  if (ex.group_c) CT_LAUNCH(1, 8);      // (always incoming)
+  else if (incoming) CT_LAUNCH(1, 4);
+  else CT_LAUNCH(0, 4);
 #undef CT_LAUNCH
   lf_prof_end(ctx);
   ctx->launches++;
@@ -541,6 +507,9 @@ static lf_status contract_impl(lf_context* ctx, ArenaCursor& cur, const op16* a,
 
 lf_status contract(lf_context* ctx, ArenaCursor& cur, const op16* a, const op16* b, op16* x, int n, int ld, int c,
                    int incoming, float scale) {
+  // Up to about eight k blocks a tile the epilogue decides, and the GEMM kernel's sixteen warps win (N = 384, 128 channels: 37 -> 31 us);
+  // from there on the contraction kernel's deeper ring does (N = 701: 101 against 111 us, N = 2048: 1.68 against 1.79 ms).
+  if (n < 512) return gemm_planes(ctx, cur, a, b, x, n, ld, c, incoming, scale);
   return contract_rect(ctx, cur, a, b, x, n, n, n, ld, ld, (int64_t)n * ld, 0, c, incoming, scale);
 }
 
