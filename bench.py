@@ -511,7 +511,7 @@ def main():
                                                    "the reference documents 195.6 ms per block for this shape through WebGPU on an A100")
         block_p.close()
         extra["evoformer_block_note"] = ("one AF2 Evoformer block at S=128, N=256, c_m=256 (the baseline's CPU-runnable configuration), "
-                                         "MSA and pair resident, mean of 6 blocks, L2 flushed between; _f32_ is the float32 SIMT mode")
+                                         "MSA and pair resident, mean of 6 blocks, L2 flushed between; _f32_ is the float32 mode")
         del flush, msa_d, pair_c1d
 
     # end to end through the public API with host buffers: pinned host pair in, pair out, every step
