@@ -15,13 +15,13 @@ using namespace tc05;
 // from the sum.  The epilogue adds the two and keeps the sum of the k blocks in its registers, in round-to-nearest, while the
 // accumulators start afresh: errors against float64 are at or below those of a float32 FMA chain (1.9e-7 against
 // 3.1e-7 to 4.8e-7 for the triangle update at 203 to 700; with all of k in TMEM 1.3e-6 for a transition of 384 channels).
-// Warp roles: 0 = TMA producer, 1 = MMA issuer (owns TMEM), 2..9 = epilogue (lane quadrant = warp % 4, half of the columns).
-// Bound by the operands' way from L2 into shared memory (96 KiB per 768 cycles of tensor work).  41 209 x 512 x 128: 28
-// TFLOP/s with 4 x 4 results a thread on the FMA pipe.
-constexpr int G3_BM = 128, G3_BN = 128, G3_BK = 64, G3_STAGES = 2, G3_EPI = 8;
+// Warp roles: 0 = TMA producer, 1 = MMA issuer (owns TMEM), 2..17 = epilogue (lane quadrant = warp % 4, a quarter of the columns).
+// With two k blocks a tile (K = 128) the epilogue is what bounds it - eight warps and scalar bias loads took 41 us a launch on average for
+// the float32 pair block at N = 203, this 35 - and the operands' way from L2 into shared memory (96 KiB per 1560 cycles of tensor work) with more.
+constexpr int G3_BM = 128, G3_BN = 128, G3_BK = 64, G3_STAGES = 2, G3_EPI = 16;
 constexpr int G3_PLANE = G3_BM * G3_BK * 2;            // 16 KiB: one term of one operand
 constexpr int G3_STAGE = 6 * G3_PLANE;
-constexpr int G3_OUT = 4096;                           // per epilogue warp: 32 rows x 32 columns of float32
+constexpr int G3_OUT = 2048;                           // per epilogue warp: 32 rows x 64 bytes
 constexpr int G3_SMEM = G3_STAGES * G3_STAGE + G3_EPI * G3_OUT + 256 + 1024;
 constexpr int G3_THREADS = 64 + 32 * G3_EPI;
 constexpr int G3_CHUNK = 1;                            // k blocks per accumulation in TMEM
@@ -139,29 +139,30 @@ gemm3_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant__ C
       }
     }
   } else {
-    const int q = warp & 3, half = (warp - 2) >> 2;      // TMEM lane quadrant, half of the tile's columns
+    const int q = warp & 3, part = (warp - 2) >> 2;      // TMEM lane quadrant, 32 of the tile's columns
     uint8_t* stage = out_stage + (warp - 2) * G3_OUT;
     const int chunks = (kblocks + G3_CHUNK - 1) / G3_CHUNK;
     uint32_t it = 0;
     bool ok = true;
     for (int64_t t = blockIdx.x; t < total && ok; t += gridDim.x) {
       const int h = (int)(t / per), rem = (int)(t % per), mi = rem / tiles_n, nj = rem % tiles_n;
-      float acc[64];
+      const int col0 = nj * G3_BN + part * 32;
+      float v[32];
 #pragma unroll 1
       for (int c = 0; c < chunks; ++c, ++it) {
         if (!mbar_wait(&tmem_full[it & 1], (it >> 1) & 1, abort_flag, p.status, 104)) { ok = false; break; }
         tc_fence_after();
-        const uint32_t d = tmem_base + ((uint32_t)(q * 32) << 16) + (it & 1) * 256 + half * 64;
+        const uint32_t d = tmem_base + ((uint32_t)(q * 32) << 16) + (it & 1) * 256 + part * 32;
 #pragma unroll
-        for (int c16 = 0; c16 < 4; ++c16) {
+        for (int c16 = 0; c16 < 2; ++c16) {
           uint32_t lead[16], rest[16];
           tmem_ld16(d + c16 * 16, lead);
           tmem_ld16(d + 128 + c16 * 16, rest);
           tmem_ld_wait();
 #pragma unroll
           for (int e = 0; e < 16; ++e) {
-            const float v = __uint_as_float(lead[e]) + __uint_as_float(rest[e]);
-            acc[c16 * 16 + e] = c ? acc[c16 * 16 + e] + v : v;
+            const float x = __uint_as_float(lead[e]) + __uint_as_float(rest[e]);
+            v[c16 * 16 + e] = c ? v[c16 * 16 + e] + x : x;
           }
         }
         tc_fence_before();
@@ -170,13 +171,18 @@ gemm3_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant__ C
       }
       if (!ok) break;
       const int row0 = mi * G3_BM + q * 32;
+      if (col0 >= (p.out ? p.n : (int)p.ldo) || row0 >= p.m) continue;
+      {
+        if (p.bias && col0 < p.bias_n) {      // through the staging rows: four at a time, the same for every lane
+          float* bias = reinterpret_cast<float*>(stage);
+          bias[lane] = col0 + lane < p.bias_n ? __ldg(p.bias + col0 + lane) : 0.f;
+          __syncwarp();
 #pragma unroll
-      for (int ch = 0; ch < 2; ++ch) {                   // 32 columns at a time
-        const int col0 = nj * G3_BN + half * 64 + ch * 32;
-        float* v = acc + ch * 32;
-        if (p.bias) {
-#pragma unroll
-          for (int e = 0; e < 32; ++e) v[e] += col0 + e < p.bias_n ? __ldg(p.bias + col0 + e) : 0.f;
+          for (int e = 0; e < 32; e += 4) {
+            const float4 b = *reinterpret_cast<const float4*>(bias + e);
+            v[e] += b.x; v[e + 1] += b.y; v[e + 2] += b.z; v[e + 3] += b.w;
+          }
+          __syncwarp();
         }
         if (p.relu) {
 #pragma unroll
@@ -185,30 +191,34 @@ gemm3_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant__ C
         if (col0 + 32 > p.sigmoid_col0 && col0 < p.sigmoid_col1) {
 #pragma unroll
           for (int e = 0; e < 32; ++e)
-            if (col0 + e >= p.sigmoid_col0 && col0 + e < p.sigmoid_col1) v[e] = 1.0f / (1.0f + expf(-v[e]));
+            if (col0 + e >= p.sigmoid_col0 && col0 + e < p.sigmoid_col1) v[e] = __frcp_rn(1.0f + expf(-v[e]));
         }
         if (p.out) {
-          // the warp's 32 x 32 values turned round in shared memory (16-byte pieces swizzled by row): whole 128-byte runs leave
+          // the warp's 32 x 32 values turned round in shared memory, 16 columns at a time (16-byte pieces swizzled by row): 64-byte runs leave
 #pragma unroll
-          for (int k4 = 0; k4 < 8; ++k4)
-            *reinterpret_cast<float4*>(stage + lane * 128 + ((k4 ^ (lane & 7)) << 4)) = make_float4(v[k4 * 4], v[k4 * 4 + 1], v[k4 * 4 + 2], v[k4 * 4 + 3]);
-          __syncwarp();
+          for (int c16 = 0; c16 < 2; ++c16) {
 #pragma unroll
-          for (int i = 0; i < 8; ++i) {
-            const int r = i * 4 + (lane >> 3), piece = lane & 7, col = col0 + piece * 4;
-            const float4 x = *reinterpret_cast<const float4*>(stage + r * 128 + ((piece ^ (r & 7)) << 4));
-            if (row0 + r < p.m) {
-              float* dst = p.out + (int64_t)h * p.batch_stride + (int64_t)(row0 + r) * p.ldo + col;
-              if (col + 4 <= p.n && (p.ldo & 3) == 0) *reinterpret_cast<float4*>(dst) = x;
-              else {
-                if (col < p.n) dst[0] = x.x;
-                if (col + 1 < p.n) dst[1] = x.y;
-                if (col + 2 < p.n) dst[2] = x.z;
-                if (col + 3 < p.n) dst[3] = x.w;
+            for (int k4 = 0; k4 < 4; ++k4)
+              *reinterpret_cast<float4*>(stage + lane * 64 + ((k4 ^ ((lane >> 1) & 3)) << 4)) =
+                  make_float4(v[c16 * 16 + k4 * 4], v[c16 * 16 + k4 * 4 + 1], v[c16 * 16 + k4 * 4 + 2], v[c16 * 16 + k4 * 4 + 3]);
+            __syncwarp();
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+              const int r = i * 8 + (lane >> 2), piece = lane & 3, col = col0 + c16 * 16 + piece * 4;
+              const float4 x = *reinterpret_cast<const float4*>(stage + r * 64 + ((piece ^ ((r >> 1) & 3)) << 4));
+              if (row0 + r < p.m) {
+                float* dst = p.out + (int64_t)h * p.batch_stride + (int64_t)(row0 + r) * p.ldo + col;
+                if (col + 4 <= p.n && (p.ldo & 3) == 0) *reinterpret_cast<float4*>(dst) = x;
+                else {
+                  if (col < p.n) dst[0] = x.x;
+                  if (col + 1 < p.n) dst[1] = x.y;
+                  if (col + 2 < p.n) dst[2] = x.z;
+                  if (col + 3 < p.n) dst[3] = x.w;
+                }
               }
             }
+            __syncwarp();
           }
-          __syncwarp();
         } else {
           // ... or their terms, 64-byte runs a row and term (ldo a multiple of 8)
 #pragma unroll 1
