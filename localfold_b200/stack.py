@@ -9,6 +9,7 @@ for the whole stack (``pairTensor`` / ``pairBuffer`` in the reference).
 from __future__ import annotations
 
 import ctypes
+import math
 
 import numpy as np
 
@@ -227,12 +228,12 @@ class EvoformerStackGpu:
 
         def resident(value, shape, copy):
             if getattr(value, "is_cuda", False):
-                if value.numel() != int(np.prod(shape)):
-                    raise nat.RangeError(f"tensor has {value.numel()} values; expected {int(np.prod(shape))}")
+                if value.numel() != math.prod(shape):
+                    raise nat.RangeError(f"tensor has {value.numel()} values; expected {math.prod(shape)}")
                 return value.view(shape), True
             host = np.asarray(value, np.float32)
-            if host.size != int(np.prod(shape)):
-                raise nat.RangeError(f"array has {host.size} values; expected {int(np.prod(shape))}")
+            if host.size != math.prod(shape):
+                raise nat.RangeError(f"array has {host.size} values; expected {math.prod(shape)}")
             return torch.from_numpy(np.array(host, np.float32, copy=copy).reshape(shape)).to(where), False
 
         stream = torch.cuda.ExternalStream(dev.stream, device=where) if dev.stream else torch.cuda.default_stream(where)
@@ -318,8 +319,8 @@ class Af3PairformerStackGpu:
             if value is None:
                 return None, False
             if getattr(value, "is_cuda", False):
-                if tuple(value.shape) != shape and value.numel() != int(np.prod(shape)):
-                    raise nat.RangeError(f"state tensor has {value.numel()} values; expected {int(np.prod(shape))}")
+                if tuple(value.shape) != shape and value.numel() != math.prod(shape):
+                    raise nat.RangeError(f"state tensor has {value.numel()} values; expected {math.prod(shape)}")
                 return value.view(shape), True
             host = np.ascontiguousarray(np.asarray(value, np.float32)).reshape(shape)
             return torch.from_numpy(host).to(where), False
@@ -417,12 +418,12 @@ class Af3MsaStackGpu:
 
         def resident(value, shape):
             if getattr(value, "is_cuda", False):
-                if value.numel() != int(np.prod(shape)):
-                    raise nat.RangeError(f"state tensor has {value.numel()} values; expected {int(np.prod(shape))}")
+                if value.numel() != math.prod(shape):
+                    raise nat.RangeError(f"state tensor has {value.numel()} values; expected {math.prod(shape)}")
                 return value.view(shape), True
             host = np.ascontiguousarray(np.asarray(value, np.float32))
-            if host.size != int(np.prod(shape)):
-                raise nat.RangeError(f"state array has {host.size} values; expected {int(np.prod(shape))}")
+            if host.size != math.prod(shape):
+                raise nat.RangeError(f"state array has {host.size} values; expected {math.prod(shape)}")
             return torch.from_numpy(host.reshape(shape)).to(where), False
 
         stream = torch.cuda.ExternalStream(dev.stream, device=where) if dev.stream else torch.cuda.default_stream(where)
