@@ -113,8 +113,9 @@ static lf_status context_create(int device_ordinal, void* stream, bool make_stre
     static std::once_flag per_device[64];
     if (device_ordinal < 64)
       std::call_once(per_device[device_ordinal], [] {
-        cudaFuncSetAttribute(rows::center_norm_kernel<float, rows::LN_TERMS>, cudaFuncAttributeMaxDynamicSharedMemorySize, 512 * 33 * 4);
-        cudaFuncSetAttribute(rows::center_norm_kernel<op16, rows::LN_HALF>, cudaFuncAttributeMaxDynamicSharedMemorySize, 512 * 33 * 4);
+        cudaFuncSetAttribute(rows::center_norm_kernel<float>, cudaFuncAttributeMaxDynamicSharedMemorySize, 512 * 33 * 4);
+        cudaFuncSetAttribute(rows::center_norm_kernel<op16>, cudaFuncAttributeMaxDynamicSharedMemorySize, 512 * 33 * 4);
+        cudaFuncSetAttribute(rows::center_norm_half_kernel<16>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)rows::center_norm_half_smem(128));
         cudaFuncSetAttribute(rows::global_mean_kernel<float>, cudaFuncAttributeMaxDynamicSharedMemorySize, 16 * 513 * 4);
         cudaFuncSetAttribute(rows::global_mean_kernel<bf16>, cudaFuncAttributeMaxDynamicSharedMemorySize, 16 * 513 * 4);
         configure_mma_attention();
@@ -1114,9 +1115,14 @@ struct TriArgs {
   const lf_weights* w;
 };
 
-// Float32 mode: every projection and the contraction as a float32 GEMM on split operands.
+// The triangle product x is stored as fp16 scaled by a power of two near 1/sqrt(n), so that sums over n terms stay far from the fp16
+// limits; the centre LayerNorm undoes the scale exactly.
+float contraction_scale(int n) { return ldexpf(1.0f, -(int)(0.5f * log2f((float)n))); }
+
+// Any width: every projection as a float32 GEMM on split operands.  The contraction is one too, or (`half`, 16-bit mode) runs on fp16
+// a, b and x, the only values of an update that are rounded to 16 bits then.
 template <typename T>
-lf_status tri_f32(lf_context* ctx, ArenaCursor& cur, const TriArgs& a) {
+lf_status tri_general(lf_context* ctx, ArenaCursor& cur, const TriArgs& a, bool half) {
   const int64_t P = (int64_t)a.n * a.n;
   const int cz = a.cz, c = a.c, n = a.n;
   const auto& f = a.w->f;
@@ -1124,26 +1130,37 @@ lf_status tri_f32(lf_context* ctx, ArenaCursor& cur, const TriArgs& a) {
   SplitMatrix none[3];
   if (cur.dry) g = none; else LF_TRY(f32_operands(ctx, a.w, &g));
   const SplitMatrix zn = take_terms(cur, P, cz);
-  const int ld = (n + 7) / 8 * 8, ldx = (n + 3) / 4 * 4;
+  const int ld = half ? (n + 15) / 16 * 16 : (n + 7) / 8 * 8, ldx = half ? ld : (n + 3) / 4 * 4;
   const int64_t plane = (int64_t)n * ld;
   const size_t base = cur.offset;
   float* p4 = cur.take<float>(P * 4 * c);
   const size_t p4_end = cur.offset;
   layer_norm<T, rows::LN_TERMS>(ctx, cur, a.z, P, cz, f[TRI_LN_G], f[TRI_LN_B], a.eps, a.variance, 0, 1, 1, (void*)zn.p, zn.term_stride);
   LF_TRY(tc::gemm_f32(ctx, cur, 0, zn, g[0], (int)P, 4 * c, cz, 1, {p4, nullptr, 4 * c, 0, 0, f[TRI_B4], 4 * c, 0, 0, 0}));
-  SplitMatrix ga, gb;
-  ga.ld = gb.ld = ld;
-  ga.batch_stride = gb.batch_stride = plane;
-  ga.term_stride = gb.term_stride = plane * c;
-  ga.p = cur.take<bf16>(3 * plane * c);
-  gb.p = cur.take<bf16>(3 * plane * c);
-  float* xf = cur.take<float>((int64_t)n * ldx * c);
-  LAUNCH(ctx, cur, rows::trimul_gate_terms_kernel, dim3((unsigned)(n * lf_ceil_div(n, 32)), lf_ceil_div(c, 32)), 256, 0, p4, a.mask, c, n, ld, (bf16*)ga.p,
-         (bf16*)gb.p, ga.term_stride);
-  // outgoing x[i][j] = sum_k a[i][k] b[j][k]; incoming x[i][j] = sum_k b[k][i] a[k][j]
-  const tc::Gemm3Out to{xf, nullptr, ldx, (int64_t)n * ldx, 0, nullptr, 0, 0, 0, 0};
-  if (!a.incoming) LF_TRY(tc::gemm_f32(ctx, cur, 0, ga, gb, n, n, n, c, to));
-  else LF_TRY(tc::gemm_f32(ctx, cur, 1, gb, ga, n, n, n, c, to));
+  op16* xh = nullptr;
+  float* xf = nullptr;
+  const float xscale = half ? contraction_scale(n) : 1.0f;
+  if (half) {
+    op16* ga = cur.take<op16>(plane * c);
+    op16* gb = cur.take<op16>(plane * c);
+    xh = cur.take<op16>(plane * c);
+    LAUNCH(ctx, cur, rows::trimul_gate_half_kernel, dim3((unsigned)(n * lf_ceil_div(n, 64)), lf_ceil_div(c, 32)), 256, 0, p4, a.mask, c, n, ld, ga, gb);
+    LF_TRY(tc::contract(ctx, cur, ga, gb, xh, n, ld, c, a.incoming, xscale));
+  } else {
+    SplitMatrix ga, gb;
+    ga.ld = gb.ld = ld;
+    ga.batch_stride = gb.batch_stride = plane;
+    ga.term_stride = gb.term_stride = plane * c;
+    ga.p = cur.take<bf16>(3 * plane * c);
+    gb.p = cur.take<bf16>(3 * plane * c);
+    xf = cur.take<float>((int64_t)n * ldx * c);
+    LAUNCH(ctx, cur, rows::trimul_gate_terms_kernel, dim3((unsigned)(n * lf_ceil_div(n, 32)), lf_ceil_div(c, 32)), 256, 0, p4, a.mask, c, n, ld, (bf16*)ga.p,
+           (bf16*)gb.p, ga.term_stride);
+    // outgoing x[i][j] = sum_k a[i][k] b[j][k]; incoming x[i][j] = sum_k b[k][i] a[k][j]
+    const tc::Gemm3Out to{xf, nullptr, ldx, (int64_t)n * ldx, 0, nullptr, 0, 0, 0, 0};
+    if (!a.incoming) LF_TRY(tc::gemm_f32(ctx, cur, 0, ga, gb, n, n, n, c, to));
+    else LF_TRY(tc::gemm_f32(ctx, cur, 1, gb, ga, n, n, n, c, to));
+  }
   // p4 is dead: the normalised x and the two outputs take its place where they fit
   const size_t end = cur.offset;
   cur.offset = base;
@@ -1156,10 +1173,21 @@ lf_status tri_f32(lf_context* ctx, ArenaCursor& cur, const TriArgs& a) {
     proj = cur.take<float>(P * cz);
     gate = cur.take<float>(P * cz);
   } else cur.offset = end;
-  const dim3 tiles((unsigned)(n * lf_ceil_div(n, 32)));
-  const size_t smem = (size_t)c * 33 * sizeof(float);
-  LAUNCH(ctx, cur, (rows::center_norm_kernel<float, rows::LN_TERMS>), tiles, 256, smem, xf, c, n, ldx, f[TRI_LNO_G], f[TRI_LNO_B], a.eps, a.variance,
-         a.divide ? 1.0f / n : 1.0f, (int)xn.ld, (void*)xn.p, xn.term_stride);
+  const float center_scale = (a.divide ? 1.0f / n : 1.0f) / xscale;
+  const unsigned tiles = (unsigned)(n * lf_ceil_div(n, 32)), half_tiles = (unsigned)(n * lf_ceil_div(n, 64));
+#define CENTER_HALF(G_)                                                                                                                              \
+  LAUNCH(ctx, cur, (rows::center_norm_half_kernel<G_>), half_tiles, 256, rows::center_norm_half_smem(c), xh, c, n, ld, f[TRI_LNO_G], f[TRI_LNO_B],  \
+         a.eps, a.variance, center_scale, (bf16*)xn.p, xn.term_stride)
+  if (half && c <= 32) CENTER_HALF(4);
+  else if (half && c <= 64) CENTER_HALF(8);
+  else if (half && c <= 128) CENTER_HALF(16);
+  else if (half)
+    LAUNCH(ctx, cur, (rows::center_norm_kernel<op16>), tiles, 256, (size_t)c * 33 * sizeof(float), xh, c, n, ldx, f[TRI_LNO_G], f[TRI_LNO_B], a.eps, a.variance,
+           center_scale, (int)xn.ld, (bf16*)xn.p, xn.term_stride);
+  else
+    LAUNCH(ctx, cur, (rows::center_norm_kernel<float>), tiles, 256, (size_t)c * 33 * sizeof(float), xf, c, n, ldx, f[TRI_LNO_G], f[TRI_LNO_B], a.eps, a.variance,
+           center_scale, (int)xn.ld, (bf16*)xn.p, xn.term_stride);
+#undef CENTER_HALF
   LF_TRY(tc::gemm_f32(ctx, cur, 0, xn, g[1], (int)P, cz, c, 1, {proj, nullptr, cz, 0, 0, f[TRI_BZ], cz, 0, 0, 0}));
   LF_TRY(tc::gemm_f32(ctx, cur, 0, zn, g[2], (int)P, cz, cz, 1, {gate, nullptr, cz, 0, 0, f[TRI_BG], cz, 0, 0, 0}));
   finish<T>(ctx, cur, proj, gate, a.residual ? a.z : nullptr, P, cz, 0, 1, 1, a.out);
@@ -1175,58 +1203,17 @@ lf_status tri_bf16(lf_context* ctx, ArenaCursor& cur, const TriArgs& a) {
   op16* gb = cur.take<op16>(plane * c);
   op16* x = cur.take<op16>(plane * c);
   LF_TRY(tc::triangle_project(ctx, cur, a.z, a.act_dtype, a.mask, n, n, ld, a.variance, a.eps, a.w, ga, gb));
-  // x is stored as fp16 scaled by a power of two near 1/sqrt(n) so that sums over n terms stay far from the fp16 limits;
-  // the centre LayerNorm undoes the scale exactly.
-  const float xscale = ldexpf(1.0f, -(int)(0.5f * log2f((float)n)));
+  const float xscale = contraction_scale(n);
   LF_TRY(tc::contract(ctx, cur, ga, gb, x, n, ld, c, a.incoming, xscale));
   const float xs = xscale * (a.divide ? (float)n : 1.0f);
   return tc::triangle_output(ctx, cur, x, n, n, ld, a.eps * xs * xs, a.z, a.act_dtype, a.variance, a.eps, a.w, a.residual ? a.z : nullptr, a.out);
 }
 
-// 16-bit path at other widths (whole groups of eight): the projections as fp16 GEMMs, the contraction as above.  64 channels,
-// N = 384: 0.20 ms an update, 0.57 ms with the projections as float32 GEMMs.
-template <typename T>
-lf_status tri_half(lf_context* ctx, ArenaCursor& cur, const TriArgs& a) {
-  const int64_t P = (int64_t)a.n * a.n;
-  const int cz = a.cz, c = a.c, n = a.n, ld = (n + 15) / 16 * 16;
-  const int64_t plane = (int64_t)n * ld;
-  const auto& f = a.w->f;
-  op16* zn = cur.take<op16>(P * cz);
-  op16* p4 = cur.take<op16>(P * 4 * c);
-  op16* ga = cur.take<op16>(plane * c);
-  op16* gb = cur.take<op16>(plane * c);
-  op16* x = cur.take<op16>(plane * c);
-  op16* xn = cur.take<op16>(P * c);
-  op16* proj = cur.take<op16>(P * cz);
-  op16* gate = cur.take<op16>(P * cz);
-  layer_norm<T, rows::LN_HALF>(ctx, cur, a.z, P, cz, f[TRI_LN_G], f[TRI_LN_B], a.eps, a.variance, 0, 1, 1, zn);
-  LF_TRY(hgemm(ctx, cur, zn, gemm_operand(a.w, 0), p4, P, 4 * c, cz, f[TRI_B4]));
-  LAUNCH(ctx, cur, rows::trimul_gate_half_kernel, dim3((unsigned)(n * lf_ceil_div(n, 64)), lf_ceil_div(c, 32)), 256, 0, p4, a.mask, c, n, ld, ga, gb);
-  const float xscale = ldexpf(1.0f, -(int)(0.5f * log2f((float)n)));
-  LF_TRY(tc::contract(ctx, cur, ga, gb, x, n, ld, c, a.incoming, xscale));
-  const float center_scale = (a.divide ? 1.0f / n : 1.0f) / xscale;
-  const unsigned center_tiles = (unsigned)(n * lf_ceil_div(n, 64));
-  const size_t center_smem = ((size_t)c * 72 + (size_t)64 * (c + 8)) * sizeof(op16);
-#define CENTER_HALF(G_) LAUNCH(ctx, cur, (rows::center_norm_half_kernel<G_>), center_tiles, 256, center_smem, x, c, n, ld, f[TRI_LNO_G], f[TRI_LNO_B], a.eps, a.variance, center_scale, xn)
-  if (c <= 32) CENTER_HALF(4);
-  else if (c <= 64) CENTER_HALF(8);
-  else if (c <= 128) CENTER_HALF(16);
-  else
-    LAUNCH(ctx, cur, (rows::center_norm_kernel<op16, rows::LN_HALF>), dim3((unsigned)(n * lf_ceil_div(n, 32))), 256, (size_t)c * 33 * sizeof(float), x, c, n, ld,
-           f[TRI_LNO_G], f[TRI_LNO_B], a.eps, a.variance, center_scale, c, (void*)xn, (int64_t)0);
-#undef CENTER_HALF
-  LF_TRY(hgemm(ctx, cur, xn, gemm_operand(a.w, 1), proj, P, cz, c, f[TRI_BZ]));
-  LF_TRY(hgemm(ctx, cur, zn, gemm_operand(a.w, 2), gate, P, cz, cz, f[TRI_BG]));
-  LAUNCH(ctx, cur, (rows::finish_gate_half_kernel<T>), lf_ceil_div(P * (cz / 8), 256), 256, 0, proj, gate, a.residual ? (const T*)a.z : (const T*)nullptr,
-         P * (cz / 8), (T*)a.out);
-  return LF_OK;
-}
-
 lf_status tri_dispatch(lf_context* ctx, ArenaCursor& cur, const TriArgs& a, int precision) {
   const bool half = precision == LF_PRECISION_BF16 && tc::contract_supported(a.n, a.c);
   if (half && tc::ln_gemm_supported(a.w)) return tri_bf16(ctx, cur, a);
-  if (half && a.w->g.size() == 3) return a.act_dtype == LF_DTYPE_BF16 ? tri_half<bf16>(ctx, cur, a) : tri_half<float>(ctx, cur, a);
-  return a.act_dtype == LF_DTYPE_BF16 ? tri_f32<bf16>(ctx, cur, a) : tri_f32<float>(ctx, cur, a);
+  const bool planes = half && a.c % 8 == 0;      // whole 16-byte pieces of channels
+  return a.act_dtype == LF_DTYPE_BF16 ? tri_general<bf16>(ctx, cur, a, planes) : tri_general<float>(ctx, cur, a, planes);
 }
 
 // ---- attention engine, float32 path ----
@@ -2046,7 +2033,7 @@ lf_status lf_pair_shard_step(lf_context* ctx, const lf_shard_step_desc* d, lf_re
   cudaSetDevice(ctx->device);
   const uint64_t before = ctx->launches;
   ArenaCursor cur{ctx, 0, false};
-  const float xscale = ldexpf(1.0f, -(int)(0.5f * log2f((float)n)));
+  const float xscale = contraction_scale(n);
   op16** b = (op16**)d->buf;
   lf_status s = LF_OK;
   switch (d->op) {
@@ -2111,7 +2098,7 @@ lf_status lf_pair_shard_exchange_step(lf_context* ctx, const lf_shard_step_desc*
   cudaSetDevice(ctx->device);
   const uint64_t before = ctx->launches;
   ArenaCursor cur{ctx, 0, false};
-  const float xscale = ldexpf(1.0f, -(int)(0.5f * log2f((float)n)));
+  const float xscale = contraction_scale(n);
   lf_status s = LF_OK;
   switch (d->op) {
     case LF_SHARD_TRIANGLE_PROJECT: {

@@ -240,12 +240,52 @@ trimul_gate_terms_kernel(const float* __restrict__ p4, const float* __restrict__
   }
 }
 
-// LayerNorm over the channels of a channel-major x[h][i][ld] -> [pairs][ldc] as terms or as fp16.  A block takes 32 pairs of one
-// pair row; the tile [c][32] sits in shared memory.
-template <typename TIn, int OUT>
+// ... as fp16 planes [c][n][ld] (c a multiple of 8, ld of 16; zeros past n): a block turns 64 pairs x 32 channels of one pair row
+// round in shared memory, a thread eight channels of a pair.
+__global__ void __launch_bounds__(256)
+trimul_gate_half_kernel(const float* __restrict__ p4, const float* __restrict__ mask, int c, int n, int ld, __half* __restrict__ a, __half* __restrict__ b) {
+  lf_chain();
+  __shared__ __align__(16) __half ta[32][72], tb[32][72];
+  const int tiles = (n + 63) / 64, i = blockIdx.x / tiles, k0 = (blockIdx.x % tiles) * 64, h0 = blockIdx.y * 32;
+  {
+    const int r = threadIdx.x >> 2, hg = (threadIdx.x & 3) * 8, k = k0 + r, h = h0 + hg;
+    if (k < n && h < c) {
+      const int64_t p = (int64_t)i * n + k;
+      const float* row = p4 + p * 4 * c + h;
+      const float m = mask[p];
+      float v[4][8];      // ap, ag, bp, bg
+#pragma unroll
+      for (int q = 0; q < 4; ++q)
+#pragma unroll
+        for (int e = 0; e < 8; e += 4) {
+          const float4 f = *reinterpret_cast<const float4*>(row + (int64_t)q * c + e);
+          v[q][e] = f.x; v[q][e + 1] = f.y; v[q][e + 2] = f.z; v[q][e + 3] = f.w;
+        }
+#pragma unroll
+      for (int e = 0; e < 8; ++e) {
+        ta[hg + e][r] = __float2half_rn(v[0][e] * sigmoidf_(v[1][e]) * m);
+        tb[hg + e][r] = __float2half_rn(v[2][e] * sigmoidf_(v[3][e]) * m);
+      }
+    } else {
+#pragma unroll
+      for (int e = 0; e < 8; ++e) ta[hg + e][r] = tb[hg + e][r] = __float2half_rn(0.f);
+    }
+  }
+  __syncthreads();
+  const int hh = threadIdx.x >> 3, k8 = (threadIdx.x & 7) * 8, h = h0 + hh;
+  if (h < c && k0 + k8 < ld) {
+    const int64_t o = ((int64_t)h * n + i) * ld + k0 + k8;
+    *reinterpret_cast<uint4*>(a + o) = *reinterpret_cast<const uint4*>(&ta[hh][k8]);
+    *reinterpret_cast<uint4*>(b + o) = *reinterpret_cast<const uint4*>(&tb[hh][k8]);
+  }
+}
+
+// LayerNorm over the channels of a channel-major x[h][i][ld] -> terms with rows of ldc.  A block takes 32 pairs of one pair row; the
+// tile [c][32] sits in shared memory.
+template <typename TIn>
 __global__ void __launch_bounds__(256)
 center_norm_kernel(const TIn* __restrict__ x, int c, int n, int ld, const float* __restrict__ gamma, const float* __restrict__ beta,
-                   float eps, int variance, float prescale, int ldc, void* __restrict__ xn, int64_t term_stride) {
+                   float eps, int variance, float prescale, int ldc, bf16* __restrict__ xn, int64_t term_stride) {
   lf_chain();
   extern __shared__ float tile[];   // [c][33]
   const int tiles = (n + 31) / 32, i = blockIdx.x / tiles, k0 = (blockIdx.x % tiles) * 32;
@@ -270,34 +310,31 @@ center_norm_kernel(const TIn* __restrict__ x, int c, int n, int ld, const float*
     for (int h = tx * 2; h < ldc; h += 64) {
       const float v0 = h < c ? (tile[h * 33 + r] - mean) * inv * gamma[h] + beta[h] : 0.f;
       const float v1 = h + 1 < c ? (tile[(h + 1) * 33 + r] - mean) * inv * gamma[h + 1] + beta[h + 1] : 0.f;
-      if (OUT == LN_HALF) *reinterpret_cast<__half2*>(reinterpret_cast<__half*>(xn) + row + h) = __floats2half2_rn(v0, v1);
-      else {
-        uint32_t t[3];
-        split_pair(v0, v1, t);
+      uint32_t t[3];
+      split_pair(v0, v1, t);
 #pragma unroll
-        for (int e = 0; e < 3; ++e) *reinterpret_cast<uint32_t*>(reinterpret_cast<bf16*>(xn) + e * term_stride + row + h) = t[e];
-      }
+      for (int e = 0; e < 3; ++e) *reinterpret_cast<uint32_t*>(xn + e * term_stride + row + h) = t[e];
     }
   }
 }
 
-// The same from fp16 to fp16 for c <= 8 GROUPS, a multiple of 8 (wider ones do not fit the registers): a block takes 64 pairs of one pair
-// row in 16-byte pieces, four threads a pair hold the channels in registers (channels 8 g + 2 part and the next), and the rows leave through
-// shared memory in 16-byte pieces.  Bound by the passes over shared memory; a value at a time with a warp a pair took 43 us for 384 x 384 x 64,
-// this 15 us.
+// The same from fp16 for c <= 8 GROUPS, a multiple of 8 (wider ones do not fit the registers): a block takes 64 pairs of one pair row in
+// 16-byte pieces, four threads a pair hold the channels in registers (channels 8 g + 2 part and the next), and the terms leave through
+// shared memory in 16-byte pieces.  Bound by the passes over shared memory.
+constexpr int kCenterPitch = 72;      // 64 pairs and 16 bytes: the four channel rows a warp reads at a time spread over the banks
+constexpr size_t center_norm_half_smem(int c) { return ((size_t)c * kCenterPitch + (size_t)3 * 64 * (c + 8)) * sizeof(uint16_t); }
 template <int GROUPS>
 __global__ void __launch_bounds__(256)
 center_norm_half_kernel(const __half* __restrict__ x, int c, int n, int ld, const float* __restrict__ gamma, const float* __restrict__ beta, float eps,
-                        int variance, float prescale, __half* __restrict__ xn) {
+                        int variance, float prescale, bf16* __restrict__ xn, int64_t term_stride) {
   lf_chain();
   extern __shared__ uint4 center_s[];
-  constexpr int PITCH = 72;                                // 64 pairs and 16 bytes: the four channel rows a warp reads at a time spread over the banks
-  __half* tile = reinterpret_cast<__half*>(center_s);      // [c][PITCH]
-  __half* rows_s = tile + c * PITCH;                       // [64][c + 8]
+  __half* tile = reinterpret_cast<__half*>(center_s);                        // [c][kCenterPitch]
+  bf16* rows_s = reinterpret_cast<bf16*>(tile + c * kCenterPitch);           // [3 terms][64][c + 8]
   const int tiles = (n + 63) / 64, i = blockIdx.x / tiles, k0 = (blockIdx.x % tiles) * 64, pieces = c >> 3;
   for (int u = threadIdx.x; u < c * 8; u += 256) {
     const int h = u >> 3, k = (u & 7) * 8;
-    *reinterpret_cast<uint4*>(tile + h * PITCH + k) =
+    *reinterpret_cast<uint4*>(tile + h * kCenterPitch + k) =
         k0 + k < ld ? *reinterpret_cast<const uint4*>(x + ((int64_t)h * n + i) * ld + k0 + k) : make_uint4(0u, 0u, 0u, 0u);
   }
   __syncthreads();
@@ -312,7 +349,7 @@ center_norm_half_kernel(const __half* __restrict__ x, int c, int n, int ld, cons
     const int h = g * 8 + part * 2;
 #pragma unroll
     for (int e = 0; e < 2; ++e) {
-      v[g][e] = g < pieces ? __half2float(tile[(h + e) * PITCH + pair]) * prescale : 0.f;
+      v[g][e] = g < pieces ? __half2float(tile[(h + e) * kCenterPitch + pair]) * prescale : 0.f;
       s += v[g][e];
       ss = fmaf(v[g][e], v[g][e], ss);
     }
@@ -333,14 +370,20 @@ center_norm_half_kernel(const __half* __restrict__ x, int c, int n, int ld, cons
 #pragma unroll
   for (int g = 0; g < GROUPS; ++g) {
     const int h = g * 8 + part * 2;
-    if (g < pieces)
-      *reinterpret_cast<__half2*>(rows_s + pair * (c + 8) + h) =
-          __floats2half2_rn((v[g][0] - mean) * inv * __ldg(gamma + h) + __ldg(beta + h), (v[g][1] - mean) * inv * __ldg(gamma + h + 1) + __ldg(beta + h + 1));
+    if (g < pieces) {
+      uint32_t t[3];
+      split_pair((v[g][0] - mean) * inv * __ldg(gamma + h) + __ldg(beta + h), (v[g][1] - mean) * inv * __ldg(gamma + h + 1) + __ldg(beta + h + 1), t);
+#pragma unroll
+      for (int e = 0; e < 3; ++e) *reinterpret_cast<uint32_t*>(rows_s + (e * 64 + pair) * (c + 8) + h) = t[e];
+    }
   }
   __syncthreads();
   for (int u = threadIdx.x; u < 64 * pieces; u += 256) {
     const int r = u / pieces, h = (u % pieces) * 8;
-    if (k0 + r < n) *reinterpret_cast<uint4*>(xn + ((int64_t)i * n + k0 + r) * c + h) = *reinterpret_cast<const uint4*>(rows_s + r * (c + 8) + h);
+    if (k0 + r >= n) continue;
+#pragma unroll
+    for (int e = 0; e < 3; ++e)
+      *reinterpret_cast<uint4*>(xn + e * term_stride + ((int64_t)i * n + k0 + r) * c + h) = *reinterpret_cast<const uint4*>(rows_s + (e * 64 + r) * (c + 8) + h);
   }
 }
 
@@ -372,56 +415,6 @@ __global__ void finish4_kernel(const float* __restrict__ proj, const float* __re
     for (int e = 0; e < 4; ++e) v[e] += x[e];
   }
   store4(out + dst * ch + c, v);
-}
-
-// 16-bit form: fp16 rows (ap | ag | bp | bg), eight channels a load -> fp16 planes [c][n][ld] (c a multiple of 8, ld of 16; zeros
-// past n).  A block turns 64 pairs x 32 channels of one pair row round in shared memory.
-__global__ void __launch_bounds__(256)
-trimul_gate_half_kernel(const __half* __restrict__ p4, const float* __restrict__ mask, int c, int n, int ld, __half* __restrict__ a, __half* __restrict__ b) {
-  lf_chain();
-  __shared__ __half ta[32][72], tb[32][72];
-  const int tiles = (n + 63) / 64, i = blockIdx.x / tiles, k0 = (blockIdx.x % tiles) * 64, h0 = blockIdx.y * 32;
-  {
-    const int r = threadIdx.x >> 2, hg = (threadIdx.x & 3) * 8, k = k0 + r, h = h0 + hg;
-    if (k < n && h < c) {
-      const int64_t p = (int64_t)i * n + k;
-      const __half* row = p4 + p * 4 * c + h;
-      const float m = mask[p];
-      uint4 raw[4];
-#pragma unroll
-      for (int q = 0; q < 4; ++q) raw[q] = *reinterpret_cast<const uint4*>(row + (int64_t)q * c);
-#pragma unroll
-      for (int e = 0; e < 8; ++e) {
-        auto at = [&](int q) { return __half2float(reinterpret_cast<const __half*>(&raw[q])[e]); };
-        ta[hg + e][r] = __float2half_rn(at(0) * sigmoidf_(at(1)) * m);
-        tb[hg + e][r] = __float2half_rn(at(2) * sigmoidf_(at(3)) * m);
-      }
-    } else {
-#pragma unroll
-      for (int e = 0; e < 8; ++e) ta[hg + e][r] = tb[hg + e][r] = __float2half_rn(0.f);
-    }
-  }
-  __syncthreads();
-  const int hh = threadIdx.x >> 3, k8 = (threadIdx.x & 7) * 8, h = h0 + hh;
-  if (h < c && k0 + k8 < ld) {
-    const int64_t o = ((int64_t)h * n + i) * ld + k0 + k8;
-    *reinterpret_cast<uint4*>(a + o) = *reinterpret_cast<const uint4*>(&ta[hh][k8]);
-    *reinterpret_cast<uint4*>(b + o) = *reinterpret_cast<const uint4*>(&tb[hh][k8]);
-  }
-}
-
-// out[r][c] = (resid ? resid[r][c] : 0) + proj[r][c] * sigmoid(gate[r][c]), fp16 projections, eight channels a thread (ch a multiple of 8)
-template <typename TAct>
-__global__ void finish_gate_half_kernel(const __half* __restrict__ proj, const __half* __restrict__ gate, const TAct* __restrict__ resid, int64_t count,
-                                        TAct* __restrict__ out) {
-  lf_chain();
-  const int64_t idx = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (idx >= count) return;
-  const uint4 p = *reinterpret_cast<const uint4*>(proj + idx * 8), g = *reinterpret_cast<const uint4*>(gate + idx * 8);
-  float v[8];
-#pragma unroll
-  for (int e = 0; e < 8; ++e) v[e] = __half2float(reinterpret_cast<const __half*>(&p)[e]) * sigmoidf_(__half2float(reinterpret_cast<const __half*>(&g)[e]));
-  simt::add_store8<TAct>(v, resid ? resid + idx * 8 : nullptr, out + idx * 8);
 }
 
 // fp16 columns col0 .. col0 + heads of rows (i * Q + j) -> bias[h][i][ldb] (zeros past Q), or its transpose when `swap`

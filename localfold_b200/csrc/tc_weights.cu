@@ -247,14 +247,6 @@ lf_status prepare_weights(lf_context* ctx, lf_weights* w, WeightCursor& cur) {
       w->head_form = true;
     }
   }
-  if (tri && w->h.empty() && w->dims.channels % 8 == 0 && w->dims.hidden % 8 == 0) {
-    const int cz = w->dims.channels, c = w->dims.hidden;
-    op16 *w4 = cur.take<op16>((size_t)4 * c * cz), *wz = cur.take<op16>((size_t)cz * c), *wg = cur.take<op16>((size_t)cz * cz);
-    prep.operand(f[TRI_W4], cz, 4 * c, 4 * c, w4);
-    prep.operand(f[TRI_WZ], c, cz, cz, wz);
-    prep.operand(f[TRI_WG], cz, cz, cz, wg);
-    w->g = {w4, wz, wg};
-  }
   if ((w->kind == LF_WEIGHTS_TRANSITION_AF2 || w->kind == LF_WEIGHTS_TRANSITION_AF3) && w->h.empty() &&
       w->dims.channels % 8 == 0 && w->dims.hidden % 8 == 0) {
     const int c = w->dims.channels, hd = w->dims.hidden, wide = w->kind == LF_WEIGHTS_TRANSITION_AF3 ? 2 * hd : hd;
