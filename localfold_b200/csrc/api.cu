@@ -975,42 +975,41 @@ void sgemm(lf_context* ctx, ArenaCursor& cur, bool ta, bool tb, int epi, int M, 
 #undef SG
 }
 
-// The attention core for any head width: terms of q | k | v | gate, or fp16, -> the gated output likewise.
+// The float32 attention core for any head width: terms of q | k | v | gate -> the gated output likewise.
 constexpr int kAttentionSmem = 96 * 1024;      // two blocks an SM
 #define ATTENTION_WIDTHS(X) X(8) X(16) X(24) X(32) X(48) X(64)
-template <int TERMS>
-void mma_attention_core(lf_context* ctx, ArenaCursor& cur, int D, const void* qkvg, const void* bias, const float* mask, mma_attention::AttentionShape s,
-                        void* out) {
+void mma_attention_core(lf_context* ctx, ArenaCursor& cur, int D, const SplitMatrix& qkvg, const float* bias, const float* mask,
+                        mma_attention::AttentionShape s, const SplitMatrix& out) {
   // eight warps, or as many as the queries have groups of 16: the groups are spread evenly over the blocks; small query
   // counts put several batch rows into a block
   const int groups = lf_ceil_div(s.Q, 16), tiles = lf_ceil_div(groups, 8);
   s.wq = lf_ceil_div(groups, tiles);
   s.wb = 8 / s.wq < s.batch ? 8 / s.wq : s.batch;
   while (s.wb > 1 && (int64_t)tiles * s.heads * lf_ceil_div(s.batch, s.wb) < ctx->sm_count) s.wb /= 2;
-  // key tiles as long as two blocks' (three in the fp16 form) shared memory allows, up to 128 keys: a barrier a tile
-  auto bytes = [&](int kt) { return mma_attention::attention_smem(D, TERMS, s.wb, kt, (s.Q < 1024 ? lf_ceil_div(s.Q, kt) : lf_ceil_div(1024, kt)) * kt); };
+  // key tiles as long as two blocks' shared memory allows, up to 128 keys: a barrier a tile
+  auto bytes = [&](int kt) { return mma_attention::attention_smem(D, s.wb, kt, (s.Q < 1024 ? lf_ceil_div(s.Q, kt) : lf_ceil_div(1024, kt)) * kt); };
   s.kt = 128;
-  while (s.kt > 32 && (s.kt >= 2 * s.Q || bytes(s.kt) > (TERMS == 1 ? kAttentionSmem * 2 / 3 : kAttentionSmem))) s.kt /= 2;
+  while (s.kt > 32 && (s.kt >= 2 * s.Q || bytes(s.kt) > kAttentionSmem)) s.kt /= 2;
   while (s.wb > 1 && bytes(s.kt) > kAttentionSmem) s.wb /= 2;
   s.mk = (s.Q < 1024 ? lf_ceil_div(s.Q, s.kt) : lf_ceil_div(1024, s.kt)) * s.kt;
+  s.ld = qkvg.ld; s.term_stride = qkvg.term_stride;
+  s.ldo = out.ld; s.out_stride = out.term_stride;
   const dim3 grid(lf_ceil_div(groups, s.wq), lf_ceil_div(s.batch, s.wb), s.heads);
   const size_t smem = bytes(s.kt);
-  const uint16_t* in = (const uint16_t*)qkvg;
-#define ATTENTION_CASE(D_)                                                                                                                             \
-  case D_:                                                                                                                                             \
-    if (bias) LAUNCH(ctx, cur, (mma_attention::attention_kernel<D_, TERMS, true>), grid, 32 * s.wb * s.wq, smem, in, bias, mask, s, (uint16_t*)out);    \
-    else LAUNCH(ctx, cur, (mma_attention::attention_kernel<D_, TERMS, false>), grid, 32 * s.wb * s.wq, smem, in, bias, mask, s, (uint16_t*)out);        \
+  const uint16_t* in = (const uint16_t*)qkvg.p;
+#define ATTENTION_CASE(D_)                                                                                                                   \
+  case D_:                                                                                                                                   \
+    if (bias) LAUNCH(ctx, cur, (mma_attention::attention_kernel<D_, true>), grid, 32 * s.wb * s.wq, smem, in, bias, mask, s, (uint16_t*)out.p);  \
+    else LAUNCH(ctx, cur, (mma_attention::attention_kernel<D_, false>), grid, 32 * s.wb * s.wq, smem, in, bias, mask, s, (uint16_t*)out.p);      \
     break;
   switch (D) { ATTENTION_WIDTHS(ATTENTION_CASE) }
 #undef ATTENTION_CASE
 }
 
 void configure_mma_attention() {
-#define ATTENTION_CASE(D_)                                                                                                              \
-  cudaFuncSetAttribute(mma_attention::attention_kernel<D_, 3, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, kAttentionSmem);   \
-  cudaFuncSetAttribute(mma_attention::attention_kernel<D_, 3, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, kAttentionSmem);  \
-  cudaFuncSetAttribute(mma_attention::attention_kernel<D_, 1, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, kAttentionSmem);   \
-  cudaFuncSetAttribute(mma_attention::attention_kernel<D_, 1, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, kAttentionSmem);
+#define ATTENTION_CASE(D_)                                                                                                       \
+  cudaFuncSetAttribute(mma_attention::attention_kernel<D_, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, kAttentionSmem);  \
+  cudaFuncSetAttribute(mma_attention::attention_kernel<D_, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, kAttentionSmem);
   ATTENTION_WIDTHS(ATTENTION_CASE)
 #undef ATTENTION_CASE
 }
@@ -1271,9 +1270,7 @@ lf_status att_f32(lf_context* ctx, ArenaCursor& cur, const AttArgs& a) {
   else if (a.bias_mode == 2)
     LAUNCH(ctx, cur, rows::bias_columns_kernel, lf_ceil_div((int64_t)a.Q * a.Q, 256), 256, 0, qkvg.p, qkvg.ld, qkvg.term_stride, 4 * HDp, a.Q, a.heads,
            a.bias_swap, bias);
-  mma_attention_core<3>(ctx, cur, D, qkvg.p, bias, a.mask,
-                        {a.batch, a.Q, a.heads, a.transpose, a.mask_mode, a.clamp, 1.0f / sqrtf((float)a.d), qkvg.ld, qkvg.term_stride, o.ld, o.term_stride, 0, 0, 1, 1, 0, 0},
-                        (void*)o.p);
+  mma_attention_core(ctx, cur, D, qkvg, bias, a.mask, {a.batch, a.Q, a.heads, a.transpose, a.mask_mode, a.clamp, 1.0f / sqrtf((float)a.d)}, o);
   LF_TRY(tc::gemm_f32(ctx, cur, 0, o, g[1], (int)R, c, HDp, 1, {proj, nullptr, c, 0, 0, f[ATT_BO], c, 0, 0, 0}));
   finish<T>(ctx, cur, proj, nullptr, a.residual ? a.act : nullptr, R, c, a.transpose, a.batch, a.Q, a.out);
   return LF_OK;
@@ -1395,42 +1392,11 @@ lf_status att_mixed(lf_context* ctx, ArenaCursor& cur, const AttArgs& a) {
   return LF_OK;
 }
 
-// 16-bit path for the head widths (or head counts, or the own pair bias at other widths) that the tcgen05 core does not take: LayerNorm to
-// fp16, q / k / v / gate (and the own pair bias) as one fp16 GEMM, the mma.sync core on fp16 rows, the output projection as a second GEMM.
-template <typename T>
-lf_status att_half(lf_context* ctx, ArenaCursor& cur, const AttArgs& a) {
-  const int64_t R = (int64_t)a.batch * a.Q;
-  const int D = head_width(a.d), HDp = a.heads * D, c = a.ch, ldb = (a.Q + 15) / 16 * 16;
-  const bool own_bias = a.w->has_pair_proj && !a.w->has_pair_norm;
-  const int wide = (4 * HDp + (own_bias ? a.heads : 0) + 7) / 8 * 8;
-  const auto& f = a.w->f;
-  op16* nrm = cur.take<op16>(R * c);
-  op16* qkvg = cur.take<op16>(R * wide);
-  op16* bias = a.bias_mode ? cur.take<op16>((int64_t)a.heads * a.Q * ldb) : nullptr;
-  op16* o = cur.take<op16>(R * HDp);
-  layer_norm<T, rows::LN_HALF>(ctx, cur, a.act, R, c, f[ATT_LN_G], f[ATT_LN_B], a.eps, a.variance, a.transpose, a.batch, a.Q, nrm);
-  LF_TRY(hgemm(ctx, cur, nrm, gemm_operand(a.w, 0), qkvg, R, wide, c, (const float*)a.w->g[2]));
-  if (a.bias_mode == 1) LF_TRY(tc::pair_bias_project(ctx, cur, a.pair, a.pair_dtype, a.Q, a.pair_variance, a.pair_eps, a.heads, a.w, bias, ldb));
-  else if (a.bias_mode == 2)
-    LAUNCH(ctx, cur, rows::bias_columns_half_kernel, lf_ceil_div((int64_t)a.Q * ldb, 256), 256, 0, qkvg, (int64_t)wide, 4 * HDp, a.Q, ldb, a.heads, a.bias_swap, bias);
-  mma_attention_core<1>(ctx, cur, D, qkvg, bias, a.mask,
-                        {a.batch, a.Q, a.heads, a.transpose, a.mask_mode, a.clamp, 1.0f / sqrtf((float)a.d), wide, 0, HDp, 0, 1, ldb, 1, 1, 0, 0}, o);
-  if (rows_in_place<T>(a.residual, a.act, a.out, c))
-    return tc::gemm_rows_f32(ctx, cur, o, 0, gemm_operand(a.w, 1), (float*)a.out, a.residual, a.batch, a.Q, 0, a.transpose, c, HDp, f[ATT_BO]);
-  LF_TRY(hgemm(ctx, cur, o, gemm_operand(a.w, 1), nrm, R, c, HDp));      // (the normalised input is dead)
-  LAUNCH(ctx, cur, (simt::finish_half_kernel<T>), lf_ceil_div(R * c / 8, 256), 256, 0, nrm, 1.0f, f[ATT_BO],
-         a.residual ? (const T*)a.act : (const T*)nullptr, R, c, a.transpose, a.batch, a.Q, (T*)a.out);
-  return LF_OK;
-}
-
 lf_status att_dispatch(lf_context* ctx, ArenaCursor& cur, const AttArgs& a, int precision) {
   if (precision == LF_PRECISION_BF16 && a.bias_mode != 1 && a.heads == 4 && a.d == 32 && tc::ln_gemm_supported(a.w)) {
     return a.act_dtype == LF_DTYPE_BF16 ? att_bf16<bf16>(ctx, cur, a) : att_bf16<float>(ctx, cur, a);
   }
-  if (precision == LF_PRECISION_BF16 && a.w->head_form && tc::contract_supported(1, 1) &&
-      (a.bias_mode != 1 || (tc::pair_bias_supported(a.w) && !a.bias_swap)))
-    return a.act_dtype == LF_DTYPE_BF16 ? att_half<bf16>(ctx, cur, a) : att_half<float>(ctx, cur, a);
-  if (precision == LF_PRECISION_BF16 && a.d == 32 && a.heads % 4 == 0 && !a.w->head_form && hgemm_supported(a.w) &&
+  if (precision == LF_PRECISION_BF16 && a.d == 32 && a.heads % 4 == 0 && hgemm_supported(a.w) &&
       (a.bias_mode == 0 || (a.bias_mode == 1 && tc::pair_bias_supported(a.w) && !a.bias_swap))) {
     return a.act_dtype == LF_DTYPE_BF16 ? att_mixed<bf16>(ctx, cur, a) : att_mixed<float>(ctx, cur, a);
   }

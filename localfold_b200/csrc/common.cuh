@@ -124,7 +124,6 @@ struct lf_weights {
   std::vector<float*> f;     // named by the per-kind enums above
   std::vector<void*> h;      // fp16 repacks (tensor-core path)
   std::vector<void*> g;      // fp16 [n_out][k] operands of the plain tensor-core GEMM (widths the fused kernels do not take)
-  bool head_form = false;    // g is (fused projection with heads padded to head_width and the own pair bias rows, output projection, float32 bias)
   int device = 0;
   void* block = nullptr;     // the one device allocation behind all of them (weight_block_take)
   size_t block_bytes = 0;

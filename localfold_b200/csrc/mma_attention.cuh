@@ -1,9 +1,7 @@
-// Gated attention core for any head width, its products on the tensor cores.  TERMS = 3, float32: every operand is taken apart into
-// three bf16 terms (8 + 8 + 8 significand bits, so nothing of it is lost) and a product into the six term products above
-// 2^-24, accumulated in float32.  TERMS = 1, 16-bit mode (head widths the tcgen05 core does not take): fp16 operands.
+// Gated float32 attention core for any head width, its products on the tensor cores: every operand is taken apart into three
+// bf16 terms (8 + 8 + 8 significand bits, so nothing of it is lost) and a product into the six term products above 2^-24,
+// accumulated in float32.  Float32 mode, and 16-bit mode for the heads that the tcgen05 core does not take.
 #pragma once
-
-#include <type_traits>
 
 #include "common.cuh"
 
@@ -48,18 +46,6 @@ __device__ __forceinline__ void mma16(float (&c)[4], const uint32_t (&a)[4], uin
   asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%0, %1, %2, %3};"
                : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3]) : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
 }
-__device__ __forceinline__ void mma16h(float (&c)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
-  asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%0, %1, %2, %3};"
-               : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3]) : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
-}
-__device__ __forceinline__ void mma8h(float (&c)[4], uint32_t a0, uint32_t a1, uint32_t b0) {
-  asm volatile("mma.sync.aligned.m16n8k8.row.col.f32.f16.f16.f32 {%0, %1, %2, %3}, {%4, %5}, {%6}, {%0, %1, %2, %3};"
-               : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3]) : "r"(a0), "r"(a1), "r"(b0));
-}
-__device__ __forceinline__ uint32_t pack_half(float lo, float hi) {
-  const __half2 h = __floats2half2_rn(lo, hi);
-  return *reinterpret_cast<const uint32_t*>(&h);
-}
 __device__ __forceinline__ void mma8(float (&c)[4], uint32_t a0, uint32_t a1, uint32_t b0) {
   asm volatile("mma.sync.aligned.m16n8k8.row.col.f32.bf16.bf16.f32 {%0, %1, %2, %3}, {%4, %5}, {%6}, {%0, %1, %2, %3};"
                : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3]) : "r"(a0), "r"(a1), "r"(b0));
@@ -90,10 +76,8 @@ struct AttentionShape {
   int batch, Q, heads;
   int transpose, mask_mode, clamp;      // mask_mode 0: logit += 1e9 (m - 1); 1: logit += m > 0 ? 0 : -1e9
   float scale;
-  int64_t ld, term_stride;              // rows and terms of q | k | v | gate, in 16-bit elements (multiples of 8)
+  int64_t ld, term_stride;              // rows and terms of q | k | v | gate, in elements (multiples of 8)
   int64_t ldo, out_stride;              // ... and of the output
-  int gate_logits;                      // fp16: the gate columns hold logits (the projection applies no sigmoid)
-  int ldb;                              // fp16 bias: elements from one query's keys to the next (a multiple of 8, as the bias's address)
   int wb, wq;                           // warps of a block: wb batch rows x wq groups of 16 queries
   int kt;                               // keys of a staged tile, a multiple of 32
   int mk;                               // keys whose mask terms are held at a time, a multiple of kt
@@ -101,19 +85,15 @@ struct AttentionShape {
 
 constexpr int AT_STEP = 32;                                                   // keys of one step of a warp
 __host__ __device__ constexpr int at_pitch(int D) { return 8 * ((D / 8) | 1); }      // odd in 16-byte units: ldmatrix rows spread over the banks
-// fp16: a step's 32 keys are dealt to the tensor core's columns so that a thread holds eight neighbouring ones (column 8 n + 2 t + e is key
-// 8 t + 2 n + e): its bias and mask terms are then whole 16-byte pieces, two loads a row and step instead of eight (291 -> 227 us, 384 x
-// 384 with 4 heads of 16).  Rows of every eight keys are shifted by 32 bytes, so that the rows of a matrix still spread over the banks.  A
-// float32 bias has no such pieces where the length is odd, and keeps the plain order.
-__host__ __device__ constexpr int at_rows(int D, int terms, int keys) { return keys * (at_pitch(D) + (terms == 1 ? 2 : 0)); }
-__host__ __device__ constexpr size_t attention_smem(int D, int terms, int wb, int kt, int mk) {
-  return (size_t)wb * (2 * 2 * terms * at_rows(D, terms, kt) * 2 + mk * 4);
+constexpr int AT_TERMS = 3;
+__host__ __device__ constexpr size_t attention_smem(int D, int wb, int kt, int mk) {
+  return (size_t)wb * (2 * 2 * AT_TERMS * kt * at_pitch(D) * 2 + mk * 4);
 }
 
-//   qkvg: [TERMS][rows][ld] = terms of (q | k | v | sigmoid(gate) | ...) in logical row order, a head of each D channels wide
+//   qkvg: [3][rows][ld] = terms of (q | k | v | sigmoid(gate) | ...) in logical row order, a head of each D channels wide
 //         (the projection's weights are padded to the instance's width, so nothing here is conditional on the true one)
-//   bias: float32 [H][Q][Q], or fp16 [H][Q][ldb], or null; mask: indexed b * Q + j, or j * batch + b when transpose
-//   out:  [TERMS][rows][ldo] = softmax(.) v * gate as terms, the operand of the output projection
+//   bias: float32 [H][Q][Q] or null; mask: indexed b * Q + j, or j * batch + b when transpose
+//   out:  [3][rows][ldo] = softmax(.) v * gate as terms, the operand of the output projection
 // A warp owns 16 queries of one (batch row, head); Q and the running output stay in registers in the tensor core's
 // fragment layout, and probabilities become the A operand of P V without leaving them.  The warps of a block share K and
 // V tiles of kt keys, copied a tile ahead as the projection wrote them, and step through them 32 keys at a time; mask terms
@@ -125,16 +105,14 @@ __host__ __device__ constexpr size_t attention_smem(int D, int terms, int wb, in
 // Bound by the latency of a warp's chain (a third of the tensor pipe, half of the issue slots, 16 warps an SM).  Measured,
 // 384 x 384 with 4 heads of 16: 0.51 ms, against 5.06 ms with a warp per query and a shuffle per key and 0.68 ms with
 // four queries a thread on packed FMAs; 203 x 203, 4 x 32: 0.19 ms against 0.98 and 0.24.
-template <int D, int TERMS, bool BIAS>
-__global__ void __launch_bounds__(256, TERMS == 3 && D > 32 ? 1 : TERMS == 1 && D <= 16 ? 3 : 2)
-attention_kernel(const uint16_t* __restrict__ qkvg, const void* __restrict__ bias_any, const float* __restrict__ mask,
-                 const AttentionShape s, uint16_t* __restrict__ out) {
+template <int D, bool BIAS>
+__global__ void __launch_bounds__(256, D > 32 ? 1 : 2)
+attention_kernel(const uint16_t* __restrict__ qkvg, const float* __restrict__ bias, const float* __restrict__ mask, const AttentionShape s,
+                 uint16_t* __restrict__ out) {
   lf_chain();
-  typedef typename std::conditional<TERMS == 1, __half, float>::type TBias;
-  const TBias* bias = static_cast<const TBias*>(bias_any);
-  constexpr int TOP = TERMS - 1;                    // highest order of a term product that is kept: i + j <= TOP
+  constexpr int TERMS = AT_TERMS, TOP = TERMS - 1;                    // highest order of a term product that is kept: i + j <= TOP
   constexpr int KT = AT_STEP, PITCH = at_pitch(D), NK = D / 16, TAIL = (D / 8) & 1, ND = D / 8;
-  const int plane = at_rows(D, TERMS, s.kt);        // elements of one term of one staged tile
+  const int plane = s.kt * PITCH;                   // elements of one term of one staged tile
   extern __shared__ uint4 at_sm[];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, g = lane >> 2, t = lane & 3;
   const int wb = warp / s.wq, wq = warp % s.wq;
@@ -156,7 +134,7 @@ attention_kernel(const uint16_t* __restrict__ qkvg, const void* __restrict__ bia
       for (int bb = 0; bb < s.wb; ++bb) {
         const bool ok = j0 + j < Q && b0 + bb < s.batch;
         const uint16_t* src = ok ? qkvg + ((int64_t)(b0 + bb) * Q + j0 + j) * ld + HD + h * D + e : qkvg;
-        uint16_t* dst = kv_s + (buf * s.wb + bb) * 2 * TERMS * plane + j * PITCH + (TERMS == 1 ? (j >> 3) * 16 : 0) + e;
+        uint16_t* dst = kv_s + (buf * s.wb + bb) * 2 * TERMS * plane + j * PITCH + e;
 #pragma unroll
         for (int which = 0; which < 2; ++which)
 #pragma unroll
@@ -198,40 +176,26 @@ attention_kernel(const uint16_t* __restrict__ qkvg, const void* __restrict__ bia
   }
 
   // the bias of a tile's keys: this thread's two rows, eight columns each
-  const int64_t bias_ld = TERMS == 1 ? s.ldb : Q;
   const bool pairs = (Q & 1) == 0;
-  constexpr int KEY_T = TERMS == 1 ? 8 : 2, KEY_N = TERMS == 1 ? 2 : 8;      // keys from a thread to the next and from a group of eight columns to the next
-  const TBias* bias0 = BIAS ? bias + ((int64_t)h * Q + (row0 < Q ? row0 : 0)) * bias_ld + KEY_T * t : nullptr;
-  const TBias* bias1 = BIAS ? bias + ((int64_t)h * Q + (row1 < Q ? row1 : 0)) * bias_ld + KEY_T * t : nullptr;
-  float bv[TERMS == 1 ? 1 : 4][4];
-  uint4 bh[2];                                      // fp16: the eight values of each row as they come
+  const float* bias0 = BIAS ? bias + ((int64_t)h * Q + (row0 < Q ? row0 : 0)) * Q + 2 * t : nullptr;
+  const float* bias1 = BIAS ? bias + ((int64_t)h * Q + (row1 < Q ? row1 : 0)) * Q + 2 * t : nullptr;
+  float bv[4][4];
   auto load_bias = [&](int j0) {
     if (!BIAS) return;
-    if constexpr (TERMS == 1) {
-      bh[0] = bh[1] = make_uint4(0u, 0u, 0u, 0u);
-      if (j0 + 8 * t + 8 <= s.ldb) {
-        bh[0] = __ldg(reinterpret_cast<const uint4*>(bias0 + j0));
-        bh[1] = __ldg(reinterpret_cast<const uint4*>(bias1 + j0));
-      }
-    } else {
 #pragma unroll
-      for (int n = 0; n < 4; ++n) {
-        const int j = j0 + n * 8;
-        if (pairs && j + 2 * t < Q) {
-          const float2 x = __ldg(reinterpret_cast<const float2*>(bias0 + j)), y = __ldg(reinterpret_cast<const float2*>(bias1 + j));
-          bv[n][0] = x.x; bv[n][1] = x.y; bv[n][2] = y.x; bv[n][3] = y.y;
-        } else {
-          bv[n][0] = j + 2 * t < Q ? __ldg(bias0 + j) : 0.f;
-          bv[n][1] = j + 2 * t + 1 < Q ? __ldg(bias0 + j + 1) : 0.f;
-          bv[n][2] = j + 2 * t < Q ? __ldg(bias1 + j) : 0.f;
-          bv[n][3] = j + 2 * t + 1 < Q ? __ldg(bias1 + j + 1) : 0.f;
-        }
+    for (int n = 0; n < 4; ++n) {
+      const int j = j0 + n * 8;
+      if (pairs && j + 2 * t < Q) {
+        const float2 x = __ldg(reinterpret_cast<const float2*>(bias0 + j)), y = __ldg(reinterpret_cast<const float2*>(bias1 + j));
+        bv[n][0] = x.x; bv[n][1] = x.y; bv[n][2] = y.x; bv[n][3] = y.y;
+      } else {
+        bv[n][0] = j + 2 * t < Q ? __ldg(bias0 + j) : 0.f;
+        bv[n][1] = j + 2 * t + 1 < Q ? __ldg(bias0 + j + 1) : 0.f;
+        bv[n][2] = j + 2 * t < Q ? __ldg(bias1 + j) : 0.f;
+        bv[n][3] = j + 2 * t + 1 < Q ? __ldg(bias1 + j + 1) : 0.f;
       }
     }
   };
-
-  // fp16: where the row of column lane % 8 of column group n lies (group n + 2 is four keys further on)
-  auto row_of = [&](int n) { return (((lane & 7) >> 1) * 8 + n * 2 + (lane & 1)) * PITCH + ((lane & 7) >> 1) * 16; };
 
   float o[ND][4];
 #pragma unroll
@@ -256,7 +220,7 @@ attention_kernel(const uint16_t* __restrict__ qkvg, const void* __restrict__ bia
 #pragma unroll 1
     for (int step = 0; step < s.kt && tile * s.kt + step < Q; step += KT) {
     const int key0 = tile * s.kt + step;
-    const uint16_t* k_s = kv_s + (buf * s.wb + wb) * 2 * TERMS * plane + at_rows(D, TERMS, step);
+    const uint16_t* k_s = kv_s + (buf * s.wb + wb) * 2 * TERMS * plane + step * PITCH;
     const uint16_t* v_s = k_s + TERMS * plane;
     const float* ms = mask_s + wb * s.mk + key0 - mask0;
     // ---- S = Q K^T for 32 keys (four accumulators in flight): small term products first, the leading one last ----
@@ -268,7 +232,7 @@ attention_kernel(const uint16_t* __restrict__ qkvg, const void* __restrict__ bia
     {
       uint32_t kb[TERMS][2][4];
       // matrices (keys 0-7, k 0-7), (keys 0-7, k 8-15), (keys 8-15, k 0-7), (keys 8-15, k 8-15) of each 16 keys
-      const uint16_t* base = k_s + (TERMS == 1 ? row_of(lane >> 4) : ((lane & 7) + (lane >> 4) * 8) * PITCH) + ((lane >> 3) & 1) * 8;
+      const uint16_t* base = k_s + ((lane & 7) + (lane >> 4) * 8) * PITCH + ((lane >> 3) & 1) * 8;
       // the term products below the leading one first, over all channels; the leading ones last
 #pragma unroll
       for (int pass = TOP; pass >= 0; pass -= 2) {
@@ -277,53 +241,35 @@ attention_kernel(const uint16_t* __restrict__ qkvg, const void* __restrict__ bia
 #pragma unroll
           for (int i = 0; i <= pass; ++i)
 #pragma unroll
-            for (int grp = 0; grp < 2; ++grp) ldmatrix4<false>(kb[i][grp], base + i * plane + grp * (TERMS == 1 ? 4 : 16) * PITCH + kk * 16);
+            for (int grp = 0; grp < 2; ++grp) ldmatrix4<false>(kb[i][grp], base + i * plane + grp * 16 * PITCH + kk * 16);
 #pragma unroll
           for (int order = pass; order >= (pass ? 1 : 0); --order)        // terms i and order - i
 #pragma unroll
             for (int i = 0; i <= order; ++i)
 #pragma unroll
-              for (int n = 0; n < 4; ++n) {
-                const uint32_t b0 = kb[order - i][n >> 1][(n & 1) * 2], b1 = kb[order - i][n >> 1][(n & 1) * 2 + 1];
-                if (TERMS == 1) mma16h(l[n], qa[i][kk], b0, b1); else mma16(l[n], qa[i][kk], b0, b1);
-              }
+              for (int n = 0; n < 4; ++n) mma16(l[n], qa[i][kk], kb[order - i][n >> 1][(n & 1) * 2], kb[order - i][n >> 1][(n & 1) * 2 + 1]);
         }
         if (TAIL) {
           // matrices: keys 0-7, 8-15, 16-23, 24-31 of the last eight channels
 #pragma unroll
-          for (int i = 0; i <= pass; ++i) ldmatrix4<false>(kb[i][0], k_s + i * plane + (TERMS == 1 ? row_of(lane >> 3) : lane * PITCH) + NK * 16);
+          for (int i = 0; i <= pass; ++i) ldmatrix4<false>(kb[i][0], k_s + i * plane + lane * PITCH + NK * 16);
 #pragma unroll
           for (int order = pass; order >= (pass ? 1 : 0); --order)
 #pragma unroll
             for (int i = 0; i <= order; ++i)
 #pragma unroll
-              for (int n = 0; n < 4; ++n) {
-                if (TERMS == 1) mma8h(l[n], qt[i][0], qt[i][1], kb[order - i][0][n]); else mma8(l[n], qt[i][0], qt[i][1], kb[order - i][0][n]);
-              }
+              for (int n = 0; n < 4; ++n) mma8(l[n], qt[i][0], qt[i][1], kb[order - i][0][n]);
         }
       }
     }
     // ---- logits ----
 #pragma unroll
     for (int n = 0; n < 4; ++n) {
-      const float2 m2 = *reinterpret_cast<const float2*>(ms + KEY_T * t + KEY_N * n);
-      float add[4] = {0.f, 0.f, 0.f, 0.f};
-      if constexpr (BIAS && TERMS == 1) {
-#pragma unroll
-        for (int r = 0; r < 2; ++r) {
-          const uint32_t w = n == 0 ? bh[r].x : n == 1 ? bh[r].y : n == 2 ? bh[r].z : bh[r].w;
-          const float2 v = __half22float2(*reinterpret_cast<const __half2*>(&w));
-          add[2 * r] = v.x;
-          add[2 * r + 1] = v.y;
-        }
-      } else if constexpr (BIAS) {
-#pragma unroll
-        for (int e = 0; e < 4; ++e) add[e] = bv[n][e];
-      }
+      const float2 m2 = *reinterpret_cast<const float2*>(ms + 2 * t + 8 * n);
 #pragma unroll
       for (int e = 0; e < 4; ++e) {
         l[n][e] = fmaf(l[n][e], s.scale, (e & 1) ? m2.y : m2.x);
-        if (BIAS) l[n][e] += add[e];
+        if (BIAS) l[n][e] += bv[n][e];
         if (s.clamp) l[n][e] = fminf(fmaxf(l[n][e], -1e8f), 1e8f);
       }
     }
@@ -332,7 +278,7 @@ attention_kernel(const uint16_t* __restrict__ qkvg, const void* __restrict__ bia
       for (int n = 0; n < 4; ++n)
 #pragma unroll
         for (int e = 0; e < 4; ++e)
-          if (key0 + KEY_T * t + KEY_N * n + (e & 1) >= Q) l[n][e] = -INFINITY;
+          if (key0 + 2 * t + 8 * n + (e & 1) >= Q) l[n][e] = -INFINITY;
     }
     if (BIAS && key0 + KT < Q) load_bias(key0 + KT);      // for the next step
     auto row_max = [&](int r) {
@@ -377,7 +323,7 @@ attention_kernel(const uint16_t* __restrict__ qkvg, const void* __restrict__ bia
       ps[1] = (c[0] + c[1]) + (c[2] + c[3]);
     };
     exponentials();
-    constexpr float kBig = TERMS == 1 ? 32768.0f : 1.1529215e18f;      // fp16 probabilities stay in range; 2^60
+    constexpr float kBig = 1.1529215e18f;      // 2^60
     if (__any_sync(0xffffffffu, !(ps[0] <= kBig) || !(ps[1] <= kBig))) {
 #pragma unroll
       for (int r = 0; r < 2; ++r) {
@@ -406,43 +352,33 @@ attention_kernel(const uint16_t* __restrict__ qkvg, const void* __restrict__ bia
 #pragma unroll
       for (int r = 0; r < 4; ++r) {      // (row0, keys 2t), (row1, same), then keys + 8
         const float x = p[grp * 2 + (r >> 1)][(r & 1) * 2], y = p[grp * 2 + (r >> 1)][(r & 1) * 2 + 1];
-        if constexpr (TERMS == 1) pa[0][r] = pack_half(x, y);
-        else {
-          uint32_t term[3];
-          split3_cut(x, y, term);
+        uint32_t term[3];
+        split3_cut(x, y, term);
 #pragma unroll
-          for (int i = 0; i < 3; ++i) pa[i][r] = term[i];
-        }
+        for (int i = 0; i < 3; ++i) pa[i][r] = term[i];
       }
 #pragma unroll
       for (int np = 0; np < ND; np += 2) {
         uint32_t vb[TERMS][4];
 #pragma unroll
         for (int i = 0; i < TERMS; ++i) {
-          const uint16_t* base = v_s + i * plane + (TERMS == 1 ? row_of((lane >> 3) & 1) + grp * 4 * PITCH : (grp * 16 + (lane & 15)) * PITCH) + np * 8;
+          const uint16_t* base = v_s + i * plane + (grp * 16 + (lane & 15)) * PITCH + np * 8;
           if (np + 1 < ND) ldmatrix4<true>(vb[i], base + (lane >> 4) * 8);
           else ldmatrix2<true>(vb[i][0], vb[i][1], base);
         }
-        if constexpr (TERMS == 1) {
-          mma16h(o[np], pa[0], vb[0][0], vb[0][1]);
-          if (np + 1 < ND) mma16h(o[np + 1], pa[0], vb[0][2], vb[0][3]);
-        } else {
 #pragma unroll
-          for (int order = TOP; order >= 0; --order)
+        for (int order = TOP; order >= 0; --order)
 #pragma unroll
-            for (int i = 0; i <= order; ++i) {
-              mma16(order ? fc[np] : f[np], pa[i], vb[order - i][0], vb[order - i][1]);
-              if (np + 1 < ND) mma16(order ? fc[np + 1] : f[np + 1], pa[i], vb[order - i][2], vb[order - i][3]);
-            }
-        }
+          for (int i = 0; i <= order; ++i) {
+            mma16(order ? fc[np] : f[np], pa[i], vb[order - i][0], vb[order - i][1]);
+            if (np + 1 < ND) mma16(order ? fc[np + 1] : f[np + 1], pa[i], vb[order - i][2], vb[order - i][3]);
+          }
       }
     }
-    if (TERMS > 1) {
 #pragma unroll
     for (int n = 0; n < ND; ++n)
 #pragma unroll
       for (int e = 0; e < 4; ++e) o[n][e] += f[n][e] + fc[n][e];
-    }
     }
   }
   if (!active) return;
@@ -457,23 +393,17 @@ attention_kernel(const uint16_t* __restrict__ qkvg, const void* __restrict__ bia
     uint16_t* dst = out + ((int64_t)b * Q + row) * s.ldo + h * D + 2 * t;
 #pragma unroll
     for (int n = 0; n < ND; ++n) {
-      if constexpr (TERMS == 1) {
-        float2 g2 = __half22float2(*reinterpret_cast<const __half2*>(gate + n * 8));
-        if (s.gate_logits) { g2.x = 1.0f / (1.0f + __expf(-g2.x)); g2.y = 1.0f / (1.0f + __expf(-g2.y)); }
-        *reinterpret_cast<uint32_t*>(dst + n * 8) = pack_half(o[n][2 * r] * inv * g2.x, o[n][2 * r + 1] * inv * g2.y);
-      } else {
-        float gx = 0.f, gy = 0.f;
+      float gx = 0.f, gy = 0.f;
 #pragma unroll
-        for (int i = 2; i >= 0; --i) {
-          const uint32_t w = *reinterpret_cast<const uint32_t*>(gate + i * s.term_stride + n * 8);
-          gx += __uint_as_float(w << 16);
-          gy += __uint_as_float(w & 0xffff0000u);
-        }
-        uint32_t term[3];
-        split3(o[n][2 * r] * inv * gx, o[n][2 * r + 1] * inv * gy, term);
-#pragma unroll
-        for (int i = 0; i < 3; ++i) *reinterpret_cast<uint32_t*>(dst + i * s.out_stride + n * 8) = term[i];
+      for (int i = 2; i >= 0; --i) {
+        const uint32_t w = *reinterpret_cast<const uint32_t*>(gate + i * s.term_stride + n * 8);
+        gx += __uint_as_float(w << 16);
+        gy += __uint_as_float(w & 0xffff0000u);
       }
+      uint32_t term[3];
+      split3(o[n][2 * r] * inv * gx, o[n][2 * r + 1] * inv * gy, term);
+#pragma unroll
+      for (int i = 0; i < 3; ++i) *reinterpret_cast<uint32_t*>(dst + i * s.out_stride + n * 8) = term[i];
     }
   }
 }

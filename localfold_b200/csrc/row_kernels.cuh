@@ -417,16 +417,6 @@ __global__ void finish4_kernel(const float* __restrict__ proj, const float* __re
   store4(out + dst * ch + c, v);
 }
 
-// fp16 columns col0 .. col0 + heads of rows (i * Q + j) -> bias[h][i][ldb] (zeros past Q), or its transpose when `swap`
-__global__ void bias_columns_half_kernel(const __half* __restrict__ in, int64_t ld, int col0, int Q, int ldb, int heads, int swap, __half* __restrict__ out) {
-  lf_chain();
-  const int64_t idx = (int64_t)blockIdx.x * blockDim.x + threadIdx.x, plane = (int64_t)Q * ldb;
-  if (idx >= plane) return;
-  const uint32_t i = (uint32_t)(idx / ldb), j = (uint32_t)(idx % ldb);
-  const __half* row = in + (swap ? (int64_t)j * Q + i : (int64_t)i * Q + j) * ld + col0;
-  for (int h = 0; h < heads; ++h) out[h * plane + idx] = j < (uint32_t)Q ? row[h] : __float2half_rn(0.f);
-}
-
 // columns col0 .. col0 + heads of rows (i * Q + j) of a terms matrix -> bias[h][i][j], or [h][j][i] when `swap`
 __global__ void bias_columns_kernel(const bf16* __restrict__ in, int64_t ld, int64_t term_stride, int col0, int Q, int heads, int swap, float* __restrict__ out) {
   lf_chain();

@@ -15,7 +15,7 @@ enum JobKind {
   JOB_BIASED,     // ... -> fp16 [n_out][K + 16], bias in k column K and zeros after it (the activations carry a column of ones there)
   JOB_FOLD,       // float [n_out]: scale * (bias[c] + sum_k vec[k] W[k][col0 + c]): a LayerNorm offset folded into a bias
   JOB_TERMS,      // ... -> three bf16 terms [3][rows][n_pad] at row0, zeros past K (n_pad = K rounded up to 8)
-  JOB_HEADS,      // the fused attention projection as terms (as fp16 without a term_stride), every head of d channels (row0) padded with zero rows to D (n_pad)
+  JOB_HEADS,      // the fused attention projection as terms, every head of d channels (row0) padded with zero rows to D (n_pad)
   JOB_HEADS_BIAS, // ... its bias vector, as float32
   JOB_HEADS_OUT,  // the output projection as terms, the k of every head padded likewise
   JOB_COLSUM      // float [n_out]: sum_k fp16(vec[k] W[k][col0 + c]): what the tensor core multiplies the mean by
@@ -69,10 +69,6 @@ __global__ void __launch_bounds__(256) weight_jobs_kernel(const __grid_constant_
       float v = 0.f;
       if (out_proj) { if (k % D < d) v = j.w[(int64_t)(k / D * d + k % D) * j.ld + n]; }
       else if (k < j.K && n % D < d) v = j.w[(int64_t)k * j.ld + n / D * d + n % D];
-      if (j.term_stride == 0) {
-        reinterpret_cast<op16*>(j.out)[(int64_t)n * kk + k] = __float2half_rn(v);
-        continue;
-      }
       bf16* t = reinterpret_cast<bf16*>(j.out) + (int64_t)n * kk + k;
 #pragma unroll
       for (int e = 0; e < 3; ++e) {
@@ -155,7 +151,6 @@ lf_status prepare_weights(lf_context* ctx, lf_weights* w, WeightCursor& cur) {
   Preparer prep{ctx, cur};
   w->h.clear();
   w->g.clear();
-  w->head_form = false;
   if (tri && w->dims.channels == 128 && w->dims.hidden == 128) {
     // the input LayerNorm's gain goes into the rows of the images, its offset into the biases: the kernels' producers
     // hand the tensor core (x - mean) / std
@@ -226,26 +221,15 @@ lf_status prepare_weights(lf_context* ctx, lf_weights* w, WeightCursor& cur) {
     prep.fold(f[TRN_W1], 128, 1024, 0, 1024, f[TRN_LN_B], f[TRN_B1], 1.0f, b1);
     w->h = {img, b1};
   }
-  // Operands of the plain fp16 GEMM for the widths the fused kernels do not take: weights [k][n] -> fp16 [n][k]
-  if (att && (w->h.empty() || !w->h[0]) && w->dims.heads > 0 && w->dims.channels % 8 == 0) {
-    const int c = w->dims.channels, H = w->dims.heads, d = w->dims.head_dim, HD = H * d;
-    const bool own_bias = w->has_pair_proj && !w->has_pair_norm;
-    if (d == 32 && H % 4 == 0 && !own_bias) {      // what the tcgen05 core takes four heads at a time
-      op16 *w4 = cur.take<op16>((size_t)4 * HD * c), *wo = cur.take<op16>((size_t)c * HD);
-      prep.operand(f[ATT_W4], c, 4 * HD, 4 * HD, w4);
-      prep.operand(f[ATT_WO], HD, c, c, wo);
-      w->g = {w4, wo};
-    } else if (d <= 64) {
-      const int D = head_width(d), heads = 4 * H * D, wide = (heads + (own_bias ? H : 0) + 7) / 8 * 8;
-      op16 *w4 = cur.take<op16>((size_t)wide * c), *wo = cur.take<op16>((size_t)c * H * D);
-      float* bias = cur.take<float>(wide);
-      prep.push(Job{f[ATT_W4], nullptr, nullptr, w4, 1.0f, JOB_HEADS, c, 4 * HD, 0, 4 * HD, heads, D, d, 0});
-      if (wide > heads) prep.push(Job{f[ATT_WB], nullptr, nullptr, w4 + (size_t)heads * c, 1.0f, JOB_OPERAND, c, H, 0, H, wide - heads, 0, 0, 0});
-      prep.push(Job{f[ATT_WO], nullptr, nullptr, wo, 1.0f, JOB_HEADS_OUT, HD, c, 0, c, H * D, D, d, 0});
-      prep.push(Job{f[ATT_B4], nullptr, nullptr, bias, 1.0f, JOB_HEADS_BIAS, 0, 0, 0, 4 * HD, wide, D, d, 0});
-      w->g = {w4, wo, bias};
-      w->head_form = true;
-    }
+  // Operands of the plain fp16 GEMM for the widths the fused kernels do not take: weights [k][n] -> fp16 [n][k]; attention: the heads
+  // that the tcgen05 core takes four at a time
+  if (att && (w->h.empty() || !w->h[0]) && w->dims.channels % 8 == 0 && w->dims.head_dim == 32 && w->dims.heads > 0 && w->dims.heads % 4 == 0 &&
+      !(w->has_pair_proj && !w->has_pair_norm)) {
+    const int c = w->dims.channels, HD = w->dims.heads * 32;
+    op16 *w4 = cur.take<op16>((size_t)4 * HD * c), *wo = cur.take<op16>((size_t)c * HD);
+    prep.operand(f[ATT_W4], c, 4 * HD, 4 * HD, w4);
+    prep.operand(f[ATT_WO], HD, c, c, wo);
+    w->g = {w4, wo};
   }
   if ((w->kind == LF_WEIGHTS_TRANSITION_AF2 || w->kind == LF_WEIGHTS_TRANSITION_AF3) && w->h.empty() &&
       w->dims.channels % 8 == 0 && w->dims.hidden % 8 == 0) {

@@ -1,6 +1,7 @@
 """What 16-bit mode rounds at widths the fused 128-channel kernels do not take: of a triangle update only a, b and the
-stored product x.  The float64 evaluation here rounds exactly those, so what is left between it and the GPU is float32
-arithmetic and the values that land on the other side of a rounding boundary because of it."""
+stored product x, of an attention whose heads the tcgen05 core does not take nothing.  The float64 evaluation of the triangle
+update here rounds exactly those, so what is left between it and the GPU is float32 arithmetic and the values that land on
+the other side of a rounding boundary because of it."""
 import numpy as np
 import pytest
 import torch
@@ -52,3 +53,19 @@ def test_triangle_update_rounds_its_contraction_only(dev, n, c, incoming):
     op = (lf.TriangleMultiplicationIncomingGpu if incoming else lf.TriangleMultiplicationOutgoingGpu)(dev)
     got = op.run({"shape": {"length": n, "cZ": c, "cHidden": c}, "z": z, "mask": mask, "weights": w}, {"precision": "bf16", "variance": "two-pass"})["output"]
     assert _relative(got, _triangle_with_16_bit_contraction(z, mask, w, incoming)) <= 1e-4
+
+
+# Heads that the tcgen05 core (groups of four heads of 32, no bias from the normalised input beside 128 channels) does not take run in
+# float32 in either mode: the float32 mode's bound.
+@pytest.mark.parametrize("q,heads,dim,transpose,own_bias", [(20, 4, 16, False, True), (65, 8, 8, True, True), (47, 12, 32, True, True), (129, 3, 24, False, True),
+                                                            (33, 8, 8, False, False), (130, 4, 16, True, False)])
+def test_attention_of_other_heads_is_float32(dev, q, heads, dim, transpose, own_bias):
+    import localfold_b200 as lf
+    d = syn.draw(5100 + q)
+    c = heads * dim
+    act, mask = d.normal(q, q, c), (d.rng.random((q, q)) > 0.2).astype(np.float32)
+    w = syn.af2_attention_weights(d, c, heads, c)
+    pb = dict(w["pairBias"], source="normalized-input") if own_bias else None
+    got = lf.AttentionGpu(dev).run({"activations": act, "mask": mask, "batch": q, "queryLength": q, "channels": c, "heads": heads, "weights": w["attention"],
+                                    "transpose": transpose, "pairBias": pb}, {"precision": "bf16", "variance": "two-pass"})["output"]
+    assert _relative(got, t2.attention_af2(act, mask, q, q, c, heads, w["attention"], transpose, pb)) <= 1e-5
