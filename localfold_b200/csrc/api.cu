@@ -1015,7 +1015,10 @@ void configure_mma_attention() {
 }
 #undef ATTENTION_WIDTHS
 
-bool aligned16(const void* p) { return ((uintptr_t)p & 15) == 0; }
+// The row kernels around the fp16 GEMMs take float32 rows 16 bytes at a time, bfloat16 ones value by value.
+bool half_rows_take(const void* resid, const void* out, int act_dtype) {
+  return act_dtype == LF_DTYPE_BF16 || (lf_aligned16(resid) && lf_aligned16(out));
+}
 
 // LayerNorm of `count` rows of c channels in one of its output forms; widths with a register form take it, others a warp a row.
 template <typename T, int OUT>
@@ -1025,7 +1028,7 @@ void layer_norm(lf_context* ctx, ArenaCursor& cur, const void* act, int64_t coun
 #define LN_CASE(NV_, L_, R_)                                                                                                                    \
   LAUNCH(ctx, cur, (rows::layer_norm_rows_kernel<T, NV_, L_, OUT, R_>), lf_ceil_div(count, 256 / L_ * R_), 256, 0, in, count, gamma, beta, eps, \
          variance, transpose, batch, Q, out, term_stride)
-  const bool wide = aligned16(act) && count < ((int64_t)1 << 32);
+  const bool wide = lf_aligned16(act) && count < ((int64_t)1 << 32);
   if (wide && c == 64) LN_CASE(1, 16, 4);
   else if (wide && c == 128) LN_CASE(1, 32, 4);
   else if (wide && c == 256) LN_CASE(2, 32, 2);
@@ -1049,7 +1052,7 @@ void layer_norm(lf_context* ctx, ArenaCursor& cur, const void* act, int64_t coun
 template <typename T>
 void finish(lf_context* ctx, ArenaCursor& cur, const float* proj, const float* gate, const void* resid, int64_t count, int c, int transpose, int batch,
             int Q, void* out) {
-  if ((c & 3) == 0 && aligned16(resid) && aligned16(out) && count < ((int64_t)1 << 32))
+  if ((c & 3) == 0 && lf_aligned16(resid) && lf_aligned16(out) && count < ((int64_t)1 << 32))
     LAUNCH(ctx, cur, (rows::finish4_kernel<T>), lf_ceil_div(count * (c / 4), 256), 256, 0, proj, gate, (const T*)resid, count, c, transpose, batch, Q, (T*)out);
   else
     LAUNCH(ctx, cur, (simt::finish_kernel<T>), lf_ceil_div(count * c, 256), 256, 0, proj, gate, (const T*)resid, count, c, transpose, batch, Q, (T*)out);
@@ -1210,7 +1213,7 @@ lf_status tri_bf16(lf_context* ctx, ArenaCursor& cur, const TriArgs& a) {
 
 lf_status tri_dispatch(lf_context* ctx, ArenaCursor& cur, const TriArgs& a, int precision) {
   const bool half = precision == LF_PRECISION_BF16 && tc::contract_supported(a.n, a.c);
-  if (half && tc::ln_gemm_supported(a.w)) return tri_bf16(ctx, cur, a);
+  if (half && tc::ln_gemm_supported(a.w) && lf_fused_takes(a.z, a.residual ? a.z : nullptr, a.out, a.act_dtype)) return tri_bf16(ctx, cur, a);
   const bool planes = half && a.c % 8 == 0;      // whole 16-byte pieces of channels
   return a.act_dtype == LF_DTYPE_BF16 ? tri_general<bf16>(ctx, cur, a, planes) : tri_general<float>(ctx, cur, a, planes);
 }
@@ -1229,11 +1232,14 @@ struct AttArgs {
   const lf_weights* w;
 };
 
+// Whether the fused projection kernel makes the bias of a.bias_mode 1 from the pair.
+bool tensor_core_bias(const AttArgs& a) { return tc::pair_bias_supported(a.w) && !a.bias_swap && lf_aligned16(a.pair); }
+
 // The pair bias of a.bias_mode 1 (a pair tensor with a LayerNorm of its own) as float32 [heads][Q][Q].
 lf_status separate_bias(lf_context* ctx, ArenaCursor& cur, const AttArgs& a, float* bias) {
   const auto& f = a.w->f;
   const int64_t QQ = (int64_t)a.Q * a.Q;
-  if (a.tc_pair_bias && tc::pair_bias_supported(a.w) && !a.bias_swap) {
+  if (a.tc_pair_bias && tensor_core_bias(a)) {
     // the pair-sized pass of this operator: LayerNorm of the pair and its projection onto the heads, fp16 out
     const int ldb = (a.Q + 15) / 16 * 16;
     op16* b16 = cur.take<op16>((int64_t)a.heads * a.Q * ldb);
@@ -1353,9 +1359,7 @@ bool hgemm_supported(const lf_weights* w) { return gemm_operand(w, 0) && gemm_op
 // Whether an output projection can leave as float32 rows straight from its GEMM: float32 activations, updated in place
 // (the rows are added to where they live) or written without a residual.
 template <typename T>
-bool rows_in_place(int residual, const void* act, const void* out, int c) {
-  return sizeof(T) == 4 && (!residual || act == out) && tc::gemm_rows_supported(out, c);
-}
+bool rows_in_place(int residual, const void* act, const void* out) { return sizeof(T) == 4 && (!residual || act == out); }
 
 // 16-bit path for the shapes the fused projection kernel does not take (MSA row attention with pair bias: c_m = 256,
 // 8 heads of 32; MSA column attention): LayerNorm to fp16, the q/k/v/gate projection as one tensor-core GEMM that writes the
@@ -1383,7 +1387,7 @@ lf_status att_mixed(lf_context* ctx, ArenaCursor& cur, const AttArgs& a) {
     LF_TRY(tc::attention_core(ctx, cur, part(0), part(1), part(2), part(3), bias16 ? bias16 + (int64_t)gi * 4 * a.Q * ldb : nullptr, ldb, a.mask, a.batch,
                               a.Q, a.transpose, a.mask_mode, a.clamp, o + (int64_t)gi * RP * 128));
   }
-  if (rows_in_place<T>(a.residual, a.act, a.out, c))
+  if (rows_in_place<T>(a.residual, a.act, a.out))
     return tc::gemm_rows_f32(ctx, cur, o, 1, gemm_operand(a.w, 1), (float*)a.out, a.residual, a.batch, a.Q, ldb, a.transpose, c, HD, f[ATT_BO]);
   op16* proj = nrm;   // the normalised input is dead
   LF_TRY(tc::gemm_rows_half(ctx, cur, o, gemm_operand(a.w, 1), proj, a.batch, a.Q, ldb, c, HD));
@@ -1393,11 +1397,13 @@ lf_status att_mixed(lf_context* ctx, ArenaCursor& cur, const AttArgs& a) {
 }
 
 lf_status att_dispatch(lf_context* ctx, ArenaCursor& cur, const AttArgs& a, int precision) {
-  if (precision == LF_PRECISION_BF16 && a.bias_mode != 1 && a.heads == 4 && a.d == 32 && tc::ln_gemm_supported(a.w)) {
+  const void* resid = a.residual ? a.act : nullptr;
+  if (precision == LF_PRECISION_BF16 && a.bias_mode != 1 && a.heads == 4 && a.d == 32 && tc::ln_gemm_supported(a.w) &&
+      lf_fused_takes(a.act, resid, a.out, a.act_dtype)) {
     return a.act_dtype == LF_DTYPE_BF16 ? att_bf16<bf16>(ctx, cur, a) : att_bf16<float>(ctx, cur, a);
   }
   if (precision == LF_PRECISION_BF16 && a.d == 32 && a.heads % 4 == 0 && hgemm_supported(a.w) &&
-      (a.bias_mode == 0 || (a.bias_mode == 1 && tc::pair_bias_supported(a.w) && !a.bias_swap))) {
+      half_rows_take(resid, a.out, a.act_dtype) && (a.bias_mode == 0 || (a.bias_mode == 1 && tensor_core_bias(a)))) {
     return a.act_dtype == LF_DTYPE_BF16 ? att_mixed<bf16>(ctx, cur, a) : att_mixed<float>(ctx, cur, a);
   }
   AttArgs b = a;
@@ -1463,7 +1469,7 @@ lf_status trn_half(lf_context* ctx, ArenaCursor& cur, const TrnArgs& a) {
     } else {
       LF_TRY(hgemm(ctx, cur, nrm, w1, h1, count, wide, c16, nullptr, 1));     // ReLU in the GEMM's epilogue
     }
-    if (rows_in_place<T>(a.residual, a.act, a.out, c)) {
+    if (rows_in_place<T>(a.residual, a.act, a.out)) {
       LF_TRY(tc::gemm_rows_f32(ctx, cur, h2, 0, w2, (float*)out, a.residual, 1, (int)count, 0, 0, c, hd, f[TRN_B2]));
       continue;
     }
@@ -1475,9 +1481,10 @@ lf_status trn_half(lf_context* ctx, ArenaCursor& cur, const TrnArgs& a) {
 }
 
 lf_status trn_dispatch(lf_context* ctx, ArenaCursor& cur, const TrnArgs& a, int precision) {
-  if (precision == LF_PRECISION_BF16 && tc::transition_supported(a.w))
-    return tc::transition_run(ctx, cur, a.act, a.act_dtype, a.rows, a.variance, a.eps, a.w, a.residual ? a.act : nullptr, a.out);
-  if (precision == LF_PRECISION_BF16 && hgemm_supported(a.w))
+  const void* resid = a.residual ? a.act : nullptr;
+  if (precision == LF_PRECISION_BF16 && tc::transition_supported(a.w) && lf_fused_takes(a.act, resid, a.out, a.act_dtype))
+    return tc::transition_run(ctx, cur, a.act, a.act_dtype, a.rows, a.variance, a.eps, a.w, resid, a.out);
+  if (precision == LF_PRECISION_BF16 && hgemm_supported(a.w) && half_rows_take(resid, a.out, a.act_dtype))
     return a.act_dtype == LF_DTYPE_BF16 ? trn_half<bf16>(ctx, cur, a) : trn_half<float>(ctx, cur, a);
   return a.act_dtype == LF_DTYPE_BF16 ? trn_f32<bf16>(ctx, cur, a) : trn_f32<float>(ctx, cur, a);
 }
@@ -1661,7 +1668,7 @@ lf_status lf_outer_product_mean_run(lf_context* ctx, const lf_opm_desc* d, lf_re
     const auto& f = w->f;
     const int ban = d->bias_after_norm ? 1 : 0;
     // 16-bit mode, widths in whole groups of 8: every GEMM of the operator runs on the tensor cores
-    const bool tc_full = d->precision == LF_PRECISION_BF16 && c % 8 == 0 && hgemm_supported(w);
+    const bool tc_full = d->precision == LF_PRECISION_BF16 && c % 8 == 0 && hgemm_supported(w) && half_rows_take(resid, out, d->act_dtype);
     float* nrm = tc_full ? nullptr : cur.take<float>(rows * cm);
     float* left = tc_full ? nullptr : cur.take<float>(rows * c);
     float* right = tc_full ? nullptr : cur.take<float>(rows * c);
@@ -1831,8 +1838,8 @@ lf_status global_attention(lf_context* ctx, ArenaCursor& cur, const lf_global_at
   LF_TRY(tc::gemm_f32(ctx, cur, 0, nrm, g[0], (int)R, wide, c, 1, {kvg, nullptr, ld, 0, 0, f[GLB_B3], wide, 0, 2 * hd, wide}));
   const bool wide_rows = c > 512;      // more channels than a lane keeps: the sums of the normalised rows, from their terms
   if (wide_rows) LAUNCH(ctx, cur, rows::global_mean_terms_kernel, n, 512, 0, nrm.p, nrm.ld, nrm.term_stride, mask, S, n, c, sums);
-  else if (c == 64 && aligned16(act)) LAUNCH(ctx, cur, (rows::global_mean_rows_kernel<T, 1, 16>), n, 512, 0, (const T*)act, mask, S, n, d->epsilon, d->variance, sums);
-  else if (c == 128 && aligned16(act)) LAUNCH(ctx, cur, (rows::global_mean_rows_kernel<T, 1, 32>), n, 512, 0, (const T*)act, mask, S, n, d->epsilon, d->variance, sums);
+  else if (c == 64 && lf_aligned16(act)) LAUNCH(ctx, cur, (rows::global_mean_rows_kernel<T, 1, 16>), n, 512, 0, (const T*)act, mask, S, n, d->epsilon, d->variance, sums);
+  else if (c == 128 && lf_aligned16(act)) LAUNCH(ctx, cur, (rows::global_mean_rows_kernel<T, 1, 32>), n, 512, 0, (const T*)act, mask, S, n, d->epsilon, d->variance, sums);
   else
     LAUNCH(ctx, cur, (rows::global_mean_kernel<T>), n, 512, (size_t)16 * (c + 1) * sizeof(float), (const T*)act, mask, S, n, c, d->epsilon, d->variance, sums);
   LAUNCH(ctx, cur, rows::global_query_kernel, n, 128, (size_t)c * sizeof(float), sums, wide_rows ? nullptr : f[GLB_LN_G], f[GLB_LN_B], c, HD, 1.0f / sqrtf((float)hd), f[GLB_WQ], q);
@@ -1996,6 +2003,9 @@ lf_status lf_pair_shard_step(lf_context* ctx, const lf_shard_step_desc* d, lf_re
     return lf_fail(ctx, LF_ERR_UNSUPPORTED, "shard step needs transition weights 128 -> 512 -> 128");
   if ((tri || d->op == LF_SHARD_ATTENTION_PROJECT) && d->variance != LF_VARIANCE_TWO_PASS && d->variance != LF_VARIANCE_FAST)
     return lf_fail(ctx, LF_ERR_ARGUMENT, "variance has no default: pass LF_VARIANCE_TWO_PASS or LF_VARIANCE_FAST");
+  const bool writes = d->op == LF_SHARD_TRIANGLE_OUTPUT || d->op == LF_SHARD_ATTENTION_OUTPUT || d->op == LF_SHARD_TRANSITION;
+  if (!lf_fused_takes(d->pair, writes ? d->pair : nullptr, writes ? d->pair : nullptr, d->act_dtype))
+    return lf_fail(ctx, LF_ERR_ARGUMENT, "shard step: the pair must lie on a 16-byte boundary (a bfloat16 pair that is updated, 32)");
   cudaSetDevice(ctx->device);
   const uint64_t before = ctx->launches;
   ArenaCursor cur{ctx, 0, false};
@@ -2061,6 +2071,7 @@ lf_status lf_pair_shard_exchange_step(lf_context* ctx, const lf_shard_step_desc*
     }
     return LF_OK;
   };
+  if (!lf_aligned16(d->pair)) return lf_fail(ctx, LF_ERR_ARGUMENT, "exchange step: the pair must lie on a 16-byte boundary");
   cudaSetDevice(ctx->device);
   const uint64_t before = ctx->launches;
   ArenaCursor cur{ctx, 0, false};

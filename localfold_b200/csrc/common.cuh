@@ -197,4 +197,13 @@ static inline void lf_weights_await(lf_context* ctx, const lf_weights* w) {
 // The pair stack with the pair left in host memory (pair_spill.cu).
 lf_status lf_pair_stack_spilled(lf_context* ctx, const lf_pair_stack_desc* d, lf_result* r);
 
+static inline bool lf_aligned16(const void* p) { return ((uintptr_t)p & 15) == 0; }
+// Whether the fused 128-channel kernels take the caller's activations where they lie (the general path takes any address): they load 16
+// bytes at a time and store by TMA, but rows that leave by threads' stores - bfloat16 ones, and float32 ones whose residual lives
+// elsewhere - take 32-byte accesses.
+static inline bool lf_fused_takes(const void* act, const void* resid, const void* out, int act_dtype) {
+  const uintptr_t low = act_dtype == LF_DTYPE_F32 && (!resid || resid == out) ? 15 : 31;
+  return lf_aligned16(act) && (((uintptr_t)resid | (uintptr_t)out) & low) == 0;
+}
+
 static inline int lf_ceil_div(int64_t a, int64_t b) { return (int)((a + b - 1) / b); }

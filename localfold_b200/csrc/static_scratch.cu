@@ -75,6 +75,9 @@ extern "C" lf_status lf_triangle_multiplication_run_static(lf_context* ctx, cons
       !tc::contract_supported(d->length, 128))
     return lf_fail(ctx, LF_ERR_UNSUPPORTED, "the no-allocation entry point covers cZ = cHidden = 128 on a device with tensor-map support");
 
+  if (!lf_fused_takes(d->z, d->residual ? d->z : nullptr, d->out, d->act_dtype))
+    return lf_fail(ctx, LF_ERR_ARGUMENT, "the no-allocation entry point needs activations on a 16-byte boundary (bfloat16 ones, or a residual apart from "
+                                         "the output, 32)");
   cudaSetDevice(ctx->device);
   void* scratch = nullptr;
   LF_TRY(static_scratch_setup(ctx, &scratch));

@@ -324,8 +324,6 @@ lf_status gemm_pieces(lf_context* ctx, ArenaCursor& cur, const op16* a, const op
   return launch<0, GM_PIECES>(ctx, LF_KERNEL_TRIANGLE_CONTRACT, ma, mb, mo, p);
 }
 
-bool gemm_rows_supported(const void* out, int n_out) { return ((uintptr_t)out & 15) == 0 && n_out % 4 == 0; }
-
 lf_status gemm_rows_f32(lf_context* ctx, ArenaCursor& cur, const op16* a, int a_pieces, const op16* w, float* out, int add, int batch, int Q, int ldq,
                         int transposed, int n_out, int k_len, const float* bias) {
   if (cur.dry) return LF_OK;

@@ -53,8 +53,7 @@ void configure_gemm();
 lf_status gemm_pieces(lf_context* ctx, ArenaCursor& cur, const op16* a, const op16* w, op16* out, int batch, int Q, int ldq, int k_len, int width,
                       const float* bias, float qscale);
 // out[dst(b, q)][n_out] (+)= a w^T + bias in float32; a = rows (b, q), or pieces [k / 128][batch][ldq * 128] when a_pieces; dst is row q * batch + b
-// when transposed
-bool gemm_rows_supported(const void* out, int n_out);
+// when transposed; out on a 16-byte boundary, n_out a multiple of 4
 lf_status gemm_rows_f32(lf_context* ctx, ArenaCursor& cur, const op16* a, int a_pieces, const op16* w, float* out, int add, int batch, int Q, int ldq,
                         int transposed, int n_out, int k_len, const float* bias);
 lf_status gemm_rows_half(lf_context* ctx, ArenaCursor& cur, const op16* a_pieces, const op16* w, op16* out, int batch, int Q, int ldq, int n_out, int k_len);
