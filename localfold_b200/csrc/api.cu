@@ -823,32 +823,41 @@ lf_status publish(lf_context* ctx, lf_weights* w, lf_status s, lf_weights** out)
   if (s == LF_OK && (cudaEventCreateWithFlags(&w->ready, cudaEventDisableTiming) != cudaSuccess || cudaEventRecord(w->ready, ctx->stream) != cudaSuccess))
     s = lf_fail(ctx, LF_ERR_CUDA, "weight preparation failed: %s", cudaGetErrorString(cudaGetLastError()));
   if (s != LF_OK) { lf_weights_destroy(w); return s; }
-  w->f32 = new lf_f32_operands();
   *out = w;
   return LF_OK;
 }
 
-// The operands of the float32 GEMM, made at the first call that needs them.
-lf_status f32_operands(lf_context* ctx, const lf_weights* w, const SplitMatrix** g) {
-  lf_f32_operands& o = *w->f32;
-  std::lock_guard<std::mutex> lock(o.mutex);
-  if (!o.made) {
-    WeightCursor dry{nullptr, 0, true};
-    LF_TRY(tc::prepare_f32_operands(ctx, w, dry, o.g));
-    if (!o.block && weight_block_take(w->device, dry.offset, &o.block, &o.block_bytes) != cudaSuccess) {
+// Makes the operands of the float32 GEMM of those of `w` that have none yet (a null entry, or a kind without them, is passed over).
+std::mutex g_f32_mutex;
+lf_status make_f32_operands(lf_context* ctx, const lf_weights* const* w, int count) {
+  std::vector<const lf_weights*> todo;
+  std::lock_guard<std::mutex> lock(g_f32_mutex);
+  for (int i = 0; i < count; ++i) {
+    if (!w[i] || w[i]->f32.made || !w[i]->f32.bytes || std::find(todo.begin(), todo.end(), w[i]) != todo.end()) continue;
+    lf_f32_operands& o = w[i]->f32;
+    if (!o.room && !o.block && weight_block_take(w[i]->device, o.bytes, &o.block, &o.block_bytes) != cudaSuccess) {
       o.block = nullptr;
-      return lf_fail(ctx, LF_ERR_MEMORY, "float32 operands of %zu bytes refused", dry.offset);
+      return lf_fail(ctx, LF_ERR_MEMORY, "float32 operands of %zu bytes refused", o.bytes);
     }
-    WeightCursor cur{static_cast<char*>(o.block), 0, false};
-    LF_TRY(tc::prepare_f32_operands(ctx, w, cur, o.g));
     if (!o.ready) LF_CUDA(ctx, cudaEventCreateWithFlags(&o.ready, cudaEventDisableTiming));
-    LF_CUDA(ctx, cudaEventRecord(o.ready, ctx->stream));
-    o.ctx = ctx;
-    o.made = true;
-  } else if (o.ctx != ctx) {
-    LF_CUDA(ctx, cudaStreamWaitEvent(ctx->stream, o.ready, 0));
+    todo.push_back(w[i]);
   }
-  *g = o.g;
+  if (todo.empty()) return LF_OK;
+  LF_TRY(tc::prepare_f32_operands(ctx, todo.data(), (int)todo.size()));
+  for (const lf_weights* x : todo) {
+    LF_CUDA(ctx, cudaEventRecord(x->f32.ready, ctx->stream));
+    x->f32.ctx = ctx;
+    x->f32.made = true;
+  }
+  return LF_OK;
+}
+
+// The operands of the float32 GEMM, made at the first call that needs them unless the weights came with them.
+lf_status f32_operands(lf_context* ctx, const lf_weights* w, const SplitMatrix** g) {
+  if (!w->f32.bytes) return lf_fail(ctx, LF_ERR_UNSUPPORTED, "weights of kind %d have no float32 GEMM operands", w->kind);
+  LF_TRY(make_f32_operands(ctx, &w, 1));
+  if (w->f32.ready && w->f32.ctx != ctx) LF_CUDA(ctx, cudaStreamWaitEvent(ctx->stream, w->f32.ready, 0));
+  *g = w->f32.g;
   return LF_OK;
 }
 
@@ -935,11 +944,8 @@ void lf_weights_destroy(lf_weights* w) {
     cudaDeviceSynchronize();      // nothing reads the blocks any more, on any stream
     weight_block_give(w->device, w->block, w->block_bytes);
   }
-  if (w->f32) {
-    if (w->f32->ready) cudaEventDestroy(w->f32->ready);
-    if (w->f32->block) weight_block_give(w->device, w->f32->block, w->f32->block_bytes);
-    delete w->f32;
-  }
+  if (w->f32.ready) cudaEventDestroy(w->f32.ready);
+  if (w->f32.block) weight_block_give(w->device, w->f32.block, w->f32.block_bytes);
   delete w;
 }
 
@@ -1940,6 +1946,14 @@ lf_status lf_pair_stack_run_from(lf_context* ctx, const lf_pair_stack_desc* d, c
     if (host && !cur.dry) cudaMemcpyAsync(pair, pair_in ? pair_in : d->pair, P * cz * es, cudaMemcpyHostToDevice, ctx->stream);
     const float* mask = (const float*)st.in(d->mask, P * 4);
     const size_t scratch_base = cur.offset;
+    if (!cur.dry && d->precision == LF_PRECISION_F32) {
+      std::vector<const lf_weights*> used;
+      for (int b = d->first_block; b < d->first_block + d->n_blocks; ++b) {
+        const lf_pair_block_weights& bw = d->blocks[b];
+        used.insert(used.end(), {bw.triangle_outgoing, bw.triangle_incoming, bw.attention_starting, bw.attention_ending, bw.transition});
+      }
+      LF_TRY(make_f32_operands(ctx, used.data(), (int)used.size()));
+    }
     for (int b = d->first_block; b < d->first_block + d->n_blocks; ++b) {
       const lf_pair_block_weights& bw = d->blocks[b];
       auto triangles = [&]() -> lf_status {

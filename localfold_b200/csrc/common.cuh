@@ -99,21 +99,24 @@ struct SplitMatrix {
   int64_t ld = 0, batch_stride = 0, term_stride = 0;
 };
 
-// Operands of the float32 GEMM, [n_out][k] terms: made at the first float32 call that uses the weights, kept with them.
+// Operands of the float32 GEMM, [n_out][k] terms, kept with the weights.  Operators that use them in either mode get them when the
+// weights are prepared, others at the first float32 call (a pair stack's all at once), in room that small ones keep in their own block.
 //   triangle: fused projection, output projection, output gate; attention: fused projection with heads padded to
 //   head_width (and the pair bias columns when the bias comes from the normalised input), output projection, and at
 //   g[2].p the projection's bias (float32); MSA averaging: values | gate, output projection;
 //   transition: both projections; global attention: key | value | gate, output projection
 constexpr int head_width(int d) { return d <= 32 ? (d + 7) / 8 * 8 : d <= 48 ? 48 : 64; }      // the attention core's instances
 struct lf_f32_operands {
-  std::mutex mutex;
-  bool made = false;
-  lf_context* ctx = nullptr;
-  void* block = nullptr;
+  bool made = false;               // with the mutex of f32_operands (api.cu) held
+  lf_context* ctx = nullptr;       // whose stream made them
+  cudaEvent_t ready = nullptr;     // null when they were made with the weights
+  size_t bytes = 0;                // 0: the kind has none
+  char* room = nullptr;            // in the weights' block, or
+  void* block = nullptr;           // a block of their own
   size_t block_bytes = 0;
-  cudaEvent_t ready = nullptr;
   SplitMatrix g[3];
 };
+constexpr size_t kF32RoomLimit = (size_t)1 << 20;      // the operators of a 128-channel pair block: 0.5 to 0.8 MiB each
 
 // Canonical device-resident weights.  Every linear is stored (in,out) row-major
 // float32 in `f[...]`; tensor-core kernels keep extra fp16 repacks (swizzled operand images) in `h[...]`.
@@ -127,7 +130,7 @@ struct lf_weights {
   int device = 0;
   void* block = nullptr;     // the one device allocation behind all of them (weight_block_take)
   size_t block_bytes = 0;
-  lf_f32_operands* f32 = nullptr;
+  mutable lf_f32_operands f32;
   cudaEvent_t ready = nullptr;   // recorded on the creating context's stream when they have been prepared
   bool has_gate_bias = false, has_out_bias = false, has_pair_norm = false, has_pair_proj = false;
 };

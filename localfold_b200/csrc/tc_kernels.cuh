@@ -31,8 +31,8 @@ struct Gemm3Out {
 void configure_gemm3();
 lf_status gemm_f32(lf_context* ctx, ArenaCursor& cur, int major, const SplitMatrix& a, const SplitMatrix& b, int m, int n, int k, int batch,
                    const Gemm3Out& o);
-// The weights' operands of it (lf_f32_operands), out of `cur`.
-lf_status prepare_f32_operands(lf_context* ctx, const lf_weights* w, WeightCursor& cur, SplitMatrix* g);
+// The weights' operands of it (lf_f32_operands), into their room or block; as few launches as the jobs of all of them fit into.
+lf_status prepare_f32_operands(lf_context* ctx, const lf_weights* const* w, int count);
 
 // Triangle contraction, batched over the c channels of channel-major fp16
 // operands a, b [c][n][ld] (ld a multiple of 8, elements past n never read):

@@ -109,11 +109,11 @@ __global__ void __launch_bounds__(256) weight_jobs_kernel(const __grid_constant_
 
 struct Preparer {
   lf_context* ctx;
-  WeightCursor& cur;
+  bool dry;
   JobList list{};
   int64_t most = 0;      // elements of the largest job
   void push(const Job& j) {
-    if (cur.dry) return;
+    if (dry) return;
     list.j[list.count++] = j;
     const int64_t elements = (int64_t)(j.K ? j.K : 1) * j.n_fill;
     if (elements > most) most = elements;
@@ -129,7 +129,7 @@ struct Preparer {
     push(Job{w, offset, bias, out, scale, JOB_FOLD, K, ld, col0, n_out, n_fill ? n_fill : n_out, 0, 0});
   }
   void flush() {
-    if (cur.dry || list.count == 0) return;
+    if (dry || list.count == 0) return;
     // eight elements a thread of the largest job
     const int blocks = most / 2048 < 16 ? 16 : most / 2048 > 592 ? 592 : (int)(most / 2048);
     weight_jobs_kernel<<<dim3(blocks, list.count), 256, 0, ctx->stream>>>(list);
@@ -138,6 +138,74 @@ struct Preparer {
     most = 0;
   }
 };
+
+// The float32 GEMM's operands of w, out of `cur`; false: the kind (or a head width past the attention core's) has none.
+bool f32_jobs(Preparer& prep, const lf_weights* w, WeightCursor& cur, SplitMatrix* g) {
+  const auto& f = w->f;
+  const auto& dims = w->dims;
+  struct Part { const float* w; int ld, col0, n; };
+  auto operand = [&](SplitMatrix& out, int K, std::initializer_list<Part> parts) {
+    const int ld = (K + 7) / 8 * 8;
+    int n = 0, row = 0;
+    for (const Part& q : parts) n += q.n;
+    bf16* p = cur.take<bf16>((size_t)3 * n * ld);
+    out.p = p;
+    out.ld = ld;
+    out.batch_stride = 0;
+    out.term_stride = (int64_t)n * ld;
+    for (const Part& q : parts) {
+      if (q.n) prep.push(Job{q.w, nullptr, nullptr, p, 1.0f, JOB_TERMS, K, q.ld, q.col0, q.n, q.n, ld, row, out.term_stride});
+      row += q.n;
+    }
+  };
+  const int c = dims.channels, HD = dims.heads * dims.head_dim;
+  switch (w->kind) {
+    case LF_WEIGHTS_TRIANGLE_AF2:
+    case LF_WEIGHTS_TRIANGLE_AF3:
+      operand(g[0], c, {{f[TRI_W4], 4 * dims.hidden, 0, 4 * dims.hidden}});
+      operand(g[1], dims.hidden, {{f[TRI_WZ], c, 0, c}});
+      operand(g[2], c, {{f[TRI_WG], c, 0, c}});
+      break;
+    case LF_WEIGHTS_TRANSITION_AF2:
+    case LF_WEIGHTS_TRANSITION_AF3: {
+      const int wide = w->kind == LF_WEIGHTS_TRANSITION_AF3 ? 2 * dims.hidden : dims.hidden;
+      operand(g[0], c, {{f[TRN_W1], wide, 0, wide}});
+      operand(g[1], dims.hidden, {{f[TRN_W2], c, 0, c}});
+      break;
+    }
+    case LF_WEIGHTS_GLOBAL_ATTENTION_AF2: {
+      const int wide = 2 * dims.head_dim + HD;
+      operand(g[0], c, {{f[GLB_W3], wide, 0, wide}});
+      operand(g[1], HD, {{f[GLB_WO], c, 0, c}});
+      break;
+    }
+    case LF_WEIGHTS_MSA_ATTENTION_AF3:
+      operand(g[0], c, {{f[ATT_W4], 4 * HD, 2 * HD, 2 * HD}});
+      operand(g[1], HD, {{f[ATT_WO], c, 0, c}});
+      break;
+    case LF_WEIGHTS_ATTENTION_AF2:
+    case LF_WEIGHTS_GRID_ATTENTION_AF3:
+    case LF_WEIGHTS_SINGLE_ATTENTION_AF3:
+      {
+        if (dims.head_dim > 64) return false;
+        const int d = dims.head_dim, D = head_width(d), wide = 4 * dims.heads * D, own_bias = w->has_pair_proj && !w->has_pair_norm ? dims.heads : 0;
+        const int ld = (c + 7) / 8 * 8;
+        bf16* p = cur.take<bf16>((size_t)3 * (wide + own_bias) * ld);
+        g[0] = SplitMatrix{p, ld, 0, (int64_t)(wide + own_bias) * ld};
+        prep.push(Job{f[ATT_W4], nullptr, nullptr, p, 1.0f, JOB_HEADS, c, 4 * HD, 0, 4 * HD, wide, D, d, g[0].term_stride});
+        if (own_bias) prep.push(Job{f[ATT_WB], nullptr, nullptr, p, 1.0f, JOB_TERMS, c, own_bias, 0, own_bias, own_bias, ld, wide, g[0].term_stride});
+        bf16* po = cur.take<bf16>((size_t)3 * c * dims.heads * D);
+        g[1] = SplitMatrix{po, (int64_t)dims.heads * D, 0, (int64_t)c * dims.heads * D};
+        prep.push(Job{f[ATT_WO], nullptr, nullptr, po, 1.0f, JOB_HEADS_OUT, HD, c, 0, c, dims.heads * D, D, d, g[1].term_stride});
+        float* bias = cur.take<float>(wide);
+        g[2].p = reinterpret_cast<const bf16*>(bias);
+        prep.push(Job{f[ATT_B4], nullptr, nullptr, bias, 1.0f, JOB_HEADS_BIAS, 0, 0, 0, 4 * HD, wide, D, d, 0});
+      }
+      break;
+    default: return false;
+  }
+  return true;
+}
 
 }  // namespace
 
@@ -148,7 +216,7 @@ lf_status prepare_weights(lf_context* ctx, lf_weights* w, WeightCursor& cur) {
   const bool tri = w->kind == LF_WEIGHTS_TRIANGLE_AF2 || w->kind == LF_WEIGHTS_TRIANGLE_AF3;
   const bool att = w->kind == LF_WEIGHTS_ATTENTION_AF2 || w->kind == LF_WEIGHTS_GRID_ATTENTION_AF3;
   const auto& f = w->f;
-  Preparer prep{ctx, cur};
+  Preparer prep{ctx, cur.dry};
   w->h.clear();
   w->g.clear();
   if (tri && w->dims.channels == 128 && w->dims.hidden == 128) {
@@ -247,78 +315,35 @@ lf_status prepare_weights(lf_context* ctx, lf_weights* w, WeightCursor& cur) {
     prep.operand(f[OPM_WOUT], c * c, cz, cz, wout);
     w->g = {wlr, wout};
   }
+  // Operands of the float32 GEMM: now for operators that run on it in 16-bit mode too, later (f32_operands in api.cu) for the others
+  const bool fused = !w->h.empty() && w->h[0], transition = w->kind == LF_WEIGHTS_TRANSITION_AF2 || w->kind == LF_WEIGHTS_TRANSITION_AF3;
+  const bool flash = (fused && w->dims.heads == 4 && w->dims.head_dim == 32) || (!w->g.empty() && (!w->has_pair_norm || pair_bias_supported(w)));
+  const bool always = tri ? !fused : att ? !flash : transition ? !fused && w->g.empty() : true;
+  lf_f32_operands& o = w->f32;
+  Preparer none{ctx, true};
+  WeightCursor size{nullptr, 0, true};
+  o.bytes = f32_jobs(none, w, size, o.g) ? size.offset : 0;
+  if (o.bytes && always) {
+    f32_jobs(prep, w, cur, o.g);
+    o.made = !cur.dry;
+    o.ctx = ctx;
+  } else if (o.bytes && o.bytes <= kF32RoomLimit) {
+    o.room = cur.take<char>(o.bytes);
+  }
   prep.flush();
   if (!cur.dry && cudaGetLastError() != cudaSuccess) return lf_fail(ctx, LF_ERR_CUDA, "weight preparation launch failed");
   return LF_OK;
 }
 
-lf_status prepare_f32_operands(lf_context* ctx, const lf_weights* w, WeightCursor& cur, SplitMatrix* g) {
-  const auto& f = w->f;
-  const auto& dims = w->dims;
-  Preparer prep{ctx, cur};
-  struct Part { const float* w; int ld, col0, n; };
-  auto operand = [&](SplitMatrix& out, int K, std::initializer_list<Part> parts) {
-    const int ld = (K + 7) / 8 * 8;
-    int n = 0, row = 0;
-    for (const Part& q : parts) n += q.n;
-    bf16* p = cur.take<bf16>((size_t)3 * n * ld);
-    out.p = p;
-    out.ld = ld;
-    out.batch_stride = 0;
-    out.term_stride = (int64_t)n * ld;
-    for (const Part& q : parts) {
-      if (q.n) prep.push(Job{q.w, nullptr, nullptr, p, 1.0f, JOB_TERMS, K, q.ld, q.col0, q.n, q.n, ld, row, out.term_stride});
-      row += q.n;
-    }
-  };
-  const int c = dims.channels, HD = dims.heads * dims.head_dim;
-  switch (w->kind) {
-    case LF_WEIGHTS_TRIANGLE_AF2:
-    case LF_WEIGHTS_TRIANGLE_AF3:
-      operand(g[0], c, {{f[TRI_W4], 4 * dims.hidden, 0, 4 * dims.hidden}});
-      operand(g[1], dims.hidden, {{f[TRI_WZ], c, 0, c}});
-      operand(g[2], c, {{f[TRI_WG], c, 0, c}});
-      break;
-    case LF_WEIGHTS_TRANSITION_AF2:
-    case LF_WEIGHTS_TRANSITION_AF3: {
-      const int wide = w->kind == LF_WEIGHTS_TRANSITION_AF3 ? 2 * dims.hidden : dims.hidden;
-      operand(g[0], c, {{f[TRN_W1], wide, 0, wide}});
-      operand(g[1], dims.hidden, {{f[TRN_W2], c, 0, c}});
-      break;
-    }
-    case LF_WEIGHTS_GLOBAL_ATTENTION_AF2: {
-      const int wide = 2 * dims.head_dim + HD;
-      operand(g[0], c, {{f[GLB_W3], wide, 0, wide}});
-      operand(g[1], HD, {{f[GLB_WO], c, 0, c}});
-      break;
-    }
-    case LF_WEIGHTS_MSA_ATTENTION_AF3:
-      operand(g[0], c, {{f[ATT_W4], 4 * HD, 2 * HD, 2 * HD}});
-      operand(g[1], HD, {{f[ATT_WO], c, 0, c}});
-      break;
-    case LF_WEIGHTS_ATTENTION_AF2:
-    case LF_WEIGHTS_GRID_ATTENTION_AF3:
-    case LF_WEIGHTS_SINGLE_ATTENTION_AF3:
-      {
-        const int d = dims.head_dim, D = head_width(d), wide = 4 * dims.heads * D, own_bias = w->has_pair_proj && !w->has_pair_norm ? dims.heads : 0;
-        const int ld = (c + 7) / 8 * 8;
-        bf16* p = cur.take<bf16>((size_t)3 * (wide + own_bias) * ld);
-        g[0] = SplitMatrix{p, ld, 0, (int64_t)(wide + own_bias) * ld};
-        prep.push(Job{f[ATT_W4], nullptr, nullptr, p, 1.0f, JOB_HEADS, c, 4 * HD, 0, 4 * HD, wide, D, d, g[0].term_stride});
-        if (own_bias) prep.push(Job{f[ATT_WB], nullptr, nullptr, p, 1.0f, JOB_TERMS, c, own_bias, 0, own_bias, own_bias, ld, wide, g[0].term_stride});
-        bf16* po = cur.take<bf16>((size_t)3 * c * dims.heads * D);
-        g[1] = SplitMatrix{po, (int64_t)dims.heads * D, 0, (int64_t)c * dims.heads * D};
-        prep.push(Job{f[ATT_WO], nullptr, nullptr, po, 1.0f, JOB_HEADS_OUT, HD, c, 0, c, dims.heads * D, D, d, g[1].term_stride});
-        float* bias = cur.take<float>(wide);
-        g[2].p = reinterpret_cast<const bf16*>(bias);
-        prep.push(Job{f[ATT_B4], nullptr, nullptr, bias, 1.0f, JOB_HEADS_BIAS, 0, 0, 0, 4 * HD, wide, D, d, 0});
-      }
-      break;
-    default: return lf_fail(ctx, LF_ERR_UNSUPPORTED, "weights of kind %d have no float32 GEMM operands", w->kind);
+lf_status prepare_f32_operands(lf_context* ctx, const lf_weights* const* w, int count) {
+  Preparer prep{ctx, false};
+  for (int i = 0; i < count; ++i) {
+    lf_f32_operands& o = w[i]->f32;
+    WeightCursor cur{o.room ? o.room : static_cast<char*>(o.block), 0, false};
+    if (!f32_jobs(prep, w[i], cur, o.g)) return lf_fail(ctx, LF_ERR_UNSUPPORTED, "weights of kind %d have no float32 GEMM operands", w[i]->kind);
   }
   prep.flush();
-  if (!cur.dry && cudaGetLastError() != cudaSuccess) return lf_fail(ctx, LF_ERR_CUDA, "weight preparation launch failed");
-  return LF_OK;
+  return cudaGetLastError() == cudaSuccess ? LF_OK : lf_fail(ctx, LF_ERR_CUDA, "weight preparation launch failed");
 }
 
 }  // namespace tc

@@ -66,3 +66,24 @@ def test_weights_used_from_another_context_at_once(dev):
     for seed in range(4):
         _transition(dev, 64, 384, 1536, 740 + seed, run_dev=other)
     other.close()
+
+
+@pytest.mark.parametrize("n,c,more", [(20, 128, 1), (33, 64, 1)])
+def test_first_float32_call_of_a_pair_stack(dev, n, c, more):
+    """What the float32 mode derives from a stack's weights at its first call is one launch more (at 64 channels the transition's alone: the
+    other operators run in float32 in either mode), also where two blocks share their weights; the results do not change."""
+    import localfold_b200 as lf
+    from localfold_b200.stack import PreparedPairBlock
+    d = syn.draw(750 + n)
+    pair, mask, w = d.normal(n, n, c), syn.residue_pair_mask(n, 0.1), syn.af2_pair_block_weights(d, c, c, 4)
+    options = {"precision": "f32", "variance": "two-pass"}
+    block = PreparedPairBlock(dev, w, c, c)
+    stack = lf.PairStackGpu(dev).prepare([block, block], c, c)
+    first, again = stack.run(pair, mask, options), stack.run(pair, mask, options)
+    assert first["launches"] - again["launches"] == more
+    assert np.array_equal(first["pair"], again["pair"])
+    other = lf.Device(0)
+    elsewhere = lf.PairStackGpu(other).prepare([block, block], c, c)
+    assert np.array_equal(elsewhere.run(pair, mask, options)["pair"], again["pair"])
+    block.close()
+    other.close()
