@@ -52,17 +52,26 @@ typedef enum lf_status {
 typedef enum lf_space { LF_SPACE_HOST = 0, LF_SPACE_DEVICE = 1 } lf_space;
 typedef enum lf_dtype { LF_DTYPE_F32 = 0, LF_DTYPE_BF16 = 1 } lf_dtype;
 
-/* Arithmetic mode.  F32: float32 storage and float32 FMA accumulation
- * (the reference's `precision: "f32"`).  BF16 names the 16-bit tensor-core
+/* Arithmetic mode.  F32: float32 storage and float32 accumulation (the
+ * reference's `precision: "f32"`), products on the tensor cores with every
+ * operand as three bf16 terms.  BF16 names the 16-bit tensor-core
  * mode: its tensor-core operands are fp16 (11-bit significand; every rounded
  * operand is bounded by construction), products accumulate in float32, and
- * LayerNorm statistics, softmax and gates are float32.  It stands where the
+ * LayerNorm statistics, softmax and gates are float32.  Outside 128 channels
+ * and heads of 32 in groups of four it rounds less: of a triangle update only
+ * the contraction's operands and product, of an attention only a separate
+ * pair bias.  It stands where the
  * reference has `precision: "f16"`; the enumerator keeps its name because the
  * pair stream this mode is usually paired with is bf16 or float32 (lf_dtype). */
 typedef enum lf_precision { LF_PRECISION_F32 = 0, LF_PRECISION_BF16 = 1 } lf_precision;
 
 /* LayerNorm variance: the reference's `variance: "two-pass" | "fast"`
- * (webgpu/kernels/triangle/shaders.js:43-58). No default: 0 is rejected. */
+ * (webgpu/kernels/triangle/shaders.js:43-58). No default: 0 is rejected.
+ * FAST permits E[x^2] - E[x]^2, it does not promise it.  Two LayerNorms of the
+ * fused 128-channel kernels (16-bit mode) use one formula whatever is passed:
+ * the projections' input norm merges partial variances pairwise, as accurate as
+ * two passes, and the triangle output's centre norm takes E[x^2] - E[x]^2 of its
+ * fp16 input (clamped at 0 for TWO_PASS).  Every other LayerNorm follows it. */
 typedef enum lf_variance { LF_VARIANCE_TWO_PASS = 1, LF_VARIANCE_FAST = 2 } lf_variance;
 
 typedef struct lf_context lf_context;
@@ -115,8 +124,8 @@ LF_API const char* lf_version(void);
  * lf_context_profile_read synchronises, then returns and clears the device
  * time and launch count accumulated for one kernel family. */
 typedef enum lf_kernel_family {
-  LF_KERNEL_SIMT = 0,              /* float32 SIMT kernels (all of them)        */
-  LF_KERNEL_TRIANGLE_CONTRACT = 1, /* tcgen05 triangle contraction              */
+  LF_KERNEL_SIMT = 0,              /* float32 GEMMs and attention core, row kernels, glue: all that has no family below */
+  LF_KERNEL_TRIANGLE_CONTRACT = 1, /* tcgen05 triangle contraction, fp16 GEMMs  */
   LF_KERNEL_LN_GEMM = 2,           /* tcgen05 LayerNorm + projection kernels    */
   LF_KERNEL_TRIANGLE_OUTPUT = 3,   /* tcgen05 centre-norm + output projection   */
   LF_KERNEL_ATTENTION = 4,         /* tcgen05 attention core                    */
