@@ -1,6 +1,6 @@
 // C ABI of the pair-stack library: context, weights, operators.
-// The float32 path composes the SIMT kernels of simt_kernels.cuh; the bf16 path
-// routes the shapes they cover to the tcgen05 kernels declared in tc_kernels.cuh.
+// 16-bit mode routes what they cover to the fused tcgen05 kernels declared in tc_kernels.cuh; everything else composes the GEMMs
+// of tc_gemm.cu (fp16) and f32_gemm.cu, the attention core of mma_attention.cuh and the kernels of row_kernels.cuh and simt_kernels.cuh.
 #include <cuda_fp16.h>
 #include <sys/mman.h>
 #include <unistd.h>
@@ -968,19 +968,12 @@ namespace {
     }                                                                        \
   } while (0)
 
-void sgemm(lf_context* ctx, ArenaCursor& cur, bool ta, bool tb, int epi, int M, int N, int K, const float* A,
-           int64_t lda, int64_t sA, const float* B, int64_t ldb, int64_t sB, float* C, int64_t ldc, int64_t sC,
-           const float* bias, int epi_col0, int batch) {
-  dim3 grid(lf_ceil_div(M, 64), lf_ceil_div(N, 64), batch), block(256);
-#define SG(TA_, TB_, E_) LAUNCH(ctx, cur, (simt::sgemm_kernel<TA_, TB_, E_>), grid, block, 0, M, N, K, A, lda, sA, B, ldb, sB, C, ldc, sC, bias, epi_col0)
-  if (!ta && !tb) {
-    if (epi == simt::EPI_NONE) SG(false, false, simt::EPI_NONE);
-    else if (epi == simt::EPI_RELU) SG(false, false, simt::EPI_RELU);
-    else SG(false, false, simt::EPI_SIGMOID_FROM_COL);
-  } else if (!ta && tb) SG(false, true, simt::EPI_NONE);
-  else if (ta && !tb) SG(true, false, simt::EPI_NONE);
-  else SG(true, true, simt::EPI_NONE);
-#undef SG
+// C[m][n] = sum_k A(m, k) B[k][n] + bias[n] on the FMA pipe; A is [K][lda] when `ta`
+void sgemm(lf_context* ctx, ArenaCursor& cur, bool ta, int M, int N, int K, const float* A, int64_t lda, const float* B, int64_t ldb, float* C, int64_t ldc,
+           const float* bias) {
+  const dim3 grid(lf_ceil_div(M, 64), lf_ceil_div(N, 64));
+  if (ta) LAUNCH(ctx, cur, simt::sgemm_kernel<true>, grid, 256, 0, M, N, K, A, lda, B, ldb, C, ldc, bias);
+  else LAUNCH(ctx, cur, simt::sgemm_kernel<false>, grid, 256, 0, M, N, K, A, lda, B, ldb, C, ldc, bias);
 }
 
 // The float32 attention core for any head width: terms of q | k | v | gate -> the gated output likewise.
@@ -1113,7 +1106,7 @@ struct Staging {
 size_t dtype_size(int dt) { return dt == LF_DTYPE_BF16 ? 2 : 4; }
 
 // 16-bit GEMM on the tensor cores for activations of any width: out[m][n] = sum_k a[m][k] w[n][k], fp16 operands
-// with k contiguous, float32 accumulation, fp16 result (the triangle contraction's kernel on one plane).
+// with k contiguous, float32 accumulation, fp16 result (gemm_kernel on fp16 rows).
 lf_status hgemm(lf_context* ctx, ArenaCursor& cur, const op16* a, const op16* w, op16* out, int64_t M, int N, int K,
                 const float* bias = nullptr, int relu = 0) {
   if (M > 0x7fffffff) return lf_fail(ctx, LF_ERR_SHAPE, "too many rows for one projection");
@@ -1235,7 +1228,7 @@ lf_status tri_dispatch(lf_context* ctx, ArenaCursor& cur, const TriArgs& a, int 
   return a.act_dtype == LF_DTYPE_BF16 ? tri_general<bf16>(ctx, cur, a, planes) : tri_general<float>(ctx, cur, a, planes);
 }
 
-// ---- attention engine, float32 path ----
+// ---- attention ----
 struct AttArgs {
   int batch, Q, ch, heads, d, transpose, variance, residual;
   int bias_mode;       // 0 none, 1 from a separate pair tensor, 2 from the normalised input
@@ -1264,10 +1257,10 @@ lf_status separate_bias(lf_context* ctx, ArenaCursor& cur, const AttArgs& a, flo
     LAUNCH(ctx, cur, simt::widen_bias_kernel, lf_ceil_div(QQ * a.heads, 256), 256, 0, b16, a.heads, a.Q, ldb, bias);
   } else if (a.pair_dtype == LF_DTYPE_BF16)
     LAUNCH(ctx, cur, (simt::pair_bias_kernel<bf16>), lf_ceil_div(QQ, 8), 256, 0, (const bf16*)a.pair, a.Q, a.pair_ch, a.heads, f[ATT_PLN_G], f[ATT_PLN_B],
-           f[ATT_WB], a.pair_eps, a.pair_variance, 0, a.bias_swap, bias);
+           f[ATT_WB], a.pair_eps, a.pair_variance, a.bias_swap, bias);
   else
     LAUNCH(ctx, cur, (simt::pair_bias_kernel<float>), lf_ceil_div(QQ, 8), 256, 0, (const float*)a.pair, a.Q, a.pair_ch, a.heads, f[ATT_PLN_G], f[ATT_PLN_B],
-           f[ATT_WB], a.pair_eps, a.pair_variance, 0, a.bias_swap, bias);
+           f[ATT_WB], a.pair_eps, a.pair_variance, a.bias_swap, bias);
   return LF_OK;
 }
 
@@ -1349,11 +1342,9 @@ void pad_attention(lf_context* ctx, ArenaCursor& cur, op16* k, op16* v, op16* bi
   LAUNCH(ctx, cur, rows::attention_padding_kernel, lf_ceil_div(rows * (ldq - Q), 256), 256, 0, (uint16_t*)k, (uint16_t*)v, (uint16_t*)bias, batch, heads, Q, ldq);
 }
 
-// 16-bit path: tensor-core LayerNorm + q/k/v/gate/bias projection, then the attention core.
-template <typename T>
+// 16-bit path at 128 channels, 4 heads of 32: tensor-core LayerNorm + q/k/v/gate/bias projection, then the attention core.
 lf_status att_bf16(lf_context* ctx, ArenaCursor& cur, const AttArgs& a) {
-  const int HD = a.heads * a.d, c = a.ch;
-  const auto& f = a.w->f;
+  const int HD = a.heads * a.d;
   const int ldb = (a.Q + 15) / 16 * 16;        // rows and keys padded to whole groups of 16
   const int64_t RP = (int64_t)a.batch * ldb;   // q, k, v, gate and o are stored in 8 x 8 pieces: rows padded per batch row
   op16* q = cur.take<op16>(RP * HD);
@@ -1367,7 +1358,6 @@ lf_status att_bf16(lf_context* ctx, ArenaCursor& cur, const AttArgs& a) {
                                a.bias_swap, a.w, q, k, v, g, bias, ldb));
   LF_TRY(tc::attention_core(ctx, cur, q, k, v, g, bias, ldb, a.mask, a.batch, a.Q, a.transpose, a.mask_mode, a.clamp, o16));
   LF_TRY(tc::attention_output(ctx, cur, o16, a.batch, a.Q, a.transpose, a.w, a.residual ? a.act : nullptr, a.out, a.act_dtype));
-  (void)f; (void)c;
   return LF_OK;
 }
 
@@ -1417,7 +1407,7 @@ lf_status att_dispatch(lf_context* ctx, ArenaCursor& cur, const AttArgs& a, int 
   const void* resid = a.residual ? a.act : nullptr;
   if (precision == LF_PRECISION_BF16 && a.bias_mode != 1 && a.heads == 4 && a.d == 32 && tc::ln_gemm_supported(a.w) &&
       lf_fused_takes(a.act, resid, a.out, a.act_dtype)) {
-    return a.act_dtype == LF_DTYPE_BF16 ? att_bf16<bf16>(ctx, cur, a) : att_bf16<float>(ctx, cur, a);
+    return att_bf16(ctx, cur, a);
   }
   if (precision == LF_PRECISION_BF16 && a.d == 32 && a.heads % 4 == 0 && hgemm_supported(a.w) &&
       half_rows_take(resid, a.out, a.act_dtype) && (a.bias_mode == 0 || (a.bias_mode == 1 && tensor_core_bias(a)))) {
@@ -1690,7 +1680,7 @@ lf_status lf_outer_product_mean_run(lf_context* ctx, const lf_opm_desc* d, lf_re
     float* left = tc_full ? nullptr : cur.take<float>(rows * c);
     float* right = tc_full ? nullptr : cur.take<float>(rows * c);
     // 16-bit mode: the outer product sum over the sequences, [(i,a)] x [(j,b)] over s, is one tensor-core GEMM
-    // (the triangle contraction's kernel in its MN-major form, one plane) with fp16 operands and fp16 sums scaled
+    // with both operands MN-major, with fp16 operands and fp16 sums scaled
     // by a power of two near 1 / S so that they stay far inside fp16 whatever the depth
     const bool tc_outer = d->precision == LF_PRECISION_BF16 && ((int64_t)N * c) % 8 == 0 && tc::contract_supported(N, 1);
     const float outer_scale = tc_outer ? ldexpf(1.0f, -(int)ceilf(log2f((float)S))) : 1.0f;
@@ -1733,8 +1723,8 @@ lf_status lf_outer_product_mean_run(lf_context* ctx, const lf_opm_desc* d, lf_re
       return LF_OK;
     }
     layer_norm<float, rows::LN_F32>(ctx, cur, msa, rows, cm, f[OPM_LN_G], f[OPM_LN_B], d->layer_norm_epsilon, d->variance, 0, 1, 1, nrm);
-    sgemm(ctx, cur, false, false, 0, (int)rows, c, cm, nrm, cm, 0, f[OPM_WL], c, 0, left, c, 0, f[OPM_BL], 0, 1);
-    sgemm(ctx, cur, false, false, 0, (int)rows, c, cm, nrm, cm, 0, f[OPM_WR], c, 0, right, c, 0, f[OPM_BR], 0, 1);
+    sgemm(ctx, cur, false, (int)rows, c, cm, nrm, cm, f[OPM_WL], c, left, c, f[OPM_BL]);
+    sgemm(ctx, cur, false, (int)rows, c, cm, nrm, cm, f[OPM_WR], c, right, c, f[OPM_BR]);
     if (tc_outer) LAUNCH(ctx, cur, simt::mask_rows_half_kernel, lf_ceil_div(rows * c, 256), 256, 0, left, right, mask, rows, c, left16, right16);
     else LAUNCH(ctx, cur, simt::mask_rows_kernel, lf_ceil_div(rows * c, 256), 256, 0, left, right, mask, rows, c);
     constexpr int JT = 8;
@@ -1756,8 +1746,7 @@ lf_status lf_outer_product_mean_run(lf_context* ctx, const lf_opm_desc* d, lf_re
                  mask, S, N, c, cz, i0, d->normalization_epsilon, ban, (const float*)resid, (float*)out);
         continue;
       }
-      sgemm(ctx, cur, true, false, 0, cnt * c, N * c, S, left + (int64_t)i0 * c, (int64_t)N * c, 0, right, (int64_t)N * c, 0,
-            outer, (int64_t)N * c, 0, nullptr, 0, 1);
+      sgemm(ctx, cur, true, cnt * c, N * c, S, left + (int64_t)i0 * c, (int64_t)N * c, right, (int64_t)N * c, outer, (int64_t)N * c, nullptr);
       if (d->act_dtype == LF_DTYPE_BF16)
         LAUNCH(ctx, cur, (simt::opm_output_kernel<bf16, JT, float>), grid, 128, smem, outer, 1.0f, f[OPM_WOUT], f[OPM_BOUT], mask, S, N, c, cz,
                i0, d->normalization_epsilon, ban, (const bf16*)resid, (bf16*)out);
@@ -1917,7 +1906,7 @@ lf_status lf_distogram_logits_run(lf_context* ctx, const lf_distogram_desc* d, l
     float* out = (float*)st.out(d->out, P * bins * 4);
     const float* x = (const float*)pair;
     float* half = cur.take<float>(P * bins);
-    sgemm(ctx, cur, false, false, 0, (int)P, bins, c, x, c, 0, w, bins, 0, half, bins, 0, bias, 0, 1);
+    sgemm(ctx, cur, false, (int)P, bins, c, x, c, w, bins, half, bins, bias);
     LAUNCH(ctx, cur, simt::symmetrise_sum_kernel, lf_ceil_div((int64_t)P * bins, 256), 256, 0, half, n, bins, out);
     st.flush();
     return LF_OK;

@@ -33,7 +33,6 @@ struct lf_context {
   // Scratch arena: one device allocation, bump-allocated per operator call.
   char* arena = nullptr;
   size_t arena_bytes = 0;
-  size_t arena_used = 0;
   size_t arena_peak = 0;
   size_t arena_limit = 0;      // 0 = none; otherwise requests above it are refused without asking the driver (lf_context_limit_scratch)
   uint64_t launches = 0;

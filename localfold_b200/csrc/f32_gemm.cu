@@ -24,7 +24,6 @@ constexpr int G3_STAGE = 6 * G3_PLANE;
 constexpr int G3_OUT = 2048;                           // per epilogue warp: 32 rows x 64 bytes
 constexpr int G3_SMEM = G3_STAGES * G3_STAGE + G3_EPI * G3_OUT + 256 + 1024;
 constexpr int G3_THREADS = 64 + 32 * G3_EPI;
-constexpr int G3_CHUNK = 1;                            // k blocks per accumulation in TMEM
 
 struct Gemm3Params {
   int m, n, k, batch;
@@ -109,12 +108,8 @@ gemm3_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant__ C
       for (int64_t t = blockIdx.x; t < total && ok; t += gridDim.x) {
         for (int kb = 0; kb < kblocks; ++kb) {
           const uint32_t d = tmem_base + (it & 1) * 256;
-          const int kc = kb % G3_CHUNK;
-          if (kc == 0) {
-            if (!mbar_wait(&tmem_empty[it & 1], ((it >> 1) & 1) ^ 1, abort_flag, p.status, 102)) { ok = false; break; }
-            tc_fence_after();
-          }
-          if (!mbar_wait(&full[stage], phase, abort_flag, p.status, 103)) { ok = false; break; }
+          if (!mbar_wait(&tmem_empty[it & 1], ((it >> 1) & 1) ^ 1, abort_flag, p.status, 102) ||
+              !mbar_wait(&full[stage], phase, abort_flag, p.status, 103)) { ok = false; break; }
           tc_fence_after();
           const uint32_t a0 = smem_u32(smem + stage * G3_STAGE), b0 = a0 + 3 * G3_PLANE;
 #pragma unroll
@@ -124,7 +119,7 @@ gemm3_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant__ C
               return MAJOR == 0 ? make_smem_desc(base + term * G3_PLANE + kk * 32, 16, 1024)
                                 : make_smem_desc(base + term * (G3_PLANE / 2) + kk * 2048, 3 * (G3_PLANE / 2), 1024);
             };
-            const uint32_t more = (kc | kk) != 0 ? 1u : 0u;
+            const uint32_t more = kk != 0 ? 1u : 0u;
             umma_f16(d + 128, desc(a0, 2), desc(b0, 0), idesc, more);
             umma_f16(d + 128, desc(a0, 1), desc(b0, 1), idesc, 1u);
             umma_f16(d + 128, desc(a0, 0), desc(b0, 2), idesc, 1u);
@@ -134,14 +129,14 @@ gemm3_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant__ C
           }
           umma_commit(&empty[stage]);
           if (++stage == G3_STAGES) { stage = 0; phase ^= 1; }
-          if (kc == G3_CHUNK - 1 || kb == kblocks - 1) { umma_commit(&tmem_full[it & 1]); ++it; }
+          umma_commit(&tmem_full[it & 1]);
+          ++it;
         }
       }
     }
   } else {
     const int q = warp & 3, part = (warp - 2) >> 2;      // TMEM lane quadrant, 32 of the tile's columns
     uint8_t* stage = out_stage + (warp - 2) * G3_OUT;
-    const int chunks = (kblocks + G3_CHUNK - 1) / G3_CHUNK;
     uint32_t it = 0;
     bool ok = true;
     for (int64_t t = blockIdx.x; t < total && ok; t += gridDim.x) {
@@ -149,7 +144,7 @@ gemm3_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant__ C
       const int col0 = nj * G3_BN + part * 32;
       float v[32];
 #pragma unroll 1
-      for (int c = 0; c < chunks; ++c, ++it) {
+      for (int kb = 0; kb < kblocks; ++kb, ++it) {
         if (!mbar_wait(&tmem_full[it & 1], (it >> 1) & 1, abort_flag, p.status, 104)) { ok = false; break; }
         tc_fence_after();
         const uint32_t d = tmem_base + ((uint32_t)(q * 32) << 16) + (it & 1) * 256 + part * 32;
@@ -162,7 +157,7 @@ gemm3_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant__ C
 #pragma unroll
           for (int e = 0; e < 16; ++e) {
             const float x = __uint_as_float(lead[e]) + __uint_as_float(rest[e]);
-            v[c16 * 16 + e] = c ? v[c16 * 16 + e] + x : x;
+            v[c16 * 16 + e] = kb ? v[c16 * 16 + e] + x : x;
           }
         }
         tc_fence_before();

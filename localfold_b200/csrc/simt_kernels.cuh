@@ -1,6 +1,6 @@
-// Float32 SIMT kernels: the precision-"f32" path of every operator and the
-// generic-shape path behind the tensor-core kernels.  All accumulation is
-// float32 FMA; statistics use warp-shuffle reductions.
+// Kernels on the FMA pipe: LayerNorm, residuals and pair bias for widths and addresses that the vectorised row kernels do not take,
+// the float32 outer product mean, the distogram's GEMM, int5 decode, and glue of the fp16 GEMMs.  Accumulation in float32,
+// statistics by warp shuffles.
 #pragma once
 
 #include "common.cuh"
@@ -87,24 +87,16 @@ __global__ void layer_norm_kernel(const TIn* __restrict__ in, int64_t rows, int 
 }
 
 // ---------------------------------------------------------------------------
-// Tiled SGEMM, batched over blockIdx.z:  C[m][n] = epi(sum_k A(m,k) B(k,n) + bias[n])
-//   A(m,k) = TA ? A[k*lda + m] : A[m*lda + k]
-//   B(k,n) = TB ? B[n*ldb + k] : B[k*ldb + n]
+// Tiled SGEMM:  C[m][n] = sum_k A(m,k) B[k*ldb + n] + bias[n],  A(m,k) = TA ? A[k*lda + m] : A[m*lda + k]
 // 64x64x16 tile, 256 threads, 4x4 micro-tile, every load and store bounds-checked.
-enum { EPI_NONE = 0, EPI_RELU = 1, EPI_SIGMOID_FROM_COL = 2 };
-
-template <bool TA, bool TB, int EPI>
+template <bool TA>
 __global__ void __launch_bounds__(256)
-sgemm_kernel(int M, int N, int K, const float* __restrict__ A, int64_t lda, int64_t strideA,
-             const float* __restrict__ B, int64_t ldb, int64_t strideB, float* __restrict__ C,
-             int64_t ldc, int64_t strideC, const float* __restrict__ bias, int epi_col0) {
+sgemm_kernel(int M, int N, int K, const float* __restrict__ A, int64_t lda, const float* __restrict__ B, int64_t ldb, float* __restrict__ C,
+             int64_t ldc, const float* __restrict__ bias) {
   lf_chain();
   constexpr int BM = 64, BN = 64, BK = 16;
   __shared__ float As[BK][BM + 4];
   __shared__ float Bs[BK][BN + 4];
-  A += (int64_t)blockIdx.z * strideA;
-  B += (int64_t)blockIdx.z * strideB;
-  C += (int64_t)blockIdx.z * strideC;
   const int m0 = blockIdx.x * BM, n0 = blockIdx.y * BN;
   const int t = threadIdx.x;
   const int tx = t & 15, ty = t >> 4;
@@ -128,12 +120,9 @@ sgemm_kernel(int M, int N, int K, const float* __restrict__ A, int64_t lda, int6
 #pragma unroll
     for (int r = 0; r < 4; ++r) {
       int idx = t + 256 * r;
-      int n, k;
-      if (TB) { k = idx & 15; n = idx >> 4; } else { n = idx & 63; k = idx >> 6; }
+      int n = idx & 63, k = idx >> 6;
       int gn = n0 + n, gk = k0 + k;
-      float v = 0.f;
-      if (gn < N && gk < K) v = TB ? B[(int64_t)gn * ldb + gk] : B[(int64_t)gk * ldb + gn];
-      Bs[k][n] = v;
+      Bs[k][n] = gn < N && gk < K ? B[(int64_t)gk * ldb + gn] : 0.f;
     }
     __syncthreads();
 #pragma unroll
@@ -157,11 +146,7 @@ sgemm_kernel(int M, int N, int K, const float* __restrict__ A, int64_t lda, int6
 #pragma unroll
     for (int j = 0; j < 4; ++j) {
       int gn = n0 + tx * 4 + j;
-      if (gn >= N) continue;
-      float v = acc[i][j] + (bias ? bias[gn] : 0.f);
-      if (EPI == EPI_RELU) v = fmaxf(v, 0.f);
-      if (EPI == EPI_SIGMOID_FROM_COL) { if (gn >= epi_col0) v = sigmoidf_(v); }
-      C[(int64_t)gm * ldc + gn] = v;
+      if (gn < N) C[(int64_t)gm * ldc + gn] = acc[i][j] + (bias ? bias[gn] : 0.f);
     }
   }
 }
@@ -189,49 +174,44 @@ __global__ void finish_kernel(const float* __restrict__ proj, const float* __res
 
 // ---------------------------------------------------------------------------
 // Pair bias: out[h][dst(p)] = LN(pair[p,:]) . W[:,h] for p = i*Q + j, dst = j*Q+i if swap.
-// One warp per pair row; `normalized` != 0 skips the LayerNorm (input already normalised).
+// One warp per pair row.
 template <typename TIn>
 __global__ void pair_bias_kernel(const TIn* __restrict__ pair, int Q, int ch, int heads,
                                  const float* __restrict__ gamma, const float* __restrict__ beta,
-                                 const float* __restrict__ w, float eps, int variance, int normalized,
-                                 int swap, float* __restrict__ out) {
+                                 const float* __restrict__ w, float eps, int variance, int swap,
+                                 float* __restrict__ out) {
   lf_chain();
   int lane = threadIdx.x & 31;
   int64_t pairs = (int64_t)Q * Q;
   int64_t p = (int64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
   if (p >= pairs) return;
   const TIn* x = pair + p * ch;
-  float mean = 0.f, inv = 1.f;
-  if (!normalized) {
-    float s = 0.f, ss = 0.f;
-    for (int c = lane; c < ch; c += 32) { float v = to_f(x[c]); s += v; ss += v * v; }
-    s = warp_sum(s);
-    mean = s / ch;
-    float var;
-    if (variance == 2) { ss = warp_sum(ss); var = ss / ch - mean * mean; }
-    else {
-      float acc = 0.f;
-      for (int c = lane; c < ch; c += 32) { float d = to_f(x[c]) - mean; acc += d * d; }
-      var = warp_sum(acc) / ch;
-    }
-    inv = rsqrtf(var + eps);
-    inv = inv * (1.5f - 0.5f * (var + eps) * inv * inv);
+  float s = 0.f, ss = 0.f;
+  for (int c = lane; c < ch; c += 32) { float v = to_f(x[c]); s += v; ss += v * v; }
+  s = warp_sum(s);
+  const float mean = s / ch;
+  float var;
+  if (variance == 2) { ss = warp_sum(ss); var = ss / ch - mean * mean; }
+  else {
+    float acc = 0.f;
+    for (int c = lane; c < ch; c += 32) { float d = to_f(x[c]) - mean; acc += d * d; }
+    var = warp_sum(acc) / ch;
   }
+  float inv = rsqrtf(var + eps);
+  inv = inv * (1.5f - 0.5f * (var + eps) * inv * inv);
   int64_t dst = p;
   if (swap) { int64_t i = p / Q, j = p % Q; dst = j * Q + i; }
   for (int h = 0; h < heads; ++h) {
     float acc = 0.f;
     for (int c = lane; c < ch; c += 32) {
-      float v = to_f(x[c]);
-      if (!normalized) v = (v - mean) * inv * gamma[c] + beta[c];
-      acc = fmaf(v, w[c * heads + h], acc);
+      acc = fmaf((to_f(x[c]) - mean) * inv * gamma[c] + beta[c], w[c * heads + h], acc);
     }
     acc = warp_sum(acc);
     if (lane == 0) out[(int64_t)h * pairs + dst] = acc;
   }
 }
 
-// Glue of the 16-bit GEMM path (activations x weights on the tensor cores through the contraction kernel).
+// Glue of the 16-bit GEMM path.
 // out[dst(r)][c] = (resid ? resid[dst(r)][c] : 0) + (proj[r][c] * scale + bias[c]) for an fp16 projection;
 // eight channels per thread (ch a multiple of 8)
 template <typename TAct>
@@ -281,8 +261,7 @@ __global__ void symmetrise_sum_kernel(const float* __restrict__ half, int tokens
 
 // ---------------------------------------------------------------------------
 // Outer product mean glue.
-// rows [S*N][c]: multiply every row by its mask value.
-// the same into fp16 copies (operands of the tensor-core outer product)
+// rows [S*N][c] times their mask values, into fp16 copies (operands of the tensor-core outer product)
 __global__ void mask_rows_half_kernel(const float* __restrict__ a, const float* __restrict__ b, const float* __restrict__ mask,
                                       int64_t rows, int c, __half* __restrict__ a16, __half* __restrict__ b16) {
   lf_chain();
@@ -334,6 +313,7 @@ __global__ void opm_finish_half_kernel(const __half* __restrict__ proj, float sc
   add_store8<TAct>(v, resid ? resid + o : nullptr, out + o);
 }
 
+// ... in place
 __global__ void mask_rows_kernel(float* __restrict__ a, float* __restrict__ b, const float* __restrict__ mask,
                                  int64_t rows, int c) {
   lf_chain();

@@ -540,8 +540,8 @@ void configure_attention() {
   cudaGetLastError();
 }
 
-lf_status make_map_f16_3d_ext(lf_context* ctx, CUtensorMap* map, const void* base, uint64_t d0, uint64_t d1, uint64_t d2,
-                              uint64_t stride1_bytes, uint64_t stride2_bytes, uint32_t b0, uint32_t b1);
+lf_status make_map_f16_3d(lf_context* ctx, CUtensorMap* map, const void* base, uint64_t d0, uint64_t d1, uint64_t d2,
+                          uint64_t stride1_bytes, uint64_t stride2_bytes, uint32_t b0, uint32_t b1, uint32_t b2 = 1);
 lf_status make_map_tiled_act(lf_context* ctx, CUtensorMap* map, const void* base, int ldq, int batch, int rows);
 
 lf_status attention_core(lf_context* ctx, ArenaCursor& cur, const op16* q, const op16* k, const op16* v, const op16* g,
@@ -554,7 +554,7 @@ lf_status attention_core(lf_context* ctx, ArenaCursor& cur, const op16* q, const
   LF_TRY(make_map_tiled_act(ctx, &mk, k, ldq, batch, FA_KT));
   LF_TRY(make_map_tiled_act(ctx, &mv, v, ldq, batch, FA_KT));
   // bias [4][Q][ldb]: boxes of 64 keys x 128 queries; without a bias the map is a stand-in that is never used
-  if (bias) LF_TRY(make_map_f16_3d_ext(ctx, &mb, bias, ldb, Q, 4, (uint64_t)ldb * 2, (uint64_t)Q * ldb * 2, 64, FA_TILE));
+  if (bias) LF_TRY(make_map_f16_3d(ctx, &mb, bias, ldb, Q, 4, (uint64_t)ldb * 2, (uint64_t)Q * ldb * 2, 64, FA_TILE));
   else mb = mq;
   FlashParams p{};
   p.batch = batch; p.Q = Q; p.qtiles = (Q + FA_TILE - 1) / FA_TILE; p.ktiles = (Q + FA_KT - 1) / FA_KT;

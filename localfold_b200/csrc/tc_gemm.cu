@@ -280,8 +280,8 @@ void configure_gemm() {
   cudaFuncSetAttribute(gemm_kernel<1, GM_GROUPED>, cudaFuncAttributeMaxDynamicSharedMemorySize, GM_SMEM);
 }
 
-lf_status make_map_f16_3d_ext(lf_context* ctx, CUtensorMap* map, const void* base, uint64_t d0, uint64_t d1, uint64_t d2,
-                              uint64_t stride1_bytes, uint64_t stride2_bytes, uint32_t b0, uint32_t b1);
+lf_status make_map_f16_3d(lf_context* ctx, CUtensorMap* map, const void* base, uint64_t d0, uint64_t d1, uint64_t d2,
+                          uint64_t stride1_bytes, uint64_t stride2_bytes, uint32_t b0, uint32_t b1, uint32_t b2 = 1);
 lf_status make_map_tiled_act(lf_context* ctx, CUtensorMap* map, const void* base, int ldq, int batch, int rows);
 lf_status make_map_f32_any(lf_context* ctx, CUtensorMap* map, const void* base, const uint64_t (&dims)[3], const uint64_t (&strides)[2], const uint32_t (&box)[3]);
 lf_status make_map_grouped(lf_context* ctx, CUtensorMap* map, const void* base, uint64_t n, uint64_t cnt);
@@ -304,9 +304,9 @@ lf_status contract_gemm(lf_context* ctx, ArenaCursor& cur, const op16* a, const 
   if (cur.dry) return LF_OK;
   if (k_len % 8 || n_out % 8) return lf_fail(ctx, LF_ERR_ARGUMENT, "GEMM rows must be whole groups of eight");
   CUtensorMap ma, mb, mo;
-  LF_TRY(make_map_f16_3d_ext(ctx, &ma, a, k_len, m_rows, 1, (uint64_t)k_len * 2, (uint64_t)m_rows * k_len * 2, GM_BK, GM_BM));
-  LF_TRY(make_map_f16_3d_ext(ctx, &mb, w, k_len, n_out, 1, (uint64_t)k_len * 2, (uint64_t)n_out * k_len * 2, GM_BK, GM_BN));
-  LF_TRY(make_map_f16_3d_ext(ctx, &mo, out, n_out, m_rows, 1, (uint64_t)n_out * 2, (uint64_t)m_rows * n_out * 2, 64, 32));
+  LF_TRY(make_map_f16_3d(ctx, &ma, a, k_len, m_rows, 1, (uint64_t)k_len * 2, (uint64_t)m_rows * k_len * 2, GM_BK, GM_BM));
+  LF_TRY(make_map_f16_3d(ctx, &mb, w, k_len, n_out, 1, (uint64_t)k_len * 2, (uint64_t)n_out * k_len * 2, GM_BK, GM_BN));
+  LF_TRY(make_map_f16_3d(ctx, &mo, out, n_out, m_rows, 1, (uint64_t)n_out * 2, (uint64_t)m_rows * n_out * 2, 64, 32));
   GemmParams p{};
   p.m = m_rows; p.n = n_out; p.k = k_len; p.batch = 1; p.scale = 1.0f; p.bias = bias; p.relu = relu;
   return launch<0, GM_HALF>(ctx, LF_KERNEL_TRIANGLE_CONTRACT, ma, mb, mo, p);
@@ -316,8 +316,8 @@ lf_status gemm_pieces(lf_context* ctx, ArenaCursor& cur, const op16* a, const op
                       const float* bias, float qscale) {
   if (cur.dry) return LF_OK;
   CUtensorMap ma, mb, mo;
-  LF_TRY(make_map_f16_3d_ext(ctx, &ma, a, k_len, Q, batch, (uint64_t)k_len * 2, (uint64_t)Q * k_len * 2, GM_BK, GM_BM));
-  LF_TRY(make_map_f16_3d_ext(ctx, &mb, w, k_len, 4 * width, 1, (uint64_t)k_len * 2, (uint64_t)4 * width * k_len * 2, GM_BK, GM_BN));
+  LF_TRY(make_map_f16_3d(ctx, &ma, a, k_len, Q, batch, (uint64_t)k_len * 2, (uint64_t)Q * k_len * 2, GM_BK, GM_BM));
+  LF_TRY(make_map_f16_3d(ctx, &mb, w, k_len, 4 * width, 1, (uint64_t)k_len * 2, (uint64_t)4 * width * k_len * 2, GM_BK, GM_BN));
   LF_TRY(make_map_tiled_act(ctx, &mo, out, ldq, batch * 4 * (width / 128), 32));
   GemmParams p{};
   p.m = Q; p.n = 4 * width; p.k = k_len; p.batch = batch; p.scale = 1.0f; p.bias = bias; p.width = width; p.qscale = qscale;
@@ -330,8 +330,8 @@ lf_status gemm_rows_f32(lf_context* ctx, ArenaCursor& cur, const op16* a, int a_
   if (!a_pieces && !transposed) { Q *= batch; batch = 1; }      // rows one after the other
   CUtensorMap ma, mb, mo;
   if (a_pieces) LF_TRY(make_map_tiled_act(ctx, &ma, a, ldq, batch * (k_len / 128), GM_BM));
-  else LF_TRY(make_map_f16_3d_ext(ctx, &ma, a, k_len, Q, batch, (uint64_t)k_len * 2, (uint64_t)Q * k_len * 2, GM_BK, GM_BM));
-  LF_TRY(make_map_f16_3d_ext(ctx, &mb, w, k_len, n_out, 1, (uint64_t)k_len * 2, (uint64_t)n_out * k_len * 2, GM_BK, GM_BN));
+  else LF_TRY(make_map_f16_3d(ctx, &ma, a, k_len, Q, batch, (uint64_t)k_len * 2, (uint64_t)Q * k_len * 2, GM_BK, GM_BM));
+  LF_TRY(make_map_f16_3d(ctx, &mb, w, k_len, n_out, 1, (uint64_t)k_len * 2, (uint64_t)n_out * k_len * 2, GM_BK, GM_BN));
   const uint64_t row = (uint64_t)n_out * 4;
   if (transposed) LF_TRY(make_map_f32_any(ctx, &mo, out, {(uint64_t)n_out, (uint64_t)batch, (uint64_t)Q}, {row, row * batch}, {32, 1, 32}));
   else LF_TRY(make_map_f32_any(ctx, &mo, out, {(uint64_t)n_out, (uint64_t)Q, (uint64_t)batch}, {row, row * Q}, {32, 32, 1}));
@@ -344,8 +344,8 @@ lf_status gemm_rows_half(lf_context* ctx, ArenaCursor& cur, const op16* a_pieces
   if (cur.dry) return LF_OK;
   CUtensorMap ma, mb, mo;
   LF_TRY(make_map_tiled_act(ctx, &ma, a_pieces, ldq, batch * (k_len / 128), GM_BM));
-  LF_TRY(make_map_f16_3d_ext(ctx, &mb, w, k_len, n_out, 1, (uint64_t)k_len * 2, (uint64_t)n_out * k_len * 2, GM_BK, GM_BN));
-  LF_TRY(make_map_f16_3d_ext(ctx, &mo, out, n_out, Q, batch, (uint64_t)n_out * 2, (uint64_t)Q * n_out * 2, 64, 32));
+  LF_TRY(make_map_f16_3d(ctx, &mb, w, k_len, n_out, 1, (uint64_t)k_len * 2, (uint64_t)n_out * k_len * 2, GM_BK, GM_BN));
+  LF_TRY(make_map_f16_3d(ctx, &mo, out, n_out, Q, batch, (uint64_t)n_out * 2, (uint64_t)Q * n_out * 2, 64, 32));
   GemmParams p{};
   p.m = Q; p.n = n_out; p.k = k_len; p.batch = batch; p.scale = 1.0f; p.a_pieces = 1;
   return launch<0, GM_HALF>(ctx, LF_KERNEL_TRIANGLE_CONTRACT, ma, mb, mo, p);
@@ -356,8 +356,8 @@ lf_status gemm_outer32(lf_context* ctx, ArenaCursor& cur, const op16* left, cons
   if (cur.dry) return LF_OK;
   CUtensorMap ma, mb, mo;
   const uint64_t row = (uint64_t)n * 64;      // both operands have rows of n * 32 values
-  LF_TRY(make_map_f16_3d_ext(ctx, &ma, left, (uint64_t)cnt * 32, k_len, 1, row, row * k_len, 64, GM_BK));
-  LF_TRY(make_map_f16_3d_ext(ctx, &mb, right, (uint64_t)n * 32, k_len, 1, row, row * k_len, 64, GM_BK));
+  LF_TRY(make_map_f16_3d(ctx, &ma, left, (uint64_t)cnt * 32, k_len, 1, row, row * k_len, 64, GM_BK));
+  LF_TRY(make_map_f16_3d(ctx, &mb, right, (uint64_t)n * 32, k_len, 1, row, row * k_len, 64, GM_BK));
   LF_TRY(make_map_grouped(ctx, &mo, out, n, cnt));
   GemmParams p{};
   p.m = cnt * 32; p.n = n * 32; p.k = k_len; p.batch = 1; p.scale = scale;
@@ -370,13 +370,13 @@ lf_status gemm_planes(lf_context* ctx, ArenaCursor& cur, const op16* a, const op
   CUtensorMap ma, mb, mo;
   const uint64_t row = (uint64_t)ld * 2, plane = row * n;
   if (!incoming) {
-    LF_TRY(make_map_f16_3d_ext(ctx, &ma, a, n, n, c, row, plane, GM_BK, GM_BM));
-    LF_TRY(make_map_f16_3d_ext(ctx, &mb, b, n, n, c, row, plane, GM_BK, GM_BN));
+    LF_TRY(make_map_f16_3d(ctx, &ma, a, n, n, c, row, plane, GM_BK, GM_BM));
+    LF_TRY(make_map_f16_3d(ctx, &mb, b, n, n, c, row, plane, GM_BK, GM_BN));
   } else {
-    LF_TRY(make_map_f16_3d_ext(ctx, &ma, b, n, n, c, row, plane, 64, GM_BK));
-    LF_TRY(make_map_f16_3d_ext(ctx, &mb, a, n, n, c, row, plane, 64, GM_BK));
+    LF_TRY(make_map_f16_3d(ctx, &ma, b, n, n, c, row, plane, 64, GM_BK));
+    LF_TRY(make_map_f16_3d(ctx, &mb, a, n, n, c, row, plane, 64, GM_BK));
   }
-  LF_TRY(make_map_f16_3d_ext(ctx, &mo, x, n, n, c, row, plane, 64, 32));
+  LF_TRY(make_map_f16_3d(ctx, &mo, x, n, n, c, row, plane, 64, 32));
   GemmParams p{};
   p.m = n; p.n = n; p.k = n; p.batch = c; p.scale = scale;
   return incoming ? launch<1, GM_HALF>(ctx, LF_KERNEL_TRIANGLE_CONTRACT, ma, mb, mo, p) : launch<0, GM_HALF>(ctx, LF_KERNEL_TRIANGLE_CONTRACT, ma, mb, mo, p);

@@ -23,10 +23,8 @@ typedef CUresult (*EncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t,
 static EncodeTiledFn g_encode = nullptr;
 static std::once_flag g_once;
 
-void configure_once();
-
-lf_status make_map_f16_3d_box(lf_context* ctx, CUtensorMap* map, const void* base, uint64_t d0, uint64_t d1, uint64_t d2,
-                              uint64_t stride1_bytes, uint64_t stride2_bytes, uint32_t b0, uint32_t b1, uint32_t b2) {
+lf_status make_map_f16_3d(lf_context* ctx, CUtensorMap* map, const void* base, uint64_t d0, uint64_t d1, uint64_t d2,
+                          uint64_t stride1_bytes, uint64_t stride2_bytes, uint32_t b0, uint32_t b1, uint32_t b2) {
   if (!g_encode) return lf_fail(ctx, LF_ERR_CUDA, "cuTensorMapEncodeTiled is not available from this driver");
   cuuint64_t dims[3] = {d0, d1, d2};
   cuuint64_t strides[2] = {stride1_bytes, stride2_bytes};
@@ -37,16 +35,6 @@ lf_status make_map_f16_3d_box(lf_context* ctx, CUtensorMap* map, const void* bas
                         CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
   if (r != CUDA_SUCCESS) return lf_fail(ctx, LF_ERR_CUDA, "cuTensorMapEncodeTiled failed with code %d", (int)r);
   return LF_OK;
-}
-
-static lf_status make_map_f16_3d(lf_context* ctx, CUtensorMap* map, const void* base, uint64_t d0, uint64_t d1,
-                                 uint64_t d2, uint64_t stride1_bytes, uint64_t stride2_bytes, uint32_t b0, uint32_t b1) {
-  return make_map_f16_3d_box(ctx, map, base, d0, d1, d2, stride1_bytes, stride2_bytes, b0, b1, 1);
-}
-
-lf_status make_map_f16_3d_ext(lf_context* ctx, CUtensorMap* map, const void* base, uint64_t d0, uint64_t d1, uint64_t d2,
-                              uint64_t stride1_bytes, uint64_t stride2_bytes, uint32_t b0, uint32_t b1) {
-  return make_map_f16_3d(ctx, map, base, d0, d1, d2, stride1_bytes, stride2_bytes, b0, b1);
 }
 
 // Attention activations q, k, v, gate, o: fp16 [batch][ldq][128] stored as 8-row x 8-channel pieces of 128
@@ -483,12 +471,12 @@ static lf_status contract_impl(lf_context* ctx, ArenaCursor& cur, const op16* a,
   CUtensorMap mapA, mapB;
   const uint64_t row_bytes = (uint64_t)ld_ab * 2;
   if (!incoming) {
-    LF_TRY(make_map_f16_3d(ctx, &mapA, a, k_len, m_rows, c, row_bytes, (uint64_t)m_rows * row_bytes, CT_BK, CT_BM));
-    LF_TRY(make_map_f16_3d(ctx, &mapB, b, k_len, n_rows, c, row_bytes, (uint64_t)n_rows * row_bytes, CT_BK, CT_BN));
+    LF_TRY(make_map_f16_3d(ctx, &mapA, a, k_len, m_rows, c, row_bytes, (uint64_t)m_rows * row_bytes, CT_BK, CT_BM, 1));
+    LF_TRY(make_map_f16_3d(ctx, &mapB, b, k_len, n_rows, c, row_bytes, (uint64_t)n_rows * row_bytes, CT_BK, CT_BN, 1));
   } else {
     // A(i,k) = b[h][k][i], B(j,k) = a[h][k][j]: boxes of 64 (i or j) x 64 (k)
-    LF_TRY(make_map_f16_3d(ctx, &mapA, b, m_rows, k_len, c, row_bytes, (uint64_t)k_len * row_bytes, 64, CT_BK));
-    LF_TRY(make_map_f16_3d(ctx, &mapB, a, n_rows, k_len, c, row_bytes, (uint64_t)k_len * row_bytes, 64, CT_BK));
+    LF_TRY(make_map_f16_3d(ctx, &mapA, b, m_rows, k_len, c, row_bytes, (uint64_t)k_len * row_bytes, 64, CT_BK, 1));
+    LF_TRY(make_map_f16_3d(ctx, &mapB, a, n_rows, k_len, c, row_bytes, (uint64_t)k_len * row_bytes, 64, CT_BK, 1));
   }
   const int tiles = c * ((m_rows + CT_BM - 1) / CT_BM) * ((n_rows + CT_BN - 1) / CT_BN);
   const int grid = tiles < ctx->sm_count ? tiles : ctx->sm_count;

@@ -1,6 +1,6 @@
 // Tensor-core (tcgen05 / TMEM / TMA) kernels for sm_100a: launchers used by api.cu.
 // Each *_supported() says whether a kernel covers a shape; api.cu routes
-// everything else to the float32 SIMT kernels.
+// everything else to the general path.
 #pragma once
 
 #include "common.cuh"
@@ -8,7 +8,7 @@
 namespace tc {
 
 // Device buffers of the other ranks of a box as mapped into this process (entry `rank` = the local
-// buffer).  Kernels only ever store to them with plain st.global.
+// buffer).  Kernels only ever store to them: plain st.global, or TMA stores without multicast.
 constexpr int kMaxPeers = 16;
 struct PeerPtrs { void* p[kMaxPeers]; };
 
@@ -59,7 +59,7 @@ lf_status gemm_rows_f32(lf_context* ctx, ArenaCursor& cur, const op16* a, int a_
 lf_status gemm_rows_half(lf_context* ctx, ArenaCursor& cur, const op16* a_pieces, const op16* w, op16* out, int batch, int Q, int ldq, int n_out, int k_len);
 lf_status gemm_outer32(lf_context* ctx, ArenaCursor& cur, const op16* left, const op16* right, op16* out, int cnt, int n, int k_len, float scale);
 lf_status gemm_planes(lf_context* ctx, ArenaCursor& cur, const op16* a, const op16* b, op16* x, int n, int ld, int c, int incoming, float scale);
-// As rows: out[m][n] = act(sum_k a[m][k] w[n][k] + bias[n]) (k contiguous in both
+// fp16 rows: out[m][n] = act(sum_k a[m][k] w[n][k] + bias[n]) (k contiguous in both
 // operands, k_len and n_out multiples of 8; bias may be null; act = ReLU when `relu`), fp16 result.
 lf_status contract_gemm(lf_context* ctx, ArenaCursor& cur, const op16* a, const op16* w, op16* out, int m_rows, int n_out,
                         int k_len, const float* bias, int relu);

@@ -3,10 +3,10 @@
 // One persistent CTA per SM.  The projection weights (W^T, fp16, up to 528 x 128)
 // stay resident in shared memory in the 128-byte-swizzled K-major layout the
 // tensor core reads; each 128-row tile of the activation is normalised in
-// registers by four producer warps (one row per warp-wide load, statistics by
-// warp shuffle), written as the fp16 A operand straight into swizzled shared
+// registers by eight producer warps (eight lanes a row, statistics by warp
+// shuffle), written as the fp16 operand straight into swizzled shared
 // memory, multiplied in chunks of up to 256 output columns into double-buffered
-// TMEM accumulators, and finished by eight epilogue warps (bias, sigmoid gates,
+// TMEM accumulators, and finished by sixteen epilogue warps (bias, sigmoid gates,
 // mask, layout change) while the next chunk's MMAs run.
 //
 // Warp roles: 0..15 epilogue (TMEM lane quadrant = warp % 4, quarter of the columns =
@@ -35,7 +35,7 @@ struct LnGemmParams {
   int64_t rows;             // logical rows
   int transpose, batch, Q;  // logical row (b, i) reads memory row i*batch + b when transpose
   float eps;                // (the LayerNorm's gain and offset are folded into wimg and bias when the weights are prepared)
-  int variance;             // 1 two-pass, 2 fast
+  int variance;             // triangle output: 1 clamps the centre LayerNorm's E[x^2] - E[x]^2 at 0, 2 does not (the input LayerNorm knows one formula: normalise)
   const uint8_t* wimg;      // swizzled fp16 image of W^T: [2 atoms][n_pad rows][128 B]
   int n_pad;
   const float* bias;        // [n_bias]
@@ -47,15 +47,12 @@ struct LnGemmParams {
   int chunk_row0[LG_MAX_CHUNKS];
   // triangle projection epilogue
   const float* mask;        // [rows]
-  op16* out_a;              // [c][n][ld]
-  op16* out_b;
   int n, ld;                // pair row length and operand row stride
   int plane_rows;           // pair rows held (n for a whole pair, fewer for a row shard)
-  // channel-sharded destinations (peer_ranks >= 1; one rank = rows inside whole planes of this device): channel h goes to rank h / ch_per_rank, plane h % ch_per_rank of
-  // its [ch_per_rank][peer_plane_rows][ld] buffer, at rows peer_row0 + local row; stores go to the peers' memory
-  int peer_ranks, ch_per_rank, peer_plane_rows, peer_row0;
-  PeerPtrs peer_a, peer_b;
-  int plane_box_h;          // planes per copy of a warp's 32 (maps in PlaneMaps)
+  // destinations (maps in PlaneMaps): channel h goes to owner h / ch_per_rank, plane h % ch_per_rank of its planes, at rows peer_row0 + local row;
+  // one owner = this device's whole planes, several = the ranks' buffers, which the copies write over NVLink
+  int ch_per_rank, peer_row0;
+  int plane_box_h;          // planes per copy of a warp's 32
   // attention projection epilogue
   op16* out_q; op16* out_k; op16* out_v; op16* out_g;   // logical rows, stored in 8 x 8 pieces (see ldq)
   op16* out_bias;           // fp16 [heads][batch rows][ldb] (head, query, key)
@@ -905,7 +902,7 @@ lf_status triangle_project(lf_context* ctx, ArenaCursor& cur, const void* z, int
   p.eps = eps; p.variance = variance;
   p.wimg = (const uint8_t*)w->h[0]; p.n_pad = 512; p.bias = (const float*)w->h[1]; p.n_bias = 512;
   p.n_chunks = 2; p.chunk_n[0] = 256; p.chunk_n[1] = 256; p.chunk_row0[0] = 0; p.chunk_row0[1] = 256;
-  p.mask = mask; p.out_a = a; p.out_b = b; p.n = n; p.ld = ld; p.status = (Status*)ctx->tc_status;
+  p.mask = mask; p.n = n; p.ld = ld; p.status = (Status*)ctx->tc_status;
   PeerPtrs pa{}, pb{};
   pa.p[0] = a; pb.p[0] = b;
   return launch_triangle<1>(ctx, p, pa, pb, 1, rows, rows);
@@ -922,9 +919,7 @@ lf_status triangle_project_scatter(lf_context* ctx, ArenaCursor& cur, const void
   p.wimg = (const uint8_t*)w->h[0]; p.n_pad = 512; p.bias = (const float*)w->h[1]; p.n_bias = 512;
   p.n_chunks = 2; p.chunk_n[0] = 256; p.chunk_n[1] = 256; p.chunk_row0[0] = 0; p.chunk_row0[1] = 256;
   p.mask = mask; p.n = n; p.ld = ld; p.status = (Status*)ctx->tc_status;
-  p.peer_ranks = ranks; p.ch_per_rank = 128 / ranks; p.peer_plane_rows = n; p.peer_row0 = row0;
-  p.peer_a = a_peers; p.peer_b = b_peers;
-  p.out_a = (op16*)a_peers.p[0]; p.out_b = (op16*)b_peers.p[0];      // ranks == 1: plain form
+  p.peer_row0 = row0;
   return launch_triangle<kMaxPeers>(ctx, p, a_peers, b_peers, ranks, rows, n);
 }
 
@@ -975,8 +970,8 @@ static lf_status attention_project_impl(lf_context* ctx, ArenaCursor& cur, const
   return LF_OK;
 }
 
-lf_status make_map_f16_3d_box(lf_context* ctx, CUtensorMap* map, const void* base, uint64_t d0, uint64_t d1, uint64_t d2,
-                              uint64_t stride1_bytes, uint64_t stride2_bytes, uint32_t b0, uint32_t b1, uint32_t b2);
+lf_status make_map_f16_3d(lf_context* ctx, CUtensorMap* map, const void* base, uint64_t d0, uint64_t d1, uint64_t d2,
+                          uint64_t stride1_bytes, uint64_t stride2_bytes, uint32_t b0, uint32_t b1, uint32_t b2);
 
 // Pair bias from a pair tensor with a LayerNorm of its own (MSA row attention with pair bias, AF3 single attention,
 // AF3 MSA pair-weighted averaging): bias[h][q][k] = LN(pair)[q][k] . W[:, h] as fp16 [heads][Q][ldb], by the
@@ -1043,8 +1038,8 @@ lf_status triangle_output(lf_context* ctx, ArenaCursor& cur, const op16* x, int 
                           void* out, int64_t x_plane_elems) {
   if (cur.dry) return LF_OK;
   CUtensorMap mapX;
-  LF_TRY(make_map_f16_3d_box(ctx, &mapX, x, n, rows, 128, (uint64_t)ld * 2,
-                             (uint64_t)(x_plane_elems ? x_plane_elems : (int64_t)rows * ld) * 2, 64, 1, 128));
+  LF_TRY(make_map_f16_3d(ctx, &mapX, x, n, rows, 128, (uint64_t)ld * 2,
+                         (uint64_t)(x_plane_elems ? x_plane_elems : (int64_t)rows * ld) * 2, 64, 1, 128));
   LnGemmParams p{};
   p.act = z; p.act_bf16 = act_dtype == LF_DTYPE_BF16; p.rows = (int64_t)rows * n; p.transpose = 0; p.batch = 1; p.Q = 1;
   p.plane_rows = rows;
