@@ -14,7 +14,7 @@ import math
 import numpy as np
 
 from . import _native as nat
-from .operators import (AttentionGpu, Af3SingleAttentionGpu, Af3TransitionGpu, OuterProductMeanGpu,
+from .operators import (AttentionGpu, Af3SingleAttentionGpu, Af3TransitionGpu, EncodedTensor, OuterProductMeanGpu,
                         PreparedWeights, TransitionGpu, _Buffer, _device, _precision, _variance,
                         prepare_single_attention_weights,
                         SINGLE_ATTENTION_AF3_ORDER, TRANSITION_AF3_ORDER, TRANSITION_WEIGHT_ORDER,
@@ -63,11 +63,18 @@ class PreparedPairBlock:
 
 
 def _same_shapes(blocks):
-    """Whether the weight objects of a stack all have the first one's tensors: then the others are as valid as it is."""
+    """Whether the weight objects of a stack are all laid out as the first one: then the others are as valid as it is.  Counts everything that
+    preparing a block checks: keys, tensor shapes, whole numbers by value, encoded tensors with their group size, payload length and offsets."""
     def shapes(value):
         if isinstance(value, dict):
             return {k: shapes(v) for k, v in value.items()}
-        return getattr(value, "shape", value if isinstance(value, (int, bool, type(None))) else type(value))
+        if isinstance(value, EncodedTensor):
+            return (value.shape, value.count, value.block, len(value.payload), value.scale_offset, value.zero_offset)
+        if value is None or isinstance(value, str):
+            return value
+        if isinstance(value, (int, np.integer)):
+            return int(value)
+        return tuple(value.shape) if hasattr(value, "shape") else np.shape(value)
     first = shapes(blocks[0])
     return all(shapes(b) == first for b in blocks[1:])
 
