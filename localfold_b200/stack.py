@@ -66,11 +66,14 @@ def _same_shapes(blocks):
     """Whether the weight objects of a stack are all laid out as the first one: then the others are as valid as it is.  Counts everything that
     preparing a block checks: keys, tensor shapes, whole numbers by value, encoded tensors with their group size, payload length and offsets."""
     def shapes(value):
+        kind = type(value)
+        if kind is np.ndarray:
+            return value.shape
+        if kind is EncodedTensor:
+            return (value.shape, value.count, value.block, len(value.payload), value.scale_offset, value.zero_offset)
         if isinstance(value, dict):
             return {k: shapes(v) for k, v in value.items()}
-        if isinstance(value, EncodedTensor):
-            return (value.shape, value.count, value.block, len(value.payload), value.scale_offset, value.zero_offset)
-        if value is None or isinstance(value, str):
+        if value is None or kind is str:
             return value
         if isinstance(value, (int, np.integer)):
             return int(value)
