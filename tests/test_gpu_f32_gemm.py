@@ -1,5 +1,5 @@
 """Float32 mode through the split-operand GEMM at the edges of its tiles (128 x 128 x 64): rows, columns and inner lengths
-around them, widths that are not whole groups of eight, contractions past one accumulation chunk of 128 - and no less
+around them, widths that are not whole groups of eight, contractions past one accumulation chunk of 64 - and no less
 accurate than a float32 product: the error against float64 stays below that of float32 rounding of every operand."""
 import numpy as np
 import pytest
