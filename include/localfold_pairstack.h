@@ -17,6 +17,11 @@
  *    only enqueues work on the context's stream - use lf_context_synchronize).
  *  - Activations in host space are float32.  In device space `act_dtype`
  *    gives their storage type.
+ *    Device buffers may start at any element; on a 16-byte boundary (bfloat16
+ *    results, or a float32 result beside a residual that lives elsewhere: 32)
+ *    the fused kernels take them, elsewhere the general path.  The shard steps
+ *    and lf_triangle_multiplication_run_static have only the fused kernels and
+ *    refuse other addresses with LF_ERR_ARGUMENT.
  *  - Weights are handed over once per operator as float32 host arrays in the
  *    reference's own layouts and field order; the library keeps its own
  *    device-resident copy (repacked for its kernels) until lf_weights_destroy.
