@@ -13,7 +13,7 @@ import sys
 HERE = os.path.dirname(os.path.abspath(__file__))
 CSRC = os.path.join(HERE, "csrc")
 LIB = os.path.join(HERE, "lib", "liblocalfold_pairstack.so")
-SOURCES = ("api.cu", "tc_kernels.cu", "tc_ln_gemm.cu", "tc_attention.cu", "tc_transition.cu", "tc_weights.cu", "f32_gemm.cu", "tc_gemm.cu", "static_scratch.cu", "peer_transpose.cu", "pair_spill.cu")
+SOURCES = ("api.cu", "tc_kernels.cu", "tc_ln_gemm.cu", "tc_attention.cu", "tc_transition.cu", "tc_weights.cu", "f32_gemm.cu", "tc_gemm.cu", "f32_attention.cu", "static_scratch.cu", "peer_transpose.cu", "pair_spill.cu")
 NVCC_FLAGS = (
     "-gencode", "arch=compute_100a,code=sm_100a", "-lineinfo", "-O3", "-std=c++17", "--threads", "0",
     "-Xcompiler", "-fPIC,-fvisibility=hidden", "-shared",

@@ -121,6 +121,7 @@ static lf_status context_create(int device_ordinal, void* stream, bool make_stre
         cudaFuncSetAttribute(rows::global_mean_kernel<float>, cudaFuncAttributeMaxDynamicSharedMemorySize, 16 * 513 * 4);
         cudaFuncSetAttribute(rows::global_mean_kernel<bf16>, cudaFuncAttributeMaxDynamicSharedMemorySize, 16 * 513 * 4);
         configure_mma_attention();
+        tc::configure_attention3();
         cudaGetLastError();
       });
   }
@@ -976,11 +977,11 @@ void sgemm(lf_context* ctx, ArenaCursor& cur, bool ta, int M, int N, int K, cons
   else LAUNCH(ctx, cur, simt::sgemm_kernel<false>, grid, 256, 0, M, N, K, A, lda, B, ldb, C, ldc, bias);
 }
 
-// The float32 attention core for any head width: terms of q | k | v | gate -> the gated output likewise.
+// The float32 attention core for any head width: terms of q | k | v and the gate -> terms of the gated output.
 constexpr int kAttentionSmem = 96 * 1024;      // two blocks an SM
 #define ATTENTION_WIDTHS(X) X(8) X(16) X(24) X(32) X(48) X(64)
-void mma_attention_core(lf_context* ctx, ArenaCursor& cur, int D, const SplitMatrix& qkvg, const float* bias, const float* mask,
-                        mma_attention::AttentionShape s, const SplitMatrix& out) {
+void mma_attention_core(lf_context* ctx, ArenaCursor& cur, int D, const SplitMatrix& qkv, const float* gate, const float* bias, const float* mask,
+                        mma_attention::AttentionShape s, const SplitMatrix& out) {      // s: up to ldb
   // eight warps, or as many as the queries have groups of 16: the groups are spread evenly over the blocks; small query
   // counts put several batch rows into a block
   const int groups = lf_ceil_div(s.Q, 16), tiles = lf_ceil_div(groups, 8);
@@ -993,15 +994,14 @@ void mma_attention_core(lf_context* ctx, ArenaCursor& cur, int D, const SplitMat
   while (s.kt > 32 && (s.kt >= 2 * s.Q || bytes(s.kt) > kAttentionSmem)) s.kt /= 2;
   while (s.wb > 1 && bytes(s.kt) > kAttentionSmem) s.wb /= 2;
   s.mk = (s.Q < 1024 ? lf_ceil_div(s.Q, s.kt) : lf_ceil_div(1024, s.kt)) * s.kt;
-  s.ld = qkvg.ld; s.term_stride = qkvg.term_stride;
-  s.ldo = out.ld; s.out_stride = out.term_stride;
+  s.out_stride = out.term_stride;
   const dim3 grid(lf_ceil_div(groups, s.wq), lf_ceil_div(s.batch, s.wb), s.heads);
   const size_t smem = bytes(s.kt);
-  const uint16_t* in = (const uint16_t*)qkvg.p;
+  const uint16_t* in = (const uint16_t*)qkv.p;
 #define ATTENTION_CASE(D_)                                                                                                                   \
   case D_:                                                                                                                                   \
-    if (bias) LAUNCH(ctx, cur, (mma_attention::attention_kernel<D_, true>), grid, 32 * s.wb * s.wq, smem, in, bias, mask, s, (uint16_t*)out.p);  \
-    else LAUNCH(ctx, cur, (mma_attention::attention_kernel<D_, false>), grid, 32 * s.wb * s.wq, smem, in, bias, mask, s, (uint16_t*)out.p);      \
+    if (bias) LAUNCH(ctx, cur, (mma_attention::attention_kernel<D_, true>), grid, 32 * s.wb * s.wq, smem, in, gate, bias, mask, s, (uint16_t*)out.p);  \
+    else LAUNCH(ctx, cur, (mma_attention::attention_kernel<D_, false>), grid, 32 * s.wb * s.wq, smem, in, gate, bias, mask, s, (uint16_t*)out.p);      \
     break;
   switch (D) { ATTENTION_WIDTHS(ATTENTION_CASE) }
 #undef ATTENTION_CASE
@@ -1251,8 +1251,8 @@ struct AttArgs {
 // Whether the fused projection kernel makes the bias of a.bias_mode 1 from the pair.
 bool tensor_core_bias(const AttArgs& a) { return tc::pair_bias_supported(a.w) && !a.bias_swap && lf_aligned16(a.pair); }
 
-// The pair bias of a.bias_mode 1 (a pair tensor with a LayerNorm of its own) as float32 [heads][Q][Q].
-lf_status separate_bias(lf_context* ctx, ArenaCursor& cur, const AttArgs& a, float* bias) {
+// The pair bias of a.bias_mode 1 (a pair tensor with a LayerNorm of its own) as float32 [heads][Q][ld].
+lf_status separate_bias(lf_context* ctx, ArenaCursor& cur, const AttArgs& a, float* bias, int ld) {
   const auto& f = a.w->f;
   const int64_t QQ = (int64_t)a.Q * a.Q;
   if (a.tc_pair_bias && tensor_core_bias(a)) {
@@ -1260,13 +1260,13 @@ lf_status separate_bias(lf_context* ctx, ArenaCursor& cur, const AttArgs& a, flo
     const int ldb = (a.Q + 15) / 16 * 16;
     op16* b16 = cur.take<op16>((int64_t)a.heads * a.Q * ldb);
     LF_TRY(tc::pair_bias_project(ctx, cur, a.pair, a.pair_dtype, a.Q, a.pair_variance, a.pair_eps, a.heads, a.w, b16, ldb));
-    LAUNCH(ctx, cur, simt::widen_bias_kernel, lf_ceil_div(QQ * a.heads, 256), 256, 0, b16, a.heads, a.Q, ldb, bias);
+    LAUNCH(ctx, cur, simt::widen_bias_kernel, lf_ceil_div(QQ * a.heads, 256), 256, 0, b16, a.heads, a.Q, ldb, bias, ld);
   } else if (a.pair_dtype == LF_DTYPE_BF16)
     LAUNCH(ctx, cur, (simt::pair_bias_kernel<bf16>), lf_ceil_div(QQ, 8), 256, 0, (const bf16*)a.pair, a.Q, a.pair_ch, a.heads, f[ATT_PLN_G], f[ATT_PLN_B],
-           f[ATT_WB], a.pair_eps, a.pair_variance, a.bias_swap, bias);
+           f[ATT_WB], a.pair_eps, a.pair_variance, a.bias_swap, bias, ld);
   else
     LAUNCH(ctx, cur, (simt::pair_bias_kernel<float>), lf_ceil_div(QQ, 8), 256, 0, (const float*)a.pair, a.Q, a.pair_ch, a.heads, f[ATT_PLN_G], f[ATT_PLN_B],
-           f[ATT_WB], a.pair_eps, a.pair_variance, a.bias_swap, bias);
+           f[ATT_WB], a.pair_eps, a.pair_variance, a.bias_swap, bias, ld);
   return LF_OK;
 }
 
@@ -1281,18 +1281,23 @@ lf_status att_f32(lf_context* ctx, ArenaCursor& cur, const AttArgs& a) {
   const SplitMatrix nrm = take_terms(cur, R, c);
   // q | k | v | sigmoid(gate) with heads of D channels, and the pair bias columns when the bias comes from the normalised input
   const int D = head_width(a.d), HDp = a.heads * D, wide = 4 * HDp + (a.bias_mode == 2 ? a.heads : 0);
-  const SplitMatrix qkvg = take_terms(cur, R, wide);
-  float* bias = a.bias_mode ? cur.take<float>((int64_t)a.heads * a.Q * a.Q) : nullptr;
-  const SplitMatrix o = take_terms(cur, R, HDp);
+  const SplitMatrix qkv = take_terms(cur, R, 3 * HDp);      // in pieces
+  float* gate = cur.take<float>(R * HDp);
+  const int ldb = (a.Q + 3) / 4 * 4;
+  float* bias = a.bias_mode ? cur.take<float>((int64_t)a.heads * a.Q * ldb) : nullptr;
+  SplitMatrix o = take_terms(cur, R, HDp);
+  o.pieces = true;
   float* proj = cur.take<float>(R * c);
   layer_norm<T, rows::LN_TERMS>(ctx, cur, a.act, R, c, f[ATT_LN_G], f[ATT_LN_B], a.eps, a.variance, a.transpose, a.batch, a.Q, (void*)nrm.p, nrm.term_stride);
   LF_TRY(tc::gemm_f32(ctx, cur, 0, nrm, g[0], (int)R, wide, c, 1,
-                      {nullptr, (bf16*)qkvg.p, qkvg.ld, 0, qkvg.term_stride, reinterpret_cast<const float*>(g[2].p), 4 * HDp, 0, 3 * HDp, 4 * HDp}));
-  if (a.bias_mode == 1) LF_TRY(separate_bias(ctx, cur, a, bias));
-  else if (a.bias_mode == 2)
-    LAUNCH(ctx, cur, rows::bias_columns_kernel, lf_ceil_div((int64_t)a.Q * a.Q, 256), 256, 0, qkvg.p, qkvg.ld, qkvg.term_stride, 4 * HDp, a.Q, a.heads,
-           a.bias_swap, bias);
-  mma_attention_core(ctx, cur, D, qkvg, bias, a.mask, {a.batch, a.Q, a.heads, a.transpose, a.mask_mode, a.clamp, 1.0f / sqrtf((float)a.d)}, o);
+                      {nullptr, (bf16*)qkv.p, qkv.ld, 0, qkv.term_stride, reinterpret_cast<const float*>(g[2].p), 4 * HDp, 0, 3 * HDp, 4 * HDp, 1,
+                       gate, bias, a.Q, ldb, a.bias_swap}));
+  if (a.bias_mode == 1) LF_TRY(separate_bias(ctx, cur, a, bias, ldb));
+  const float scale = 1.0f / sqrtf((float)a.d);
+  if (tc::attention3_wins(ctx, D, a.batch, a.Q, a.heads))
+    LF_TRY(tc::attention3(ctx, cur, D, qkv, gate, bias, ldb, a.mask, a.batch, a.Q, a.heads, a.transpose, a.mask_mode, a.clamp, scale, o));
+  else
+    mma_attention_core(ctx, cur, D, qkv, gate, bias, a.mask, {a.batch, a.Q, a.heads, a.transpose, a.mask_mode, a.clamp, scale, R, qkv.term_stride, ldb}, o);
   LF_TRY(tc::gemm_f32(ctx, cur, 0, o, g[1], (int)R, c, HDp, 1, {proj, nullptr, c, 0, 0, f[ATT_BO], c, 0, 0, 0}));
   finish<T>(ctx, cur, proj, nullptr, a.residual ? a.act : nullptr, R, c, a.transpose, a.batch, a.Q, a.out);
   return LF_OK;
@@ -1327,7 +1332,7 @@ lf_status msa_average(lf_context* ctx, ArenaCursor& cur, const AttArgs& a) {
   const SplitMatrix o = take_terms(cur, R, HD);
   float* proj = cur.take<float>(R * c);
   if ((int64_t)S * d > 0x7fffffff) return lf_fail(ctx, LF_ERR_SHAPE, "too many sequences for one average");
-  LF_TRY(separate_bias(ctx, cur, a, bias));
+  LF_TRY(separate_bias(ctx, cur, a, bias, n));
   LAUNCH(ctx, cur, rows::key_mask_kernel, lf_ceil_div(n, 32), dim3(32, 32), 0, a.mask, S, n, key);
   LAUNCH(ctx, cur, rows::average_weights_kernel, dim3(lf_ceil_div(n, 32), H), 256, 0, bias, key, n, (int)w.ld, (bf16*)w.p, w.term_stride);
   layer_norm<float, rows::LN_TERMS>(ctx, cur, a.act, R, c, f[ATT_LN_G], f[ATT_LN_B], a.eps, a.variance, 0, 1, 1, (void*)nrm.p, nrm.term_stride);

@@ -96,6 +96,7 @@ enum { GLB_LN_G, GLB_LN_B, GLB_WQ, GLB_W3, GLB_B3, GLB_WO, GLB_BO, GLB_COUNT };
 struct SplitMatrix {
   const bf16* p = nullptr;
   int64_t ld = 0, batch_stride = 0, term_stride = 0;
+  bool pieces = false;      // in pieces of eight columns: element (i, j) of a term at (j / 8) * rows * 8 + i * 8 + j % 8
 };
 
 // Operands of the float32 GEMM, [n_out][k] terms, kept with the weights.  Operators that use them in either mode get them when the

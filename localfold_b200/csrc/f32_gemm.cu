@@ -32,6 +32,10 @@ struct Gemm3Params {
   int64_t ldo, batch_stride, term_stride;
   const float* bias;           // or null
   int bias_n, relu, sigmoid_col0, sigmoid_col1;
+  int pieces;                  // terms in pieces of eight columns, behind them a gate and a pair bias (Gemm3Out)
+  float* gate;
+  float* pair_bias;
+  int bias_q, bias_ld, bias_swap;
   Status* status;
 };
 
@@ -40,7 +44,8 @@ __host__ __device__ constexpr uint32_t make_idesc_bf16(int M, int N, int major) 
   return make_idesc_f16(M, N, major, major) | (1u << 7) | (1u << 10);
 }
 
-template <int MAJOR>      // 0: k contiguous in both operands; 1: the row index contiguous in both
+// MAJOR 0: k contiguous in both operands; 1: the row index contiguous in both.  PIECES: A in pieces of eight k, the unswizzled operand format
+template <int MAJOR, bool PIECES>
 __global__ void __launch_bounds__(G3_THREADS, 1)
 gemm3_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant__ CUtensorMap mapB, const Gemm3Params p) {
   extern __shared__ uint8_t smem_raw[];
@@ -85,8 +90,9 @@ gemm3_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant__ C
           uint8_t* sA = smem + stage * G3_STAGE;
           uint8_t* sB = sA + 3 * G3_PLANE;
           mbar_expect_tx(&full[stage], G3_STAGE);
-          if (MAJOR == 0) {      // [term][128 rows][64 k]
-            tma_load_4d(sA, &mapA, &full[stage], kb * G3_BK, mi * G3_BM, h, 0);
+          if (MAJOR == 0) {      // [term][128 rows][64 k], or [term][8 pieces][128 rows]
+            if (PIECES) tma_load_4d(sA, &mapA, &full[stage], mi * G3_BM * 2, 0, kb * (G3_BK / 8), 0);
+            else tma_load_4d(sA, &mapA, &full[stage], kb * G3_BK, mi * G3_BM, h, 0);
             tma_load_4d(sB, &mapB, &full[stage], kb * G3_BK, nj * G3_BN, h, 0);
           } else {               // per 64 rows: [term][64 k][64 rows]
 #pragma unroll
@@ -119,13 +125,14 @@ gemm3_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant__ C
               return MAJOR == 0 ? make_smem_desc(base + term * G3_PLANE + kk * 32, 16, 1024)
                                 : make_smem_desc(base + term * (G3_PLANE / 2) + kk * 2048, 3 * (G3_PLANE / 2), 1024);
             };
+            auto adesc = [&](int term) { return PIECES ? make_smem_desc_plain(a0 + term * G3_PLANE + kk * 2 * G3_BM * 16, G3_BM * 16, 128) : desc(a0, term); };
             const uint32_t more = kk != 0 ? 1u : 0u;
-            umma_f16(d + 128, desc(a0, 2), desc(b0, 0), idesc, more);
-            umma_f16(d + 128, desc(a0, 1), desc(b0, 1), idesc, 1u);
-            umma_f16(d + 128, desc(a0, 0), desc(b0, 2), idesc, 1u);
-            umma_f16(d + 128, desc(a0, 1), desc(b0, 0), idesc, 1u);
-            umma_f16(d + 128, desc(a0, 0), desc(b0, 1), idesc, 1u);
-            umma_f16(d, desc(a0, 0), desc(b0, 0), idesc, more);
+            umma_f16(d + 128, adesc(2), desc(b0, 0), idesc, more);
+            umma_f16(d + 128, adesc(1), desc(b0, 1), idesc, 1u);
+            umma_f16(d + 128, adesc(0), desc(b0, 2), idesc, 1u);
+            umma_f16(d + 128, adesc(1), desc(b0, 0), idesc, 1u);
+            umma_f16(d + 128, adesc(0), desc(b0, 1), idesc, 1u);
+            umma_f16(d, adesc(0), desc(b0, 0), idesc, more);
           }
           umma_commit(&empty[stage]);
           if (++stage == G3_STAGES) { stage = 0; phase ^= 1; }
@@ -166,7 +173,7 @@ gemm3_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant__ C
       }
       if (!ok) break;
       const int row0 = mi * G3_BM + q * 32;
-      if (col0 >= (p.out ? p.n : (int)p.ldo) || row0 >= p.m) continue;
+      if (col0 >= (p.out || p.pieces ? p.n : (int)p.ldo) || row0 >= p.m) continue;
       {
         if (p.bias && col0 < p.bias_n) {      // through the staging rows: four at a time, the same for every lane
           float* bias = reinterpret_cast<float*>(stage);
@@ -214,6 +221,48 @@ gemm3_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant__ C
             }
             __syncwarp();
           }
+        } else if (p.pieces) {
+          const int row = row0 + lane;
+          const int terms = (int)p.ldo, gates = terms / 3 * 4;      // first column of the gate, of the pair bias
+          if (row < p.m && col0 + 32 > terms) {
+#pragma unroll
+            for (int k8 = 0; k8 < 4; ++k8) {
+              const int col = col0 + k8 * 8;
+              if (col >= terms && col < gates) {
+                float* dst = p.gate + ((int64_t)((col - terms) / 8) * p.m + row) * 8;
+                *reinterpret_cast<float4*>(dst) = make_float4(v[k8 * 8], v[k8 * 8 + 1], v[k8 * 8 + 2], v[k8 * 8 + 3]);
+                *reinterpret_cast<float4*>(dst + 4) = make_float4(v[k8 * 8 + 4], v[k8 * 8 + 5], v[k8 * 8 + 6], v[k8 * 8 + 7]);
+              }
+            }
+            if (col0 + 32 > gates && gates < p.n) {
+              const int i = row / p.bias_q, j = row - i * p.bias_q;
+              float* dst = p.pair_bias + (p.bias_swap ? (int64_t)j * p.bias_ld + i : (int64_t)i * p.bias_ld + j);
+              const int64_t head = (int64_t)p.bias_q * p.bias_ld;
+#pragma unroll
+              for (int e = 0; e < 32; ++e)
+                if (col0 + e >= gates && col0 + e < p.n) dst[(col0 + e - gates) * head] = v[e];
+            }
+          }
+          if (row < p.m && col0 < terms) {
+            // a lane's eight columns are 16 bytes and its neighbour's row follows: whole lines leave without a turn through shared memory
+            bf16* dst = p.terms + ((int64_t)(col0 / 8) * p.m + row) * 8;
+#pragma unroll
+            for (int term = 0; term < 3; ++term) {
+#pragma unroll
+              for (int k8 = 0; k8 < 4; ++k8) {
+                uint32_t w[4];
+#pragma unroll
+                for (int e = 0; e < 4; ++e) {
+                  const __nv_bfloat162 b2 = __floats2bfloat162_rn(v[k8 * 8 + 2 * e], v[k8 * 8 + 2 * e + 1]);
+                  w[e] = *reinterpret_cast<const uint32_t*>(&b2);
+                  v[k8 * 8 + 2 * e] -= __low2float(b2);
+                  v[k8 * 8 + 2 * e + 1] -= __high2float(b2);
+                }
+                if (col0 + k8 * 8 < terms)
+                  *reinterpret_cast<uint4*>(dst + term * p.term_stride + (int64_t)k8 * p.m * 8) = make_uint4(w[0], w[1], w[2], w[3]);
+              }
+            }
+          }
         } else {
           // ... or their terms, 64-byte runs a row and term (ldo a multiple of 8)
 #pragma unroll 1
@@ -251,10 +300,12 @@ gemm3_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant__ C
 }
 
 void configure_gemm3() {
-  cudaFuncSetAttribute(gemm3_kernel<0>, cudaFuncAttributeMaxDynamicSharedMemorySize, G3_SMEM);
-  cudaFuncSetAttribute(gemm3_kernel<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, G3_SMEM);
+  cudaFuncSetAttribute(gemm3_kernel<0, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, G3_SMEM);
+  cudaFuncSetAttribute(gemm3_kernel<0, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, G3_SMEM);
+  cudaFuncSetAttribute(gemm3_kernel<1, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, G3_SMEM);
 }
 
+lf_status make_map_term_pieces(lf_context* ctx, CUtensorMap* map, const SplitMatrix& a, int Q, int batch, uint32_t rows, uint32_t batch_rows, uint32_t pieces, uint32_t terms);
 lf_status make_map_terms(lf_context* ctx, CUtensorMap* map, const SplitMatrix& a, uint64_t d0, uint64_t d1, uint64_t batch, uint32_t b1);
 
 lf_status gemm_f32(lf_context* ctx, ArenaCursor& cur, int major, const SplitMatrix& a, const SplitMatrix& b, int m, int n, int k, int batch,
@@ -264,7 +315,8 @@ lf_status gemm_f32(lf_context* ctx, ArenaCursor& cur, int major, const SplitMatr
     return lf_fail(ctx, LF_ERR_ARGUMENT, "split operands need strides of whole groups of eight");
   CUtensorMap ma, mb;
   if (major == 0) {
-    LF_TRY(make_map_terms(ctx, &ma, a, k, m, batch, G3_BM));
+    if (a.pieces) LF_TRY(make_map_term_pieces(ctx, &ma, a, m, 1, G3_BM, 1, G3_BK / 8, 3));
+    else LF_TRY(make_map_terms(ctx, &ma, a, k, m, batch, G3_BM));
     LF_TRY(make_map_terms(ctx, &mb, b, k, n, batch, G3_BN));
   } else {
     LF_TRY(make_map_terms(ctx, &ma, a, m, k, batch, G3_BK));
@@ -274,12 +326,14 @@ lf_status gemm_f32(lf_context* ctx, ArenaCursor& cur, int major, const SplitMatr
   p.m = m; p.n = n; p.k = k; p.batch = batch;
   p.out = o.out; p.terms = o.terms; p.ldo = o.ld; p.batch_stride = o.batch_stride; p.term_stride = o.term_stride;
   p.bias = o.bias; p.bias_n = o.bias_n; p.relu = o.relu; p.sigmoid_col0 = o.sigmoid_col0; p.sigmoid_col1 = o.sigmoid_col1;
+  p.pieces = o.pieces; p.gate = o.gate; p.pair_bias = o.pair_bias; p.bias_q = o.bias_q; p.bias_ld = o.bias_ld; p.bias_swap = o.bias_swap;
   p.status = (Status*)ctx->tc_status;
   const int64_t tiles = (int64_t)batch * ((m + G3_BM - 1) / G3_BM) * ((n + G3_BN - 1) / G3_BN);
   const int grid = (int)(tiles < ctx->sm_count ? tiles : ctx->sm_count);
   lf_prof_begin(ctx, LF_KERNEL_SIMT);
-  if (major == 0) lf_launch(ctx, gemm3_kernel<0>, grid, G3_THREADS, G3_SMEM, ma, mb, p);
-  else lf_launch(ctx, gemm3_kernel<1>, grid, G3_THREADS, G3_SMEM, ma, mb, p);
+  if (a.pieces) lf_launch(ctx, gemm3_kernel<0, true>, grid, G3_THREADS, G3_SMEM, ma, mb, p);
+  else if (major == 0) lf_launch(ctx, gemm3_kernel<0, false>, grid, G3_THREADS, G3_SMEM, ma, mb, p);
+  else lf_launch(ctx, gemm3_kernel<1, false>, grid, G3_THREADS, G3_SMEM, ma, mb, p);
   lf_prof_end(ctx);
   ctx->launches++;
   return LF_OK;

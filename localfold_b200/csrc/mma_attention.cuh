@@ -1,6 +1,7 @@
 // Gated float32 attention core for any head width, its products on the tensor cores: every operand is taken apart into three
 // bf16 terms (8 + 8 + 8 significand bits, so nothing of it is lost) and a product into the six term products above 2^-24,
-// accumulated in float32.  Float32 mode, and 16-bit mode for the heads that the tcgen05 core does not take.
+// accumulated in float32.  Float32 mode, and 16-bit mode for the heads that the tcgen05 core does not take; few logits, and the head widths that
+// f32_attention.cu does not have.
 #pragma once
 
 #include "common.cuh"
@@ -76,8 +77,9 @@ struct AttentionShape {
   int batch, Q, heads;
   int transpose, mask_mode, clamp;      // mask_mode 0: logit += 1e9 (m - 1); 1: logit += m > 0 ? 0 : -1e9
   float scale;
-  int64_t ld, term_stride;              // rows and terms of q | k | v | gate, in elements (multiples of 8)
-  int64_t ldo, out_stride;              // ... and of the output
+  int64_t rows, term_stride;            // rows and terms of q | k | v in pieces of eight channels: [3][channels / 8][rows][8]
+  int ldb;                              // rows of the bias
+  int64_t out_stride;                   // terms of the output
   int wb, wq;                           // warps of a block: wb batch rows x wq groups of 16 queries
   int kt;                               // keys of a staged tile, a multiple of 32
   int mk;                               // keys whose mask terms are held at a time, a multiple of kt
@@ -90,10 +92,10 @@ __host__ __device__ constexpr size_t attention_smem(int D, int wb, int kt, int m
   return (size_t)wb * (2 * 2 * AT_TERMS * kt * at_pitch(D) * 2 + mk * 4);
 }
 
-//   qkvg: [3][rows][ld] = terms of (q | k | v | sigmoid(gate) | ...) in logical row order, a head of each D channels wide
-//         (the projection's weights are padded to the instance's width, so nothing here is conditional on the true one)
-//   bias: float32 [H][Q][Q] or null; mask: indexed b * Q + j, or j * batch + b when transpose
-//   out:  [3][rows][ldo] = softmax(.) v * gate as terms, the operand of the output projection
+//   qkv: terms of (q | k | v) in pieces and logical row order, a head of each D channels wide, gate: sigmoid(gate) likewise in
+//        float32 (the projection's weights are padded to the instance's width, so nothing here is conditional on the true one)
+//   bias: float32 [H][Q][ldb] or null; mask: indexed b * Q + j, or j * batch + b when transpose
+//   out:  softmax(.) v * gate as terms in pieces, the operand of the output projection
 // A warp owns 16 queries of one (batch row, head); Q and the running output stay in registers in the tensor core's
 // fragment layout, and probabilities become the A operand of P V without leaving them.  The warps of a block share K and
 // V tiles of kt keys, copied a tile ahead as the projection wrote them, and step through them 32 keys at a time; mask terms
@@ -107,7 +109,7 @@ __host__ __device__ constexpr size_t attention_smem(int D, int wb, int kt, int m
 // four queries a thread on packed FMAs; 203 x 203, 4 x 32: 0.19 ms against 0.98 and 0.24.
 template <int D, bool BIAS>
 __global__ void __launch_bounds__(256, D > 32 ? 1 : 2)
-attention_kernel(const uint16_t* __restrict__ qkvg, const float* __restrict__ bias, const float* __restrict__ mask, const AttentionShape s,
+attention_kernel(const uint16_t* __restrict__ qkv, const float* __restrict__ gates, const float* __restrict__ bias, const float* __restrict__ mask, const AttentionShape s,
                  uint16_t* __restrict__ out) {
   lf_chain();
   constexpr int TERMS = AT_TERMS, TOP = TERMS - 1;                    // highest order of a term product that is kept: i + j <= TOP
@@ -117,7 +119,7 @@ attention_kernel(const uint16_t* __restrict__ qkvg, const float* __restrict__ bi
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, g = lane >> 2, t = lane & 3;
   const int wb = warp / s.wq, wq = warp % s.wq;
   const int Q = s.Q, HD = s.heads * D;
-  const int64_t ld = s.ld;
+  const int64_t piece = s.rows * 8;
   const int h = blockIdx.z, b0 = blockIdx.y * s.wb, b = b0 + wb;
   const int q0 = (blockIdx.x * s.wq + wq) * 16;
   // [2 buffers][wb][K: TERMS | V: TERMS][kt][PITCH], then [wb][mk] mask terms
@@ -133,13 +135,13 @@ attention_kernel(const uint16_t* __restrict__ qkvg, const float* __restrict__ bi
       const int e = (u % ND) * 8, j = u / ND;
       for (int bb = 0; bb < s.wb; ++bb) {
         const bool ok = j0 + j < Q && b0 + bb < s.batch;
-        const uint16_t* src = ok ? qkvg + ((int64_t)(b0 + bb) * Q + j0 + j) * ld + HD + h * D + e : qkvg;
+        const uint16_t* src = ok ? qkv + (HD + h * D + e) / 8 * piece + ((int64_t)(b0 + bb) * Q + j0 + j) * 8 : qkv;
         uint16_t* dst = kv_s + (buf * s.wb + bb) * 2 * TERMS * plane + j * PITCH + e;
 #pragma unroll
         for (int which = 0; which < 2; ++which)
 #pragma unroll
           for (int i = 0; i < TERMS; ++i)
-            copy_async16(dst + (which * TERMS + i) * plane, ok ? src + which * HD + i * s.term_stride : src, ok ? 16 : 0);
+            copy_async16(dst + (which * TERMS + i) * plane, ok ? src + which * (HD / 8) * piece + i * s.term_stride : src, ok ? 16 : 0);
       }
     }
     copy_async_commit();
@@ -161,7 +163,7 @@ attention_kernel(const uint16_t* __restrict__ qkvg, const float* __restrict__ bi
   uint32_t qa[TERMS][NK > 0 ? NK : 1][4], qt[TERMS][2];      // qt: the last 8 channels of an odd number of them
   const int row0 = q0 + g, row1 = q0 + g + 8;
   auto q_pair = [&](int row, int term, int e) {
-    return active && row < Q ? *reinterpret_cast<const uint32_t*>(qkvg + term * s.term_stride + ((int64_t)b * Q + row) * ld + h * D + e) : 0u;
+    return active && row < Q ? *reinterpret_cast<const uint32_t*>(qkv + term * s.term_stride + (h * D + e) / 8 * piece + ((int64_t)b * Q + row) * 8 + (e & 7)) : 0u;
   };
 #pragma unroll
   for (int i = 0; i < TERMS; ++i) {
@@ -176,16 +178,16 @@ attention_kernel(const uint16_t* __restrict__ qkvg, const float* __restrict__ bi
   }
 
   // the bias of a tile's keys: this thread's two rows, eight columns each
-  const bool pairs = (Q & 1) == 0;
-  const float* bias0 = BIAS ? bias + ((int64_t)h * Q + (row0 < Q ? row0 : 0)) * Q + 2 * t : nullptr;
-  const float* bias1 = BIAS ? bias + ((int64_t)h * Q + (row1 < Q ? row1 : 0)) * Q + 2 * t : nullptr;
+  const bool pairs = (s.ldb & 1) == 0;
+  const float* bias0 = BIAS ? bias + ((int64_t)h * Q + (row0 < Q ? row0 : 0)) * s.ldb + 2 * t : nullptr;
+  const float* bias1 = BIAS ? bias + ((int64_t)h * Q + (row1 < Q ? row1 : 0)) * s.ldb + 2 * t : nullptr;
   float bv[4][4];
   auto load_bias = [&](int j0) {
     if (!BIAS) return;
 #pragma unroll
     for (int n = 0; n < 4; ++n) {
       const int j = j0 + n * 8;
-      if (pairs && j + 2 * t < Q) {
+      if (pairs && j + 2 * t + 1 < Q) {
         const float2 x = __ldg(reinterpret_cast<const float2*>(bias0 + j)), y = __ldg(reinterpret_cast<const float2*>(bias1 + j));
         bv[n][0] = x.x; bv[n][1] = x.y; bv[n][2] = y.x; bv[n][3] = y.y;
       } else {
@@ -396,21 +398,15 @@ attention_kernel(const uint16_t* __restrict__ qkvg, const float* __restrict__ bi
     const int row = r ? row1 : row0;
     if (row >= Q) continue;
     const float inv = 1.0f / sum[r];
-    const uint16_t* gate = qkvg + ((int64_t)b * Q + row) * ld + 3 * HD + h * D + 2 * t;
-    uint16_t* dst = out + ((int64_t)b * Q + row) * s.ldo + h * D + 2 * t;
+    const float* gate = gates + h * D / 8 * piece + ((int64_t)b * Q + row) * 8 + 2 * t;
+    uint16_t* dst = out + h * D / 8 * piece + ((int64_t)b * Q + row) * 8 + 2 * t;
 #pragma unroll
     for (int n = 0; n < ND; ++n) {
-      float gx = 0.f, gy = 0.f;
-#pragma unroll
-      for (int i = 2; i >= 0; --i) {
-        const uint32_t w = *reinterpret_cast<const uint32_t*>(gate + i * s.term_stride + n * 8);
-        gx += __uint_as_float(w << 16);
-        gy += __uint_as_float(w & 0xffff0000u);
-      }
+      const float2 gv = __ldg(reinterpret_cast<const float2*>(gate + n * piece));
       uint32_t term[3];
-      split3(o[n][2 * r] * inv * gx, o[n][2 * r + 1] * inv * gy, term);
+      split3(o[n][2 * r] * inv * gv.x, o[n][2 * r + 1] * inv * gv.y, term);
 #pragma unroll
-      for (int i = 0; i < 3; ++i) *reinterpret_cast<uint32_t*>(dst + i * s.out_stride + n * 8) = term[i];
+      for (int i = 0; i < 3; ++i) *reinterpret_cast<uint32_t*>(dst + i * s.out_stride + n * piece) = term[i];
     }
   }
 }

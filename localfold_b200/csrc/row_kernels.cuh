@@ -417,16 +417,6 @@ __global__ void finish4_kernel(const float* __restrict__ proj, const float* __re
   store4(out + dst * ch + c, v);
 }
 
-// columns col0 .. col0 + heads of rows (i * Q + j) of a terms matrix -> bias[h][i][j], or [h][j][i] when `swap`
-__global__ void bias_columns_kernel(const bf16* __restrict__ in, int64_t ld, int64_t term_stride, int col0, int Q, int heads, int swap, float* __restrict__ out) {
-  lf_chain();
-  const int64_t idx = (int64_t)blockIdx.x * blockDim.x + threadIdx.x, pairs = (int64_t)Q * Q;
-  if (idx >= pairs) return;
-  const uint32_t i = (uint32_t)idx / (uint32_t)Q, j = (uint32_t)idx % (uint32_t)Q;
-  const bf16* row = in + (swap ? (int64_t)j * Q + i : idx) * ld + col0;      // thread order follows the destination
-  for (int h = 0; h < heads; ++h) out[h * pairs + idx] = to_f(row[h]) + (to_f(row[h + term_stride]) + to_f(row[h + 2 * term_stride]));
-}
-
 // ---- AF3 MSA pair-weighted averaging: the weights do not depend on the sequence, so they are made once and the averages
 // of all sequences are one GEMM per head ----
 

@@ -173,13 +173,13 @@ __global__ void finish_kernel(const float* __restrict__ proj, const float* __res
 }
 
 // ---------------------------------------------------------------------------
-// Pair bias: out[h][dst(p)] = LN(pair[p,:]) . W[:,h] for p = i*Q + j, dst = j*Q+i if swap.
+// Pair bias: out[h][i][j] = LN(pair[p,:]) . W[:,h] for p = i*Q + j, [h][j][i] if swap; rows of ldo.
 // One warp per pair row.
 template <typename TIn>
 __global__ void pair_bias_kernel(const TIn* __restrict__ pair, int Q, int ch, int heads,
                                  const float* __restrict__ gamma, const float* __restrict__ beta,
                                  const float* __restrict__ w, float eps, int variance, int swap,
-                                 float* __restrict__ out) {
+                                 float* __restrict__ out, int ldo) {
   lf_chain();
   int lane = threadIdx.x & 31;
   int64_t pairs = (int64_t)Q * Q;
@@ -199,15 +199,14 @@ __global__ void pair_bias_kernel(const TIn* __restrict__ pair, int Q, int ch, in
   }
   float inv = rsqrtf(var + eps);
   inv = inv * (1.5f - 0.5f * (var + eps) * inv * inv);
-  int64_t dst = p;
-  if (swap) { int64_t i = p / Q, j = p % Q; dst = j * Q + i; }
+  const int64_t i = p / Q, j = p % Q, dst = swap ? j * ldo + i : i * ldo + j;
   for (int h = 0; h < heads; ++h) {
     float acc = 0.f;
     for (int c = lane; c < ch; c += 32) {
       acc = fmaf((to_f(x[c]) - mean) * inv * gamma[c] + beta[c], w[c * heads + h], acc);
     }
     acc = warp_sum(acc);
-    if (lane == 0) out[(int64_t)h * pairs + dst] = acc;
+    if (lane == 0) out[(int64_t)h * Q * ldo + dst] = acc;
   }
 }
 
@@ -236,15 +235,15 @@ __global__ void finish_half_kernel(const __half* __restrict__ proj, float scale,
   add_store8<TAct>(v, rs, o);
 }
 
-// fp16 pair bias [heads][Q][ld] (rows padded to ld) -> float32 [heads][Q][Q]
-__global__ void widen_bias_kernel(const __half* __restrict__ in, int heads, int Q, int ld, float* __restrict__ out) {
+// fp16 pair bias [heads][Q][ld] (rows padded to ld) -> float32 [heads][Q][ldo]
+__global__ void widen_bias_kernel(const __half* __restrict__ in, int heads, int Q, int ld, float* __restrict__ out, int ldo) {
   lf_chain();
   int64_t idx = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   int64_t total = (int64_t)heads * Q * Q;
   if (idx >= total) return;
   int k = (int)(idx % Q);
   int64_t hq = idx / Q;
-  out[idx] = __half2float(in[hq * ld + k]);
+  out[hq * ldo + k] = __half2float(in[hq * ld + k]);
 }
 
 // out[i][j][b] = half[i][j][b] + half[j][i][b]: a sum over the two token orders, not a mean.

@@ -71,6 +71,21 @@ lf_status make_map_terms(lf_context* ctx, CUtensorMap* map, const SplitMatrix& a
   return LF_OK;
 }
 
+// Terms in pieces of eight columns over rows (batch, Q), seen as (8-byte halves of a row's piece, batch row, piece, term): as 8-byte elements, 128 rows
+// fit a box, and what lies past the end of a batch row arrives as zeros.  Boxes of `rows` rows of `batch_rows` batch rows, `pieces` and `terms`.
+lf_status make_map_term_pieces(lf_context* ctx, CUtensorMap* map, const SplitMatrix& a, int Q, int batch, uint32_t rows, uint32_t batch_rows,
+                               uint32_t pieces, uint32_t terms) {
+  if (!g_encode) return lf_fail(ctx, LF_ERR_CUDA, "cuTensorMapEncodeTiled is not available from this driver");
+  cuuint64_t dims[4] = {(cuuint64_t)Q * 2, (cuuint64_t)batch, (cuuint64_t)a.ld / 8, 3};
+  cuuint64_t strides[3] = {(cuuint64_t)Q * 16, (cuuint64_t)batch * Q * 16, (cuuint64_t)a.term_stride * 2};
+  cuuint32_t box[4] = {rows * 2, batch_rows, pieces, terms};
+  cuuint32_t estr[4] = {1, 1, 1, 1};
+  CUresult r = g_encode(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT64, 4, const_cast<bf16*>(a.p), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
+                        CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+  if (r != CUDA_SUCCESS) return lf_fail(ctx, LF_ERR_CUDA, "cuTensorMapEncodeTiled (term pieces) failed with code %d", (int)r);
+  return LF_OK;
+}
+
 // float32 rows of 128 channels seen as (channel, d1, d2); boxes of 32 channels (one 128-byte swizzled row) x b1 x b2
 lf_status make_map_f32_rows(lf_context* ctx, CUtensorMap* map, const void* base, uint64_t d1, uint64_t d2, uint64_t stride1_bytes,
                             uint64_t stride2_bytes, uint32_t b1, uint32_t b2) {

@@ -19,7 +19,8 @@ lf_status prepare_weights(lf_context* ctx, lf_weights* w, WeightCursor& cur);
 lf_status check_status(lf_context* ctx);
 
 // Float32 GEMM on the tensor cores (f32_gemm.cu), batched: out[b][i][j] = act(sum_k A(b, i, k) B(b, j, k) + bias[j]), both operands
-// as bf16 terms; major 0: k contiguous (A [m][ld], B [n][ld]); major 1: the row index contiguous (A [k][ld], B [k][ld]).
+// as bf16 terms; major 0: k contiguous (A [m][ld], or in pieces of eight columns over m rows when a.pieces, B [n][ld]); major 1: the row index
+// contiguous (A [k][ld], B [k][ld]).
 struct Gemm3Out {
   float* out;                  // float32 result, or null:
   bf16* terms;                 // its terms (ld a multiple of 8)
@@ -27,11 +28,24 @@ struct Gemm3Out {
   const float* bias;           // or null; columns from bias_n on have none
   int bias_n, relu;
   int sigmoid_col0, sigmoid_col1;      // columns through a sigmoid (empty range: none)
+  // Terms in pieces of eight columns, [3][ld / 8][m][8] (element (t, i, j) at t * term_stride + (j / 8) * m * 8 + i * 8 + j % 8), what
+  // the attention cores read.  Columns from ld on (a multiple of 8; the projection has ld / 3 of them) are the gate then, float32 pieces [ld / 24][m][8]; the ones behind
+  // a pair bias, row i * bias_q + j -> float32 pair_bias[column][i][bias_ld] at j, or [j] at i when bias_swap.
+  int pieces = 0;
+  float* gate = nullptr;
+  float* pair_bias = nullptr;
+  int bias_q = 0, bias_ld = 0, bias_swap = 0;
 };
 void configure_gemm3();
 lf_status gemm_f32(lf_context* ctx, ArenaCursor& cur, int major, const SplitMatrix& a, const SplitMatrix& b, int m, int n, int k, int batch,
                    const Gemm3Out& o);
-// The weights' operands of it (lf_f32_operands), into their room or block; as few launches as the jobs of all of them fit into.
+// Attention core on split operands (f32_attention.cu): qkv = the terms of q | k | v in pieces over rows (batch, Q), heads of D channels, gate = sigmoid(gate) likewise in float32;
+// bias float32 [heads][Q][ldb] (ldb a multiple of 4) or null; out = terms in pieces.
+void configure_attention3();
+bool attention3_wins(const lf_context* ctx, int D, int batch, int Q, int heads);      // over mma_attention.cuh
+lf_status attention3(lf_context* ctx, ArenaCursor& cur, int D, const SplitMatrix& qkv, const float* gate, const float* bias, int ldb, const float* mask, int batch,
+                     int Q, int heads, int transpose, int mask_mode, int clamp, float scale, const SplitMatrix& out);
+// The weights' operands of the float32 GEMM (lf_f32_operands), into their room or block; as few launches as the jobs of all of them fit into.
 lf_status prepare_f32_operands(lf_context* ctx, const lf_weights* const* w, int count);
 
 // Triangle contraction, batched over the c channels of channel-major fp16

@@ -1,0 +1,81 @@
+"""The float32 attention core on tcgen05 (heads of 8, 16 and 32 channels, enough logits to pay): query counts around the tiles of 128 queries and
+32 keys, batch rows that do not fill a group of four, more items than blocks, both orientations, rows whose reference has to be
+raised, fully masked rows; and that what is not finite stays in its batch row.
+
+The bound is the float32 mode's: logits of size 100 come with errors of 100 x 2^-24 x a few, which the exponentials pass on; with
+weights of the usual size the error is below 5e-7."""
+import numpy as np
+import pytest
+
+from localfold_b200 import synthetic as syn
+from oracle import tier2_torch as t2
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(scope="module")
+def dev():
+    import localfold_b200 as lf
+    d = lf.Device(0)
+    yield d
+    d.close()
+
+
+def _relative(got, want):
+    got, want = np.asarray(got, np.float64), np.asarray(want, np.float64)
+    return np.linalg.norm(got - want) / np.linalg.norm(want)
+
+
+def _case(q, batch, heads, dim, transpose, bias, big=1):
+    d = syn.draw(6000 + q)
+    c = heads * dim
+    act = d.normal(batch * q, c)
+    mask = (d.rng.random((q, batch) if transpose else (batch, q)) > 0.25).astype(np.float32)
+    w = syn.af2_attention_weights(d, c, heads, 32, separate=True)
+    att = dict(w["attention"], queryWeight=w["attention"]["queryWeight"] * big, keyWeight=w["attention"]["keyWeight"] * big)
+    pb = None
+    if bias:
+        pb = dict(w["pairBias"], source="separate", channels=32, activations=d.normal(q, q, 32))
+        pb["projectionWeight"] = pb["projectionWeight"] * (big + 2)
+    return {"activations": act, "mask": mask, "batch": batch, "queryLength": q, "channels": c, "heads": heads, "weights": att, "transpose": transpose,
+            "pairBias": pb}
+
+
+def _want(g):
+    return t2.attention_af2(g["activations"], g["mask"], g["batch"], g["queryLength"], g["channels"], g["heads"], g["weights"], g["transpose"], g["pairBias"])
+
+
+# every one of these goes to the tcgen05 kernel (attention3_wins)
+SIZES = [(94, 131, 4, 16, False, True), (96, 97, 4, 32, True, True), (97, 99, 4, 32, False, False), (127, 130, 4, 16, True, False), (128, 66, 4, 32, False, True),
+         (200, 129, 8, 8, False, True), (160, 131, 8, 8, True, False), (203, 40, 4, 32, True, True), (256, 70, 8, 16, False, True), (385, 41, 4, 16, True, True)]
+
+
+@pytest.mark.parametrize("q,batch,heads,dim,transpose,bias", SIZES)
+def test_attention_core_edges(dev, q, batch, heads, dim, transpose, bias):
+    import localfold_b200 as lf
+    given = _case(q, batch, heads, dim, transpose, bias)
+    got = lf.AttentionGpu(dev).run(given, {"precision": "f32", "variance": "two-pass"})["output"]
+    assert _relative(got, _want(given)) <= 1e-6
+
+
+@pytest.mark.parametrize("q,batch,heads,dim,transpose,bias", [SIZES[1], SIZES[3], SIZES[5], SIZES[9]])
+def test_raised_references_and_masked_rows(dev, q, batch, heads, dim, transpose, bias):
+    import localfold_b200 as lf
+    given = _case(q, batch, heads, dim, transpose, bias, big=6)
+    by_row = given["mask"].T if transpose else given["mask"]
+    by_row[0, :40] = 0           # the first tile of a row is masked: its reference is raised from near -1e9
+    by_row[1] = 0                # no key is left
+    by_row[2, 33:] = 0
+    got = lf.AttentionGpu(dev).run(given, {"precision": "f32", "variance": "two-pass"})["output"]
+    assert np.isfinite(got).all()
+    assert _relative(got, _want(given)) <= 1e-5
+
+
+def test_what_is_not_finite_stays_in_its_row(dev):
+    import localfold_b200 as lf
+    given = _case(97, 99, 4, 32, False, False)
+    clean = lf.AttentionGpu(dev).run(given, {"precision": "f32"})["output"].reshape(99, 97, -1)
+    given["activations"].reshape(99, 97, -1)[6, 96] = np.inf      # a row between others of its group, the key a partial tile ends on
+    got = lf.AttentionGpu(dev).run(given, {"precision": "f32"})["output"].reshape(99, 97, -1)
+    rest = np.arange(99) != 6
+    assert np.isnan(got[6]).any() and np.array_equal(got[rest], clean[rest])
