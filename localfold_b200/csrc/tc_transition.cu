@@ -46,11 +46,6 @@ __device__ __forceinline__ float sigmoid_tanh(float v) {   // one MUFU: 0.5 + 0.
   return fmaf(0.5f, t, 0.5f);
 }
 
-__device__ __forceinline__ void bulk_load(void* dst, const void* src, uint32_t bytes, uint64_t* bar) {
-  asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(smem_u32(dst)),
-               "l"(reinterpret_cast<uint64_t>(src)), "r"(bytes), "r"(smem_u32(bar))
-               : "memory");
-}
 
 template <bool SWIGLU>
 __global__ void __launch_bounds__(TR_THREADS, 1) transition_kernel(const __grid_constant__ CUtensorMap mapO, const TransitionParams p) {
