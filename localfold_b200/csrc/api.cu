@@ -1050,13 +1050,28 @@ void layer_norm(lf_context* ctx, ArenaCursor& cur, const void* act, int64_t coun
 #undef LN_CASE
 }
 
+// The end of an operator: out[dst(r)] = (resid ? resid[dst(r)] : 0) + (a w^T + bias)[r] * (factor ? factor[r] : 1) over `count` rows of c channels, a [count][k];
+// transposed_q: rows (b, q) go to row q * batch + b.  Float32 activations updated in place, or written without a residual, by the GEMM
+// itself; others (bfloat16, another buffer's residual, broken alignment) by a pass of their own behind it.
 template <typename T>
-void finish(lf_context* ctx, ArenaCursor& cur, const float* proj, const float* gate, const void* resid, int64_t count, int c, int transpose, int batch,
-            int Q, void* out) {
+lf_status finish(lf_context* ctx, ArenaCursor& cur, const SplitMatrix& a, const SplitMatrix& w, int64_t count, int c, int k, const float* bias, const float* factor,
+                 const T* resid, T* out, int batch = 1, int transposed_q = 0) {
+  // (a plan does not know the addresses: it has room for the pass)
+  if (!cur.dry && sizeof(T) == 4 && (!resid || resid == out) && (c & 3) == 0 && lf_aligned16(out)) {
+    tc::Gemm3Out to{nullptr, nullptr, c, 0, 0, bias, c, 0, 0, 0};
+    to.act = (float*)out; to.act_add = resid != nullptr; to.factor = factor; to.act_batch = batch; to.act_q = transposed_q;
+    return tc::gemm_f32(ctx, cur, 0, a, w, (int)count, c, k, 1, to);
+  }
+  const size_t end = cur.offset;
+  float* proj = cur.take<float>(count * c);
+  LF_TRY(tc::gemm_f32(ctx, cur, 0, a, w, (int)count, c, k, 1, {proj, nullptr, c, 0, 0, bias, c, 0, 0, 0}));
+  const int transpose = transposed_q != 0;
   if ((c & 3) == 0 && lf_aligned16(resid) && lf_aligned16(out) && count < ((int64_t)1 << 32))
-    LAUNCH(ctx, cur, (rows::finish4_kernel<T>), lf_ceil_div(count * (c / 4), 256), 256, 0, proj, gate, (const T*)resid, count, c, transpose, batch, Q, (T*)out);
+    LAUNCH(ctx, cur, (rows::finish4_kernel<T>), lf_ceil_div(count * (c / 4), 256), 256, 0, proj, factor, resid, count, c, transpose, batch, transposed_q, out);
   else
-    LAUNCH(ctx, cur, (simt::finish_kernel<T>), lf_ceil_div(count * c, 256), 256, 0, proj, gate, (const T*)resid, count, c, transpose, batch, Q, (T*)out);
+    LAUNCH(ctx, cur, (simt::finish_kernel<T>), lf_ceil_div(count * c, 256), 256, 0, proj, factor, resid, count, c, transpose, batch, transposed_q, out);
+  cur.offset = end;
+  return LF_OK;
 }
 
 // A terms matrix of `count` rows of c (rows of whole groups of eight) out of the arena.
@@ -1150,11 +1165,13 @@ lf_status tri_general(lf_context* ctx, ArenaCursor& cur, const TriArgs& a, bool 
   const SplitMatrix zn = take_terms(cur, P, cz);
   const int ld = half ? (n + 15) / 16 * 16 : (n + 7) / 8 * 8, ldx = half ? ld : (n + 3) / 4 * 4;
   const int64_t plane = (int64_t)n * ld;
-  const size_t base = cur.offset;
-  float* p4 = cur.take<float>(P * 4 * c);
-  const size_t p4_end = cur.offset;
   layer_norm<T, rows::LN_TERMS>(ctx, cur, a.z, P, cz, f[TRI_LN_G], f[TRI_LN_B], a.eps, a.variance, 0, 1, 1, (void*)zn.p, zn.term_stride);
-  LF_TRY(tc::gemm_f32(ctx, cur, 0, zn, g[0], (int)P, 4 * c, cz, 1, {p4, nullptr, 4 * c, 0, 0, f[TRI_B4], 4 * c, 0, 0, 0}));
+  // mask (projection) sigmoid(gate) straight into the planes
+  auto project = [&](void* to_a, void* to_b, int64_t term_stride) {
+    tc::Gemm3Out to{nullptr, nullptr, ld, 0, term_stride, f[TRI_B4], 0, 0, 0, 0};
+    to.plane_mask = a.mask; to.plane[0] = to_a; to.plane[1] = to_b; to.plane_n = n; to.plane_c = c; to.plane_half = half;
+    return tc::gemm_f32(ctx, cur, 0, zn, g[0], (int)P, tc::gated_columns(c), cz, 1, to);
+  };
   op16* xh = nullptr;
   float* xf = nullptr;
   const float xscale = half ? contraction_scale(n) : 1.0f;
@@ -1162,7 +1179,7 @@ lf_status tri_general(lf_context* ctx, ArenaCursor& cur, const TriArgs& a, bool 
     op16* ga = cur.take<op16>(plane * c);
     op16* gb = cur.take<op16>(plane * c);
     xh = cur.take<op16>(plane * c);
-    LAUNCH(ctx, cur, rows::trimul_gate_half_kernel, dim3((unsigned)(n * lf_ceil_div(n, 64)), lf_ceil_div(c, 32)), 256, 0, p4, a.mask, c, n, ld, ga, gb);
+    LF_TRY(project(ga, gb, 0));
     LF_TRY(tc::contract(ctx, cur, ga, gb, xh, n, ld, c, a.incoming, xscale));
   } else {
     SplitMatrix ga, gb;
@@ -1172,25 +1189,14 @@ lf_status tri_general(lf_context* ctx, ArenaCursor& cur, const TriArgs& a, bool 
     ga.p = cur.take<bf16>(3 * plane * c);
     gb.p = cur.take<bf16>(3 * plane * c);
     xf = cur.take<float>((int64_t)n * ldx * c);
-    LAUNCH(ctx, cur, rows::trimul_gate_terms_kernel, dim3((unsigned)(n * lf_ceil_div(n, 32)), lf_ceil_div(c, 32)), 256, 0, p4, a.mask, c, n, ld, (bf16*)ga.p,
-           (bf16*)gb.p, ga.term_stride);
+    LF_TRY(project((void*)ga.p, (void*)gb.p, ga.term_stride));
     // outgoing x[i][j] = sum_k a[i][k] b[j][k]; incoming x[i][j] = sum_k b[k][i] a[k][j]
     const tc::Gemm3Out to{xf, nullptr, ldx, (int64_t)n * ldx, 0, nullptr, 0, 0, 0, 0};
     if (!a.incoming) LF_TRY(tc::gemm_f32(ctx, cur, 0, ga, gb, n, n, n, c, to));
     else LF_TRY(tc::gemm_f32(ctx, cur, 1, gb, ga, n, n, n, c, to));
   }
-  // p4 is dead: the normalised x and the two outputs take its place where they fit
-  const size_t end = cur.offset;
-  cur.offset = base;
-  SplitMatrix xn = take_terms(cur, P, c);
-  float* proj = cur.take<float>(P * cz);
+  const SplitMatrix xn = take_terms(cur, P, c);
   float* gate = cur.take<float>(P * cz);
-  if (cur.offset > p4_end) {
-    cur.offset = end;
-    xn = take_terms(cur, P, c);
-    proj = cur.take<float>(P * cz);
-    gate = cur.take<float>(P * cz);
-  } else cur.offset = end;
   const float center_scale = (a.divide ? 1.0f / n : 1.0f) / xscale;
   const unsigned tiles = (unsigned)(n * lf_ceil_div(n, 32)), half_tiles = (unsigned)(n * lf_ceil_div(n, 64));
 #define CENTER_HALF(G_)                                                                                                                              \
@@ -1206,10 +1212,8 @@ lf_status tri_general(lf_context* ctx, ArenaCursor& cur, const TriArgs& a, bool 
     LAUNCH(ctx, cur, (rows::center_norm_kernel<float>), tiles, 256, (size_t)c * 33 * sizeof(float), xf, c, n, ldx, f[TRI_LNO_G], f[TRI_LNO_B], a.eps, a.variance,
            center_scale, (int)xn.ld, (bf16*)xn.p, xn.term_stride);
 #undef CENTER_HALF
-  LF_TRY(tc::gemm_f32(ctx, cur, 0, xn, g[1], (int)P, cz, c, 1, {proj, nullptr, cz, 0, 0, f[TRI_BZ], cz, 0, 0, 0}));
-  LF_TRY(tc::gemm_f32(ctx, cur, 0, zn, g[2], (int)P, cz, cz, 1, {gate, nullptr, cz, 0, 0, f[TRI_BG], cz, 0, 0, 0}));
-  finish<T>(ctx, cur, proj, gate, a.residual ? a.z : nullptr, P, cz, 0, 1, 1, a.out);
-  return LF_OK;
+  LF_TRY(tc::gemm_f32(ctx, cur, 0, zn, g[2], (int)P, cz, cz, 1, {gate, nullptr, cz, 0, 0, f[TRI_BG], cz, 0, 0, cz}));
+  return finish<T>(ctx, cur, xn, g[1], P, cz, c, f[TRI_BZ], gate, a.residual ? (const T*)a.z : nullptr, (T*)a.out);
 }
 
 // 16-bit path at 128 channels: fp16 operands a, b, x, float32 LayerNorm statistics and gates, everything on the fused kernels.
@@ -1287,7 +1291,6 @@ lf_status att_f32(lf_context* ctx, ArenaCursor& cur, const AttArgs& a) {
   float* bias = a.bias_mode ? cur.take<float>((int64_t)a.heads * a.Q * ldb) : nullptr;
   SplitMatrix o = take_terms(cur, R, HDp);
   o.pieces = true;
-  float* proj = cur.take<float>(R * c);
   layer_norm<T, rows::LN_TERMS>(ctx, cur, a.act, R, c, f[ATT_LN_G], f[ATT_LN_B], a.eps, a.variance, a.transpose, a.batch, a.Q, (void*)nrm.p, nrm.term_stride);
   LF_TRY(tc::gemm_f32(ctx, cur, 0, nrm, g[0], (int)R, wide, c, 1,
                       {nullptr, (bf16*)qkv.p, qkv.ld, 0, qkv.term_stride, reinterpret_cast<const float*>(g[2].p), 4 * HDp, 0, 3 * HDp, 4 * HDp, 1,
@@ -1298,9 +1301,7 @@ lf_status att_f32(lf_context* ctx, ArenaCursor& cur, const AttArgs& a) {
     LF_TRY(tc::attention3(ctx, cur, D, qkv, gate, bias, ldb, a.mask, a.batch, a.Q, a.heads, a.transpose, a.mask_mode, a.clamp, scale, o));
   else
     mma_attention_core(ctx, cur, D, qkv, gate, bias, a.mask, {a.batch, a.Q, a.heads, a.transpose, a.mask_mode, a.clamp, scale, R, qkv.term_stride, ldb}, o);
-  LF_TRY(tc::gemm_f32(ctx, cur, 0, o, g[1], (int)R, c, HDp, 1, {proj, nullptr, c, 0, 0, f[ATT_BO], c, 0, 0, 0}));
-  finish<T>(ctx, cur, proj, nullptr, a.residual ? a.act : nullptr, R, c, a.transpose, a.batch, a.Q, a.out);
-  return LF_OK;
+  return finish<T>(ctx, cur, o, g[1], R, c, HDp, f[ATT_BO], nullptr, a.residual ? (const T*)a.act : nullptr, (T*)a.out, a.batch, a.transpose ? a.Q : 0);
 }
 
 // AF3 MSA pair-weighted averaging (no query, no key): the weights are the softmax of the pair bias under one key mask - a token
@@ -1330,7 +1331,6 @@ lf_status msa_average(lf_context* ctx, ArenaCursor& cur, const AttArgs& a) {
   const int64_t ldx = ((int64_t)S * d + 3) / 4 * 4;
   float* x = cur.take<float>((int64_t)H * n * ldx);
   const SplitMatrix o = take_terms(cur, R, HD);
-  float* proj = cur.take<float>(R * c);
   if ((int64_t)S * d > 0x7fffffff) return lf_fail(ctx, LF_ERR_SHAPE, "too many sequences for one average");
   LF_TRY(separate_bias(ctx, cur, a, bias, n));
   LAUNCH(ctx, cur, rows::key_mask_kernel, lf_ceil_div(n, 32), dim3(32, 32), 0, a.mask, S, n, key);
@@ -1341,9 +1341,7 @@ lf_status msa_average(lf_context* ctx, ArenaCursor& cur, const AttArgs& a) {
   LF_TRY(tc::gemm_f32(ctx, cur, 1, w, v, n, S * d, n, H, {x, nullptr, ldx, (int64_t)n * ldx, 0, nullptr, 0, 0, 0, 0}));
   LAUNCH(ctx, cur, rows::average_gate_kernel, lf_ceil_div(R * (o.ld / 2), 256), 256, 0, x, ldx, vg + HD, (int64_t)2 * HD, S, n, H, d, (int)o.ld, (bf16*)o.p,
          o.term_stride);
-  LF_TRY(tc::gemm_f32(ctx, cur, 0, o, g[1], (int)R, c, HD, 1, {proj, nullptr, c, 0, 0, f[ATT_BO], c, 0, 0, 0}));
-  finish<float>(ctx, cur, proj, nullptr, a.residual ? a.act : nullptr, R, c, 0, 1, 1, a.out);
-  return LF_OK;
+  return finish<float>(ctx, cur, o, g[1], R, c, HD, f[ATT_BO], nullptr, a.residual ? (const float*)a.act : nullptr, (float*)a.out);
 }
 
 // The padding the attention core reads (as keys past the end, masked out) must hold finite values.
@@ -1445,7 +1443,6 @@ lf_status trn_f32(lf_context* ctx, ArenaCursor& cur, const TrnArgs& a) {
   if (cur.dry) g = none; else LF_TRY(f32_operands(ctx, a.w, &g));
   const SplitMatrix nrm = take_terms(cur, chunk, c), hid = take_terms(cur, chunk, hd);
   float* h1 = a.swiglu ? cur.take<float>(chunk * wide) : nullptr;
-  float* proj = cur.take<float>(chunk * c);
   for (int64_t r0 = 0; r0 < a.rows; r0 += chunk) {
     const int64_t count = a.rows - r0 < chunk ? a.rows - r0 : chunk;
     const T* in = (const T*)a.act + r0 * c;
@@ -1457,8 +1454,7 @@ lf_status trn_f32(lf_context* ctx, ArenaCursor& cur, const TrnArgs& a) {
     } else {
       LF_TRY(tc::gemm_f32(ctx, cur, 0, nrm, g[0], (int)count, wide, c, 1, {nullptr, (bf16*)hid.p, hid.ld, 0, hid.term_stride, f[TRN_B1], wide, 1, 0, 0}));
     }
-    LF_TRY(tc::gemm_f32(ctx, cur, 0, hid, g[1], (int)count, c, hd, 1, {proj, nullptr, c, 0, 0, f[TRN_B2], c, 0, 0, 0}));
-    finish<T>(ctx, cur, proj, nullptr, a.residual ? in : (const T*)nullptr, count, c, 0, 1, 1, out);
+    LF_TRY(finish<T>(ctx, cur, hid, g[1], count, c, hd, f[TRN_B2], nullptr, a.residual ? in : (const T*)nullptr, out));
   }
   return LF_OK;
 }
@@ -1850,7 +1846,6 @@ lf_status global_attention(lf_context* ctx, ArenaCursor& cur, const lf_global_at
   float* sums = cur.take<float>((int64_t)n * (c + 1));
   float* q = cur.take<float>((int64_t)n * HD);
   float* attended = cur.take<float>((int64_t)n * HD);
-  float* proj = cur.take<float>(R * c);
   layer_norm<T, rows::LN_TERMS>(ctx, cur, act, R, c, f[GLB_LN_G], f[GLB_LN_B], d->epsilon, d->variance, 0, 1, 1, (void*)nrm.p, nrm.term_stride);
   LF_TRY(tc::gemm_f32(ctx, cur, 0, nrm, g[0], (int)R, wide, c, 1, {kvg, nullptr, ld, 0, 0, f[GLB_B3], wide, 0, 2 * hd, wide}));
   const bool wide_rows = c > 512;      // more channels than a lane keeps: the sums of the normalised rows, from their terms
@@ -1865,8 +1860,7 @@ lf_status global_attention(lf_context* ctx, ArenaCursor& cur, const lf_global_at
   const int per = lf_ceil_div((int64_t)n * (gated.ld / 4), 256);
   LAUNCH(ctx, cur, rows::global_gate_kernel, (unsigned)((int64_t)per * S), 256, 0, kvg, (int64_t)ld, 2 * hd, attended, per, n, HD, (int)gated.ld,
          (bf16*)gated.p, gated.term_stride);
-  LF_TRY(tc::gemm_f32(ctx, cur, 0, gated, g[1], (int)R, c, HD, 1, {proj, nullptr, c, 0, 0, f[GLB_BO], c, 0, 0, 0}));
-  finish<T>(ctx, cur, proj, nullptr, d->residual ? act : nullptr, R, c, 0, 1, 1, out);
+  LF_TRY(finish<T>(ctx, cur, gated, g[1], R, c, HD, f[GLB_BO], nullptr, d->residual ? (const T*)act : nullptr, (T*)out));
   return LF_OK;
 }
 }  // namespace

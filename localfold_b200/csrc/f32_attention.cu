@@ -570,12 +570,7 @@ attention3_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_constan
             const float4 g4 = gate[pc * 2 + (e >> 1)];
             float x = o[pc * 8 + 2 * e] * inv * (e & 1 ? g4.z : g4.x), y = o[pc * 8 + 2 * e + 1] * inv * (e & 1 ? g4.w : g4.y);
 #pragma unroll
-            for (int i = 0; i < 3; ++i) {
-              const __nv_bfloat162 b2 = __floats2bfloat162_rn(x, y);
-              w[i][e] = *reinterpret_cast<const uint32_t*>(&b2);
-              x -= __low2float(b2);
-              y -= __high2float(b2);
-            }
+            for (int i = 0; i < 3; ++i) w[i][e] = split_bf16(x, y);
           }
 #pragma unroll
           for (int i = 0; i < 3; ++i) *reinterpret_cast<uint4*>(dst + i * p.out_stride + pc * p.rows * 8) = make_uint4(w[i][0], w[i][1], w[i][2], w[i][3]);

@@ -198,88 +198,6 @@ __global__ void swiglu_half_kernel(const __half* __restrict__ wide, int64_t coun
   *reinterpret_cast<uint4*>(out + row * inter + c) = o;
 }
 
-// p4 rows (ap | ag | bp | bg) -> the contraction's operands a, b = mask * p * sigmoid(g) as terms, channel-major
-// [3][c][n][ld] (ld a multiple of 8; what lies past n is clipped by the tensor maps).  A block turns 32 pairs x 32
-// channels of one pair row round in shared memory.
-__global__ void __launch_bounds__(256)
-trimul_gate_terms_kernel(const float* __restrict__ p4, const float* __restrict__ mask, int c, int n, int ld, bf16* __restrict__ a,
-                         bf16* __restrict__ b, int64_t term_stride) {
-  lf_chain();
-  __shared__ float ta[32][33], tb[32][33];
-  const int tiles = (n + 31) / 32, i = blockIdx.x / tiles, k0 = (blockIdx.x % tiles) * 32, h0 = blockIdx.y * 32;
-  const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
-#pragma unroll
-  for (int r = ty; r < 32; r += 8) {
-    const int k = k0 + r, h = h0 + tx;
-    float va = 0.f, vb = 0.f;
-    if (k < n && h < c) {
-      const int64_t p = (int64_t)i * n + k;
-      const float* row = p4 + p * 4 * c;
-      const float m = mask[p];
-      va = row[h] * sigmoidf_(row[c + h]) * m;
-      vb = row[2 * c + h] * sigmoidf_(row[3 * c + h]) * m;
-    }
-    ta[r][tx] = va;
-    tb[r][tx] = vb;
-  }
-  __syncthreads();
-  // 16 threads a channel, two pairs each
-  const int k2 = (threadIdx.x & 15) * 2;
-#pragma unroll
-  for (int hh = threadIdx.x >> 4; hh < 32; hh += 16) {
-    const int h = h0 + hh;
-    if (h >= c || k0 + k2 >= ld) continue;
-    const int64_t o = ((int64_t)h * n + i) * ld + k0 + k2;
-    uint32_t t[3];
-    split_pair(ta[k2][hh], ta[k2 + 1][hh], t);
-#pragma unroll
-    for (int e = 0; e < 3; ++e) *reinterpret_cast<uint32_t*>(a + e * term_stride + o) = t[e];
-    split_pair(tb[k2][hh], tb[k2 + 1][hh], t);
-#pragma unroll
-    for (int e = 0; e < 3; ++e) *reinterpret_cast<uint32_t*>(b + e * term_stride + o) = t[e];
-  }
-}
-
-// ... as fp16 planes [c][n][ld] (c a multiple of 8, ld of 16; zeros past n): a block turns 64 pairs x 32 channels of one pair row
-// round in shared memory, a thread eight channels of a pair.
-__global__ void __launch_bounds__(256)
-trimul_gate_half_kernel(const float* __restrict__ p4, const float* __restrict__ mask, int c, int n, int ld, __half* __restrict__ a, __half* __restrict__ b) {
-  lf_chain();
-  __shared__ __align__(16) __half ta[32][72], tb[32][72];
-  const int tiles = (n + 63) / 64, i = blockIdx.x / tiles, k0 = (blockIdx.x % tiles) * 64, h0 = blockIdx.y * 32;
-  {
-    const int r = threadIdx.x >> 2, hg = (threadIdx.x & 3) * 8, k = k0 + r, h = h0 + hg;
-    if (k < n && h < c) {
-      const int64_t p = (int64_t)i * n + k;
-      const float* row = p4 + p * 4 * c + h;
-      const float m = mask[p];
-      float v[4][8];      // ap, ag, bp, bg
-#pragma unroll
-      for (int q = 0; q < 4; ++q)
-#pragma unroll
-        for (int e = 0; e < 8; e += 4) {
-          const float4 f = *reinterpret_cast<const float4*>(row + (int64_t)q * c + e);
-          v[q][e] = f.x; v[q][e + 1] = f.y; v[q][e + 2] = f.z; v[q][e + 3] = f.w;
-        }
-#pragma unroll
-      for (int e = 0; e < 8; ++e) {
-        ta[hg + e][r] = __float2half_rn(v[0][e] * sigmoidf_(v[1][e]) * m);
-        tb[hg + e][r] = __float2half_rn(v[2][e] * sigmoidf_(v[3][e]) * m);
-      }
-    } else {
-#pragma unroll
-      for (int e = 0; e < 8; ++e) ta[hg + e][r] = tb[hg + e][r] = __float2half_rn(0.f);
-    }
-  }
-  __syncthreads();
-  const int hh = threadIdx.x >> 3, k8 = (threadIdx.x & 7) * 8, h = h0 + hh;
-  if (h < c && k0 + k8 < ld) {
-    const int64_t o = ((int64_t)h * n + i) * ld + k0 + k8;
-    *reinterpret_cast<uint4*>(a + o) = *reinterpret_cast<const uint4*>(&ta[hh][k8]);
-    *reinterpret_cast<uint4*>(b + o) = *reinterpret_cast<const uint4*>(&tb[hh][k8]);
-  }
-}
-
 // LayerNorm over the channels of a channel-major x[h][i][ld] -> terms with rows of ldc.  A block takes 32 pairs of one pair row; the
 // tile [c][32] sits in shared memory.
 template <typename TIn>
@@ -387,10 +305,10 @@ center_norm_half_kernel(const __half* __restrict__ x, int c, int n, int ld, cons
   }
 }
 
-// out[dst(r)][c] = (resid ? resid[dst(r)][c] : 0) + proj[r][c] * (gate ? sigmoid(gate[r][c]) : 1), four channels a thread
+// out[dst(r)][c] = (resid ? resid[dst(r)][c] : 0) + proj[r][c] * (factor ? factor[r][c] : 1), four channels a thread
 // (ch a multiple of 4); dst(r) follows the transposed-orientation rule of the attention operator.
 template <typename TAct>
-__global__ void finish4_kernel(const float* __restrict__ proj, const float* __restrict__ gate, const TAct* __restrict__ resid, int64_t count,
+__global__ void finish4_kernel(const float* __restrict__ proj, const float* __restrict__ factor, const TAct* __restrict__ resid, int64_t count,
                                int ch, int transpose, int batch, int Q, TAct* __restrict__ out) {
   lf_chain();
   const int64_t idx = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
@@ -402,11 +320,11 @@ __global__ void finish4_kernel(const float* __restrict__ proj, const float* __re
   if (transpose) { const uint32_t u = (uint32_t)r, uq = (uint32_t)Q; dst = (int64_t)(u % uq) * batch + u / uq; }
   float v[4];
   load4(proj + r * ch + c, v);
-  if (gate) {
+  if (factor) {
     float g[4];
-    load4(gate + r * ch + c, g);
+    load4(factor + r * ch + c, g);
 #pragma unroll
-    for (int e = 0; e < 4; ++e) v[e] *= sigmoidf_(g[e]);
+    for (int e = 0; e < 4; ++e) v[e] *= g[e];
   }
   if (resid) {
     float x[4];

@@ -152,10 +152,10 @@ sgemm_kernel(int M, int N, int K, const float* __restrict__ A, int64_t lda, cons
 }
 
 // ---------------------------------------------------------------------------
-// out[dst(r)][c] = (resid ? resid[dst(r)][c] : 0) + proj[r][c] * (gate ? sigmoid(gate[r][c]) : 1)
+// out[dst(r)][c] = (resid ? resid[dst(r)][c] : 0) + proj[r][c] * (factor ? factor[r][c] : 1)
 // dst(r) follows the transposed-orientation rule of the attention operator.
 template <typename TAct>
-__global__ void finish_kernel(const float* __restrict__ proj, const float* __restrict__ gate,
+__global__ void finish_kernel(const float* __restrict__ proj, const float* __restrict__ factor,
                               const TAct* __restrict__ resid, int64_t rows, int ch, int transpose,
                               int batch, int Q, TAct* __restrict__ out) {
   lf_chain();
@@ -167,7 +167,7 @@ __global__ void finish_kernel(const float* __restrict__ proj, const float* __res
   int64_t dst = r;
   if (transpose) { int64_t b = r / Q, i = r % Q; dst = i * batch + b; }
   float v = proj[idx];
-  if (gate) v *= sigmoidf_(gate[idx]);
+  if (factor) v *= factor[idx];
   if (resid) v += to_f(resid[dst * ch + c]);
   out[dst * ch + c] = from_f<TAct>(v);
 }

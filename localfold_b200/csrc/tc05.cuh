@@ -386,6 +386,18 @@ __device__ __forceinline__ void ld_global_v8(const void* ptr, uint32_t (&v)[8]) 
                : "memory");
 }
 
+// The leading bf16 terms of x and y (x in the low half), which keep what is left of them, exactly: mixed-precision multiply-adds by -1
+__device__ __forceinline__ uint32_t split_bf16(float& x, float& y) {
+  uint32_t w;
+  asm("{\n\t.reg .b16 lo, hi, m;\n\t"
+      "cvt.rn.bf16x2.f32 %2, %1, %0;\n\t"
+      "mov.b32 {lo, hi}, %2;\n\t"
+      "mov.b16 m, 0xBF80;\n\t"
+      "fma.rn.f32.bf16 %0, lo, m, %0;\n\t"
+      "fma.rn.f32.bf16 %1, hi, m, %1;\n\t}"
+      : "+f"(x), "+f"(y), "=&r"(w));
+  return w;
+}
 __device__ __forceinline__ uint32_t pack_half2(float lo, float hi) {
   __half2 v = __floats2half2_rn(lo, hi);
   return *reinterpret_cast<uint32_t*>(&v);

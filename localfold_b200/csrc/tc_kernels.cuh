@@ -35,7 +35,19 @@ struct Gemm3Out {
   float* gate = nullptr;
   float* pair_bias = nullptr;
   int bias_q = 0, bias_ld = 0, bias_swap = 0;
+  // Or the operands of a triangle product: columns in groups of 32, 16 channels of a projection and the 16 of its gate (the fused projection's operand
+  // is laid out so; all groups of a, then all of b, channels padded to whole groups), rows = pairs (i, k) of length plane_n:
+  // planes[channel][i][k] = mask (projection + bias) sigmoid(gate + bias), rows of ld, fp16 when plane_half, else terms; bias = [4][plane_c]
+  const float* plane_mask = nullptr;
+  void* plane[2] = {nullptr, nullptr};
+  int plane_n = 0, plane_c = 0, plane_half = 0;
+  // Or the end of an operator in float32, rows of n (a multiple of 4) on 16-byte boundaries: act[dst(i)][j] (+)= value * (factor ? factor[i][j] : 1), added when
+  // act_add; rows (b, q) go to row q * act_batch + b when act_q is not 0 (i = b * act_q + q)
+  float* act = nullptr;
+  const float* factor = nullptr;      // rows of n
+  int act_add = 0, act_batch = 0, act_q = 0;
 };
+constexpr int gated_columns(int c) { return 4 * ((c + 15) / 16 * 16); }
 void configure_gemm3();
 lf_status gemm_f32(lf_context* ctx, ArenaCursor& cur, int major, const SplitMatrix& a, const SplitMatrix& b, int m, int n, int k, int batch,
                    const Gemm3Out& o);

@@ -15,6 +15,7 @@ enum JobKind {
   JOB_BIASED,     // ... -> fp16 [n_out][K + 16], bias in k column K and zeros after it (the activations carry a column of ones there)
   JOB_FOLD,       // float [n_out]: scale * (bias[c] + sum_k vec[k] W[k][col0 + c]): a LayerNorm offset folded into a bias
   JOB_TERMS,      // ... -> three bf16 terms [3][rows][n_pad] at row0, zeros past K (n_pad = K rounded up to 8)
+  JOB_GATED,      // the fused triangle projection (four roles of n_out columns) as terms [3][n_fill][n_pad], rows as Gemm3Out's planes want them
   JOB_HEADS,      // the fused attention projection as terms, every head of d channels (row0) padded with zero rows to D (n_pad)
   JOB_HEADS_BIAS, // ... its bias vector, as float32
   JOB_HEADS_OUT,  // the output projection as terms, the k of every head padded likewise
@@ -58,6 +59,20 @@ __global__ void __launch_bounds__(256) weight_jobs_kernel(const __grid_constant_
   if (j.kind == JOB_HEADS_BIAS) {
     for (int64_t n = first; n < j.n_fill; n += stride)
       reinterpret_cast<float*>(j.out)[n] = n % D < d && n / D * d + n % D < j.n_out ? j.w[n / D * d + n % D] : 0.f;
+    return;
+  }
+  if (j.kind == JOB_GATED) {
+    for (int64_t i = first; i < (int64_t)j.n_pad * j.n_fill; i += stride) {
+      const int k = (int)(i / j.n_fill), n = (int)(i % j.n_fill), half = j.n_fill / 2, which = n / half, in = n % half, h = in / 32 * 16 + in % 16;
+      float v = k < j.K && h < j.n_out ? j.w[(int64_t)k * j.ld + (which * 2 + in % 32 / 16) * j.n_out + h] : 0.f;
+      bf16* t = reinterpret_cast<bf16*>(j.out) + (int64_t)n * j.n_pad + k;
+#pragma unroll
+      for (int e = 0; e < 3; ++e) {
+        const bf16 b = __float2bfloat16_rn(v);
+        t[e * j.term_stride] = b;
+        v -= __bfloat162float(b);
+      }
+    }
     return;
   }
   if (j.kind == JOB_HEADS || j.kind == JOB_HEADS_OUT) {
@@ -162,7 +177,12 @@ bool f32_jobs(Preparer& prep, const lf_weights* w, WeightCursor& cur, SplitMatri
   switch (w->kind) {
     case LF_WEIGHTS_TRIANGLE_AF2:
     case LF_WEIGHTS_TRIANGLE_AF3:
-      operand(g[0], c, {{f[TRI_W4], 4 * dims.hidden, 0, 4 * dims.hidden}});
+      {
+        const int ld = (c + 7) / 8 * 8, rows = gated_columns(dims.hidden);
+        bf16* p = cur.take<bf16>((size_t)3 * rows * ld);
+        g[0] = SplitMatrix{p, ld, 0, (int64_t)rows * ld};
+        prep.push(Job{f[TRI_W4], nullptr, nullptr, p, 1.0f, JOB_GATED, c, 4 * dims.hidden, 0, dims.hidden, rows, ld, 0, g[0].term_stride});
+      }
       operand(g[1], dims.hidden, {{f[TRI_WZ], c, 0, c}});
       operand(g[2], c, {{f[TRI_WG], c, 0, c}});
       break;
