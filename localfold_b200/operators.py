@@ -82,6 +82,8 @@ class Device:
         self.stream = int(self.lib.lf_context_stream(handle) or 0)
         self._finalizer = weakref.finalize(self, self.lib.lf_context_destroy, handle)
         self._own_stream = stream is None
+        self._uploads = None
+        self._scratch_limit = 0
 
     def wait_for_torch(self):
         """Makes the context's own stream wait (on the device, no host wait) for the work torch has enqueued so
@@ -135,11 +137,29 @@ class Device:
         """Upper bound on the scratch arena (0 = none); a host-space pair stack that needs more keeps the pair
         in host memory and streams it through the device in chunks."""
         self.check(self.lib.lf_context_limit_scratch(self.handle, int(nbytes)))
+        self._scratch_limit = int(nbytes)
+        if self._uploads is not None:
+            self._uploads.limit_scratch(nbytes)
 
     def release_scratch(self):
         self.lib.lf_context_release_scratch(self.handle)
+        if self._uploads is not None:
+            self._uploads.release_scratch()
+
+    def uploads(self):
+        """A context of the same GPU with a stream of its own, made at the first use and closed with this one: weights prepared
+        there are copied, decoded and laid out while this context computes, and the calls that use them wait for them on
+        the device."""
+        if self._uploads is None:
+            self._uploads = Device(self.ordinal)
+            if self._scratch_limit:
+                self._uploads.limit_scratch(self._scratch_limit)
+        return self._uploads
 
     def close(self):
+        if self._uploads is not None:
+            self._uploads.close()
+            self._uploads = None
         self._finalizer()
 
 

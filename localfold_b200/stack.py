@@ -93,9 +93,10 @@ class PairStackGpu:
         self.blocks = []
         self.shape = None
 
-    def prepare(self, block_weights, c_z, c_hidden):
+    def prepare(self, block_weights, c_z, c_hidden, device=None):
+        """``device``: the context that prepares the weights, this stack's by default."""
         self.close()
-        self.blocks = [w if isinstance(w, PreparedPairBlock) else PreparedPairBlock(self.device, w, c_z, c_hidden)
+        self.blocks = [w if isinstance(w, PreparedPairBlock) else PreparedPairBlock(device or self.device, w, c_z, c_hidden)
                        for w in block_weights]
         self.shape = (c_z, c_hidden)
         self._table = (nat.PairBlockWeights * len(self.blocks))(*[b.struct() for b in self.blocks])
@@ -344,21 +345,22 @@ class Af3PairformerStackGpu:
             if single is not None:
                 seq_mask, _ = resident(state["seqMask"], (n,))
             def prepare(b):
-                stacks[b] = PairStackGpu(dev).prepare([blocks[b]], cz, cz)
+                stacks[b] = PairStackGpu(dev).prepare([blocks[b]], cz, cz, uploads)
                 if single is not None:
                     t = blocks[b]["singleTransition"]
-                    single_w[b] = (prepare_single_attention_weights(dev, blocks[b], cs, cz),
-                                   PreparedWeights(dev, nat.WEIGHTS_TRANSITION_AF3,
+                    single_w[b] = (prepare_single_attention_weights(uploads, blocks[b], cs, cz),
+                                   PreparedWeights(uploads, nat.WEIGHTS_TRANSITION_AF3,
                                                    {"channels": cs, "hidden": int(t["transition2"].shape[0])},
                                                    [t[k] for k in TRANSITION_AF3_ORDER]))
 
+            uploads = dev.uploads()
             stacks, single_w = {}, {}
             launches = 0
             sub = {"precision": opts.get("precision", "f32"), "residual": True}
             start, stop = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
             start.record(stream)
             try:
-                # A block's resident weights are prepared while the GPU works on the block before; when the blocks are not
+                # A block's resident weights are prepared, on a stream of their own, while the GPU works on the block before; when the blocks are not
                 # all of one shape, all of them before the first block runs, so that a wrong tensor is found before any update.
                 if not _same_shapes(blocks):
                     for b in range(len(blocks)):
@@ -453,16 +455,17 @@ class Af3MsaStackGpu:
                            "outputWeight": opm["outputW"], "outputBias": opm["outputB"]}
                 t = w["msaTransition"]
                 prepared[b] = (co,
-                               PreparedWeights(dev, nat.WEIGHTS_OPM_AF2, {"channels": cm, "hidden": co, "out_channels": cz},
+                               PreparedWeights(uploads, nat.WEIGHTS_OPM_AF2, {"channels": cm, "hidden": co, "out_channels": cz},
                                                [opm_af2[k] for k in OPM_WEIGHT_ORDER]),
-                               prepare_msa_attention_weights(dev, w["msaAttention1"], cm, cz),
-                               PreparedWeights(dev, nat.WEIGHTS_TRANSITION_AF3,
+                               prepare_msa_attention_weights(uploads, w["msaAttention1"], cm, cz),
+                               PreparedWeights(uploads, nat.WEIGHTS_TRANSITION_AF3,
                                                {"channels": cm, "hidden": int(np.asarray(t["transition2"]).shape[0])},
                                                [t[k] for k in TRANSITION_AF3_ORDER]))
 
             def prepare_pair(b):
-                stacks[b] = PairStackGpu(dev).prepare([blocks[b]], cz, cz)
+                stacks[b] = PairStackGpu(dev).prepare([blocks[b]], cz, cz, uploads)
 
+            uploads = dev.uploads()
             prepared, stacks = {}, {}
             sub = {"precision": opts.get("precision", "f32"), "residual": True}
             launches = 0
