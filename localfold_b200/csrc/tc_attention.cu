@@ -166,7 +166,8 @@ flash_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_constant__ C
     for (uint32_t item = blockIdx.x; item < items && ok; item += gridDim.x, ++n_item) {
       const auto [b, hp, tile] = locate_item<ROWS>(p, item);
       if (lane == 0) {
-        if (!mbar_wait_parked(q_empty, (n_item & 1) ^ 1, abort_flag, p.status, 20)) ok = false;
+        // (rows: not parked, see the issuers)
+        if (!(ROWS ? mbar_wait(q_empty, (n_item & 1) ^ 1, abort_flag, p.status, 20) : mbar_wait_parked(q_empty, (n_item & 1) ^ 1, abort_flag, p.status, 20))) ok = false;
         else {
           mbar_expect_tx(q_full, 2 * FA_Q_BYTES);
           // coordinates: position in four pieces, four pieces along channels (two per head pair), piece along rows, batch row
@@ -314,18 +315,26 @@ flash_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_constant__ C
         }
       };
 
-      for (uint32_t u0 = 0; u0 < 2 && u0 < U && ok; ++u0) {
-        ok = qk_ready();
-        if (!ok) break;
+      // The next item's Q comes late (its buffer is free only when the item's last S has been made): while products are outstanding it is not waited
+      // for.  (It was: the item's last two products waited with it, 2000 cycles of the 24 000 of an item of eight tiles; a launch of 384 x 384 queries 109.8 -> 100.7 us.
+      // The form of pairs of tiles, 592 us at 701 x 701, lost 5 us to the extra test: its items are longer and its sides share K and V.)
+      uint32_t qk = 0;      // next tile whose S is to be made
+      auto q_late = [&]() { return ROWS && qk_t == 0 && !__all_sync(0xffffffffu, mbar_test(q_full, qk_itpar)); };
+      auto scores = [&]() {
         tc_fence_after();
-        if (elect_one()) qk_issue(u0);
+        if (elect_one()) qk_issue(qk);
         __syncwarp();
         qk_advance();
+        ++qk;
+      };
+      while (qk < 2 && qk < U && ok) {
+        ok = qk_ready();
+        if (ok) scores();
       }
       uint32_t pv_t = 0;
       for (uint32_t u = 0; u < U && ok; ++u) {
-        const bool more = u + 2 < U;
         if (!mbar_wait(&p_full[w * 2 + (u & 1)], (u >> 1) & 1, abort_flag, p.status, 33)) { ok = false; break; }
+        const bool more = qk < U && !q_late();
         if (more && !qk_ready()) { ok = false; break; }
         tc_fence_after();
         const uint32_t v_addr = smem_u32(sV + pv_st * FA_KV_BYTES);
@@ -346,10 +355,14 @@ flash_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_constant__ C
           }
           if (pv_t + 1 == (uint32_t)T) umma_commit(&o_full[w]);     // one phase per item: its last P V has landed
           umma_commit(&kv_empty[pv_st]);   // this issuer's streams are done with the stage
-          if (more) qk_issue(u + 2);       // into the buffers these P V steps free
+          if (more) qk_issue(qk);          // into the buffers these P V steps free
         }
         __syncwarp();
-        if (more) qk_advance();
+        if (more) { qk_advance(); ++qk; }
+        while (ROWS && qk < U && qk < u + 3 && (qk == u + 1 || !q_late()) && ok) {      // what was put off; with no product outstanding it is waited for
+          ok = qk_ready();
+          if (ok) scores();
+        }
         if (++pv_t == (uint32_t)T) pv_t = 0;
         if ((pv_st += PER) >= FA_STAGES) pv_st -= FA_STAGES;
       }
