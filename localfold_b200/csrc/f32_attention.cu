@@ -116,7 +116,7 @@ attention3_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_constan
   typedef F3Form<D> F;
   constexpr int NS = F3_STREAMS, ST = F::STAGES, PIECES = F::PIECES, QB = F::Q_BUFFERS, SB = F::S_BUFFERS;
   extern __shared__ uint8_t smem_raw[];
-  uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
+  uint8_t* smem = align_shared(smem_raw);
   if (D == 32 && smem != smem_raw) {      // never seen
     if (threadIdx.x == 0 && p.status && atomicCAS(&p.status->code, 0u, 1u) == 0u) { p.status->where = 59; p.status->block = blockIdx.x; }
     return;

@@ -64,7 +64,7 @@ template <int MAJOR, bool PIECES, int OUT>
 __global__ void __launch_bounds__(G3_THREADS, 1)
 gemm3_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant__ CUtensorMap mapB, const Gemm3Params p) {
   extern __shared__ uint8_t smem_raw[];
-  uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
+  uint8_t* smem = align_shared(smem_raw);
   uint8_t* out_stage = smem + G3_STAGES * G3_STAGE;
   uint64_t* bars = reinterpret_cast<uint64_t*>(out_stage + G3_EPI * G3_OUT);
   uint64_t* full = bars;                       // [STAGES]

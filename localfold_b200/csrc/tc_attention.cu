@@ -102,7 +102,7 @@ flash_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_constant__ C
              const __grid_constant__ CUtensorMap mapV, const __grid_constant__ CUtensorMap mapB, const FlashParams p) {
   constexpr int FA_STAGES = FlashForm<ROWS>::STAGES, PER = FlashForm<ROWS>::PER, RINGS = FlashForm<ROWS>::RINGS;
   extern __shared__ uint8_t smem_raw[];
-  uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
+  uint8_t* smem = ROWS ? align_shared(smem_raw) : align_generic(smem_raw);
   uint8_t* sQ = smem;                                    // [side]
   uint8_t* sK = sQ + 2 * FA_Q_BYTES;                     // [stage]
   uint8_t* sV = sK + FA_STAGES * FA_KV_BYTES;            // [stage]

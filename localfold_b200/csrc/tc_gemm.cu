@@ -54,7 +54,7 @@ __global__ void __launch_bounds__(GM_THREADS, 1)
 gemm_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant__ CUtensorMap mapB, const __grid_constant__ CUtensorMap mapO,
             const GemmParams p) {
   extern __shared__ uint8_t smem_raw[];
-  uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
+  uint8_t* smem = align_shared(smem_raw);
   uint8_t* out_stage = smem + GM_STAGES * GM_STAGE;
   float* bias_s = reinterpret_cast<float*>(out_stage + GM_EPI * GM_OUT);      // [epilogue warp][its columns]
   uint64_t* bars = reinterpret_cast<uint64_t*>(bias_s + GM_EPI * GM_SHARE);

@@ -222,7 +222,7 @@ contract_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant_
                 float scale, Status* status, const __grid_constant__ PeerPtrs xpeer, int rows_per_rank, int ch0,
                 const ContractExtra ex) {
   extern __shared__ uint8_t smem_raw[];
-  uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
+  uint8_t* smem = align_shared(smem_raw);
   constexpr int ST = EW == 8 ? 3 : CT_STAGES;      // = ct_stages(EW)
   uint64_t* bars = reinterpret_cast<uint64_t*>(smem + ST * CT_STAGE_BYTES);
   uint64_t* full = bars;                       // [STAGES]

@@ -119,7 +119,7 @@ ln_gemm_kernel(const __grid_constant__ CUtensorMap mapX, const __grid_constant__
   // output rows in that tile's x buffer, which its MMAs have finished with by then
   constexpr int NS = 2;
   extern __shared__ uint8_t smem_raw[];
-  uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
+  uint8_t* smem = EPI == LG_EPI_ATTENTION ? align_generic(smem_raw) : align_shared(smem_raw);
   const int w_bytes = p.n_pad * 256;
   uint8_t* sW = smem;
   uint8_t* sA = smem + w_bytes;                       // 2 stages (w_bytes is a multiple of 1024: n_pad % 8 == 0... x256)
@@ -130,7 +130,7 @@ ln_gemm_kernel(const __grid_constant__ CUtensorMap mapX, const __grid_constant__
   float* sBias = reinterpret_cast<float*>(sStage + (EPI == LG_EPI_OUTPUT ? LG_EPI_WARPS * 4096
                                                     : EPI == LG_EPI_TRIANGLE ? LG_EPI_WARPS * 2048 : 0));
   float* sStat = sBias + (EPI == LG_EPI_TRIANGLE ? 0 : 544 + 256);      // [2 stages][2][128]: inverse std, inverse std * mean
-  uint64_t* bars = reinterpret_cast<uint64_t*>(sStat + (EPI == LG_EPI_TRIANGLE ? LG_MASKS * LG_ROWS : 512));
+  uint64_t* bars = reinterpret_cast<uint64_t*>(align_shared(smem_raw) + (reinterpret_cast<uint8_t*>(sStat + (EPI == LG_EPI_TRIANGLE ? LG_MASKS * LG_ROWS : 512)) - smem));
   uint64_t* a_full = bars;          // [2]
   uint64_t* a_empty = bars + 2;     // [2]
   uint64_t* acc_full = bars + 4;    // [2]

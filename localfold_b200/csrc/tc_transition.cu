@@ -53,7 +53,7 @@ __global__ void __launch_bounds__(TR_THREADS, 1) transition_kernel(const __grid_
   constexpr int HK = SWIGLU ? 64 : 128;                     // hidden channels per chunk = K of the second GEMM
   constexpr uint32_t W_BYTES = SWIGLU ? 3 * TR_TILE_BYTES / 2 : 2 * TR_TILE_BYTES;   // bytes streamed per chunk
   extern __shared__ uint8_t smem_raw[];
-  uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
+  uint8_t* smem = align_shared(smem_raw);
   uint8_t* sW = smem;                              // [2 stages][W1 slice | W2 slice]
   uint8_t* sA = sW + 2 * TR_W_STAGE;               // normalised activations (A of GEMM 1)
   uint8_t* sH = sA + TR_TILE_BYTES;                // hidden chunk (A of GEMM 2)
