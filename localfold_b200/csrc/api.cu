@@ -1,6 +1,6 @@
 // C ABI of the pair-stack library: context, weights, operators.
 // 16-bit mode routes what they cover to the fused tcgen05 kernels declared in tc_kernels.cuh; everything else composes the GEMMs
-// of tc_gemm.cu (fp16) and f32_gemm.cu, the attention core of mma_attention.cuh and the kernels of row_kernels.cuh and simt_kernels.cuh.
+// of tc_gemm.cu (fp16) and f32_gemm.cu, the attention cores of f32_attention.cu and mma_attention.cuh and the kernels of row_kernels.cuh and simt_kernels.cuh.
 #include <cuda_fp16.h>
 #include <sys/mman.h>
 #include <unistd.h>

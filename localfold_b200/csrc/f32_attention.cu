@@ -16,8 +16,8 @@
 // What bounds it: issue slots (65 % of them busy at 384 x 384) and the round trips of a tile; the exponents take a quarter of their unit's time, the tensor
 // core a third.  An exponential costs its share of 17 instructions, six of them to take it apart and three to add the products up.  Two streams
 // with tiles of 64 keys, two softmax warps a scheduler, took a tenth longer; with the next logits requested during the exponentials another tenth.
-// Against the mma.sync kernel (mma_attention.cuh; a warp's chain of dependent MMAs): 384 x 384, 4 heads of 16: 465 -> 204 us; 203 x 203,
-// 4 x 32: 184 -> 87; 1024 x 256, 8 x 8: 936 -> 466.
+// Against the mma.sync kernel (mma_attention.cuh; a warp's chain of dependent MMAs): 384 x 384, 4 heads of 16: 465 -> 192 us; 203 x 203,
+// 4 x 32: 184 -> 85; 1024 x 256, 8 x 8: 936 -> 478.
 #include <cuda.h>
 
 #include "tc05.cuh"
@@ -602,7 +602,7 @@ lf_status make_map_f32_any(lf_context* ctx, CUtensorMap* map, const void* base, 
 
 // A round of the blocks takes a key tile in 1.7 us, with heads of 32 channels in 2.6, after 3 us of start-up, however few of them have work; the mma.sync kernel's
 // time follows the number of logits, 1.75 / 2.05 / 5.5 us a million at 8 / 16 / 32 channels.  64 x 64, 4 heads of 32: 13.2 against its 9.5 us;
-// 96 x 96: 17.0 against 23.0; 8 rows of 384, 4 x 16: 28.5 against 18.9; 32 rows: 29.2 against 43.4.
+// 96 x 96: 16.5 against 23.0; 8 rows of 384, 4 x 16: 28.5 against 18.9; 32 rows: 27.6 against 43.4.
 bool attention3_wins(const lf_context* ctx, int D, int batch, int Q, int heads) {
   if (D != 8 && D != 16 && D != 32) return false;
   const int64_t items = (int64_t)((batch + F3_STREAMS - 1) / F3_STREAMS) * heads * ((Q + F3_QT - 1) / F3_QT);

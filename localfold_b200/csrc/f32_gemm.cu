@@ -17,7 +17,9 @@ using namespace tc05;
 // 3.1e-7 to 4.8e-7 for the triangle update at 203 to 700; with all of k in TMEM 1.3e-6 for a transition of 384 channels).
 // Warp roles: 0 = TMA producer, 1 = MMA issuer (owns TMEM), 2..17 = epilogue (lane quadrant = warp % 4, a quarter of the columns).
 // With two k blocks a tile (K = 128) the epilogue is what bounds it - eight warps and scalar bias loads took 41 us a launch on average for
-// the float32 pair block at N = 203, this 35 - and the operands' way from L2 into shared memory (96 KiB per 1560 cycles of tensor work) with more.
+// the float32 pair block at N = 203, sixteen 35 - and the operands' way from L2 into shared memory (96 KiB per 1560 cycles of tensor work) with
+// more.  An instance per form of output: what a shared epilogue left to passes of their own (triangle gates 38 us, ends of operators 10, bias columns)
+// is done here, and 16 launches of the same block take 25 to 46 us, 456 in all, against 486 before with 190 of such passes beside them.
 constexpr int G3_BM = 128, G3_BN = 128, G3_BK = 64, G3_STAGES = 2, G3_EPI = 16;
 constexpr int G3_PLANE = G3_BM * G3_BK * 2;            // 16 KiB: one term of one operand
 constexpr int G3_STAGE = 6 * G3_PLANE;
