@@ -29,10 +29,35 @@ __device__ __forceinline__ uint32_t smem_u32(const void* p) {
 // offset: triangle projection 39.9 -> 38.0 us, triangle output 44.5 -> 41.4, transition 68.7 -> 64.5, GEMM 31.1 -> 29.3 (N = 384); float32
 // attention core 208 -> 189, float32 projections 59 -> 57.5, 41 -> 38.6 and 34.6 -> 32.6 (template pair, N = 384).  Two kernels that are short
 // of registers keep the generic pointer, for the compiler spills or reorders with the other one: attention projection 50.3 -> 54.4 (its
-// barriers alone by the offset: 49.2), flash core's stream form 593 -> 648 at N = 701 (its barriers alone: 609).
+// barriers alone by the offset: 49.2), flash core's tiles form 593 -> 648 at N = 701 (its barriers alone: 609).
 __device__ __forceinline__ uint8_t* align_shared(uint8_t* raw) { return raw + ((0u - smem_u32(raw)) & 1023u); }
 __device__ __forceinline__ uint8_t* align_generic(uint8_t* raw) {
   return reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(raw) + 1023) & ~(uintptr_t)1023);
+}
+
+// Two float32 operations in one instruction: a * b + c, a + b.
+__device__ __forceinline__ float2 fma2(float2 a, float2 b, float2 c) {
+  float2 y;
+  asm("{\n\t.reg .b64 a, b, c;\n\t"
+      "mov.b64 a, {%2, %3};\n\t"
+      "mov.b64 b, {%4, %5};\n\t"
+      "mov.b64 c, {%6, %7};\n\t"
+      "fma.rn.f32x2 a, a, b, c;\n\t"
+      "mov.b64 {%0, %1}, a;\n\t}"
+      : "=f"(y.x), "=f"(y.y)
+      : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y), "f"(c.x), "f"(c.y));
+  return y;
+}
+__device__ __forceinline__ float2 add2(float2 a, float2 b) {
+  float2 y;
+  asm("{\n\t.reg .b64 a, b;\n\t"
+      "mov.b64 a, {%2, %3};\n\t"
+      "mov.b64 b, {%4, %5};\n\t"
+      "add.rn.f32x2 a, a, b;\n\t"
+      "mov.b64 {%0, %1}, a;\n\t}"
+      : "=f"(y.x), "=f"(y.y)
+      : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y));
+  return y;
 }
 
 __device__ __forceinline__ uint64_t global_timer_ns() {

@@ -1,8 +1,8 @@
 // Gated attention core on tcgen05 for 4 heads x 32 (128-channel) activations.
 //
 // Work item = two sides of two streams (one a head of the head pair) each, in one of two forms:
-//   tiles: a batch row and two neighbouring 128-query tiles; the sides share the K and V tiles of the head pair;
-//   rows:  a query tile of two neighbouring batch rows; the sides share the bias tiles.
+//   rows:  a query tile of two neighbouring batch rows; the sides share the bias tiles;
+//   tiles: a batch row and two neighbouring 128-query tiles; the sides share the K and V tiles of the head pair (few batch rows).
 // K and V stream through a TMA ring of 48-key tiles.  Q, K, V (and the gate and the output) live in memory as
 // 8-row x 8-channel pieces of 128 bytes; 5-d tensor maps bring a tile's pieces in as
 // [rows / 8][8 pieces of the head pair][8 rows][16 B], which is the tensor core's unswizzled
@@ -435,15 +435,28 @@ flash_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_constant__ C
         // handing the exponent unit from warp to warp in turn (to keep the four warps of a scheduler out
         // of step) measured no gain - the wake-up costs what the stagger saves
         auto exponentials = [&](const uint32_t (&su)[16], uint32_t (&w)[8]) {
-          float ps[8];
+          if constexpr (ROWS) {
+            // packed multiply-adds and sums: 825 queries 772 -> 761 us (in the tiles form, whose bias traffic reacts to any change of pace, 593 -> 637)
+            float2 ps[8];
 #pragma unroll
-          for (int e = 0; e < 8; ++e) {
-            const float p0 = ex2f(fmaf(__uint_as_float(su[2 * e]), L2E, neg));
-            const float p1 = ex2f(fmaf(__uint_as_float(su[2 * e + 1]), L2E, neg));
-            ps[e] = p0 + p1;
-            w[e] = pack_half2(p0, p1);
+            for (int e = 0; e < 8; ++e) {
+              const float2 x = fma2(make_float2(__uint_as_float(su[2 * e]), __uint_as_float(su[2 * e + 1])), make_float2(L2E, L2E), make_float2(neg, neg));
+              ps[e] = make_float2(ex2f(x.x), ex2f(x.y));
+              w[e] = pack_half2(ps[e].x, ps[e].y);
+            }
+            const float2 sum = add2(add2(add2(ps[0], ps[1]), add2(ps[2], ps[3])), add2(add2(ps[4], ps[5]), add2(ps[6], ps[7])));
+            return sum.x + sum.y;
+          } else {
+            float ps[8];
+#pragma unroll
+            for (int e = 0; e < 8; ++e) {
+              const float p0 = ex2f(fmaf(__uint_as_float(su[2 * e]), L2E, neg));
+              const float p1 = ex2f(fmaf(__uint_as_float(su[2 * e + 1]), L2E, neg));
+              ps[e] = p0 + p1;
+              w[e] = pack_half2(p0, p1);
+            }
+            return ((ps[0] + ps[1]) + (ps[2] + ps[3])) + ((ps[4] + ps[5]) + (ps[6] + ps[7]));
           }
-          return ((ps[0] + ps[1]) + (ps[2] + ps[3])) + ((ps[4] + ps[5]) + (ps[6] + ps[7]));
         };
         load_s();
         if (t == 0) {
@@ -573,11 +586,14 @@ lf_status attention_core(lf_context* ctx, ArenaCursor& cur, const op16* q, const
   p.batch = batch; p.Q = Q; p.qtiles = (Q + FA_TILE - 1) / FA_TILE; p.ktiles = (Q + FA_KT - 1) / FA_KT;
   p.transpose = transpose; p.mask_mode = mask_mode; p.clamp = clamp; p.mask = mask; p.has_bias = bias ? 1 : 0; p.ldb = ldb; p.ldq = ldq;
   p.gate = g; p.out = out; p.status = (Status*)ctx->tc_status;
-  // Rows: with an odd number of query tiles, pairs of tiles leave half an item empty a row.  A key tile takes 9 % longer than with
-  // the sides sharing K and V (two ring entries), so pairs of tiles win again from eleven tiles on.  Four launches at
-  // 384 x 384 queries: 567 -> 452 us, six over 825 queries: 4.65 -> 4.48 ms.
-  const bool rows = (p.qtiles & 1) && p.qtiles <= 9 && batch > 1;
-  const int64_t items = rows ? (int64_t)((batch + 1) / 2) * p.qtiles * 2 : (int64_t)batch * ((p.qtiles + 1) / 2) * 2;
+  // Rows, whose sides bring 56 KB a key tile from L2 (with a bias; tiles: 77), unless tiles need fewer rounds of the blocks by more than the 2 %
+  // that a round is longer: few batch rows of many queries.  (Where the number of query tiles is odd, tiles leave half an item a row empty.)
+  // Tiles -> rows, two launches: 2048 queries 24.1 -> 23.6 ms (block 38.9 -> 38.2), 701 1192 -> 1199 us alone (block 2707 -> 2671, under the power cap); the six
+  // of an evoformer block with 825 and 512 queries, two of them tiles before: 4.13 -> 4.05 ms.
+  const int64_t by_rows = (int64_t)((batch + 1) / 2) * p.qtiles * 2, by_tiles = (int64_t)batch * ((p.qtiles + 1) / 2) * 2;
+  auto rounds = [&](int64_t n) { return (n + ctx->sm_count - 1) / ctx->sm_count; };
+  const bool rows = batch > 1 && 50 * rounds(by_rows) <= 51 * rounds(by_tiles);
+  const int64_t items = rows ? by_rows : by_tiles;
   if (items > INT32_MAX) return lf_fail(ctx, LF_ERR_UNSUPPORTED, "attention over %d rows of %d queries exceeds the work index", batch, Q);
   const int grid = (int)(items < ctx->sm_count ? items : ctx->sm_count);
   lf_prof_begin(ctx, LF_KERNEL_ATTENTION);
