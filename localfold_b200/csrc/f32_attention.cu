@@ -391,9 +391,10 @@ attention3_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_constan
 #pragma unroll
       for (int e = 0; e < D; ++e) o[e] = 0.f;
       // p = 2^(l log2(e) - ref2) with a whole ref2, so that a change of it scales by a power of two, exactly.  A masked row's logits
-      // are near -1e9, where their product with log2(e) is rounded to whole powers of two: such a warp (far) subtracts ref first.
+      // are near -1e9, where their product with log2(e) is rounded to whole powers of two: such a query (far) subtracts ref first, so its
+      // base is ref log2(e).  A query keeps the form that its own reference asks for, whatever the others of its warp do.
       float ref = 0.f, ref2 = 0.f, sum = 0.f, lost = 0.f;      // lost: what the additions to the sum have rounded away so far, negated
-      bool far = false;
+      bool far = false, any_far = false;                       // any_far: of the warp's queries
       // P V of tile m times c onto the output
       auto add_product = [&](uint32_t m, float c) -> bool {
         if (!mbar_wait(&o_full[g], m & 1, abort_flag, p.status, 70)) return false;
@@ -473,8 +474,7 @@ attention3_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_constan
         };
         // the reference stays while every exponential is at most 2^60
         float top = row_max(), carry = 1.f;      // carry: factor of the product that is still to be added
-        auto over = [&]() { return !((far ? (top - ref) * L2E : fmaf(top, L2E, -ref2)) <= 60.f); };
-        if (__any_sync(0xffffffffu, t == 0 || far || over())) {
+        if (__any_sync(0xffffffffu, t == 0 || any_far || !(fmaf(top, L2E, -ref2) <= 60.f))) {
           if (p.clamp) {      // changes the result of such rows only: everywhere else what it raises has probability 0 with and without it
 #pragma unroll
             for (int j = 0; j < F3_KT; ++j) l[j] = j < left ? fminf(fmaxf(l[j], -1e8f), 1e8f) : l[j];
@@ -483,9 +483,11 @@ attention3_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_constan
           if (t == 0) {
             ref = top;      // key 0 exists: finite
             ref2 = rintf(ref * L2E);
-          } else if (over()) {
+          } else if (!((far ? (top - ref) * L2E : fmaf(top, L2E, -ref2)) <= 60.f)) {
             const float next = fmaxf(ref, top), next2 = rintf(next * L2E);
-            carry = f3_ex2(far ? (ref - next) * L2E : ref2 - next2);
+            const bool next_far = fabsf(next) > 65536.f;
+            // from the base that sum and output have to the one that they get
+            carry = f3_ex2(far ? (next_far ? (ref - next) * L2E : fmaf(ref, L2E, -next2)) : next_far ? fmaf(-next, L2E, ref2) : ref2 - next2);
             ref = next;
             ref2 = next2;
             sum *= carry;
@@ -493,13 +495,15 @@ attention3_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_constan
 #pragma unroll
             for (int e = 0; e < D; ++e) o[e] *= carry;
           }
-          far = __any_sync(0xffffffffu, fabsf(ref) > 65536.f);
+          far = fabsf(ref) > 65536.f;
+          any_far = __any_sync(0xffffffffu, far);
         }
         float shift = -ref2;
-        if (far) {      // a pass of its own in front
-          shift = 0.f;
+        if (any_far) {      // a pass of its own in front
+          const float first = far ? ref : 0.f;
+          if (far) shift = 0.f;
 #pragma unroll
-          for (int j = 0; j < F3_KT; ++j) l[j] -= ref;
+          for (int j = 0; j < F3_KT; ++j) l[j] -= first;
         }
         // exponentials, and the terms of the 16 keys before by truncation: keys 2i, 2i + 1 -> column i of each term
 #pragma unroll

@@ -79,3 +79,32 @@ def test_what_is_not_finite_stays_in_its_row(dev):
     got = lf.AttentionGpu(dev).run(given, {"precision": "f32"})["output"].reshape(99, 97, -1)
     rest = np.arange(99) != 6
     assert np.isnan(got[6]).any() and np.array_equal(got[rest], clean[rest])
+
+
+# Runs of keys (first, one behind the last) with logits of +-8e4 or +-2.4e5, a query each: up across 65536 behind the first key tile; from below
+# -65536 back to the others' size and up; up twice beyond 65536; below it where the reference is not theirs.  Three neighbouring lanes, another warp.
+FAR = {3: [(40, 41, 8e4)], 4: [(0, 35, -8e4), (70, 71, 8e4)], 5: [(33, 34, 8e4), (66, 67, 2.4e5)], 37: [(0, 33, -2.4e5), (64, 90, -8e4)]}
+
+
+@pytest.mark.parametrize("q,batch,heads,dim,transpose,bias", [SIZES[0], SIZES[1], SIZES[5]])
+def test_queries_with_far_logits_leave_the_others_alone(dev, q, batch, heads, dim, transpose, bias):
+    import localfold_b200 as lf
+    given = _case(q, batch, heads, dim, transpose, bias)
+    given["mask"][:] = 1
+    # Pair rows of +1 and -1 in equal numbers have mean 0 exactly, so their last four channels are 0 after the LayerNorm; rows of +-8 in two of these
+    # channels and nothing else have +-4 there.
+    pair = np.zeros((q, q, 32), np.float32)
+    pair[..., :28] = syn.draw(6100 + q).rng.permuted(np.tile(np.repeat(np.float32([1, -1]), 14), (q, q, 1)), axis=-1)
+    for query, runs in FAR.items():
+        for first, last, logit in runs:
+            pair[query, first:last] = 0
+            at = 30 if abs(logit) == 8e4 else 28
+            pair[query, first:last, at:at + 2] = np.float32([8, -8]) * np.sign(logit)
+    given["pairBias"]["activations"] = pair
+    given["pairBias"]["projectionWeight"][28:] = np.float32([3e4, -3e4, 1e4, -1e4])[:, None]
+    got, want = lf.AttentionGpu(dev).run(given, {"precision": "f32", "variance": "two-pass"})["output"], _want(given)
+    by_query = (lambda x: x.reshape(q, batch, -1).swapaxes(0, 1)) if transpose else (lambda x: x.reshape(batch, q, -1))
+    got, want = by_query(got), by_query(want)
+    ordinary = ~np.isin(np.arange(q), list(FAR))
+    assert _relative(got[:, ordinary], want[:, ordinary]) <= 1e-6
+    assert _relative(got[:, ~ordinary], want[:, ~ordinary]) <= 1e-6      # each of them ends on one key or on ordinary ones
