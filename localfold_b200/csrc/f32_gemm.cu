@@ -51,10 +51,11 @@ __host__ __device__ constexpr uint32_t make_idesc_bf16(int M, int N, int major) 
   return make_idesc_f16(M, N, major, major) | (1u << 7) | (1u << 10);
 }
 
-// 1 / (1 + e^-v): the quotient by Newton's iteration on the approximate reciprocal, without the branches of the correctly rounded one
+// 1 / (1 + e^-v): the quotient by Newton's iteration on the approximate reciprocal, without the branches of the correctly rounded one.
+// The bound keeps infinity out of the iteration (a result below 2^-126 is 0) and lets a NaN through, which fminf would drop.
 __device__ __forceinline__ float g3_sigmoid(float v) {
-  const float y = fminf(1.0f + expf(-v), 3e38f);
-  float r;
+  float y, r;
+  asm("min.NaN.f32 %0, %1, %2;" : "=f"(y) : "f"(1.0f + expf(-v)), "f"(3e38f));
   asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(y));
   return fmaf(r, fmaf(-y, r, 1.0f), r);
 }

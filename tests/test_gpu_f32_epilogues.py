@@ -63,3 +63,57 @@ def test_attention_with_a_residual(dev, n, heads, dim, transpose):
                                     "transpose": transpose, "pairBias": pb}, {"precision": "f32", "variance": "two-pass", "residual": True})["output"]
     want = t2.attention_af2(act, mask, n, n, c, heads, w["attention"], transpose, pb)
     assert _relative(got, act.astype(np.float64) + want) <= 1e-6
+
+
+# ---- a gate that is not a number: one channel of the gating weights ----
+
+
+def _spoiled(w, name, channel):
+    w = dict(w, **{name: w[name].copy()})
+    w[name][..., channel] = np.nan
+    return w
+
+
+@pytest.mark.parametrize("precision", ["f32", "bf16"])
+@pytest.mark.parametrize("c", [24, 64, 128])
+def test_gates_of_the_triangle_pass_a_nan_on(dev, c, precision):
+    import localfold_b200 as lf
+    d, n = syn.draw(7300 + c), 40
+    z, mask, w = d.normal(n, n, c), np.ones((n, n), np.float32), syn.af2_triangle_weights(d, c, c)
+
+    def nans(name, channel):
+        got = lf.TriangleMultiplicationOutgoingGpu(dev).run({"shape": {"length": n, "cZ": c, "cHidden": c}, "z": z, "mask": mask, "weights": _spoiled(w, name, channel)},
+                                                            {"precision": precision, "variance": "two-pass"})["output"]
+        return np.isnan(got)
+
+    nan = nans("linearGBias", 5)
+    assert nan[..., 5].all() and not np.delete(nan, 5, -1).any()
+    for name in ("linearAGBias", "linearBGBias"):      # a channel of a contraction operand: all of it, so every pair's centre LayerNorm
+        assert nans(name, 7).all()
+
+
+@pytest.mark.parametrize("precision", ["f32", "bf16"])
+@pytest.mark.parametrize("q,heads,dim", [(24, 2, 8), (97, 4, 16), (96, 4, 32), (40, 8, 32), (33, 3, 22)])
+def test_gates_of_the_attention_pass_a_nan_on(dev, q, heads, dim, precision):
+    import localfold_b200 as lf
+    d, c = syn.draw(7400 + q), heads * dim
+    w = syn.af2_attention_weights(d, c, heads)["attention"]
+    got = lf.AttentionGpu(dev).run({"activations": d.normal(q, q, c), "mask": np.ones((q, q), np.float32), "batch": q, "queryLength": q, "channels": c, "heads": heads,
+                                    "weights": _spoiled(w, "gatingBias", 3)}, {"precision": precision, "variance": "two-pass"})["output"]
+    assert np.isnan(got).all()
+
+
+@pytest.mark.parametrize("precision", ["f32", "bf16"])
+def test_gates_of_global_attention_and_averaging_pass_a_nan_on(dev, precision):
+    import localfold_b200 as lf
+    d, s, n = syn.draw(7500), 20, 33
+    act, mask = d.normal(s, n, 64), np.ones((s, n), np.float32)
+    w = _spoiled(syn.af2_global_attention_weights(d, 64, 8, 8), "gatingBias", 3)
+    assert np.isnan(lf.GlobalColumnAttentionGpu(dev).run({"activations": act, "mask": mask, "sequences": s, "length": n, "channels": 64, "weights": w},
+                                                         {"precision": precision})["output"]).all()
+    w = syn.af3_msa_attention_weights(d, 64, 128, 8, 8)
+    w["gatingQuery"] = w["gatingQuery"].copy()
+    w["gatingQuery"].reshape(-1)[3] = np.nan
+    got = lf.Af3MsaAttentionGpu(dev).run(act, mask, d.normal(n, n, 128), {"sequences": s, "tokens": n, "msaChannels": 64, "pairChannels": 128}, w,
+                                         {"precision": precision})["output"]
+    assert np.isnan(got).all()
