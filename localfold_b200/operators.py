@@ -115,7 +115,9 @@ class Device:
         self.check(self.lib.lf_context_synchronize(self.handle))
 
     def launch_count(self) -> int:
-        return int(self.lib.lf_context_launch_count(self.handle))
+        """Kernels launched so far, those that prepared weights on ``uploads()`` among them."""
+        devices = [self] if self._uploads is None else [self, self._uploads]
+        return sum(int(d.lib.lf_context_launch_count(d.handle)) for d in devices)
 
     def profile(self, enable: bool):
         """Bracket every kernel launch with CUDA events (off by default)."""
@@ -134,12 +136,13 @@ class Device:
         self.check(self.lib.lf_context_reserve(self.handle, int(nbytes)))
 
     def limit_scratch(self, nbytes: int):
-        """Upper bound on the scratch arena (0 = none); a host-space pair stack that needs more keeps the pair
-        in host memory and streams it through the device in chunks."""
+        """Upper bound on the device's scratch arena (0 = none); a host-space pair stack that needs more keeps the pair
+        in host memory and streams it through the device in chunks.  A device with a bound has one arena: ``uploads()``
+        is the device itself then, and what it had apart is given back."""
         self.check(self.lib.lf_context_limit_scratch(self.handle, int(nbytes)))
         self._scratch_limit = int(nbytes)
-        if self._uploads is not None:
-            self._uploads.limit_scratch(nbytes)
+        if self._scratch_limit and self._uploads is not None:
+            self._uploads.release_scratch()
 
     def release_scratch(self):
         self.lib.lf_context_release_scratch(self.handle)
@@ -149,11 +152,12 @@ class Device:
     def uploads(self):
         """A context of the same GPU with a stream of its own, made at the first use and closed with this one: weights prepared
         there are copied, decoded and laid out while this context computes, and the calls that use them wait for them on
-        the device."""
+        the device.  It has an arena of its own (a few MiB: the bytes of the largest operator); under ``limit_scratch`` this
+        context itself."""
+        if self._scratch_limit:
+            return self
         if self._uploads is None:
             self._uploads = Device(self.ordinal)
-            if self._scratch_limit:
-                self._uploads.limit_scratch(self._scratch_limit)
         return self._uploads
 
     def close(self):

@@ -43,3 +43,26 @@ def test_stacks_of_several_threads_and_devices():
     dev.release_scratch()
     assert all(np.array_equal(a, b) for a, b in zip(_run(dev, blocks, 17), want[17]))
     dev.close()
+
+
+def test_a_scratch_limit_and_the_launch_count_cover_the_weights():
+    """A device counts the launches of one that prepares its weights itself; a limit leaves it one arena."""
+    import localfold_b200 as lf
+    d = syn.draw(8200)
+    blocks = [syn.af3_pairformer_block_weights(d, 128, 384, 4, 16) for _ in range(2)]
+    counts, results = [], []
+    for limit in (0, 1 << 30):
+        dev = lf.Device(0)
+        dev.limit_scratch(limit)
+        before = dev.launch_count()
+        results.append(_run(dev, blocks, 33))
+        counts.append(dev.launch_count() - before)
+        assert (dev.uploads() is dev) == (limit != 0)
+        dev.limit_scratch(1 << 30)
+        assert dev.uploads() is dev
+        results.append(_run(dev, blocks, 33))
+        dev.limit_scratch(0)
+        assert dev.uploads() is not dev
+        dev.close()
+    assert counts[0] == counts[1]
+    assert all(np.array_equal(a, b) for r in results[1:] for a, b in zip(r, results[0]))
