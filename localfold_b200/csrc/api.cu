@@ -1056,8 +1056,7 @@ void layer_norm(lf_context* ctx, ArenaCursor& cur, const void* act, int64_t coun
 template <typename T>
 lf_status finish(lf_context* ctx, ArenaCursor& cur, const SplitMatrix& a, const SplitMatrix& w, int64_t count, int c, int k, const float* bias, const float* factor,
                  const T* resid, T* out, int batch = 1, int transposed_q = 0) {
-  // (a plan does not know the addresses: it has room for the pass)
-  if (!cur.dry && sizeof(T) == 4 && (!resid || resid == out) && (c & 3) == 0 && lf_aligned16(out)) {
+  if (sizeof(T) == 4 && (!resid || resid == out) && (c & 3) == 0 && lf_aligned16(out)) {
     tc::Gemm3Out to{nullptr, nullptr, c, 0, 0, bias, c, 0, 0, 0};
     to.act = (float*)out; to.act_add = resid != nullptr; to.factor = factor; to.act_batch = batch; to.act_q = transposed_q;
     return tc::gemm_f32(ctx, cur, 0, a, w, (int)count, c, k, 1, to);

@@ -167,12 +167,14 @@ static inline size_t lf_align_up(size_t v, size_t a) { return (v + a - 1) / a * 
 struct ArenaCursor {
   lf_context* ctx;
   size_t offset;
-  bool dry;       // planning pass: only adds sizes up
+  // Planning pass: only adds sizes up.  Its addresses are stand-ins, aligned and distinct as the real ones are, so that whatever a call decides by
+  // address - where a residual lives, how an output is aligned - it decides alike in both passes.
+  bool dry;
   size_t peak = 0;   // high-water mark (callers may rewind `offset` between operators)
   template <typename T>
   T* take(size_t count) {
     size_t bytes = lf_align_up(count * sizeof(T), 256);
-    T* p = dry ? nullptr : reinterpret_cast<T*>(ctx->arena + offset);
+    T* p = dry ? reinterpret_cast<T*>((uintptr_t)256 + offset) : reinterpret_cast<T*>(ctx->arena + offset);
     offset += bytes;
     if (offset > peak) peak = offset;
     return p;
