@@ -50,11 +50,12 @@ lf_status lf_arena_ensure(lf_context* ctx, size_t bytes) {
   LF_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
   if (ctx->arena) { cudaFree(ctx->arena); ctx->arena = nullptr; ctx->arena_bytes = 0; }
   size_t want = lf_align_up(bytes + bytes / 8, (size_t)1 << 21);
+  if (ctx->arena_limit && want > ctx->arena_limit) want = ctx->arena_limit;
   cudaError_t e = cudaMalloc(&ctx->arena, want);
   if (e != cudaSuccess) {
     cudaGetLastError();
     lf_block_cache_release(ctx->device);
-    want = lf_align_up(bytes, (size_t)1 << 21);
+    want = std::min(lf_align_up(bytes, (size_t)1 << 21), want);
     e = cudaMalloc(&ctx->arena, want);
   }
   if (e != cudaSuccess) {

@@ -76,3 +76,18 @@ def test_a_limit_of_what_a_call_takes(op, offset, apart):
         limit = used["memory"]["peakBytes"]
         dev.close()
     assert np.array_equal(results[0], results[1])
+
+
+def test_the_arena_stays_within_its_limit():
+    """The room an arena gets to grow into ends at the limit (what the driver hands out is whole pieces of 2 MiB)."""
+    import localfold_b200 as lf
+    import torch
+    dev, limit = lf.Device(0), 512 << 20
+    dev.limit_scratch(limit)
+    dev.synchronize()
+    free = torch.cuda.mem_get_info()[0]
+    dev.reserve(limit)
+    assert 0 <= free - torch.cuda.mem_get_info()[0] - limit <= 2 << 20
+    with pytest.raises(MemoryError):
+        dev.reserve(limit + 1)
+    dev.close()
