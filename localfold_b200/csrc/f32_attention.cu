@@ -118,7 +118,7 @@ attention3_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_constan
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = align_shared(smem_raw);
   if (D == 32 && smem != smem_raw) {      // never seen
-    if (threadIdx.x == 0 && p.status && atomicCAS(&p.status->code, 0u, 1u) == 0u) { p.status->where = 59; p.status->block = blockIdx.x; }
+    if (threadIdx.x == 0 && p.status && atomicCAS(&p.status->code, 0u, kStatusAlignment) == 0u) { p.status->where = 59; p.status->block = blockIdx.x; }
     return;
   }
   uint8_t* sBias = smem;                                  // [stage][128 queries][32 keys], 128-byte swizzle
@@ -370,7 +370,7 @@ attention3_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_constan
         const bool late = now - since > kWaitLimitNs;
         if (late && *abort_flag == 0) {
           *abort_flag = 1;
-          if (p.status && atomicCAS(&p.status->code, 0u, 1u) == 0u) { p.status->where = 64; p.status->block = blockIdx.x; }
+          if (p.status && atomicCAS(&p.status->code, 0u, kStatusTimeout) == 0u) { p.status->where = 64; p.status->block = blockIdx.x; }
         }
         if (__any_sync(0xffffffffu, late || *abort_flag != 0)) break;
       }

@@ -12,10 +12,11 @@
 
 namespace tc05 {
 
-// Error word the kernels set when a bounded wait runs out; the host reads it
-// after synchronising (see tc::check_status).
+// Error word the kernels set when a bounded wait runs out, or when shared memory is not aligned as a kernel needs it; the host
+// reads it after synchronising (see tc::check_status).
+constexpr unsigned int kStatusTimeout = 1, kStatusAlignment = 2;
 struct Status {
-  unsigned int code;     // 0 ok, 1 wait timed out
+  unsigned int code;     // 0 ok, or one of the above
   unsigned int where;    // which wait (kernel-specific tag)
   unsigned int block;
 };
@@ -134,7 +135,7 @@ __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, volati
       if (start == 0) start = now;
       else if (now - start > kWaitLimitNs) {
         *abort_flag = 1;
-        if (status && atomicCAS(&status->code, 0u, 1u) == 0u) { status->where = where; status->block = blockIdx.x; }
+        if (status && atomicCAS(&status->code, 0u, kStatusTimeout) == 0u) { status->where = where; status->block = blockIdx.x; }
         return false;
       }
     }
@@ -154,7 +155,7 @@ __device__ __forceinline__ bool mbar_wait_parked(uint64_t* bar, uint32_t parity,
       if (start == 0) start = now;
       else if (now - start > kWaitLimitNs) {
         *abort_flag = 1;
-        if (status && atomicCAS(&status->code, 0u, 1u) == 0u) { status->where = where; status->block = blockIdx.x; }
+        if (status && atomicCAS(&status->code, 0u, kStatusTimeout) == 0u) { status->where = where; status->block = blockIdx.x; }
         return false;
       }
     }

@@ -180,6 +180,8 @@ lf_status check_status(lf_context* ctx) {
   } else LF_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
   if (st.code != 0) {
     cudaMemset(ctx->tc_status, 0, sizeof st);
+    if (st.code == kStatusAlignment)
+      return lf_fail(ctx, LF_ERR_CUDA, "a kernel's shared memory is not on the boundary that it needs (%u, block %u): nothing was computed", st.where, st.block);
     return lf_fail(ctx, LF_ERR_TIMEOUT, "a bounded wait expired in a tensor-core kernel (wait %u, block %u)", st.where, st.block);
   }
   return LF_OK;
