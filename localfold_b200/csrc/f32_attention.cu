@@ -75,36 +75,6 @@ __device__ __forceinline__ float f3_ex2(float x) {      // relative error 2^-22
 }
 // the leading bf16 terms of x, y by truncation
 __device__ __forceinline__ uint32_t f3_pack(float x, float y) { return __byte_perm(__float_as_uint(x), __float_as_uint(y), 0x7632); }
-// x, y minus the terms in w, exactly: a mixed-precision multiply-add by -1 each
-__device__ __forceinline__ void f3_rest(float& x, float& y, uint32_t w) {
-  asm("{\n\t.reg .b16 lo, hi, m;\n\t"
-      "mov.b32 {lo, hi}, %2;\n\t"
-      "mov.b16 m, 0xBF80;\n\t"
-      "fma.rn.f32.bf16 %0, lo, m, %0;\n\t"
-      "fma.rn.f32.bf16 %1, hi, m, %1;\n\t}"
-      : "+f"(x), "+f"(y)
-      : "r"(w));
-}
-// two float32 operations in one instruction
-__device__ __forceinline__ void f3_fma2(float& x0, float& x1, float a0, float a1, float b0, float b1, float c0, float c1) {
-  asm("{\n\t.reg .b64 a, b, c;\n\t"
-      "mov.b64 a, {%2, %3};\n\t"
-      "mov.b64 b, {%4, %5};\n\t"
-      "mov.b64 c, {%6, %7};\n\t"
-      "fma.rn.f32x2 a, a, b, c;\n\t"
-      "mov.b64 {%0, %1}, a;\n\t}"
-      : "=f"(x0), "=f"(x1)
-      : "f"(a0), "f"(a1), "f"(b0), "f"(b1), "f"(c0), "f"(c1));
-}
-__device__ __forceinline__ void f3_add2(float& x0, float& x1, float a0, float a1) {      // x += a
-  asm("{\n\t.reg .b64 a, b;\n\t"
-      "mov.b64 a, {%0, %1};\n\t"
-      "mov.b64 b, {%2, %3};\n\t"
-      "add.rn.f32x2 a, a, b;\n\t"
-      "mov.b64 {%0, %1}, a;\n\t}"
-      : "+f"(x0), "+f"(x1)
-      : "f"(a0), "f"(a1));
-}
 __host__ __device__ constexpr uint32_t f3_idesc(int N, int b_major) {      // 128 x N, bf16 operands, A K-major
   return make_idesc_f16(F3_QT, N, 0, b_major) | (1u << 7) | (1u << 10);
 }
@@ -444,8 +414,9 @@ attention3_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_constan
 #pragma unroll
             for (int j4 = 0; j4 < 8; ++j4) {
               const float4 b = bias4(j4);
-              f3_fma2(l[j4 * 4], l[j4 * 4 + 1], l[j4 * 4], l[j4 * 4 + 1], p.scale, p.scale, b.x, b.y);
-              f3_fma2(l[j4 * 4 + 2], l[j4 * 4 + 3], l[j4 * 4 + 2], l[j4 * 4 + 3], p.scale, p.scale, b.z, b.w);
+              const float2 lo = fma2(make_float2(l[j4 * 4], l[j4 * 4 + 1]), make_float2(p.scale, p.scale), make_float2(b.x, b.y));
+              const float2 hi = fma2(make_float2(l[j4 * 4 + 2], l[j4 * 4 + 3]), make_float2(p.scale, p.scale), make_float2(b.z, b.w));
+              l[j4 * 4] = lo.x; l[j4 * 4 + 1] = lo.y; l[j4 * 4 + 2] = hi.x; l[j4 * 4 + 3] = hi.y;
             }
           } else {
             const float* ms = sMask + (g * F::MASKS + slot) * F3_KT;
@@ -511,22 +482,22 @@ attention3_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_constan
           if (c < 2) {
 #pragma unroll
             for (int j = 0; j < 16; j += 2) {
-              f3_fma2(l[c * 16 + j], l[c * 16 + j + 1], l[c * 16 + j], l[c * 16 + j + 1], L2E, L2E, shift, shift);
-              l[c * 16 + j] = f3_ex2(l[c * 16 + j]);
-              l[c * 16 + j + 1] = f3_ex2(l[c * 16 + j + 1]);
+              const float2 x = fma2(make_float2(l[c * 16 + j], l[c * 16 + j + 1]), make_float2(L2E, L2E), make_float2(shift, shift));
+              l[c * 16 + j] = f3_ex2(x.x);
+              l[c * 16 + j + 1] = f3_ex2(x.y);
             }
           }
           if (c == 1 && t > 0 && !add_product(n - 1, carry)) { ok = false; break; }
           if (c > 0) {
             float* x16 = l + (c - 1) * 16;
-            float a0 = x16[0], a1 = x16[1], a2 = x16[2], a3 = x16[3];
+            float2 a = make_float2(x16[0], x16[1]), b = make_float2(x16[2], x16[3]);
 #pragma unroll
             for (int j = 4; j < 16; j += 4) {
-              f3_add2(a0, a1, x16[j], x16[j + 1]);
-              f3_add2(a2, a3, x16[j + 2], x16[j + 3]);
+              a = add2(a, make_float2(x16[j], x16[j + 1]));
+              b = add2(b, make_float2(x16[j + 2], x16[j + 3]));
             }
-            f3_add2(a0, a1, a2, a3);
-            const float more = (a0 + a1) - lost, next = sum + more;
+            a = add2(a, b);
+            const float more = (a.x + a.y) - lost, next = sum + more;
             lost = (next - sum) - more;
             sum = next;
             uint32_t w[3][8];
@@ -536,7 +507,7 @@ attention3_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_constan
 #pragma unroll
               for (int i = 0; i < 3; ++i) {
                 w[i][e] = f3_pack(x, y);
-                if (i < 2) f3_rest(x, y, w[i][e]);
+                if (i < 2) bf16_rest(x, y, w[i][e]);
               }
             }
             tmem_st8(sbuf + (c - 1) * 16, w[0]);

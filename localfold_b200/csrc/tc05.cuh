@@ -423,16 +423,21 @@ __device__ __forceinline__ void ld_global_v8(const void* ptr, uint32_t (&v)[8]) 
                : "memory");
 }
 
-// The leading bf16 terms of x and y (x in the low half), which keep what is left of them, exactly: mixed-precision multiply-adds by -1
-__device__ __forceinline__ uint32_t split_bf16(float& x, float& y) {
-  uint32_t w;
+// x and y minus the bf16 terms in w (x's in the low half), exactly: mixed-precision multiply-adds by -1
+__device__ __forceinline__ void bf16_rest(float& x, float& y, uint32_t w) {
   asm("{\n\t.reg .b16 lo, hi, m;\n\t"
-      "cvt.rn.bf16x2.f32 %2, %1, %0;\n\t"
       "mov.b32 {lo, hi}, %2;\n\t"
       "mov.b16 m, 0xBF80;\n\t"
       "fma.rn.f32.bf16 %0, lo, m, %0;\n\t"
       "fma.rn.f32.bf16 %1, hi, m, %1;\n\t}"
-      : "+f"(x), "+f"(y), "=&r"(w));
+      : "+f"(x), "+f"(y)
+      : "r"(w));
+}
+// The leading bf16 terms of x and y, which keep what is left of them
+__device__ __forceinline__ uint32_t split_bf16(float& x, float& y) {
+  uint32_t w;
+  asm("cvt.rn.bf16x2.f32 %0, %2, %1;" : "=r"(w) : "f"(x), "f"(y));
+  bf16_rest(x, y, w);
   return w;
 }
 __device__ __forceinline__ uint32_t pack_half2(float lo, float hi) {
