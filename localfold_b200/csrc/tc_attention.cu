@@ -586,13 +586,15 @@ lf_status attention_core(lf_context* ctx, ArenaCursor& cur, const op16* q, const
   p.batch = batch; p.Q = Q; p.qtiles = (Q + FA_TILE - 1) / FA_TILE; p.ktiles = (Q + FA_KT - 1) / FA_KT;
   p.transpose = transpose; p.mask_mode = mask_mode; p.clamp = clamp; p.mask = mask; p.has_bias = bias ? 1 : 0; p.ldb = ldb; p.ldq = ldq;
   p.gate = g; p.out = out; p.status = (Status*)ctx->tc_status;
-  // Rows, whose sides bring 56 KB a key tile from L2 (with a bias; tiles: 77), unless tiles need fewer rounds of the blocks by more than the 2 %
-  // that a round is longer: few batch rows of many queries.  (Where the number of query tiles is odd, tiles leave half an item a row empty.)
-  // Tiles -> rows, two launches: 2048 queries 24.1 -> 23.6 ms (block 38.9 -> 38.2), 701 1192 -> 1199 us alone (block 2707 -> 2671, under the power cap); the six
-  // of an evoformer block with 825 and 512 queries, two of them tiles before: 4.13 -> 4.05 ms.
+  // A round of the blocks costs what its key tiles cost, so the form with fewer rounds (where the number of query tiles is odd, tiles leave half an
+  // item a row empty).  At equal rounds, with a bias: rows, whose sides share its tiles (56 KB a key tile from L2, tiles 77); 0.6 to 7 % a launch from
+  // 128 to 2048 queries and 2 to 222 rounds (256 x 256: 52.7 -> 50.4 us; 2048 x 2048: 12.34 -> 12.07 ms), about what a round more in 50 takes.
+  // Without one rows bring K and V twice and share nothing: up to five rounds tiles (203 x 203: 37.3 -> 35.3 us; 184 x 500: 91.4 -> 88.3), from then on rows,
+  // whose packed arithmetic shows (444 x 256: 74.2 -> 71.0; 444 x 512: 188.9 -> 184.8; queries that end a key tile early -2 to +1 %).
   const int64_t by_rows = (int64_t)((batch + 1) / 2) * p.qtiles * 2, by_tiles = (int64_t)batch * ((p.qtiles + 1) / 2) * 2;
   auto rounds = [&](int64_t n) { return (n + ctx->sm_count - 1) / ctx->sm_count; };
-  const bool rows = batch > 1 && 50 * rounds(by_rows) <= 51 * rounds(by_tiles);
+  const int64_t r = rounds(by_rows), t = rounds(by_tiles);
+  const bool rows = batch > 1 && (bias ? 50 * r <= 51 * t : r < t || (r == t && r > 5));
   const int64_t items = rows ? by_rows : by_tiles;
   if (items > INT32_MAX) return lf_fail(ctx, LF_ERR_UNSUPPORTED, "attention over %d rows of %d queries exceeds the work index", batch, Q);
   const int grid = (int)(items < ctx->sm_count ? items : ctx->sm_count);

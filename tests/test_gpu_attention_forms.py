@@ -20,9 +20,10 @@ def dev():
     d.close()
 
 
-# rows: up to 36 rows of 500 queries fill one round either way, 37 only as tiles, 38 neither; one row is always tiles
+# With a bias: up to 36 rows of 500 queries fill one round either way, 37 only as tiles, 38 neither; without one, 370 rows of two query tiles are five
+# rounds and the last ones as tiles; one row is always tiles
 @pytest.mark.parametrize("q,batch,transpose", [(256, 2, False), (250, 3, True), (129, 5, False), (500, 36, False), (500, 37, False), (511, 37, True), (500, 38, True),
-                                               (700, 1, False), (200, 1, True), (1100, 9, False)])
+                                               (700, 1, False), (200, 1, True), (1100, 9, False), (130, 370, False), (130, 371, True)])
 @pytest.mark.parametrize("bias", [True, False])
 def test_forms(dev, q, batch, transpose, bias):
     import localfold_b200 as lf
@@ -30,10 +31,14 @@ def test_forms(dev, q, batch, transpose, bias):
     heads, c = 4, 128
     act = d.normal(batch * q, c)
     mask = (d.rng.random((q, batch) if transpose else (batch, q)) > 0.2).astype(np.float32)
-    w = syn.af2_attention_weights(d, c, heads, 32, separate=True)
-    pb = dict(w["pairBias"], source="separate", channels=32, activations=d.normal(q, q, 32)) if bias else None
+    w = syn.af2_attention_weights(d, c, heads, 128, separate=True)
+    pb = dict(w["pairBias"], source="separate", channels=128, activations=d.normal(q, q, 128)) if bias else None
+    dev.profile(True)
     got = lf.AttentionGpu(dev).run({"activations": act, "mask": mask, "batch": batch, "queryLength": q, "channels": c, "heads": heads, "weights": w["attention"],
                                     "transpose": transpose, "pairBias": pb}, {"precision": "bf16", "variance": "two-pass"})["output"]
+    launches = dev.profile_read()["attention"][1]
+    dev.profile(False)
+    assert launches == 1      # this core, not the float32 one
     want = np.asarray(t2.attention_af2(act, mask, batch, q, c, heads, w["attention"], transpose, pb), np.float64)
     got = np.asarray(got, np.float64).reshape(want.shape)
     assert np.linalg.norm(got - want) <= 1e-3 * np.linalg.norm(want)
