@@ -45,6 +45,22 @@ def test_stacks_of_several_threads_and_devices():
     dev.close()
 
 
+def test_weights_outlive_the_devices_that_prepared_them():
+    import localfold_b200 as lf
+    d = syn.draw(8150)
+    pair, mask, w = d.normal(40, 40, 128), np.ones((40, 40), np.float32), syn.af2_pair_block_weights(d)
+    first, dev = lf.Device(0), lf.Device(0)
+    stack = lf.PairStackGpu(dev).prepare([w], 128, 128, first.uploads())
+    want = {p: stack.run(pair, mask, {"precision": p, "variance": "two-pass"})["pair"] for p in ("bf16", "f32")}
+    again = lf.PairStackGpu(dev).prepare([w], 128, 128, first.uploads())
+    first.close()      # the weights' contexts go, then the one that uses them, then the weights
+    for p in want:
+        assert np.array_equal(again.run(pair, mask, {"precision": p, "variance": "two-pass"})["pair"], want[p])
+    dev.close()
+    stack.close()
+    again.close()
+
+
 def test_a_scratch_limit_and_the_launch_count_cover_the_weights():
     """A device counts the launches of one that prepares its weights itself; a limit leaves it one arena."""
     import localfold_b200 as lf
