@@ -120,7 +120,7 @@ class Device:
         return sum(int(d.lib.lf_context_launch_count(d.handle)) for d in devices)
 
     def profile(self, enable: bool):
-        """Bracket every kernel launch with CUDA events (off by default)."""
+        """Bracket every kernel launch of the operators with CUDA events (off by default; what prepares weights is not timed)."""
         self.check(self.lib.lf_context_profile(self.handle, 1 if enable else 0))
 
     def profile_read(self) -> dict:
