@@ -278,7 +278,8 @@ gemm3_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant__ C
         for (int e = 0; e < 32; ++e) v[e] = col0 + e >= p.sigmoid_col0 && col0 + e < p.sigmoid_col1 ? g3_sigmoid(v[e]) : v[e];
       }
       if (OUT == G3_ACT) {
-        // as below, added where the activations live (no residual is read here: loads in the epilogue took 56 us where this and a pass of its own took 41)
+        // as below, added where the activations live (no residual is read here: loads in the epilogue took 56 us where this and a pass of its own took 41).
+        // The reduction flushes subnormal operands and sums to zero, where an addition in registers keeps them.
         int64_t to[4];
 #pragma unroll
         for (int i = 0; i < 4; ++i) {
@@ -434,6 +435,12 @@ lf_status gemm_f32(lf_context* ctx, ArenaCursor& cur, int major, const SplitMatr
   if (cur.dry) return LF_OK;
   if (a.ld % 8 || b.ld % 8 || a.batch_stride % 8 || b.batch_stride % 8 || a.term_stride % 8 || b.term_stride % 8 || (o.terms && o.ld % 8))
     return lf_fail(ctx, LF_ERR_ARGUMENT, "split operands need strides of whole groups of eight");
+  // What no instance below does: another output of an operand in pieces or of the row-contiguous form, a batch of what is laid out for one product
+  const int outputs = (o.out != nullptr) + (o.terms != nullptr) + (o.act != nullptr) + (o.plane_mask != nullptr);
+  if (outputs != 1 || b.pieces || (a.pieces && (major || !(o.out || o.act))) || (major && !o.out) || (batch != 1 && (a.pieces || o.pieces || o.act || o.plane_mask)) ||
+      (o.pieces && (!o.terms || !o.gate || (n > o.ld / 3 * 4 && !o.pair_bias))) || (o.act && (n % 4 || !lf_aligned16(o.act))) ||
+      (o.plane_mask && (m != (int64_t)o.plane_n * o.plane_n || n != gated_columns(o.plane_c))))
+    return lf_fail(ctx, LF_ERR_UNSUPPORTED, "float32 GEMM: no kernel of this form (%d x %d x %d, batch %d)", m, n, k, batch);
   CUtensorMap ma, mb;
   if (major == 0) {
     if (a.pieces) LF_TRY(make_map_term_pieces(ctx, &ma, a, m, 1, G3_BM, 1, G3_BK / 8, 3));
