@@ -47,7 +47,8 @@ def _want(g):
 
 # every one of these goes to the tcgen05 kernel (attention3_wins)
 SIZES = [(94, 131, 4, 16, False, True), (96, 97, 4, 32, True, True), (97, 99, 4, 32, False, False), (127, 130, 4, 16, True, False), (128, 66, 4, 32, False, True),
-         (200, 129, 8, 8, False, True), (160, 131, 8, 8, True, False), (203, 40, 4, 32, True, True), (256, 70, 8, 16, False, True), (385, 41, 4, 16, True, True)]
+         (200, 129, 8, 8, False, True), (160, 131, 8, 8, True, False), (203, 40, 4, 32, True, True), (256, 70, 8, 16, False, True), (385, 41, 4, 16, True, True),
+         (131, 161, 4, 32, False, True), (32, 885, 4, 32, True, True)]      # 32 channels with two and six items a block, of several key tiles and of one
 
 
 @pytest.mark.parametrize("q,batch,heads,dim,transpose,bias", SIZES)
@@ -69,6 +70,48 @@ def test_raised_references_and_masked_rows(dev, q, batch, heads, dim, transpose,
     got = lf.AttentionGpu(dev).run(given, {"precision": "f32", "variance": "two-pass"})["output"]
     assert np.isfinite(got).all()
     assert _relative(got, _want(given)) <= 1e-5
+
+
+def test_these_sizes_run_this_kernel(dev):
+    import localfold_b200 as lf
+    import torch
+    calls = [_case(*size) for size in SIZES] + [_square(*size)[0] for size in SQUARES]
+    with torch.profiler.profile(activities=[torch.profiler.ProfilerActivity.CUDA]) as prof:
+        for given in calls:
+            lf.AttentionGpu(dev).run(given, {"precision": "f32"})
+    names = [e.name for e in prof.events()]
+    assert sum("attention3_kernel" in name for name in names) == len(calls)
+    assert not any("mma_attention" in name for name in names)
+
+
+# the pair bias as columns of the projection: 97 is one item a block, 203 are three
+SQUARES = [(97, 4, 32, True), (203, 4, 32, False), (200, 4, 16, True), (202, 8, 8, False)]
+
+
+def _square(n, heads, dim, transpose):
+    d, c = syn.draw(6200 + n), heads * dim
+    w = syn.af2_attention_weights(d, c, heads, c)
+    return {"activations": d.normal(n * n, c), "mask": (d.rng.random((n, n)) > 0.25).astype(np.float32), "batch": n, "queryLength": n, "channels": c, "heads": heads,
+            "weights": w["attention"], "transpose": transpose, "pairBias": dict(w["pairBias"], source="normalized-input")}, d
+
+
+@pytest.mark.parametrize("n,heads,dim,transpose", SQUARES)
+def test_bias_from_the_normalised_input(dev, n, heads, dim, transpose):
+    import localfold_b200 as lf
+    given, d = _square(n, heads, dim, transpose)
+    given["pairBias"]["projectionWeight"] = given["pairBias"]["projectionWeight"] * 3
+    got = lf.AttentionGpu(dev).run(given, {"precision": "f32", "variance": "two-pass"})["output"]
+    assert _relative(got, _want(given)) <= 1e-6
+
+
+@pytest.mark.parametrize("n", [98, 131])
+@pytest.mark.parametrize("transpose,swap", [(False, False), (True, False), (True, True)])
+def test_bias_of_the_transposed_dialects(dev, n, transpose, swap):
+    import localfold_b200 as lf
+    d = syn.draw(6300 + n)
+    pair, mask, w = d.normal(n, n, 128), (d.rng.random((n, n)) > 0.25).astype(np.float32), syn.af3_grid_attention_weights(d, 128, 4, 32)
+    got = lf.Af3GridSelfAttentionGpu(dev).run(pair, mask, {"n": n, "channels": 128, "transpose": transpose}, w, {"swapTransposedBias": swap}, {"precision": "f32"})["output"]
+    assert _relative(got, t2.grid_attention_af3(pair, mask, w, transpose, swap)) <= 1e-6
 
 
 def test_what_is_not_finite_stays_in_its_row(dev):

@@ -65,6 +65,52 @@ def test_attention_with_a_residual(dev, n, heads, dim, transpose):
     assert _relative(got, act.astype(np.float64) + want) <= 1e-6
 
 
+# ---- device tensors updated in place: the last GEMM adds to them, a launch less than from host arrays, whose result goes to another buffer ----
+
+OPTIONS = {"precision": "f32", "variance": "two-pass", "residual": True}
+
+
+def _in_place(run, act, mask):
+    import torch
+    x = torch.from_numpy(act).cuda()
+    here, there = run(x, torch.from_numpy(mask).cuda(), x), run(act, mask, None)
+    assert here["launches"] == there["launches"] - 1
+    return x.cpu().numpy()
+
+
+@pytest.mark.parametrize("n,c,hidden", [(1, 16, 16), (31, 20, 24), (40, 64, 64), (129, 4, 30)])
+def test_triangle_update_in_place(dev, n, c, hidden):
+    import localfold_b200 as lf
+    d = syn.draw(7600 + n)
+    z, mask, w = d.normal(n, n, c), (d.rng.random((n, n)) > 0.2).astype(np.float32), _with_biases(d, syn.af2_triangle_weights(d, c, hidden))
+    mask[0, 0] = 1
+    op, shape = lf.TriangleMultiplicationOutgoingGpu(dev), {"length": n, "cZ": c, "cHidden": hidden}
+    got = _in_place(lambda z, mask, out: op.run({"shape": shape, "z": z, "mask": mask, "weights": w}, OPTIONS, out=out), z, mask)
+    assert _relative(got, z + t2.trimul_af2(z, mask, w)) <= 1e-6
+
+
+@pytest.mark.parametrize("rows,c", [(1, 8), (130, 36), (257, 64)])
+def test_transition_in_place(dev, rows, c):
+    import localfold_b200 as lf
+    d = syn.draw(7700 + rows)
+    act, w = d.normal(rows, c), _with_biases(d, syn.af2_transition_weights(d, c))
+    given = {"rows": rows, "channels": c, "hiddenChannels": 4 * c, "weights": w}
+    got = _in_place(lambda act, _, out: lf.TransitionGpu(dev).run(dict(given, activations=act), OPTIONS, out=out), act, np.ones(1, np.float32))
+    assert _relative(got, act + t2.transition_af2(act, w)) <= 1e-6
+
+
+@pytest.mark.parametrize("transpose", [False, True])
+@pytest.mark.parametrize("batch,q,heads,dim", [(3, 31, 1, 8), (65, 33, 2, 22), (97, 97, 4, 32)])
+def test_attention_in_place(dev, batch, q, heads, dim, transpose):
+    import localfold_b200 as lf
+    d, c = syn.draw(7800 + q), heads * dim
+    act, mask = d.normal(batch * q, c), np.ones((q, batch) if transpose else (batch, q), np.float32)
+    w = _with_biases(d, syn.af2_attention_weights(d, c, heads)["attention"])
+    given = {"batch": batch, "queryLength": q, "channels": c, "heads": heads, "weights": w, "transpose": transpose}
+    got = _in_place(lambda act, mask, out: lf.AttentionGpu(dev).run(dict(given, activations=act, mask=mask), OPTIONS, out=out), act, mask)
+    assert _relative(got, act + t2.attention_af2(act, mask, batch, q, c, heads, w, transpose)) <= 1e-6
+
+
 # ---- a gate that is not a number: one channel of the gating weights ----
 
 
