@@ -16,8 +16,8 @@
 // What bounds it: issue slots (65 % of them busy at 384 x 384) and the round trips of a tile; the exponents take a quarter of their unit's time, the tensor
 // core a third.  An exponential costs its share of 17 instructions, six of them to take it apart and three to add the products up.  Two streams
 // with tiles of 64 keys, two softmax warps a scheduler, took a tenth longer; with the next logits requested during the exponentials another tenth.
-// Against the mma.sync kernel (mma_attention.cuh; a warp's chain of dependent MMAs): 384 x 384, 4 heads of 16: 465 -> 192 us; 203 x 203,
-// 4 x 32: 184 -> 85; 1024 x 256, 8 x 8: 936 -> 478.
+// Against the mma.sync kernel (mma_attention.cuh; a warp's chain of dependent MMAs): 384 x 384, 4 heads of 16: 465 -> 198 us; 203 x 203,
+// 4 x 32: 184 -> 84; 1024 x 256, 8 x 8: 936 -> 485.
 #include <cuda.h>
 
 #include "tc05.cuh"

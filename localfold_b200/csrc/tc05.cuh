@@ -27,7 +27,7 @@ __device__ __forceinline__ uint32_t smem_u32(const void* p) {
 
 // The first 1024-byte boundary of a block's shared memory.  align_shared is an offset to the array: a pointer that went through an integer
 // (align_generic) is a generic one to the compiler, and the accesses and barrier addresses by it cost more instructions.  With the
-// offset: triangle projection 39.9 -> 38.0 us, triangle output 44.5 -> 41.4, transition 68.7 -> 64.5, GEMM 31.1 -> 29.3 (N = 384); float32
+// offset, pairs timed in turn (later runs of the float32 core: 198): triangle projection 39.9 -> 38.0 us, triangle output 44.5 -> 41.4, transition 68.7 -> 64.5, GEMM 31.1 -> 29.3 (N = 384); float32
 // attention core 208 -> 189, float32 projections 59 -> 57.5, 41 -> 38.6 and 34.6 -> 32.6 (template pair, N = 384).  Two kernels that are short
 // of registers keep the generic pointer, for the compiler spills or reorders with the other one: attention projection 50.3 -> 54.4 (its
 // barriers alone by the offset: 49.2), flash core's tiles form 593 -> 648 at N = 701 (its barriers alone: 609).
